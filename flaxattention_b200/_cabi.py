@@ -12,6 +12,7 @@ from typing import Optional
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libflaxattn.so")
+HOST_PATH = os.path.join(_HERE, "_host.so")
 
 FA_F16, FA_BF16, FA_F32 = 0, 1, 2
 FLAG_ROUND_SCORES = 1
@@ -34,6 +35,7 @@ class FaBlockTables(C.Structure):
         ("q_block_size", C.c_int32), ("kv_block_size", C.c_int32),
         ("mask_bits", C.c_void_p), ("mask_bits_stride", C.c_int64), ("mask_bits_rows", C.c_int32),
         ("mask_bits_B", C.c_int32), ("mask_bits_H", C.c_int32),
+        ("mask_bits_t", C.c_void_p), ("mask_bits_t_stride", C.c_int64), ("mask_bits_t_rows", C.c_int32),
     ]
 
 
@@ -67,7 +69,7 @@ EXPORTS = [
     "fa_bwd", "fa_decode_num_splits", "fa_decode_workspace_bytes", "fa_decode",
     "fa_block_mask_workspace_bytes", "fa_block_mask", "fa_decode_static_capacity", "fa_decode_static",
     "fa_profile_enable", "fa_profile_read", "fa_decode_packs_heads", "fa_selftest_bounded_wait",
-    "fa_mask_bits_row_words", "fa_mask_bits",
+    "fa_mask_bits_row_words", "fa_mask_bits", "fa_block_mask_build",
 ]
 
 
@@ -133,6 +135,34 @@ def lib() -> C.CDLL:
             pass
     _lib = L
     return L
+
+
+_host = None
+
+
+def host():
+    """The native host path (csrc/host.cpp).  Raises if it has not been built, like ``lib()``."""
+    global _host
+    if _host is not None:
+        return _host
+    lib()  # _host.so links against it and uses the same copy
+    from .csrc.build import host_is_current
+
+    if not os.path.exists(HOST_PATH) or not host_is_current():
+        raise FlaxAttnError(
+            -3, f"{HOST_PATH} is missing or was built from other sources; build it with "
+                "`python -m flaxattention_b200.csrc.build`")
+    import importlib.machinery
+    import importlib.util
+
+    import torch  # noqa: F401  (its libraries have to be loaded first)
+
+    loader = importlib.machinery.ExtensionFileLoader("_host", HOST_PATH)
+    spec = importlib.util.spec_from_file_location("_host", HOST_PATH, loader=loader)
+    mod = importlib.util.module_from_spec(spec)
+    loader.exec_module(mod)
+    _host = mod
+    return mod
 
 
 def check(rc: int) -> None:

@@ -18,17 +18,13 @@ import numpy as np
 import torch
 
 from . import _cabi
-from .blockmask import BlockMask, bind_mod_buffers, module_for, noop_mask
+from .blockmask import BlockMask, bind_mod_buffers, identity_score as _identity, module_for, noop_mask
 
 _DTYPES = {torch.float16: _cabi.FA_F16, torch.bfloat16: _cabi.FA_BF16, torch.float32: _cabi.FA_F32}
 
 # decode path: query blocks of at most this many rows go through the split-KV kernel
 DECODE_MAX_SQ = 64
 DECODE_MIN_SKV = 512
-
-
-def _identity(score, batch, head, token_q, token_kv):
-    return score
 
 
 def _validate_sdpa_input(query, key, value):
@@ -86,6 +82,7 @@ def _status() -> torch.Tensor:
     global _status_word
     if _status_word is None:
         _status_word = torch.zeros(1, dtype=torch.int32).pin_memory()
+        _cabi.host().setup(_status_word.data_ptr(), _identity, noop_mask, _cabi.FlaxAttnError)
     return _status_word
 
 
@@ -168,13 +165,17 @@ class _Call:
             t.mask_B, t.mask_H = bm.kv_indices.shape[0], bm.kv_indices.shape[1]
             t.num_q_blocks, t.num_kv_blocks = bm.kv_indices.shape[2], bm.kv_indices.shape[3]
             t.q_block_size, t.kv_block_size = bm.BLOCK_SIZE
-            mb = getattr(bm, "mask_bits", None)
+            mb = bm.mask_bits if bm.bits_hold() else None
             if mb is not None and self.mask_mod is bm.mask_mod and mb.device == q.device and mb.shape[2] >= self.Sq \
                     and mb.shape[3] * 32 >= self.Skv and mb.shape[0] in (1, self.B) and mb.shape[1] in (1, self.Hq):
                 if mb.dtype != torch.int32 or not mb.is_contiguous():
                     raise ValueError("BlockMask.mask_bits must be a contiguous int32 tensor")
                 t.mask_bits, t.mask_bits_stride, t.mask_bits_rows = mb.data_ptr(), mb.shape[3], mb.shape[2]
                 t.mask_bits_B, t.mask_bits_H = mb.shape[0], mb.shape[1]
+                mt = bm.mask_bits_t
+                if mt is not None and mt.device == q.device and mt.dtype == torch.int32 and mt.is_contiguous() \
+                        and mt.shape[:2] == mb.shape[:2] and mt.shape[2] >= self.Skv and mt.shape[3] * 32 >= self.Sq:
+                    t.mask_bits_t, t.mask_bits_t_stride, t.mask_bits_t_rows = mt.data_ptr(), mt.shape[3], mt.shape[2]
             for x in (bm.kv_num_blocks, bm.kv_indices, bm.full_kv_num_blocks, bm.full_kv_indices, bm.q_num_blocks,
                       bm.q_indices, bm.full_q_num_blocks, bm.full_q_indices):
                 if x is not None and (x.dtype != torch.int32 or not x.is_contiguous()):
@@ -296,6 +297,12 @@ def flax_attention(
     ``b_offset`` / ``h_offset`` are the global indices of the first batch / head of a
     batch x heads shard; the mods see global indices.
     """
+    if kernel_options is None and isinstance(query, torch.Tensor) and query.is_cuda:
+        res = _cabi.host().attention(query, key, value, score_mod, None, block_mask, scale, enable_gqa, return_lse, False,
+                                     True, b_offset, h_offset)
+        if res is not None:
+            return res
+    # not a plain call on CUDA tensors with mods that are known already
     query, from_np = _as_cuda(query)
     key, _ = _as_cuda(key)
     value, _ = _as_cuda(value)
@@ -388,6 +395,11 @@ def flax_attention_pallas(
     validates it), and an optional ``block_mask`` enables block skipping (its ``mask_mod``
     is used when ``mask_mod`` is not given)."""
     del block_q, block_k
+    if isinstance(query, torch.Tensor) and query.is_cuda:
+        res = _cabi.host().attention(query, key, value, score_mod, mask_mod, block_mask, sm_scale, enable_gqa, return_lse,
+                                     not bhln, False, b_offset, h_offset)
+        if res is not None:
+            return res
     query, from_np = _as_cuda(query)
     key, _ = _as_cuda(key)
     value, _ = _as_cuda(value)

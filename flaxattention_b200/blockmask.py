@@ -28,7 +28,7 @@ from typing import Callable, Optional, Tuple, Union
 
 import torch
 
-from . import _cabi
+from . import _cabi, modtrace
 from .modtrace import lower_mods, mod_arity
 
 _DEFAULT_SPARSE_BLOCK_SIZE = 128
@@ -114,9 +114,12 @@ class BlockMask:
     # not part of the reference's BlockMask: the kernels read it on partial tiles instead of
     # evaluating mask_mod there
     mask_bits: Optional[torch.Tensor] = None
+    # the same matrix transposed [1 or B, 1 or H, KV_LEN, words], or None
+    mask_bits_t: Optional[torch.Tensor] = None
 
     def __init__(self, kv_num_blocks, kv_indices, full_kv_num_blocks, full_kv_indices, q_num_blocks, q_indices,
-                 full_q_num_blocks, full_q_indices, BLOCK_SIZE, mask_mod, mask_bits=None):
+                 full_q_num_blocks, full_q_indices, BLOCK_SIZE, mask_mod, mask_bits=None, mask_bits_t=None,
+                 _bits_sources=()):
         if kv_indices.ndim < 2:
             raise RuntimeError("BlockMask must have at least 2 dimensions")
         assert kv_num_blocks is not None, "kv_num_blocks must be provided"
@@ -140,6 +143,15 @@ class BlockMask:
         self.BLOCK_SIZE = BLOCK_SIZE
         self.mask_mod = mask_mod
         self.mask_bits = mask_bits
+        self.mask_bits_t = mask_bits_t
+        # the bit matrices hold for this mask_mod, and while the tensors it captures are at these versions
+        self._bits_mod = mask_mod
+        self._bits_sources = _bits_sources
+
+    def bits_hold(self) -> bool:
+        """Whether ``mask_bits`` is still what ``mask_mod`` gives."""
+        return (self.mask_bits is not None and self.mask_mod is self._bits_mod
+                and all(t._version == v for t, v in self._bits_sources))
 
     @classmethod
     def from_kv_blocks(cls, kv_num_blocks, kv_indices, full_kv_num_blocks=None, full_kv_indices=None,
@@ -207,7 +219,13 @@ class BlockMask:
         return BlockMask(mv(self.kv_num_blocks), mv(self.kv_indices), mv(self.full_kv_num_blocks),
                          mv(self.full_kv_indices), mv(self.q_num_blocks), mv(self.q_indices),
                          mv(self.full_q_num_blocks), mv(self.full_q_indices), self.BLOCK_SIZE, self.mask_mod,
-                         mv(self.mask_bits))
+                         *self._moved_bits(mv))
+
+    def _moved_bits(self, fn):
+        """(mask_bits, mask_bits_t, sources) of a copy whose tensors went through ``fn``."""
+        if not self.bits_hold():
+            return None, None, ()
+        return fn(self.mask_bits), fn(self.mask_bits_t), self._bits_sources
 
     def shard(self, b_slice: slice, h_slice: slice) -> "BlockMask":
         """Tables of one batch x heads shard (broadcast axes are kept whole)."""
@@ -220,7 +238,7 @@ class BlockMask:
         return BlockMask(cut(self.kv_num_blocks), cut(self.kv_indices), cut(self.full_kv_num_blocks),
                          cut(self.full_kv_indices), cut(self.q_num_blocks), cut(self.q_indices),
                          cut(self.full_q_num_blocks), cut(self.full_q_indices), self.BLOCK_SIZE, self.mask_mod,
-                         cut(self.mask_bits))
+                         *self._moved_bits(cut))
 
     def __repr__(self):
         def shape_or_none(x):
@@ -263,15 +281,33 @@ _MODULES = {}
 
 
 def module_for(score_mod: Optional[Callable], mask_mod: Optional[Callable]):
-    """Lowered mods -> compiled-kernel module, cached per generated source."""
+    """Lowered mods -> compiled-kernel module, cached per generated source.  The pair is also made
+    known to the native host path, which then takes calls with it."""
     if mask_mod is noop_mask:
         mask_mod = None
+    if score_mod is identity_score:
+        score_mod = None
     ms = lower_mods(score_mod, mask_mod)
     m = _MODULES.get(ms.key)
     if m is None:
         m = _cabi.Module(ms.source)
         _MODULES[ms.key] = m
+    if all(isinstance(t, torch.Tensor) for t in ms.buffers):
+        _cabi.host().register(score_mod, mask_mod, m, m.handle.value, tuple(ms.buffers))
     return m
+
+
+def identity_score(score, batch, head, token_q, token_kv):
+    """The score_mod of a call without one."""
+    return score
+
+
+def _forget_pair(score_id: int, mask_id: int) -> None:
+    if _cabi._host is not None:
+        _cabi._host.forget(score_id, mask_id)
+
+
+modtrace._ON_FORGET.append(_forget_pair)
 
 
 _DEVICE_BUFFERS = {}
@@ -284,10 +320,19 @@ def bind_mod_buffers(module, score_mod: Optional[Callable], mask_mod: Optional[C
     copied to `device` once per tensor version; the copies are kept while the mods are cached."""
     if mask_mod is noop_mask:
         mask_mod = None
+    if score_mod is identity_score:
+        score_mod = None
     ms = lower_mods(score_mod, mask_mod)
     if not ms.buffers:
         return
-    ptrs, keep = [], []
+    keep = _device_buffers(ms, device)
+    module.set_buffers([t.data_ptr() for t in keep])
+    module._bound_buffers = keep  # the addresses stay valid at least until the next binding
+
+
+def _device_buffers(ms, device):
+    """The captured tensors of a lowered pair on ``device``."""
+    keep = []
     for t in ms.buffers:
         if not isinstance(t, torch.Tensor):
             t = torch.as_tensor(t)
@@ -304,9 +349,7 @@ def bind_mod_buffers(module, score_mod: Optional[Callable], mask_mod: Optional[C
                 _DEVICE_BUFFERS[key] = hit
             t = hit[1]
         keep.append(t)
-        ptrs.append(t.data_ptr())
-    module.set_buffers(ptrs)
-    module._bound_buffers = keep  # the addresses stay valid at least until the next binding
+    return keep
 
 
 # finished tables of create_block_mask(..., _compile=True), least recently used first
@@ -318,6 +361,8 @@ def _require_cuda(device) -> torch.device:
     if not torch.cuda.is_available():
         raise RuntimeError("flaxattention_b200 needs a CUDA device (B200, sm_100a); there is no CPU path")
     dev = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
+    if dev.type == "cuda" and dev.index is None:
+        dev = torch.device("cuda", torch.cuda.current_device())
     if dev.type != "cuda":
         raise RuntimeError(f"flaxattention_b200 tensors must live on a CUDA device, got {dev}")
     return dev
@@ -326,31 +371,17 @@ def _require_cuda(device) -> torch.device:
 _MASK_BITS_MAX_BYTES = 64 << 20
 
 
-def _build_mask_bits(module, mask_mod, B, H, Q_LEN, KV_LEN, b_offset, h_offset, dev, force):
-    """The bit matrix of ``mask_mod`` (see create_block_mask), or None.  Called with ``dev`` current
-    and the module's captured buffers bound."""
-    if force is False or mask_mod is noop_mask:
-        return None
-    ms = lower_mods(None, mask_mod)
-    if ms.buffers and force is not True:
-        return None
-    # a mask whose device code never names b (h) is the same for every batch entry (head)
-    import re
-    m = re.search(r"fa_mask_mod\(int b, int h, int q, int kv\) \{(.*?)\n\}", ms.source, re.S)
-    body = m.group(1) if m else "b h"
-    reads_b, reads_h = re.search(r"\bb\b", body) is not None, re.search(r"\bh\b", body) is not None
-    nb = B if reads_b else 1
-    nh = H if reads_h else 1
-    L = _cabi.lib()
-    words = int(L.fa_mask_bits_row_words(KV_LEN))
-    if force is not True and nb * nh * Q_LEN * words * 4 > _MASK_BITS_MAX_BYTES:
-        return None
-    if nb * nh > 65535 or Q_LEN > 65535:
-        return None
-    bits = torch.empty(nb, nh, Q_LEN, words, dtype=torch.int32, device=dev)
-    _cabi.check(L.fa_mask_bits(module.handle, nb, nh, Q_LEN, KV_LEN, b_offset if reads_b else 0,
-                               h_offset if reads_h else 0, bits.data_ptr(), torch.cuda.current_stream(dev).cuda_stream))
-    return bits
+def _wants_bits(ms, nb, nh, Q_LEN, KV_LEN, Q_BLOCK_SIZE, KV_BLOCK_SIZE, force) -> bool:
+    """Whether the bit matrices of a mask are built beside its tables."""
+    if force is False or ms.mask is None:
+        return False
+    if (Q_LEN > Q_BLOCK_SIZE and Q_BLOCK_SIZE % 32) or (KV_LEN > KV_BLOCK_SIZE and KV_BLOCK_SIZE % 32):
+        return False  # blocks of part words
+    if force is True:
+        return True
+    if any(not isinstance(t, torch.Tensor) or t.is_inference() for t in ms.buffers):
+        return False  # no version counter: a later change of the captured tensor could not be noticed
+    return nb * nh * Q_LEN * (KV_LEN + 127) // 128 * 16 <= _MASK_BITS_MAX_BYTES
 
 
 def create_block_mask(
@@ -381,8 +412,10 @@ def create_block_mask(
     position where the reference's ``create_mask`` materialises a boolean,
     flaxattention/core/blockmask.py:277-322), one entry along batch / heads when ``mask_mod`` does
     not read ``b`` / ``h``: on the partial tiles the attention kernels read a row's words instead of
-    evaluating ``mask_mod`` 128 times per row.  It is built when it takes at most 64 MiB and the mask
-    reads no captured tensor (``_mask_bits=True`` / ``False`` forces it on or off).
+    evaluating ``mask_mod`` 128 times per row.  It is built when it takes at most 64 MiB
+    (``_mask_bits=True`` / ``False`` forces it on or off), from the same evaluation as the tables.  For a
+    mask that reads captured tensors the attention calls use it only as long as these have not been
+    written to since (their version counters tell).
     """
     if mod_arity(mask_mod) not in (4, 5):
         raise AssertionError("mask_mod must take (b, h, q_idx, kv_idx) or (score, b, h, q_idx, kv_idx)")
@@ -402,35 +435,33 @@ def create_block_mask(
     KV_LEN = _round_up_to_multiple(KV_LEN, KV_BLOCK_SIZE)
     dev = _require_cuda(device)
     nq, nkv = Q_LEN // Q_BLOCK_SIZE, KV_LEN // KV_BLOCK_SIZE
-    module = module_for(None, mask_mod)
+    mask = None if mask_mod is noop_mask else mask_mod
+    host = _cabi.host()
+    module = module_for(None, mask)
+    ms = lower_mods(None, mask)
     cache_key = None
-    if _compile:
-        ms = lower_mods(None, None if mask_mod is noop_mask else mask_mod)
-        if not ms.buffers:
-            cache_key = (ms.key, B, H, Q_LEN, KV_LEN, Q_BLOCK_SIZE, KV_BLOCK_SIZE, int(b_offset), int(h_offset), str(dev))
-            hit = _TABLE_CACHE.get(cache_key)
-            if hit is not None:
-                _TABLE_CACHE.move_to_end(cache_key)
-                return BlockMask(*hit[:8], (Q_BLOCK_SIZE, KV_BLOCK_SIZE), mask_mod, hit[8])
-    L = _cabi.lib()
-    with torch.cuda.device(dev):
-        mk = lambda *s: torch.empty(*s, dtype=torch.int32, device=dev)  # noqa: E731
-        kv_num, kv_idx = mk(B, H, nq), mk(B, H, nq, nkv)
-        fkv_num, fkv_idx = mk(B, H, nq), mk(B, H, nq, nkv)
-        q_num, q_idx = mk(B, H, nkv), mk(B, H, nkv, nq)
-        fq_num, fq_idx = mk(B, H, nkv), mk(B, H, nkv, nq)
-        ws_bytes = L.fa_block_mask_workspace_bytes(B, H, Q_LEN, KV_LEN, Q_BLOCK_SIZE, KV_BLOCK_SIZE)
-        ws = torch.empty(ws_bytes, dtype=torch.int8, device=dev)
-        bind_mod_buffers(module, None, mask_mod, dev)
-        _cabi.check(L.fa_block_mask(
-            module.handle, B, H, Q_LEN, KV_LEN, Q_BLOCK_SIZE, KV_BLOCK_SIZE, b_offset, h_offset,
-            kv_num.data_ptr(), kv_idx.data_ptr(), fkv_num.data_ptr(), fkv_idx.data_ptr(),
-            q_num.data_ptr(), q_idx.data_ptr(), fq_num.data_ptr(), fq_idx.data_ptr(),
-            ws.data_ptr(), ws_bytes, torch.cuda.current_stream(dev).cuda_stream))
-        bits = _build_mask_bits(module, mask_mod, B, H, Q_LEN, KV_LEN, b_offset, h_offset, dev, _mask_bits)
+    if _compile and not ms.buffers:
+        cache_key = (ms.key, B, H, Q_LEN, KV_LEN, Q_BLOCK_SIZE, KV_BLOCK_SIZE, int(b_offset), int(h_offset), str(dev))
+        hit = _TABLE_CACHE.get(cache_key)
+        if hit is not None:
+            _TABLE_CACHE.move_to_end(cache_key)
+            return BlockMask(*hit[:8], (Q_BLOCK_SIZE, KV_BLOCK_SIZE), mask_mod, *hit[8:])
+    # a mask that does not read the batch (head) index is evaluated once for all of them
+    nb, nh = (B if ms.mask_reads_b else 1), (H if ms.mask_reads_h else 1)
+    b0, h0 = (int(b_offset) if ms.mask_reads_b else 0), (int(h_offset) if ms.mask_reads_h else 0)
+    want_bits = _wants_bits(ms, nb, nh, Q_LEN, KV_LEN, Q_BLOCK_SIZE, KV_BLOCK_SIZE, _mask_bits)
+    sources = tuple((t, t._version) for t in ms.buffers) if want_bits and ms.buffers and not any(
+        not isinstance(t, torch.Tensor) or t.is_inference() for t in ms.buffers) else ()
+    elsewhere = any(not isinstance(t, torch.Tensor) or t.device != dev for t in ms.buffers)
+    if elsewhere:
+        # captured arrays that live elsewhere: this build reads their copies on `dev`
+        host.register(None, mask, module, module.handle.value, tuple(_device_buffers(ms, dev)))
+    tables = host.build_block_mask(None, mask, dev.index, B, H, nb, nh, Q_LEN, KV_LEN, Q_BLOCK_SIZE, KV_BLOCK_SIZE, b0, h0,
+                                   int(want_bits))
+    if elsewhere:
+        host.forget(0, id(mask))
     if cache_key is not None:
-        _TABLE_CACHE[cache_key] = (kv_num, kv_idx, fkv_num, fkv_idx, q_num, q_idx, fq_num, fq_idx, bits)
+        _TABLE_CACHE[cache_key] = tables
         while len(_TABLE_CACHE) > _TABLE_CACHE_MAX:
             _TABLE_CACHE.popitem(last=False)
-    return BlockMask(kv_num, kv_idx, fkv_num, fkv_idx, q_num, q_idx, fq_num, fq_idx,
-                     (Q_BLOCK_SIZE, KV_BLOCK_SIZE), mask_mod, bits)
+    return BlockMask(*tables[:8], (Q_BLOCK_SIZE, KV_BLOCK_SIZE), mask_mod, tables[8], tables[9], sources)

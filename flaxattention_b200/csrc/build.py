@@ -15,6 +15,8 @@ NVCC = os.path.join(CUDA_HOME, "bin", "nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 
+HOST = os.path.join(PKG, "_host.so")
+HOST_STAMP = HOST + ".sources"  # the same for the native host path
 STAMP = LIB + ".sources"  # hash of the sources the library was built from
 
 
@@ -64,6 +66,46 @@ def build_library(force: bool = False, verbose: bool = False) -> str:
     return LIB
 
 
+def host_hash() -> str:
+    """Hash of what _host.so is compiled from: its source, the C ABI, and the torch it is built against."""
+    import torch
+
+    h = hashlib.sha256(torch.__version__.encode())
+    for path in (os.path.join(HERE, "host.cpp"), os.path.join(PKG, "..", "include", "flaxattn.h")):
+        with open(path, "rb") as f:
+            h.update(f.read())
+        h.update(b"\0")
+    return h.hexdigest()
+
+
+def host_is_current() -> bool:
+    if not (os.path.exists(HOST) and os.path.exists(HOST_STAMP)):
+        return False
+    with open(HOST_STAMP) as f:
+        return f.read().strip() == host_hash()
+
+
+def build_host(force: bool = False) -> str:
+    """Builds _host.so, the CPython module of host.cpp (links libflaxattn.so and the installed torch)."""
+    if not force and host_is_current():
+        return HOST
+    import sysconfig
+
+    import torch
+
+    tdir = os.path.dirname(torch.__file__)
+    inc = [os.path.join(tdir, "include"), os.path.join(tdir, "include", "torch", "csrc", "api", "include"),
+           os.path.join(CUDA_HOME, "include"), sysconfig.get_paths()["include"]]
+    cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", os.path.join(HERE, "host.cpp"), "-o", HOST,
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(x for p in inc for x in ("-isystem", p)),
+           "-L" + PKG, "-l:libflaxattn.so", "-Wl,-rpath,$ORIGIN", "-L" + os.path.join(tdir, "lib"),
+           "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", "-ltorch_python"]
+    subprocess.run(cmd, check=True, cwd=HERE)
+    with open(HOST_STAMP, "w") as f:
+        f.write(host_hash() + "\n")
+    return HOST
+
+
 def build_ffi_shim() -> str:
     """Builds libflaxattn_ffi.so (the jax.ffi handlers of ffi_shim.cc).  Needs the XLA FFI headers
     that ship with jaxlib; raises where JAX is not installed."""
@@ -79,5 +121,6 @@ def build_ffi_shim() -> str:
 
 if __name__ == "__main__":
     print(build_library(force="--force" in sys.argv, verbose="-v" in sys.argv))
+    print(build_host(force="--force" in sys.argv))
     if "--ffi" in sys.argv:
         print(build_ffi_shim())

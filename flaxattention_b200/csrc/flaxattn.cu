@@ -25,6 +25,7 @@
 #include <mutex>
 #include <sstream>
 #include <string>
+#include <unordered_map>
 #include <vector>
 
 #include "../../include/flaxattn.h"
@@ -161,7 +162,7 @@ struct Kernel {
   cudaLibrary_t lib = nullptr;
   cudaKernel_t fn = nullptr;
   int smem = 0;
-  unsigned long long smem_set_mask = 0;  // devices on which the dynamic smem limit was raised
+  std::atomic<unsigned long long> ready{0};  // devices on which the kernel is loaded and its dynamic smem limit raised
   fa_module* owner = nullptr;
   // device address of the kernel image's `fa_mod_buf` table per device (null: the image has none)
   void* buf_table[64] = {nullptr};
@@ -170,11 +171,11 @@ struct Kernel {
 
 }  // namespace
 
-constexpr int kMaxModBuffers = 8;
+constexpr int kMaxModBuffers = FA_MAX_MOD_BUFS;
 
 struct fa_module {
   std::string mod_source;
-  std::map<std::string, Kernel*> kernels;  // key: template + defines
+  std::unordered_map<uint64_t, Kernel*> kernels;  // key: kernel_key of the variant
   const void* bufs[kMaxModBuffers] = {nullptr};  // device addresses of the captured buffers of the mods
   int nbufs = 0;
 };
@@ -187,19 +188,29 @@ const char* const kDefaultMods =
     "__device__ __forceinline__ float fa_score_mod_grad(float, int, int, int, int) { return 1.0f; }\n"
     "__device__ __forceinline__ bool fa_mask_mod(int, int, int, int) { return true; }\n";
 
-// Returns the compiled kernel `entry` of `tmpl` with the given defines (compiling if needed).
-int get_kernel(fa_module* m, const std::string& tmpl, const std::string& defines, const std::string& entry,
-               int smem, Kernel** out) {
+// A kernel variant of a module as a number: every launch looks its kernel up by it, and the define text
+// is only put together when the variant has to be compiled or fetched from the cache on disk.
+enum KernelId : int { kIdFwd, kIdFwdTc, kIdBwdDq, kIdBwdDkdv, kIdBwdTc, kIdDecode, kIdMaskScan, kIdMaskClassify, kIdSelftest };
+uint64_t kernel_key(KernelId id, std::initializer_list<std::pair<int, int>> fields) {  // (value, bits)
+  uint64_t k = 0;
+  for (auto& f : fields) k = (k << f.second) | (uint64_t)f.first;
+  return k | (uint64_t)id << 58;
+}
+
+// Returns the compiled kernel `entry` of `tmpl` with the defines `make_defines` writes (compiling if needed).
+template <class MakeDefines>
+int get_kernel(fa_module* m, uint64_t key, const char* tmpl, MakeDefines make_defines, const char* entry, int smem,
+               Kernel** out) {
   std::lock_guard<std::mutex> lk(g_mu);
-  const std::string key = tmpl + "|" + defines + "|" + entry;
   auto it = m->kernels.find(key);
   if (it != m->kernels.end()) {
     *out = it->second;
     return FA_OK;
   }
+  const std::string defines = make_defines();
   std::string th;
   if (int rc = templates_hash(th)) return rc;
-  std::string src = defines + "\n" + m->mod_source + "\n#include \"" + tmpl + "\"\n";
+  std::string src = defines + "\n" + m->mod_source + "\n#include \"" + std::string(tmpl) + "\"\n";
   std::vector<std::string> opts = {"--gpu-architecture=sm_100a", "-std=c++17", "-lineinfo",
                                    "-I" + kernel_dir()};
   int major = 0, minor = 0;
@@ -234,23 +245,25 @@ int get_kernel(fa_module* m, const std::string& tmpl, const std::string& defines
 
 // Loads the kernel on first launch and raises its dynamic shared-memory limit on this device.
 int ready_kernel(Kernel* k) {
+  int dev = 0;
+  FA_CUDA_CHECK(cudaGetDevice(&dev));
+  const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
+  if (bit != 0 && (k->ready.load(std::memory_order_acquire) & bit)) return FA_OK;
   std::lock_guard<std::mutex> lk(g_mu);
   if (k->fn == nullptr) {
     FA_CUDA_CHECK(cudaLibraryLoadData(&k->lib, k->cubin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0));
     FA_CUDA_CHECK(cudaLibraryGetKernel(&k->fn, k->lib, k->entry.c_str()));
   }
-  int dev = 0;
-  FA_CUDA_CHECK(cudaGetDevice(&dev));
-  if (dev < 64 && !(k->smem_set_mask >> dev & 1ull)) {
-    if (k->smem > 48 * 1024)
-      FA_CUDA_CHECK(cudaFuncSetAttribute((const void*)k->fn, cudaFuncAttributeMaxDynamicSharedMemorySize, k->smem));
-    k->smem_set_mask |= 1ull << dev;
-  }
+  if (k->smem > 48 * 1024)
+    FA_CUDA_CHECK(cudaFuncSetAttribute((const void*)k->fn, cudaFuncAttributeMaxDynamicSharedMemorySize, k->smem));
+  k->ready.fetch_or(bit, std::memory_order_release);
   return FA_OK;
 }
 
-// Mods that read captured buffers find their addresses in the `fa_mod_buf` table of the kernel
-// image: it is rewritten, in stream order, before every launch of a kernel of such a module.
+// Mods that read captured buffers find their addresses in the `fa_mod_buf` table.  Generated mods keep it
+// in shared memory, filled from the kernel parameters; a hand-written mod source may declare it
+// __constant__ instead, and then the table of the kernel image is rewritten, in stream order, before
+// every launch of a kernel of such a module.
 int upload_buffers(Kernel* k, void* stream) {
   fa_module* m = k->owner;
   if (m == nullptr) return FA_OK;
@@ -337,19 +350,47 @@ struct ProfScope {
   }
 };
 
+// Every kernel of the library begins with griddepcontrol.wait, before its first access to global memory,
+// and is launched with programmatic stream serialisation: its CTAs may be scheduled as soon as those of
+// the kernel in front of it on the stream have all finished or let their dependents go
+// (griddepcontrol.launch_dependents), and the launch itself hides behind that kernel's tail.  The wait
+// returns when the kernel in front is complete and its writes are visible.
+cudaLaunchConfig_t launch_config(dim3 grid, dim3 block, int smem, void* stream, cudaLaunchAttribute* attr) {
+  attr->id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr->val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = (size_t)smem;
+  cfg.stream = (cudaStream_t)stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cfg;
+}
 int launch(Kernel* k, dim3 grid, dim3 block, void* params, void* stream) {
   if (int rc = ready_kernel(k)) return rc;
   if (int rc = upload_buffers(k, stream)) return rc;
   void* args[] = {params};
   ProfScope prof(k->entry.c_str(), stream);
-  FA_CUDA_CHECK(cudaLaunchKernel((const void*)k->fn, grid, block, args, (size_t)k->smem, (cudaStream_t)stream));
+  cudaLaunchAttribute attr;
+  const cudaLaunchConfig_t cfg = launch_config(grid, block, k->smem, stream, &attr);
+  FA_CUDA_CHECK(cudaLaunchKernelExC(&cfg, (const void*)k->fn, args));
+  return FA_OK;
+}
+// the same for the kernels of this file
+template <class... P, class... A>
+int launch_here(const char* name, void (*fn)(P...), dim3 grid, dim3 block, void* stream, A... args) {
+  ProfScope prof(name, stream);
+  cudaLaunchAttribute attr;
+  const cudaLaunchConfig_t cfg = launch_config(grid, block, 0, stream, &attr);
+  FA_CUDA_CHECK(cudaLaunchKernelEx(&cfg, fn, P(args)...));
   return FA_OK;
 }
 
 // ---- configuration ---------------------------------------------------------------------
 int esize(int dtype) { return dtype == FA_F32 ? 4 : 2; }
 int pitch(int cols, int es) { return cols * es + 16; }
-constexpr int kMaxSmem = 227 * 1024;
+constexpr int kMaxSmem = 227 * 1024 - 128;  // (the table of captured buffers is static shared memory)
 
 struct FwdCfg {
   int BM, BN, warps, smem;
@@ -490,6 +531,11 @@ int check_common(fa_module* m, const fa_attn_params* p) {
     if (!(t.mask_bits_B == 1 || t.mask_bits_B == p->B) || !(t.mask_bits_H == 1 || t.mask_bits_H == p->Hq))
       return fail(FA_EINVAL, "mask_bits batch/head dims must be 1 or match B/Hq");
   }
+  if (t.mask_bits_t) {
+    if (!t.mask_bits) return fail(FA_EINVAL, "mask_bits_t comes with mask_bits");
+    if (((uintptr_t)t.mask_bits_t & 15) || t.mask_bits_t_stride % 4 || t.mask_bits_t_stride * 32 < p->Sq || t.mask_bits_t_rows < p->Skv)
+      return fail(FA_EINVAL, "mask_bits_t: 16-byte aligned, rows of a multiple of 4 words that cover Sq, at least Skv rows");
+  }
   return FA_OK;
 }
 
@@ -503,11 +549,19 @@ FaTables cvt_tables(const fa_block_tables& t) {
   r.QB = t.q_block_size; r.KVB = t.kv_block_size;
   r.mask_bits = t.mask_bits; r.mask_stride = t.mask_bits_stride; r.mask_rows = t.mask_bits_rows;
   r.mask_B = t.mask_bits_B; r.mask_H = t.mask_bits_H;
+  r.mask_bits_t = t.mask_bits_t; r.mask_t_stride = t.mask_bits_t_stride; r.mask_t_rows = t.mask_bits_t_rows;
   return r;
 }
 
-void fill_params(const fa_attn_params* p, FaParams& k) {
+// the captured buffers of a module as they are now (fa_module_set_buffers)
+void fill_buffers(fa_module* m, const void* (&out)[FA_MAX_MOD_BUFS]) {
+  std::lock_guard<std::mutex> lk(g_mu);
+  for (int i = 0; i < FA_MAX_MOD_BUFS; ++i) out[i] = i < m->nbufs ? m->bufs[i] : nullptr;
+}
+
+void fill_params(fa_module* m, const fa_attn_params* p, FaParams& k) {
   memset(&k, 0, sizeof k);
+  fill_buffers(m, k.mod_buf);
   k.q = cvt(p->q); k.k = cvt(p->k); k.v = cvt(p->v); k.o = cvt(p->o);
   k.lse = p->lse; k.status = p->status;
   k.B = p->B; k.Hq = p->Hq; k.Hkv = p->Hkv; k.Sq = p->Sq; k.Skv = p->Skv; k.D = p->D; k.Dv = p->Dv;
@@ -517,43 +571,60 @@ void fill_params(const fa_attn_params* p, FaParams& k) {
 
 // ---- kernels that do not depend on the mods --------------------------------------------
 
-// One warp per table row.  The reference orders a row by a stable descending argsort of the
-// 0/1 block grid (flaxattention/core/blockmask.py:57-64): set columns ascending, then the
-// unset columns ascending.  `transposed` builds the q-tables from the same class grid.
-__global__ void fa_tables_kernel(const signed char* __restrict__ cls, int rows_per_bh, int cols, int want,
-                                 bool transposed, int nQ, int nKV, long long n_rows,
-                                 int* __restrict__ num_out, int* __restrict__ idx_out) {
+// The eight tables of a BlockMask from the class grid, in one launch: one warp per row of the kv tables
+// and per row of the q tables (the same grid read along the other axis), each writing its partial and
+// its full list.  The reference orders a row by a stable descending argsort of the 0/1 block grid
+// (flaxattention/core/blockmask.py:57-64): set columns ascending, then the unset columns ascending.
+// The class grid may have fewer (batch, head) entries than the tables (masks that do not read the batch
+// or the head index are evaluated once).
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+struct FaTableOut {
+  int *num[4], *idx[4];  // partial and full lists of the kv tables, then of the q tables (null: not wanted)
+};
+__global__ void __launch_bounds__(128) fa_tables_kernel(const signed char* __restrict__ cls, int B, int H, int clsB, int clsH, int nQ,
+                                                        int nKV, FaTableOut out) {
+  grid_wait();
   const long long row = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (row >= n_rows) return;
   const int lane = threadIdx.x & 31;
-  const long long bh = row / rows_per_bh;
-  const int r = (int)(row - bh * rows_per_bh);
-  const signed char* g = cls + bh * (long long)nQ * nKV;
-  auto is_set = [&](int c) -> bool {
-    const signed char v = transposed ? g[(long long)c * nKV + r] : g[(long long)r * nKV + c];
-    return v == want;
-  };
-  int total = 0;
+  const long long n_kv_rows = (long long)B * H * nQ, n_rows = n_kv_rows + (long long)B * H * nKV;
+  if (row >= n_rows) return;
+  const bool transposed = row >= n_kv_rows;
+  const int rows_per_bh = transposed ? nKV : nQ, cols = transposed ? nQ : nKV;
+  const long long trow = transposed ? row - n_kv_rows : row;  // row of the table
+  const long long bh = trow / rows_per_bh;
+  const int r = (int)(trow - bh * rows_per_bh);
+  const int b = (int)(bh / H), h = (int)(bh - (long long)b * H);
+  const long long cbh = (long long)(clsB == 1 ? 0 : b) * clsH + (clsH == 1 ? 0 : h);
+  const signed char* g = cls + cbh * (long long)nQ * nKV + (transposed ? (long long)r : (long long)r * nKV);
+  const int step = transposed ? nKV : 1;
+  int total[2] = {0, 0};
   for (int c0 = 0; c0 < cols; c0 += 32) {
     const int c = c0 + lane;
-    const bool s = c < cols && is_set(c);
-    total += __popc(__ballot_sync(0xffffffffu, s));
+    const int v = c < cols ? (int)g[(long long)c * step] : 0;
+    total[0] += __popc(__ballot_sync(0xffffffffu, v == 1));
+    total[1] += __popc(__ballot_sync(0xffffffffu, v == 2));
   }
-  int n_set = 0, n_unset = 0;
-  int* out = idx_out + row * cols;
-  for (int c0 = 0; c0 < cols; c0 += 32) {
-    const int c = c0 + lane;
-    const bool in = c < cols;
-    const bool s = in && is_set(c);
-    const unsigned bs = __ballot_sync(0xffffffffu, s);
-    const unsigned bu = __ballot_sync(0xffffffffu, in && !s);
-    const unsigned lt = (1u << lane) - 1u;
-    if (s) out[n_set + __popc(bs & lt)] = c;
-    else if (in) out[total + n_unset + __popc(bu & lt)] = c;
-    n_set += __popc(bs);
-    n_unset += __popc(bu);
+  const unsigned lt = (1u << lane) - 1u;
+#pragma unroll
+  for (int which = 0; which < 2; ++which) {
+    int* num = transposed ? out.num[2 + which] : out.num[which];
+    int* idx = transposed ? out.idx[2 + which] : out.idx[which];
+    if (num == nullptr) continue;
+    idx += trow * cols;
+    int n_set = 0;
+    for (int c0 = 0; c0 < cols; c0 += 32) {
+      const int c = c0 + lane;
+      const bool in = c < cols;
+      const bool s = in && (int)g[(long long)c * step] == which + 1;
+      const unsigned bs = __ballot_sync(0xffffffffu, s);
+      const int before = n_set + __popc(bs & lt);  // set columns in front of this one
+      if (in) idx[s ? before : total[which] + c - before] = c;
+      n_set += __popc(bs);
+    }
+    if (lane == 0) num[trow] = total[which];
   }
-  if (lane == 0) num_out[row] = total;
 }
 
 
@@ -562,6 +633,8 @@ __global__ void fa_tables_kernel(const signed char* __restrict__ cls, int rows_p
 template <int DT, int LPR>
 __global__ void fa_delta_kernel(FaTensor o, FaTensor dout, float* __restrict__ delta, int Hq, int Sq, int Dv,
                                 long long n_rows) {
+  grid_wait();
+  grid_release();
   constexpr int ES = DT == FA_F32 ? 4 : 2;
   constexpr int EPC = 16 / ES;  // elements per 16-byte chunk
   const long long gt = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -611,6 +684,8 @@ __global__ void fa_bwd_prep_kernel(FaTensor o, FaTensor dout, const float* __res
   // grid: x over groups of R * (256 / LPR) padded rows of one (batch, head), LPR lanes per row; (y, z) over the heads.
   // A thread works on R rows, 256 / LPR apart, and has the loads of all of them in flight before it uses the first
   // (Dv <= 128: at most two 16-byte pieces of O and of dO per lane and row).
+  grid_wait();
+  grid_release();
   constexpr int R = 4, ROWS = 256 / LPR;
   const int bh = blockIdx.y + blockIdx.z * gridDim.y;
   const int rloc = threadIdx.x / LPR, sub = threadIdx.x % LPR;
@@ -678,6 +753,7 @@ template <int DT>
 __global__ void fa_dq_convert_kernel(const float* __restrict__ acc, FaTensor dq, int Hq, int Sq, int sq_pad, float scale,
                                      int n_bh) {
   // grid: x over the rows of one (batch, head), one 8-element output chunk per thread; (y, z) over the heads
+  grid_wait();
   const int bh = blockIdx.y + blockIdx.z * gridDim.y;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int k8 = i & 7, q = i >> 3;
@@ -707,6 +783,7 @@ __global__ void fa_dq_convert_kernel(const float* __restrict__ acc, FaTensor dq,
 template <int DT>
 __global__ void fa_dq_convert_t_kernel(const float* __restrict__ acc, FaTensor dq, int Hq, int Sq, int sq_pad, float scale,
                                        int n_bh) {
+  grid_wait();
   const int bh = blockIdx.y + blockIdx.z * gridDim.y;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int dg = (i >> 5) & 15, q = ((i >> 9) << 5) | (i & 31);
@@ -740,6 +817,7 @@ template <int DT>
 __global__ void fa_decode_combine_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
                                          FaTensor o, float* __restrict__ lse, int Hq, int Sq, int Dv, int ns,
                                          long long n_rows) {
+  grid_wait();
   const long long row = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= n_rows) return;
   const int lane = threadIdx.x & 31;
@@ -844,8 +922,9 @@ int fa_selftest_bounded_wait(unsigned long long limit_ns, int* status, int* gave
     }
   }
   Kernel* k = nullptr;
-  const std::string defs = "#define FA_WAIT_LIMIT_NS " + std::to_string(limit_ns) + "ull\n";
-  if (int rc = get_kernel(mod, "fa_selftest.cuh", defs, "fa_wait_selftest_kernel", 0, &k)) return rc;
+  const auto defs = [&] { return "#define FA_WAIT_LIMIT_NS " + std::to_string(limit_ns) + "ull\n"; };
+  if (int rc = get_kernel(mod, kernel_key(kIdSelftest, {{(int)limit_ns, 32}}), "fa_selftest.cuh", defs, "fa_wait_selftest_kernel", 0, &k))
+    return rc;
   struct { int* status; int* gave_up; unsigned long long* waited_ns; } prm = {status, gave_up, waited_ns};
   return launch(k, dim3(1), dim3(64), &prm, stream);
 }
@@ -886,22 +965,26 @@ namespace {
 int round_flag(int dtype, int flags) { return (dtype != FA_F32 && (flags & FA_FLAG_ROUND_SCORES)) ? 1 : 0; }
 
 int get_fwd_kernel(fa_module* m, int dtype, int D, int Dv, int flags, const FwdCfg& c, Kernel** k) {
-  return get_kernel(m, "fa_fwd.cuh",
-                    defs({{"FA_DTYPE", dtype}, {"FA_D", D}, {"FA_DV", Dv}, {"FA_BM", c.BM}, {"FA_BN", c.BN},
-                          {"FA_WARPS", c.warps}, {"FA_ROUND_SCORES", round_flag(dtype, flags)}}),
+  const int rnd = round_flag(dtype, flags);
+  return get_kernel(m, kernel_key(kIdFwd, {{dtype, 2}, {D, 9}, {Dv, 9}, {c.BM, 9}, {c.BN, 9}, {c.warps, 5}, {rnd, 1}}), "fa_fwd.cuh",
+                    [&] { return defs({{"FA_DTYPE", dtype}, {"FA_D", D}, {"FA_DV", Dv}, {"FA_BM", c.BM}, {"FA_BN", c.BN},
+                                       {"FA_WARPS", c.warps}, {"FA_ROUND_SCORES", rnd}}); },
                     "fa_fwd_kernel", c.smem, k);
 }
 int get_bwd_kernel(fa_module* m, int dtype, int D, int Dv, int flags, const BwdCfg& c, bool dq, Kernel** k) {
-  return get_kernel(m, "fa_bwd.cuh",
-                    defs({{"FA_DTYPE", dtype}, {"FA_D", D}, {"FA_DV", Dv}, {"FA_BQ", c.tile}, {"FA_BK", c.tile},
-                          {"FA_WARPS", c.warps}, {"FA_ROUND_SCORES", round_flag(dtype, flags)}}),
+  const int rnd = round_flag(dtype, flags);
+  return get_kernel(m, kernel_key(dq ? kIdBwdDq : kIdBwdDkdv, {{dtype, 2}, {D, 9}, {Dv, 9}, {c.tile, 9}, {c.warps, 5}, {rnd, 1}}),
+                    "fa_bwd.cuh",
+                    [&] { return defs({{"FA_DTYPE", dtype}, {"FA_D", D}, {"FA_DV", Dv}, {"FA_BQ", c.tile}, {"FA_BK", c.tile},
+                                       {"FA_WARPS", c.warps}, {"FA_ROUND_SCORES", rnd}}); },
                     dq ? "fa_bwd_dq_kernel" : "fa_bwd_dkdv_kernel", dq ? c.smem_dq : c.smem_dkdv, k);
 }
 int get_decode_kernel(fa_module* m, int dtype, int D, int Dv, int flags, const DecCfg& c, bool pack, Kernel** k) {
-  return get_kernel(m, "fa_decode.cuh",
-                    defs({{"FA_DTYPE", dtype}, {"FA_D", D}, {"FA_DV", Dv}, {"FA_BM", c.BM}, {"FA_BN", c.BN},
-                          {"FA_STAGES", c.stages}, {"FA_ROUND_SCORES", round_flag(dtype, flags)},
-                          {"FA_PACK_HEADS", pack ? 1 : 0}}),
+  const int rnd = round_flag(dtype, flags);
+  return get_kernel(m, kernel_key(kIdDecode, {{dtype, 2}, {D, 9}, {Dv, 9}, {c.BM, 9}, {c.BN, 9}, {c.stages, 4}, {rnd, 1}, {pack ? 1 : 0, 1}}),
+                    "fa_decode.cuh",
+                    [&] { return defs({{"FA_DTYPE", dtype}, {"FA_D", D}, {"FA_DV", Dv}, {"FA_BM", c.BM}, {"FA_BN", c.BN},
+                                       {"FA_STAGES", c.stages}, {"FA_ROUND_SCORES", rnd}, {"FA_PACK_HEADS", pack ? 1 : 0}}); },
                     "fa_decode_kernel", c.smem, k);
 }
 // Grouped-query decode: the G query heads of a kv head share one CTA (their G * Sq rows form one
@@ -978,8 +1061,10 @@ int get_fwd_tc_kernel(fa_module* m, int dtype, int D, int flags, Kernel** k, boo
   const int atoms = D / 64, nstage = decode ? 5 : (D == 64 ? 3 : 2);
   const int smem = 2 * atoms * 16384 + 2 * nstage * atoms * 16384 + (1 + 4 * nstage + 8) * 8 + 16 + 256 * 2 + 256 * 2 +
                    2 * 256 + (256 / 32) * 4 + 1024;
-  std::string d = defs({{"FA_DTYPE", dtype}, {"FA_D", D}, {"FA_ROUND_SCORES", round_flag(dtype, flags)}, {"FA_TC_DECODE", decode ? 1 : 0}});
-  return get_kernel(m, "fa_fwd_tc.cuh", d, "fa_fwd_tc_kernel", smem, k);
+  const int rnd = round_flag(dtype, flags);
+  return get_kernel(m, kernel_key(kIdFwdTc, {{dtype, 2}, {D, 9}, {rnd, 1}, {decode ? 1 : 0, 1}}), "fa_fwd_tc.cuh",
+                    [&] { return defs({{"FA_DTYPE", dtype}, {"FA_D", D}, {"FA_ROUND_SCORES", rnd}, {"FA_TC_DECODE", decode ? 1 : 0}}); },
+                    "fa_fwd_tc_kernel", smem, k);
 }
 
 // Shapes the split-KV variant of the tcgen05 kernel covers (`num_splits` CTAs per (batch, head), one
@@ -1089,9 +1174,10 @@ int get_bwd_tc_kernel(fa_module* m, int dtype, int D, int flags, bool kv2, Kerne
   const int kv_bytes = (D / 64) * 16384, q_bytes = 16384, ds_bytes = (bq / 64) * 16384;
   const int smem = 2 * kvbuf * kv_bytes + 2 * nstage * q_bytes + ds_bytes + 128 * 32 * 4 + nstage * 2 * bq * 4 +
                    (2 + 3 * nstage + 15) * 8 + 16 + 16 + 2 * bwd_tc_max_pairs(D) * 4 + 256 + 1024;
-  std::string d = defs({{"FA_DTYPE", dtype}, {"FA_D", D}, {"FA_ROUND_SCORES", round_flag(dtype, flags)},
-                        {"FA_BWD_KV2", kvbuf == 2 ? 1 : 0}});
-  return get_kernel(m, "fa_bwd_tc.cuh", d, "fa_bwd_tc_kernel", smem, k);
+  const int rnd = round_flag(dtype, flags);
+  return get_kernel(m, kernel_key(kIdBwdTc, {{dtype, 2}, {D, 9}, {rnd, 1}, {kvbuf, 2}}), "fa_bwd_tc.cuh",
+                    [&] { return defs({{"FA_DTYPE", dtype}, {"FA_D", D}, {"FA_ROUND_SCORES", rnd}, {"FA_BWD_KV2", kvbuf == 2 ? 1 : 0}}); },
+                    "fa_bwd_tc_kernel", smem, k);
 }
 
 // With a BlockMask the items are short or uneven and the variant with two K / V buffers wins: under a
@@ -1103,12 +1189,10 @@ bool bwd_tc_kv2(const fa_attn_params* p) {
   return (long long)((p->Sq + 127) / 128) * (p->Hq / p->Hkv) <= 64;
 }
 
-int get_mask_bits_kernel(fa_module* m, Kernel** k) {
-  return get_kernel(m, "fa_blockmask.cuh", "", "fa_mask_bits_kernel", 0, k);
-}
-
-int get_blockmask_kernel(fa_module* m, Kernel** k) {
-  return get_kernel(m, "fa_blockmask.cuh", "", "fa_blockmask_classify_kernel", 0, k);
+// scan = false: the kernel that takes any block size
+int get_blockmask_kernel(fa_module* m, bool scan, Kernel** k) {
+  return get_kernel(m, kernel_key(scan ? kIdMaskScan : kIdMaskClassify, {}), "fa_blockmask.cuh", [] { return std::string(); },
+                    scan ? "fa_mask_scan_kernel" : "fa_blockmask_classify_kernel", 0, k);
 }
 
 }  // namespace
@@ -1145,8 +1229,7 @@ int fa_module_prepare(fa_module* m, int kind, int dtype, int D, int Dv, int Sq_h
       return get_decode_kernel(m, dtype, D, Dv, 0, c, false, &k);
     }
     case FA_KIND_BLOCKMASK:
-      if (int rc = get_mask_bits_kernel(m, &k)) return rc;
-      return get_blockmask_kernel(m, &k);
+      return get_blockmask_kernel(m, true, &k);
     default:
       return fail(FA_EUNSUPPORTED, "fa_module_prepare: unknown kind");
   }
@@ -1156,7 +1239,7 @@ int fa_fwd(fa_module* m, const fa_attn_params* p, void* stream) {
   if (int rc = check_common(m, p)) return rc;
   prof_reset();
   FaParams kp;
-  fill_params(p, kp);
+  fill_params(m, p, kp);
   if (tc_fwd_eligible(p)) return launch_fwd_tc(m, p, kp, stream);
   FwdCfg c;
   if (int rc = pick_fwd(p->dtype, p->D, p->Dv, p->Sq, &kp.t, c)) return rc;
@@ -1190,7 +1273,7 @@ int fa_bwd(fa_module* m, const fa_attn_params* p, const fa_tensor* dout, const f
   if (!workspace || workspace_bytes < need) return fail(FA_EWORKSPACE, "backward workspace too small");
   prof_reset();
   FaParams kp;
-  fill_params(p, kp);
+  fill_params(m, p, kp);
   kp.dout = cvt(*dout); kp.dq = cvt(*dq); kp.dk = cvt(*dk); kp.dv = cvt(*dv);
   kp.delta = (float*)workspace;
   const bool use_tc = tc_bwd_eligible(p);
@@ -1205,7 +1288,6 @@ int fa_bwd(fa_module* m, const fa_attn_params* p, const fa_tensor* dout, const f
   }
   if (use_tc) {
     // workspace: nlse2 | ndelta (padded rows) | dq accumulator
-    cudaStream_t st = (cudaStream_t)stream;
     float* nlse2 = (float*)workspace;
     float* ndelta = (float*)((char*)workspace + rows_pad_bytes(p));
     float* dq_acc = (float*)((char*)workspace + 2 * rows_pad_bytes(p));
@@ -1217,12 +1299,10 @@ int fa_bwd(fa_module* m, const fa_attn_params* p, const fa_tensor* dout, const f
       // row scalars; the same pass clears the dQ accumulator
       // 8 lanes per row, 4 rows per thread: 128 rows per block (sq_pad is a multiple of 128)
       const dim3 grid((unsigned)(sq_pad / 128), (unsigned)gy, (unsigned)((n_bh + gy - 1) / gy));
-      ProfScope prof("fa_bwd_prep_kernel", stream);
-      if (p->dtype == FA_F16)
-        fa_bwd_prep_kernel<FA_F16, 8><<<grid, 256, 0, st>>>(kp.o, kp.dout, p->lse, nlse2, ndelta, dq_acc, work_counter, p->Hq, p->Sq, sq_pad, p->Dv, p->D, n_bh);
-      else
-        fa_bwd_prep_kernel<FA_BF16, 8><<<grid, 256, 0, st>>>(kp.o, kp.dout, p->lse, nlse2, ndelta, dq_acc, work_counter, p->Hq, p->Sq, sq_pad, p->Dv, p->D, n_bh);
-      FA_CUDA_CHECK(cudaGetLastError());
+      if (int rc = launch_here("fa_bwd_prep_kernel", p->dtype == FA_F16 ? fa_bwd_prep_kernel<FA_F16, 8> : fa_bwd_prep_kernel<FA_BF16, 8>,
+                               grid, dim3(256), stream, kp.o, kp.dout, p->lse, nlse2, ndelta, dq_acc, work_counter, p->Hq, p->Sq,
+                               sq_pad, p->Dv, p->D, n_bh))
+        return rc;
     }
     FaBwdTcParamsHost tp;
     tp.p = kp;
@@ -1243,31 +1323,21 @@ int fa_bwd(fa_module* m, const fa_attn_params* p, const fa_tensor* dout, const f
     {
       // one 16-byte output chunk per thread: D / 8 chunks per row
       const dim3 grid((unsigned)(((long long)sq_pad * (p->D / 8) + 255) / 256), (unsigned)gy, (unsigned)((n_bh + gy - 1) / gy));
-      ProfScope prof("fa_dq_convert_kernel", stream);
-      if (p->D == 64) {
-        if (p->dtype == FA_F16)
-          fa_dq_convert_kernel<FA_F16><<<grid, 256, 0, st>>>(dq_acc, kp.dq, p->Hq, p->Sq, sq_pad, p->scale, n_bh);
-        else
-          fa_dq_convert_kernel<FA_BF16><<<grid, 256, 0, st>>>(dq_acc, kp.dq, p->Hq, p->Sq, sq_pad, p->scale, n_bh);
-      } else {
-        if (p->dtype == FA_F16)
-          fa_dq_convert_t_kernel<FA_F16><<<grid, 256, 0, st>>>(dq_acc, kp.dq, p->Hq, p->Sq, sq_pad, p->scale, n_bh);
-        else
-          fa_dq_convert_t_kernel<FA_BF16><<<grid, 256, 0, st>>>(dq_acc, kp.dq, p->Hq, p->Sq, sq_pad, p->scale, n_bh);
-      }
-      FA_CUDA_CHECK(cudaGetLastError());
+      const auto convert = p->D == 64 ? (p->dtype == FA_F16 ? fa_dq_convert_kernel<FA_F16> : fa_dq_convert_kernel<FA_BF16>)
+                                      : (p->dtype == FA_F16 ? fa_dq_convert_t_kernel<FA_F16> : fa_dq_convert_t_kernel<FA_BF16>);
+      if (int rc = launch_here("fa_dq_convert_kernel", convert, grid, dim3(256), stream, dq_acc, kp.dq, p->Hq, p->Sq, sq_pad, p->scale, n_bh))
+        return rc;
     }
     return FA_OK;
   }
   {
-    cudaStream_t st = (cudaStream_t)stream;
     const long long n_rows = (long long)p->B * p->Hq * p->Sq;
     const int chunks = p->Dv * es / 16;
     const int lpr = chunks >= 8 ? 8 : (chunks >= 4 ? 4 : (chunks >= 2 ? 2 : 1));
     const long long threads = n_rows * lpr;
     const unsigned blocks = (unsigned)((threads + 255) / 256);
-    ProfScope prof("fa_delta_kernel", stream);
-#define FA_DELTA(DT, L) fa_delta_kernel<DT, L><<<blocks, 256, 0, st>>>(kp.o, kp.dout, kp.delta, p->Hq, p->Sq, p->Dv, n_rows)
+    void (*delta)(FaTensor, FaTensor, float*, int, int, int, long long) = nullptr;
+#define FA_DELTA(DT, L) delta = fa_delta_kernel<DT, L>
 #define FA_DELTA_DT(L)                                      \
   do {                                                      \
     if (p->dtype == FA_F16) FA_DELTA(FA_F16, L);            \
@@ -1280,7 +1350,8 @@ int fa_bwd(fa_module* m, const fa_attn_params* p, const fa_tensor* dout, const f
     else FA_DELTA_DT(1);
 #undef FA_DELTA_DT
 #undef FA_DELTA
-    FA_CUDA_CHECK(cudaGetLastError());
+    if (int rc = launch_here("fa_delta_kernel", delta, dim3(blocks), dim3(256), stream, kp.o, kp.dout, kp.delta, p->Hq, p->Sq, p->Dv, n_rows))
+      return rc;
   }
   if (int rc = launch(kdkdv, dim3((p->Skv + c.tile - 1) / c.tile, p->Hkv, p->B), dim3(c.warps * 32), &kp, stream))
     return rc;
@@ -1345,7 +1416,7 @@ int fa_decode(fa_module* m, const fa_attn_params* p, int num_splits, void* works
   if (num_splits > 65535) return fail(FA_EINVAL, "too many splits");
   prof_reset();
   FaParams kp;
-  fill_params(p, kp);
+  fill_params(m, p, kp);
   const bool pack = decode_packs_heads(p);
   const bool tc = !pack && tc_decode_eligible(p) && num_splits >= 2;
   DecCfg c;
@@ -1371,13 +1442,9 @@ int fa_decode(fa_module* m, const fa_attn_params* p, int num_splits, void* works
   if (num_splits > 1) {
     const long long n_rows = (long long)p->B * p->Hq * p->Sq;
     const unsigned blocks = (unsigned)((n_rows + 3) / 4);
-    cudaStream_t st = (cudaStream_t)stream;
-    ProfScope prof("fa_decode_combine_kernel", stream);
-    if (p->dtype == FA_F16)
-      fa_decode_combine_kernel<FA_F16><<<blocks, 128, 0, st>>>(kp.part_o, kp.part_ml, kp.o, kp.lse, p->Hq, p->Sq, p->Dv, num_splits, n_rows);
-    else
-      fa_decode_combine_kernel<FA_BF16><<<blocks, 128, 0, st>>>(kp.part_o, kp.part_ml, kp.o, kp.lse, p->Hq, p->Sq, p->Dv, num_splits, n_rows);
-    FA_CUDA_CHECK(cudaGetLastError());
+    if (int rc = launch_here("fa_decode_combine_kernel", p->dtype == FA_F16 ? fa_decode_combine_kernel<FA_F16> : fa_decode_combine_kernel<FA_BF16>,
+                             dim3(blocks), dim3(128), stream, kp.part_o, kp.part_ml, kp.o, kp.lse, p->Hq, p->Sq, p->Dv, num_splits, n_rows))
+      return rc;
   }
   return FA_OK;
 }
@@ -1392,62 +1459,80 @@ int64_t fa_mask_bits_row_words(int KV_LEN) { return KV_LEN <= 0 ? 0 : (int64_t)(
 
 int fa_mask_bits(fa_module* m, int B, int H, int Q_LEN, int KV_LEN, int b_offset, int h_offset, uint32_t* bits,
                  void* stream) {
-  if (!m) return fail(FA_EINVAL, "module is null");
   if (B <= 0 || H <= 0 || Q_LEN <= 0 || KV_LEN <= 0) return fail(FA_EINVAL, "B, H, Q_LEN and KV_LEN must be positive");
-  if (!bits || ((uintptr_t)bits & 15)) return fail(FA_EINVAL, "bits must be a 16-byte aligned device pointer");
-  if ((long long)B * H > 65535 || Q_LEN > 65535) return fail(FA_EUNSUPPORTED, "B*H and Q_LEN must not exceed 65535");
-  Kernel* k = nullptr;
-  if (int rc = get_mask_bits_kernel(m, &k)) return rc;
-  FaMaskBitsParams mp;
-  mp.bits = bits;
-  mp.stride = fa_mask_bits_row_words(KV_LEN);
-  mp.B = B; mp.H = H; mp.Q_LEN = Q_LEN; mp.KV_LEN = KV_LEN;
-  mp.b_off = b_offset; mp.h_off = h_offset;
-  return launch(k, dim3((unsigned)((mp.stride + 255) / 256), (unsigned)Q_LEN, (unsigned)(B * H)), dim3(256), &mp, stream);
+  if (!bits) return fail(FA_EINVAL, "bits is null");
+  fa_mask_build mb{};
+  mb.B = mb.distinct_B = B; mb.H = mb.distinct_H = H;
+  mb.Q_LEN = Q_LEN; mb.KV_LEN = KV_LEN; mb.q_block = 128; mb.kv_block = 128;
+  mb.b_offset = b_offset; mb.h_offset = h_offset;
+  mb.bits = bits;
+  return fa_block_mask_build(m, &mb, stream);
 }
 
 int fa_block_mask(fa_module* m, int B, int H, int Q_LEN, int KV_LEN, int q_block, int kv_block, int b_offset,
                   int h_offset, int32_t* kv_num_blocks, int32_t* kv_indices, int32_t* full_kv_num_blocks,
                   int32_t* full_kv_indices, int32_t* q_num_blocks, int32_t* q_indices, int32_t* full_q_num_blocks,
                   int32_t* full_q_indices, void* workspace, size_t workspace_bytes, void* stream) {
-  if (!m) return fail(FA_EINVAL, "module is null");
-  const size_t need = fa_block_mask_workspace_bytes(B, H, Q_LEN, KV_LEN, q_block, kv_block);
-  if (need == 0) return fail(FA_EINVAL, "B, H, Q_LEN, KV_LEN and block sizes must be positive");
   if (!kv_num_blocks || !kv_indices) return fail(FA_EINVAL, "kv_num_blocks / kv_indices are null");
-  if ((full_kv_num_blocks == nullptr) != (full_kv_indices == nullptr))
-    return fail(FA_EINVAL, "full_kv_num_blocks and full_kv_indices must be both given or both null");
-  if ((q_num_blocks == nullptr) != (q_indices == nullptr) || (full_q_num_blocks == nullptr) != (full_q_indices == nullptr))
-    return fail(FA_EINVAL, "q tables must be given as (num, indices) pairs");
-  if (full_q_num_blocks && !full_kv_num_blocks) return fail(FA_EINVAL, "full q tables need full kv tables");
-  if (!workspace || workspace_bytes < need) return fail(FA_EWORKSPACE, "block-mask workspace too small");
-  const int nQ = (Q_LEN + q_block - 1) / q_block, nKV = (KV_LEN + kv_block - 1) / kv_block;
-  if ((long long)B * H > 65535 || nQ > 65535) return fail(FA_EUNSUPPORTED, "B*H and the q-block count must not exceed 65535");
-  Kernel* k = nullptr;
-  if (int rc = get_blockmask_kernel(m, &k)) return rc;
-  FaMaskParams mp;
-  mp.cls = (signed char*)workspace;
-  mp.B = B; mp.H = H; mp.nQ = nQ; mp.nKV = nKV; mp.QB = q_block; mp.KVB = kv_block;
-  mp.b_off = b_offset; mp.h_off = h_offset;
-  if (int rc = launch(k, dim3(nKV, nQ, B * H), dim3(256), &mp, stream)) return rc;
+  fa_mask_build mb{};
+  mb.B = mb.distinct_B = B; mb.H = mb.distinct_H = H;
+  mb.Q_LEN = Q_LEN; mb.KV_LEN = KV_LEN; mb.q_block = q_block; mb.kv_block = kv_block;
+  mb.b_offset = b_offset; mb.h_offset = h_offset;
+  mb.kv_num_blocks = kv_num_blocks; mb.kv_indices = kv_indices;
+  mb.full_kv_num_blocks = full_kv_num_blocks; mb.full_kv_indices = full_kv_indices;
+  mb.q_num_blocks = q_num_blocks; mb.q_indices = q_indices;
+  mb.full_q_num_blocks = full_q_num_blocks; mb.full_q_indices = full_q_indices;
+  mb.workspace = workspace; mb.workspace_bytes = workspace_bytes;
+  return fa_block_mask_build(m, &mb, stream);
+}
 
-  cudaStream_t st = (cudaStream_t)stream;
-  const int wpb = 4;
-  auto run = [&](int want, bool transposed, int32_t* num, int32_t* idx) -> int {
-    if (!num) return FA_OK;
-    const int rows = transposed ? nKV : nQ, cols = transposed ? nQ : nKV;
-    const long long n_rows = (long long)B * H * rows;
-    const unsigned blocks = (unsigned)((n_rows + wpb - 1) / wpb);
-    fa_tables_kernel<<<blocks, wpb * 32, 0, st>>>(mp.cls, rows, cols, want, transposed, nQ, nKV, n_rows, num, idx);
-    FA_CUDA_CHECK(cudaGetLastError());
-    return FA_OK;
-  };
-  // Without separate full tables every non-empty block is listed as partial.
-  if (!full_kv_num_blocks) return fail(FA_EUNSUPPORTED, "tables without separate full blocks are not implemented");
-  if (int rc = run(1, false, kv_num_blocks, kv_indices)) return rc;
-  if (int rc = run(2, false, full_kv_num_blocks, full_kv_indices)) return rc;
-  if (int rc = run(1, true, q_num_blocks, q_indices)) return rc;
-  if (int rc = run(2, true, full_q_num_blocks, full_q_indices)) return rc;
-  return FA_OK;
+int fa_block_mask_build(fa_module* m, const fa_mask_build* mb, void* stream) {
+  if (!m) return fail(FA_EINVAL, "module is null");
+  if (!mb) return fail(FA_EINVAL, "the description is null");
+  const int QB = mb->q_block, KVB = mb->kv_block;
+  if (mb->B <= 0 || mb->H <= 0 || mb->Q_LEN <= 0 || mb->KV_LEN <= 0 || QB <= 0 || KVB <= 0)
+    return fail(FA_EINVAL, "B, H, Q_LEN, KV_LEN and block sizes must be positive");
+  if (!(mb->distinct_B == 1 || mb->distinct_B == mb->B) || !(mb->distinct_H == 1 || mb->distinct_H == mb->H))
+    return fail(FA_EINVAL, "the distinct entries along batch / heads must be 1 or B / H");
+  const bool tables = mb->kv_num_blocks != nullptr;
+  const size_t need = fa_block_mask_workspace_bytes(mb->distinct_B, mb->distinct_H, mb->Q_LEN, mb->KV_LEN, QB, KVB);
+  if (tables) {
+    if (!mb->kv_indices) return fail(FA_EINVAL, "kv_num_blocks / kv_indices are null");
+    if ((mb->full_kv_num_blocks == nullptr) != (mb->full_kv_indices == nullptr))
+      return fail(FA_EINVAL, "full_kv_num_blocks and full_kv_indices must be both given or both null");
+    if ((mb->q_num_blocks == nullptr) != (mb->q_indices == nullptr) || (mb->full_q_num_blocks == nullptr) != (mb->full_q_indices == nullptr))
+      return fail(FA_EINVAL, "q tables must be given as (num, indices) pairs");
+    if (mb->full_q_num_blocks && !mb->full_kv_num_blocks) return fail(FA_EINVAL, "full q tables need full kv tables");
+    if (!mb->workspace || mb->workspace_bytes < need) return fail(FA_EWORKSPACE, "block-mask workspace too small");
+    // Without separate full tables every non-empty block is listed as partial.
+    if (!mb->full_kv_num_blocks) return fail(FA_EUNSUPPORTED, "tables without separate full blocks are not implemented");
+  }
+  if (((uintptr_t)mb->bits & 15) || ((uintptr_t)mb->bits_t & 15)) return fail(FA_EINVAL, "bits must be 16-byte aligned");
+  const int nQ = (mb->Q_LEN + QB - 1) / QB, nKV = (mb->KV_LEN + KVB - 1) / KVB;
+  const long long nbh = (long long)mb->distinct_B * mb->distinct_H;
+  if ((long long)mb->B * mb->H > 65535 || nQ > 65535)
+    return fail(FA_EUNSUPPORTED, "B*H and the q-block count must not exceed 65535");
+  const bool words = (nQ == 1 || QB % 32 == 0) && (nKV == 1 || KVB % 32 == 0) && (long long)QB * KVB < (1ll << 31);
+  if (!words && (mb->bits || mb->bits_t)) return fail(FA_EUNSUPPORTED, "bit matrices need blocks of whole 32-bit words");
+  Kernel* k = nullptr;
+  if (int rc = get_blockmask_kernel(m, words, &k)) return rc;
+  prof_reset();
+  FaMaskParams mp;
+  memset(&mp, 0, sizeof mp);
+  mp.cls = tables ? (signed char*)mb->workspace : nullptr;
+  mp.bits = mb->bits; mp.bits_t = mb->bits_t;
+  mp.stride = fa_mask_bits_row_words(mb->KV_LEN); mp.stride_t = fa_mask_bits_row_words(mb->Q_LEN);
+  mp.B = mb->distinct_B; mp.H = mb->distinct_H; mp.nQ = nQ; mp.nKV = nKV; mp.QB = QB; mp.KVB = KVB;
+  mp.Q_LEN = mb->Q_LEN; mp.KV_LEN = mb->KV_LEN;
+  mp.b_off = mb->b_offset; mp.h_off = mb->h_offset;
+  fill_buffers(m, mp.mod_buf);
+  if (int rc = launch(k, dim3(nKV, nQ, (unsigned)nbh), dim3(words ? 128 : 256), &mp, stream)) return rc;
+  if (!tables) return FA_OK;
+  FaTableOut out = {{mb->kv_num_blocks, mb->full_kv_num_blocks, mb->q_num_blocks, mb->full_q_num_blocks},
+                    {mb->kv_indices, mb->full_kv_indices, mb->q_indices, mb->full_q_indices}};
+  const long long n_rows = (long long)mb->B * mb->H * ((long long)nQ + (mb->q_num_blocks || mb->full_q_num_blocks ? nKV : 0));
+  return launch_here("fa_tables_kernel", fa_tables_kernel, dim3((unsigned)((n_rows + 3) / 4)), dim3(128), stream, mp.cls, mb->B,
+                     mb->H, mb->distinct_B, mb->distinct_H, nQ, nKV, out);
 }
 
 }  // extern "C"

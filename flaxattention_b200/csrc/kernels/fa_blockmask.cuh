@@ -1,14 +1,133 @@
-// Block classification for create_block_mask.  Replaces the dense-mask route of
-// flaxattention/core/blockmask.py:277-369 (create_mask -> reshape -> block sums): one CTA
-// evaluates mask_mod on the QB x KVB positions of one block and writes its class
-// (0 = no position kept, 1 = some, 2 = all) without materialising the [B,H,Q,KV] mask.
-// Positions beyond Q_LEN / KV_LEN are evaluated like any other, because the reference
-// classifies on the lengths rounded up to whole blocks (core/blockmask.py:440-444).
+// mask_mod over a block grid, for create_block_mask.  Replaces the dense-mask route of
+// flaxattention/core/blockmask.py:277-369 (create_mask -> reshape -> block sums): every position is
+// evaluated once, the class of each block (0 = no position kept, 1 = some, 2 = all) comes from the
+// counts, and the mask itself is kept as bit matrices (row-major and transposed) where the caller wants
+// them; a dense [B,H,Q,KV] mask does not exist.
+// Positions beyond Q_LEN / KV_LEN are classified like any other, because the reference classifies on
+// the lengths rounded up to whole blocks (core/blockmask.py:440-444); in the bit matrices they are 0.
 // The mod fragment (fa_mask_mod, FA_HAS_MASK_MOD) is placed before this file.
 #pragma once
 #include "fa_params.h"
 
+// One CTA of four warps per block, in 128 x 128 sub-tiles: a warp takes 32 rows, a lane one key out of each
+// group of 32.  Lane = key makes what a mask reads per key (a captured document id) a coalesced load
+// outside the row loop and what it reads per query a broadcast; a ballot per row gives 32 keys of the
+// row-major matrix and the lane's own bits over the rows are a word of the transposed one, so both
+// matrices and the block's count come out of one evaluation.  (A thread per position with a 64-bit
+// division for its row, and a second kernel that evaluated the mask again for the bits, took 35 + 4 us
+// on a 4096 x 4096 document mask.)  Needs key blocks of whole 32-bit words and query blocks of whole
+// words or a single one; other block sizes go to the classify kernel below.
+constexpr int FA_SCAN_WARPS = 4;
+extern "C" __global__ void __launch_bounds__(128) fa_mask_scan_kernel(const __grid_constant__ FaMaskParams p) {
+  FA_MOD_BUFS_INIT(p);
+  fa_grid_wait();
+  __shared__ unsigned t_words[128][FA_SCAN_WARPS];
+  __shared__ int s_cnt[FA_SCAN_WARPS];
+  __syncthreads();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int kvb = blockIdx.x, qb = blockIdx.y, bh = blockIdx.z;
+  const int b = bh / p.H, h = bh - b * p.H;
+  const int gb = b + p.b_off, gh = h + p.h_off;
+  const int q0 = qb * p.QB, k0 = kvb * p.KVB;
+  int cnt = 0;
+  for (int r0 = 0; r0 < p.QB; r0 += 128) {
+    for (int c0 = 0; c0 < p.KVB; c0 += 128) {
+      const int rbase = r0 + warp * 32;  // first row of this warp inside the block
+      unsigned roww[4] = {0u, 0u, 0u, 0u}, colw[4] = {0u, 0u, 0u, 0u};
+      const int nrows = min(32, p.QB - rbase);
+      if (c0 + 128 <= p.KVB && nrows == 32) {
+#pragma unroll 8
+        for (int r = 0; r < 32; ++r) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            const bool keep = fa_mask_mod(gb, gh, q0 + rbase + r, k0 + c0 + 32 * c + lane);
+            const unsigned vote = __ballot_sync(0xffffffffu, keep);
+            if (lane == r) roww[c] = vote;
+            colw[c] |= (keep ? 1u : 0u) << r;
+          }
+        }
+      } else {
+        for (int r = 0; r < nrows; ++r) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            const int col = c0 + 32 * c + lane;
+            const bool keep = col < p.KVB && fa_mask_mod(gb, gh, q0 + rbase + r, k0 + col);
+            const unsigned vote = __ballot_sync(0xffffffffu, keep);
+            if (lane == r) roww[c] = vote;
+            colw[c] |= (keep ? 1u : 0u) << r;
+          }
+        }
+      }
+      cnt += __popc(roww[0]) + __popc(roww[1]) + __popc(roww[2]) + __popc(roww[3]);
+      if (p.bits != nullptr) {
+        // the row's words of this sub-tile; keys beyond KV_LEN are 0, and the last block also writes the padding words
+        const int q = q0 + rbase + lane;
+        if (lane < nrows && q < p.Q_LEN) {
+          unsigned* dst = p.bits + ((long long)bh * p.Q_LEN + q) * p.stride;
+          const int w0 = (k0 + c0) >> 5;
+          const int wend = (kvb == p.nKV - 1 && c0 + 128 >= p.KVB) ? (int)p.stride : min(w0 + 4, (k0 + p.KVB) >> 5);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            const int left = p.KV_LEN - (k0 + c0 + 32 * c);
+            if (left < 32) roww[c] &= left <= 0 ? 0u : (1u << left) - 1u;
+          }
+          if ((w0 & 3) == 0 && w0 + 4 <= wend) {
+            *(uint4*)(dst + w0) = make_uint4(roww[0], roww[1], roww[2], roww[3]);
+          } else {
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+              if (w0 + c < wend) dst[w0 + c] = roww[c];
+          }
+          for (int w = w0 + 4; w < wend; ++w) dst[w] = 0u;
+        }
+      }
+      if (p.bits_t != nullptr) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) t_words[32 * c + lane][warp] = colw[c];
+        __syncthreads();
+        const int col = c0 + (int)threadIdx.x, kv = k0 + col;
+        if (col < p.KVB && kv < p.KV_LEN) {
+          unsigned* dst = p.bits_t + ((long long)bh * p.KV_LEN + kv) * p.stride_t;
+          const int w0 = (q0 + r0) >> 5;
+          const int wend = (qb == p.nQ - 1 && r0 + 128 >= p.QB) ? (int)p.stride_t : min(w0 + 4, (q0 + p.QB) >> 5);
+          unsigned w[4];
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            w[c] = t_words[threadIdx.x][c];
+            const int left = p.Q_LEN - (q0 + r0 + 32 * c);
+            if (left < 32) w[c] &= left <= 0 ? 0u : (1u << left) - 1u;
+          }
+          if ((w0 & 3) == 0 && w0 + 4 <= wend) {
+            *(uint4*)(dst + w0) = make_uint4(w[0], w[1], w[2], w[3]);
+          } else {
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+              if (w0 + c < wend) dst[w0 + c] = w[c];
+          }
+          for (int i = w0 + 4; i < wend; ++i) dst[i] = 0u;
+        }
+        __syncthreads();
+      }
+    }
+  }
+  if (p.cls == nullptr) return;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
+  if (lane == 0) s_cnt[warp] = cnt;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const int c = s_cnt[0] + s_cnt[1] + s_cnt[2] + s_cnt[3];
+    p.cls[((long long)bh * p.nQ + qb) * p.nKV + kvb] = (signed char)(c == 0 ? 0 : (c == p.QB * p.KVB ? 2 : 1));
+  }
+}
+
+// Any block size: one CTA per block counts the positions kept.
 extern "C" __global__ void __launch_bounds__(256) fa_blockmask_classify_kernel(const __grid_constant__ FaMaskParams p) {
+  FA_MOD_BUFS_INIT(p);
+  fa_grid_wait();
+  __shared__ long long s_cnt;
+  if (threadIdx.x == 0) s_cnt = 0;
+  __syncthreads();
   const int kvb = blockIdx.x, qb = blockIdx.y;
   const int bh = blockIdx.z;
   const int b = bh / p.H, h = bh - b * p.H;
@@ -25,41 +144,11 @@ extern "C" __global__ void __launch_bounds__(256) fa_blockmask_classify_kernel(c
 #else
   for (long long i = threadIdx.x; i < total; i += 256) cnt += 1;
 #endif
-  __shared__ long long s_cnt;
-  if (threadIdx.x == 0) s_cnt = 0;
-  __syncthreads();
   for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
   if ((threadIdx.x & 31) == 0) atomicAdd((unsigned long long*)&s_cnt, (unsigned long long)cnt);
   __syncthreads();
   if (threadIdx.x == 0) {
     const long long c = s_cnt;
-    p.cls[(((long long)b * p.H + h) * p.nQ + qb) * p.nKV + kvb] = (signed char)(c == 0 ? 0 : (c == total ? 2 : 1));
+    p.cls[((long long)bh * p.nQ + qb) * p.nKV + kvb] = (signed char)(c == 0 ? 0 : (c == total ? 2 : 1));
   }
-}
-
-// mask_mod of every (query, key) position as a bit matrix: one word (32 keys) per thread, bits of
-// keys beyond KV_LEN and the padding words of a row are 0.  The attention kernels read a row's words
-// on the tiles the BlockMask lists as partial instead of evaluating mask_mod 128 times per row
-// there (the reference materialises the whole boolean mask for the same purpose,
-// flaxattention/core/blockmask.py:277-322; this is 1 bit per position).
-extern "C" __global__ void __launch_bounds__(256) fa_mask_bits_kernel(const __grid_constant__ FaMaskBitsParams p) {
-  const long long w = (long long)blockIdx.x * 256 + threadIdx.x;  // word inside the row
-  const int q = blockIdx.y;
-  const int bh = blockIdx.z;
-  if (w >= p.stride) return;
-  const int b = bh / p.H, h = bh - b * p.H;
-  unsigned m = 0;
-#if FA_HAS_MASK_MOD
-  const int gb = b + p.b_off, gh = h + p.h_off;
-  const long long k0 = w * 32;
-#pragma unroll 4
-  for (int e = 0; e < 32; ++e) {
-    const long long kv = k0 + e;
-    if (kv < p.KV_LEN && fa_mask_mod(gb, gh, q, (int)kv)) m |= 1u << e;
-  }
-#else
-  const long long left = (long long)p.KV_LEN - w * 32;
-  m = left >= 32 ? 0xffffffffu : (left <= 0 ? 0u : ((1u << (int)left) - 1u));
-#endif
-  p.bits[(((long long)b * p.H + h) * p.Q_LEN + q) * p.stride + w] = m;
 }

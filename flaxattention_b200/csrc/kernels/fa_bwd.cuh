@@ -68,6 +68,8 @@ constexpr int DQ_SMEM = BQ * PQ + BQ * PV + 2 * BK * PQ + 2 * BK * PV + (F32 ? B
 extern "C" __global__ void __launch_bounds__(fa_bwd::NT) fa_bwd_dq_kernel(const __grid_constant__ FaParams p) {
   using namespace fa_bwd;
   extern __shared__ __align__(128) unsigned char smem[];
+  FA_MOD_BUFS_INIT(p);
+  fa_grid_wait();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int qt = gridDim.x - 1 - blockIdx.x;
   const int h = blockIdx.y, b = blockIdx.z;
@@ -201,6 +203,8 @@ constexpr int DKDV_SMEM = BK * PQ + BK * PV + 2 * BQ * PQ + 2 * BQ * PV + 2 * RO
 extern "C" __global__ void __launch_bounds__(fa_bwd::NT) fa_bwd_dkdv_kernel(const __grid_constant__ FaParams p) {
   using namespace fa_bwd;
   extern __shared__ __align__(128) unsigned char smem[];
+  FA_MOD_BUFS_INIT(p);
+  fa_grid_wait();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int kt = blockIdx.x;
   const int hk = blockIdx.y, b = blockIdx.z;

@@ -339,6 +339,7 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
     if (threadIdx.x == 0 && p.status != nullptr) atomicOr(p.status, FA_STATUS_BAD_LAUNCH);
     return;
   }
+  FA_MOD_BUFS_INIT(p);
   const fa_u32 raw = fa_smem_u32(smem_raw);
   const fa_u32 sb = (raw + 1023u) & ~1023u;
   unsigned char* sm = smem_raw + (sb - raw);
@@ -396,6 +397,7 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
     fa_tma_prefetch_desc(&P.tdo);
   }
   if (warp == WARP_MMA) fa_tmem_alloc(sb + OFF_MISC, TMEM_COLS);
+  fa_grid_wait();
   fa_tc_fence_before();
   __syncthreads();
   fa_tc_fence_after();

@@ -61,6 +61,8 @@ static_assert(WN % 16 == 0, "each warp needs at least 16 kv columns per tile");
 extern "C" __global__ void __launch_bounds__(fa_dec::NT) fa_decode_kernel(const __grid_constant__ FaParams p) {
   using namespace fa_dec;
   extern __shared__ __align__(128) unsigned char smem[];
+  FA_MOD_BUFS_INIT(p);
+  fa_grid_wait();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int rg = warp % RG, cg = warp / RG;
   // grid: (splits, query heads, batch), or (splits, kv heads, batch) when the heads of a group are packed
@@ -235,6 +237,7 @@ extern "C" __global__ void __launch_bounds__(fa_dec::NT) fa_decode_kernel(const 
     cur = (cur + 1) % STAGES;
   }
 
+  fa_grid_release();
   // ---- merge the CG column groups ------------------------------------------------------
   fa_cp_wait<0>();
   __syncthreads();

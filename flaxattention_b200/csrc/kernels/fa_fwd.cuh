@@ -107,6 +107,8 @@ __device__ __forceinline__ void softmax_tile(float (&s)[WM][BN / 8][4], float (&
 extern "C" __global__ void __launch_bounds__(fa_fwd::NT) fa_fwd_kernel(const __grid_constant__ FaParams p) {
   using namespace fa_fwd;
   extern __shared__ __align__(128) unsigned char smem[];
+  FA_MOD_BUFS_INIT(p);
+  fa_grid_wait();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int qt = gridDim.x - 1 - blockIdx.x;  // heavy (late) causal rows first
   const int h = blockIdx.y, b = blockIdx.z;

@@ -415,6 +415,8 @@ extern "C" __global__ void __launch_bounds__(fa_tc::NT, 1) fa_fwd_tc_kernel(cons
     if (threadIdx.x == 0 && p.status != nullptr) atomicOr(p.status, FA_STATUS_BAD_LAUNCH);
     return;
   }
+  FA_MOD_BUFS_INIT(p);
+  fa_grid_wait();
   const fa_u32 raw = fa_smem_u32(smem_raw);
   const fa_u32 sb = (raw + 1023u) & ~1023u;  // shared-window address of the aligned base
   unsigned char* sm = smem_raw + (sb - raw);

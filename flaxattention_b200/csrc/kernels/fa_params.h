@@ -31,7 +31,27 @@ struct FaTables {
   long long mask_stride;  // words per row (a multiple of 4: rows start on 16-byte boundaries)
   int mask_rows;          // rows per (batch, head) entry
   int mask_B, mask_H;     // entries of the matrix along batch / heads (1 = broadcast)
+  // the same matrix transposed, for the kernels whose threads own a key: bit (q % 32) of word
+  // [((bb * mask_H + hb) * mask_t_rows + kv) * mask_t_stride + q / 32].  Null: not built.
+  const unsigned* mask_bits_t;
+  long long mask_t_stride;
+  int mask_t_rows;
 };
+
+// Tensors a score_mod / mask_mod may capture and index (fa_module_set_buffers).  Their addresses travel
+// with the kernel parameters; a kernel whose mods read any copies them into the table the generated code
+// looks them up in (FA_MOD_BUFS_INIT), and its first block-wide barrier makes the table visible.
+#define FA_MAX_MOD_BUFS 8
+#ifdef FA_NUM_MOD_BUFS
+#define FA_MOD_BUFS_INIT(P)                                                                      \
+  do {                                                                                           \
+    if (threadIdx.x < FA_NUM_MOD_BUFS) fa_mod_buf[threadIdx.x] = (P).mod_buf[threadIdx.x];       \
+  } while (0)
+#else
+#define FA_MOD_BUFS_INIT(P) \
+  do {                      \
+  } while (0)
+#endif
 
 struct FaParams {
   FaTensor q, k, v, o;
@@ -46,19 +66,27 @@ struct FaParams {
   int num_splits;
   int n_q_tiles;
   float scale;
+  const void* mod_buf[FA_MAX_MOD_BUFS];
   FaTables t;
 };
 
-// Block classification grid -> ordered tables.
+// Evaluation of mask_mod over a block grid: the class of every block and, optionally, the mask itself as
+// bit matrices.  `B`, `H`: entries evaluated (1 where the mask does not read the batch / head index).
 struct FaMaskParams {
-  signed char* cls;  // [B,H,nQ,nKV]: 0 empty, 1 partial, 2 full
-  int B, H, nQ, nKV, QB, KVB;
+  signed char* cls;  // [B,H,nQ,nKV]: 0 empty, 1 partial, 2 full; or null
+  unsigned* bits;    // [B,H,Q_LEN,stride] words, or null
+  unsigned* bits_t;  // [B,H,KV_LEN,stride_t] words, or null
+  long long stride, stride_t;
+  int B, H, nQ, nKV, QB, KVB, Q_LEN, KV_LEN;
   int b_off, h_off;
+  const void* mod_buf[FA_MAX_MOD_BUFS];
 };
 
-struct FaMaskBitsParams {
-  unsigned* bits;      // [B,H,Q_LEN,stride] words
-  long long stride;    // words per row
-  int B, H, Q_LEN, KV_LEN;
-  int b_off, h_off;
-};
+#ifdef __CUDACC_RTC__
+// Programmatic dependent launch: a kernel of this library may be scheduled while the one in front of it on
+// the stream is finishing.  fa_grid_wait returns when that one is complete and its writes are visible
+// (every kernel calls it before its first access to global memory); fa_grid_release lets the next
+// kernel be scheduled as soon as every CTA of this one has called it or has exited.
+__device__ __forceinline__ void fa_grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void fa_grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+#endif

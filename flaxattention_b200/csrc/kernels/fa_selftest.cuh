@@ -14,6 +14,7 @@ struct FaSelftestParams {
 };
 
 extern "C" __global__ void __launch_bounds__(64, 1) fa_wait_selftest_kernel(const __grid_constant__ FaSelftestParams p) {
+  fa_grid_wait();
   __shared__ __align__(8) unsigned long long bar;
   __shared__ int abort_word;
   const fa_u32 b = fa_smem_u32(&bar);

@@ -21,12 +21,19 @@ Python scalars are weakly typed the way JAX treats them: ``int32 * 8.0`` is floa
 """
 from __future__ import annotations
 
+import builtins
+import copy
+import dis
+import functools
 import hashlib
 import inspect
 import math
+import types
+import weakref
 from typing import Callable, Dict, List, Optional, Sequence, Tuple
 
 import numpy as np
+import torch
 
 I32, F32, B1 = "i32", "f32", "b1"
 
@@ -407,11 +414,13 @@ def _lift(x) -> Expr:
     if isinstance(x, (float, np.floating)):
         return _B.const(float(x), F32)
     if isinstance(x, np.ndarray) and x.ndim == 0:
+        _note_tensor_value()
         return _lift(x.item())
     try:  # 0-d torch tensors captured as constants
         import torch
 
         if isinstance(x, torch.Tensor) and x.ndim == 0:
+            _note_tensor_value()
             return _lift(x.item())
     except ImportError:  # pragma: no cover
         pass
@@ -433,6 +442,12 @@ _ELEM_TYPES = {
     "int32": ("i32", I32), "int64": ("i64", I32), "uint8": ("u8", I32), "bool": ("u8", B1), "float32": ("f32", F32),
 }
 _TRACE_BUFFERS: Optional[List[object]] = None  # buffers of the mod pair being traced
+_TENSOR_VALUES_READ = False  # set when a trace turns the contents of a tensor into a constant
+
+
+def _note_tensor_value():
+    global _TENSOR_VALUES_READ
+    _TENSOR_VALUES_READ = True
 
 
 def _buffer_load(buf, index) -> "Sym":
@@ -799,6 +814,10 @@ _TORCH_FUNCS = {
 def mod_arity(fn: Callable) -> int:
     """Number of parameters without a default: 5 marks a score_mod, 4 a mask_mod
     (flaxattention/core/common.py:20-39)."""
+    if type(fn) is types.FunctionType and not fn.__dict__:
+        code = fn.__code__
+        if not code.co_flags & (inspect.CO_VARARGS | inspect.CO_VARKEYWORDS) and not code.co_kwonlyargcount:
+            return code.co_argcount - len(fn.__defaults__ or ())  # what inspect.signature takes 10 us to find
     return sum(
         1 for p in inspect.signature(fn).parameters.values() if p.default is inspect.Parameter.empty
     )
@@ -1438,8 +1457,8 @@ __device__ __forceinline__ float fa_pymod_f32(float a, float b) {
 
 
 _BUFFER_PRELUDE = r"""
-// Captured buffers: the host writes the device addresses here before every launch.
-__constant__ const void* fa_mod_buf[FA_NUM_MOD_BUFS];
+// Captured buffers: every kernel fills this table from its parameters (FA_MOD_BUFS_INIT).
+__shared__ const void* fa_mod_buf[FA_NUM_MOD_BUFS];
 __device__ __forceinline__ int fa_ld_i32(int k, int i) { return __ldg((const int*)fa_mod_buf[k] + i); }
 __device__ __forceinline__ int fa_ld_i64(int k, int i) { return (int)__ldg((const long long*)fa_mod_buf[k] + i); }
 __device__ __forceinline__ int fa_ld_u8(int k, int i) { return (int)__ldg((const unsigned char*)fa_mod_buf[k] + i); }
@@ -1502,6 +1521,9 @@ class ModSet:
                 "__device__ __forceinline__ float fa_score_mod(float score, int, int, int, int) { return score; }\n"
                 "__device__ __forceinline__ float fa_score_mod_grad(float, int, int, int, int) { return 1.0f; }\n"
             )
+        # whether the mask differs between batch entries / heads
+        self.mask_reads_b = self.mask is not None and _depends_on(self.mask.root, "b", {})
+        self.mask_reads_h = self.mask is not None and _depends_on(self.mask.root, "h", {})
         if self.mask is not None:
             parts.append(to_cuda(self.mask, "fa_mask_mod"))
         else:
@@ -1528,22 +1550,171 @@ def _trace_any(fn: Callable, kind: str, bufs: List[object]) -> TracedMod:
             raise first from None
 
 
-_MODSET_CACHE: Dict[Tuple[Optional[int], Optional[int]], Tuple[object, object, ModSet]] = {}
+# --------------------------------------------------------------------------------------
+# what a mod's trace depends on
+# --------------------------------------------------------------------------------------
+# A training loop over packed documents makes a new mask_mod for every batch, the same code over
+# another tensor.  Tracing and lowering it takes 100-200 us; what the trace can depend on (the code, the
+# constants it closes over, shape, strides and type of its tensors) is gone through in about 10, and a pair
+# of mods with equal fingerprints shares the lowered text and only brings its own tensors.
+@functools.lru_cache(maxsize=1024)
+def _code_facts(code):
+    """(names the code and the code nested in it use, whether it branches on a value)."""
+    names, branches = set(code.co_names), False
+    for ins in dis.get_instructions(code):
+        if "JUMP_IF" in ins.opname:
+            branches = True
+    for c in code.co_consts:
+        if isinstance(c, types.CodeType):
+            n, br = _code_facts(c)
+            names |= set(n)
+            branches = branches or br
+    return tuple(sorted(names)), branches
+
+
+class _Unknown(Exception):
+    """The trace may depend on something a fingerprint does not cover."""
+
+
+def _fingerprint_value(x, tensors: List[object], out: List[object], depth: int) -> None:
+    t = type(x)
+    if x is None or t in (bool, int, float, str):
+        out.append((t, x))
+    elif t is types.FunctionType:
+        _fingerprint_function(x, tensors, out, depth + 1)
+    elif t in (tuple, list):
+        out.append((t, len(x)))
+        for y in x:
+            _fingerprint_value(y, tensors, out, depth + 1)
+    elif t is torch.Tensor:
+        k = next((i for i, y in enumerate(tensors) if y is x), len(tensors))
+        if k == len(tensors):
+            tensors.append(x)
+        out.append(("tensor", k, x.dtype, tuple(x.shape), x.stride()))
+    else:
+        raise _Unknown
+
+
+def _fingerprint_function(fn, tensors: List[object], out: List[object], depth: int = 0) -> None:
+    if depth > 8:
+        raise _Unknown
+    code = fn.__code__
+    names, branches = _code_facts(code)
+    out.append(code)
+    before = len(tensors)
+    for cell in fn.__closure__ or ():
+        try:
+            _fingerprint_value(cell.cell_contents, tensors, out, depth)
+        except ValueError:  # an empty cell
+            raise _Unknown from None
+    for d in (fn.__defaults__, tuple(sorted((fn.__kwdefaults__ or {}).items()))):
+        _fingerprint_value(d, tensors, out, depth)
+    g = fn.__globals__
+    modules = [g[n] for n in names if isinstance(g.get(n), types.ModuleType)]
+    for n in names:
+        if n in g:
+            if isinstance(g[n], types.ModuleType):
+                out.append(("module", n, id(g[n])))
+            else:
+                out.append(n)
+                _fingerprint_value(g[n], tensors, out, depth)
+        elif hasattr(builtins, n):
+            if n != "abs":
+                raise _Unknown  # int(tensor), len(...) and the like
+        elif any(hasattr(m, n) for m in modules):
+            # an attribute of a module: a function of it, or a constant
+            for m in modules:
+                x = getattr(m, n, None)
+                if isinstance(x, (bool, int, float)):
+                    out.append((n, x))
+                elif isinstance(x, (torch.Tensor, np.ndarray)):
+                    raise _Unknown
+                else:
+                    out.append((n, id(x)))
+        else:
+            raise _Unknown  # a method or an attribute of a value
+    if branches and len(tensors) > before:
+        raise _Unknown  # may branch on the contents of a tensor
+
+
+class _Template:
+    """A lowered pair of mods without its tensors."""
+
+    def __init__(self, ms: ModSet, which: List[int]):
+        self.ms = copy.copy(ms)
+        self.ms.buffers = []
+        if ms.buffers:  # the graphs stay, the tensors they were traced over do not
+            for name in ("score", "mask"):
+                m = getattr(ms, name)
+                setattr(self.ms, name, None if m is None else TracedMod(m.kind, m.root))
+        self.which = which  # per buffer, its place among the fingerprint's tensors
+
+    def bind(self, tensors: List[object]) -> ModSet:
+        ms = copy.copy(self.ms)
+        ms.buffers = [tensors[k] for k in self.which]
+        return ms
+
+
+_TEMPLATES: Dict[object, _Template] = {}
+# per pair of callables (by identity, 0: no mod), as long as both exist: what keeps track of them, and the lowered pair
+_MODSET_CACHE: Dict[Tuple[int, int], Tuple[object, object, ModSet]] = {}
+_ON_FORGET: List[Callable[[int, int], None]] = []  # told when a pair leaves the cache
+
+
+def _forget(key: Tuple[int, int]) -> None:
+    _MODSET_CACHE.pop(key, None)
+    for f in _ON_FORGET:
+        f(*key)
+
+
+def _hold(fn, key):
+    """A callable that gives ``fn``, and that lets the pair's entry go with ``fn``."""
+    if fn is None:
+        return lambda: None
+    try:
+        return weakref.ref(fn, lambda _: _forget(key))
+    except TypeError:  # no weak references to this type of callable: it stays
+        return lambda: fn
 
 
 def lower_mods(score_mod: Optional[Callable], mask_mod: Optional[Callable]) -> ModSet:
     """Traces and lowers a pair of mods; cached on the identity of the callables (the
     reference keys its jit cache the same way: mods are static arguments,
-    flaxattention/core/attention.py:169)."""
-    k = (None if score_mod is None else id(score_mod), None if mask_mod is None else id(mask_mod))
-    hit = _MODSET_CACHE.get(k)
-    if hit is not None and hit[0] is score_mod and hit[1] is mask_mod:
+    flaxattention/core/attention.py:169) for as long as they exist."""
+    key = (0 if score_mod is None else id(score_mod), 0 if mask_mod is None else id(mask_mod))
+    hit = _MODSET_CACHE.get(key)
+    if hit is not None and hit[0]() is score_mod and hit[1]() is mask_mod:
         return hit[2]
-    bufs: List[object] = []
-    s = _trace_any(score_mod, "score", bufs) if score_mod is not None else None
-    m = _trace_any(mask_mod, "mask", bufs) if mask_mod is not None else None
-    ms = ModSet(s, m, bufs)
+    tensors: List[object] = []
+    fp = None
+    try:
+        parts: List[object] = []
+        for fn in (score_mod, mask_mod):
+            parts.append("|")
+            if fn is not None:
+                if type(fn) is not types.FunctionType:
+                    raise _Unknown
+                _fingerprint_function(fn, tensors, parts)
+        fp = tuple(parts)
+    except _Unknown:
+        fp = None
+    tpl = _TEMPLATES.get(fp) if fp is not None else None
+    if tpl is not None:
+        ms = tpl.bind(tensors)
+    else:
+        global _TENSOR_VALUES_READ
+        _TENSOR_VALUES_READ = False
+        bufs: List[object] = []
+        s = _trace_any(score_mod, "score", bufs) if score_mod is not None else None
+        m = _trace_any(mask_mod, "mask", bufs) if mask_mod is not None else None
+        ms = ModSet(s, m, bufs)
+        which = [next((i for i, t in enumerate(tensors) if t is b), -1) for b in ms.buffers]
+        if fp is not None and -1 not in which and len(set(which)) == len(tensors) and not _TENSOR_VALUES_READ:
+            if len(_TEMPLATES) >= 1024:
+                _TEMPLATES.clear()
+            _TEMPLATES[fp] = _Template(ms, which)
     if len(_MODSET_CACHE) > 4096:
-        _MODSET_CACHE.clear()
-    _MODSET_CACHE[k] = (score_mod, mask_mod, ms)
+        for k in list(_MODSET_CACHE):
+            _forget(k)
+    _MODSET_CACHE[key] = (_hold(score_mod, key), _hold(mask_mod, key), ms)
     return ms

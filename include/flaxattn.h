@@ -86,6 +86,11 @@ typedef struct fa_block_tables {
   int64_t mask_bits_stride; /* words per row, fa_mask_bits_row_words(KV_LEN) */
   int32_t mask_bits_rows;   /* rows per (batch, head) entry (Q_LEN) */
   int32_t mask_bits_B, mask_bits_H; /* 1 or B / Hq */
+  /* Optional, with mask_bits: the same matrix transposed, bit (q % 32) of word
+   * [((bb * mask_bits_H + hb) * mask_bits_t_rows + kv) * mask_bits_t_stride + q / 32]. */
+  const uint32_t* mask_bits_t;
+  int64_t mask_bits_t_stride; /* words per row, fa_mask_bits_row_words(Q_LEN) */
+  int32_t mask_bits_t_rows;   /* rows per (batch, head) entry (KV_LEN) */
 } fa_block_tables;
 
 typedef struct fa_attn_params {
@@ -117,9 +122,11 @@ void fa_module_destroy(fa_module* m);
 /* Device addresses of the buffers the mods of this module read (`fa_mod_buf[k]` in mod_source, at
  * most 8): the tensors a score_mod / mask_mod closes over and indexes with b, h, q, kv - the
  * reference's score_mod_other_buffers / mask_mod_other_buffers (flaxattention/core/attention.py:22-23,
- * :35-52), there jaxpr constants.  The addresses are copied into the kernel image, in stream order,
- * before every later launch of a kernel of the module; calls that use one module with different
- * buffer sets must not overlap, and such launches cannot be stream-captured. */
+ * :35-52), there jaxpr constants.  Later launches of kernels of the module take the addresses along as
+ * kernel parameters (a mod_source that declares `__shared__ const void* fa_mod_buf[n]`, as generated
+ * ones do, gets the table filled by the kernel).  A mod_source that declares the table __constant__ has
+ * it rewritten in the kernel image, in stream order, before every launch; calls that use such a module
+ * with different buffer sets must not overlap, and such launches cannot be stream-captured. */
 int fa_module_set_buffers(fa_module* m, const void* const* ptrs, int n);
 /* Compiles (or fetches from the cache) the kernels of one kind for a dtype / head-dim pair.
  * Needs no GPU.  seq_hint selects the tile configuration the same way a later launch would. */
@@ -205,6 +212,21 @@ int fa_block_mask(fa_module* m, int B, int H, int Q_LEN, int KV_LEN, int q_block
                   int32_t* q_num_blocks, int32_t* q_indices,
                   int32_t* full_q_num_blocks, int32_t* full_q_indices,
                   void* workspace, size_t workspace_bytes, void* stream);
+
+/* The same with the options of one description: the mask is evaluated for distinct_B x distinct_H entries
+ * (1 where mask_mod does not read the batch / head index; the tables are still written for B x H), and
+ * the evaluation also leaves the mask as bit matrices when asked to.  workspace:
+ * fa_block_mask_workspace_bytes(distinct_B, distinct_H, ...). */
+typedef struct fa_mask_build {
+  int32_t B, H, distinct_B, distinct_H, Q_LEN, KV_LEN, q_block, kv_block, b_offset, h_offset;
+  int32_t *kv_num_blocks, *kv_indices, *full_kv_num_blocks, *full_kv_indices; /* all null: bit matrices only */
+  int32_t *q_num_blocks, *q_indices, *full_q_num_blocks, *full_q_indices;
+  uint32_t* bits;   /* [distinct_B, distinct_H, Q_LEN, fa_mask_bits_row_words(KV_LEN)] or null */
+  uint32_t* bits_t; /* [distinct_B, distinct_H, KV_LEN, fa_mask_bits_row_words(Q_LEN)] or null */
+  void* workspace;
+  size_t workspace_bytes;
+} fa_mask_build;
+int fa_block_mask_build(fa_module* m, const fa_mask_build* mb, void* stream);
 
 /* mask_mod of every position as a bit matrix [B, H, Q_LEN, fa_mask_bits_row_words(KV_LEN)] (uint32,
  * device, 16-byte aligned) for fa_block_tables::mask_bits.  The reference materialises the boolean

@@ -1,0 +1,61 @@
+"""The one-evaluation mask construction (fa_mask_scan_kernel) at the edges of its 128 x 128 sub-tiles and
+32-bit words: tables and both bit matrices against the CPU oracle, and bit matrices over captured
+tensors that change after they were built."""
+import numpy as np
+import pytest
+import torch
+
+from cases import TABLE_KEYS, head_dependent
+from oracle.blockmask_oracle import create_block_mask_oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def _unpack(bits, n):
+    a = bits.cpu().numpy().view(np.uint32)
+    return ((a[..., None] >> np.arange(32, dtype=np.uint32)) & 1).astype(bool).reshape(*a.shape[:-1], -1)[..., :n]
+
+
+@pytest.mark.parametrize("Q,KV,block", [
+    (1, 32, (128, 32)), (50, 192, (64, 64)), (127, 512, (128, 128)), (128, 128, (128, 128)), (192, 320, (96, 160)),
+    (256, 384, (32, 384)), (512, 640, (256, 64)), (384, 288, (128, 288)), (130, 200, (130, 100)),
+])
+def test_tables_and_bits_at_word_and_tile_edges(Q, KV, block):
+    import flaxattention_b200 as fa
+
+    B, H = 2, 3
+    whole_words = block[1] % 32 == 0 or KV <= block[1]
+    bm = fa.create_block_mask(head_dependent, B, H, Q, KV, BLOCK_SIZE=block)
+    torch.cuda.synchronize()
+    want = create_block_mask_oracle(head_dependent, B, H, Q, KV, BLOCK_SIZE=block)
+    for k in TABLE_KEYS:
+        assert np.array_equal(getattr(bm, k).cpu().numpy(), want[k]), k
+    assert (bm.mask_bits is not None) == whole_words
+    if whole_words:
+        q, kv = np.arange(Q)[:, None], np.arange(KV)[None, :]
+        for b in range(B):
+            for h in range(H):
+                dense = head_dependent(b, h, q, kv)
+                assert np.array_equal(_unpack(bm.mask_bits, KV)[b, h][:Q], dense)
+                assert np.array_equal(_unpack(bm.mask_bits_t, Q)[b, h][:KV], dense.T)
+
+
+def test_bits_over_a_captured_tensor_are_dropped_when_it_changes():
+    """The tables keep what they were built from; on the partial tiles the mask is evaluated again."""
+    import flaxattention_b200 as fa
+
+    S = 256
+    limit = torch.full((S,), 200, dtype=torch.int32, device="cuda")
+
+    def up_to_limit(b, h, q_idx, kv_idx):
+        return kv_idx < limit[q_idx]
+
+    q, k, v = (torch.randn(1, 2, S, 64, device="cuda", dtype=torch.float16) for _ in range(3))
+    bm = fa.create_block_mask(up_to_limit, None, None, S, S)
+    assert bm.bits_hold() and bm.mask_bits_t is not None
+    fa.flax_attention(q, k, v, block_mask=bm)
+    limit.fill_(150)  # the second key block is still partial
+    assert not bm.bits_hold()
+    got = fa.flax_attention(q, k, v, block_mask=bm)
+    fresh = fa.flax_attention(q, k, v, block_mask=fa.create_block_mask(up_to_limit, None, None, S, S))
+    assert torch.equal(got, fresh)
