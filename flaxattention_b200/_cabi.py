@@ -70,6 +70,7 @@ EXPORTS = [
     "fa_block_mask_workspace_bytes", "fa_block_mask", "fa_decode_static_capacity", "fa_decode_static",
     "fa_profile_enable", "fa_profile_read", "fa_decode_packs_heads", "fa_selftest_bounded_wait",
     "fa_mask_bits_row_words", "fa_mask_bits", "fa_block_mask_build",
+    "fa_fwd_workspace_bytes", "fa_fwd_ws",
 ]
 
 
@@ -98,6 +99,9 @@ def lib() -> C.CDLL:
     L.fa_set_kernel_dir.argtypes = [C.c_char_p]
     L.fa_set_cache_dir.argtypes = [C.c_char_p]
     L.fa_fwd.argtypes = [C.c_void_p, C.POINTER(FaAttnParams), C.c_void_p]
+    L.fa_fwd_workspace_bytes.restype = C.c_size_t
+    L.fa_fwd_workspace_bytes.argtypes = [C.POINTER(FaAttnParams)]
+    L.fa_fwd_ws.argtypes = [C.c_void_p, C.POINTER(FaAttnParams), C.c_void_p, C.c_size_t, C.c_void_p]
     L.fa_block_mask_workspace_bytes.restype = C.c_size_t
     L.fa_block_mask_workspace_bytes.argtypes = [C.c_int] * 6
     L.fa_block_mask.argtypes = [C.c_void_p] + [C.c_int] * 8 + [C.c_void_p] * 8 + [C.c_void_p, C.c_size_t, C.c_void_p]

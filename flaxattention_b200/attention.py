@@ -214,7 +214,9 @@ def _forward(call: _Call, q, k, v):
             ws = torch.empty(max(nbytes, 16), dtype=torch.uint8, device=q.device)
             _cabi.check(L.fa_decode(call.module.handle, p, splits, ws.data_ptr(), nbytes, stream))
         else:
-            _cabi.check(L.fa_fwd(call.module.handle, p, stream))
+            nbytes = L.fa_fwd_workspace_bytes(p)
+            ws = torch.empty(nbytes, dtype=torch.uint8, device=q.device) if nbytes else None
+            _cabi.check(L.fa_fwd_ws(call.module.handle, p, _ptr(ws), nbytes, stream))
     return out, lse
 
 

@@ -110,7 +110,7 @@ std::string cache_dir() {
 }
 
 const char* const kTemplateFiles[] = {"fa_params.h", "fa_common.cuh", "fa_fwd.cuh", "fa_bwd.cuh",
-                                      "fa_decode.cuh", "fa_blockmask.cuh", "fa_sm100.cuh", "fa_fwd_tc.cuh", "fa_bwd_tc.cuh", "fa_selftest.cuh"};
+                                      "fa_decode.cuh", "fa_blockmask.cuh", "fa_sm100.cuh", "fa_fwd_tc.cuh", "fa_bwd_tc.cuh", "fa_bwd_f32.cuh", "fa_selftest.cuh"};
 std::string g_templates_hash;
 int templates_hash(std::string& out) {
   if (g_templates_hash.empty()) {
@@ -190,7 +190,7 @@ const char* const kDefaultMods =
 
 // A kernel variant of a module as a number: every launch looks its kernel up by it, and the define text
 // is only put together when the variant has to be compiled or fetched from the cache on disk.
-enum KernelId : int { kIdFwd, kIdFwdTc, kIdBwdDq, kIdBwdDkdv, kIdBwdTc, kIdDecode, kIdMaskScan, kIdMaskClassify, kIdSelftest };
+enum KernelId : int { kIdFwd, kIdFwdTc, kIdBwdDq, kIdBwdDkdv, kIdBwdTc, kIdBwdF32, kIdDecode, kIdMaskScan, kIdMaskClassify, kIdSelftest };
 uint64_t kernel_key(KernelId id, std::initializer_list<std::pair<int, int>> fields) {  // (value, bits)
   uint64_t k = 0;
   for (auto& f : fields) k = (k << f.second) | (uint64_t)f.first;
@@ -628,6 +628,83 @@ __global__ void __launch_bounds__(128) fa_tables_kernel(const signed char* __res
 }
 
 
+// fp32 rows of 64 values as rows of three bf16 parts, [hi | mid | lo] (192 values, contiguous), for the
+// tcgen05 kernels with fp32 inputs: hi is the value rounded to bf16, mid the remainder rounded, lo the
+// rest.  Up to four tensors in one launch (blockIdx.y), 8 threads per row: a thread reads 32 bytes and
+// writes 16 bytes of each part.  Bound by memory: 4 bytes in and 6 out per value.
+//
+// In front of the backward the same pass does the rest of its preparation: with q it clears dQ (the kernel adds
+// to it), with dO it leaves the per-row scalars nlse2 = -lse * log2(e) (-inf for rows without mass or beyond
+// Sq) and ndelta = -sum_d O * dO (0 beyond Sq), padded to whole 128-row tiles.
+struct FaSplitJob {
+  FaTensor src;
+  uint4* dst;
+  int H, S, S_rows;  // S_rows: rows gone through per (batch, head), at least S
+  long long rows;
+  FaTensor clear;    // cleared rows (ptr null: none)
+  FaTensor o;        // with it the row scalars (ptr null: none)
+  const float* lse;
+  float *nlse2, *ndelta;
+};
+struct FaSplitJobs {
+  FaSplitJob job[4];
+  int* counter;  // set to zero (or null)
+};
+__global__ void __launch_bounds__(256) fa_split3_kernel(const __grid_constant__ FaSplitJobs jobs) {
+  grid_wait();
+  grid_release();
+  const FaSplitJob& j = jobs.job[blockIdx.y];
+  const long long t = (long long)blockIdx.x * 256 + threadIdx.x;
+  if (t == 0 && blockIdx.y == 0 && jobs.counter != nullptr) *jobs.counter = 0;
+  const long long row = t >> 3;
+  const int c = (int)t & 7;
+  if (row >= j.rows) return;  // (the eight threads of a row together)
+  const long long bh = row / j.S_rows;
+  const int s = (int)(row - bh * j.S_rows);
+  const int b = (int)(bh / j.H), h = (int)(bh - (long long)b * j.H);
+  auto at = [&](const FaTensor& x) {
+    return (float4*)((float*)x.ptr + (long long)b * x.sb + (long long)h * x.sh + (long long)s * x.ss) + 2 * c;
+  };
+  const bool valid = s < j.S;
+  float4 lo4 = make_float4(0.f, 0.f, 0.f, 0.f), hi4 = lo4;
+  if (valid) {
+    lo4 = at(j.src)[0];
+    hi4 = at(j.src)[1];
+    const float x[8] = {lo4.x, lo4.y, lo4.z, lo4.w, hi4.x, hi4.y, hi4.z, hi4.w};
+    unsigned part[3][4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      float2 v = make_float2(x[2 * e], x[2 * e + 1]);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        const __nv_bfloat162 r = __floats2bfloat162_rn(v.x, v.y);
+        part[k][e] = *reinterpret_cast<const unsigned*>(&r);
+        const float2 f = __bfloat1622float2(r);
+        v.x -= f.x;
+        v.y -= f.y;
+      }
+    }
+    uint4* dst = j.dst + (bh * j.S + s) * 24 + c;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) dst[8 * k] = make_uint4(part[k][0], part[k][1], part[k][2], part[k][3]);
+    if (j.clear.ptr != nullptr) at(j.clear)[0] = at(j.clear)[1] = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  if (j.o.ptr == nullptr) return;  // (the same for the whole launch row)
+  float acc = 0.f;
+  if (valid) {
+    const float4 a = at(j.o)[0], d = at(j.o)[1];
+    acc = a.x * lo4.x + a.y * lo4.y + a.z * lo4.z + a.w * lo4.w + d.x * hi4.x + d.y * hi4.y + d.z * hi4.z + d.w * hi4.w;
+  }
+  const unsigned group = 0xffu << (threadIdx.x & 24);
+#pragma unroll
+  for (int off = 4; off > 0; off >>= 1) acc += __shfl_xor_sync(group, acc, off);
+  if (c == 0) {
+    const float l = valid ? j.lse[bh * j.S + s] : -INFINITY;
+    j.nlse2[row] = l != -INFINITY ? -(l * 1.4426950408889634f) : -INFINITY;
+    j.ndelta[row] = -acc;
+  }
+}
+
 // delta[b,h,q] = sum_d O[b,h,q,d] * dO[b,h,q,d]  (flaxattention/kernel/attention.py:338-345).
 // LPR lanes cooperate on one row; each lane reads 16-byte pieces.
 template <int DT, int LPR>
@@ -1024,15 +1101,19 @@ int encode_fn(EncodeTiledFn* out) {
   return FA_OK;
 }
 
-// 4-d map (D, S, H, B) over a [.., S, D]-strided tensor; box = 64 elements x box_rows rows, 128-byte swizzle
+// 4-d map (D, S, H, B) over a [.., S, D]-strided tensor; box = 128 bytes x box_rows rows, 128-byte swizzle
 int make_map(FaTensorMapHost* out, int dtype, const fa_tensor& t, int D, int S, int H, int B, int box_rows = 128) {
   EncodeTiledFn enc = nullptr;
   if (int rc = encode_fn(&enc)) return rc;
   const cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)S, (cuuint64_t)H, (cuuint64_t)B};
-  const cuuint64_t strides[3] = {(cuuint64_t)t.stride_s * 2, (cuuint64_t)t.stride_h * 2, (cuuint64_t)t.stride_b * 2};
-  const cuuint32_t box[4] = {64, (cuuint32_t)box_rows, 1, 1};
+  const cuuint64_t es = (cuuint64_t)esize(dtype);
+  const cuuint64_t strides[3] = {(cuuint64_t)t.stride_s * es, (cuuint64_t)t.stride_h * es, (cuuint64_t)t.stride_b * es};
+  const cuuint32_t box[4] = {(cuuint32_t)(128 / es), (cuuint32_t)box_rows, 1, 1};
   const cuuint32_t estr[4] = {1, 1, 1, 1};
-  CUresult r = enc((CUtensorMap*)out, dtype == FA_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4,
+  const CUtensorMapDataType type = dtype == FA_F16    ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
+                                   : dtype == FA_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
+                                                      : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
+  CUresult r = enc((CUtensorMap*)out, type, 4,
                    t.ptr, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(FA_ECUDA, "cuTensorMapEncodeTiled failed with code " + std::to_string((int)r));
@@ -1058,13 +1139,60 @@ bool tc_fwd_eligible(const fa_attn_params* p) {
 // decode = true selects the split-KV variant of the kernel (one query tile per CTA, partial results)
 int get_fwd_tc_kernel(fa_module* m, int dtype, int D, int flags, Kernel** k, bool decode = false) {
   // must match the shared-memory map of fa_fwd_tc.cuh (fa_tc::SMEM_BYTES)
-  const int atoms = D / 64, nstage = decode ? 5 : (D == 64 ? 3 : 2);
+  const int atoms = dtype == FA_F32 ? 3 : D / 64, nstage = decode ? 5 : (dtype == FA_F32 ? 1 : (D == 64 ? 3 : 2));
   const int smem = 2 * atoms * 16384 + 2 * nstage * atoms * 16384 + (1 + 4 * nstage + 8) * 8 + 16 + 256 * 2 + 256 * 2 +
                    2 * 256 + (256 / 32) * 4 + 1024;
   const int rnd = round_flag(dtype, flags);
   return get_kernel(m, kernel_key(kIdFwdTc, {{dtype, 2}, {D, 9}, {rnd, 1}, {decode ? 1 : 0, 1}}), "fa_fwd_tc.cuh",
                     [&] { return defs({{"FA_DTYPE", dtype}, {"FA_D", D}, {"FA_ROUND_SCORES", rnd}, {"FA_TC_DECODE", decode ? 1 : 0}}); },
                     "fa_fwd_tc_kernel", smem, k);
+}
+
+// fp32 on the tensor cores: the operands as three bf16 parts (fa_fwd_tc.cuh).
+bool tc_fwd_f32_eligible(const fa_attn_params* p) {
+  if (p->flags & FA_FLAG_GENERAL_KERNELS) return false;
+  if (p->dtype != FA_F32 || p->D != 64 || p->Dv != 64) return false;
+  if (p->Skv > 32768 || !(p->scale > 0.f)) return false;
+  const fa_block_tables& t = p->tables;
+  if (t.kv_num_blocks) {
+    if (!(t.num_q_blocks == 1 || t.q_block_size % 128 == 0)) return false;
+    if (!(t.num_kv_blocks == 1 || t.kv_block_size % 128 == 0)) return false;
+  }
+  return true;
+}
+// bytes of a [B, H, S, 64] tensor as three bf16 parts
+size_t split3_bytes(int B, int H, int S) { return (size_t)B * H * S * 192 * 2; }
+fa_tensor split3_tensor(void* ptr, int H, int S) { return fa_tensor{ptr, (int64_t)H * S * 192, (int64_t)S * 192, 192}; }
+FaSplitJob split_job(const fa_tensor& src, void* dst, int B, int H, int S) {
+  FaSplitJob j;
+  memset(&j, 0, sizeof j);
+  j.src = cvt(src); j.dst = (uint4*)dst; j.H = H; j.S = j.S_rows = S; j.rows = (long long)B * H * S;
+  return j;
+}
+int launch_split3(const FaSplitJobs& jobs, int n, void* stream) {
+  long long rows = 0;
+  for (int i = 0; i < n; ++i) rows = std::max(rows, jobs.job[i].rows);
+  return launch_here("fa_split3_kernel", fa_split3_kernel, dim3((unsigned)((rows * 8 + 255) / 256), (unsigned)n), dim3(256), stream, jobs);
+}
+int launch_fwd_f32_tc(fa_module* m, const fa_attn_params* p, const FaParams& kp, void* workspace, void* stream) {
+  Kernel* k = nullptr;
+  if (int rc = get_fwd_tc_kernel(m, p->dtype, p->D, p->flags, &k)) return rc;
+  char* ws = (char*)workspace;
+  char* wk = ws + split3_bytes(p->B, p->Hq, p->Sq);
+  char* wv = wk + split3_bytes(p->B, p->Hkv, p->Skv);
+  FaSplitJobs jobs;
+  memset(&jobs, 0, sizeof jobs);
+  jobs.job[0] = split_job(p->q, ws, p->B, p->Hq, p->Sq);
+  jobs.job[1] = split_job(p->k, wk, p->B, p->Hkv, p->Skv);
+  jobs.job[2] = split_job(p->v, wv, p->B, p->Hkv, p->Skv);
+  if (int rc = launch_split3(jobs, 3, stream)) return rc;
+  FaTcParamsHost tp;
+  tp.p = kp;
+  if (int rc = make_map(&tp.tq, FA_BF16, split3_tensor(ws, p->Hq, p->Sq), 192, p->Sq, p->Hq, p->B)) return rc;
+  if (int rc = make_map(&tp.tk, FA_BF16, split3_tensor(wk, p->Hkv, p->Skv), 192, p->Skv, p->Hkv, p->B)) return rc;
+  if (int rc = make_map(&tp.tv, FA_BF16, split3_tensor(wv, p->Hkv, p->Skv), 192, p->Skv, p->Hkv, p->B)) return rc;
+  if (int rc = make_map(&tp.to, FA_F32, p->o, p->Dv, p->Sq, p->Hq, p->B)) return rc;
+  return launch(k, dim3(p->Hq, p->B, (p->Sq + 255) / 256), dim3(384), &tp, stream);
 }
 
 // Shapes the split-KV variant of the tcgen05 kernel covers (`num_splits` CTAs per (batch, head), one
@@ -1167,6 +1295,61 @@ size_t dq_acc_bytes(const fa_attn_params* p) {
   return (size_t)p->B * p->Hq * sq_pad * p->D * sizeof(float);
 }
 
+// fp32 on the tensor cores (fa_bwd_f32.cuh)
+struct FaBwdF32ParamsHost {
+  FaParams p;
+  FaTensorMapHost tq, tk, tv, tdo;
+  const float* nlse2;
+  const float* ndelta;
+  int* work_counter;
+};
+bool tc_bwd_f32_eligible(const fa_attn_params* p) {
+  if (!tc_fwd_f32_eligible(p)) return false;
+  const int n_qtiles = (p->Sq + 127) / 128;
+  // the pair list of an item (fa_bf32::MAXPL pairs of 64 query rows)
+  return n_qtiles <= 256 && (long long)2 * n_qtiles * (p->Hq / p->Hkv) <= 512;
+}
+// workspace: parts of q, k, v, dO | nlse2 | ndelta | item counter
+size_t bwd_f32_workspace(const fa_attn_params* p) {
+  return 2 * split3_bytes(p->B, p->Hq, p->Sq) + 2 * split3_bytes(p->B, p->Hkv, p->Skv) + 2 * rows_pad_bytes(p) + 256;
+}
+int launch_bwd_f32_tc(fa_module* m, const fa_attn_params* p, const FaParams& kp, const fa_tensor& dout, void* workspace, void* stream) {
+  // must match the shared-memory map of fa_bwd_f32.cuh (fa_bf32::SMEM_BYTES)
+  const int smem = 9 * 16384 + 9 * 8192 + 3 * 2 * 64 * 4 + 21 * 8 + 8 + 16 + 16 + 2 * 512 * 4 + 256 + 1024;
+  Kernel* k = nullptr;
+  if (int rc = get_kernel(m, kernel_key(kIdBwdF32, {}), "fa_bwd_f32.cuh", [] { return std::string(); }, "fa_bwd_f32_kernel", smem, &k)) return rc;
+  const int sq_pad = (p->Sq + 127) / 128 * 128;
+  char* w[4];
+  w[0] = (char*)workspace;
+  w[1] = w[0] + split3_bytes(p->B, p->Hq, p->Sq);
+  w[2] = w[1] + split3_bytes(p->B, p->Hkv, p->Skv);
+  w[3] = w[2] + split3_bytes(p->B, p->Hkv, p->Skv);
+  float* nlse2 = (float*)(w[3] + split3_bytes(p->B, p->Hq, p->Sq));
+  float* ndelta = (float*)((char*)nlse2 + rows_pad_bytes(p));
+  FaBwdF32ParamsHost tp;
+  tp.p = kp;
+  tp.nlse2 = nlse2;
+  tp.ndelta = ndelta;
+  tp.work_counter = (int*)((char*)ndelta + rows_pad_bytes(p));
+  FaSplitJobs jobs;
+  memset(&jobs, 0, sizeof jobs);
+  jobs.counter = tp.work_counter;
+  jobs.job[0] = split_job(p->q, w[0], p->B, p->Hq, p->Sq);
+  jobs.job[0].clear = kp.dq;
+  jobs.job[1] = split_job(p->k, w[1], p->B, p->Hkv, p->Skv);
+  jobs.job[2] = split_job(p->v, w[2], p->B, p->Hkv, p->Skv);
+  FaSplitJob& jd = jobs.job[3] = split_job(dout, w[3], p->B, p->Hq, p->Sq);
+  jd.S_rows = sq_pad; jd.rows = (long long)p->B * p->Hq * sq_pad;
+  jd.o = kp.o; jd.lse = p->lse; jd.nlse2 = nlse2; jd.ndelta = ndelta;
+  if (int rc = launch_split3(jobs, 4, stream)) return rc;
+  if (int rc = make_map(&tp.tq, FA_BF16, split3_tensor(w[0], p->Hq, p->Sq), 192, p->Sq, p->Hq, p->B, 64)) return rc;
+  if (int rc = make_map(&tp.tk, FA_BF16, split3_tensor(w[1], p->Hkv, p->Skv), 192, p->Skv, p->Hkv, p->B)) return rc;
+  if (int rc = make_map(&tp.tv, FA_BF16, split3_tensor(w[2], p->Hkv, p->Skv), 192, p->Skv, p->Hkv, p->B)) return rc;
+  if (int rc = make_map(&tp.tdo, FA_BF16, split3_tensor(w[3], p->Hq, p->Sq), 192, p->Sq, p->Hq, p->B, 64)) return rc;
+  const long long n_items = (long long)p->Hkv * p->B * ((p->Skv + 127) / 128);
+  return launch(k, dim3((unsigned)std::min<long long>(n_items, device_sm_count())), dim3(512), &tp, stream);
+}
+
 // kv2: two K / V buffers with a three-stage Q / dO ring instead of one with four (head dim 64)
 int get_bwd_tc_kernel(fa_module* m, int dtype, int D, int flags, bool kv2, Kernel** k) {
   // must match the shared-memory map of fa_bwd_tc.cuh (fa_btc::SMEM_BYTES)
@@ -1235,12 +1418,22 @@ int fa_module_prepare(fa_module* m, int kind, int dtype, int D, int Dv, int Sq_h
   }
 }
 
-int fa_fwd(fa_module* m, const fa_attn_params* p, void* stream) {
+int fa_fwd(fa_module* m, const fa_attn_params* p, void* stream) { return fa_fwd_ws(m, p, nullptr, 0, stream); }
+
+size_t fa_fwd_workspace_bytes(const fa_attn_params* p) {
+  if (!p || p->B <= 0 || p->Hq <= 0 || p->Hkv <= 0 || p->Sq <= 0 || p->Skv <= 0 || !tc_fwd_f32_eligible(p)) return 0;
+  return split3_bytes(p->B, p->Hq, p->Sq) + 2 * split3_bytes(p->B, p->Hkv, p->Skv);
+}
+
+int fa_fwd_ws(fa_module* m, const fa_attn_params* p, void* workspace, size_t workspace_bytes, void* stream) {
   if (int rc = check_common(m, p)) return rc;
+  if (workspace && ((uintptr_t)workspace & 15)) return fail(FA_EINVAL, "workspace must be 16-byte aligned");
   prof_reset();
   FaParams kp;
   fill_params(m, p, kp);
   if (tc_fwd_eligible(p)) return launch_fwd_tc(m, p, kp, stream);
+  const size_t ws_need = fa_fwd_workspace_bytes(p);
+  if (ws_need && workspace && workspace_bytes >= ws_need) return launch_fwd_f32_tc(m, p, kp, workspace, stream);
   FwdCfg c;
   if (int rc = pick_fwd(p->dtype, p->D, p->Dv, p->Sq, &kp.t, c)) return rc;
   Kernel* k = nullptr;
@@ -1251,6 +1444,7 @@ int fa_fwd(fa_module* m, const fa_attn_params* p, void* stream) {
 
 size_t fa_bwd_workspace_bytes(const fa_attn_params* p) {
   if (!p || p->B <= 0 || p->Hq <= 0 || p->Sq <= 0) return 0;
+  if (p->Hkv > 0 && p->Hq % p->Hkv == 0 && tc_bwd_f32_eligible(p)) return bwd_f32_workspace(p);
   if (p->Hkv > 0 && p->Hq % p->Hkv == 0 && tc_bwd_eligible(p)) return 2 * rows_pad_bytes(p) + dq_acc_bytes(p) + 256;
   return delta_bytes(p);
 }
@@ -1276,6 +1470,7 @@ int fa_bwd(fa_module* m, const fa_attn_params* p, const fa_tensor* dout, const f
   fill_params(m, p, kp);
   kp.dout = cvt(*dout); kp.dq = cvt(*dq); kp.dk = cvt(*dk); kp.dv = cvt(*dv);
   kp.delta = (float*)workspace;
+  if (tc_bwd_f32_eligible(p)) return launch_bwd_f32_tc(m, p, kp, *dout, workspace, stream);
   const bool use_tc = tc_bwd_eligible(p);
   BwdCfg c{};
   Kernel *kdq = nullptr, *kdkdv = nullptr, *ktc = nullptr;

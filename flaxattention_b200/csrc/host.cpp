@@ -154,8 +154,11 @@ std::pair<at::Tensor, at::Tensor> forward(const Call& c, const at::Tensor& q, co
     rc = buffers.rc != FA_OK ? buffers.rc
                              : fa_decode(c.mods->module, &p, splits, bytes > 0 ? ws.mutable_data_ptr() : nullptr, bytes, stream);
   } else {
+    const size_t bytes = fa_fwd_workspace_bytes(&p);
+    at::Tensor ws;
+    if (bytes > 0) ws = empty({(int64_t)bytes}, at::kByte, q.device());
     BuffersLock buffers(*c.mods);
-    rc = buffers.rc != FA_OK ? buffers.rc : fa_fwd(c.mods->module, &p, stream);
+    rc = buffers.rc != FA_OK ? buffers.rc : fa_fwd_ws(c.mods->module, &p, bytes > 0 ? ws.mutable_data_ptr() : nullptr, bytes, stream);
   }
   if (rc != FA_OK) raise(rc);
   return {std::move(out), std::move(lse)};

@@ -6,15 +6,27 @@
 //   with D = 64, over the score columns with D = 128).
 // Same math and BlockMask walk as fa_fwd.cuh (see there for the reference citations); this
 // kernel covers fp16 / bf16, D = Dv in {64, 128}, block sizes that are multiples of 128 and a
-// positive scale.
+// positive scale; and fp32, D = Dv = 64, in the form described next.
+//
+// fp32 (FA_DTYPE 2).  The tensor cores multiply no fp32 operands without dropping mantissa bits, so
+// every operand is written as a sum of three bf16 values, hi + mid + lo, which holds all 24 mantissa bits
+// (each part is the rounding of what the parts before it leave; bf16 has the exponent range of fp32):
+// q, k and v by a small kernel in front of this one, whose rows are [hi | mid | lo] (192 values), and the
+// probabilities by the softmax threads.  A product is then the six bf16 products hi.hi, hi.mid,
+// mid.hi, mid.mid, hi.lo, lo.hi, accumulated in fp32, smallest first; the three left out are below
+// 2^-25 of hi.hi, half a unit in the last place of an fp32 product.  The tensor core adds into its fp32
+// accumulator without rounding to nearest, so nothing is accumulated there for long: the P.V product
+// of every kv step starts from zero and the softmax threads add it to the output row they keep in
+// registers (with O accumulated in TMEM over all steps the error grew to five times that of the FMA
+// kernel at 1024 keys).  The softmax keeps the operations and their order of fa_fwd.cuh.
 //
 // One CTA owns two 128-row query tiles of one (batch, head) and streams 128-row K/V tiles
 // past both.  Warp roles (12 warps = 3 warpgroups):
 //   warps 0-3  softmax warpgroup of query tile 0      warps 4-7  of query tile 1
 //   warp 8     TMA producer (one lane)
-//   warps 9-10 MMA issuers (one lane each); warp 9 also allocates / frees TMEM.  With D = 64 warp 9
-//              issues the S products and warp 10 the PV products; with D = 128 warp 9 issues both
-//              products of query tile 0 and warp 10 those of tile 1; warp 11 is idle
+//   warps 9-10 MMA issuers; warp 9 also allocates / frees TMEM.  With D = 64 warp 9 issues the S products and
+//              warp 10 the PV products (one lane each); where P lies over S (D = 128, fp32) warp 9 issues
+//              all products of both query tiles in turn; warp 11 is idle
 // Registers are moved from the third warpgroup to the two softmax warpgroups (setmaxnreg),
 // which hold a whole 128-column score row per thread.
 // The S columns of a tile are released as soon as its scores are in registers, so with D = 64
@@ -26,7 +38,7 @@
 // Every mbarrier wait is bounded; on expiry the CTA raises FA_STATUS_WAIT_TIMEOUT in the
 // status word, all roles leave their loops, TMEM is freed and the kernel returns.
 //
-// Compile-time parameters (macros): FA_DTYPE (0 fp16, 1 bf16), FA_D (64 or 128), FA_TC_DECODE
+// Compile-time parameters (macros): FA_DTYPE (0 fp16, 1 bf16, 2 fp32), FA_D (64 or 128), FA_TC_DECODE
 // (split-KV variant, see below).
 #pragma once
 #include "fa_sm100.cuh"
@@ -39,10 +51,12 @@ struct FaTcParams {
 
 namespace fa_tc {
 
-constexpr int DT = FA_DTYPE;
+constexpr bool F32 = FA_DTYPE == FA_DT_F32;
+constexpr int DT = F32 ? FA_DT_BF16 : FA_DTYPE;  // type of the tensor-core operands
 constexpr int D = FA_D;
 constexpr int BM = 128, BN = 128;
-constexpr int ATOMS = D / 64;            // 64-element (128-byte) column groups per row
+constexpr int NPART = F32 ? 3 : 1;       // bf16 parts of an operand value
+constexpr int ATOMS = NPART * D / 64;    // 64-element (128-byte) column groups per row (fp32: one per part)
 constexpr int ATOM_BYTES = 128 * 128;    // 128 rows x 128 bytes
 // Split-KV decode variant (FA_TC_DECODE, D = 64, at most 64 query rows): the CTA owns a contiguous
 // share of the kv tiles the BlockMask lists and the two softmax warpgroups take alternate kv tiles
@@ -60,7 +74,9 @@ constexpr int ATOM_BYTES = 128 * 128;    // 128 rows x 128 bytes
 #define FA_TC_DECODE 0
 #endif
 constexpr bool DECODE = FA_TC_DECODE != 0;
-constexpr int NSTAGE = DECODE ? 5 : (D == 64 ? 3 : 2);
+// (fp32: the parts of two query tiles, a K and a V tile fill shared memory; K of the next step is loaded
+// during the softmax and the PV products of this one, V during the next S products)
+constexpr int NSTAGE = DECODE ? 5 : (F32 ? 1 : (D == 64 ? 3 : 2));
 constexpr int Q_BYTES = 2 * ATOMS * ATOM_BYTES;
 constexpr int KV_STAGE = ATOMS * ATOM_BYTES;
 constexpr int MAXT = 256;                // kv tiles per row of the block grid (Skv <= 32768)
@@ -75,11 +91,14 @@ constexpr int OFF_CLS = OFF_MODE + MAXT * 2;        // uchar cls[2][MAXT]
 constexpr int OFF_WCNT = OFF_CLS + 2 * MAXT;        // int wcount[MAXT / 32]: listed tiles per warp of the schedule build
 constexpr int SMEM_BYTES = OFF_WCNT + (MAXT / 32) * 4 + 1024;  // + slack for the 1024-byte alignment
 constexpr int TMEM_COLS = 512;
-constexpr int COL_S = 0, COL_O = 256;
+// fp32: scores of tile i in columns 192 i .. + 127.  The softmax writes the parts of P over the scores it
+// has just read, 16 columns (32 keys) at a time: hi and mid of keys 32 c .. + 31 go to columns 32 c .. + 15
+// and 32 c + 16 .. + 31, lo to 128 + 16 c .. + 15.  O of tile i and step in 384 + 64 i.
+constexpr int COL_S = 0, COL_O = F32 ? 384 : 256, S_STRIDE = F32 ? 192 : 128;
 // With D = 64 there is TMEM left for P next to S (columns 384..511): S of the next kv step can
 // then be produced while the softmax of the current step is still writing P.  With D = 128 the
 // 512 columns are taken by S and O, and P overwrites the S columns it was computed from.
-constexpr bool SEP_P = D == 64;
+constexpr bool SEP_P = D == 64 && !F32;
 constexpr int COL_P = 384;
 // One pair of exponentials in FA_TC_POLY_EVERY goes to the FMA pipe (a cubic, see fa_ex2_poly2).
 // Measured (B8 H8 S2048 D64): every fourth pair takes the forward without a score_mod from 0.118 to
@@ -100,7 +119,10 @@ constexpr float RESCALE_THRESHOLD = 8.0f;  // log2 units
 
 static_assert(D == 64 || D == 128, "head dim 64 or 128");
 static_assert(!DECODE || D == 64, "the decode variant is written for head dim 64");
-static_assert(DT == FA_DT_F16 || DT == FA_DT_BF16, "16-bit inputs");
+static_assert(!F32 || (D == 64 && !DECODE), "fp32: head dim 64, forward");
+// the pairs of parts whose products are kept, smallest first
+constexpr int NPROD = F32 ? 6 : 1;
+__device__ constexpr int PROD_A[6] = {F32 ? 1 : 0, 0, 2, 0, 1, 0}, PROD_B[6] = {F32 ? 1 : 0, 2, 0, 1, 0, 0};
 
 __device__ __forceinline__ fa_u32 bar_addr(fa_u32 sbase, int i) { return sbase + OFF_BAR + i * 8; }
 constexpr int BAR_Q = 0;
@@ -403,6 +425,113 @@ __device__ __forceinline__ bool softmax_step(SoftmaxCtx& c, const int j, const i
   return true;
 }
 
+#if FA_DTYPE == FA_DT_F32
+// One kv step of a tile with fp32 inputs.  The scores are gone through twice, 32 columns at a time, so that the
+// output row (acc, 64 values) fits into the registers beside them: first for the row maximum, then
+// for the exponentials and their parts.  A score_mod that adds something is evaluated in the first
+// pass only and its results are written back; one that only multiplies is cheap enough for both.
+#if FA_HAS_SCORE_MOD && !defined(FA_SCORE_MUL_ONLY)
+constexpr bool WRITE_BACK = true;
+#else
+constexpr bool WRITE_BACK = false;
+#endif
+// the scores of 32 columns in log2 units (raw without a score_mod: the exponent's FMA applies the scale then)
+template <int C0>
+__device__ __forceinline__ void mod32_f32(float (&v)[32], const SoftmaxCtx& c, int n0) {
+#if FA_HAS_SCORE_MOD && defined(FA_SCORE_MUL_ONLY)
+#pragma unroll
+  for (int e = 0; e < 32; ++e) v[e] *= fa_score_mul(0.f, c.gb, c.gh, c.qi, n0 | (C0 + e)) * c.sc2;
+#elif FA_HAS_SCORE_MOD
+  // (an additive bias is applied before the change to log2 units, as in fa_fwd.cuh: folding the factor into it
+  //  would round a large bias at another place)
+#pragma unroll
+  for (int e = 0; e < 32; ++e) v[e] = fa_score_mod(v[e] * c.p.scale, c.gb, c.gh, c.qi, n0 | (C0 + e)) * FA_LOG2E;
+#endif
+}
+__device__ __forceinline__ bool softmax_step_f32(SoftmaxCtx& c, float (&acc)[D], const int j, const int mode, const bool masked) {
+  const FaParams& p = c.p;
+  const fa_u32 t_s = c.t_s;
+  const int n0 = (int)c.sched_tile[j] * BN;
+  if (!fa_mbar_wait_warp(bar_addr(c.sb, BAR_S + c.i), c.cnt & 1u, c.abort_flag)) return false;
+  fa_tc_fence_after();
+  float a[32], b[32];
+  constexpr bool mod = FA_HAS_SCORE_MOD;
+  fa_u32 keep[4] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu};
+  fa_tmem_ld32(t_s, a);
+  if (masked) mask_bits(keep, FA_HAS_MASK_MOD && mode == 1, n0, c.qi, c.gb, c.gh, p.Skv, c.rowbits);
+  float mx0 = FA_NEG_INF, mx1 = FA_NEG_INF;
+#define FA_P1(V, N, C)                                                                                  \
+  fa_tmem_wait_ld();                                                                                    \
+  if ((C) + 32 < BN) fa_tmem_ld32(t_s + (C) + 32, N);                                                   \
+  mod32_f32<C>(V, c, n0);                                                                               \
+  if (masked) mask_apply(V, keep[(C) >> 5]);                                                            \
+  if (WRITE_BACK || masked) fa_tmem_st32(t_s + (C), V);                                                 \
+  _Pragma("unroll") for (int e = 0; e < 32; e += 4) {                                                   \
+    mx0 = fa_max3(mx0, V[e], V[e + 1]);                                                                 \
+    mx1 = fa_max3(mx1, V[e + 2], V[e + 3]);                                                             \
+  }
+  FA_P1(a, b, 0) FA_P1(b, a, 32) FA_P1(a, b, 64) FA_P1(b, a, 96)
+#undef FA_P1
+  if (c.cnt > 0) fa_tmem_ld32(c.t_o, a);
+  float mx = fmaxf(mx0, mx1);
+  if (!mod) mx *= c.sc2;
+  const float m_new = fmaxf(c.m_ref, mx);
+  float corr = 1.f;
+  if (c.m_ref == FA_NEG_INF) {
+    c.m_ref = m_new;
+  } else if (m_new - c.m_ref > RESCALE_THRESHOLD) {
+    corr = fa_ex2(c.m_ref - m_new);
+    c.m_ref = m_new;
+    c.l *= corr;
+  }
+  if (c.cnt > 0) {
+    // S of this step was issued behind P.V of the last one, so that product is complete too
+    fa_tmem_wait_ld();
+    fa_tmem_ld32(c.t_o + 32, b);
+#pragma unroll
+    for (int e = 0; e < 32; ++e) acc[e] = (acc[e] + a[e]) * corr;
+    fa_tmem_wait_ld();
+#pragma unroll
+    for (int e = 0; e < 32; ++e) acc[32 + e] = (acc[32 + e] + b[e]) * corr;
+  }
+  if (WRITE_BACK || masked) fa_tmem_wait_st();
+  fa_tmem_ld32(t_s, a);
+  const float m_use = (c.m_ref == FA_NEG_INF) ? 0.f : c.m_ref;
+  const fa_u64 negm = fa_f2(-m_use, -m_use);
+  const float cm = mod ? 1.f : c.sc2;
+  const fa_u64 cmul = fa_f2(cm, cm);
+  fa_u64 sum_a = fa_f2(0.f, 0.f), sum_b = fa_f2(0.f, 0.f);
+#define FA_P2(V, N, C)                                                                                  \
+  fa_tmem_wait_ld();                                                                                    \
+  if ((C) + 32 < BN) fa_tmem_ld32(t_s + (C) + 32, N);                                                   \
+  if (mod && !WRITE_BACK && !masked) mod32_f32<C>(V, c, n0);                                            \
+  _Pragma("unroll") for (int hf = 0; hf < 2; ++hf) {                                                    \
+    fa_u32 hi[8], mid[8], lo[8];                                                                        \
+    _Pragma("unroll") for (int e = 0; e < 8; ++e) {                                                     \
+      float x0, x1;                                                                                     \
+      fa_f2_unpack(fa_fma2(fa_f2(V[16 * hf + 2 * e], V[16 * hf + 2 * e + 1]), cmul, negm), x0, x1);     \
+      const fa_u64 pf = fa_f2(fa_ex2(x0), fa_ex2(x1));                                                  \
+      if (e & 1) sum_b = fa_add2(sum_b, pf);                                                            \
+      else sum_a = fa_add2(sum_a, pf);                                                                  \
+      fa_split3(pf, hi[e], mid[e], lo[e]);                                                              \
+    }                                                                                                   \
+    fa_tmem_st8(t_s + (C) + 8 * hf, hi);                                                                \
+    fa_tmem_st8(t_s + (C) + 16 + 8 * hf, mid);                                                          \
+    fa_tmem_st8(t_s + 128 + (C) / 2 + 8 * hf, lo);                                                      \
+  }
+  FA_P2(a, b, 0) FA_P2(b, a, 32) FA_P2(a, b, 64) FA_P2(b, a, 96)
+#undef FA_P2
+  float s0, s1;
+  fa_f2_unpack(fa_add2(sum_a, sum_b), s0, s1);
+  c.l += s0 + s1;
+  fa_tmem_wait_st();
+  fa_tc_fence_before();
+  fa_mbar_arrive(bar_addr(c.sb, BAR_P + c.i));
+  ++c.cnt;
+  return true;
+}
+#endif
+
 }  // namespace fa_tc
 
 extern "C" __global__ void __launch_bounds__(fa_tc::NT, 1) fa_fwd_tc_kernel(const __grid_constant__ FaTcParams P) {
@@ -470,10 +599,9 @@ extern "C" __global__ void __launch_bounds__(fa_tc::NT, 1) fa_fwd_tc_kernel(cons
     fa_mbar_init(bar_addr(sb, BAR_Q), 1);
     for (int s = 0; s < NSTAGE; ++s) {
       fa_mbar_init(bar_addr(sb, BAR_KFULL + s), 1);
-      // with D = 128 each of the two issuing warps releases a stage once
-      fa_mbar_init(bar_addr(sb, BAR_KEMPTY + s), SEP_P ? 1 : 2);
+      fa_mbar_init(bar_addr(sb, BAR_KEMPTY + s), 1);
       fa_mbar_init(bar_addr(sb, BAR_VFULL + s), 1);
-      fa_mbar_init(bar_addr(sb, BAR_VEMPTY + s), SEP_P ? 1 : 2);
+      fa_mbar_init(bar_addr(sb, BAR_VEMPTY + s), 1);
     }
     for (int i = 0; i < 2; ++i) {
       fa_mbar_init(bar_addr(sb, BAR_S + i), 1);
@@ -680,87 +808,93 @@ extern "C" __global__ void __launch_bounds__(fa_tc::NT, 1) fa_fwd_tc_kernel(cons
         }
       }
     }
-  } else if (!SEP_P && (warp == WARP_MMA || warp == WARP_MMA_B)) {
-    // ============ two MMA issuers (D = 128): warp A issues both products of query tile 0, warp B of tile 1 ====
+  } else if (!SEP_P && warp == WARP_MMA) {
+    // ============ one MMA issuer for both query tiles (D = 128, fp32) ======================
     // P overwrites the S columns here, so the products of one tile form a chain  PV_i(j), S_i(j+1),
-    // PV_i(j+1) ...; the chains of the two tiles only share the K / V stages.  Issuing the sixteen
-    // instructions of a step's two products takes one thread about as long as the tensor core needs
-    // to run them, so each chain gets its own issuing warp; a K / V stage is released by one
-    // arrival from each.  The whole warp runs the loop and one elected lane issues: in uniform
-    // control flow the operands of tcgen05.mma sit in uniform registers, which makes the
-    // instructions cheaper to issue than from a single-lane branch (attention-sink forward,
-    // B4 H16 S8192: 0.80 ms with one issuing lane, 0.70 with one per tile, 0.65 with elected lanes).
+    // PV_i(j+1) ...  One warp issues the two chains in turn, PV_0(j) S_0(j+1) PV_1(j) S_1(j+1), so that the
+    // products of a tile run as one block while the other tile is in its softmax.  (With an issuing warp
+    // per tile the tensor core took instructions of both in turn, both tiles got their scores at the
+    // same time, and the products of one never ran under the softmax of the other: clock stamps of a
+    // step showed both waiting for the tensor core and both in the softmax together.)  The whole
+    // warp runs the loop and one elected lane issues: in uniform control flow the operands of tcgen05.mma
+    // sit in uniform registers, which makes the instructions cheaper to issue than from a single-lane branch.
     {
       const bool leader = fa_elect_one();
       const fa_u32 tmem_u = __shfl_sync(0xffffffffu, tmem, 0);
       const int nsteps_u = __shfl_sync(0xffffffffu, nsteps, 0);
-      const int i = warp == WARP_MMA ? 0 : 1;
       constexpr fa_u32 IDESC_S = fa_idesc(DT, BM, BN, 0, 0);
       constexpr fa_u32 IDESC_O = fa_idesc(DT, BM, D, 0, 1);
       bool ok = nsteps_u == 0 || fa_mbar_wait_all(bar_addr(sb, BAR_Q), 0, abort_flag);
-      fa_u32 cnt = 0;  // PV products of this tile issued so far
+      fa_u32 cnt[2] = {0, 0};  // PV products of each tile issued so far
       // Descriptors: constant high word; the low word (start address and MN-chunk distance in
       // 16-byte units) is stepped with one add per k-step.
       constexpr fa_u32 HI = fa_desc_hi_sw128();
-      // S_i = Q_i K^T for step j into TMEM columns COL_S + 128 i
-      auto issue_s = [&](int j) {
+      // S_i = Q_i K^T for step j
+      auto issue_s = [&](int j, int i) {
         const int s = j % NSTAGE;
         const fa_u32 loQ = fa_desc_lo(sb + i * ATOMS * ATOM_BYTES, 16);
         const fa_u32 loK = fa_desc_lo(sb + OFF_K + s * KV_STAGE, 16);
 #pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) {
-          const fa_u32 koff = ((kk / 4) * ATOM_BYTES + (kk % 4) * 32) >> 4;
-          if (leader) fa_mma_ss(tmem_u + COL_S + i * BN, fa_desc_make(loQ + koff, HI), fa_desc_make(loK + koff, HI), IDESC_S, kk > 0);
+        for (int pr = 0; pr < NPROD; ++pr) {
+#pragma unroll
+          for (int kk = 0; kk < D / 16; ++kk) {
+            const fa_u32 koff = ((kk / 4) * ATOM_BYTES + (kk % 4) * 32) >> 4;
+            const fa_u32 pa = (PROD_A[pr] * ATOM_BYTES) >> 4, pb = (PROD_B[pr] * ATOM_BYTES) >> 4;
+            if (leader)
+              fa_mma_ss(tmem_u + COL_S + i * S_STRIDE, fa_desc_make(loQ + pa + koff, HI), fa_desc_make(loK + pb + koff, HI), IDESC_S, pr > 0 || kk > 0);
+          }
         }
         if (leader) fa_mma_commit(bar_addr(sb, BAR_S + i));
       };
-      // O_i += P_i V for step j (P_i: 16-bit, in the first 64 columns of S_i)
-      auto issue_pv = [&](int j, bool first) {
+      // O_i += P_i V for step j (P_i: 16-bit, from the first column of S_i on; fp32: three parts, and O_i = P_i V)
+      auto issue_pv = [&](int j, int i, bool first) {
         const int s = j % NSTAGE;
         const fa_u32 loV = fa_desc_lo(sb + OFF_V + s * KV_STAGE, ATOM_BYTES);
-        const fa_u32 acc = !first;
+        const fa_u32 acc = !F32 && !first;
 #pragma unroll
-        for (int kk = 0; kk < BN / 16; ++kk)
-          if (leader) fa_mma_ts(tmem_u + COL_O + i * D, tmem_u + COL_S + i * BN + kk * 8, fa_desc_make(loV + kk * 128, HI), IDESC_O, acc | (kk > 0));
+        for (int pr = 0; pr < NPROD; ++pr) {
+#pragma unroll
+          for (int kk = 0; kk < BN / 16; ++kk)
+            if (leader)
+              fa_mma_ts(tmem_u + COL_O + i * D, tmem_u + COL_S + i * S_STRIDE + (!F32 ? kk * 8 : (PROD_A[pr] == 2 ? 128 + kk * 8 : (kk >> 1) * 32 + PROD_A[pr] * 16 + (kk & 1) * 8)),
+                        fa_desc_make(loV + ((PROD_B[pr] * ATOM_BYTES) >> 4) + kk * 128, HI), IDESC_O, acc | (pr > 0 || kk > 0));
+        }
         if (leader) fa_mma_commit(bar_addr(sb, BAR_O + i));
       };
       if (ok && nsteps_u > 0) {
         ok = fa_mbar_wait_all(bar_addr(sb, BAR_KFULL + 0), 0, abort_flag);
         if (ok) {
           fa_tc_fence_after();
-          if (sched_mode[i]) issue_s(0);
-          if (leader) fa_mma_commit(bar_addr(sb, BAR_KEMPTY + 0));  // (a commit with nothing outstanding arrives at once)
+          for (int i = 0; i < 2; ++i)
+            if (sched_mode[i]) issue_s(0, i);
+          if (leader) fa_mma_commit(bar_addr(sb, BAR_KEMPTY + 0));
         }
       }
       for (int j = 0; j < nsteps_u && ok; ++j) {
-        const int s = j % NSTAGE;
-        const fa_u32 ph = (fa_u32)((j / NSTAGE) & 1);
+        const int s = j % NSTAGE, s1 = (j + 1) % NSTAGE;
         const bool more = j + 1 < nsteps_u;
-        const int s1 = (j + 1) % NSTAGE;
-        const fa_u32 ph1 = (fa_u32)(((j + 1) / NSTAGE) & 1);
-        // Every step waits for its stage to be full before it releases it, with or without a
-        // product of this tile: the load of a stage follows both releases of its previous use, so a
-        // warp whose tile skips several steps cannot release a stage twice before the other warp
-        // has released it once.
-        ok = fa_mbar_wait_all(bar_addr(sb, BAR_VFULL + s), ph, abort_flag);
-        if (!ok) break;
-        if (sched_mode[2 * j + i]) {
-          ok = fa_mbar_wait_all(bar_addr(sb, BAR_P + i), cnt & 1u, abort_flag);
-          if (!ok) break;
-          fa_tc_fence_after();
-          issue_pv(j, cnt == 0);
-          ++cnt;
-        }
-        if (leader) fa_mma_commit(bar_addr(sb, BAR_VEMPTY + s));
-        if (more) {
-          ok = fa_mbar_wait_all(bar_addr(sb, BAR_KFULL + s1), ph1, abort_flag);
-          if (!ok) break;
-          // S of the next step overwrites the columns P was read from: it follows the PV product
-          if (sched_mode[2 * (j + 1) + i]) {
+        ok = fa_mbar_wait_all(bar_addr(sb, BAR_VFULL + s), (fa_u32)((j / NSTAGE) & 1), abort_flag);
+#pragma unroll 1
+        for (int i = 0; i < 2 && ok; ++i) {
+          if (sched_mode[2 * j + i]) {
+            ok = fa_mbar_wait_all(bar_addr(sb, BAR_P + i), cnt[i] & 1u, abort_flag);
+            if (!ok) break;
             fa_tc_fence_after();
-            issue_s(j + 1);
+            issue_pv(j, i, cnt[i] == 0);
+            ++cnt[i];
           }
-          if (leader) fa_mma_commit(bar_addr(sb, BAR_KEMPTY + s1));
+          if (i == 1 && leader) fa_mma_commit(bar_addr(sb, BAR_VEMPTY + s));
+          if (more) {
+            // (every step waits for its stage to be full before it releases it, with or without a product)
+            ok = fa_mbar_wait_all(bar_addr(sb, BAR_KFULL + s1), (fa_u32)(((j + 1) / NSTAGE) & 1), abort_flag);
+            if (!ok) break;
+            // S of the next step overwrites the columns P was read from: it follows the PV product
+            if (sched_mode[2 * (j + 1) + i]) {
+              fa_tc_fence_after();
+              issue_s(j + 1, i);
+            }
+            if (i == 1 && leader) fa_mma_commit(bar_addr(sb, BAR_KEMPTY + s1));
+          }
         }
       }
     }
@@ -775,7 +909,7 @@ extern "C" __global__ void __launch_bounds__(fa_tc::NT, 1) fa_fwd_tc_kernel(cons
     // decode variant: warps whose 32 rows are all padding (fewer than 33 queries) only keep the barrier protocol going
     const bool warp_active = !DECODE || (lane_base & 63) < p.Sq;
     fa_u32 idle_cnt = 0;
-    const fa_u32 t_s = tmem + ((fa_u32)lane_base << 16) + COL_S + i * BN;
+    const fa_u32 t_s = tmem + ((fa_u32)lane_base << 16) + COL_S + i * S_STRIDE;
     const fa_u32 t_o = tmem + ((fa_u32)lane_base << 16) + COL_O + i * D;
     const fa_u32 t_p = SEP_P ? tmem + ((fa_u32)lane_base << 16) + COL_P + i * 64 : t_s;
     bool ok = true;
@@ -793,6 +927,11 @@ extern "C" __global__ void __launch_bounds__(fa_tc::NT, 1) fa_fwd_tc_kernel(cons
       fa_tmem_st16(t_p + (1 - half) * 32 + 16, z);
       fa_tmem_wait_st();
     }
+#if FA_DTYPE == FA_DT_F32
+    float acc[D];
+#pragma unroll
+    for (int e = 0; e < D; ++e) acc[e] = 0.f;
+#endif
     for (int j = 0; j < nsteps && ok; ++j) {
       const int mode = sched_mode[2 * j + i];
       if (mode == 0) continue;
@@ -812,7 +951,11 @@ extern "C" __global__ void __launch_bounds__(fa_tc::NT, 1) fa_fwd_tc_kernel(cons
         continue;
       }
       const bool masked = (FA_HAS_MASK_MOD && mode == 1) || (int)sched_tile[DECODE ? 2 * j + i : j] * BN + BN > p.Skv;
-      if (D == 64) ok = softmax_step<2>(c, j, mode, masked);
+#if FA_DTYPE == FA_DT_F32
+      ok = softmax_step_f32(c, acc, j, mode, masked);
+      continue;
+#endif
+      if (SEP_P) ok = softmax_step<2>(c, j, mode, masked);
       else ok = masked ? softmax_step<1>(c, j, mode, true) : softmax_step<0>(c, j, mode, false);
     }
     const float m_ref = c.m_ref, l = c.l;
@@ -910,6 +1053,17 @@ extern "C" __global__ void __launch_bounds__(fa_tc::NT, 1) fa_fwd_tc_kernel(cons
 #pragma unroll
             for (int e = 0; e < 32; ++e) o[e] = 0.f;
           }
+#if FA_DTYPE == FA_DT_F32
+          {
+            // 32 fp32 columns are one 128-byte row of a 128 x 128-byte block
+            unsigned char* strow = sm + (i * ATOMS + c) * ATOM_BYTES + r * 128;
+#pragma unroll
+            for (int e = 0; e < 32; e += 4)
+              *(float4*)(strow + (((e >> 2) ^ (r & 7)) * 16)) = make_float4((acc[32 * c + e] + o[e]) * inv, (acc[32 * c + e + 1] + o[e + 1]) * inv,
+                                                                                 (acc[32 * c + e + 2] + o[e + 2]) * inv, (acc[32 * c + e + 3] + o[e + 3]) * inv);
+            continue;
+          }
+#endif
           unsigned char* strow = sm + (i * ATOMS + (c >> 1)) * ATOM_BYTES + r * 128;
 #pragma unroll
           for (int e = 0; e < 32; e += 8) {
@@ -922,12 +1076,14 @@ extern "C" __global__ void __launch_bounds__(fa_tc::NT, 1) fa_fwd_tc_kernel(cons
           }
         }
         if (p.lse != nullptr && qi < p.Sq)
-          p.lse[((long long)b * p.Hq + h) * p.Sq + qi] = (l > 0.f && m_ref != FA_NEG_INF) ? (m_ref + fa_lg2(l)) * FA_LN2 : FA_NEG_INF;
+          p.lse[((long long)b * p.Hq + h) * p.Sq + qi] = (l > 0.f && m_ref != FA_NEG_INF) ? (m_ref + (F32 ? log2f(l) : fa_lg2(l))) * FA_LN2 : FA_NEG_INF;
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       asm volatile("bar.sync %0, 128;" ::"r"(3 + i) : "memory");
       if ((warp & 3) == 0 && lane == 0 && *abort_flag == 0 && m0 + i * BM < p.Sq) {
-        for (int a = 0; a < ATOMS; ++a) fa_tma_store_4d(&P.to, sb + (i * ATOMS + a) * ATOM_BYTES, a * 64, m0 + i * BM, h, b);
+        // (a 128-byte column group of the output: 64 values of a 16-bit type, 32 of fp32)
+        for (int a = 0; a < (F32 ? D / 32 : D / 64); ++a)
+          fa_tma_store_4d(&P.to, sb + (i * ATOMS + a) * ATOM_BYTES, a * (F32 ? 32 : 64), m0 + i * BM, h, b);
         asm volatile("cp.async.bulk.commit_group;" ::: "memory");
         asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // the tile must outlive the reads of the store
       }

@@ -188,6 +188,11 @@ __device__ __forceinline__ void fa_tmem_st16(fa_u32 taddr, const fa_u32 (&v)[16]
         "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
       : "memory");
 }
+__device__ __forceinline__ void fa_tmem_st8(fa_u32 taddr, const fa_u32 (&v)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+               ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+               : "memory");
+}
 
 // ---- tcgen05.mma -----------------------------------------------------------------------
 // Shared-memory matrix descriptor, 128-byte swizzle, 16-bit elements.  Both canonical forms
@@ -266,6 +271,20 @@ __device__ __forceinline__ fa_u64 fa_fma2(fa_u64 a, fa_u64 b, fa_u64 c) {
   fa_u64 r;
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
   return r;
+}
+// A pair of fp32 values as three pairs of bf16 values whose sum is exact: hi is the value rounded to bf16,
+// mid the remainder rounded, lo what is left of it (at most 8 bits, so the last rounding is exact).
+__device__ __forceinline__ void fa_split3(fa_u64 x, fa_u32& hi, fa_u32& mid, fa_u32& lo) {
+  float x0, x1;
+  fa_f2_unpack(x, x0, x1);
+  hi = fa_pack2<FA_DT_BF16>(x0, x1);
+  const fa_u64 minus1 = fa_f2(-1.f, -1.f);
+  fa_u64 r = fa_fma2(fa_f2(__uint_as_float(hi << 16), __uint_as_float(hi & 0xffff0000u)), minus1, x);
+  fa_f2_unpack(r, x0, x1);
+  mid = fa_pack2<FA_DT_BF16>(x0, x1);
+  r = fa_fma2(fa_f2(__uint_as_float(mid << 16), __uint_as_float(mid & 0xffff0000u)), minus1, r);
+  fa_f2_unpack(r, x0, x1);
+  lo = fa_pack2<FA_DT_BF16>(x0, x1);
 }
 // 2^x for a pair of values on the FMA pipe instead of the SFU: x = n + r with n = round(x) taken
 // from the mantissa of x + 1.5 * 2^23, a cubic for 2^r on [-0.5, 0.5] (Chebyshev interpolant,

@@ -158,6 +158,12 @@ int fa_profile_enable(int on);
 int fa_profile_read(int max_kernels, float* ms, const char** names);
 
 int fa_fwd(fa_module* m, const fa_attn_params* p, void* stream);
+/* The same with a workspace (device, 16-byte aligned): fp32 problems of head dim 64 then run on the tensor
+ * cores, on operands split into three bf16 parts that hold all their mantissa bits.
+ * fa_fwd_workspace_bytes is 0 where no workspace is of use; without one, or with a smaller one, the
+ * kernel that needs none runs. */
+size_t fa_fwd_workspace_bytes(const fa_attn_params* p);
+int fa_fwd_ws(fa_module* m, const fa_attn_params* p, void* workspace, size_t workspace_bytes, void* stream);
 
 size_t fa_bwd_workspace_bytes(const fa_attn_params* p);
 int fa_bwd(fa_module* m, const fa_attn_params* p, const fa_tensor* dout, const fa_tensor* dq,
