@@ -1250,6 +1250,7 @@ struct FaBwdTcParamsHost {
   const float* nlse2;
   const float* ndelta;
   int* work_counter;
+  int chunk_heads;
 };
 
 // SMs of the current device (148 on a B200; asked once per device)
@@ -1350,26 +1351,39 @@ int launch_bwd_f32_tc(fa_module* m, const fa_attn_params* p, const FaParams& kp,
   return launch(k, dim3((unsigned)std::min<long long>(n_items, device_sm_count())), dim3(512), &tp, stream);
 }
 
-// kv2: two K / V buffers with a three-stage Q / dO ring instead of one with four (head dim 64)
+// kv2: two K / V buffers and one of dS^T instead of one and two (head dim 64)
 int get_bwd_tc_kernel(fa_module* m, int dtype, int D, int flags, bool kv2, Kernel** k) {
   // must match the shared-memory map of fa_bwd_tc.cuh (fa_btc::SMEM_BYTES)
-  const int bq = D == 64 ? 128 : 64, kvbuf = (D == 64 && kv2) ? 2 : 1, nstage = (D == 64 && kvbuf == 1) ? 4 : 3;
+  const int bq = D == 64 ? 128 : 64, kvbuf = (D == 64 && kv2) ? 2 : 1, nstage = 3, nds = kvbuf == 1 ? 2 : 1;
   const int kv_bytes = (D / 64) * 16384, q_bytes = 16384, ds_bytes = (bq / 64) * 16384;
-  const int smem = 2 * kvbuf * kv_bytes + 2 * nstage * q_bytes + ds_bytes + 128 * 32 * 4 + nstage * 2 * bq * 4 +
-                   (2 + 3 * nstage + 15) * 8 + 16 + 16 + 2 * bwd_tc_max_pairs(D) * 4 + 256 + 1024;
+  const int smem = 2 * kvbuf * kv_bytes + 2 * nstage * q_bytes + nds * ds_bytes + 128 * 32 * 4 + nstage * 2 * bq * 4 +
+                   (2 + 3 * nstage + 15) * 8 + 16 + 32 + 2 * bwd_tc_max_pairs(D) * 4 + 256 + 1024;
   const int rnd = round_flag(dtype, flags);
   return get_kernel(m, kernel_key(kIdBwdTc, {{dtype, 2}, {D, 9}, {rnd, 1}, {kvbuf, 2}}), "fa_bwd_tc.cuh",
                     [&] { return defs({{"FA_DTYPE", dtype}, {"FA_D", D}, {"FA_ROUND_SCORES", rnd}, {"FA_BWD_KV2", kvbuf == 2 ? 1 : 0}}); },
                     "fa_bwd_tc_kernel", smem, k);
 }
 
-// With a BlockMask the items are short or uneven and the variant with two K / V buffers wins: under a
-// causal mask 97 against 103 us at S=1024 (B16 H8), 150 / 160 at 2048, 197 / 209 at 3072, 263 / 283
-// at 4096, 289 / 303 at 6144 (48 q tiles, 24 pairs per item on average).  Without one every item
-// has all the q tiles and the four-stage ring wins (S=2048, 16 pairs per item: 206 against 215 us).
+// With a BlockMask the items are short or uneven and the variant with two K / V buffers wins: under a causal
+// mask (us, against two dS^T buffers) 35 / 38 at S=512 (B8 H8), 174 / 190 at 2048, 233 / 233 at 8192 (B1 H8).
+// Without one every item has all the q tiles and two dS^T buffers win.
 bool bwd_tc_kv2(const fa_attn_params* p) {
   if (p->D != 64 || !p->tables.kv_num_blocks) return false;
   return (long long)((p->Sq + 127) / 128) * (p->Hq / p->Hkv) <= 64;
+}
+
+// (batch, kv head) pairs whose items the backward works through together (item_of in fa_bwd_tc.cuh): as many as
+// keep their dQ accumulators, Q and dO in L2 (126 MB), if that leaves an item for every SM, or three where items
+// are uneven (tables: the heavy items of a late chunk end up alone otherwise, causal B2 H16/4 S3001 D128
+// 388 -> 435 us).  Measured with all heads together and with chunks (us): attention sink B4 H16 S8192 D128
+// 1061 -> 1023 with 96 MB; dense B4 H8 S4096 D128 745 -> 738 with 96 MB, 714 with 24 MB.  Where the items are
+// uneven small chunks cost balance: causal + ALiBi B8 H8 S2048 D64 174 -> 189 with 24 MB.
+int bwd_tc_chunk_heads(const fa_attn_params* p) {
+  const long long heads = (long long)p->B * p->Hkv, n_kvt = (p->Skv + 127) / 128;
+  const long long per_head = (long long)(p->Hq / p->Hkv) * ((p->Sq + 127) / 128 * 128) * p->D * (4 + 2 + 2);
+  const bool uneven = p->tables.kv_num_blocks != nullptr;
+  const long long ch = (uneven ? 96ll << 20 : 24ll << 20) / per_head;
+  return (int)(ch >= heads || ch * n_kvt < (uneven ? 3 : 1) * device_sm_count() ? heads : ch);
 }
 
 // scan = false: the kernel that takes any block size
@@ -1505,6 +1519,7 @@ int fa_bwd(fa_module* m, const fa_attn_params* p, const fa_tensor* dout, const f
     tp.nlse2 = nlse2;
     tp.ndelta = ndelta;
     tp.work_counter = work_counter;
+    tp.chunk_heads = bwd_tc_chunk_heads(p);
     const int bq = p->D == 64 ? 128 : 64;  // q rows of a (kv tile, q tile) pair of the kernel
     if (int rc = make_map(&tp.tq, p->dtype, p->q, p->D, p->Sq, p->Hq, p->B, bq)) return rc;
     if (int rc = make_map(&tp.tk, p->dtype, p->k, p->D, p->Skv, p->Hkv, p->B)) return rc;

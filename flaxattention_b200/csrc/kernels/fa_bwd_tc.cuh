@@ -36,7 +36,7 @@
 // Every mbarrier wait is bounded (see fa_sm100.cuh).
 //
 // Compile-time parameters (macros): FA_DTYPE (0 fp16, 1 bf16), FA_D (64 or 128; Dv = D), FA_BWD_KV2
-// (two K / V buffers and a three-stage ring, head dim 64 only).
+// (two K / V buffers and one of dS^T instead of one and two, head dim 64 only).
 #pragma once
 #include "fa_sm100.cuh"
 
@@ -52,6 +52,7 @@ struct FaBwdTcParams {
   const float* nlse2;           // [B, Hq, ceil(Sq/128)*128]: -lse * log2(e); -inf for rows without mass / beyond Sq
   const float* ndelta;          // same shape: -rowsum(O * dO); 0 beyond Sq
   int* work_counter;            // zero at launch: items beyond the first of every CTA are handed out through it
+  int chunk_heads;              // (batch, kv head) pairs whose items are numbered together (see item_of)
 };
 
 namespace fa_btc {
@@ -68,17 +69,23 @@ constexpr int KV_BYTES = DATOMS * ATOM_BYTES;        // one K or V tile
 constexpr int Q_ATOM_BYTES = BQ * 128;               // BQ rows x 128 bytes
 constexpr int Q_BYTES = DATOMS * Q_ATOM_BYTES;       // one Q or dO tile (16 KB in both configurations)
 constexpr int DS_ATOMS = BQ / 64;                    // dS^T: [128 kv][BQ q] as atoms of 64 q columns
-// K / V buffers and Q / dO ring depth.  With D = 64 shared memory holds either one K / V buffer and a
-// ring of four stages, or two K / V buffers and a ring of three (FA_BWD_KV2): with two, K and V of the
-// next item are loaded while the current one is computed and nothing waits at the change of items,
-// which pays when items are short (causal S=2048, 8.5 pairs per item on average: 150 against 158 us)
-// and costs when they are long (dense S=2048, 16 pairs: 215 against 206 us - the fourth stage matters
-// more than the bubble).  The host picks.  With D = 128 there is one buffer and three stages.
+// K / V and dS^T buffers.  The pace of a pair is set by the hand-over of P^T and dS^T: with one dS^T buffer the
+// compute warps may store pair n + 1 only when products 3-5 of pair n are complete.  With two they wait for
+// product 3 of pair n (issued first) and, by the order of issue, products 4-5 of pair n - 1, which is
+// long past; the Q / dO ring gives up its fourth stage for it at D = 64.  Measured against one buffer and four
+// (three at D = 128) stages, backward alone, us: dense B8 H8 S2048 D64 231 -> 225, B4 H16/4 S2048 D64
+// 251 -> 239, dense B4 H8 S4096 D128 769 -> 745, causal B2 H16/4 S3001 D128 403 -> 388.
+// With D = 64 shared memory holds, instead of the second dS^T buffer, a second K / V buffer (FA_BWD_KV2): K and V of
+// the next item are loaded while the current one is computed and nothing waits at the change of items, which pays
+// when items are short (causal S=2048, 8.5 pairs per item on average: 174 against 190 us) and costs when they
+// are long.  The host picks.
 #ifndef FA_BWD_KV2
 #define FA_BWD_KV2 0
 #endif
 constexpr int KVBUF = (D == 64 && FA_BWD_KV2) ? 2 : 1;
-constexpr int NSTAGE = (D == 64 && KVBUF == 1) ? 4 : 3;
+constexpr int NSTAGE = 3;
+constexpr int NDS = KVBUF == 1 ? 2 : 1;                // dS^T buffers
+constexpr int DS_BYTES = DS_ATOMS * ATOM_BYTES;
 constexpr int MAXPL = D == 64 ? 1024 : 2048;  // (head, q tile) pairs of one item (two such lists fit in shared memory)
 constexpr int MAXC = 256;                // 128-row q tiles per head (Sq <= 32768)
 constexpr int NT = 512;
@@ -99,14 +106,14 @@ constexpr int OFF_V = OFF_K + KVBUF * KV_BYTES;
 constexpr int OFF_Q = OFF_V + KVBUF * KV_BYTES;             // NSTAGE tiles
 constexpr int OFF_DO = OFF_Q + NSTAGE * Q_BYTES;            // NSTAGE tiles
 constexpr int OFF_DS = OFF_DO + NSTAGE * Q_BYTES;           // dS^T
-constexpr int OFF_DQ = OFF_DS + DS_ATOMS * ATOM_BYTES;      // fp32 staging 128 x 32 (half of the dQ tile at a time)
+constexpr int OFF_DQ = OFF_DS + NDS * DS_BYTES;      // fp32 staging 128 x 32 (half of the dQ tile at a time)
 constexpr int DQ_HALF_BYTES = 128 * 32 * 4;
 constexpr int OFF_ROW = OFF_DQ + DQ_HALF_BYTES;             // NSTAGE x (nlse2[BQ], ndelta[BQ]) floats
 constexpr int OFF_BAR = OFF_ROW + NSTAGE * 2 * BQ * 4;
 constexpr int NBARS = 2 + 3 * NSTAGE + 15;
 constexpr int OFF_MISC = OFF_BAR + NBARS * 8;               // tmem base, abort, -, drain flag
-constexpr int OFF_ITEM = OFF_MISC + 16;                     // int item[2][2]: item number, pairs (-1: no more work)
-constexpr int OFF_PAIR = OFF_ITEM + 16;                     // int pair[2][MAXPL]: q tile | mode << 16 | g << 20
+constexpr int OFF_ITEM = OFF_MISC + 16;                     // int item[2][4]: kv head (KV2: item number), batch, kv tile, pairs (-1: no more work)
+constexpr int OFF_PAIR = OFF_ITEM + 32;                     // int pair[2][MAXPL]: q tile | mode << 16 | g << 20
 constexpr int OFF_CLS = OFF_PAIR + 2 * MAXPL * 4;           // uchar cls[MAXC] (scratch of the list builder)
 constexpr int SMEM_BYTES = OFF_CLS + MAXC + 1024;
 static_assert(SMEM_BYTES <= 227 * 1024, "shared memory");
@@ -124,7 +131,7 @@ constexpr int BAR_QFULL = 2, BAR_QEMPTY = 2 + NSTAGE, BAR_DOEMPTY = 2 + 2 * NSTA
 constexpr int BAR_SFULL = 2 + 3 * NSTAGE;   // S^T and dP^T of a pair are in TMEM
 constexpr int BAR_SFREE = BAR_SFULL + 1;    // compute warps hold them in registers (256 arrivals)
 constexpr int BAR_PREADY = BAR_SFULL + 2;   // P^T in TMEM and dS^T in smem (256 arrivals)
-constexpr int BAR_PFREE = BAR_SFULL + 3;    // products 3-5 of the pair are complete
+constexpr int BAR_PFREE = BAR_SFULL + 3;    // P^T and the next dS^T buffer may be written (see NDS)
 constexpr int BAR_DQFULL = BAR_SFULL + 4;   // dQ of the pair is in TMEM
 constexpr int BAR_DQFREE = BAR_SFULL + 5;   // drain warps hold it in registers (128 arrivals)
 constexpr int BAR_FINAL = BAR_SFULL + 6;    // [2] products 3-5 of the last pair of the item in buffer kb are complete
@@ -263,6 +270,42 @@ __device__ __forceinline__ void chunk(const float (&s)[W], const float (&dp)[W],
 }
 
 
+// Item number -> (kv head, batch, kv tile).  The first kv tiles of all heads come first (under a causal mask and
+// with attention sinks they are the heaviest), then chunk by chunk of `ch` heads, in a chunk heads fastest and the
+// kv tile slowest.  The CTAs work through the items in this order, so that at any time the dQ accumulator, Q and dO
+// of about one chunk of heads are in use: the host sizes it to stay in L2.  (Not with two K / V buffers: there the
+// items are short and the time to their first loads counts, causal B1 H8 S8192 D64 228 -> 242 us.)
+struct Item {
+  int hk, b, kt;
+};
+__device__ __forceinline__ Item item_of(int idx, int Hkv, int B, int n_kvt, int ch) {
+  if (KVBUF == 2) return {idx % Hkv, (idx / Hkv) % B, idx / (Hkv * B)};
+  const unsigned heads = Hkv * B, i = idx;
+  unsigned head = i, kt = 0;
+  if ((unsigned)ch >= heads) {  // one chunk
+    kt = i / heads;
+    head = i - kt * heads;
+  } else if (i >= heads) {
+    const unsigned r = i - heads, per = ch * (n_kvt - 1), c = r / per, rr = r - c * per;
+    const unsigned n = min((unsigned)ch, heads - c * ch);
+    kt = rr / n;
+    head = c * ch + rr - kt * n;
+    ++kt;
+  }
+  const unsigned b = head / Hkv;
+  return {(int)(head - b * Hkv), (int)b, (int)kt};
+}
+
+// What the producer has published of an item.  (Two K / V buffers: its number, taken apart here; reading the three
+// parts made the compute warps spill and the kernel 4 % slower, causal B1 H8 S8192 D64 230 -> 241 us.)
+__device__ __forceinline__ Item read_item(const volatile int* item, int Hkv, int B) {
+  if (KVBUF == 2) {
+    const int idx = item[0];
+    return {idx % Hkv, (idx / Hkv) % B, idx / (Hkv * B)};
+  }
+  return {item[0], item[1], item[2]};
+}
+
 // The (query head, q tile) pairs of one item, written to `pl` by one warp: per head of the group,
 // the 128-row q tiles the BlockMask lists for the item's kv tile (class 1: apply mask_mod, 2: full)
 // in ascending order, each as 128 / BQ pairs.  Without tables every tile is listed.  Returns the
@@ -276,7 +319,10 @@ __device__ __forceinline__ int build_pair_list(const FaParams& p, int hk, int b,
     if (!tables) {
       const int nq = (p.Sq + BQ - 1) / BQ;
       const int mode = FA_HAS_MASK_MOD ? 1 : 2;
-      for (int e = lane; e < nq && w + e < MAXPL; e += 32) pl[w + e] = e | (mode << 16) | (g << 20);
+      // the items of a head start at different q tiles, so that the CTAs on one head do not add to the same
+      // dQ tile at the same time
+      const int rot = kt % nq;
+      for (int e = lane; e < nq && w + e < MAXPL; e += 32) pl[w + e] = (e + rot < nq ? e + rot : e + rot - nq) | (mode << 16) | (g << 20);
       w += nq;
       continue;
     }
@@ -354,10 +400,10 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
 
   volatile int* misc = (volatile int*)(sm + OFF_MISC);  // [0] tmem base, [1] abort, [2] unused, [3] drain warps leave
   int* pairs = (int*)(sm + OFF_PAIR);                   // two lists of MAXPL pairs
-  volatile int* item = (volatile int*)(sm + OFF_ITEM);  // per list: item number, pairs
+  volatile int* item = (volatile int*)(sm + OFF_ITEM);  // per list: kv head, batch, kv tile, pairs
 
-  // An item is the 128-row kv tile of one (batch, kv head); items are numbered with the head
-  // fastest and the kv tile slowest (under a causal mask the heaviest come first).  The kernel is
+  // An item is the 128-row kv tile of one (batch, kv head); items are numbered so that the
+  // heaviest come early and heads stay together (item_of).  The kernel is
   // persistent: CTA c starts with item c and takes further items from a counter in global memory,
   // so TMEM, the barriers and the descriptors are set up once per CTA, the loads of an item run
   // under the tail of the one before, and the CTAs stay level whatever the mask does to the work
@@ -423,12 +469,15 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
       if (itc >= 2) ok = fa_mbar_wait_warp(bar_addr(sb, BAR_LISTFREE + lb), (fa_u32)(((itc >> 1) - 1) & 1), abort_flag);
       if (!ok) break;
       int* pl = pairs + lb * MAXPL;
-      const int hk = idx % p.Hkv, b = (idx / p.Hkv) % p.B, kt = idx / (p.Hkv * p.B);
+      const Item it = item_of(min(idx, n_items - 1), p.Hkv, p.B, n_kvt, P.chunk_heads);
+      const int hk = it.hk, b = it.b, kt = it.kt;
       int np = -1;
       if (idx < n_items) np = build_pair_list(p, hk, b, kt, G, n_ctiles, sm + OFF_CLS, pl, lane);
       if (lane == 0) {
-        item[2 * lb] = idx;
-        item[2 * lb + 1] = np;
+        item[4 * lb] = KVBUF == 2 ? idx : hk;
+        item[4 * lb + 1] = b;
+        item[4 * lb + 2] = kt;
+        item[4 * lb + 3] = np;
       }
       __syncwarp();
       if (lane == 0) fa_mbar_arrive(bar_addr(sb, BAR_LISTFULL + lb));
@@ -476,7 +525,8 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
         // K and V of the next item are asked into L2 now; their loads can only start when this
         // item is complete, and then they find the tiles close by
         if (KVBUF == 1 && ok && next < n_items) {
-          const int hk2 = next % p.Hkv, b2 = (next / p.Hkv) % p.B, n2 = (next / (p.Hkv * p.B)) * BT;
+          const Item i2 = item_of(next, p.Hkv, p.B, n_kvt, P.chunk_heads);
+          const int hk2 = i2.hk, b2 = i2.b, n2 = i2.kt * BT;
           for (int a = 0; a < DATOMS; ++a) {
             tma_prefetch_l2_4d(&P.tk, a * 64, n2, hk2, b2);
             tma_prefetch_l2_4d(&P.tv, a * 64, n2, hk2, b2);
@@ -504,7 +554,7 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
       const int lb = itc & 1;
       ok = fa_mbar_wait_all(bar_addr(sb, BAR_LISTFULL + lb), (fa_u32)((itc >> 1) & 1), abort_flag);
       if (!ok) break;
-      const int np = __shfl_sync(0xffffffffu, item[2 * lb + 1], 0);
+      const int np = __shfl_sync(0xffffffffu, item[4 * lb + 3], 0);
       if (leader) fa_mbar_arrive(bar_addr(sb, BAR_LISTFREE + lb));  // (the issuers need the count only)
       if (np < 0) break;
       if (np == 0) continue;
@@ -541,14 +591,13 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
     const bool leader = fa_elect_one();
     constexpr fa_u32 IDESC_TN = fa_idesc(DT, 128, D, 0, 1);    // A K-major (TMEM or smem), B MN-major, N = D
     constexpr fa_u32 HI = fa_desc_hi_sw128();
-    const fa_u32 loDS_k = fa_desc_lo(sb + OFF_DS, 16);
     bool ok = true;
     int gn = 0, kvc = 0;
     for (int itc = 0; ok; ++itc) {
       const int lb = itc & 1;
       ok = fa_mbar_wait_all(bar_addr(sb, BAR_LISTFULL + lb), (fa_u32)((itc >> 1) & 1), abort_flag);
       if (!ok) break;
-      const int np = __shfl_sync(0xffffffffu, item[2 * lb + 1], 0);
+      const int np = __shfl_sync(0xffffffffu, item[4 * lb + 3], 0);
       if (leader) fa_mbar_arrive(bar_addr(sb, BAR_LISTFREE + lb));
       if (np < 0) break;
       if (np == 0) continue;
@@ -564,12 +613,17 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
         // k-step is 16 q rows = 2048 bytes
         const fa_u32 loQ_mn = fa_desc_lo(sb + OFF_Q + s * Q_BYTES, Q_ATOM_BYTES);
         const fa_u32 loDO_mn = fa_desc_lo(sb + OFF_DO + s * Q_BYTES, Q_ATOM_BYTES);
+        const fa_u32 loDS_k = fa_desc_lo(sb + OFF_DS + (gn % NDS) * DS_BYTES, 16);
         const fa_u32 acc = n > 0;  // the first pair of an item starts its dK and dV
         // 3. dV += P^T dO      (K = BQ q values; A from TMEM)
 #pragma unroll
         for (int kk = 0; kk < BQ / 16; ++kk)
           if (leader) fa_mma_ts(tmem_u + COL_DV, tmem_u + COL_P + kk * 8, fa_desc_make(loDO_mn + kk * 128, HI), IDESC_TN, acc | (kk > 0));
-        if (leader) fa_mma_commit(bar_addr(sb, BAR_DOEMPTY + s));  // second arrival: the dO tile is free
+        if (leader) {
+          fa_mma_commit(bar_addr(sb, BAR_DOEMPTY + s));  // second arrival: the dO tile is free
+          // two dS^T buffers: P^T is free, and so is the other buffer (product 4 of the previous pair came before)
+          if (NDS == 2) fa_mma_commit(bar_addr(sb, BAR_PFREE));
+        }
         // 4. dK += dS^T Q     (A = dS^T K-major: k-step kk is 32 bytes into atom kk / 4)
 #pragma unroll
         for (int kk = 0; kk < BQ / 16; ++kk)
@@ -578,7 +632,7 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
                       fa_desc_make(loQ_mn + kk * 128, HI), IDESC_TN, acc | (kk > 0));
         if (leader) {
           fa_mma_commit(bar_addr(sb, BAR_QEMPTY + s));   // second arrival: the Q tile and row scalars are free
-          fa_mma_commit(bar_addr(sb, BAR_PFREE));        // one of the two arrivals that free P^T and dS^T
+          if (NDS == 1) fa_mma_commit(bar_addr(sb, BAR_PFREE));  // one of the two arrivals that free P^T and dS^T
           if (n + 1 == np) fa_mma_commit(bar_addr(sb, BAR_FINAL + kvc % KVBUF));
         }
       }
@@ -591,14 +645,13 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
     const bool leader = fa_elect_one();
     constexpr fa_u32 IDESC_NN = fa_idesc(DT, 128, 64, 1, 1);    // A, B MN-major, M = 128, N = 64
     constexpr fa_u32 HI = fa_desc_hi_sw128();
-    const fa_u32 loDS_mn = fa_desc_lo(sb + OFF_DS, ATOM_BYTES);
     bool ok = true;
     int gn = 0, kvc = 0;
     for (int itc = 0; ok; ++itc) {
       const int lb = itc & 1;
       ok = fa_mbar_wait_all(bar_addr(sb, BAR_LISTFULL + lb), (fa_u32)((itc >> 1) & 1), abort_flag);
       if (!ok) break;
-      const int np = __shfl_sync(0xffffffffu, item[2 * lb + 1], 0);
+      const int np = __shfl_sync(0xffffffffu, item[4 * lb + 3], 0);
       if (leader) fa_mbar_arrive(bar_addr(sb, BAR_LISTFREE + lb));
       if (np < 0) break;
       if (np == 0) continue;
@@ -607,10 +660,16 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
       ok = fa_mbar_wait_all(bar_addr(sb, BAR_KV + kb), (fa_u32)((kvc / KVBUF) & 1), abort_flag);
       for (int n = 0; n < np && ok; ++n, ++gn) {
         ok = fa_mbar_wait_all(bar_addr(sb, BAR_PREADY), (fa_u32)(gn & 1), abort_flag);
+        if (NDS == 2 && ok && leader) {
+          // product 5 of the previous pair is the last reader of the other dS^T buffer
+          if (gn > 0) fa_mma_commit(bar_addr(sb, BAR_PFREE));
+          else fa_mbar_arrive(bar_addr(sb, BAR_PFREE));
+        }
         // the drain warps must have emptied the dQ columns of the previous pair
         if (ok && gn > 0) ok = fa_mbar_wait_all(bar_addr(sb, BAR_DQFREE), (fa_u32)((gn - 1) & 1), abort_flag);
         if (!ok) break;
         fa_tc_fence_after();
+        const fa_u32 loDS_mn = fa_desc_lo(sb + OFF_DS + (gn % NDS) * DS_BYTES, ATOM_BYTES);
         // 5. K = 128 kv rows, a k-step is 16 rows = 2048 bytes of either operand.
         //    D = 64:  dQ = dS K       A = dS^T read MN-major (M = 128 q: two 64-column atoms), B = K (N = 64 d)
         //    D = 128: dQ^T = K^T dS^T A = K read MN-major (M = 128 d: two atoms), B = dS^T (N = 64 q)
@@ -623,7 +682,7 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
               fa_mma_ss(tmem_u + COL_DQ, fa_desc_make(loK_mn + kk * 128, HI), fa_desc_make(loDS_mn + kk * 128, HI), IDESC_NN, kk > 0);
           }
         if (leader) {
-          fa_mma_commit(bar_addr(sb, BAR_PFREE));
+          if (NDS == 1) fa_mma_commit(bar_addr(sb, BAR_PFREE));
           fa_mma_commit(bar_addr(sb, BAR_DQFULL));
           if (n + 1 == np) fa_mma_commit(bar_addr(sb, BAR_FINAL + kb));  // (this product is the last reader of K)
         }
@@ -644,10 +703,11 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
       const int lb = itc & 1;
       ok = fa_mbar_wait_warp(bar_addr(sb, BAR_LISTFULL + lb), (fa_u32)((itc >> 1) & 1), abort_flag);
       if (!ok) break;
-      const int idx = item[2 * lb], np = item[2 * lb + 1];
+      const int np = item[4 * lb + 3];
       if (np < 0) break;
       const int* pl = pairs + lb * MAXPL;
-      const int hk = idx % p.Hkv, b = (idx / p.Hkv) % p.B, n0 = (idx / (p.Hkv * p.B)) * BT;
+      const Item it = read_item(item + 4 * lb, p.Hkv, p.B);
+      const int hk = it.hk, b = it.b, n0 = it.kt * BT;
       const int gb = b + p.b_off;
       const int kv = n0 + r;
       const bool row_ok = kv < p.Skv;
@@ -707,7 +767,8 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
         // wait that follows, onto the critical path between two groups of products
 #pragma unroll
         for (int e = 0; e < CW / 2; ++e) asm volatile("" : "+r"(pp[e]), "+r"(ds[e]));
-        // products 3-5 of the previous pair must be done with P^T and dS^T
+        // product 3 of the previous pair must be done with P^T, and products 4-5 of the last pair that used this
+        // dS^T buffer with that
         if (gn > 0) {
           ok = fa_mbar_wait_warp(bar_addr(sb, BAR_PFREE), (fa_u32)((gn - 1) & 1), abort_flag);
           if (!ok) break;
@@ -722,7 +783,7 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
 #pragma unroll
           for (int c = 0; c < CW / 8; ++c) {
             const int col = half * CW + 8 * c;
-            unsigned char* dsrow = sm + OFF_DS + (col >> 6) * ATOM_BYTES + r * 128;
+            unsigned char* dsrow = sm + OFF_DS + (gn % NDS) * DS_BYTES + (col >> 6) * ATOM_BYTES + r * 128;
             uint4 w;
             w.x = ds[4 * c]; w.y = ds[4 * c + 1]; w.z = ds[4 * c + 2]; w.w = ds[4 * c + 3];
             *(uint4*)(dsrow + ((((col & 63) >> 3) ^ (r & 7)) * 16)) = w;
@@ -760,10 +821,11 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
         ok = false;
         break;
       }
-      const int idx = item[2 * lb], np = item[2 * lb + 1];
+      const int np = item[4 * lb + 3];
       if (np < 0) break;  // (the same in all four warps)
       const int* pl = pairs + lb * MAXPL;
-      const int hk = idx % p.Hkv, b = (idx / p.Hkv) % p.B, n0 = (idx / (p.Hkv * p.B)) * BT;
+      const Item it = read_item(item + 4 * lb, p.Hkv, p.B);
+      const int hk = it.hk, b = it.b, n0 = it.kt * BT;
       for (int n = 0; n < np && ok; ++n, ++gn) {
         const int pr = pl[n];
         const int qt = pr & 0xffff, h = hk * G + (pr >> 20);
