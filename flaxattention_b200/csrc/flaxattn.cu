@@ -452,7 +452,7 @@ int pick_bwd(int dtype, int D, int Dv, const FaTables* t, BwdCfg& c) {
 }
 
 struct DecCfg {
-  int BM, BN, stages, smem;
+  int BM, BN, smem;
 };
 int pick_decode(int dtype, int D, int Dv, int Sq, const FaTables* t, DecCfg& c) {
   if (dtype == FA_F32) return fail(FA_EUNSUPPORTED, "the decode kernel takes fp16 / bf16 inputs");
@@ -464,17 +464,15 @@ int pick_decode(int dtype, int D, int Dv, int Sq, const FaTables* t, DecCfg& c) 
     if (BN / CG < 16) continue;
     if (D > 64 && BN > 64) continue;
     if (t && t->kv_num && !divides_or_single(BN, t->KVB, t->nKV)) continue;
-    // Two stages first: the kernel is bound by the latency its few resident warps can hide, and
+    // Two buffers of K and of V: the kernel is bound by the latency its few resident warps can hide, and
     // the smaller ring lets a third CTA share the SM (B32 H8 Skv16384 D64: 0.187 ms with two
     // stages against 0.218 ms with three at one query row, 0.224 against 0.269 at sixteen).
-    for (int stages : {2, 3}) {
-      const int pipe = stages * (BN * pitch(D, 2) + BN * pitch(Dv, 2));
-      const int mrg = CG * BM * (Dv + 4) * 4;
-      const int smem = BM * pitch(D, 2) + (pipe > mrg ? pipe : mrg);
-      if (smem > kMaxSmem) continue;
-      c = {BM, BN, stages, smem};
-      return FA_OK;
-    }
+    const int pipe = 2 * (BN * pitch(D, 2) + BN * pitch(Dv, 2));
+    const int mrg = CG * BM * (Dv + 4) * 4;
+    const int smem = BM * pitch(D, 2) + (pipe > mrg ? pipe : mrg);
+    if (smem > kMaxSmem) continue;
+    c = {BM, BN, smem};
+    return FA_OK;
   }
   return fail(FA_EUNSUPPORTED, "no decode tile configuration fits this head dim / BlockMask block size");
 }
@@ -1058,10 +1056,10 @@ int get_bwd_kernel(fa_module* m, int dtype, int D, int Dv, int flags, const BwdC
 }
 int get_decode_kernel(fa_module* m, int dtype, int D, int Dv, int flags, const DecCfg& c, bool pack, Kernel** k) {
   const int rnd = round_flag(dtype, flags);
-  return get_kernel(m, kernel_key(kIdDecode, {{dtype, 2}, {D, 9}, {Dv, 9}, {c.BM, 9}, {c.BN, 9}, {c.stages, 4}, {rnd, 1}, {pack ? 1 : 0, 1}}),
+  return get_kernel(m, kernel_key(kIdDecode, {{dtype, 2}, {D, 9}, {Dv, 9}, {c.BM, 9}, {c.BN, 9}, {rnd, 1}, {pack ? 1 : 0, 1}}),
                     "fa_decode.cuh",
                     [&] { return defs({{"FA_DTYPE", dtype}, {"FA_D", D}, {"FA_DV", Dv}, {"FA_BM", c.BM}, {"FA_BN", c.BN},
-                                       {"FA_STAGES", c.stages}, {"FA_ROUND_SCORES", rnd}, {"FA_PACK_HEADS", pack ? 1 : 0}}); },
+                                       {"FA_ROUND_SCORES", rnd}, {"FA_PACK_HEADS", pack ? 1 : 0}}); },
                     "fa_decode_kernel", c.smem, k);
 }
 // Grouped-query decode: the G query heads of a kv head share one CTA (their G * Sq rows form one

@@ -96,6 +96,9 @@ __device__ __forceinline__ void fa_round_acc(float (&acc)[N][4]) {
 __device__ __forceinline__ void fa_cp_async16(fa_u32 dst, const void* src, int src_bytes) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
 }
+__device__ __forceinline__ void fa_cp_async16_full(fa_u32 dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
 __device__ __forceinline__ void fa_cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void fa_cp_wait() {
@@ -142,6 +145,24 @@ __device__ __forceinline__ void fa_load_tile(fa_u32 smem, const char* gbase, lon
   constexpr int CPR = COLS * ESIZE / 16;  // 16-byte chunks per row
   constexpr int PITCH = FaTile<COLS, ESIZE>::PITCH;
   const int total = rows * CPR;
+  // A whole tile: the threads keep their column and step through the rows, one address addition per copy.  (With
+  // the row, its validity and its address worked out for every copy, these were the greater part of the 680
+  // instructions per warp and tile of the decode kernel, whose issue they bound: decode B32 H8 Skv16384 D64
+  // 206 -> 196 us together with the two-way prefetch there, B16 H32/8 Skv8191 D128 130 -> 125.)
+  if (NT % CPR == 0 && valid_rows >= rows && total % NT == 0) {
+    constexpr int STEP = NT % CPR == 0 ? NT / CPR : 1;
+    const int r = tid / CPR, c = tid % CPR;
+    const char* src = gbase + (long long)r * row_stride_bytes + c * 16;
+    const fa_u32 dst = smem + r * PITCH + c * 16;
+    const long long step = STEP * row_stride_bytes;
+    const int n = total / NT;
+#pragma unroll
+    for (int k = 0; k < n; ++k) {
+      fa_cp_async16_full(dst + k * STEP * PITCH, src);
+      src += step;
+    }
+    return;
+  }
   for (int i = tid; i < total; i += NT) {
     const int r = i / CPR, c = i - r * CPR;
     const bool ok = r < valid_rows;
@@ -206,7 +227,12 @@ struct FaWalk {
   // slot -> first token of the tile (or -1 when the tile lies beyond S); full = skip mask_mod
   template <int T>
   __device__ __forceinline__ int tile_start(int slot, bool& full) const {
-    int bi = slot / tpb;
+    if (idx[0] == nullptr) {  // no tables
+      full = false;
+      const long long n0 = (long long)slot * T;
+      return n0 < S ? (int)n0 : -1;
+    }
+    int bi = tpb == 1 ? slot : slot / tpb;
     const int ti = slot - bi * tpb;
     int which = 0;
     if (bi >= num[0]) { bi -= num[0]; which = 1; }

@@ -18,7 +18,7 @@
 // which is why the host packs only when the tables do not depend on the head.
 //
 // Compile-time parameters (macros): FA_DTYPE (fp16 / bf16), FA_D, FA_DV, FA_BM (16, 32, 64),
-// FA_BN (kv tile), FA_STAGES, FA_PACK_HEADS.
+// FA_BN (kv tile), FA_PACK_HEADS.
 #pragma once
 #include "fa_common.cuh"
 
@@ -35,7 +35,7 @@ constexpr int D = FA_D;
 constexpr int DV = FA_DV;
 constexpr int BM = FA_BM;
 constexpr int BN = FA_BN;
-constexpr int STAGES = FA_STAGES;
+constexpr int STAGES = 2;
 constexpr int NWARPS = 4;
 constexpr int NT = NWARPS * 32;
 constexpr int RG = BM / 16;
@@ -112,15 +112,21 @@ extern "C" __global__ void __launch_bounds__(fa_dec::NT) fa_decode_kernel(const 
   // just those rows itself and the warps run as independent pipelines, with no block-wide
   // barrier inside the kv loop.  With several row groups the tile is loaded cooperatively.
   constexpr bool PRIVATE = RG == 1;
-  auto load_kv = [&](int stage, int n0) {
+  auto load_k = [&](int stage, int n0) {
     if (PRIVATE) {
       const int first = n0 + cg * WN, vr = p.Skv - first;
       const long long koff = vr > 0 ? (long long)first * p.k.ss * ES : 0;
-      const long long voff = vr > 0 ? (long long)first * p.v.ss * ES : 0;
       fa_load_tile<D, ES, 32>(sK + stage * K_BYTES + cg * WN * PQ, kg + koff, p.k.ss * ES, WN, vr, lane);
-      fa_load_tile<DV, ES, 32>(sV + stage * V_BYTES + cg * WN * PV, vg + voff, p.v.ss * ES, WN, vr, lane);
     } else {
       fa_load_tile<D, ES, NT>(sK + stage * K_BYTES, kg + (long long)n0 * p.k.ss * ES, p.k.ss * ES, BN, p.Skv - n0, tid);
+    }
+  };
+  auto load_v = [&](int stage, int n0) {
+    if (PRIVATE) {
+      const int first = n0 + cg * WN, vr = p.Skv - first;
+      const long long voff = vr > 0 ? (long long)first * p.v.ss * ES : 0;
+      fa_load_tile<DV, ES, 32>(sV + stage * V_BYTES + cg * WN * PV, vg + voff, p.v.ss * ES, WN, vr, lane);
+    } else {
       fa_load_tile<DV, ES, NT>(sV + stage * V_BYTES, vg + (long long)n0 * p.v.ss * ES, p.v.ss * ES, BN, p.Skv - n0, tid);
     }
   };
@@ -130,38 +136,39 @@ extern "C" __global__ void __launch_bounds__(fa_dec::NT) fa_decode_kernel(const 
   for (int j = 0; j < DV / 8; ++j) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f;
   float m_run[2] = {FA_NEG_INF, FA_NEG_INF}, l_run[2] = {0.f, 0.f};
 
-  // prologue: fill STAGES-1 stages
-  int n0s[STAGES];
-  bool fulls[STAGES];
-  bool haves[STAGES];
-#pragma unroll
-  for (int i = 0; i < STAGES; ++i) { n0s[i] = 0; fulls[i] = false; haves[i] = false; }
-#pragma unroll
-  for (int i = 0; i < STAGES - 1; ++i) {
-    haves[i] = next_tile(n0s[i], fulls[i]);
-    if (haves[i]) load_kv(i, n0s[i]);
-    fa_cp_commit();
+  // K and V are released and asked for separately: the K buffer of a tile is free as soon as its scores are
+  // there, so K of the tile after next is under way during this tile's P.V, and V of the next one during its
+  // scores.  One and a half tiles are always in flight from two buffers of each (with both loads issued
+  // together at the top of the loop it was one).
+  int n0_cur = 0, n0_nxt = 0;
+  bool full_cur = false, full_nxt = false;
+  bool have = next_tile(n0_cur, full_cur), have_nxt = false;
+  if (have) load_k(0, n0_cur);
+  fa_cp_commit();
+  if (have) {
+    load_v(0, n0_cur);
+    have_nxt = next_tile(n0_nxt, full_nxt);
   }
+  fa_cp_commit();
+  if (have_nxt) load_k(1, n0_nxt);
+  fa_cp_commit();
   fa_u32 qf[D / 16][4];
   bool q_loaded = false;
-  int cur = 0;  // ring position of the tile being computed
+  int cur = 0;  // buffer of the tile being computed
 
-  while (haves[cur]) {
-    // prefetch into the stage that was consumed last iteration
-    const int pf = (cur + STAGES - 1) % STAGES;
-    haves[pf] = next_tile(n0s[pf], fulls[pf]);
-    if (haves[pf]) load_kv(pf, n0s[pf]);
-    fa_cp_commit();
-    fa_cp_wait<STAGES - 1>();
+  while (have) {
+    fa_cp_wait<2>();  // K of this tile (V of it and K of the next one may still be on their way)
     if (PRIVATE && q_loaded) __syncwarp();
     else __syncthreads();  // (first iteration: the query tile was loaded by all threads)
+    if (have_nxt) load_v(cur ^ 1, n0_nxt);
+    fa_cp_commit();
 
     if (!q_loaded) {
       q_loaded = true;
       fa_load_a_frags<D>(qf, sQ, PQ, rg * 16, lane);
     }
-    const int n0 = n0s[cur] + cg * WN;
-    const bool full = fulls[cur];
+    const int n0 = n0_cur + cg * WN;
+    const bool full = full_cur;
     float s[WN / 8][4];
 #pragma unroll
     for (int j = 0; j < WN / 8; ++j) s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
@@ -224,17 +231,26 @@ extern "C" __global__ void __launch_bounds__(fa_dec::NT) fa_decode_kernel(const 
         }
       }
       l_run[hh] = l_run[hh] * corr + sum;
+      // (after the first tiles the maximum seldom moves)
+      if (__any_sync(0xffffffffu, corr != 1.f)) {
 #pragma unroll
-      for (int j = 0; j < DV / 8; ++j) {
-        o[j][hh * 2] *= corr;
-        o[j][hh * 2 + 1] *= corr;
+        for (int j = 0; j < DV / 8; ++j) {
+          o[j][hh * 2] *= corr;
+          o[j][hh * 2 + 1] *= corr;
+        }
       }
     }
-    fa_mma_nn<DT, WN, DV>(o, s, sV + cur * V_BYTES + cg * WN * PV, PV, lane);
-
+    fa_cp_wait<2>();  // V of this tile
     if (PRIVATE) __syncwarp();
     else __syncthreads();
-    cur = (cur + 1) % STAGES;
+    have = have_nxt;
+    n0_cur = n0_nxt;
+    full_cur = full_nxt;
+    have_nxt = have && next_tile(n0_nxt, full_nxt);
+    if (have_nxt) load_k(cur, n0_nxt);
+    fa_cp_commit();
+    fa_mma_nn<DT, WN, DV>(o, s, sV + cur * V_BYTES + cg * WN * PV, PV, lane);
+    cur ^= 1;
   }
 
   fa_grid_release();
