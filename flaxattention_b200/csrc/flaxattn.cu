@@ -1134,15 +1134,15 @@ bool tc_fwd_eligible(const fa_attn_params* p) {
   return true;
 }
 
-// decode = true selects the split-KV variant of the kernel (one query tile per CTA, partial results)
-int get_fwd_tc_kernel(fa_module* m, int dtype, int D, int flags, Kernel** k, bool decode = false) {
+// decode = true selects the split-KV variant of the kernel (partial results); nq: query tiles of a CTA
+int get_fwd_tc_kernel(fa_module* m, int dtype, int D, int flags, Kernel** k, bool decode = false, int nq = 2) {
   // must match the shared-memory map of fa_fwd_tc.cuh (fa_tc::SMEM_BYTES)
-  const int atoms = dtype == FA_F32 ? 3 : D / 64, nstage = decode ? 5 : (dtype == FA_F32 ? 1 : (D == 64 ? 3 : 2));
-  const int smem = 2 * atoms * 16384 + 2 * nstage * atoms * 16384 + (1 + 4 * nstage + 8) * 8 + 16 + 256 * 2 + 256 * 2 +
+  const int atoms = dtype == FA_F32 ? 3 : D / 64, nstage = decode ? 5 : (dtype == FA_F32 ? 1 : (D == 64 ? nq + 1 : nq));
+  const int smem = nq * atoms * 16384 + 2 * nstage * atoms * 16384 + (1 + 4 * nstage + 8) * 8 + 16 + 256 * 2 + 256 * 2 +
                    2 * 256 + (256 / 32) * 4 + 1024;
   const int rnd = round_flag(dtype, flags);
-  return get_kernel(m, kernel_key(kIdFwdTc, {{dtype, 2}, {D, 9}, {rnd, 1}, {decode ? 1 : 0, 1}}), "fa_fwd_tc.cuh",
-                    [&] { return defs({{"FA_DTYPE", dtype}, {"FA_D", D}, {"FA_ROUND_SCORES", rnd}, {"FA_TC_DECODE", decode ? 1 : 0}}); },
+  return get_kernel(m, kernel_key(kIdFwdTc, {{dtype, 2}, {D, 9}, {rnd, 1}, {decode ? 1 : 0, 1}, {nq, 2}}), "fa_fwd_tc.cuh",
+                    [&] { return defs({{"FA_DTYPE", dtype}, {"FA_D", D}, {"FA_ROUND_SCORES", rnd}, {"FA_TC_DECODE", decode ? 1 : 0}, {"FA_TC_NQ", nq}}); },
                     "fa_fwd_tc_kernel", smem, k);
 }
 
@@ -1225,9 +1225,31 @@ int launch_decode_tc(fa_module* m, const fa_attn_params* p, const FaParams& kp, 
   return launch(k, dim3(num_splits, p->Hq, p->B), dim3(384), &tp, stream);
 }
 
+// SMs of the current device (148 on a B200; asked once per device)
+int device_sm_count() {
+  static std::atomic<int> cached[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+  int n = cached[dev].load(std::memory_order_relaxed);
+  if (n > 0) return n;
+  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+  cached[dev].store(n, std::memory_order_relaxed);
+  return n;
+}
+
+// Query tiles of a forward CTA.  With one, two CTAs share an SM: the fixed part of a CTA is hidden and the tail of
+// the grid is shorter, but a step costs more (K and V are loaded per 128 rows, and with D = 128 the products of
+// the two CTAs of an SM are not kept in turn).  So it is one where a CTA has few steps or there are no more tiles
+// than SMs (us, two against one; D = 64: B8 H8 S2048 dense 121 / 118, causal 87 / 83, B8 H8 S512 causal 19.3 / 17.8,
+// B4 H8 S333 16.4 / 14.3, but B2 H8 S4096 causal 61 / 64, dense 111 / 119; D = 128: S1024 49 / 51, S4096 268 / 282).
+int fwd_tc_query_tiles(const fa_attn_params* p) {
+  const long long tiles = (long long)p->B * p->Hq * ((p->Sq + 127) / 128);
+  return (p->D == 64 && p->Skv <= 2048) || tiles <= device_sm_count() ? 1 : 2;
+}
 int launch_fwd_tc(fa_module* m, const fa_attn_params* p, const FaParams& kp, void* stream) {
   Kernel* k = nullptr;
-  if (int rc = get_fwd_tc_kernel(m, p->dtype, p->D, p->flags, &k)) return rc;
+  const int nq = fwd_tc_query_tiles(p);
+  if (int rc = get_fwd_tc_kernel(m, p->dtype, p->D, p->flags, &k, false, nq)) return rc;
   FaTcParamsHost tp;
   tp.p = kp;
   if (int rc = make_map(&tp.tq, p->dtype, p->q, p->D, p->Sq, p->Hq, p->B)) return rc;
@@ -1237,7 +1259,7 @@ int launch_fwd_tc(fa_module* m, const fa_attn_params* p, const FaParams& kp, voi
   // Heads vary fastest and the query tile pair slowest (the kernel walks the pairs from the last one
   // down), so that under a causal mask the CTAs with the most kv tiles are dispatched first for
   // all heads: longest-first order keeps the tail of the grid short.
-  return launch(k, dim3(p->Hq, p->B, (p->Sq + 255) / 256), dim3(384), &tp, stream);
+  return launch(k, dim3(p->Hq, p->B, (p->Sq + 128 * nq - 1) / (128 * nq)), dim3(nq == 1 ? 256 : 384), &tp, stream);
 }
 
 // ---- tcgen05 backward ----------------------------------------------------------------------
@@ -1250,18 +1272,6 @@ struct FaBwdTcParamsHost {
   int* work_counter;
   int chunk_heads;
 };
-
-// SMs of the current device (148 on a B200; asked once per device)
-int device_sm_count() {
-  static std::atomic<int> cached[64];
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
-  int n = cached[dev].load(std::memory_order_relaxed);
-  if (n > 0) return n;
-  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-  cached[dev].store(n, std::memory_order_relaxed);
-  return n;
-}
 
 // pairs one item of fa_bwd_tc.cuh may list (fa_btc::MAXPL)
 int bwd_tc_max_pairs(int D) { return D == 64 ? 1024 : 2048; }
@@ -1403,7 +1413,8 @@ int fa_module_prepare(fa_module* m, int kind, int dtype, int D, int Dv, int Sq_h
       FwdCfg c;
       if (int rc = pick_fwd(dtype, D, Dv, Sq_hint, nullptr, c)) return rc;
       if (dtype != FA_F32 && D == Dv && (D == 64 || D == 128) && Sq_hint >= 128)
-        if (int rc = get_fwd_tc_kernel(m, dtype, D, 0, &k)) return rc;
+        for (int nq : {1, 2})
+          if (int rc = get_fwd_tc_kernel(m, dtype, D, 0, &k, false, nq)) return rc;
       return get_fwd_kernel(m, dtype, D, Dv, 0, c, &k);
     }
     case FA_KIND_BWD: {

@@ -21,7 +21,7 @@
 // kernel at 1024 keys).  The softmax keeps the operations and their order of fa_fwd.cuh.
 //
 // One CTA owns two 128-row query tiles of one (batch, head) and streams 128-row K/V tiles
-// past both.  Warp roles (12 warps = 3 warpgroups):
+// past both (or one, see NQ: then without warps 4-7, and the roles below move up).  Warp roles (12 warps = 3 warpgroups):
 //   warps 0-3  softmax warpgroup of query tile 0      warps 4-7  of query tile 1
 //   warp 8     TMA producer (one lane)
 //   warps 9-10 MMA issuers; warp 9 also allocates / frees TMEM.  With D = 64 warp 9 issues the S products and
@@ -39,7 +39,7 @@
 // status word, all roles leave their loops, TMEM is freed and the kernel returns.
 //
 // Compile-time parameters (macros): FA_DTYPE (0 fp16, 1 bf16, 2 fp32), FA_D (64 or 128), FA_TC_DECODE
-// (split-KV variant, see below).
+// (split-KV variant, see below), FA_TC_NQ (query tiles of a CTA, see below).
 #pragma once
 #include "fa_sm100.cuh"
 
@@ -76,8 +76,16 @@ constexpr int ATOM_BYTES = 128 * 128;    // 128 rows x 128 bytes
 constexpr bool DECODE = FA_TC_DECODE != 0;
 // (fp32: the parts of two query tiles, a K and a V tile fill shared memory; K of the next step is loaded
 // during the softmax and the PV products of this one, V during the next S products)
-constexpr int NSTAGE = DECODE ? 5 : (F32 ? 1 : (D == 64 ? 3 : 2));
-constexpr int Q_BYTES = 2 * ATOMS * ATOM_BYTES;
+// Query tiles of a CTA (decode: copies of the query tile).  One (FA_TC_NQ 1): two CTAs share an SM, so that the
+// set-up, first loads and epilogue of one run under the steps of the other and the last wave of the grid is
+// finer; K and V are then loaded for every query tile, through a shorter ring.  The host picks.
+#ifndef FA_TC_NQ
+#define FA_TC_NQ 2
+#endif
+constexpr int NQ = FA_TC_NQ;
+static_assert(NQ == 2 || (NQ == 1 && !DECODE && !F32), "one query tile: 16-bit forward");
+constexpr int NSTAGE = DECODE ? 5 : (F32 ? 1 : (D == 64 ? NQ + 1 : NQ));
+constexpr int Q_BYTES = NQ * ATOMS * ATOM_BYTES;
 constexpr int KV_STAGE = ATOMS * ATOM_BYTES;
 constexpr int MAXT = 256;                // kv tiles per row of the block grid (Skv <= 32768)
 constexpr int NBARS = 1 + 4 * NSTAGE + 8;
@@ -90,16 +98,16 @@ constexpr int OFF_MODE = OFF_SCHED + MAXT * 2;      // uchar mode[MAXT][2]
 constexpr int OFF_CLS = OFF_MODE + MAXT * 2;        // uchar cls[2][MAXT]
 constexpr int OFF_WCNT = OFF_CLS + 2 * MAXT;        // int wcount[MAXT / 32]: listed tiles per warp of the schedule build
 constexpr int SMEM_BYTES = OFF_WCNT + (MAXT / 32) * 4 + 1024;  // + slack for the 1024-byte alignment
-constexpr int TMEM_COLS = 512;
+constexpr int TMEM_COLS = 256 * NQ;
 // fp32: scores of tile i in columns 192 i .. + 127.  The softmax writes the parts of P over the scores it
 // has just read, 16 columns (32 keys) at a time: hi and mid of keys 32 c .. + 31 go to columns 32 c .. + 15
 // and 32 c + 16 .. + 31, lo to 128 + 16 c .. + 15.  O of tile i and step in 384 + 64 i.
-constexpr int COL_S = 0, COL_O = F32 ? 384 : 256, S_STRIDE = F32 ? 192 : 128;
+constexpr int COL_S = 0, COL_O = F32 ? 384 : 128 * NQ, S_STRIDE = F32 ? 192 : 128;
 // With D = 64 there is TMEM left for P next to S (columns 384..511): S of the next kv step can
 // then be produced while the softmax of the current step is still writing P.  With D = 128 the
 // 512 columns are taken by S and O, and P overwrites the S columns it was computed from.
 constexpr bool SEP_P = D == 64 && !F32;
-constexpr int COL_P = 384;
+constexpr int COL_P = 192 * NQ;
 // One pair of exponentials in FA_TC_POLY_EVERY goes to the FMA pipe (a cubic, see fa_ex2_poly2).
 // Measured (B8 H8 S2048 D64): every fourth pair takes the forward without a score_mod from 0.118 to
 // 0.114 ms, with the checkerboard mod from 0.133 to 0.129 and causal + ALiBi from 0.088 to 0.085;
@@ -107,14 +115,15 @@ constexpr int COL_P = 384;
 #ifndef FA_TC_POLY_EVERY
 #define FA_TC_POLY_EVERY 4
 #endif
-constexpr int NT = 384;
-// Register split (setmaxnreg): the kernel starts with 168 registers per thread (65536 / 384, rounded
-// down to a multiple of 8).  The third warpgroup gives up 72 each (128 x 72 = 9216) and the two
-// softmax warpgroups take 32 each (256 x 32 = 8192).  The increase must not ask for more than the
+constexpr int NSOFT = 4 * NQ;           // softmax warps
+constexpr int NT = (NSOFT + 4) * 32;
+// Register split (setmaxnreg): a thread starts with 168 registers with two query tiles (65536 / 384, rounded
+// down to a multiple of 8) and with 128 with one (two CTAs of 256 threads on an SM).  The last warpgroup gives
+// some up and the softmax warpgroups take them.  The increase must not ask for more than the
 // decrease releases: setmaxnreg.inc blocks until the registers are there, without a time limit.
-constexpr int REGS_SOFTMAX = 200, REGS_OTHER = 96;
-static_assert(256 * (REGS_SOFTMAX - 168) <= 128 * (168 - REGS_OTHER), "setmaxnreg.inc would wait forever");
-constexpr int WARP_PRODUCER = 8, WARP_MMA = 9, WARP_MMA_B = 10;
+constexpr int REGS_LAUNCH = NQ == 2 ? 168 : 128, REGS_SOFTMAX = NQ == 2 ? 200 : 192, REGS_OTHER = NQ == 2 ? 96 : 64;
+static_assert(NQ * (REGS_SOFTMAX - REGS_LAUNCH) <= REGS_LAUNCH - REGS_OTHER, "setmaxnreg.inc would wait forever");
+constexpr int WARP_PRODUCER = NSOFT, WARP_MMA = NSOFT + 1, WARP_MMA_B = NSOFT + 2;
 constexpr float RESCALE_THRESHOLD = 8.0f;  // log2 units
 
 static_assert(D == 64 || D == 128, "head dim 64 or 128");
@@ -534,7 +543,7 @@ __device__ __forceinline__ bool softmax_step_f32(SoftmaxCtx& c, float (&acc)[D],
 
 }  // namespace fa_tc
 
-extern "C" __global__ void __launch_bounds__(fa_tc::NT, 1) fa_fwd_tc_kernel(const __grid_constant__ FaTcParams P) {
+extern "C" __global__ void __launch_bounds__(fa_tc::NT, fa_tc::NQ == 1 ? 2 : 1) fa_fwd_tc_kernel(const __grid_constant__ FaTcParams P) {
   using namespace fa_tc;
   const FaParams& p = P.p;
   extern __shared__ unsigned char smem_raw[];
@@ -557,7 +566,7 @@ extern "C" __global__ void __launch_bounds__(fa_tc::NT, 1) fa_fwd_tc_kernel(cons
 #else
   const int pair = gridDim.z - 1 - blockIdx.z;  // grid: (heads, batch, tile pairs), the last pair first
   const int h = blockIdx.x, b = blockIdx.y;
-  const int m0 = pair * 2 * BM;
+  const int m0 = pair * NQ * BM;
 #endif
   const int hk = h / (p.Hq / p.Hkv);
   const int gb = b + p.b_off, gh = h + p.h_off;
@@ -571,7 +580,7 @@ extern "C" __global__ void __launch_bounds__(fa_tc::NT, 1) fa_fwd_tc_kernel(cons
   // thread's entry of the two index lists, for both query tiles.  They are all issued before any is
   // used (one round trip to memory instead of a chain of four dependent ones) and they are in flight
   // while the barriers are set up and TMEM is allocated.
-  constexpr int NI = DECODE ? 1 : 2;
+  constexpr int NI = DECODE ? 1 : NQ;
   const int ntiles = min((p.Skv + BN - 1) / BN, MAXT);
   const bool tables = p.t.kv_num != nullptr;
   const int tpb = tables ? (p.t.nKV == 1 ? ntiles : p.t.KVB / BN) : 1;
@@ -618,7 +627,7 @@ extern "C" __global__ void __launch_bounds__(fa_tc::NT, 1) fa_fwd_tc_kernel(cons
     // (decode variant: the query map's box is 64 rows and each warpgroup's tile gets the queries
     //  twice, in rows 0-63 and in rows 64-127; rows beyond Sq are out of range and read as zero)
     fa_mbar_expect_tx(bar_addr(sb, BAR_Q), Q_BYTES);
-    for (int i = 0; i < 2; ++i)
+    for (int i = 0; i < NQ; ++i)
       for (int a = 0; a < ATOMS; ++a) {
         if (DECODE) {
           fa_tma_load_4d(sb + (i * ATOMS + a) * ATOM_BYTES, &P.tq, bar_addr(sb, BAR_Q), a * 64, 0, h, b);
@@ -665,7 +674,7 @@ extern "C" __global__ void __launch_bounds__(fa_tc::NT, 1) fa_fwd_tc_kernel(cons
     int* wcount = (int*)(sm + OFF_WCNT);
     const bool mine = tid < MAXT;
     const unsigned char c0 = (mine && tid < ntiles) ? cls[tid] : 0;
-    const unsigned char c1 = (!DECODE && mine && tid < ntiles) ? cls[MAXT + tid] : 0;
+    const unsigned char c1 = (!DECODE && NQ == 2 && mine && tid < ntiles) ? cls[MAXT + tid] : 0;
     const bool listed = (c0 | c1) != 0;
     const unsigned vote = __ballot_sync(0xffffffffu, listed);
     if (mine && lane == 0) wcount[warp] = __popc(vote);
@@ -713,7 +722,7 @@ extern "C" __global__ void __launch_bounds__(fa_tc::NT, 1) fa_fwd_tc_kernel(cons
   const int nloads = misc[3];   // kv tiles the producer brings in (two per step in the decode variant)
   volatile int* abort_flag = misc + 1;
 
-  if (warp >= 8) fa_setmaxnreg_dec<REGS_OTHER>();
+  if (warp >= NSOFT) fa_setmaxnreg_dec<REGS_OTHER>();
   if (warp == WARP_PRODUCER) {
     // ================================ TMA producer =======================================
     if (lane == 0) {
@@ -752,7 +761,7 @@ extern "C" __global__ void __launch_bounds__(fa_tc::NT, 1) fa_fwd_tc_kernel(cons
           // tiles of the CTA's share in the decode variant
           int s = j % NSTAGE;
           if (!DECODE) ok = fa_mbar_wait(bar_addr(sb, BAR_KFULL + s), (fa_u32)((j / NSTAGE) & 1), abort_flag);
-          for (int i = 0; i < 2 && ok; ++i) {
+          for (int i = 0; i < NQ && ok; ++i) {
             if (!sched_mode[2 * j + i]) continue;
             if (DECODE) {
               const int t = 2 * j + i;
@@ -784,7 +793,7 @@ extern "C" __global__ void __launch_bounds__(fa_tc::NT, 1) fa_fwd_tc_kernel(cons
         for (int j = 0; j < nsteps && ok; ++j) {
           int s = j % NSTAGE;
           if (!DECODE) ok = fa_mbar_wait(bar_addr(sb, BAR_VFULL + s), (fa_u32)((j / NSTAGE) & 1), abort_flag);
-          for (int i = 0; i < 2 && ok; ++i) {
+          for (int i = 0; i < NQ && ok; ++i) {
             if (!sched_mode[2 * j + i]) continue;
             if (DECODE) {
               const int t = 2 * j + i;
@@ -865,7 +874,7 @@ extern "C" __global__ void __launch_bounds__(fa_tc::NT, 1) fa_fwd_tc_kernel(cons
         ok = fa_mbar_wait_all(bar_addr(sb, BAR_KFULL + 0), 0, abort_flag);
         if (ok) {
           fa_tc_fence_after();
-          for (int i = 0; i < 2; ++i)
+          for (int i = 0; i < NQ; ++i)
             if (sched_mode[i]) issue_s(0, i);
           if (leader) fa_mma_commit(bar_addr(sb, BAR_KEMPTY + 0));
         }
@@ -875,7 +884,7 @@ extern "C" __global__ void __launch_bounds__(fa_tc::NT, 1) fa_fwd_tc_kernel(cons
         const bool more = j + 1 < nsteps_u;
         ok = fa_mbar_wait_all(bar_addr(sb, BAR_VFULL + s), (fa_u32)((j / NSTAGE) & 1), abort_flag);
 #pragma unroll 1
-        for (int i = 0; i < 2 && ok; ++i) {
+        for (int i = 0; i < NQ && ok; ++i) {
           if (sched_mode[2 * j + i]) {
             ok = fa_mbar_wait_all(bar_addr(sb, BAR_P + i), cnt[i] & 1u, abort_flag);
             if (!ok) break;
@@ -883,7 +892,7 @@ extern "C" __global__ void __launch_bounds__(fa_tc::NT, 1) fa_fwd_tc_kernel(cons
             issue_pv(j, i, cnt[i] == 0);
             ++cnt[i];
           }
-          if (i == 1 && leader) fa_mma_commit(bar_addr(sb, BAR_VEMPTY + s));
+          if (i == NQ - 1 && leader) fa_mma_commit(bar_addr(sb, BAR_VEMPTY + s));
           if (more) {
             // (every step waits for its stage to be full before it releases it, with or without a product)
             ok = fa_mbar_wait_all(bar_addr(sb, BAR_KFULL + s1), (fa_u32)(((j + 1) / NSTAGE) & 1), abort_flag);
@@ -893,12 +902,12 @@ extern "C" __global__ void __launch_bounds__(fa_tc::NT, 1) fa_fwd_tc_kernel(cons
               fa_tc_fence_after();
               issue_s(j + 1, i);
             }
-            if (i == 1 && leader) fa_mma_commit(bar_addr(sb, BAR_KEMPTY + s1));
+            if (i == NQ - 1 && leader) fa_mma_commit(bar_addr(sb, BAR_KEMPTY + s1));
           }
         }
       }
     }
-  } else if (warp < 8) {
+  } else if (warp < NSOFT) {
     // ================================ softmax warpgroups ==================================
     fa_setmaxnreg_inc<REGS_SOFTMAX>();
     const int i = warp >> 2;                       // query tile of this warpgroup
