@@ -1365,7 +1365,7 @@ int get_bwd_tc_kernel(fa_module* m, int dtype, int D, int flags, bool kv2, Kerne
   const int bq = D == 64 ? 128 : 64, kvbuf = (D == 64 && kv2) ? 2 : 1, nstage = 3, nds = kvbuf == 1 ? 2 : 1;
   const int kv_bytes = (D / 64) * 16384, q_bytes = 16384, ds_bytes = (bq / 64) * 16384;
   const int smem = 2 * kvbuf * kv_bytes + 2 * nstage * q_bytes + nds * ds_bytes + 128 * 32 * 4 + nstage * 2 * bq * 4 +
-                   (2 + 3 * nstage + 15) * 8 + 16 + 32 + 2 * bwd_tc_max_pairs(D) * 4 + 256 + 1024;
+                   (2 + 3 * nstage + 15) * 8 + 16 + 32 + 2 * bwd_tc_max_pairs(D) * 4 + 64 + 1024;
   const int rnd = round_flag(dtype, flags);
   return get_kernel(m, kernel_key(kIdBwdTc, {{dtype, 2}, {D, 9}, {rnd, 1}, {kvbuf, 2}}), "fa_bwd_tc.cuh",
                     [&] { return defs({{"FA_DTYPE", dtype}, {"FA_D", D}, {"FA_ROUND_SCORES", rnd}, {"FA_BWD_KV2", kvbuf == 2 ? 1 : 0}}); },

@@ -114,8 +114,10 @@ constexpr int NBARS = 2 + 3 * NSTAGE + 15;
 constexpr int OFF_MISC = OFF_BAR + NBARS * 8;               // tmem base, abort, -, drain flag
 constexpr int OFF_ITEM = OFF_MISC + 16;                     // int item[2][4]: kv head (KV2: item number), batch, kv tile, pairs (-1: no more work)
 constexpr int OFF_PAIR = OFF_ITEM + 32;                     // int pair[2][MAXPL]: q tile | mode << 16 | g << 20
-constexpr int OFF_CLS = OFF_PAIR + 2 * MAXPL * 4;           // uchar cls[MAXC] (scratch of the list builder)
-constexpr int SMEM_BYTES = OFF_CLS + MAXC + 1024;
+constexpr int OFF_CLS = OFF_PAIR + 2 * MAXPL * 4;           // unsigned cls[2][MAXC / 32] (scratch of the list builder)
+constexpr int SMEM_BYTES = OFF_CLS + 2 * MAXC / 8 + 1024;
+// (the pointers of up to eight captured buffers are static shared memory beside this)
+static_assert(SMEM_BYTES + 8 * 8 <= 227 * 1024, "shared memory");
 static_assert(SMEM_BYTES <= 227 * 1024, "shared memory");
 constexpr int TMEM_COLS = 512;
 constexpr int COL_S = 0, COL_DP = BQ, COL_P = 2 * BQ;
@@ -296,22 +298,20 @@ __device__ __forceinline__ Item item_of(int idx, int Hkv, int B, int n_kvt, int 
   return {(int)(head - b * Hkv), (int)b, (int)kt};
 }
 
-// What the producer has published of an item.  (Two K / V buffers: its number, taken apart here; reading the three
-// parts made the compute warps spill and the kernel 4 % slower, causal B1 H8 S8192 D64 230 -> 241 us.)
-__device__ __forceinline__ Item read_item(const volatile int* item, int Hkv, int B) {
-  if (KVBUF == 2) {
-    const int idx = item[0];
-    return {idx % Hkv, (idx / Hkv) % B, idx / (Hkv * B)};
-  }
+// What the producer has published of an item.  With two K / V buffers that is the item's number, `idx`, which the
+// callers read together with the number of pairs and which is taken apart here: reading the three parts made the
+// compute warps spill and the kernel 4 % slower (causal B1 H8 S8192 D64 230 -> 241 us).
+__device__ __forceinline__ Item read_item(int idx, const volatile int* item, int Hkv, int B) {
+  if (KVBUF == 2) return {idx % Hkv, (idx / Hkv) % B, idx / (Hkv * B)};
   return {item[0], item[1], item[2]};
 }
 
 // The (query head, q tile) pairs of one item, written to `pl` by one warp: per head of the group,
 // the 128-row q tiles the BlockMask lists for the item's kv tile (class 1: apply mask_mod, 2: full)
 // in ascending order, each as 128 / BQ pairs.  Without tables every tile is listed.  Returns the
-// number of pairs (the same in every lane).  `cl` is MAXC bytes of scratch.
+// number of pairs (the same in every lane).  `cl` is scratch: one bit per q tile and class.
 __device__ __forceinline__ int build_pair_list(const FaParams& p, int hk, int b, int kt, int G, int n_ctiles,
-                                               unsigned char* cl, int* pl, int lane) {
+                                               unsigned* cl, int* pl, int lane) {
   constexpr int PPT = 128 / BQ;
   const bool tables = p.t.kv_num != nullptr && p.t.q_num != nullptr;
   int w = 0;
@@ -327,7 +327,7 @@ __device__ __forceinline__ int build_pair_list(const FaParams& p, int hk, int b,
       continue;
     }
     const int h = hk * G + g;
-    ((uint2*)cl)[lane] = make_uint2(0u, 0u);  // MAXC = 256 bytes
+    if (lane < 2 * MAXC / 32) cl[lane] = 0u;
     __syncwarp();
     {
       // both counts are read before either index list (two round trips to memory, not four)
@@ -347,14 +347,15 @@ __device__ __forceinline__ int build_pair_list(const FaParams& p, int hk, int b,
         for (int e = lane; e < num[which]; e += 32) {
           const int bi = e / tpb, ti = e - bi * tpb;
           const int t = min(max(idxp[row * p.t.nQ + bi], 0), p.t.nQ - 1) * tpb + ti;
-          if (t < n_ctiles) cl[t] = (unsigned char)(which ? 2 : 1);
+          if (t < n_ctiles) atomicOr(cl + which * (MAXC / 32) + (t >> 5), 1u << (t & 31));
         }
         __syncwarp();
       }
     }
     for (int t0 = 0; t0 < n_ctiles; t0 += 32) {
       const int t = t0 + lane;
-      const int c = t < n_ctiles ? (int)cl[t] : 0;
+      // (only tiles below n_ctiles have a bit; a tile in both lists counts as full)
+      const int c = (cl[MAXC / 32 + (t0 >> 5)] >> lane) & 1u ? 2 : (int)((cl[t0 >> 5] >> lane) & 1u);
       int n_t = 0;
       if (c != 0)
         for (int v = 0; v < PPT; ++v) n_t += (t * PPT + v) * BQ < p.Sq ? 1 : 0;
@@ -472,7 +473,7 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
       const Item it = item_of(min(idx, n_items - 1), p.Hkv, p.B, n_kvt, P.chunk_heads);
       const int hk = it.hk, b = it.b, kt = it.kt;
       int np = -1;
-      if (idx < n_items) np = build_pair_list(p, hk, b, kt, G, n_ctiles, sm + OFF_CLS, pl, lane);
+      if (idx < n_items) np = build_pair_list(p, hk, b, kt, G, n_ctiles, (unsigned*)(sm + OFF_CLS), pl, lane);
       if (lane == 0) {
         item[4 * lb] = KVBUF == 2 ? idx : hk;
         item[4 * lb + 1] = b;
@@ -703,10 +704,10 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
       const int lb = itc & 1;
       ok = fa_mbar_wait_warp(bar_addr(sb, BAR_LISTFULL + lb), (fa_u32)((itc >> 1) & 1), abort_flag);
       if (!ok) break;
-      const int np = item[4 * lb + 3];
+      const int idx = KVBUF == 2 ? item[4 * lb] : 0, np = item[4 * lb + 3];
       if (np < 0) break;
       const int* pl = pairs + lb * MAXPL;
-      const Item it = read_item(item + 4 * lb, p.Hkv, p.B);
+      const Item it = read_item(idx, item + 4 * lb, p.Hkv, p.B);
       const int hk = it.hk, b = it.b, n0 = it.kt * BT;
       const int gb = b + p.b_off;
       const int kv = n0 + r;
@@ -821,10 +822,10 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
         ok = false;
         break;
       }
-      const int np = item[4 * lb + 3];
+      const int idx = KVBUF == 2 ? item[4 * lb] : 0, np = item[4 * lb + 3];
       if (np < 0) break;  // (the same in all four warps)
       const int* pl = pairs + lb * MAXPL;
-      const Item it = read_item(item + 4 * lb, p.Hkv, p.B);
+      const Item it = read_item(idx, item + 4 * lb, p.Hkv, p.B);
       const int hk = it.hk, b = it.b, n0 = it.kt * BT;
       for (int n = 0; n < np && ok; ++n, ++gn) {
         const int pr = pl[n];
