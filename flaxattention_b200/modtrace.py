@@ -22,18 +22,21 @@ Python scalars are weakly typed the way JAX treats them: ``int32 * 8.0`` is floa
 from __future__ import annotations
 
 import builtins
+import contextlib
 import copy
 import dis
 import functools
 import hashlib
 import inspect
 import math
+import struct
 import types
 import weakref
 from typing import Callable, Dict, List, Optional, Sequence, Tuple
 
 import numpy as np
 import torch
+from torch.utils._python_dispatch import TorchDispatchMode
 
 I32, F32, B1 = "i32", "f32", "b1"
 
@@ -414,13 +417,11 @@ def _lift(x) -> Expr:
     if isinstance(x, (float, np.floating)):
         return _B.const(float(x), F32)
     if isinstance(x, np.ndarray) and x.ndim == 0:
-        _note_tensor_value()
         return _lift(x.item())
     try:  # 0-d torch tensors captured as constants
         import torch
 
         if isinstance(x, torch.Tensor) and x.ndim == 0:
-            _note_tensor_value()
             return _lift(x.item())
     except ImportError:  # pragma: no cover
         pass
@@ -442,12 +443,6 @@ _ELEM_TYPES = {
     "int32": ("i32", I32), "int64": ("i64", I32), "uint8": ("u8", I32), "bool": ("u8", B1), "float32": ("f32", F32),
 }
 _TRACE_BUFFERS: Optional[List[object]] = None  # buffers of the mod pair being traced
-_TENSOR_VALUES_READ = False  # set when a trace turns the contents of a tensor into a constant
-
-
-def _note_tensor_value():
-    global _TENSOR_VALUES_READ
-    _TENSOR_VALUES_READ = True
 
 
 def _buffer_load(buf, index) -> "Sym":
@@ -1559,84 +1554,140 @@ def _trace_any(fn: Callable, kind: str, bufs: List[object]) -> TracedMod:
 # another tensor.  Tracing and lowering it takes 100-200 us; what the trace can depend on (the code, the
 # constants it closes over, shape, strides and type of its tensors) is gone through in about 10, and a pair
 # of mods with equal fingerprints shares the lowered text and only brings its own tensors.
+# What counts as known is kept narrow, because a miss is silent: names are followed to their values through
+# the globals and through modules, functions found there are gone through like the mod itself, and whatever
+# is not one of the types below, a function of this module or one of a fixed list of pure functions of
+# torch, numpy and math makes the pair one that is traced every time.
 @functools.lru_cache(maxsize=1024)
 def _code_facts(code):
-    """(names the code and the code nested in it use, whether it branches on a value)."""
-    names, branches = set(code.co_names), False
-    for ins in dis.get_instructions(code):
-        if "JUMP_IF" in ins.opname:
+    """(chains of names the code and the code nested in it look up: a global and the attributes taken of it
+    right away, whether it branches on a value, whether it does anything else that reaches outside)."""
+    chains, branches, opaque = set(), False, False
+    ins = list(dis.get_instructions(code))
+    i = 0
+    while i < len(ins):
+        op, arg = ins[i].opname, ins[i].argval
+        i += 1
+        if op in ("LOAD_GLOBAL", "LOAD_NAME"):
+            chain = [arg]
+            while i < len(ins) and ins[i].opname in ("LOAD_ATTR", "LOAD_METHOD"):
+                chain.append(ins[i].argval)
+                i += 1
+            chains.add(tuple(chain))
+        elif "JUMP_IF" in op:
             branches = True
+        elif op in ("LOAD_ATTR", "LOAD_METHOD", "LOAD_SUPER_ATTR", "IMPORT_NAME", "IMPORT_FROM", "STORE_GLOBAL",
+                    "DELETE_GLOBAL", "STORE_ATTR", "DELETE_ATTR", "STORE_NAME", "LOAD_BUILD_CLASS"):
+            opaque = True  # a method or an attribute of a value, or state that changes
+        elif op == "STORE_DEREF" and arg in code.co_freevars:
+            opaque = True
     for c in code.co_consts:
         if isinstance(c, types.CodeType):
-            n, br = _code_facts(c)
-            names |= set(n)
-            branches = branches or br
-    return tuple(sorted(names)), branches
+            n, br, o = _code_facts(c)
+            chains |= set(n)
+            branches, opaque = branches or br, opaque or o
+    return tuple(sorted(chains)), branches, opaque
 
 
 class _Unknown(Exception):
     """The trace may depend on something a fingerprint does not cover."""
 
 
-def _fingerprint_value(x, tensors: List[object], out: List[object], depth: int) -> None:
-    t = type(x)
-    if x is None or t in (bool, int, float, str):
-        out.append((t, x))
-    elif t is types.FunctionType:
-        _fingerprint_function(x, tensors, out, depth + 1)
-    elif t in (tuple, list):
-        out.append((t, len(x)))
-        for y in x:
-            _fingerprint_value(y, tensors, out, depth + 1)
-    elif t is torch.Tensor:
-        k = next((i for i, y in enumerate(tensors) if y is x), len(tensors))
-        if k == len(tensors):
-            tensors.append(x)
-        out.append(("tensor", k, x.dtype, tuple(x.shape), x.stride()))
-    else:
-        raise _Unknown
+# functions of numpy and torch that give the same for the same arguments and read nothing else
+_PURE = {"torch": frozenset(_TORCH_FUNCS), "numpy": frozenset(_NP_UFUNCS) | {"where", "float32", "int32"}}
 
 
-def _fingerprint_function(fn, tensors: List[object], out: List[object], depth: int = 0) -> None:
-    if depth > 8:
-        raise _Unknown
-    code = fn.__code__
-    names, branches = _code_facts(code)
-    out.append(code)
-    before = len(tensors)
-    for cell in fn.__closure__ or ():
-        try:
-            _fingerprint_value(cell.cell_contents, tensors, out, depth)
-        except ValueError:  # an empty cell
-            raise _Unknown from None
-    for d in (fn.__defaults__, tuple(sorted((fn.__kwdefaults__ or {}).items()))):
-        _fingerprint_value(d, tensors, out, depth)
-    g = fn.__globals__
-    modules = [g[n] for n in names if isinstance(g.get(n), types.ModuleType)]
-    for n in names:
-        if n in g:
-            if isinstance(g[n], types.ModuleType):
-                out.append(("module", n, id(g[n])))
-            else:
-                out.append(n)
-                _fingerprint_value(g[n], tensors, out, depth)
-        elif hasattr(builtins, n):
-            if n != "abs":
-                raise _Unknown  # int(tensor), len(...) and the like
-        elif any(hasattr(m, n) for m in modules):
-            # an attribute of a module: a function of it, or a constant
-            for m in modules:
-                x = getattr(m, n, None)
-                if isinstance(x, (bool, int, float)):
-                    out.append((n, x))
-                elif isinstance(x, (torch.Tensor, np.ndarray)):
+class _Fingerprint:
+    """What the trace of a mod pair can depend on, gathered in ``parts``, apart from the contents of the
+    tensors found on the way (``tensors``); raises ``_Unknown`` where that cannot be said."""
+
+    def __init__(self, *fns):
+        self.tensors: List[object] = []
+        self.parts: List[object] = []
+        self.host_math = False  # calls functions that could turn a tensor into a number
+        for fn in fns:
+            self.parts.append("|")
+            if fn is not None:
+                if type(fn) is not types.FunctionType:
                     raise _Unknown
-                else:
-                    out.append((n, id(x)))
+                self.function(fn, 0)
+        if self.host_math and self.tensors:
+            raise _Unknown
+        self.key = tuple(self.parts)
+
+    def value(self, x, depth: int) -> None:
+        t = type(x)
+        if t is float:
+            self.parts.append((t, struct.pack("<d", x)))  # (0.0 == -0.0, and nan != nan)
+        elif x is None or t in (bool, int, str, torch.dtype):
+            self.parts.append((t, x))
+        elif t is types.FunctionType:
+            if x.__module__ == __name__:
+                self.parts.append(x)  # (by identity, and kept alive by the key)
+            else:
+                self.function(x, depth + 1)
+        elif t in (tuple, list):
+            self.parts.append((t, len(x)))
+            for y in x:
+                self.value(y, depth + 1)
+        elif t is torch.Tensor:
+            k = next((i for i, y in enumerate(self.tensors) if y is x), len(self.tensors))
+            if k == len(self.tensors):
+                self.tensors.append(x)
+            self.parts.append(("tensor", k, x.dtype, tuple(x.shape), x.stride()))
         else:
-            raise _Unknown  # a method or an attribute of a value
-    if branches and len(tensors) > before:
-        raise _Unknown  # may branch on the contents of a tensor
+            raise _Unknown
+
+    def chain(self, g, names, depth: int) -> None:
+        """The value of ``names[0]`` in the globals ``g``, or of an attribute of the module it is."""
+        self.parts.append(names)
+        if names[0] not in g:
+            if names != ("abs",):  # int(tensor), len(...) and the like
+                raise _Unknown
+            self.parts.append(getattr(builtins, "abs"))
+            return
+        x, parent, rest = g[names[0]], None, list(names[1:])
+        while isinstance(x, types.ModuleType):
+            if not rest or rest[0] not in vars(x):
+                raise _Unknown
+            parent, x = x, vars(x)[rest[0]]
+            last = rest.pop(0)
+        if rest:
+            raise _Unknown  # an attribute of a value
+        if parent is not None and (parent is math or last in _PURE.get(parent.__name__, ())) and callable(x):
+            self.host_math = self.host_math or parent.__name__ != "torch"
+            self.parts.append(x)
+        else:
+            self.value(x, depth)
+
+    def function(self, fn, depth: int) -> None:
+        chains, branches, opaque = _code_facts(fn.__code__)
+        if depth > 8 or opaque:
+            raise _Unknown
+        self.parts.append(fn.__code__)
+        before = len(self.tensors)
+        for cell in fn.__closure__ or ():
+            try:
+                self.value(cell.cell_contents, depth)
+            except ValueError:  # an empty cell
+                raise _Unknown from None
+        for d in (fn.__defaults__, tuple(sorted((fn.__kwdefaults__ or {}).items()))):
+            self.value(d, depth)
+        for names in chains:
+            self.chain(fn.__globals__, names, depth)
+        if branches and len(self.tensors) > before:
+            raise _Unknown  # may branch on the contents of a tensor
+
+
+class _TensorWatch(TorchDispatchMode):
+    """Notices every operation on a tensor.  A trace in which there was none has read no tensor (indexing one
+    with a traced value is not an operation on it), so its text holds for other tensors of the same form."""
+
+    used = False
+
+    def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+        self.used = True
+        return func(*args, **(kwargs or {}))
 
 
 class _Template:
@@ -1687,34 +1738,26 @@ def lower_mods(score_mod: Optional[Callable], mask_mod: Optional[Callable]) -> M
     hit = _MODSET_CACHE.get(key)
     if hit is not None and hit[0]() is score_mod and hit[1]() is mask_mod:
         return hit[2]
-    tensors: List[object] = []
-    fp = None
     try:
-        parts: List[object] = []
-        for fn in (score_mod, mask_mod):
-            parts.append("|")
-            if fn is not None:
-                if type(fn) is not types.FunctionType:
-                    raise _Unknown
-                _fingerprint_function(fn, tensors, parts)
-        fp = tuple(parts)
+        fp = _Fingerprint(score_mod, mask_mod)
     except _Unknown:
         fp = None
-    tpl = _TEMPLATES.get(fp) if fp is not None else None
+    tpl = _TEMPLATES.get(fp.key) if fp is not None else None
     if tpl is not None:
-        ms = tpl.bind(tensors)
+        ms = tpl.bind(fp.tensors)
     else:
-        global _TENSOR_VALUES_READ
-        _TENSOR_VALUES_READ = False
         bufs: List[object] = []
-        s = _trace_any(score_mod, "score", bufs) if score_mod is not None else None
-        m = _trace_any(mask_mod, "mask", bufs) if mask_mod is not None else None
+        watch = _TensorWatch()
+        with watch if fp is not None else contextlib.nullcontext():
+            s = _trace_any(score_mod, "score", bufs) if score_mod is not None else None
+            m = _trace_any(mask_mod, "mask", bufs) if mask_mod is not None else None
         ms = ModSet(s, m, bufs)
-        which = [next((i for i, t in enumerate(tensors) if t is b), -1) for b in ms.buffers]
-        if fp is not None and -1 not in which and len(set(which)) == len(tensors) and not _TENSOR_VALUES_READ:
-            if len(_TEMPLATES) >= 1024:
-                _TEMPLATES.clear()
-            _TEMPLATES[fp] = _Template(ms, which)
+        if fp is not None and not watch.used:
+            which = [next((i for i, t in enumerate(fp.tensors) if t is b), -1) for b in ms.buffers]
+            if -1 not in which and len(set(which)) == len(fp.tensors):
+                if len(_TEMPLATES) >= 1024:
+                    _TEMPLATES.clear()
+                _TEMPLATES[fp.key] = _Template(ms, which)
     if len(_MODSET_CACHE) > 4096:
         for k in list(_MODSET_CACHE):
             _forget(k)

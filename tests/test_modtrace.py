@@ -1,8 +1,12 @@
 """Tracer / lowering tests (CPU): the expression graph recorded from a mod must evaluate
 to what the Python mod itself returns on numpy arrays, the symbolic derivative must match
 a finite difference, and the generated CUDA text must compile for sm_100a."""
+import math
+import types
+
 import numpy as np
 import pytest
+import torch
 
 from flaxattention_b200 import _cabi, fnp, modtrace
 from flaxattention_b200.blockmask import and_masks, or_masks, noop_mask
@@ -317,3 +321,124 @@ def test_bias_that_is_linear_in_an_index_gets_a_slope():
     for fn in (checkerboard, quadratic, huge):
         src = mt.lower_mods(fn, None).source
         assert "FA_SCORE_LINEAR_KV" not in src, fn.__name__
+
+
+def _module(source):
+    m = types.ModuleType("some_settings")
+    exec(source, m.__dict__)
+    return m
+
+
+settings = None  # a module, as a mod's globals see it
+
+
+def _changing_mods():
+    """name -> (make, change): ``make()`` gives a new mask_mod of the same code each time, ``change()`` changes
+    something its trace depends on."""
+    global settings
+    settings = _module("WINDOW = 64\nCFG = {'w': 64}\nSCALE = [64]\nTABLE = None\n"
+                  "def near(q, kv):\n    return q - kv < WINDOW\n"
+                  "def listed(q, kv):\n    return q - kv < SCALE[0]\n"
+                  "def keyed(q, kv):\n    return q - kv < CFG['w']\n")
+    box = types.SimpleNamespace(doc=torch.arange(8, dtype=torch.int32), pair=(1.0, 0.0), n=3)
+
+    def through_module_function():
+        return lambda b, h, q, kv: settings.near(q, kv)
+
+    def through_module_list():
+        return lambda b, h, q, kv: settings.listed(q, kv)
+
+    def through_module_dict():
+        return lambda b, h, q, kv: settings.keyed(q, kv)
+
+    def module_number():
+        return lambda b, h, q, kv: q - kv < settings.WINDOW
+
+    def module_container():
+        return lambda b, h, q, kv: q - kv < settings.SCALE[0]
+
+    def attribute_of_a_value():
+        return lambda b, h, q, kv: q - kv < box.n
+
+    def over(f):
+        def make():
+            doc = box.doc
+            return f(doc)
+        return make
+
+    def new_doc():
+        box.doc = torch.arange(8, dtype=torch.int32) + 5
+
+    def host_function(doc):
+        return lambda b, h, q, kv: doc[kv] < math.floor(doc[0])
+
+    def as_an_index(doc):
+        steps = [2, 3, 4, 5, 6, 7, 8, 9]
+        return lambda b, h, q, kv: doc[kv] < steps[doc[0]]
+
+    def compared(doc):
+        return lambda b, h, q, kv: doc[kv] < torch.equal(doc, doc.sort()[0]) + torch.remainder(doc[1], 3)
+
+    def through_a_list(doc):
+        return lambda b, h, q, kv: doc[kv] < doc.tolist()[0]
+
+    def through_numpy(doc):
+        return lambda b, h, q, kv: doc[kv] < np.float32(np.maximum(doc, 2)[0])
+
+    def signed_zero():
+        z = box.pair[1]
+        return lambda score, b, h, q, kv: fnp.where(q > kv, score, z)
+
+    def set_attr(o, k, x):
+        return lambda: setattr(o, k, x)
+
+    return {
+        "function of a module": (through_module_function, set_attr(settings, "WINDOW", 16)),
+        "list behind a function of a module": (through_module_list, lambda: settings.SCALE.__setitem__(0, 16)),
+        "dict behind a function of a module": (through_module_dict, lambda: settings.CFG.__setitem__("w", 16)),
+        "number of a module": (module_number, set_attr(settings, "WINDOW", 16)),
+        "list of a module": (module_container, lambda: settings.SCALE.__setitem__(0, 16)),
+        "attribute": (attribute_of_a_value, set_attr(box, "n", 5)),
+        "tensor value through math": (over(host_function), new_doc),
+        "tensor value as an index": (over(as_an_index), new_doc),
+        "tensor value through a torch comparison": (over(compared), new_doc),
+        "tensor value through a list": (over(through_a_list), new_doc),
+        "tensor value through numpy": (over(through_numpy), new_doc),
+        "sign of zero": (signed_zero, set_attr(box, "pair", (1.0, -0.0))),
+    }
+
+
+@pytest.mark.parametrize("name", list(_changing_mods()))
+def test_a_new_closure_is_lowered_from_what_it_reads_now(name):
+    """A second closure of the same code, made after something it reads has changed, must not get the text
+    lowered for the first one."""
+    make, change = _changing_mods()[name]
+
+    def lowered(fn):
+        return (modtrace.lower_mods(fn, None) if modtrace.mod_arity(fn) == 5 else modtrace.lower_mods(None, fn)).source
+
+    modtrace._TEMPLATES.clear()
+    first = make()
+    before = lowered(first)
+    change()
+    second = make()
+    got = lowered(second)
+    modtrace._TEMPLATES.clear()
+    third = make()
+    assert got == lowered(third)
+    assert got != before  # the change shows in the text
+
+
+def test_closures_over_other_tensors_of_the_same_form_share_the_text():
+    modtrace._TEMPLATES.clear()
+
+    def make(doc, w):
+        return lambda b, h, q, kv: (doc[q] == doc[kv]) & (q >= kv) & (fnp.abs(q - kv) <= w)
+
+    docs = [torch.arange(16, dtype=torch.int32) + i for i in range(3)]
+    mods = [make(d, 4) for d in docs]
+    ms = [modtrace.lower_mods(None, m) for m in mods]
+    assert len(modtrace._TEMPLATES) == 1 and ms[0].source == ms[1].source == ms[2].source
+    assert all(m.buffers[0] is d for m, d in zip(ms, docs))
+    wide = make(docs[0], 5)
+    assert modtrace.lower_mods(None, wide).source != ms[0].source
