@@ -36,6 +36,7 @@ class FaBlockTables(C.Structure):
         ("mask_bits", C.c_void_p), ("mask_bits_stride", C.c_int64), ("mask_bits_rows", C.c_int32),
         ("mask_bits_B", C.c_int32), ("mask_bits_H", C.c_int32),
         ("mask_bits_t", C.c_void_p), ("mask_bits_t_stride", C.c_int64), ("mask_bits_t_rows", C.c_int32),
+        ("mask_bits_hold", C.c_void_p),
     ]
 
 
@@ -70,6 +71,7 @@ EXPORTS = [
     "fa_block_mask_workspace_bytes", "fa_block_mask", "fa_decode_static_capacity", "fa_decode_static",
     "fa_profile_enable", "fa_profile_read", "fa_decode_packs_heads", "fa_selftest_bounded_wait",
     "fa_mask_bits_row_words", "fa_mask_bits", "fa_block_mask_build",
+    "fa_snapshot_bytes", "fa_snapshot", "fa_snapshot_holds",
     "fa_fwd_workspace_bytes", "fa_fwd_ws",
 ]
 
@@ -122,6 +124,11 @@ def lib() -> C.CDLL:
     L.fa_profile_enable.argtypes = [C.c_int]
     L.fa_profile_read.argtypes = [C.c_int, C.POINTER(C.c_float), C.POINTER(C.c_char_p)]
     L.fa_selftest_bounded_wait.argtypes = [C.c_ulonglong, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]
+    ranges = [C.POINTER(C.c_void_p), C.POINTER(C.c_size_t), C.c_int]
+    L.fa_snapshot_bytes.restype = C.c_size_t
+    L.fa_snapshot_bytes.argtypes = ranges[1:]
+    L.fa_snapshot.argtypes = ranges + [C.c_void_p, C.c_void_p]
+    L.fa_snapshot_holds.argtypes = ranges + [C.c_void_p, C.c_void_p, C.c_void_p]
     L.fa_mask_bits_row_words.restype = C.c_int64
     L.fa_mask_bits_row_words.argtypes = [C.c_int]
     L.fa_mask_bits.argtypes = [C.c_void_p] + [C.c_int] * 6 + [C.c_void_p, C.c_void_p]
@@ -198,6 +205,13 @@ class Module:
                 self.handle = None
         except Exception:
             pass
+
+
+def ranges(tensors):
+    """(addresses, byte counts, number) of the memory that tensors span, as fa_snapshot takes them."""
+    n = len(tensors)
+    size = [(1 + sum((d - 1) * s for d, s in zip(t.shape, t.stride()))) * t.element_size() for t in tensors]
+    return (C.c_void_p * n)(*(t.data_ptr() for t in tensors)), (C.c_size_t * n)(*size), n
 
 
 def profile_enable(on: bool) -> None:

@@ -18,7 +18,8 @@ import numpy as np
 import torch
 
 from . import _cabi
-from .blockmask import BlockMask, bind_mod_buffers, identity_score as _identity, module_for, noop_mask
+from .blockmask import BlockMask, bind_mod_buffers, device_buffers, identity_score as _identity, module_for, noop_mask
+from .modtrace import lower_mods
 
 _DTYPES = {torch.float16: _cabi.FA_F16, torch.bfloat16: _cabi.FA_BF16, torch.float32: _cabi.FA_F32}
 
@@ -140,7 +141,10 @@ class _Call:
         self.options = dict(options or {})
         self.round_scores = bool(self.options.get("round_scores", round_scores))
 
-    def params(self, q, k, v, o, lse) -> _cabi.FaAttnParams:
+    def params(self, q, k, v, o, lse, stream=None) -> _cabi.FaAttnParams:
+        """The parameter block of a launch.  With ``stream``, the block is for one launch that follows on it
+        at once; without, it may be launched again later, and bit matrices over captured tensors, which hold
+        only as long as these stay what they were, are left out."""
         p = _cabi.FaAttnParams()
         p.dtype = _DTYPES[self.dtype]
         p.B, p.Hq, p.Hkv, p.Sq, p.Skv, p.D, p.Dv = self.B, self.Hq, self.Hkv, self.Sq, self.Skv, self.D, self.Dv
@@ -165,13 +169,16 @@ class _Call:
             t.mask_B, t.mask_H = bm.kv_indices.shape[0], bm.kv_indices.shape[1]
             t.num_q_blocks, t.num_kv_blocks = bm.kv_indices.shape[2], bm.kv_indices.shape[3]
             t.q_block_size, t.kv_block_size = bm.BLOCK_SIZE
-            mb = bm.mask_bits if bm.bits_hold() else None
+            mb = bm.mask_bits if bm.bits_hold() and (not bm._bits_sources or stream is not None) else None
             if mb is not None and self.mask_mod is bm.mask_mod and mb.device == q.device and mb.shape[2] >= self.Sq \
                     and mb.shape[3] * 32 >= self.Skv and mb.shape[0] in (1, self.B) and mb.shape[1] in (1, self.Hq):
                 if mb.dtype != torch.int32 or not mb.is_contiguous():
                     raise ValueError("BlockMask.mask_bits must be a contiguous int32 tensor")
                 t.mask_bits, t.mask_bits_stride, t.mask_bits_rows = mb.data_ptr(), mb.shape[3], mb.shape[2]
                 t.mask_bits_B, t.mask_bits_H = mb.shape[0], mb.shape[1]
+                if bm._bits_sources:
+                    p.hold = bm.launch_check(self.module_buffers(q.device), stream)  # (kept with the block)
+                    t.mask_bits_hold = p.hold.data_ptr()
                 mt = bm.mask_bits_t
                 if mt is not None and mt.device == q.device and mt.dtype == torch.int32 and mt.is_contiguous() \
                         and mt.shape[:2] == mb.shape[:2] and mt.shape[2] >= self.Skv and mt.shape[3] * 32 >= self.Sq:
@@ -181,6 +188,10 @@ class _Call:
                 if x is not None and (x.dtype != torch.int32 or not x.is_contiguous()):
                     raise ValueError("BlockMask tables must be contiguous int32 tensors")
         return p
+
+    def module_buffers(self, device):
+        """The tensors the mask_mod captures, on ``device``."""
+        return device_buffers(lower_mods(None, self.mask_mod), device)
 
     def use_decode(self) -> bool:
         force = self.options.get("path")
@@ -201,9 +212,9 @@ def _forward(call: _Call, q, k, v):
     check_status()
     out = call.out_like(q)
     lse = torch.empty(call.B, call.Hq, call.Sq, dtype=torch.float32, device=q.device)
-    p = call.params(q, k, v, out, lse)
     stream = torch.cuda.current_stream(q.device).cuda_stream
     with torch.cuda.device(q.device):
+        p = call.params(q, k, v, out, lse, stream)
         bind_mod_buffers(call.module, call.score_mod, call.mask_mod, q.device)
         if call.use_decode():
             splits = int(call.options.get("num_splits", 0))
@@ -226,11 +237,11 @@ def _backward(call: _Call, q, k, v, out, lse, dout):
     if dout.stride(-1) != 1:
         dout = dout.contiguous()
     dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-    p = call.params(q, k, v, out, lse)
-    nbytes = L.fa_bwd_workspace_bytes(p)
-    ws = torch.empty(max(nbytes, 16), dtype=torch.uint8, device=q.device)
     stream = torch.cuda.current_stream(q.device).cuda_stream
     with torch.cuda.device(q.device):
+        p = call.params(q, k, v, out, lse, stream)
+        nbytes = L.fa_bwd_workspace_bytes(p)
+        ws = torch.empty(max(nbytes, 16), dtype=torch.uint8, device=q.device)
         bind_mod_buffers(call.module, call.score_mod, call.mask_mod, q.device)
         _cabi.check(L.fa_bwd(call.module.handle, p, _tensor(dout, call.layout), _tensor(dq, call.layout),
                              _tensor(dk, call.layout), _tensor(dv, call.layout), ws.data_ptr(), nbytes, stream))

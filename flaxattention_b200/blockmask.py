@@ -119,7 +119,7 @@ class BlockMask:
 
     def __init__(self, kv_num_blocks, kv_indices, full_kv_num_blocks, full_kv_indices, q_num_blocks, q_indices,
                  full_q_num_blocks, full_q_indices, BLOCK_SIZE, mask_mod, mask_bits=None, mask_bits_t=None,
-                 _bits_sources=()):
+                 _bits_sources=(), _bits_snapshot=None):
         if kv_indices.ndim < 2:
             raise RuntimeError("BlockMask must have at least 2 dimensions")
         assert kv_num_blocks is not None, "kv_num_blocks must be provided"
@@ -144,14 +144,30 @@ class BlockMask:
         self.mask_mod = mask_mod
         self.mask_bits = mask_bits
         self.mask_bits_t = mask_bits_t
-        # the bit matrices hold for this mask_mod, and while the tensors it captures are at these versions
+        # The bit matrices hold for this mask_mod, and while the tensors it captures are what they were: at
+        # these versions, and, because a version does not move with every write (`.data`, other
+        # libraries, a replayed graph), byte for byte the same as this copy of them, which every
+        # launch that would use the matrices looks at on the device.
         self._bits_mod = mask_mod
         self._bits_sources = _bits_sources
+        self._bits_snapshot = _bits_snapshot
 
     def bits_hold(self) -> bool:
-        """Whether ``mask_bits`` is still what ``mask_mod`` gives."""
+        """Whether ``mask_bits`` is still what ``mask_mod`` gives, as far as the host can see."""
         return (self.mask_bits is not None and self.mask_mod is self._bits_mod
-                and all(t._version == v for t, v in self._bits_sources))
+                and all(t is None or t._version == v for t, v in self._bits_sources))
+
+    def launch_check(self, buffers, stream) -> torch.Tensor:
+        """Queues the comparison of the captured tensors (``buffers``, on the device) with the copy taken when
+        the bit matrices were built; returns the device word it writes."""
+        hold = torch.empty(1, dtype=torch.int32, device=self.mask_bits.device)
+        addr, size, n = _cabi.ranges(buffers)
+        L = _cabi.lib()
+        if int(L.fa_snapshot_bytes(size, n)) == self._bits_snapshot.numel():
+            _cabi.check(L.fa_snapshot_holds(addr, size, n, self._bits_snapshot.data_ptr(), hold.data_ptr(), stream))
+        else:
+            hold.zero_()
+        return hold
 
     @classmethod
     def from_kv_blocks(cls, kv_num_blocks, kv_indices, full_kv_num_blocks=None, full_kv_indices=None,
@@ -222,10 +238,13 @@ class BlockMask:
                          *self._moved_bits(mv))
 
     def _moved_bits(self, fn):
-        """(mask_bits, mask_bits_t, sources) of a copy whose tensors went through ``fn``."""
+        """(mask_bits, mask_bits_t, sources, snapshot) of a copy whose tensors went through ``fn``."""
         if not self.bits_hold():
-            return None, None, ()
-        return fn(self.mask_bits), fn(self.mask_bits_t), self._bits_sources
+            return None, None, (), None
+        bits, snapshot = fn(self.mask_bits), self._bits_snapshot
+        if snapshot is not None and snapshot.device != bits.device:
+            snapshot = snapshot.to(bits.device)
+        return bits, fn(self.mask_bits_t), self._bits_sources, snapshot
 
     def shard(self, b_slice: slice, h_slice: slice) -> "BlockMask":
         """Tables of one batch x heads shard (broadcast axes are kept whole)."""
@@ -325,12 +344,12 @@ def bind_mod_buffers(module, score_mod: Optional[Callable], mask_mod: Optional[C
     ms = lower_mods(score_mod, mask_mod)
     if not ms.buffers:
         return
-    keep = _device_buffers(ms, device)
+    keep = device_buffers(ms, device)
     module.set_buffers([t.data_ptr() for t in keep])
     module._bound_buffers = keep  # the addresses stay valid at least until the next binding
 
 
-def _device_buffers(ms, device):
+def device_buffers(ms, device):
     """The captured tensors of a lowered pair on ``device``."""
     keep = []
     for t in ms.buffers:
@@ -369,9 +388,10 @@ def _require_cuda(device) -> torch.device:
 
 
 _MASK_BITS_MAX_BYTES = 64 << 20
+_SNAPSHOT_MAX_BYTES = 256 << 10  # (one CTA compares the copy at every launch that uses the matrices)
 
 
-def _wants_bits(ms, nb, nh, Q_LEN, KV_LEN, Q_BLOCK_SIZE, KV_BLOCK_SIZE, force) -> bool:
+def _wants_bits(ms, dev, nb, nh, Q_LEN, KV_LEN, Q_BLOCK_SIZE, KV_BLOCK_SIZE, force) -> bool:
     """Whether the bit matrices of a mask are built beside its tables."""
     if force is False or ms.mask is None:
         return False
@@ -379,8 +399,10 @@ def _wants_bits(ms, nb, nh, Q_LEN, KV_LEN, Q_BLOCK_SIZE, KV_BLOCK_SIZE, force) -
         return False  # blocks of part words
     if force is True:
         return True
-    if any(not isinstance(t, torch.Tensor) or t.is_inference() for t in ms.buffers):
-        return False  # no version counter: a later change of the captured tensor could not be noticed
+    if any(not isinstance(t, torch.Tensor) or t.is_inference() or t.device != dev for t in ms.buffers):
+        return False
+    if ms.buffers and _cabi.lib().fa_snapshot_bytes(*_cabi.ranges(ms.buffers)[1:]) > _SNAPSHOT_MAX_BYTES:
+        return False
     return nb * nh * Q_LEN * (KV_LEN + 127) // 128 * 16 <= _MASK_BITS_MAX_BYTES
 
 
@@ -413,9 +435,10 @@ def create_block_mask(
     flaxattention/core/blockmask.py:277-322), one entry along batch / heads when ``mask_mod`` does
     not read ``b`` / ``h``: on the partial tiles the attention kernels read a row's words instead of
     evaluating ``mask_mod`` 128 times per row.  It is built when it takes at most 64 MiB
-    (``_mask_bits=True`` / ``False`` forces it on or off), from the same evaluation as the tables.  For a
-    mask that reads captured tensors the attention calls use it only as long as these have not been
-    written to since (their version counters tell).
+    (``_mask_bits=True`` / ``False`` forces it on or off), from the same evaluation as the tables.  A mask
+    that reads captured tensors gets one when these are on the device and take at most 256 KiB; the
+    attention calls then compare them, on the device, with a copy taken here, and evaluate ``mask_mod``
+    if anything in them has changed since.
     """
     if mod_arity(mask_mod) not in (4, 5):
         raise AssertionError("mask_mod must take (b, h, q_idx, kv_idx) or (score, b, h, q_idx, kv_idx)")
@@ -449,13 +472,21 @@ def create_block_mask(
     # a mask that does not read the batch (head) index is evaluated once for all of them
     nb, nh = (B if ms.mask_reads_b else 1), (H if ms.mask_reads_h else 1)
     b0, h0 = (int(b_offset) if ms.mask_reads_b else 0), (int(h_offset) if ms.mask_reads_h else 0)
-    want_bits = _wants_bits(ms, nb, nh, Q_LEN, KV_LEN, Q_BLOCK_SIZE, KV_BLOCK_SIZE, _mask_bits)
-    sources = tuple((t, t._version) for t in ms.buffers) if want_bits and ms.buffers and not any(
-        not isinstance(t, torch.Tensor) or t.is_inference() for t in ms.buffers) else ()
-    elsewhere = any(not isinstance(t, torch.Tensor) or t.device != dev for t in ms.buffers)
+    want_bits = _wants_bits(ms, dev, nb, nh, Q_LEN, KV_LEN, Q_BLOCK_SIZE, KV_BLOCK_SIZE, _mask_bits)
+    buffers = device_buffers(ms, dev)
+    elsewhere = any(t is not x for t, x in zip(buffers, ms.buffers))
+    sources, snapshot = (), None
+    if want_bits and buffers:
+        # (an inference tensor has no version, the copy alone tells)
+        sources = tuple((t, t._version) if isinstance(t, torch.Tensor) and not t.is_inference() else (None, 0) for t in ms.buffers)
+        addr, size, n = _cabi.ranges(buffers)
+        L = _cabi.lib()
+        with torch.cuda.device(dev):
+            snapshot = torch.empty(int(L.fa_snapshot_bytes(size, n)), dtype=torch.uint8, device=dev)
+            _cabi.check(L.fa_snapshot(addr, size, n, snapshot.data_ptr(), torch.cuda.current_stream(dev).cuda_stream))
     if elsewhere:
         # captured arrays that live elsewhere: this build reads their copies on `dev`
-        host.register(None, mask, module, module.handle.value, tuple(_device_buffers(ms, dev)))
+        host.register(None, mask, module, module.handle.value, tuple(buffers))
     tables = host.build_block_mask(None, mask, dev.index, B, H, nb, nh, Q_LEN, KV_LEN, Q_BLOCK_SIZE, KV_BLOCK_SIZE, b0, h0,
                                    int(want_bits))
     if elsewhere:
@@ -464,4 +495,4 @@ def create_block_mask(
         _TABLE_CACHE[cache_key] = tables
         while len(_TABLE_CACHE) > _TABLE_CACHE_MAX:
             _TABLE_CACHE.popitem(last=False)
-    return BlockMask(*tables[:8], (Q_BLOCK_SIZE, KV_BLOCK_SIZE), mask_mod, tables[8], tables[9], sources)
+    return BlockMask(*tables[:8], (Q_BLOCK_SIZE, KV_BLOCK_SIZE), mask_mod, tables[8], tables[9], sources, snapshot)

@@ -65,7 +65,7 @@ PyObject *g_identity = nullptr, *g_noop = nullptr, *g_error = nullptr;
 // lock, so that calls with other tensors on the same module from other threads do not come between.
 std::mutex g_buffers_mu;
 
-PyObject *s_mask_mod, *s_block_size, *s_mask_bits, *s_mask_bits_t, *s_bits_mod, *s_bits_sources;
+PyObject *s_mask_mod, *s_block_size, *s_mask_bits, *s_mask_bits_t, *s_bits_mod, *s_bits_sources, *s_bits_snapshot;
 PyObject* s_tables[8];
 
 // A reference that is dropped at the end of its scope.
@@ -83,6 +83,9 @@ struct Call {
   fa_attn_params p;          // shapes, scale, offsets, tables, flags; tensors are filled in per launch
   bool bshd = false;
   std::vector<at::Tensor> tables;  // keeps the BlockMask tensors alive
+  // bit matrices over captured tensors: these tensors, and the copy of them the matrices belong to
+  std::vector<at::Tensor> sources;
+  at::Tensor snapshot;
 };
 
 fa_tensor describe(const at::Tensor& t, bool bshd) {
@@ -130,6 +133,31 @@ void check_buffers(const Mods& m, c10::Device dev) {
   for (const auto& t : m.buffers) TORCH_CHECK(t.device() == dev, "a captured tensor has moved to another device");
 }
 
+// Queues the comparison of the tensors a mask captures with what they were when its bit matrices were built; the
+// kernels launched next with `p` look at the word it writes (returned, to be kept until then).
+at::Tensor check_snapshot(const Call& c, fa_attn_params& p, c10::Device dev, void* stream) {
+  if (!c.snapshot.defined()) return {};
+  const void* src[8];
+  size_t bytes[8];
+  const int n = (int)c.sources.size();
+  for (int i = 0; i < n; ++i) {
+    const at::Tensor& t = c.sources[i];
+    int64_t span = 1;
+    for (int64_t d = 0; d < t.dim(); ++d) span += (t.size(d) - 1) * t.stride(d);
+    src[i] = t.const_data_ptr();
+    bytes[i] = t.numel() == 0 ? 0 : (size_t)span * t.element_size();
+  }
+  if (fa_snapshot_bytes(bytes, n) != (size_t)c.snapshot.numel()) {
+    p.tables.mask_bits = p.tables.mask_bits_t = nullptr;
+    return {};
+  }
+  at::Tensor hold = empty({1}, at::kInt, dev);
+  p.tables.mask_bits_hold = hold.mutable_data_ptr<int32_t>();
+  const int rc = fa_snapshot_holds(src, bytes, n, c.snapshot.const_data_ptr(), hold.mutable_data_ptr<int32_t>(), stream);
+  if (rc != FA_OK) raise(rc);
+  return hold;
+}
+
 // q, k, v -> out, lse; throws FlaxAttnError
 std::pair<at::Tensor, at::Tensor> forward(const Call& c, const at::Tensor& q, const at::Tensor& k, const at::Tensor& v) {
   const fa_attn_params& s = c.p;
@@ -144,6 +172,7 @@ std::pair<at::Tensor, at::Tensor> forward(const Call& c, const at::Tensor& q, co
   p.o = describe(out, c.bshd);
   p.lse = lse.mutable_data_ptr<float>();
   void* stream = (void*)c10::cuda::getCurrentCUDAStream(q.device().index()).stream();
+  const at::Tensor hold = check_snapshot(c, p, q.device(), stream);
   int rc = FA_OK;
   if (p.Sq <= kDecodeMaxSq && p.Skv >= kDecodeMinSkv && p.dtype != FA_F32) {
     const int splits = fa_decode_num_splits(&p, 0);
@@ -195,6 +224,8 @@ struct AttentionBackward : public torch::autograd::Node {
     const size_t bytes = fa_bwd_workspace_bytes(&p);
     at::Tensor ws = empty({(int64_t)std::max<size_t>(bytes, 16)}, at::kByte, q.device());
     void* stream = (void*)c10::cuda::getCurrentCUDAStream(q.device().index()).stream();
+    at::Tensor hold;
+    if (p.dtype == FA_F32) hold = check_snapshot(call, p, q.device(), stream);  // (the 16-bit backward reads no matrix)
     int rc;
     {
       BuffersLock buffers(*call.mods);
@@ -262,7 +293,15 @@ bool read_block_mask(PyObject* bm, PyObject* mask_mod, c10::Device dev, Call& c)
     PyObject* pair = PyTuple_GET_ITEM(src.p, i);  // (tensor, version)
     if (!PyTuple_Check(pair) || !THPVariable_Check(PyTuple_GET_ITEM(pair, 0))) return true;
     const at::Tensor& s = THPVariable_Unpack(PyTuple_GET_ITEM(pair, 0));
-    if ((long)s._version() != PyLong_AsLong(PyTuple_GET_ITEM(pair, 1))) return true;
+    if ((long)s._version() != PyLong_AsLong(PyTuple_GET_ITEM(pair, 1)) || s.device() != dev) return true;
+    c.sources.push_back(s);
+  }
+  if (!c.sources.empty()) {
+    Ref snap(PyObject_GetAttr(bm, s_bits_snapshot));
+    const at::Tensor* t = nullptr;
+    if (snap.p == nullptr) return false;
+    if (c.sources.size() > 8 || !plain_tensor(snap.p, &t) || t->device() != dev) return true;
+    c.snapshot = *t;
   }
   bool none = false;
   const int32_t* b = table(bits.p, dev, c.tables, &none);
@@ -530,5 +569,6 @@ PyMODINIT_FUNC PyInit__host(void) {
   s_mask_bits_t = PyUnicode_InternFromString("mask_bits_t");
   s_bits_mod = PyUnicode_InternFromString("_bits_mod");
   s_bits_sources = PyUnicode_InternFromString("_bits_sources");
+  s_bits_snapshot = PyUnicode_InternFromString("_bits_snapshot");
   return PyModule_Create(&kModule);
 }

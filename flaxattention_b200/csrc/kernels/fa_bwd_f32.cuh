@@ -401,6 +401,7 @@ extern "C" __global__ void __launch_bounds__(fa_bf32::NT, 1) fa_bwd_f32_kernel(c
     const int r = lane_base + lane;           // kv row inside the tile
     const fa_u32 t_row = tmem + ((fa_u32)lane_base << 16);
     const float sc2 = p.scale * FA_LOG2E;
+    const bool bits = p.t.mask_bits_t != nullptr && (p.t.mask_hold == nullptr || *p.t.mask_hold != 0);
     bool ok = true;
     int gn = 0;
     for (int itc = 0; ok; ++itc) {
@@ -421,7 +422,7 @@ extern "C" __global__ void __launch_bounds__(fa_bf32::NT, 1) fa_bwd_f32_kernel(c
         fa_u32 keep = kv < p.Skv ? 0xffffffffu : 0u;
 #if FA_HAS_MASK_MOD
         if (mode == 1 && kv < p.Skv) {
-          if (p.t.mask_bits_t != nullptr) {
+          if (bits) {
             // (the words of a row cover whole 128-query tiles of at least Sq queries)
             const long long e = (long long)(p.t.mask_B == 1 ? 0 : b) * p.t.mask_H + (p.t.mask_H == 1 ? 0 : h);
             keep = p.t.mask_bits_t[(e * p.t.mask_t_rows + kv) * p.t.mask_t_stride + (q0 >> 5)];

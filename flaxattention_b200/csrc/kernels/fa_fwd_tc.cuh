@@ -923,7 +923,7 @@ extern "C" __global__ void __launch_bounds__(fa_tc::NT, fa_tc::NQ == 1 ? 2 : 1) 
     const fa_u32 t_p = SEP_P ? tmem + ((fa_u32)lane_base << 16) + COL_P + i * 64 : t_s;
     bool ok = true;
     // (rows beyond Sq have no row in the bit matrix: their scores are never stored, the mask is evaluated)
-    const unsigned* rowbits = (p.t.mask_bits != nullptr && qi < p.Sq)
+    const unsigned* rowbits = (p.t.mask_bits != nullptr && qi < p.Sq && (p.t.mask_hold == nullptr || *p.t.mask_hold != 0))
         ? p.t.mask_bits + (((long long)(p.t.mask_B == 1 ? 0 : b) * p.t.mask_H + (p.t.mask_H == 1 ? 0 : h)) * p.t.mask_rows + qi) * p.t.mask_stride
         : nullptr;
     SoftmaxCtx c = {p, sb, t_s, t_o, t_p, i, warp, qi, gb, gh, half, p.scale * FA_LOG2E, abort_flag, sched_tile, FA_NEG_INF, 0.f, 0u, rowbits};

@@ -36,6 +36,7 @@ struct FaTables {
   const unsigned* mask_bits_t;
   long long mask_t_stride;
   int mask_t_rows;
+  const int* mask_hold;  // device word or null: 0 - the matrices do not hold any more, evaluate mask_mod
 };
 
 // Tensors a score_mod / mask_mod may capture and index (fa_module_set_buffers).  Their addresses travel

@@ -91,6 +91,9 @@ typedef struct fa_block_tables {
   const uint32_t* mask_bits_t;
   int64_t mask_bits_t_stride; /* words per row, fa_mask_bits_row_words(Q_LEN) */
   int32_t mask_bits_t_rows;   /* rows per (batch, head) entry (KV_LEN) */
+  /* Optional, with mask_bits: a device word the kernels look at before they use the matrices; 0: evaluate mask_mod
+   * (fa_snapshot_holds writes such a word). */
+  const int32_t* mask_bits_hold;
 } fa_block_tables;
 
 typedef struct fa_attn_params {
@@ -239,6 +242,14 @@ int fa_block_mask_build(fa_module* m, const fa_mask_build* mb, void* stream);
  * mask itself (create_mask, flaxattention/core/blockmask.py:277-322); this is its 1-bit form and is
  * optional: it saves the kernels the evaluation of mask_mod on partial tiles. */
 int64_t fa_mask_bits_row_words(int KV_LEN);
+
+/* Whether memory still holds what it held: n <= 8 ranges of device memory (the tensors a mask_mod captures, where
+ * bit matrices were built from them) are copied into a snapshot of fa_snapshot_bytes (device, 16-byte aligned), and
+ * later compared with it: *holds becomes 1 where every byte is the same, else 0.  One launch each. */
+size_t fa_snapshot_bytes(const size_t* bytes, int n);
+int fa_snapshot(const void* const* src, const size_t* bytes, int n, void* snapshot, void* stream);
+int fa_snapshot_holds(const void* const* src, const size_t* bytes, int n, const void* snapshot, int32_t* holds,
+                      void* stream);
 int fa_mask_bits(fa_module* m, int B, int H, int Q_LEN, int KV_LEN, int b_offset, int h_offset, uint32_t* bits,
                  void* stream);
 
