@@ -190,7 +190,7 @@ const char* const kDefaultMods =
 
 // A kernel variant of a module as a number: every launch looks its kernel up by it, and the define text
 // is only put together when the variant has to be compiled or fetched from the cache on disk.
-enum KernelId : int { kIdFwd, kIdFwdTc, kIdBwdDq, kIdBwdDkdv, kIdBwdTc, kIdBwdF32, kIdDecode, kIdMaskScan, kIdMaskClassify, kIdSelftest };
+enum KernelId : int { kIdFwd, kIdFwdRerun, kIdBwdRerun, kIdFwdTc, kIdBwdDq, kIdBwdDkdv, kIdBwdTc, kIdBwdF32, kIdDecode, kIdMaskScan, kIdMaskClassify, kIdSelftest };
 uint64_t kernel_key(KernelId id, std::initializer_list<std::pair<int, int>> fields) {  // (value, bits)
   uint64_t k = 0;
   for (auto& f : fields) k = (k << f.second) | (uint64_t)f.first;
@@ -632,6 +632,10 @@ __global__ void __launch_bounds__(128) fa_tables_kernel(const signed char* __res
 // rest.  Up to four tensors in one launch (blockIdx.y), 8 threads per row: a thread reads 32 bytes and
 // writes 16 bytes of each part.  Bound by memory: 4 bytes in and 6 out per value.
 //
+// Infinities, NaN and values near the end of the range have no such parts (inf - inf, 0 * inf), and sums of
+// products of large ones leave it.  A byte per block says whether it saw one, |x| >= 2^30 with room
+// for the products of products in the backward; the fp32 kernels launched behind then do these heads over.
+//
 // In front of the backward the same pass does the rest of its preparation: with q it clears dQ (the kernel adds
 // to it), with dO it leaves the per-row scalars nlse2 = -lse * log2(e) (-inf for rows without mass or beyond
 // Sq) and ndelta = -sum_d O * dO (0 beyond Sq), padded to whole 128-row tiles.
@@ -644,6 +648,8 @@ struct FaSplitJob {
   FaTensor o;        // with it the row scalars (ptr null: none)
   const float* lse;
   float *nlse2, *ndelta;
+  float* delta;      // [B, H, S]: sum_d O * dO, for the fp32 kernels
+  unsigned char* beyond;  // per block of 32 rows
 };
 struct FaSplitJobs {
   FaSplitJob job[4];
@@ -657,20 +663,22 @@ __global__ void __launch_bounds__(256) fa_split3_kernel(const __grid_constant__ 
   if (t == 0 && blockIdx.y == 0 && jobs.counter != nullptr) *jobs.counter = 0;
   const long long row = t >> 3;
   const int c = (int)t & 7;
-  if (row >= j.rows) return;  // (the eight threads of a row together)
   const long long bh = row / j.S_rows;
   const int s = (int)(row - bh * j.S_rows);
   const int b = (int)(bh / j.H), h = (int)(bh - (long long)b * j.H);
   auto at = [&](const FaTensor& x) {
     return (float4*)((float*)x.ptr + (long long)b * x.sb + (long long)h * x.sh + (long long)s * x.ss) + 2 * c;
   };
-  const bool valid = s < j.S;
+  const bool valid = row < j.rows && s < j.S;  // (the same for the eight threads of a row)
+  unsigned largest = 0u;
   float4 lo4 = make_float4(0.f, 0.f, 0.f, 0.f), hi4 = lo4;
   if (valid) {
     lo4 = at(j.src)[0];
     hi4 = at(j.src)[1];
     const float x[8] = {lo4.x, lo4.y, lo4.z, lo4.w, hi4.x, hi4.y, hi4.z, hi4.w};
     unsigned part[3][4];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) largest = max(largest, __float_as_uint(x[e]) & 0x7fffffffu);
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       float2 v = make_float2(x[2 * e], x[2 * e + 1]);
@@ -688,7 +696,9 @@ __global__ void __launch_bounds__(256) fa_split3_kernel(const __grid_constant__ 
     for (int k = 0; k < 3; ++k) dst[8 * k] = make_uint4(part[k][0], part[k][1], part[k][2], part[k][3]);
     if (j.clear.ptr != nullptr) at(j.clear)[0] = at(j.clear)[1] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
-  if (j.o.ptr == nullptr) return;  // (the same for the whole launch row)
+  const int any = __syncthreads_or(largest >= __float_as_uint(1073741824.f) ? 1 : 0);  // 2^30; inf and NaN are above it
+  if (threadIdx.x == 0 && row < j.rows) j.beyond[blockIdx.x] = any ? 1 : 0;
+  if (j.o.ptr == nullptr || row >= j.rows) return;
   float acc = 0.f;
   if (valid) {
     const float4 a = at(j.o)[0], d = at(j.o)[1];
@@ -701,6 +711,7 @@ __global__ void __launch_bounds__(256) fa_split3_kernel(const __grid_constant__ 
     const float l = valid ? j.lse[bh * j.S + s] : -INFINITY;
     j.nlse2[row] = l != -INFINITY ? -(l * 1.4426950408889634f) : -INFINITY;
     j.ndelta[row] = -acc;
+    if (valid) j.delta[bh * j.S + s] = acc;
   }
 }
 
@@ -1082,12 +1093,12 @@ namespace {
 
 int round_flag(int dtype, int flags) { return (dtype != FA_F32 && (flags & FA_FLAG_ROUND_SCORES)) ? 1 : 0; }
 
-int get_fwd_kernel(fa_module* m, int dtype, int D, int Dv, int flags, const FwdCfg& c, Kernel** k) {
+int get_fwd_kernel(fa_module* m, int dtype, int D, int Dv, int flags, const FwdCfg& c, Kernel** k, bool rerun = false) {
   const int rnd = round_flag(dtype, flags);
-  return get_kernel(m, kernel_key(kIdFwd, {{dtype, 2}, {D, 9}, {Dv, 9}, {c.BM, 9}, {c.BN, 9}, {c.warps, 5}, {rnd, 1}}), "fa_fwd.cuh",
+  return get_kernel(m, kernel_key(rerun ? kIdFwdRerun : kIdFwd, {{dtype, 2}, {D, 9}, {Dv, 9}, {c.BM, 9}, {c.BN, 9}, {c.warps, 5}, {rnd, 1}}), "fa_fwd.cuh",
                     [&] { return defs({{"FA_DTYPE", dtype}, {"FA_D", D}, {"FA_DV", Dv}, {"FA_BM", c.BM}, {"FA_BN", c.BN},
-                                       {"FA_WARPS", c.warps}, {"FA_ROUND_SCORES", rnd}}); },
-                    "fa_fwd_kernel", c.smem, k);
+                                       {"FA_WARPS", c.warps}, {"FA_ROUND_SCORES", rnd}, {"FA_RERUN", rerun}}); },
+                    rerun ? "fa_fwd_rerun_kernel" : "fa_fwd_kernel", c.smem, k);
 }
 int get_bwd_kernel(fa_module* m, int dtype, int D, int Dv, int flags, const BwdCfg& c, bool dq, Kernel** k) {
   const int rnd = round_flag(dtype, flags);
@@ -1096,6 +1107,12 @@ int get_bwd_kernel(fa_module* m, int dtype, int D, int Dv, int flags, const BwdC
                     [&] { return defs({{"FA_DTYPE", dtype}, {"FA_D", D}, {"FA_DV", Dv}, {"FA_BQ", c.tile}, {"FA_BK", c.tile},
                                        {"FA_WARPS", c.warps}, {"FA_ROUND_SCORES", rnd}}); },
                     dq ? "fa_bwd_dq_kernel" : "fa_bwd_dkdv_kernel", dq ? c.smem_dq : c.smem_dkdv, k);
+}
+int get_bwd_rerun_kernel(fa_module* m, int dtype, int D, int Dv, const BwdCfg& c, Kernel** k) {
+  return get_kernel(m, kernel_key(kIdBwdRerun, {{dtype, 2}, {D, 9}, {Dv, 9}, {c.tile, 9}, {c.warps, 5}}), "fa_bwd.cuh",
+                    [&] { return defs({{"FA_DTYPE", dtype}, {"FA_D", D}, {"FA_DV", Dv}, {"FA_BQ", c.tile}, {"FA_BK", c.tile},
+                                       {"FA_WARPS", c.warps}, {"FA_ROUND_SCORES", 0}, {"FA_RERUN", 1}}); },
+                    "fa_bwd_rerun_kernel", std::max(c.smem_dq, c.smem_dkdv), k);
 }
 int get_decode_kernel(fa_module* m, int dtype, int D, int Dv, int flags, const DecCfg& c, bool pack, Kernel** k) {
   const int rnd = round_flag(dtype, flags);
@@ -1189,6 +1206,18 @@ int get_fwd_tc_kernel(fa_module* m, int dtype, int D, int flags, Kernel** k, boo
                     "fa_fwd_tc_kernel", smem, k);
 }
 
+// SMs of the current device (148 on a B200; asked once per device)
+int device_sm_count() {
+  static std::atomic<int> cached[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+  int n = cached[dev].load(std::memory_order_relaxed);
+  if (n > 0) return n;
+  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+  cached[dev].store(n, std::memory_order_relaxed);
+  return n;
+}
+
 // fp32 on the tensor cores: the operands as three bf16 parts (fa_fwd_tc.cuh).
 bool tc_fwd_f32_eligible(const fa_attn_params* p) {
   if (p->flags & FA_FLAG_GENERAL_KERNELS) return false;
@@ -1204,9 +1233,12 @@ bool tc_fwd_f32_eligible(const fa_attn_params* p) {
 // bytes of a [B, H, S, 64] tensor as three bf16 parts
 size_t split3_bytes(int B, int H, int S) { return (size_t)B * H * S * 192 * 2; }
 fa_tensor split3_tensor(void* ptr, int H, int S) { return fa_tensor{ptr, (int64_t)H * S * 192, (int64_t)S * 192, 192}; }
-FaSplitJob split_job(const fa_tensor& src, void* dst, int B, int H, int S) {
+// bytes of FaParams::beyond for `rows` rows
+size_t beyond_bytes(long long rows) { return (size_t)((rows + 31) / 32 + 15) / 16 * 16; }
+FaSplitJob split_job(const fa_tensor& src, void* dst, int B, int H, int S, const unsigned char** beyond) {
   FaSplitJob j;
   memset(&j, 0, sizeof j);
+  j.beyond = (unsigned char*)*beyond;
   j.src = cvt(src); j.dst = (uint4*)dst; j.H = H; j.S = j.S_rows = S; j.rows = (long long)B * H * S;
   return j;
 }
@@ -1215,17 +1247,31 @@ int launch_split3(const FaSplitJobs& jobs, int n, void* stream) {
   for (int i = 0; i < n; ++i) rows = std::max(rows, jobs.job[i].rows);
   return launch_here("fa_split3_kernel", fa_split3_kernel, dim3((unsigned)((rows * 8 + 255) / 256), (unsigned)n), dim3(256), stream, jobs);
 }
-int launch_fwd_f32_tc(fa_module* m, const fa_attn_params* p, const FaParams& kp, void* workspace, void* stream) {
-  Kernel* k = nullptr;
+// workspace of the forward: parts of q, k, v | bytes of the blocks with values beyond them
+size_t fwd_f32_workspace(const fa_attn_params* p) {
+  const long long rq = (long long)p->B * p->Hq * p->Sq, rk = (long long)p->B * p->Hkv * p->Skv;
+  return split3_bytes(p->B, p->Hq, p->Sq) + 2 * split3_bytes(p->B, p->Hkv, p->Skv) + beyond_bytes(rq) + 2 * beyond_bytes(rk);
+}
+// CTAs per head of an fp32 kernel launched behind the ones that work on parts: about two for every SM
+unsigned rerun_ctas(int n_tiles, long long heads) { return (unsigned)std::max<long long>(1, std::min<long long>(n_tiles, 2 * device_sm_count() / heads)); }
+int launch_fwd_f32_tc(fa_module* m, const fa_attn_params* p, FaParams kp, void* workspace, void* stream) {
+  Kernel *k = nullptr, *kf = nullptr;
+  FwdCfg c;
+  if (int rc = pick_fwd(p->dtype, p->D, p->Dv, p->Sq, &kp.t, c)) return rc;
   if (int rc = get_fwd_tc_kernel(m, p->dtype, p->D, p->flags, &k)) return rc;
+  if (int rc = get_fwd_kernel(m, p->dtype, p->D, p->Dv, p->flags, c, &kf, true)) return rc;
+  kp.n_q_tiles = (p->Sq + c.BM - 1) / c.BM;
   char* ws = (char*)workspace;
   char* wk = ws + split3_bytes(p->B, p->Hq, p->Sq);
   char* wv = wk + split3_bytes(p->B, p->Hkv, p->Skv);
+  kp.beyond[0] = (unsigned char*)(wv + split3_bytes(p->B, p->Hkv, p->Skv));
+  kp.beyond[1] = kp.beyond[0] + beyond_bytes((long long)p->B * p->Hq * p->Sq);
+  kp.beyond[2] = kp.beyond[1] + beyond_bytes((long long)p->B * p->Hkv * p->Skv);
   FaSplitJobs jobs;
   memset(&jobs, 0, sizeof jobs);
-  jobs.job[0] = split_job(p->q, ws, p->B, p->Hq, p->Sq);
-  jobs.job[1] = split_job(p->k, wk, p->B, p->Hkv, p->Skv);
-  jobs.job[2] = split_job(p->v, wv, p->B, p->Hkv, p->Skv);
+  jobs.job[0] = split_job(p->q, ws, p->B, p->Hq, p->Sq, &kp.beyond[0]);
+  jobs.job[1] = split_job(p->k, wk, p->B, p->Hkv, p->Skv, &kp.beyond[1]);
+  jobs.job[2] = split_job(p->v, wv, p->B, p->Hkv, p->Skv, &kp.beyond[2]);
   if (int rc = launch_split3(jobs, 3, stream)) return rc;
   FaTcParamsHost tp;
   tp.p = kp;
@@ -1233,7 +1279,8 @@ int launch_fwd_f32_tc(fa_module* m, const fa_attn_params* p, const FaParams& kp,
   if (int rc = make_map(&tp.tk, FA_BF16, split3_tensor(wk, p->Hkv, p->Skv), 192, p->Skv, p->Hkv, p->B)) return rc;
   if (int rc = make_map(&tp.tv, FA_BF16, split3_tensor(wv, p->Hkv, p->Skv), 192, p->Skv, p->Hkv, p->B)) return rc;
   if (int rc = make_map(&tp.to, FA_F32, p->o, p->Dv, p->Sq, p->Hq, p->B)) return rc;
-  return launch(k, dim3(p->Hq, p->B, (p->Sq + 255) / 256), dim3(384), &tp, stream);
+  if (int rc = launch(k, dim3(p->Hq, p->B, (p->Sq + 255) / 256), dim3(384), &tp, stream)) return rc;
+  return launch(kf, dim3(rerun_ctas(kp.n_q_tiles, (long long)p->B * p->Hq), p->Hq, p->B), dim3(c.warps * 32), &kp, stream);
 }
 
 // Shapes the split-KV variant of the tcgen05 kernel covers (`num_splits` CTAs per (batch, head), one
@@ -1266,18 +1313,6 @@ int launch_decode_tc(fa_module* m, const fa_attn_params* p, const FaParams& kp, 
   if (int rc = make_map(&tp.tv, p->dtype, p->v, p->Dv, p->Skv, p->Hkv, p->B)) return rc;
   memset(&tp.to, 0, sizeof(tp.to));  // (the decode variant writes partial results, not the output)
   return launch(k, dim3(num_splits, p->Hq, p->B), dim3(384), &tp, stream);
-}
-
-// SMs of the current device (148 on a B200; asked once per device)
-int device_sm_count() {
-  static std::atomic<int> cached[64];
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
-  int n = cached[dev].load(std::memory_order_relaxed);
-  if (n > 0) return n;
-  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-  cached[dev].store(n, std::memory_order_relaxed);
-  return n;
 }
 
 // Query tiles of a forward CTA.  With one, two CTAs share an SM: the fixed part of a CTA is hidden and the tail of
@@ -1361,15 +1396,21 @@ bool tc_bwd_f32_eligible(const fa_attn_params* p) {
   // the pair list of an item (fa_bf32::MAXPL pairs of 64 query rows)
   return n_qtiles <= 256 && (long long)2 * n_qtiles * (p->Hq / p->Hkv) <= 512;
 }
-// workspace: parts of q, k, v, dO | nlse2 | ndelta | item counter
+// workspace: parts of q, k, v, dO | nlse2 | ndelta | item counter | delta | bytes of the blocks with values beyond the parts
 size_t bwd_f32_workspace(const fa_attn_params* p) {
-  return 2 * split3_bytes(p->B, p->Hq, p->Sq) + 2 * split3_bytes(p->B, p->Hkv, p->Skv) + 2 * rows_pad_bytes(p) + 256;
+  const long long rq = (long long)p->B * p->Hq * p->Sq, rk = (long long)p->B * p->Hkv * p->Skv;
+  return 2 * split3_bytes(p->B, p->Hq, p->Sq) + 2 * split3_bytes(p->B, p->Hkv, p->Skv) + 2 * rows_pad_bytes(p) + 256 +
+         delta_bytes(p) + beyond_bytes(rq) + 2 * beyond_bytes(rk) + rows_pad_bytes(p) / 128;
 }
-int launch_bwd_f32_tc(fa_module* m, const fa_attn_params* p, const FaParams& kp, const fa_tensor& dout, void* workspace, void* stream) {
+int launch_bwd_f32_tc(fa_module* m, const fa_attn_params* p, FaParams kp, const fa_tensor& dout, void* workspace, void* stream) {
   // must match the shared-memory map of fa_bwd_f32.cuh (fa_bf32::SMEM_BYTES)
   const int smem = 9 * 16384 + 9 * 8192 + 3 * 2 * 64 * 4 + 21 * 8 + 8 + 16 + 16 + 2 * 512 * 4 + 256 + 1024;
   Kernel* k = nullptr;
   if (int rc = get_kernel(m, kernel_key(kIdBwdF32, {}), "fa_bwd_f32.cuh", [] { return std::string(); }, "fa_bwd_f32_kernel", smem, &k)) return rc;
+  Kernel* kf = nullptr;
+  BwdCfg c{};
+  if (int rc = pick_bwd(p->dtype, p->D, p->Dv, &kp.t, c)) return rc;
+  if (int rc = get_bwd_rerun_kernel(m, p->dtype, p->D, p->Dv, c, &kf)) return rc;
   const int sq_pad = (p->Sq + 127) / 128 * 128;
   char* w[4];
   w[0] = (char*)workspace;
@@ -1378,28 +1419,36 @@ int launch_bwd_f32_tc(fa_module* m, const fa_attn_params* p, const FaParams& kp,
   w[3] = w[2] + split3_bytes(p->B, p->Hkv, p->Skv);
   float* nlse2 = (float*)(w[3] + split3_bytes(p->B, p->Hq, p->Sq));
   float* ndelta = (float*)((char*)nlse2 + rows_pad_bytes(p));
+  int* work_counter = (int*)((char*)ndelta + rows_pad_bytes(p));
+  kp.delta = (float*)((char*)work_counter + 256);
+  kp.beyond[0] = (unsigned char*)kp.delta + delta_bytes(p);
+  kp.beyond[1] = kp.beyond[0] + beyond_bytes((long long)p->B * p->Hq * p->Sq);
+  kp.beyond[2] = kp.beyond[1] + beyond_bytes((long long)p->B * p->Hkv * p->Skv);
+  kp.beyond[3] = kp.beyond[2] + beyond_bytes((long long)p->B * p->Hkv * p->Skv);
   FaBwdF32ParamsHost tp;
   tp.p = kp;
   tp.nlse2 = nlse2;
   tp.ndelta = ndelta;
-  tp.work_counter = (int*)((char*)ndelta + rows_pad_bytes(p));
+  tp.work_counter = work_counter;
   FaSplitJobs jobs;
   memset(&jobs, 0, sizeof jobs);
   jobs.counter = tp.work_counter;
-  jobs.job[0] = split_job(p->q, w[0], p->B, p->Hq, p->Sq);
+  jobs.job[0] = split_job(p->q, w[0], p->B, p->Hq, p->Sq, &kp.beyond[0]);
   jobs.job[0].clear = kp.dq;
-  jobs.job[1] = split_job(p->k, w[1], p->B, p->Hkv, p->Skv);
-  jobs.job[2] = split_job(p->v, w[2], p->B, p->Hkv, p->Skv);
-  FaSplitJob& jd = jobs.job[3] = split_job(dout, w[3], p->B, p->Hq, p->Sq);
+  jobs.job[1] = split_job(p->k, w[1], p->B, p->Hkv, p->Skv, &kp.beyond[1]);
+  jobs.job[2] = split_job(p->v, w[2], p->B, p->Hkv, p->Skv, &kp.beyond[2]);
+  FaSplitJob& jd = jobs.job[3] = split_job(dout, w[3], p->B, p->Hq, p->Sq, &kp.beyond[3]);
   jd.S_rows = sq_pad; jd.rows = (long long)p->B * p->Hq * sq_pad;
-  jd.o = kp.o; jd.lse = p->lse; jd.nlse2 = nlse2; jd.ndelta = ndelta;
+  jd.o = kp.o; jd.lse = p->lse; jd.nlse2 = nlse2; jd.ndelta = ndelta; jd.delta = kp.delta;
   if (int rc = launch_split3(jobs, 4, stream)) return rc;
   if (int rc = make_map(&tp.tq, FA_BF16, split3_tensor(w[0], p->Hq, p->Sq), 192, p->Sq, p->Hq, p->B, 64)) return rc;
   if (int rc = make_map(&tp.tk, FA_BF16, split3_tensor(w[1], p->Hkv, p->Skv), 192, p->Skv, p->Hkv, p->B)) return rc;
   if (int rc = make_map(&tp.tv, FA_BF16, split3_tensor(w[2], p->Hkv, p->Skv), 192, p->Skv, p->Hkv, p->B)) return rc;
   if (int rc = make_map(&tp.tdo, FA_BF16, split3_tensor(w[3], p->Hq, p->Sq), 192, p->Sq, p->Hq, p->B, 64)) return rc;
   const long long n_items = (long long)p->Hkv * p->B * ((p->Skv + 127) / 128);
-  return launch(k, dim3((unsigned)std::min<long long>(n_items, device_sm_count())), dim3(512), &tp, stream);
+  if (int rc = launch(k, dim3((unsigned)std::min<long long>(n_items, device_sm_count())), dim3(512), &tp, stream)) return rc;
+  const int n_tiles = (std::max(p->Sq, p->Skv) + c.tile - 1) / c.tile;
+  return launch(kf, dim3(rerun_ctas(n_tiles, (long long)p->B * p->Hkv), p->Hkv, p->B), dim3(c.warps * 32), &kp, stream);
 }
 
 // kv2: two K / V buffers and one of dS^T instead of one and two (head dim 64)
@@ -1488,7 +1537,7 @@ int fa_fwd(fa_module* m, const fa_attn_params* p, void* stream) { return fa_fwd_
 
 size_t fa_fwd_workspace_bytes(const fa_attn_params* p) {
   if (!p || p->B <= 0 || p->Hq <= 0 || p->Hkv <= 0 || p->Sq <= 0 || p->Skv <= 0 || !tc_fwd_f32_eligible(p)) return 0;
-  return split3_bytes(p->B, p->Hq, p->Sq) + 2 * split3_bytes(p->B, p->Hkv, p->Skv);
+  return fwd_f32_workspace(p);
 }
 
 int fa_fwd_ws(fa_module* m, const fa_attn_params* p, void* workspace, size_t workspace_bytes, void* stream) {

@@ -11,7 +11,7 @@
 //   dV = P^T dO, dP = dO V^T, dS = p * (dP - delta) * score_mod'(s),
 //   dQ = scale * dS K, dK = scale * dS^T Q.
 //
-// Compile-time parameters (macros): FA_DTYPE, FA_D, FA_DV, FA_BQ, FA_BK, FA_WARPS.
+// Compile-time parameters (macros): FA_DTYPE, FA_D, FA_DV, FA_BQ, FA_BK, FA_WARPS, FA_RERUN (fp32, see the end).
 // FA_BQ = 16 * FA_WARPS rows per q-tile CTA (dq kernel) and FA_BK = 16 * FA_WARPS rows per
 // kv-tile CTA (dkdv kernel); the inner tile is FA_BK resp. FA_BQ wide.
 #pragma once
@@ -65,14 +65,10 @@ constexpr int PPK = FaTile<BK, 4>::PITCH;  // fp32 staging tile [BQ][BK] (fp32 p
 constexpr int DQ_SMEM = BQ * PQ + BQ * PV + 2 * BK * PQ + 2 * BK * PV + (F32 ? BQ * PPK : 0);
 }  // namespace fa_bwd
 
-extern "C" __global__ void __launch_bounds__(fa_bwd::NT) fa_bwd_dq_kernel(const __grid_constant__ FaParams p) {
+// dQ of one query tile of one (batch, head).
+__device__ __forceinline__ void fa_bwd_dq_tile(const FaParams& p, unsigned char* smem, const int qt, const int h, const int b) {
   using namespace fa_bwd;
-  extern __shared__ __align__(128) unsigned char smem[];
-  FA_MOD_BUFS_INIT(p);
-  fa_grid_wait();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int qt = gridDim.x - 1 - blockIdx.x;
-  const int h = blockIdx.y, b = blockIdx.z;
   const int m0 = qt * BQ;
   if (m0 >= p.Sq) return;
   const int hk = h / (p.Hq / p.Hkv);
@@ -200,14 +196,10 @@ constexpr int ROWS_BYTES = 2 * BQ * 4;     // lse2 and delta of one q tile
 constexpr int DKDV_SMEM = BK * PQ + BK * PV + 2 * BQ * PQ + 2 * BQ * PV + 2 * ROWS_BYTES + (F32 ? BK * PPQ : 0);
 }  // namespace fa_bwd
 
-extern "C" __global__ void __launch_bounds__(fa_bwd::NT) fa_bwd_dkdv_kernel(const __grid_constant__ FaParams p) {
+// dK and dV of one kv tile of one (batch, kv head).
+__device__ __forceinline__ void fa_bwd_dkdv_tile(const FaParams& p, unsigned char* smem, const int kt, const int hk, const int b) {
   using namespace fa_bwd;
-  extern __shared__ __align__(128) unsigned char smem[];
-  FA_MOD_BUFS_INIT(p);
-  fa_grid_wait();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int kt = blockIdx.x;
-  const int hk = blockIdx.y, b = blockIdx.z;
   const int n0 = kt * BK;
   if (n0 >= p.Skv) return;
   const int G = p.Hq / p.Hkv;
@@ -348,3 +340,38 @@ extern "C" __global__ void __launch_bounds__(fa_bwd::NT) fa_bwd_dkdv_kernel(cons
   fa_store_tile<D, ES, NT>(dkg, p.dk.ss * ES, Qs, min(BK, p.Skv - n0), tid);
   fa_store_tile<DV, ES, NT>(dvg, p.dv.ss * ES, dOs, min(BK, p.Skv - n0), tid);
 }
+
+#if FA_RERUN
+// Behind the tensor-core kernel (fa_bwd_f32.cuh): the (batch, kv head) groups with a value that has no bf16 parts, as
+// in fa_fwd.cuh.
+extern "C" __global__ void __launch_bounds__(fa_bwd::NT) fa_bwd_rerun_kernel(const __grid_constant__ FaParams p) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  FA_MOD_BUFS_INIT(p);
+  fa_grid_wait();
+  const int hk = blockIdx.y, b = blockIdx.z, G = p.Hq / p.Hkv;
+  if (!fa_beyond_parts(p, b, hk * G, G, hk)) return;
+  const int n_kt = (p.Skv + fa_bwd::BK - 1) / fa_bwd::BK, n_qt = (p.Sq + fa_bwd::BQ - 1) / fa_bwd::BQ;
+  for (int kt = (int)blockIdx.x; kt < n_kt; kt += (int)gridDim.x) {
+    fa_bwd_dkdv_tile(p, smem, kt, hk, b);
+    __syncthreads();  // the output tiles have been read
+  }
+  for (int i = (int)blockIdx.x; i < n_qt * G; i += (int)gridDim.x) {
+    fa_bwd_dq_tile(p, smem, i / G, hk * G + i % G, b);
+    __syncthreads();
+  }
+}
+#else
+extern "C" __global__ void __launch_bounds__(fa_bwd::NT) fa_bwd_dq_kernel(const __grid_constant__ FaParams p) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  FA_MOD_BUFS_INIT(p);
+  fa_grid_wait();
+  fa_bwd_dq_tile(p, smem, gridDim.x - 1 - blockIdx.x, blockIdx.y, blockIdx.z);
+}
+
+extern "C" __global__ void __launch_bounds__(fa_bwd::NT) fa_bwd_dkdv_kernel(const __grid_constant__ FaParams p) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  FA_MOD_BUFS_INIT(p);
+  fa_grid_wait();
+  fa_bwd_dkdv_tile(p, smem, blockIdx.x, blockIdx.y, blockIdx.z);
+}
+#endif

@@ -253,6 +253,24 @@ struct FaWalk {
   }
 };
 
+// ---- fp32 values beyond the bf16 parts --------------------------------------------------
+// Whether query heads h0 .. h0 + nh - 1 of batch entry b, which share kv head hk, have a value that the bf16 parts
+// do not take (FaParams::beyond).  Called by the whole block.
+__device__ __forceinline__ bool fa_beyond_parts(const FaParams& p, int b, int h0, int nh, int hk) {
+  const int sq_pad = (p.Sq + 127) / 128 * 128;
+  int any = 0;
+#pragma unroll 1
+  for (int i = 0; i < 4; ++i) {
+    if (p.beyond[i] == nullptr) continue;
+    const bool kv = i == 1 || i == 2;
+    const long long S = kv ? p.Skv : (i == 3 ? sq_pad : p.Sq);
+    const long long head = kv ? (long long)b * p.Hkv + hk : (long long)b * p.Hq + h0;
+    const long long last = ((head + (kv ? 1 : nh)) * S - 1) >> 5;
+    for (long long w = ((head * S) >> 5) + threadIdx.x; w <= last; w += blockDim.x) any |= p.beyond[i][w];
+  }
+  return __syncthreads_or(any) != 0;
+}
+
 // ---- warp-level tile products (one m16 row tile per warp) ----------------------------
 // Accumulator layout is that of mma.sync m16n8k16: acc[nj][0..1] = row g, cols nj*8+2t+{0,1};
 // acc[nj][2..3] = row g+8, same cols (g = lane/4, t = lane%4).

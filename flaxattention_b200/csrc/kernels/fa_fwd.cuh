@@ -9,7 +9,7 @@
 // 16-bit inputs use mma.sync m16n8k16 with fp32 accumulation; fp32 inputs use plain FMA
 // so that the result is accurate to fp32 rounding.
 //
-// Compile-time parameters (macros): FA_DTYPE, FA_D, FA_DV, FA_BM, FA_BN, FA_WARPS.
+// Compile-time parameters (macros): FA_DTYPE, FA_D, FA_DV, FA_BM, FA_BN, FA_WARPS, FA_RERUN (fp32, see the end).
 // The mod fragment (fa_score_mod, fa_mask_mod, FA_HAS_*) is placed before this file.
 #pragma once
 #include "fa_common.cuh"
@@ -104,14 +104,10 @@ __device__ __forceinline__ void softmax_tile(float (&s)[WM][BN / 8][4], float (&
 
 }  // namespace fa_fwd
 
-extern "C" __global__ void __launch_bounds__(fa_fwd::NT) fa_fwd_kernel(const __grid_constant__ FaParams p) {
+// One query tile of one (batch, head).
+__device__ __forceinline__ void fa_fwd_tile(const FaParams& p, unsigned char* smem, const int qt, const int h, const int b) {
   using namespace fa_fwd;
-  extern __shared__ __align__(128) unsigned char smem[];
-  FA_MOD_BUFS_INIT(p);
-  fa_grid_wait();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int qt = gridDim.x - 1 - blockIdx.x;  // heavy (late) causal rows first
-  const int h = blockIdx.y, b = blockIdx.z;
   const int m0 = qt * BM;
   if (m0 >= p.Sq) return;
   const int hk = h / (p.Hq / p.Hkv);
@@ -345,3 +341,27 @@ extern "C" __global__ void __launch_bounds__(fa_fwd::NT) fa_fwd_kernel(const __g
     }
   }
 }
+
+#if FA_RERUN
+// Behind the tensor-core kernel (fa_fwd_tc.cuh with fp32 inputs): the heads with a value that has no bf16 parts.
+// The grid has a few CTAs per head, which go through its tiles; nearly always none has anything to do
+// (the launch then costs 3 us).
+extern "C" __global__ void __launch_bounds__(fa_fwd::NT) fa_fwd_rerun_kernel(const __grid_constant__ FaParams p) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  FA_MOD_BUFS_INIT(p);
+  fa_grid_wait();
+  const int h = blockIdx.y, b = blockIdx.z;
+  if (!fa_beyond_parts(p, b, h, 1, h / (p.Hq / p.Hkv))) return;
+  for (int qt = (int)blockIdx.x; qt < p.n_q_tiles; qt += (int)gridDim.x) {
+    fa_fwd_tile(p, smem, qt, h, b);
+    __syncthreads();  // the output tile has been read
+  }
+}
+#else
+extern "C" __global__ void __launch_bounds__(fa_fwd::NT) fa_fwd_kernel(const __grid_constant__ FaParams p) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  FA_MOD_BUFS_INIT(p);
+  fa_grid_wait();
+  fa_fwd_tile(p, smem, gridDim.x - 1 - blockIdx.x, blockIdx.y, blockIdx.z);  // heavy (late) causal rows first
+}
+#endif

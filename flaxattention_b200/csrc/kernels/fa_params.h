@@ -69,6 +69,9 @@ struct FaParams {
   float scale;
   const void* mod_buf[FA_MAX_MOD_BUFS];
   FaTables t;
+  // fp32 inputs as bf16 parts: one byte per 32 rows of q, k, v and dO, set where a value has no such parts, the
+  // rows numbered through [B, H, S] (dO, backward only: S rounded up to 128)
+  const unsigned char* beyond[4];
 };
 
 // Evaluation of mask_mod over a block grid: the class of every block and, optionally, the mask itself as
