@@ -1252,8 +1252,8 @@ size_t fwd_f32_workspace(const fa_attn_params* p) {
   const long long rq = (long long)p->B * p->Hq * p->Sq, rk = (long long)p->B * p->Hkv * p->Skv;
   return split3_bytes(p->B, p->Hq, p->Sq) + 2 * split3_bytes(p->B, p->Hkv, p->Skv) + beyond_bytes(rq) + 2 * beyond_bytes(rk);
 }
-// CTAs per head of an fp32 kernel launched behind the ones that work on parts: about two for every SM
-unsigned rerun_ctas(int n_tiles, long long heads) { return (unsigned)std::max<long long>(1, std::min<long long>(n_tiles, 2 * device_sm_count() / heads)); }
+// CTAs of an fp32 kernel launched behind the ones that work on parts: what the SMs hold, no more than tiles
+dim3 rerun_grid(long long tiles, int smem) { return dim3((unsigned)std::min<long long>(tiles, (2 * (smem + 1024) <= 228 * 1024 ? 2 : 1) * device_sm_count())); }
 int launch_fwd_f32_tc(fa_module* m, const fa_attn_params* p, FaParams kp, void* workspace, void* stream) {
   Kernel *k = nullptr, *kf = nullptr;
   FwdCfg c;
@@ -1280,7 +1280,7 @@ int launch_fwd_f32_tc(fa_module* m, const fa_attn_params* p, FaParams kp, void* 
   if (int rc = make_map(&tp.tv, FA_BF16, split3_tensor(wv, p->Hkv, p->Skv), 192, p->Skv, p->Hkv, p->B)) return rc;
   if (int rc = make_map(&tp.to, FA_F32, p->o, p->Dv, p->Sq, p->Hq, p->B)) return rc;
   if (int rc = launch(k, dim3(p->Hq, p->B, (p->Sq + 255) / 256), dim3(384), &tp, stream)) return rc;
-  return launch(kf, dim3(rerun_ctas(kp.n_q_tiles, (long long)p->B * p->Hq), p->Hq, p->B), dim3(c.warps * 32), &kp, stream);
+  return launch(kf, rerun_grid((long long)p->B * p->Hq * kp.n_q_tiles, kf->smem), dim3(c.warps * 32), &kp, stream);
 }
 
 // Shapes the split-KV variant of the tcgen05 kernel covers (`num_splits` CTAs per (batch, head), one
@@ -1448,7 +1448,7 @@ int launch_bwd_f32_tc(fa_module* m, const fa_attn_params* p, FaParams kp, const 
   const long long n_items = (long long)p->Hkv * p->B * ((p->Skv + 127) / 128);
   if (int rc = launch(k, dim3((unsigned)std::min<long long>(n_items, device_sm_count())), dim3(512), &tp, stream)) return rc;
   const int n_tiles = (std::max(p->Sq, p->Skv) + c.tile - 1) / c.tile;
-  return launch(kf, dim3(rerun_ctas(n_tiles, (long long)p->B * p->Hkv), p->Hkv, p->B), dim3(c.warps * 32), &kp, stream);
+  return launch(kf, rerun_grid((long long)p->B * p->Hkv * n_tiles, kf->smem), dim3(c.warps * 32), &kp, stream);
 }
 
 // kv2: two K / V buffers and one of dS^T instead of one and two (head dim 64)

@@ -348,16 +348,20 @@ extern "C" __global__ void __launch_bounds__(fa_bwd::NT) fa_bwd_rerun_kernel(con
   extern __shared__ __align__(128) unsigned char smem[];
   FA_MOD_BUFS_INIT(p);
   fa_grid_wait();
-  const int hk = blockIdx.y, b = blockIdx.z, G = p.Hq / p.Hkv;
-  if (!fa_beyond_parts(p, b, hk * G, G, hk)) return;
+  const int G = p.Hq / p.Hkv;
   const int n_kt = (p.Skv + fa_bwd::BK - 1) / fa_bwd::BK, n_qt = (p.Sq + fa_bwd::BQ - 1) / fa_bwd::BQ;
-  for (int kt = (int)blockIdx.x; kt < n_kt; kt += (int)gridDim.x) {
-    fa_bwd_dkdv_tile(p, smem, kt, hk, b);
-    __syncthreads();  // the output tiles have been read
-  }
-  for (int i = (int)blockIdx.x; i < n_qt * G; i += (int)gridDim.x) {
-    fa_bwd_dq_tile(p, smem, i / G, hk * G + i % G, b);
-    __syncthreads();
+  const unsigned groups = p.B * p.Hkv, per_group = max(1u, gridDim.x / groups);
+  for (unsigned u = blockIdx.x; u < groups * per_group; u += gridDim.x) {
+    const int b = u / per_group / p.Hkv, hk = u / per_group - b * p.Hkv;
+    if (!fa_beyond_parts(p, b, hk * G, G, hk)) continue;
+    for (int kt = u % per_group; kt < n_kt; kt += per_group) {
+      fa_bwd_dkdv_tile(p, smem, kt, hk, b);
+      __syncthreads();  // the output tiles have been read
+    }
+    for (int i = u % per_group; i < n_qt * G; i += per_group) {
+      fa_bwd_dq_tile(p, smem, i / G, hk * G + i % G, b);
+      __syncthreads();
+    }
   }
 }
 #else

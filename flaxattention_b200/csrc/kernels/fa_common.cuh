@@ -258,16 +258,24 @@ struct FaWalk {
 // do not take (FaParams::beyond).  Called by the whole block.
 __device__ __forceinline__ bool fa_beyond_parts(const FaParams& p, int b, int h0, int nh, int hk) {
   const int sq_pad = (p.Sq + 127) / 128 * 128;
-  int any = 0;
-#pragma unroll 1
+  const unsigned char* at[4];
+  int n[4], any = 0;
+#pragma unroll
   for (int i = 0; i < 4; ++i) {
-    if (p.beyond[i] == nullptr) continue;
     const bool kv = i == 1 || i == 2;
     const long long S = kv ? p.Skv : (i == 3 ? sq_pad : p.Sq);
     const long long head = kv ? (long long)b * p.Hkv + hk : (long long)b * p.Hq + h0;
-    const long long last = ((head + (kv ? 1 : nh)) * S - 1) >> 5;
-    for (long long w = ((head * S) >> 5) + threadIdx.x; w <= last; w += blockDim.x) any |= p.beyond[i][w];
+    const long long first = (head * S) >> 5;
+    at[i] = p.beyond[i] + first;
+    n[i] = p.beyond[i] == nullptr ? 0 : (int)((((head + (kv ? 1 : nh)) * S - 1) >> 5) - first) + 1;
   }
+  // (the first loads of all four are in flight together)
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    if ((int)threadIdx.x < n[i]) any |= at[i][threadIdx.x];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    for (int w = threadIdx.x + blockDim.x; w < n[i]; w += blockDim.x) any |= at[i][w];
   return __syncthreads_or(any) != 0;
 }
 

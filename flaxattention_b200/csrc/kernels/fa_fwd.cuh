@@ -344,17 +344,20 @@ __device__ __forceinline__ void fa_fwd_tile(const FaParams& p, unsigned char* sm
 
 #if FA_RERUN
 // Behind the tensor-core kernel (fa_fwd_tc.cuh with fp32 inputs): the heads with a value that has no bf16 parts.
-// The grid has a few CTAs per head, which go through its tiles; nearly always none has anything to do
-// (the launch then costs 3 us).
+// The grid is what the SMs hold, so that the launch costs 2-3 us when there is nothing to do, as nearly always (with
+// at least a CTA per head it was 10-15 at 512 heads): a head gets one or several CTAs, or a CTA several heads.
 extern "C" __global__ void __launch_bounds__(fa_fwd::NT) fa_fwd_rerun_kernel(const __grid_constant__ FaParams p) {
   extern __shared__ __align__(128) unsigned char smem[];
   FA_MOD_BUFS_INIT(p);
   fa_grid_wait();
-  const int h = blockIdx.y, b = blockIdx.z;
-  if (!fa_beyond_parts(p, b, h, 1, h / (p.Hq / p.Hkv))) return;
-  for (int qt = (int)blockIdx.x; qt < p.n_q_tiles; qt += (int)gridDim.x) {
-    fa_fwd_tile(p, smem, qt, h, b);
-    __syncthreads();  // the output tile has been read
+  const unsigned heads = p.B * p.Hq, per_head = max(1u, gridDim.x / heads);
+  for (unsigned u = blockIdx.x; u < heads * per_head; u += gridDim.x) {
+    const int b = u / per_head / p.Hq, h = u / per_head - b * p.Hq;
+    if (!fa_beyond_parts(p, b, h, 1, h / (p.Hq / p.Hkv))) continue;
+    for (int qt = u % per_head; qt < p.n_q_tiles; qt += per_head) {
+      fa_fwd_tile(p, smem, qt, h, b);
+      __syncthreads();  // the output tile has been read
+    }
   }
 }
 #else
