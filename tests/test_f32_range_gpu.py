@@ -71,3 +71,14 @@ def test_the_largest_values_that_keep_the_parts():
     want = torch.softmax(q.double() @ k.double().transpose(-1, -2) * 0.125, -1) @ v.double()
     assert (got[0].double() - want).abs().max().item() <= 2e-5 * want.abs().max().item()
     assert not torch.equal(got[0][0, 0], _run(q, k, v, do, {"kernels": "general"})[0][0, 0])
+
+
+@pytest.mark.parametrize("Sq,Skv", [(64, 64), (1, 1), (300, 64), (64, 65), (1, 65)])
+def test_the_forward_up_to_one_tile_of_keys(Sq, Skv):
+    """Up to 64 keys the forward is the fp32 kernel; the results agree on both sides (fp64, as in test_f32_tensor_core_gpu)."""
+    q, k, v = (t.cuda() for t in qkv(2, 2, 2, Sq, Skv, 64))
+    do = torch.randn(2, 2, Sq, 64, device="cuda", generator=torch.Generator("cuda").manual_seed(2))
+    got, general = _run(q, k, v, do, None), _run(q, k, v, do, {"kernels": "general"})
+    assert torch.equal(got[0], general[0]) == (Skv <= 64)
+    want = torch.softmax(q.double() @ k.double().transpose(-1, -2) * 0.125, -1) @ v.double()
+    assert (got[0].double() - want).abs().max().item() <= 2e-5
