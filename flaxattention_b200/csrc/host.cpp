@@ -371,6 +371,11 @@ PyObject* attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
     Py_RETURN_NONE;
   }
   p.flags = a[10] == Py_True ? FA_FLAG_ROUND_SCORES : 0;
+  const int return_lse = PyObject_IsTrue(a[8]);  // (1 and numpy.True_ too)
+  if (return_lse < 0) {
+    PyErr_Clear();
+    Py_RETURN_NONE;
+  }
   p.status = (int32_t*)g_status;
 
   // the mods: an explicit mask_mod, or the one of the BlockMask
@@ -412,7 +417,7 @@ PyObject* attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
       node->lse_ = torch::autograd::SavedVariable(lse, false);
     }
   }
-  if (a[8] != Py_True) return THPVariable_Wrap(out);
+  if (!return_lse) return THPVariable_Wrap(out);
   Ref o(THPVariable_Wrap(out)), l(THPVariable_Wrap(lse));
   if (o.p == nullptr || l.p == nullptr) return nullptr;
   return PyTuple_Pack(2, o.p, l.p);

@@ -1,0 +1,60 @@
+"""The native host path of the entry points (csrc/host.cpp) against the Python layer: which calls it takes, and that
+a call is answered alike on both.  The first call with a pair of mods goes through the Python layer, later ones are
+taken natively; ``kernel_options={}`` always goes through Python."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _inputs(B=1, Hq=2, Hkv=2, S=256, dtype=torch.float16, layout="bhsd"):
+    g = torch.Generator("cuda").manual_seed(3)
+
+    def mk(H):
+        shape = (B, H, S, 64) if layout == "bhsd" else (B, S, H, 64)
+        return torch.randn(shape, device="cuda", generator=g).to(dtype)
+
+    return mk(Hq), mk(Hkv), mk(Hkv), mk(Hq)
+
+
+def _fresh_mod():
+    return lambda score, b, h, q_idx, kv_idx: score * 1.5
+
+
+@pytest.mark.parametrize("flag", [True, 1, np.True_, "yes", False, 0, np.False_, None, ""])
+@pytest.mark.parametrize("entry", ["flax", "pallas"])
+def test_return_lse_takes_any_truth_value(flag, entry):
+    import flaxattention_b200 as fa
+
+    q, k, v, _ = _inputs()
+    f = fa.flax_attention if entry == "flax" else fa.flax_attention_pallas
+    mod = _fresh_mod()
+    first, second = (f(q, k, v, score_mod=mod, return_lse=flag) for _ in range(2))
+    assert isinstance(first, tuple) == isinstance(second, tuple) == bool(flag)
+    for a, b in zip(first, second) if flag else [(first, second)]:
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("gqa", [True, 1, np.True_])
+@pytest.mark.parametrize("layout", ["bhsd", "bshd"])
+@pytest.mark.parametrize("strided", [False, True])
+def test_both_layers_give_the_same(gqa, layout, strided):
+    """Grouped heads, both layouts, strided inputs, with gradients: native call against the Python layer's first one."""
+    import flaxattention_b200 as fa
+
+    q, k, v, do = _inputs(2, 4, 2, 200, torch.bfloat16, layout)
+    if strided:
+        q, k, v = (torch.cat((t, t), -2)[..., :t.shape[-2], :] for t in (q, k, v))
+        assert not q.is_contiguous()
+    mod, res = _fresh_mod(), []
+    for _ in range(2):
+        ts = [t.detach().requires_grad_(True) for t in (q, k, v)]
+        out, lse = fa.flax_attention_pallas(*ts, score_mod=mod, enable_gqa=gqa, bhln=layout == "bhsd", return_lse=True)
+        res.append((out.detach(), lse, *torch.autograd.grad(out, ts, do)))
+        assert not lse.requires_grad
+    for i, (a, b) in enumerate(zip(*res)):
+        if i == 2:  # dQ: no fixed order of the sums over the kv tiles
+            assert (a.float() - b.float()).norm() <= 1e-2 * b.float().norm()
+        else:
+            assert torch.equal(a, b)
