@@ -13,7 +13,10 @@
 #include <Python.h>
 
 #include <ATen/ATen.h>
+#include <ATen/TracerMode.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
@@ -244,6 +247,13 @@ bool plain_tensor(PyObject* o, const at::Tensor** t) {
   return (*t)->defined() && (*t)->is_cuda() && (*t)->has_storage() && (*t)->layout() == at::kStrided;
 }
 
+// Calls that something looks on at: a tracer, a dispatch mode, a functorch transform.  This path makes its tensors
+// and its autograd node without them, so such calls belong to the Python layer, which they see (or which refuses).
+bool watched() {
+  return at::tracer::impl::is_dispatch_enabled() || c10::impl::TorchDispatchModeTLS::any_modes_set() ||
+         c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode);
+}
+
 // int32, contiguous, on `dev`: its address, with the tensor kept in `keep`; null on failure (None gives null with *none)
 const int32_t* table(PyObject* o, c10::Device dev, std::vector<at::Tensor>& keep, bool* none) {
   *none = o == Py_None;
@@ -339,7 +349,9 @@ PyObject* attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
   }
   const at::Tensor *q, *k, *v;
   if (g_status == nullptr || *g_status != 0) Py_RETURN_NONE;
-  if (!plain_tensor(a[0], &q) || !plain_tensor(a[1], &k) || !plain_tensor(a[2], &v)) Py_RETURN_NONE;
+  if (!plain_tensor(a[0], &q) || !plain_tensor(a[1], &k) || !plain_tensor(a[2], &v) || watched()) Py_RETURN_NONE;
+  // forward-mode derivatives: there is no rule for them, which torch.autograd.Function says
+  if (q->_fw_grad(0).defined() || k->_fw_grad(0).defined() || v->_fw_grad(0).defined()) Py_RETURN_NONE;
   const at::ScalarType dt = q->scalar_type();
   if (k->scalar_type() != dt || v->scalar_type() != dt || k->device() != q->device() || v->device() != q->device()) Py_RETURN_NONE;
   if (dt != at::kHalf && dt != at::kBFloat16 && dt != at::kFloat) Py_RETURN_NONE;

@@ -58,3 +58,54 @@ def test_both_layers_give_the_same(gqa, layout, strided):
             assert (a.float() - b.float()).norm() <= 1e-2 * b.float().norm()
         else:
             assert torch.equal(a, b)
+
+
+def _dual(f, q):
+    import torch.autograd.forward_ad as ad
+
+    with ad.dual_level():
+        f(ad.make_dual(q.clone().requires_grad_(True), torch.ones_like(q)))
+
+
+def _dispatch_mode(f, q):
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    class Mode(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+
+    with Mode():
+        f(q)
+
+
+def _in_vmap(f, q):
+    w = q.clone().requires_grad_(True)
+    torch.func.vmap(lambda x: f(w).float().sum() + x)(torch.ones(3, device="cuda"))
+
+
+@pytest.mark.parametrize("where,python,refused", [
+    (lambda f, q: f(q), False, None),
+    (_dual, True, NotImplementedError),
+    (lambda f, q: torch.jit.trace(f, (q,), check_trace=False), True, Exception),  # (whether a trace of it succeeds is left open)
+    (_dispatch_mode, True, None),
+    (_in_vmap, True, RuntimeError),
+    (lambda f, q: torch.func.grad(lambda x: f(x).float().sum())(q), True, RuntimeError),
+    (lambda f, q: torch.func.vmap(f)(q[None]), True, RuntimeError),
+], ids=["plain", "dual", "jit", "mode", "in_vmap", "func_grad", "vmap"])
+@pytest.mark.filterwarnings("ignore::torch.jit.TracerWarning")
+def test_calls_that_are_watched_go_through_the_python_layer(where, python, refused, monkeypatch):
+    import flaxattention_b200 as fa
+    from flaxattention_b200 import attention
+
+    q, k, v, _ = _inputs()
+    fa.flax_attention(q, k, v)
+    seen, run = [], attention._run
+    monkeypatch.setattr(attention, "_run", lambda *a: (seen.append(1), run(*a))[1])
+    error = None
+    try:
+        where(lambda x: fa.flax_attention(x, k, v), q)
+    except Exception as e:
+        error = type(e)
+    if refused is not Exception:
+        assert error is refused
+    assert bool(seen) == python
