@@ -83,7 +83,7 @@ def _status() -> torch.Tensor:
     global _status_word
     if _status_word is None:
         _status_word = torch.zeros(1, dtype=torch.int32).pin_memory()
-        _cabi.host().setup(_status_word.data_ptr(), _identity, noop_mask, _cabi.FlaxAttnError)
+        _cabi.host().setup(_status_word.data_ptr(), _identity, noop_mask, _cabi.FlaxAttnError, check_status)
     return _status_word
 
 

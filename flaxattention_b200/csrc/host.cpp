@@ -63,7 +63,7 @@ struct PairHash {
 // All of these are read and written with the GIL held.
 std::unordered_map<std::pair<PyObject*, PyObject*>, ModsPtr, PairHash>* g_mods = nullptr;
 volatile int* g_status = nullptr;  // the process's status word (pinned host memory)
-PyObject *g_identity = nullptr, *g_noop = nullptr, *g_error = nullptr;
+PyObject *g_identity = nullptr, *g_noop = nullptr, *g_error = nullptr, *g_check_status = nullptr;
 // Launches of modules with captured buffers: the addresses are set and taken over by the launch under this
 // lock, so that calls with other tensors on the same module from other threads do not come between.
 std::mutex g_buffers_mu;
@@ -130,6 +130,20 @@ struct BuffersLock {
   err.persist();
   PyGILState_Release(g);
   throw err;
+}
+
+// What the Python layer raises when an earlier launch has reported an error in the status word
+void check_status() {
+  if (*g_status == 0) return;
+  PyGILState_STATE g = PyGILState_Ensure();
+  Ref r(PyObject_CallNoArgs(g_check_status));
+  if (r.p == nullptr) {
+    python_error err;
+    err.persist();
+    PyGILState_Release(g);
+    throw err;
+  }
+  PyGILState_Release(g);
 }
 
 void check_buffers(const Mods& m, c10::Device dev) {
@@ -212,6 +226,7 @@ struct AttentionBackward : public torch::autograd::Node {
   torch::autograd::variable_list apply(torch::autograd::variable_list&& grads) override {
     const at::Tensor q = q_.unpack(), k = k_.unpack(), v = v_.unpack(), out = out_.unpack(shared_from_this()), lse = lse_.unpack();
     at::NoGradGuard no_grad;
+    check_status();
     c10::cuda::OptionalCUDAGuard guard(q.device());
     at::Tensor dout = grads[0].defined() ? grads[0] : at::zeros_like(out);
     if (dout.stride(-1) != 1) dout = dout.contiguous();
@@ -549,10 +564,10 @@ PyObject* forget(PyObject*, PyObject* const* a, Py_ssize_t n) {
   Py_RETURN_NONE;
 }
 
-// setup(status_address, identity_score_mod, noop_mask, FlaxAttnError)
+// setup(status_address, identity_score_mod, noop_mask, FlaxAttnError, check_status)
 PyObject* setup(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  if (n != 4) {
-    PyErr_SetString(PyExc_TypeError, "setup takes 4 arguments");
+  if (n != 5) {
+    PyErr_SetString(PyExc_TypeError, "setup takes 5 arguments");
     return nullptr;
   }
   g_status = (volatile int*)PyLong_AsVoidPtr(a[0]);
@@ -560,6 +575,7 @@ PyObject* setup(PyObject*, PyObject* const* a, Py_ssize_t n) {
   g_identity = Py_NewRef(a[1]);
   g_noop = Py_NewRef(a[2]);
   g_error = Py_NewRef(a[3]);
+  g_check_status = Py_NewRef(a[4]);
   Py_RETURN_NONE;
 }
 

@@ -109,3 +109,20 @@ def test_calls_that_are_watched_go_through_the_python_layer(where, python, refus
     if refused is not Exception:
         assert error is refused
     assert bool(seen) == python
+
+
+def test_the_backward_looks_at_the_status_word():
+    """An error that an earlier launch reported is raised before the gradients are computed, once."""
+    import flaxattention_b200 as fa
+    from flaxattention_b200 import _cabi, attention
+
+    q, k, v, do = _inputs()
+    x = q.clone().requires_grad_(True)
+    for options in (None, {}):
+        for _ in range(2):
+            out = fa.flax_attention(x, k, v, kernel_options=options)
+        torch.cuda.synchronize()
+        attention._status()[0] = 1
+        with pytest.raises(_cabi.FlaxAttnError, match="status bits 0x1"):
+            torch.autograd.grad(out, x, do, retain_graph=True)
+        torch.autograd.grad(out, x, do)
