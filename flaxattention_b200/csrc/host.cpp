@@ -92,6 +92,7 @@ struct Call {
 };
 
 fa_tensor describe(const at::Tensor& t, bool bshd) {
+  TORCH_CHECK_VALUE(t.stride(3) == 1, "the head dimension must be contiguous");
   fa_tensor r;
   r.ptr = t.data_ptr();
   r.stride_b = t.stride(0);
@@ -227,6 +228,19 @@ struct AttentionBackward : public torch::autograd::Node {
     const at::Tensor q = q_.unpack(), k = k_.unpack(), v = v_.unpack(), out = out_.unpack(shared_from_this()), lse = lse_.unpack();
     at::NoGradGuard no_grad;
     check_status();
+    {
+      // (a saved-tensor hook may have given back something else than it was given)
+      const fa_attn_params& p = call.p;
+      const auto same = [&](const at::Tensor& t, int64_t H, int64_t S, int64_t D) {
+        return t.device() == q.device() && t.scalar_type() == q.scalar_type() &&
+               (call.bshd ? t.sizes() == at::IntArrayRef({p.B, S, H, D}) : t.sizes() == at::IntArrayRef({p.B, H, S, D}));
+      };
+      const auto type = p.dtype == FA_F16 ? at::kHalf : p.dtype == FA_BF16 ? at::kBFloat16 : at::kFloat;
+      TORCH_CHECK(q.is_cuda() && q.scalar_type() == type && same(q, p.Hq, p.Sq, p.D) && same(k, p.Hkv, p.Skv, p.D) &&
+                      same(v, p.Hkv, p.Skv, p.Dv) && same(out, p.Hq, p.Sq, p.Dv) && lse.device() == q.device() &&
+                      lse.scalar_type() == at::kFloat && lse.is_contiguous() && lse.numel() == (int64_t)p.B * p.Hq * p.Sq,
+                  "a saved tensor has come back with another shape, type or device");
+    }
     c10::cuda::OptionalCUDAGuard guard(q.device());
     at::Tensor dout = grads[0].defined() ? grads[0] : at::zeros_like(out);
     if (dout.stride(-1) != 1) dout = dout.contiguous();

@@ -126,3 +126,26 @@ def test_the_backward_looks_at_the_status_word():
         with pytest.raises(_cabi.FlaxAttnError, match="status bits 0x1"):
             torch.autograd.grad(out, x, do, retain_graph=True)
         torch.autograd.grad(out, x, do)
+
+
+def test_tensors_that_saved_tensor_hooks_give_back():
+    """Moved to the host and back: the same gradients; with every second value of a row twice as long: refused, as
+    such inputs are; with another type: refused."""
+    import flaxattention_b200 as fa
+
+    q, k, v, do = _inputs()
+    fa.flax_attention(q, k, v)
+    ts = [t.clone().requires_grad_(True) for t in (q, k, v)]
+    want = torch.autograd.grad(fa.flax_attention(*ts), ts, do)
+
+    def grads(pack, unpack):
+        with torch.autograd.graph.saved_tensors_hooks(pack, unpack):
+            out = fa.flax_attention(*ts)
+        return torch.autograd.grad(out, ts, do)
+
+    got = grads(lambda t: t.cpu(), lambda t: t.cuda())
+    assert torch.equal(got[1], want[1]) and torch.equal(got[2], want[2])
+    with pytest.raises(ValueError, match="head dimension must be contiguous"):
+        grads(lambda t: t, lambda t: t if t.ndim == 3 else torch.stack((t, t), -1).flatten(-2)[..., ::2])
+    with pytest.raises(RuntimeError, match="another shape, type or device"):
+        grads(lambda t: t, lambda t: t.float())
