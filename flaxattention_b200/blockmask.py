@@ -474,7 +474,6 @@ def create_block_mask(
     b0, h0 = (int(b_offset) if ms.mask_reads_b else 0), (int(h_offset) if ms.mask_reads_h else 0)
     want_bits = _wants_bits(ms, dev, nb, nh, Q_LEN, KV_LEN, Q_BLOCK_SIZE, KV_BLOCK_SIZE, _mask_bits)
     buffers = device_buffers(ms, dev)
-    elsewhere = any(t is not x for t, x in zip(buffers, ms.buffers))
     sources, snapshot = (), None
     if want_bits and buffers:
         # (an inference tensor has no version, the copy alone tells)
@@ -484,13 +483,8 @@ def create_block_mask(
         with torch.cuda.device(dev):
             snapshot = torch.empty(int(L.fa_snapshot_bytes(size, n)), dtype=torch.uint8, device=dev)
             _cabi.check(L.fa_snapshot(addr, size, n, snapshot.data_ptr(), torch.cuda.current_stream(dev).cuda_stream))
-    if elsewhere:
-        # captured arrays that live elsewhere: this build reads their copies on `dev`
-        host.register(None, mask, module, module.handle.value, tuple(buffers))
-    tables = host.build_block_mask(None, mask, dev.index, B, H, nb, nh, Q_LEN, KV_LEN, Q_BLOCK_SIZE, KV_BLOCK_SIZE, b0, h0,
-                                   int(want_bits))
-    if elsewhere:
-        host.forget(0, id(mask))
+    tables = host.build_block_mask(module.handle.value, tuple(buffers), dev.index, B, H, nb, nh, Q_LEN, KV_LEN, Q_BLOCK_SIZE,
+                                   KV_BLOCK_SIZE, b0, h0, int(want_bits))
     if cache_key is not None:
         _TABLE_CACHE[cache_key] = tables
         while len(_TABLE_CACHE) > _TABLE_CACHE_MAX:

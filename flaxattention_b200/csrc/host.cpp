@@ -112,12 +112,13 @@ at::Tensor empty_as(const at::Tensor& t) {
 struct BuffersLock {
   std::unique_lock<std::mutex> lk;
   int rc = FA_OK;
-  explicit BuffersLock(const Mods& m) {
-    if (m.buffers.empty()) return;
+  explicit BuffersLock(const Mods& m) : BuffersLock(m.module, m.buffers) {}
+  BuffersLock(fa_module* module, const std::vector<at::Tensor>& buffers) {
+    if (buffers.empty()) return;
     lk = std::unique_lock<std::mutex>(g_buffers_mu);
     const void* ptrs[8];
-    for (size_t i = 0; i < m.buffers.size(); ++i) ptrs[i] = m.buffers[i].const_data_ptr();
-    rc = fa_module_set_buffers(m.module, ptrs, (int)m.buffers.size());
+    for (size_t i = 0; i < buffers.size(); ++i) ptrs[i] = buffers[i].const_data_ptr();
+    rc = fa_module_set_buffers(module, ptrs, (int)buffers.size());
   }
 };
 
@@ -145,10 +146,6 @@ void check_status() {
     throw err;
   }
   PyGILState_Release(g);
-}
-
-void check_buffers(const Mods& m, c10::Device dev) {
-  for (const auto& t : m.buffers) TORCH_CHECK(t.device() == dev, "a captured tensor has moved to another device");
 }
 
 // Queues the comparison of the tensors a mask captures with what they were when its bit matrices were built; the
@@ -473,17 +470,29 @@ at::Tensor part(const at::Tensor& base, int64_t offset, at::IntArrayRef sizes) {
   return at::Tensor(std::move(impl));
 }
 
-// build_block_mask(score_mod, mask_mod, device, B, H, distinct_B, distinct_H, Q_LEN, KV_LEN, q_block, kv_block, b_offset,
+// The tensors of a tuple (at most 8)
+std::vector<at::Tensor> tensors(PyObject* o) {
+  TORCH_CHECK(PyTuple_Check(o) && PyTuple_GET_SIZE(o) <= 8, "buffers: a tuple of at most 8 tensors");
+  std::vector<at::Tensor> r;
+  for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(o); ++i) {
+    TORCH_CHECK(THPVariable_Check(PyTuple_GET_ITEM(o, i)), "buffers: tensors");
+    r.push_back(THPVariable_Unpack(PyTuple_GET_ITEM(o, i)));
+  }
+  return r;
+}
+
+// build_block_mask(module handle, buffers, device, B, H, distinct_B, distinct_H, Q_LEN, KV_LEN, q_block, kv_block, b_offset,
 //                  h_offset, want_bits) -> the eight tables, mask_bits, mask_bits_t
+// buffers: the tensors the mask_mod captures, on the device
 PyObject* build_block_mask(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   if (n != 14) {
     PyErr_SetString(PyExc_TypeError, "build_block_mask takes 14 arguments");
     return nullptr;
   }
-  const auto hit = g_mods->find({a[0] == Py_None ? nullptr : a[0], a[1] == Py_None ? nullptr : a[1]});
-  TORCH_CHECK(hit != g_mods->end(), "the mods are not registered");
-  const ModsPtr mods = hit->second;
+  fa_module* module = (fa_module*)PyLong_AsVoidPtr(a[0]);
+  if (PyErr_Occurred()) return nullptr;
+  const std::vector<at::Tensor> captured = tensors(a[1]);
   long x[12];
   for (int i = 0; i < 12; ++i) x[i] = PyLong_AsLong(a[2 + i]);
   if (PyErr_Occurred()) return nullptr;
@@ -493,7 +502,7 @@ PyObject* build_block_mask(PyObject*, PyObject* const* a, Py_ssize_t n) {
   mb.B = (int)x[1]; mb.H = (int)x[2]; mb.distinct_B = (int)x[3]; mb.distinct_H = (int)x[4];
   mb.Q_LEN = (int)x[5]; mb.KV_LEN = (int)x[6]; mb.q_block = (int)x[7]; mb.kv_block = (int)x[8];
   mb.b_offset = (int)x[9]; mb.h_offset = (int)x[10];
-  check_buffers(*mods, dev);
+  for (const auto& t : captured) TORCH_CHECK(t.device() == dev, "a captured tensor is on another device");
   std::vector<at::Tensor> out;
   {
     pybind11::gil_scoped_release no_gil;
@@ -525,8 +534,8 @@ PyObject* build_block_mask(PyObject*, PyObject* const* a, Py_ssize_t n) {
       mb.bits_t = (uint32_t*)out[9].mutable_data_ptr();
     }
     void* stream = (void*)c10::cuda::getCurrentCUDAStream(dev.index()).stream();
-    BuffersLock buffers(*mods);
-    const int rc = buffers.rc != FA_OK ? buffers.rc : fa_block_mask_build(mods->module, &mb, stream);
+    BuffersLock buffers(module, captured);
+    const int rc = buffers.rc != FA_OK ? buffers.rc : fa_block_mask_build(module, &mb, stream);
     if (rc != FA_OK) raise(rc);
   }
   PyObject* t = PyTuple_New(10);
@@ -554,12 +563,7 @@ PyObject* register_mods(PyObject*, PyObject* const* a, Py_ssize_t n) {
   auto m = std::make_shared<Mods>();
   m->module = (fa_module*)PyLong_AsVoidPtr(a[3]);
   if (PyErr_Occurred()) return nullptr;
-  TORCH_CHECK(PyTuple_Check(a[4]) && PyTuple_GET_SIZE(a[4]) <= 8, "buffers: a tuple of at most 8 tensors");
-  for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(a[4]); ++i) {
-    PyObject* o = PyTuple_GET_ITEM(a[4], i);
-    TORCH_CHECK(THPVariable_Check(o), "buffers: tensors");
-    m->buffers.push_back(THPVariable_Unpack(o));
-  }
+  m->buffers = tensors(a[4]);
   m->keep = Py_NewRef(a[2]);
   (*g_mods)[{a[0] == Py_None ? nullptr : a[0], a[1] == Py_None ? nullptr : a[1]}] = std::move(m);
   Py_RETURN_NONE;

@@ -149,3 +149,27 @@ def test_tensors_that_saved_tensor_hooks_give_back():
         grads(lambda t: t, lambda t: t if t.ndim == 3 else torch.stack((t, t), -1).flatten(-2)[..., ::2])
     with pytest.raises(RuntimeError, match="another shape, type or device"):
         grads(lambda t: t, lambda t: t.float())
+
+
+def test_a_captured_tensor_elsewhere_after_a_build_that_failed():
+    """create_block_mask reads a copy on the device; attention calls go on looking at the tensor itself."""
+    import flaxattention_b200 as fa
+    from flaxattention_b200 import _cabi
+
+    S = 256
+    limit = torch.full((S,), 200, dtype=torch.int32)
+
+    def up_to_limit(b, h, q_idx, kv_idx):
+        return kv_idx < limit[q_idx]
+
+    q, k, v, _ = _inputs()
+    bm = fa.create_block_mask(up_to_limit, None, None, S, S)
+    fa.flax_attention(q, k, v, block_mask=bm)
+    with pytest.raises(_cabi.FlaxAttnError):
+        fa.create_block_mask(up_to_limit, 300, 300, S, S)  # more than 65535 heads
+    for _ in range(2):
+        before = fa.flax_attention(q, k, v, block_mask=bm)
+    limit.fill_(150)
+    now = fa.flax_attention(q, k, v, block_mask=bm)
+    assert not torch.equal(now, before)
+    assert torch.equal(now, fa.flax_attention(q, k, v, block_mask=fa.create_block_mask(up_to_limit, None, None, S, S)))
