@@ -391,19 +391,23 @@ _MASK_BITS_MAX_BYTES = 64 << 20
 _SNAPSHOT_MAX_BYTES = 256 << 10  # (one CTA compares the copy at every launch that uses the matrices)
 
 
-def _wants_bits(ms, dev, nb, nh, Q_LEN, KV_LEN, Q_BLOCK_SIZE, KV_BLOCK_SIZE, force) -> bool:
-    """Whether the bit matrices of a mask are built beside its tables."""
+def _wants_bits(ms, dev, nb, nh, Q_LEN, KV_LEN, Q_BLOCK_SIZE, KV_BLOCK_SIZE, force) -> int:
+    """Bit matrices built beside the tables of a mask: 0 none, 1 the matrix, 2 the transposed one too."""
     if force is False or ms.mask is None:
-        return False
-    if (Q_LEN > Q_BLOCK_SIZE and Q_BLOCK_SIZE % 32) or (KV_LEN > KV_BLOCK_SIZE and KV_BLOCK_SIZE % 32):
-        return False  # blocks of part words
+        return 0
+    L = _cabi.lib()
+    row_major = nb * nh * Q_LEN * int(L.fa_mask_bits_row_words(KV_LEN)) * 4
+    transposed = nb * nh * KV_LEN * int(L.fa_mask_bits_row_words(Q_LEN)) * 4
+    both = 2 if row_major + transposed <= _MASK_BITS_MAX_BYTES else 1
     if force is True:
-        return True
+        return both
+    if (Q_LEN > Q_BLOCK_SIZE and Q_BLOCK_SIZE % 32) or (KV_LEN > KV_BLOCK_SIZE and KV_BLOCK_SIZE % 32):
+        return 0  # (no kernel that takes such blocks reads the matrix)
     if any(not isinstance(t, torch.Tensor) or t.is_inference() or t.device != dev for t in ms.buffers):
-        return False
-    if ms.buffers and _cabi.lib().fa_snapshot_bytes(*_cabi.ranges(ms.buffers)[1:]) > _SNAPSHOT_MAX_BYTES:
-        return False
-    return nb * nh * Q_LEN * (KV_LEN + 127) // 128 * 16 <= _MASK_BITS_MAX_BYTES
+        return 0
+    if ms.buffers and L.fa_snapshot_bytes(*_cabi.ranges(ms.buffers)[1:]) > _SNAPSHOT_MAX_BYTES:
+        return 0
+    return both if row_major <= _MASK_BITS_MAX_BYTES else 0
 
 
 def create_block_mask(
@@ -434,7 +438,8 @@ def create_block_mask(
     position where the reference's ``create_mask`` materialises a boolean,
     flaxattention/core/blockmask.py:277-322), one entry along batch / heads when ``mask_mod`` does
     not read ``b`` / ``h``: on the partial tiles the attention kernels read a row's words instead of
-    evaluating ``mask_mod`` 128 times per row.  It is built when it takes at most 64 MiB
+    evaluating ``mask_mod`` 128 times per row.  It is built when it takes at most 64 MiB, and transposed too
+    (for the fp32 backward) when both together do
     (``_mask_bits=True`` / ``False`` forces it on or off), from the same evaluation as the tables.  A mask
     that reads captured tensors gets one when these are on the device and take at most 256 KiB; the
     attention calls then compare them, on the device, with a copy taken here, and evaluate ``mask_mod``
@@ -484,7 +489,7 @@ def create_block_mask(
             snapshot = torch.empty(int(L.fa_snapshot_bytes(size, n)), dtype=torch.uint8, device=dev)
             _cabi.check(L.fa_snapshot(addr, size, n, snapshot.data_ptr(), torch.cuda.current_stream(dev).cuda_stream))
     tables = host.build_block_mask(module.handle.value, tuple(buffers), dev.index, B, H, nb, nh, Q_LEN, KV_LEN, Q_BLOCK_SIZE,
-                                   KV_BLOCK_SIZE, b0, h0, int(want_bits))
+                                   KV_BLOCK_SIZE, b0, h0, want_bits)
     if cache_key is not None:
         _TABLE_CACHE[cache_key] = tables
         while len(_TABLE_CACHE) > _TABLE_CACHE_MAX:

@@ -482,7 +482,7 @@ std::vector<at::Tensor> tensors(PyObject* o) {
 }
 
 // build_block_mask(module handle, buffers, device, B, H, distinct_B, distinct_H, Q_LEN, KV_LEN, q_block, kv_block, b_offset,
-//                  h_offset, want_bits) -> the eight tables, mask_bits, mask_bits_t
+//                  h_offset, want_bits: 0, 1 or 2 matrices) -> the eight tables, mask_bits, mask_bits_t
 // buffers: the tensors the mask_mod captures, on the device
 PyObject* build_block_mask(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
@@ -497,7 +497,7 @@ PyObject* build_block_mask(PyObject*, PyObject* const* a, Py_ssize_t n) {
   for (int i = 0; i < 12; ++i) x[i] = PyLong_AsLong(a[2 + i]);
   if (PyErr_Occurred()) return nullptr;
   const c10::Device dev(c10::kCUDA, (c10::DeviceIndex)x[0]);
-  const bool want_bits = x[11] != 0;
+  const int want_bits = (int)x[11];
   fa_mask_build mb{};
   mb.B = (int)x[1]; mb.H = (int)x[2]; mb.distinct_B = (int)x[3]; mb.distinct_H = (int)x[4];
   mb.Q_LEN = (int)x[5]; mb.KV_LEN = (int)x[6]; mb.q_block = (int)x[7]; mb.kv_block = (int)x[8];
@@ -527,15 +527,24 @@ PyObject* build_block_mask(PyObject*, PyObject* const* a, Py_ssize_t n) {
     mb.q_num_blocks = ptr[4]; mb.q_indices = ptr[5]; mb.full_q_num_blocks = ptr[6]; mb.full_q_indices = ptr[7];
     mb.workspace = work.mutable_data_ptr();
     mb.workspace_bytes = ws;
+    // the matrices come out of the same evaluation where the blocks are whole words, else out of one of their own
+    const bool apart = want_bits && ((nq > 1 && mb.q_block % 32) || (nkv > 1 && mb.kv_block % 32));
+    fa_mask_build own = mb;
+    own.kv_num_blocks = nullptr;
+    own.q_block = own.kv_block = 128;
+    fa_mask_build& with_bits = apart ? own : mb;
     if (want_bits) {
       out.push_back(empty({mb.distinct_B, mb.distinct_H, mb.Q_LEN, fa_mask_bits_row_words(mb.KV_LEN)}, at::kInt, dev));
+      with_bits.bits = (uint32_t*)out[8].mutable_data_ptr();
+    }
+    if (want_bits > 1) {
       out.push_back(empty({mb.distinct_B, mb.distinct_H, mb.KV_LEN, fa_mask_bits_row_words(mb.Q_LEN)}, at::kInt, dev));
-      mb.bits = (uint32_t*)out[8].mutable_data_ptr();
-      mb.bits_t = (uint32_t*)out[9].mutable_data_ptr();
+      with_bits.bits_t = (uint32_t*)out[9].mutable_data_ptr();
     }
     void* stream = (void*)c10::cuda::getCurrentCUDAStream(dev.index()).stream();
     BuffersLock buffers(module, captured);
-    const int rc = buffers.rc != FA_OK ? buffers.rc : fa_block_mask_build(module, &mb, stream);
+    int rc = buffers.rc != FA_OK ? buffers.rc : fa_block_mask_build(module, &mb, stream);
+    if (rc == FA_OK && apart) rc = fa_block_mask_build(module, &own, stream);
     if (rc != FA_OK) raise(rc);
   }
   PyObject* t = PyTuple_New(10);

@@ -59,3 +59,34 @@ def test_bits_over_a_captured_tensor_are_dropped_when_it_changes():
     got = fa.flax_attention(q, k, v, block_mask=bm)
     fresh = fa.flax_attention(q, k, v, block_mask=fa.create_block_mask(up_to_limit, None, None, S, S))
     assert torch.equal(got, fresh)
+
+
+def test_the_size_limit_counts_both_matrices(monkeypatch):
+    """256 x 256: 8 KiB row-major and as much transposed."""
+    import flaxattention_b200 as fa
+    from flaxattention_b200 import blockmask
+    from flaxattention_b200.masks import causal_mask
+
+    for limit, row_major, transposed in ((8191, False, False), (8192, True, False), (16383, True, False), (16384, True, True)):
+        monkeypatch.setattr(blockmask, "_MASK_BITS_MAX_BYTES", limit)
+        bm = fa.create_block_mask(causal_mask, None, None, 256, 256)
+        assert (bm.mask_bits is not None, bm.mask_bits_t is not None) == (row_major, transposed)
+        q, k, v = (torch.randn(1, 2, 256, 64, device="cuda").requires_grad_(True) for _ in range(3))
+        plain = fa.create_block_mask(causal_mask, None, None, 256, 256, _mask_bits=False)
+        grads = [torch.autograd.grad(fa.flax_attention(q, k, v, block_mask=m).sum(), (k, v)) for m in (bm, plain)]
+        assert all(torch.equal(a, b) for a, b in zip(*grads))
+
+
+@pytest.mark.parametrize("Q,KV,block", [(96, 96, (48, 48)), (192, 200, (64, 50)), (130, 300, (26, 100))])
+def test_bits_asked_for_beside_blocks_of_part_words(Q, KV, block):
+    import flaxattention_b200 as fa
+
+    bm = fa.create_block_mask(head_dependent, 1, 3, Q, KV, BLOCK_SIZE=block, _mask_bits=True)
+    want = create_block_mask_oracle(head_dependent, 1, 3, Q, KV, BLOCK_SIZE=block)
+    for k in TABLE_KEYS:
+        assert np.array_equal(getattr(bm, k).cpu().numpy(), want[k]), k
+    q, kv = np.arange(Q)[:, None], np.arange(KV)[None, :]
+    for h in range(3):
+        dense = head_dependent(0, h, q, kv)
+        assert np.array_equal(_unpack(bm.mask_bits, KV)[0, h][:Q], dense)
+        assert np.array_equal(_unpack(bm.mask_bits_t, Q)[0, h][:KV], dense.T)
