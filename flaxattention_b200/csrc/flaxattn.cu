@@ -1406,11 +1406,14 @@ size_t bwd_f32_workspace(const fa_attn_params* p) {
   return 2 * split3_bytes(p->B, p->Hq, p->Sq) + 2 * split3_bytes(p->B, p->Hkv, p->Skv) + 2 * rows_pad_bytes(p) + 256 +
          delta_bytes(p) + beyond_bytes(rq) + 2 * beyond_bytes(rk) + rows_pad_bytes(p) / 128;
 }
-int launch_bwd_f32_tc(fa_module* m, const fa_attn_params* p, FaParams kp, const fa_tensor& dout, void* workspace, void* stream) {
+int get_bwd_f32_kernel(fa_module* m, Kernel** k) {
   // must match the shared-memory map of fa_bwd_f32.cuh (fa_bf32::SMEM_BYTES)
   const int smem = 9 * 16384 + 9 * 8192 + 3 * 2 * 64 * 4 + 21 * 8 + 8 + 16 + 16 + 2 * 512 * 4 + 256 + 1024;
+  return get_kernel(m, kernel_key(kIdBwdF32, {}), "fa_bwd_f32.cuh", [] { return std::string(); }, "fa_bwd_f32_kernel", smem, k);
+}
+int launch_bwd_f32_tc(fa_module* m, const fa_attn_params* p, FaParams kp, const fa_tensor& dout, void* workspace, void* stream) {
   Kernel* k = nullptr;
-  if (int rc = get_kernel(m, kernel_key(kIdBwdF32, {}), "fa_bwd_f32.cuh", [] { return std::string(); }, "fa_bwd_f32_kernel", smem, &k)) return rc;
+  if (int rc = get_bwd_f32_kernel(m, &k)) return rc;
   Kernel* kf = nullptr;
   BwdCfg c{};
   if (int rc = pick_bwd(p->dtype, p->D, p->Dv, &kp.t, c)) return rc;
@@ -1502,7 +1505,6 @@ extern "C" {
 
 int fa_module_prepare(fa_module* m, int kind, int dtype, int D, int Dv, int Sq_hint, int Skv_hint) {
   if (!m) return fail(FA_EINVAL, "module is null");
-  (void)Skv_hint;
   Kernel* k = nullptr;
   switch (kind) {
     case FA_KIND_FWD: {
@@ -1511,15 +1513,24 @@ int fa_module_prepare(fa_module* m, int kind, int dtype, int D, int Dv, int Sq_h
       if (dtype != FA_F32 && D == Dv && (D == 64 || D == 128) && Sq_hint >= 128)
         for (int nq : {1, 2})
           if (int rc = get_fwd_tc_kernel(m, dtype, D, 0, &k, false, nq)) return rc;
+      if (dtype == FA_F32 && D == 64 && Dv == 64 && Skv_hint > 64) {
+        if (int rc = get_fwd_tc_kernel(m, dtype, D, 0, &k)) return rc;
+        if (int rc = get_fwd_kernel(m, dtype, D, Dv, 0, c, &k, true)) return rc;
+      }
       return get_fwd_kernel(m, dtype, D, Dv, 0, c, &k);
     }
     case FA_KIND_BWD: {
       BwdCfg c;
       if (int rc = pick_bwd(dtype, D, Dv, nullptr, c)) return rc;
-      if (dtype != FA_F32 && D == Dv && (D == 64 || D == 128) && Sq_hint >= 128)
+      if (dtype != FA_F32 && D == Dv && (D == 64 || D == 128) && Sq_hint >= 128) {
         if (int rc = get_bwd_tc_kernel(m, dtype, D, 0, false, &k)) return rc;
         if (D == 64)
           if (int rc = get_bwd_tc_kernel(m, dtype, D, 0, true, &k)) return rc;
+      }
+      if (dtype == FA_F32 && D == 64 && Dv == 64) {
+        if (int rc = get_bwd_f32_kernel(m, &k)) return rc;
+        if (int rc = get_bwd_rerun_kernel(m, dtype, D, Dv, c, &k)) return rc;
+      }
       if (int rc = get_bwd_kernel(m, dtype, D, Dv, 0, c, true, &k)) return rc;
       return get_bwd_kernel(m, dtype, D, Dv, 0, c, false, &k);
     }
@@ -1531,6 +1542,7 @@ int fa_module_prepare(fa_module* m, int kind, int dtype, int D, int Dv, int Sq_h
       return get_decode_kernel(m, dtype, D, Dv, 0, c, false, &k);
     }
     case FA_KIND_BLOCKMASK:
+      if (int rc = get_blockmask_kernel(m, false, &k)) return rc;
       return get_blockmask_kernel(m, true, &k);
     default:
       return fail(FA_EUNSUPPORTED, "fa_module_prepare: unknown kind");

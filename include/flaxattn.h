@@ -132,7 +132,8 @@ void fa_module_destroy(fa_module* m);
  * with different buffer sets must not overlap, and such launches cannot be stream-captured. */
 int fa_module_set_buffers(fa_module* m, const void* const* ptrs, int n);
 /* Compiles (or fetches from the cache) the kernels of one kind for a dtype / head-dim pair.
- * Needs no GPU.  seq_hint selects the tile configuration the same way a later launch would. */
+ * Needs no GPU.  The hints select the variants the same way a later launch (without FA_FLAG_ROUND_SCORES) of
+ * these lengths would; what a launch with a BlockMask of other block sizes needs is prepared beside them. */
 int fa_module_prepare(fa_module* m, int kind, int dtype, int D, int Dv, int Sq_hint, int Skv_hint);
 /* Number of kernels compiled (not fetched from a cache) since the library was loaded. */
 int fa_compile_count(void);

@@ -173,3 +173,34 @@ def test_a_captured_tensor_elsewhere_after_a_build_that_failed():
     now = fa.flax_attention(q, k, v, block_mask=bm)
     assert not torch.equal(now, before)
     assert torch.equal(now, fa.flax_attention(q, k, v, block_mask=fa.create_block_mask(up_to_limit, None, None, S, S)))
+
+
+@pytest.mark.parametrize("dtype,D,S,block", [(torch.float32, 64, 256, 128), (torch.float32, 64, 48, 48), (torch.float32, 32, 128, 128),
+                                             (torch.float16, 64, 256, 128), (torch.bfloat16, 128, 256, 128), (torch.float16, 64, 96, 96)])
+def test_a_prepared_module_compiles_nothing_at_its_first_call(dtype, D, S, block):
+    import random
+
+    import flaxattention_b200 as fa
+    from flaxattention_b200 import _cabi
+    from flaxattention_b200.blockmask import module_for
+
+    c = random.SystemRandom().random()  # (a text that no cache on disk holds)
+
+    def score(s, b, h, q_idx, kv_idx):
+        return s * c
+
+    def mask(b, h, q_idx, kv_idx):
+        return (q_idx >= kv_idx) | (q_idx * c > 1e9)
+
+    q, k, v = (torch.randn(1, 2, S, D, device="cuda").to(dtype).requires_grad_(True) for _ in range(3))
+    code = {torch.float16: _cabi.FA_F16, torch.bfloat16: _cabi.FA_BF16, torch.float32: _cabi.FA_F32}[dtype]
+    module_for(None, mask).prepare(_cabi.KIND_BLOCKMASK, code, D, D)
+    for kind in (_cabi.KIND_FWD, _cabi.KIND_BWD):
+        module_for(score, mask).prepare(kind, code, D, D, S, S)
+    before = _cabi.lib().fa_compile_count()
+    fa.create_block_mask(mask, None, None, 96, 96, BLOCK_SIZE=24)  # not whole words
+    bm = fa.create_block_mask(mask, None, None, S, S, BLOCK_SIZE=block)
+    out = fa.flax_attention_pallas(q, k, v, score_mod=score, block_mask=bm)
+    torch.autograd.grad(out.float().sum(), (q, k, v))
+    torch.cuda.synchronize()
+    assert _cabi.lib().fa_compile_count() == before
