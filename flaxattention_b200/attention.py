@@ -231,6 +231,12 @@ def _forward(call: _Call, q, k, v):
     return out, lse
 
 
+def backward_flags(dtype) -> int:
+    """With ``torch.use_deterministic_algorithms`` fp32 gradients come from the general kernels: over bf16 parts
+    dQ is added up in no fixed order."""
+    return _cabi.FLAG_GENERAL_KERNELS if dtype == torch.float32 and torch.are_deterministic_algorithms_enabled() else 0
+
+
 def _backward(call: _Call, q, k, v, out, lse, dout):
     L = _cabi.lib()
     check_status()
@@ -240,6 +246,7 @@ def _backward(call: _Call, q, k, v, out, lse, dout):
     stream = torch.cuda.current_stream(q.device).cuda_stream
     with torch.cuda.device(q.device):
         p = call.params(q, k, v, out, lse, stream)
+        p.flags |= backward_flags(q.dtype)
         nbytes = L.fa_bwd_workspace_bytes(p)
         ws = torch.empty(max(nbytes, 16), dtype=torch.uint8, device=q.device)
         bind_mod_buffers(call.module, call.score_mod, call.mask_mod, q.device)
@@ -304,6 +311,8 @@ def flax_attention(
     Returns the output in the input dtype and, with ``return_lse``, the natural-log
     logsumexp ``[B, Hq, Sq]`` in float32 (``-inf`` for fully masked rows, whose output is 0).
     ``kernel_options``: ``{"path": "fwd" | "decode", "num_splits": int, "round_scores": bool}``.
+    The gradient of ``query`` is summed over the key tiles in no fixed order (16-bit types, and fp32 of head dim
+    64 unless ``torch.use_deterministic_algorithms`` is on); everything else is the same every time.
     For fp16 / bf16 inputs the scores are rounded to the input dtype before the scale, as in
     the reference's dense path (``jnp.matmul`` in the input dtype, core/attention.py:27);
     ``round_scores=False`` keeps the fp32 product like ``flax_attention_pallas`` does.

@@ -248,6 +248,8 @@ struct AttentionBackward : public torch::autograd::Node {
     p.v = describe(v, call.bshd);
     p.o = describe(out, call.bshd);
     p.lse = (float*)lse.data_ptr();
+    // dQ over bf16 parts is added up in no fixed order; the general fp32 kernels have one
+    if (p.dtype == FA_F32 && at::globalContext().deterministicAlgorithms()) p.flags |= FA_FLAG_GENERAL_KERNELS;
     const fa_tensor gdo = describe(dout, call.bshd), gdq = describe(dq, call.bshd), gdk = describe(dk, call.bshd),
                     gdv = describe(dv, call.bshd);
     const size_t bytes = fa_bwd_workspace_bytes(&p);

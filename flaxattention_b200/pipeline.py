@@ -32,7 +32,7 @@ from typing import Callable, List, Optional, Tuple
 import torch
 
 from . import _cabi
-from .attention import _Call, _identity, check_status
+from .attention import _Call, _identity, backward_flags, check_status
 from .blockmask import BlockMask, bind_mod_buffers, noop_mask
 from .modtrace import lower_mods
 
@@ -179,7 +179,7 @@ class HostPipeline:
                 self._enqueue(torch.cuda.current_stream(self.dev), backward, *args)
                 self._warm = True
                 return
-            key = (backward,) + tuple(0 if t is None else t.data_ptr() for t in args)
+            key = (backward, backward_flags(self.dtype)) + tuple(0 if t is None else t.data_ptr() for t in args)
             g = self._graphs.get(key)
             if g is None:
                 if len(self._graphs) >= 8:
@@ -222,7 +222,9 @@ class HostPipeline:
             self.ev_fwd[i].record(self.s_cmp)
             if backward:
                 g = ent["g"]
-                _cabi.check(L.fa_bwd(self.module.handle, C.byref(ent["p"]), C.byref(g[0]), C.byref(g[1]),
+                pb = _cabi.FaAttnParams.from_buffer_copy(ent["p"])
+                pb.flags |= backward_flags(self.dtype)
+                _cabi.check(L.fa_bwd(self.module.handle, C.byref(pb), C.byref(g[0]), C.byref(g[1]),
                                      C.byref(g[2]), C.byref(g[3]), s.ws.data_ptr(), self.ws_bytes, raw))
             self.ev_cmp[i].record(self.s_cmp)
             with torch.cuda.stream(self.s_out):

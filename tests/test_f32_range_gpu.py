@@ -82,3 +82,41 @@ def test_the_forward_up_to_one_tile_of_keys(Sq, Skv):
     assert torch.equal(got[0], general[0]) == (Skv <= 64)
     want = torch.softmax(q.double() @ k.double().transpose(-1, -2) * 0.125, -1) @ v.double()
     assert (got[0].double() - want).abs().max().item() <= 2e-5
+
+
+@pytest.mark.parametrize("path", ["native", "python", "pipeline"])
+def test_gradients_are_the_same_every_time_when_asked_for(path):
+    import flaxattention_b200 as fa
+
+    B, H, S = 2, 4, 1024
+    q, k, v = (t.cuda() for t in qkv(B, H, H, S, S, 64))
+    do = torch.randn(B, H, S, 64, device="cuda", generator=torch.Generator("cuda").manual_seed(2))
+    if path == "pipeline":
+        host = [t.cpu().pin_memory() for t in (q, k, v)]
+        res = [torch.empty(B, H, S, 64).pin_memory() for _ in range(4)]
+        hdo = do.cpu().pin_memory()
+        pipe = fa.HostPipeline(B, H, H, S, S, 64, dtype=torch.float32)
+
+        def grads():
+            pipe.step(*host, *res, hdo)
+            torch.cuda.synchronize()
+            return [t.clone().cuda() for t in res[1:]]
+    else:
+        options = None if path == "native" else {}
+        ts = [t.clone().requires_grad_(True) for t in (q, k, v)]
+        for _ in range(2):
+            out = fa.flax_attention_pallas(*ts) if path == "native" else fa.flax_attention(*ts, kernel_options=options)
+
+        def grads():
+            return torch.autograd.grad(out, ts, do, retain_graph=True)
+
+    usual = grads()
+    torch.use_deterministic_algorithms(True)
+    try:
+        several = [grads() for _ in range(6)]
+    finally:
+        torch.use_deterministic_algorithms(False)
+    for g in several[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(g, several[0]))
+    for a, b in zip(usual, several[0]):
+        assert (a - b).abs().max().item() <= 2e-5 * max(1.0, b.abs().max().item())  # (as in test_f32_tensor_core_gpu)
