@@ -207,6 +207,20 @@ class _Call:
         return torch.empty(self.B, self.Sq, self.Hq, self.Dv, dtype=query.dtype, device=query.device)
 
 
+def _workspace(p, need, device):
+    """(scratch memory of a launch of ``p``, its size); where that of the fp32 kernels over bf16 parts does not
+    fit, the general kernels are asked for instead."""
+    nbytes = need(p)
+    try:
+        return torch.empty(max(nbytes, 16), dtype=torch.uint8, device=device), nbytes
+    except torch.OutOfMemoryError:
+        if p.dtype != _cabi.FA_F32 or p.flags & _cabi.FLAG_GENERAL_KERNELS:
+            raise
+    p.flags |= _cabi.FLAG_GENERAL_KERNELS
+    nbytes = need(p)
+    return torch.empty(max(nbytes, 16), dtype=torch.uint8, device=device), nbytes
+
+
 def _forward(call: _Call, q, k, v):
     L = _cabi.lib()
     check_status()
@@ -225,8 +239,7 @@ def _forward(call: _Call, q, k, v):
             ws = torch.empty(max(nbytes, 16), dtype=torch.uint8, device=q.device)
             _cabi.check(L.fa_decode(call.module.handle, p, splits, ws.data_ptr(), nbytes, stream))
         else:
-            nbytes = L.fa_fwd_workspace_bytes(p)
-            ws = torch.empty(nbytes, dtype=torch.uint8, device=q.device) if nbytes else None
+            ws, nbytes = _workspace(p, L.fa_fwd_workspace_bytes, q.device)
             _cabi.check(L.fa_fwd_ws(call.module.handle, p, _ptr(ws), nbytes, stream))
     return out, lse
 
@@ -247,8 +260,7 @@ def _backward(call: _Call, q, k, v, out, lse, dout):
     with torch.cuda.device(q.device):
         p = call.params(q, k, v, out, lse, stream)
         p.flags |= backward_flags(q.dtype)
-        nbytes = L.fa_bwd_workspace_bytes(p)
-        ws = torch.empty(max(nbytes, 16), dtype=torch.uint8, device=q.device)
+        ws, nbytes = _workspace(p, L.fa_bwd_workspace_bytes, q.device)
         bind_mod_buffers(call.module, call.score_mod, call.mask_mod, q.device)
         _cabi.check(L.fa_bwd(call.module.handle, p, _tensor(dout, call.layout), _tensor(dq, call.layout),
                              _tensor(dk, call.layout), _tensor(dv, call.layout), ws.data_ptr(), nbytes, stream))

@@ -108,6 +108,20 @@ at::Tensor empty_as(const at::Tensor& t) {
   return t.is_contiguous() ? empty(t.sizes(), t.scalar_type(), t.device()) : at::empty_like(t);
 }
 
+// The scratch memory of a launch of `p`.  The fp32 kernels over bf16 parts need up to one and a half times the inputs;
+// where that does not fit, the general kernels, which need next to none, are asked for instead.
+at::Tensor workspace(fa_attn_params& p, size_t (*need)(const fa_attn_params*), c10::Device dev, size_t& bytes) {
+  bytes = need(&p);
+  try {
+    return bytes > 0 ? empty({(int64_t)bytes}, at::kByte, dev) : at::Tensor();
+  } catch (const c10::OutOfMemoryError&) {
+    if (p.dtype != FA_F32 || (p.flags & FA_FLAG_GENERAL_KERNELS)) throw;
+  }
+  p.flags |= FA_FLAG_GENERAL_KERNELS;
+  bytes = need(&p);
+  return bytes > 0 ? empty({(int64_t)bytes}, at::kByte, dev) : at::Tensor();
+}
+
 // Holds the addresses of the captured buffers in the module for the duration of one launch.
 struct BuffersLock {
   std::unique_lock<std::mutex> lk;
@@ -198,9 +212,8 @@ std::pair<at::Tensor, at::Tensor> forward(const Call& c, const at::Tensor& q, co
     rc = buffers.rc != FA_OK ? buffers.rc
                              : fa_decode(c.mods->module, &p, splits, bytes > 0 ? ws.mutable_data_ptr() : nullptr, bytes, stream);
   } else {
-    const size_t bytes = fa_fwd_workspace_bytes(&p);
-    at::Tensor ws;
-    if (bytes > 0) ws = empty({(int64_t)bytes}, at::kByte, q.device());
+    size_t bytes = 0;
+    const at::Tensor ws = workspace(p, fa_fwd_workspace_bytes, q.device(), bytes);
     BuffersLock buffers(*c.mods);
     rc = buffers.rc != FA_OK ? buffers.rc : fa_fwd_ws(c.mods->module, &p, bytes > 0 ? ws.mutable_data_ptr() : nullptr, bytes, stream);
   }
@@ -252,8 +265,8 @@ struct AttentionBackward : public torch::autograd::Node {
     if (p.dtype == FA_F32 && at::globalContext().deterministicAlgorithms()) p.flags |= FA_FLAG_GENERAL_KERNELS;
     const fa_tensor gdo = describe(dout, call.bshd), gdq = describe(dq, call.bshd), gdk = describe(dk, call.bshd),
                     gdv = describe(dv, call.bshd);
-    const size_t bytes = fa_bwd_workspace_bytes(&p);
-    at::Tensor ws = empty({(int64_t)std::max<size_t>(bytes, 16)}, at::kByte, q.device());
+    size_t bytes = 0;
+    const at::Tensor ws = workspace(p, fa_bwd_workspace_bytes, q.device(), bytes);
     void* stream = (void*)c10::cuda::getCurrentCUDAStream(q.device().index()).stream();
     at::Tensor hold;
     if (p.dtype == FA_F32) hold = check_snapshot(call, p, q.device(), stream);  // (the 16-bit backward reads no matrix)

@@ -120,3 +120,34 @@ def test_gradients_are_the_same_every_time_when_asked_for(path):
         assert all(torch.equal(a, b) for a, b in zip(g, several[0]))
     for a, b in zip(usual, several[0]):
         assert (a - b).abs().max().item() <= 2e-5 * max(1.0, b.abs().max().item())  # (as in test_f32_tensor_core_gpu)
+
+
+@pytest.mark.parametrize("options", [None, {}])
+def test_without_room_for_the_parts(options):
+    """Forward and gradients fit where inputs and results do, as with the kernels that need no parts."""
+    import flaxattention_b200 as fa
+
+    H, S, MB = 8, 8192, 1 << 20  # 16 MiB a tensor; the parts take 72 and 96 MiB
+    q, k, v, do = (torch.randn(1, H, S, 64, device="cuda") for _ in range(4))
+    ts = [t.requires_grad_(True) for t in (q, k, v)]
+    small = [t[:, :, :256].detach().requires_grad_(True) for t in ts]
+    for o in (options, {"kernels": "general"}):
+        for _ in range(2):  # (compiled, loaded and registered)
+            torch.autograd.grad(fa.flax_attention(*small, kernel_options=o).sum(), small)
+    total = torch.cuda.get_device_properties(0).total_memory
+
+    def limit(room):
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + room * MB) / total)
+
+    try:
+        limit(40)
+        out = fa.flax_attention(*ts, kernel_options=options)
+        limit(80)
+        got = torch.autograd.grad(out, ts, do)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    ref = fa.flax_attention(*ts, kernel_options={"kernels": "general"})
+    assert torch.equal(out, ref)
+    assert all(torch.equal(a, b) for a, b in zip(got, torch.autograd.grad(ref, ts, do)))
