@@ -207,11 +207,15 @@ class Module:
             pass
 
 
+def span_bytes(t) -> int:
+    """Bytes of memory from the first to the last element of a tensor."""
+    return (1 + sum((d - 1) * s for d, s in zip(t.shape, t.stride()))) * t.element_size()
+
+
 def ranges(tensors):
     """(addresses, byte counts, number) of the memory that tensors span, as fa_snapshot takes them."""
     n = len(tensors)
-    size = [(1 + sum((d - 1) * s for d, s in zip(t.shape, t.stride()))) * t.element_size() for t in tensors]
-    return (C.c_void_p * n)(*(t.data_ptr() for t in tensors)), (C.c_size_t * n)(*size), n
+    return (C.c_void_p * n)(*(t.data_ptr() for t in tensors)), (C.c_size_t * n)(*map(span_bytes, tensors)), n
 
 
 def profile_enable(on: bool) -> None:

@@ -395,9 +395,8 @@ def _wants_bits(ms, dev, nb, nh, Q_LEN, KV_LEN, Q_BLOCK_SIZE, KV_BLOCK_SIZE, for
     """Bit matrices built beside the tables of a mask: 0 none, 1 the matrix, 2 the transposed one too."""
     if force is False or ms.mask is None:
         return 0
-    L = _cabi.lib()
-    row_major = nb * nh * Q_LEN * int(L.fa_mask_bits_row_words(KV_LEN)) * 4
-    transposed = nb * nh * KV_LEN * int(L.fa_mask_bits_row_words(Q_LEN)) * 4
+    row_major = nb * nh * Q_LEN * ((KV_LEN + 127) // 128) * 16
+    transposed = nb * nh * KV_LEN * ((Q_LEN + 127) // 128) * 16
     both = 2 if row_major + transposed <= _MASK_BITS_MAX_BYTES else 1
     if force is True:
         return both
@@ -405,7 +404,7 @@ def _wants_bits(ms, dev, nb, nh, Q_LEN, KV_LEN, Q_BLOCK_SIZE, KV_BLOCK_SIZE, for
         return 0  # (no kernel that takes such blocks reads the matrix)
     if any(not isinstance(t, torch.Tensor) or t.is_inference() or t.device != dev for t in ms.buffers):
         return 0
-    if ms.buffers and L.fa_snapshot_bytes(*_cabi.ranges(ms.buffers)[1:]) > _SNAPSHOT_MAX_BYTES:
+    if sum(_cabi.span_bytes(t) for t in ms.buffers) > _SNAPSHOT_MAX_BYTES:
         return 0
     return both if row_major <= _MASK_BITS_MAX_BYTES else 0
 
@@ -473,25 +472,20 @@ def create_block_mask(
         hit = _TABLE_CACHE.get(cache_key)
         if hit is not None:
             _TABLE_CACHE.move_to_end(cache_key)
-            return BlockMask(*hit[:8], (Q_BLOCK_SIZE, KV_BLOCK_SIZE), mask_mod, *hit[8:])
+            return BlockMask(*hit[:8], (Q_BLOCK_SIZE, KV_BLOCK_SIZE), mask_mod, hit[8], hit[9])
     # a mask that does not read the batch (head) index is evaluated once for all of them
     nb, nh = (B if ms.mask_reads_b else 1), (H if ms.mask_reads_h else 1)
     b0, h0 = (int(b_offset) if ms.mask_reads_b else 0), (int(h_offset) if ms.mask_reads_h else 0)
     want_bits = _wants_bits(ms, dev, nb, nh, Q_LEN, KV_LEN, Q_BLOCK_SIZE, KV_BLOCK_SIZE, _mask_bits)
     buffers = device_buffers(ms, dev)
-    sources, snapshot = (), None
+    sources = ()
     if want_bits and buffers:
         # (an inference tensor has no version, the copy alone tells)
         sources = tuple((t, t._version) if isinstance(t, torch.Tensor) and not t.is_inference() else (None, 0) for t in ms.buffers)
-        addr, size, n = _cabi.ranges(buffers)
-        L = _cabi.lib()
-        with torch.cuda.device(dev):
-            snapshot = torch.empty(int(L.fa_snapshot_bytes(size, n)), dtype=torch.uint8, device=dev)
-            _cabi.check(L.fa_snapshot(addr, size, n, snapshot.data_ptr(), torch.cuda.current_stream(dev).cuda_stream))
     tables = host.build_block_mask(module.handle.value, tuple(buffers), dev.index, B, H, nb, nh, Q_LEN, KV_LEN, Q_BLOCK_SIZE,
                                    KV_BLOCK_SIZE, b0, h0, want_bits)
     if cache_key is not None:
         _TABLE_CACHE[cache_key] = tables
         while len(_TABLE_CACHE) > _TABLE_CACHE_MAX:
             _TABLE_CACHE.popitem(last=False)
-    return BlockMask(*tables[:8], (Q_BLOCK_SIZE, KV_BLOCK_SIZE), mask_mod, tables[8], tables[9], sources, snapshot)
+    return BlockMask(*tables[:8], (Q_BLOCK_SIZE, KV_BLOCK_SIZE), mask_mod, tables[8], tables[9], sources, tables[10])

@@ -162,27 +162,34 @@ void check_status() {
   PyGILState_Release(g);
 }
 
+// The memory that tensors span, as fa_snapshot takes it (at most 8)
+struct Ranges {
+  const void* src[8];
+  size_t bytes[8];
+  int n;
+  explicit Ranges(const std::vector<at::Tensor>& ts) : n((int)ts.size()) {
+    for (int i = 0; i < n; ++i) {
+      const at::Tensor& t = ts[i];
+      int64_t span = 1;
+      for (int64_t d = 0; d < t.dim(); ++d) span += (t.size(d) - 1) * t.stride(d);
+      src[i] = t.const_data_ptr();
+      bytes[i] = t.numel() == 0 ? 0 : (size_t)span * t.element_size();
+    }
+  }
+};
+
 // Queues the comparison of the tensors a mask captures with what they were when its bit matrices were built; the
 // kernels launched next with `p` look at the word it writes (returned, to be kept until then).
 at::Tensor check_snapshot(const Call& c, fa_attn_params& p, c10::Device dev, void* stream) {
   if (!c.snapshot.defined()) return {};
-  const void* src[8];
-  size_t bytes[8];
-  const int n = (int)c.sources.size();
-  for (int i = 0; i < n; ++i) {
-    const at::Tensor& t = c.sources[i];
-    int64_t span = 1;
-    for (int64_t d = 0; d < t.dim(); ++d) span += (t.size(d) - 1) * t.stride(d);
-    src[i] = t.const_data_ptr();
-    bytes[i] = t.numel() == 0 ? 0 : (size_t)span * t.element_size();
-  }
-  if (fa_snapshot_bytes(bytes, n) != (size_t)c.snapshot.numel()) {
+  const Ranges r(c.sources);
+  if (fa_snapshot_bytes(r.bytes, r.n) != (size_t)c.snapshot.numel()) {
     p.tables.mask_bits = p.tables.mask_bits_t = nullptr;
     return {};
   }
   at::Tensor hold = empty({1}, at::kInt, dev);
   p.tables.mask_bits_hold = hold.mutable_data_ptr<int32_t>();
-  const int rc = fa_snapshot_holds(src, bytes, n, c.snapshot.const_data_ptr(), hold.mutable_data_ptr<int32_t>(), stream);
+  const int rc = fa_snapshot_holds(r.src, r.bytes, r.n, c.snapshot.const_data_ptr(), hold.mutable_data_ptr<int32_t>(), stream);
   if (rc != FA_OK) raise(rc);
   return hold;
 }
@@ -497,7 +504,8 @@ std::vector<at::Tensor> tensors(PyObject* o) {
 }
 
 // build_block_mask(module handle, buffers, device, B, H, distinct_B, distinct_H, Q_LEN, KV_LEN, q_block, kv_block, b_offset,
-//                  h_offset, want_bits: 0, 1 or 2 matrices) -> the eight tables, mask_bits, mask_bits_t
+//                  h_offset, want_bits: 0, 1 or 2 matrices) -> the eight tables, mask_bits, mask_bits_t, copy of the buffers if
+//                  there are matrices
 // buffers: the tensors the mask_mod captures, on the device
 PyObject* build_block_mask(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
@@ -557,15 +565,22 @@ PyObject* build_block_mask(PyObject*, PyObject* const* a, Py_ssize_t n) {
       with_bits.bits_t = (uint32_t*)out[9].mutable_data_ptr();
     }
     void* stream = (void*)c10::cuda::getCurrentCUDAStream(dev.index()).stream();
+    out.resize(10);
+    if (want_bits && !captured.empty()) {
+      const Ranges r(captured);
+      out.push_back(empty({(int64_t)fa_snapshot_bytes(r.bytes, r.n)}, at::kByte, dev));
+      const int rc = fa_snapshot(r.src, r.bytes, r.n, out.back().mutable_data_ptr(), stream);
+      if (rc != FA_OK) raise(rc);
+    }
     BuffersLock buffers(module, captured);
     int rc = buffers.rc != FA_OK ? buffers.rc : fa_block_mask_build(module, &mb, stream);
     if (rc == FA_OK && apart) rc = fa_block_mask_build(module, &own, stream);
     if (rc != FA_OK) raise(rc);
   }
-  PyObject* t = PyTuple_New(10);
+  PyObject* t = PyTuple_New(11);
   if (t == nullptr) return nullptr;
-  for (int i = 0; i < 10; ++i) {
-    PyObject* o = i < (int)out.size() ? THPVariable_Wrap(out[i]) : Py_NewRef(Py_None);
+  for (int i = 0; i < 11; ++i) {
+    PyObject* o = i < (int)out.size() && out[i].defined() ? THPVariable_Wrap(out[i]) : Py_NewRef(Py_None);
     if (o == nullptr) {
       Py_DECREF(t);
       return nullptr;
