@@ -1293,11 +1293,12 @@ bool tc_decode_eligible(const fa_attn_params* p) {
   if (p->flags & FA_FLAG_GENERAL_KERNELS) return false;
   if (p->dtype == FA_F32) return false;
   if (p->D != 64 || p->Dv != 64) return false;
-  // The kernel gives every query row two threads (64 kv columns of a tile each), whatever Sq is:
-  // measured on B32 H8 Skv16384 against the general decode kernel it takes 0.225 ms at 64 rows
-  // (general: 0.55), 0.209 at 16 (general: 0.231), 0.209 at 2 and 0.208 at 1 (general: 0.206): it
-  // streams K / V through TMA and a five-stage ring at the same rate whatever the row count, so it
-  // takes everything from two rows up.
+  // The kernel gives every query row two threads (64 kv columns of a tile each), whatever Sq is: it streams K / V
+  // through TMA and a five-stage ring at the same rate whatever the row count, and takes everything from two rows up.
+  // Measured against the general decode kernel (us, this one / general): B32 H8 Skv16384 226 / 378 at 64 rows,
+  // 214 / 251 at 32, 207 / 192 at 16, 206 / 188 at 2; B1 H8 Skv32768 38 / 54 at 2 to 64 rows; B8 H8 Skv4096 28 / 31 at
+  // 2, 30 / 42 at 64; but B32 H8 Skv2048 56 / 42 at 2, 58 / 43 at 32, 64 / 59 at 64, B4 H32 Skv8192 93 / 77 at 2,
+  // 95 / 91 at 32, 105 / 129 at 64: with many heads and up to 16 rows the general kernel has become the faster one.
   if (p->Sq < 2 || p->Sq > 64 || p->Skv < 1024 || p->Skv > 32768) return false;
   if (!(p->scale > 0.f)) return false;
   const fa_block_tables& t = p->tables;
@@ -1321,9 +1322,15 @@ int launch_decode_tc(fa_module* m, const fa_attn_params* p, const FaParams& kp, 
 
 // Query tiles of a forward CTA.  With one, two CTAs share an SM: the fixed part of a CTA is hidden and the tail of
 // the grid is shorter, but a step costs more (K and V are loaded per 128 rows, and with D = 128 the products of
-// the two CTAs of an SM are not kept in turn).  So it is one where a CTA has few steps or there are no more tiles
-// than SMs (us, two against one; D = 64: B8 H8 S2048 dense 121 / 118, causal 87 / 83, B8 H8 S512 causal 19.3 / 17.8,
-// B4 H8 S333 16.4 / 14.3, but B2 H8 S4096 causal 61 / 64, dense 111 / 119; D = 128: S1024 49 / 51, S4096 268 / 282).
+// the two CTAs of an SM are not kept in turn).  So it is one where there are no more tiles than SMs, and at D = 64
+// up to 2048 keys.  Forward alone, us, two against one:
+//   at most 148 tiles  D = 64 : S1024 22.5 / 18.4, S2048 32.8 / 28.7, S8192 100 / 84, S16384 189 / 157
+//                      D = 128: S1024 24.6 / 23.4, S2048 41.0 / 38.9, S8192 127 / 121, S16384 242 / 229
+//   more, D = 64       dense S2048 121 / 115, S2560 107 / 100, S3072 126 / 133, S4096 109 / 118;
+//                      causal S2048 78 / 76, S2560 59 / 57, S3072 77 / 76, S4096 62 / 64
+//   more, D = 128      dense S2048 152 / 152, S3072 160 / 164, S4096 139 / 145; causal 98 / 94, 98 / 98, 80 / 82
+// The dense lengths cross between 2560 and 3072 keys.  A mask that leaves few steps of many keys would rather have one
+// (window of 256: S4096 33.5 / 31.5, S8192 60 / 52, at D = 128 42 / 39, 77 / 66), but the host does not know the steps.
 int fwd_tc_query_tiles(const fa_attn_params* p) {
   const long long tiles = (long long)p->B * p->Hq * ((p->Sq + 127) / 128);
   return (p->D == 64 && p->Skv <= 2048) || tiles <= device_sm_count() ? 1 : 2;

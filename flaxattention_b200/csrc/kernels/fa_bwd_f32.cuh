@@ -3,7 +3,7 @@
 // parts, hi + mid + lo, which hold all the mantissa bits of an fp32 value; a product is the six bf16
 // products of parts above 2^-25 of the largest, accumulated in fp32 (fa_fwd_tc.cuh describes the form).
 // q, k, v and dO come as rows [hi | mid | lo] from a small kernel in front of this one, P and dS are split
-// by the threads that compute them.
+// by the threads that compute them.  Heads with a value that has no parts are done over by fa_bwd_rerun_kernel.
 //
 // A pair is 128 kv rows x 64 query rows.  What shapes the kernel:
 //   * Shared memory: the parts of K, V (96 KB), dS (48 KB) and three Q / dO tiles (72 KB).  Q and dO tiles pass

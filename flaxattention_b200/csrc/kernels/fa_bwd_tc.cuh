@@ -118,7 +118,6 @@ constexpr int OFF_CLS = OFF_PAIR + 2 * MAXPL * 4;           // unsigned cls[2][M
 constexpr int SMEM_BYTES = OFF_CLS + 2 * MAXC / 8 + 1024;
 // (the pointers of up to eight captured buffers are static shared memory beside this)
 static_assert(SMEM_BYTES + 8 * 8 <= 227 * 1024, "shared memory");
-static_assert(SMEM_BYTES <= 227 * 1024, "shared memory");
 constexpr int TMEM_COLS = 512;
 constexpr int COL_S = 0, COL_DP = BQ, COL_P = 2 * BQ;
 constexpr int COL_DQ = D == 64 ? 448 : 192;

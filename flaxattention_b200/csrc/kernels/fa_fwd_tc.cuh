@@ -18,7 +18,10 @@
 // accumulator without rounding to nearest, so nothing is accumulated there for long: the P.V product
 // of every kv step starts from zero and the softmax threads add it to the output row they keep in
 // registers (with O accumulated in TMEM over all steps the error grew to five times that of the FMA
-// kernel at 1024 keys).  The softmax keeps the operations and their order of fa_fwd.cuh.
+// kernel at 1024 keys).  The softmax keeps the operations and their order of fa_fwd.cuh.  Error against 64 bits
+// (2-norm of the difference over that of the output): 1.7e-7 to 3.7e-7 where the FMA kernel has 3.3e-7 to 1.2e-6
+// (97 to 4096 keys).  Infinities, NaN and |x| >= 2^30 have no parts that give the right result (inf - inf, 0 * inf, sums
+// that leave the range): the split kernel notes them, and fa_fwd_rerun_kernel does those heads over.
 //
 // One CTA owns two 128-row query tiles of one (batch, head) and streams 128-row K/V tiles
 // past both (or one, see NQ: then without warps 4-7, and the roles below move up).  Warp roles (12 warps = 3 warpgroups):
