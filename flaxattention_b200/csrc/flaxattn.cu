@@ -1478,9 +1478,10 @@ int get_bwd_tc_kernel(fa_module* m, int dtype, int D, int flags, bool kv2, Kerne
                     "fa_bwd_tc_kernel", smem, k);
 }
 
-// With a BlockMask the items are short or uneven and the variant with two K / V buffers wins: under a causal
-// mask (us, against two dS^T buffers) 35 / 38 at S=512 (B8 H8), 174 / 190 at 2048, 233 / 233 at 8192 (B1 H8).
-// Without one every item has all the q tiles and two dS^T buffers win.
+// With a BlockMask the items are short or uneven and the variant with two K / V buffers wins or ties (us, against two
+// dS^T buffers): causal S512 35.8 / 35.8, S1024 64.5 / 66.6, S2048 150.5 / 154.6 (B8 H8), S4096 136 / 138, S6144 261 /
+// 261 (B2 H8); at 64 q tiles it loses, causal S8192 230 / 228 (B1 H8), attention sink S8192 247 / 239 (B2 H8).  Without
+// one every item has all the q tiles and two dS^T buffers win.
 bool bwd_tc_kv2(const fa_attn_params* p) {
   if (p->D != 64 || !p->tables.kv_num_blocks) return false;
   return (long long)((p->Sq + 127) / 128) * (p->Hq / p->Hkv) <= 64;
