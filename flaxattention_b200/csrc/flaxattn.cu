@@ -367,13 +367,20 @@ cudaLaunchConfig_t launch_config(dim3 grid, dim3 block, int smem, void* stream, 
   cfg.numAttrs = 1;
   return cfg;
 }
-int launch(Kernel* k, dim3 grid, dim3 block, void* params, void* stream) {
+// cluster: CTAs along x that make a thread-block cluster (grid.x is a multiple of it)
+int launch(Kernel* k, dim3 grid, dim3 block, void* params, void* stream, int cluster = 1) {
   if (int rc = ready_kernel(k)) return rc;
   if (int rc = upload_buffers(k, stream)) return rc;
   void* args[] = {params};
   ProfScope prof(k->entry.c_str(), stream);
-  cudaLaunchAttribute attr;
-  const cudaLaunchConfig_t cfg = launch_config(grid, block, k->smem, stream, &attr);
+  cudaLaunchAttribute attr[2];
+  cudaLaunchConfig_t cfg = launch_config(grid, block, k->smem, stream, attr);
+  if (cluster > 1) {
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = (unsigned)cluster;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.numAttrs = 2;
+  }
   FA_CUDA_CHECK(cudaLaunchKernelExC(&cfg, (const void*)k->fn, args));
   return FA_OK;
 }
@@ -938,10 +945,10 @@ __global__ void fa_dq_convert_t_kernel(const float* __restrict__ acc, FaTensor d
   }
 }
 
-// Combines the per-split partial results of the decode kernels: one warp per output row.  Lane s
-// takes the (max, sum) pair of split s and its weight 2^(m_s - m*), 32 splits at a time; the
-// weights then go round by shuffle while every lane accumulates its output columns, each read of
-// a partial row being one contiguous run of floats.
+// Combines the per-split partial results of the decode kernels: one warp per output row.  Lane s takes the (max, sum)
+// pair of split s and its weight 2^(m_s - m*), 32 splits at a time; the weights then go round by shuffle.  A lane owns four
+// columns, and where the row has fewer than 128 the warp takes several splits at once; the reads of eight rounds
+// are under way together (one at a time, the latency of each was paid in turn: half a microsecond per split).
 template <int DT>
 __global__ void fa_decode_combine_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
                                          FaTensor o, float* __restrict__ lse, int Hq, int Sq, int Dv, int ns,
@@ -959,10 +966,13 @@ __global__ void fa_decode_combine_kernel(const float* __restrict__ part_o, const
     if (s0 + lane < ns) mstar = fmaxf(mstar, part_ml[prow(s0 + lane) * 2]);
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) mstar = fmaxf(mstar, __shfl_xor_sync(0xffffffffu, mstar, off));
-  constexpr int MAXC = 8;  // output columns per lane: head dims up to 256
-  float acc[MAXC];
-#pragma unroll
-  for (int c = 0; c < MAXC; ++c) acc[c] = 0.f;
+  const int groups = Dv >> 2;                           // of four columns
+  const int per = groups < 32 ? groups : 32;            // lanes of a split
+  const int sub = 32 / per, mine = lane / per;          // splits at once; this lane's (beyond sub: idle)
+  const int c0 = (lane - mine * per) * 4;               // first column; head dims above 128: and 128 columns on
+  const bool active = mine < sub, second = c0 + 128 < Dv;
+  constexpr int U = 8;
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f), acc2 = acc;
   float lstar = 0.f;
   for (int s0 = 0; s0 < ns; s0 += 32) {
     float w = 0.f;
@@ -972,28 +982,52 @@ __global__ void fa_decode_combine_kernel(const float* __restrict__ part_o, const
       lstar += w * ml.y;
     }
     const int cnt = ns - s0 < 32 ? ns - s0 : 32;
-    for (int t = 0; t < cnt; ++t) {
-      const float wt = __shfl_sync(0xffffffffu, w, t);
-      if (wt == 0.f) continue;
-      const float* src = part_o + prow(s0 + t) * Dv;
+    for (int t0 = 0; t0 < cnt; t0 += U * sub) {
+      float wt[U];
+      float4 x[U], y[U];
 #pragma unroll
-      for (int c = 0; c < MAXC; ++c)
-        if (c * 32 + lane < Dv) acc[c] += wt * src[c * 32 + lane];
+      for (int u = 0; u < U; ++u) {
+        const int t = t0 + u * sub + mine;
+        wt[u] = __shfl_sync(0xffffffffu, w, t & 31);
+        if (!active || t >= cnt) wt[u] = 0.f;
+        const float* src = part_o + prow(s0 + t) * Dv + c0;
+        x[u] = wt[u] != 0.f ? *(const float4*)src : make_float4(0.f, 0.f, 0.f, 0.f);
+        y[u] = wt[u] != 0.f && second ? *(const float4*)(src + 128) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        acc.x += wt[u] * x[u].x; acc.y += wt[u] * x[u].y; acc.z += wt[u] * x[u].z; acc.w += wt[u] * x[u].w;
+        acc2.x += wt[u] * y[u].x; acc2.y += wt[u] * y[u].y; acc2.z += wt[u] * y[u].z; acc2.w += wt[u] * y[u].w;
+      }
     }
   }
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) lstar += __shfl_xor_sync(0xffffffffu, lstar, off);
-  const float inv = lstar > 0.f ? 1.f / lstar : 0.f;
-  char* og = (char*)o.ptr + ((long long)b * o.sb + (long long)h * o.sh + (long long)q * o.ss) * 2;
-#pragma unroll
-  for (int c = 0; c < MAXC; ++c) {
-    const int col = c * 32 + lane;
-    if (col < Dv) {
-      if (DT == FA_F16) ((__half*)og)[col] = __float2half_rn(acc[c] * inv);
-      else ((__nv_bfloat16*)og)[col] = __float2bfloat16_rn(acc[c] * inv);
-    }
+  const float4 own = acc;
+  for (int k = 1; k < sub; ++k) {
+    const int from = (lane + k * per) & 31;  // (lanes of the first split add the others' sums up)
+    acc.x += __shfl_sync(0xffffffffu, own.x, from);
+    acc.y += __shfl_sync(0xffffffffu, own.y, from);
+    acc.z += __shfl_sync(0xffffffffu, own.z, from);
+    acc.w += __shfl_sync(0xffffffffu, own.w, from);
   }
   if (lane == 0 && lse != nullptr) lse[row] = lstar > 0.f ? (mstar + log2f(lstar)) * 0.6931471805599453f : -INFINITY;
+  if (mine != 0) return;
+  const float inv = lstar > 0.f ? 1.f / lstar : 0.f;
+  char* og = (char*)o.ptr + ((long long)b * o.sb + (long long)h * o.sh + (long long)q * o.ss + c0) * 2;
+  auto put = [&](char* dst, const float4& v) {
+    uint2 r;
+    if (DT == FA_F16) {
+      const __half2 lo = __floats2half2_rn(v.x * inv, v.y * inv), hi = __floats2half2_rn(v.z * inv, v.w * inv);
+      r = make_uint2(*reinterpret_cast<const unsigned*>(&lo), *reinterpret_cast<const unsigned*>(&hi));
+    } else {
+      const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x * inv, v.y * inv), hi = __floats2bfloat162_rn(v.z * inv, v.w * inv);
+      r = make_uint2(*reinterpret_cast<const unsigned*>(&lo), *reinterpret_cast<const unsigned*>(&hi));
+    }
+    *(uint2*)dst = r;
+  };
+  put(og, acc);
+  if (second) put(og + 256, acc2);
 }
 
 }  // namespace
@@ -1293,13 +1327,17 @@ bool tc_decode_eligible(const fa_attn_params* p) {
   if (p->flags & FA_FLAG_GENERAL_KERNELS) return false;
   if (p->dtype == FA_F32) return false;
   if (p->D != 64 || p->Dv != 64) return false;
-  // The kernel gives every query row two threads (64 kv columns of a tile each), whatever Sq is: it streams K / V
-  // through TMA and a five-stage ring at the same rate whatever the row count, and takes everything from two rows up.
-  // Measured against the general decode kernel (us, this one / general): B32 H8 Skv16384 226 / 378 at 64 rows,
-  // 214 / 251 at 32, 207 / 192 at 16, 206 / 188 at 2; B1 H8 Skv32768 38 / 54 at 2 to 64 rows; B8 H8 Skv4096 28 / 31 at
-  // 2, 30 / 42 at 64; but B32 H8 Skv2048 56 / 42 at 2, 58 / 43 at 32, 64 / 59 at 64, B4 H32 Skv8192 93 / 77 at 2,
-  // 95 / 91 at 32, 105 / 129 at 64: with many heads and up to 16 rows the general kernel has become the faster one.
-  if (p->Sq < 2 || p->Sq > 64 || p->Skv < 1024 || p->Skv > 32768) return false;
+  // The kernel gives every query row two threads (64 kv columns of a tile each), whatever Sq is, and streams K / V through TMA
+  // and a five-stage ring; the general kernel's time grows with the row groups of 16, but two or three of its CTAs share an SM, and
+  // its splits are merged in a cluster.  Measured (us, this one / general, 8 heads unless said, L2 flushed):
+  //   rows      B1 Skv4096   B1 32768     B8 2048      B8 16384     B16 8192     B32 2048     B32 16384
+  //   2         17.4 / 13.3  29.7 / 29.7  21.5 / 16.8  74.8 / 65.6  83.0 / 65.6  52.4 / 37.8  196.6 / 185.3
+  //   16        19.5 / 14.6  31.7 / 31.7  21.5 / 18.5  74.8 / 69.6  83.0 / 68.6  54.3 / 40.9  199.6 / 192.6
+  //   32        19.5 / 17.4  31.7 / 35.8  21.5 / 20.5  76.8 / 73.7  89.1 / 71.9  58.4 / 42.0  205.8 / 233.5
+  //   64        19.5 / 21.5  31.7 / 46.1  23.6 / 27.5  80.8 / 107   99.3 / 107   68.6 / 61.4  220.2 / 374.8
+  // So: up to 16 rows the general kernel, up to 32 over at most 4096 keys, beyond that many heads over short caches.
+  if (p->Sq > 64 || p->Skv < 1024 || p->Skv > 32768) return false;
+  if (p->Sq <= 16 || (p->Sq <= 32 && p->Skv <= 4096) || (p->Skv <= 2048 && (long long)p->B * p->Hq >= 128)) return false;
   if (!(p->scale > 0.f)) return false;
   const fa_block_tables& t = p->tables;
   if (t.kv_num_blocks) {
@@ -1545,7 +1583,7 @@ int fa_module_prepare(fa_module* m, int kind, int dtype, int D, int Dv, int Sq_h
     case FA_KIND_DECODE: {
       DecCfg c;
       if (int rc = pick_decode(dtype, D, Dv, Sq_hint, nullptr, c)) return rc;
-      if (dtype != FA_F32 && D == 64 && Dv == 64 && Sq_hint >= 2)
+      if (dtype != FA_F32 && D == 64 && Dv == 64 && Sq_hint > 16)
         if (int rc = get_fwd_tc_kernel(m, dtype, D, 0, &k, true)) return rc;
       return get_decode_kernel(m, dtype, D, Dv, 0, c, false, &k);
     }
@@ -1710,6 +1748,34 @@ static int fill_waves(long long bh, int cmax, int slots) {
   return best;
 }
 
+// Splits of the general decode kernel for `bh` tiles of query rows over `tiles` 128-key tiles.
+//   * Two CTAs per SM, all resident at once, stream as fast as more do, and every further split costs its start and its
+//     merge; at least four tiles per CTA.
+//   * Many heads: one split leaves SMs with one CTA beside SMs with two.  Over long caches (24 tiles per CTA and more) several
+//     waves that end nearly full are faster then.
+//   * Few heads: up to FA_DECODE_MAX_CLUSTER splits are merged inside a cluster, more by the combine kernel; where even a
+//     cluster per head leaves SMs idle, one CTA per SM.
+// Against as many CTAs as fit with the last wave 95 % full (us, before / now): B16 H32/8 Skv8191 D128 124 / 113, B4 H32
+// Skv8192 D64 76.8 / 65.6, B4 H8 Skv8192 D128 54 / 41, B8 H32/8 8 rows Skv5000 D128 76.8 / 55.3, B32 H8 Skv2048 42.0 / 38.9.
+static int general_decode_splits(long long bh, int tiles, int per_sm, int sm_count) {
+  const int cmax = std::min(std::max(tiles / 4, 1), 64);
+  const int c = (int)std::min<long long>(cmax, std::max<long long>(1, std::min(per_sm, 2) * sm_count / bh));
+  if (c == 1) {
+    int best = 1;
+    double best_fill = 0.88;
+    for (int k = 2; k <= std::min(FA_DECODE_MAX_CLUSTER, tiles / 24); ++k) {
+      const double waves = (double)(bh * k) / (per_sm * sm_count), fill = waves / (double)(long long)(waves + 0.999999);
+      if (waves > 1.0 && fill > best_fill) {
+        best = k;
+        best_fill = fill;
+      }
+    }
+    return best;
+  }
+  if (c <= FA_DECODE_MAX_CLUSTER) return c;
+  return std::max(FA_DECODE_MAX_CLUSTER, (int)std::min<long long>(c, (sm_count + bh - 1) / bh));
+}
+
 int fa_decode_packs_heads(const fa_attn_params* p) { return (p && decode_packs_heads(p)) ? 1 : 0; }
 
 int fa_decode_num_splits(const fa_attn_params* p, int sm_count) {
@@ -1725,17 +1791,14 @@ int fa_decode_num_splits(const fa_attn_params* p, int sm_count) {
     const int c = fill_waves(bh, cmax, sm_count);
     return c < 2 ? 2 : c;
   }
-  // general kernel: as many CTAs per SM as its shared memory allows (at most four by registers),
-  // at least four kv tiles per CTA.  A grid that ends in a part-filled wave costs more than a few
-  // extra partial results.
+  // general kernel: as many CTAs per SM as its shared memory allows (at most four by registers)
   int per_sm = 2;
   DecCfg c;
   if (pick_decode(p->dtype, p->D, p->Dv, pack ? p->Sq * (p->Hq / p->Hkv) : p->Sq, nullptr, c) == FA_OK) {
     per_sm = (228 * 1024) / (c.smem + 1024);
     per_sm = per_sm < 1 ? 1 : (per_sm > 4 ? 4 : per_sm);
   }
-  const int cmax = tiles / 4 > 1 ? (tiles / 4 < 64 ? tiles / 4 : 64) : 1;
-  return fill_waves(bh, cmax, per_sm * sm_count);
+  return general_decode_splits(bh, tiles, per_sm, sm_count);
 }
 
 size_t fa_decode_workspace_bytes(const fa_attn_params* p, int num_splits) {
@@ -1761,7 +1824,13 @@ int fa_decode(fa_module* m, const fa_attn_params* p, int num_splits, void* works
   if (need && (!workspace || workspace_bytes < need)) return fail(FA_EWORKSPACE, "decode workspace too small");
   if (need && ((uintptr_t)workspace & 15)) return fail(FA_EINVAL, "workspace must be 16-byte aligned");
   kp.num_splits = num_splits;
-  if (need) {
+  // The splits of a tile of rows are merged inside a thread-block cluster where all CTAs are resident at once: no second launch and no
+  // partial results in memory (us: B8 H8 Skv2048 D64 21.4 -> 16.4, B4 H8 Skv8192 D128 46 -> 41).  Where the grid takes several waves
+  // a cluster has to wait for room for all its CTAs (B32 H8 Skv16384 D64, five splits: 188 -> 197), and the partial
+  // results go through memory and the combine kernel.
+  const bool cluster = !tc && num_splits > 1 && num_splits <= FA_DECODE_MAX_CLUSTER &&
+                       (long long)p->B * (pack ? p->Hkv : p->Hq) * num_splits <= 2 * device_sm_count();
+  if (need && !cluster) {
     const size_t rows = (size_t)p->B * p->Hq * num_splits * p->Sq;
     kp.part_o = (float*)workspace;
     kp.part_ml = (float*)((char*)workspace + (rows * p->Dv * sizeof(float) + 255) / 256 * 256);
@@ -1772,9 +1841,9 @@ int fa_decode(fa_module* m, const fa_attn_params* p, int num_splits, void* works
   } else {
     Kernel* k = nullptr;
     if (int rc = get_decode_kernel(m, p->dtype, p->D, p->Dv, p->flags, c, pack, &k)) return rc;
-    if (int rc = launch(k, dim3(num_splits, pack ? p->Hkv : p->Hq, p->B), dim3(128), &kp, stream)) return rc;
+    if (int rc = launch(k, dim3(num_splits, pack ? p->Hkv : p->Hq, p->B), dim3(128), &kp, stream, cluster ? num_splits : 1)) return rc;
   }
-  if (num_splits > 1) {
+  if (num_splits > 1 && !cluster) {
     const long long n_rows = (long long)p->B * p->Hq * p->Sq;
     const unsigned blocks = (unsigned)((n_rows + 3) / 4);
     if (int rc = launch_here("fa_decode_combine_kernel", p->dtype == FA_F16 ? fa_decode_combine_kernel<FA_F16> : fa_decode_combine_kernel<FA_BF16>,

@@ -8,8 +8,9 @@
 // warps share the K/V tiles, which stream through a cp.async ring in 128-bit pieces; warp
 // (rg, cg) owns query rows 16*rg.. and the cg-th slice of each kv tile and keeps its own
 // running (max, sum, O).  The CG partial results are merged through shared memory at the
-// end; with more than one split the CTA writes un-normalised (O, max, sum) to the workspace
-// and a second kernel combines the splits, with one split it writes O and LSE directly.
+// end.  With one split the CTA then writes O and LSE.  With several, the CTAs of a tile of rows are a thread-block cluster
+// and merge through each other's shared memory (up to FA_DECODE_MAX_CLUSTER splits, when the host launches them so),
+// or write un-normalised (O, max, sum) to the workspace for a second kernel to combine.
 //
 // With grouped-query attention the G query heads of a kv head can share one CTA
 // (FA_PACK_HEADS): its G * Sq query rows form one tile, row r belonging to head r / Sq and
@@ -21,6 +22,26 @@
 // FA_BN (kv tile), FA_PACK_HEADS.
 #pragma once
 #include "fa_common.cuh"
+
+// ---- thread-block clusters: barrier over all threads, reads of another CTA's shared memory ----
+__device__ __forceinline__ void fa_cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ fa_u32 fa_mapa(fa_u32 addr, int rank) {
+  fa_u32 r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ float2 fa_ld_cluster_f2(fa_u32 addr) {
+  float2 v;
+  asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ float4 fa_ld_cluster_f4(fa_u32 addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+  return v;
+}
 
 #ifndef FA_PACK_HEADS
 #define FA_PACK_HEADS 0
@@ -278,6 +299,10 @@ extern "C" __global__ void __launch_bounds__(fa_dec::NT) fa_decode_kernel(const 
   }
   __syncthreads();
   const int rows = min(R, BM);
+  // Splits in one cluster: the CTA's merged rows stay in shared memory, O over the first column group's and the
+  // maximum and sum over the query tile, and the CTAs of the cluster read each other's.
+  const bool in_cluster = p.num_splits > 1 && p.part_o == nullptr;
+  float2* ml = (float2*)smem;  // [BM]
   for (int i = tid; i < rows * DV; i += NT) {
     const int r = i / DV, c = i - r * DV;
     const int g_row = PACK ? r / p.Sq : 0, qr = r - g_row * p.Sq, h = h0 + g_row;
@@ -293,7 +318,10 @@ extern "C" __global__ void __launch_bounds__(fa_dec::NT) fa_decode_kernel(const 
       acc += w * row[c];
       lstar += w * row[DV + 1];
     }
-    if (p.num_splits > 1) {
+    if (in_cluster) {
+      mrg[(long long)r * MRG_PITCH + c] = acc;  // (this thread alone reads column c of the row)
+      if (c == 0) ml[r] = make_float2(mstar, lstar);
+    } else if (p.num_splits > 1) {
       const long long prow = (bh * p.num_splits + split) * p.Sq + qr;
       p.part_o[prow * DV + c] = acc;
       if (c == 0) {
@@ -314,7 +342,39 @@ extern "C" __global__ void __launch_bounds__(fa_dec::NT) fa_decode_kernel(const 
         ((fa_u16*)og)[c] = hv;
       }
       if (c == 0 && p.lse != nullptr)
-        p.lse[bh * p.Sq + qr] = lstar > 0.f ? (mstar + fa_lg2(lstar)) * FA_LN2 : FA_NEG_INF;
+        p.lse[bh * p.Sq + qr] = lstar > 0.f ? (mstar + log2f(lstar)) * FA_LN2 : FA_NEG_INF;
     }
   }
+  if (!in_cluster) return;
+  // ---- merge the splits: four columns of a row per thread, the rows spread over the CTAs -----------
+  fa_cluster_sync();
+  const int ns = p.num_splits;
+  for (int i = split * NT + tid; i < rows * (DV / 4); i += ns * NT) {
+    const int r = i / (DV / 4), c = (i - r * (DV / 4)) * 4;
+    const int g_row = PACK ? r / p.Sq : 0, qr = r - g_row * p.Sq, h = h0 + g_row;
+    const fa_u32 ml_addr = fa_smem_u32(ml + r), o_addr = fa_smem_u32(mrg + (long long)r * MRG_PITCH + c);
+    float2 part[FA_DECODE_MAX_CLUSTER];
+    float mstar = FA_NEG_INF;
+#pragma unroll
+    for (int s = 0; s < FA_DECODE_MAX_CLUSTER; ++s) {
+      part[s] = s < ns ? fa_ld_cluster_f2(fa_mapa(ml_addr, s)) : make_float2(FA_NEG_INF, 0.f);
+      mstar = fmaxf(mstar, part[s].x);
+    }
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    float lstar = 0.f;
+#pragma unroll
+    for (int s = 0; s < FA_DECODE_MAX_CLUSTER; ++s) {
+      const float w = part[s].x == FA_NEG_INF ? 0.f : exp2f(part[s].x - mstar);
+      if (w == 0.f) continue;
+      const float4 x = fa_ld_cluster_f4(fa_mapa(o_addr, s));
+      acc.x += w * x.x; acc.y += w * x.y; acc.z += w * x.z; acc.w += w * x.w;
+      lstar += w * part[s].y;
+    }
+    const float inv = lstar > 0.f ? 1.f / lstar : 0.f;
+    char* og = (char*)p.o.ptr + ((long long)b * p.o.sb + (long long)h * p.o.sh + (long long)qr * p.o.ss + c) * ES;
+    *(uint2*)og = make_uint2(fa_pack2<DT>(acc.x * inv, acc.y * inv), fa_pack2<DT>(acc.z * inv, acc.w * inv));
+    if (c == 0 && p.lse != nullptr)
+      p.lse[((long long)b * p.Hq + h) * p.Sq + qr] = lstar > 0.f ? (mstar + log2f(lstar)) * FA_LN2 : FA_NEG_INF;
+  }
+  fa_cluster_sync();  // nobody leaves while its rows are being read
 }

@@ -54,6 +54,9 @@ struct FaTables {
   } while (0)
 #endif
 
+// CTAs of a (batch, head) whose decode splits are merged inside a thread-block cluster (the portable cluster size)
+#define FA_DECODE_MAX_CLUSTER 8
+
 struct FaParams {
   FaTensor q, k, v, o;
   FaTensor dout, dq, dk, dv;
