@@ -9,19 +9,31 @@
 #pragma once
 #include "fa_params.h"
 
-// One CTA of four warps per block, in 128 x 128 sub-tiles: a warp takes 32 rows, a lane one key out of each
-// group of 32.  Lane = key makes what a mask reads per key (a captured document id) a coalesced load
-// outside the row loop and what it reads per query a broadcast; a ballot per row gives 32 keys of the
-// row-major matrix and the lane's own bits over the rows are a word of the transposed one, so both
-// matrices and the block's count come out of one evaluation.  (A thread per position with a 64-bit
-// division for its row, and a second kernel that evaluated the mask again for the bits, took 35 + 4 us
-// on a 4096 x 4096 document mask.)  Needs key blocks of whole 32-bit words and query blocks of whole
-// words or a single one; other block sizes go to the classify kernel below.
+// One CTA of four warps per block, in 128 x 128 sub-tiles: a warp takes 32 rows, a lane one of them, 32 keys at a time.  The
+// lane's own bits over the keys are a word of the row-major matrix (one predicated OR per position), what a mask reads per
+// query (a captured document id) is loaded once per lane and what it reads per key is a broadcast; five exchange steps
+// between the lanes turn the 32 words into those of the transposed matrix (some 25 instructions per 1024 positions).  Both matrices and
+// the block's count come out of one evaluation.  Bound by instruction issue.  8192 x 8192 positions of an attention-sink mask:
+// 29 us; with lane = key, a ballot per row and a select for its word, 41.
+// Needs key blocks of whole 32-bit words and query blocks of whole words or a single one; other block sizes go to the
+// classify kernel below.
 constexpr int FA_SCAN_WARPS = 4;
+// the transpose of the 32 x 32 bit matrix whose row i is lane i's word
+__device__ __forceinline__ unsigned fa_bit_transpose(unsigned x, int lane) {
+  unsigned m = 0x0000ffffu;
+#pragma unroll
+  for (int s = 16; s > 0; s >>= 1) {
+    const unsigned y = __shfl_xor_sync(0xffffffffu, x, s);
+    x = (lane & s) ? (x & ~m) | ((y & ~m) >> s) : (x & m) | ((y & m) << s);
+    m ^= m << (s >> 1);
+  }
+  return x;
+}
 extern "C" __global__ void __launch_bounds__(128) fa_mask_scan_kernel(const __grid_constant__ FaMaskParams p) {
   FA_MOD_BUFS_INIT(p);
   fa_grid_wait();
-  __shared__ unsigned t_words[128][FA_SCAN_WARPS];
+  __shared__ __align__(16) unsigned t_words[128][FA_SCAN_WARPS];
+  __shared__ unsigned r_words[4][128];
   __shared__ int s_cnt[FA_SCAN_WARPS];
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -31,44 +43,35 @@ extern "C" __global__ void __launch_bounds__(128) fa_mask_scan_kernel(const __gr
   const int q0 = qb * p.QB, k0 = kvb * p.KVB;
   int cnt = 0;
   for (int r0 = 0; r0 < p.QB; r0 += 128) {
+    const int row = r0 + warp * 32 + lane, q = q0 + row;  // this lane's row inside the block, and its query
+    const bool row_in = row < p.QB;
     for (int c0 = 0; c0 < p.KVB; c0 += 128) {
-      const int rbase = r0 + warp * 32;  // first row of this warp inside the block
-      unsigned roww[4] = {0u, 0u, 0u, 0u}, colw[4] = {0u, 0u, 0u, 0u};
-      const int nrows = min(32, p.QB - rbase);
-      if (c0 + 128 <= p.KVB && nrows == 32) {
-#pragma unroll 8
-        for (int r = 0; r < 32; ++r) {
+#pragma unroll 1
+      for (int c = 0; c < 4; ++c) {
+        const int kv = k0 + c0 + 32 * c, left = p.KVB - (c0 + 32 * c);
+        unsigned w = 0u;
+        if (left > 0) {  // (the same for all threads)
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            const bool keep = fa_mask_mod(gb, gh, q0 + rbase + r, k0 + c0 + 32 * c + lane);
-            const unsigned vote = __ballot_sync(0xffffffffu, keep);
-            if (lane == r) roww[c] = vote;
-            colw[c] |= (keep ? 1u : 0u) << r;
-          }
+          for (int e = 0; e < 32; ++e)
+            if (fa_mask_mod(gb, gh, q, kv + e)) w |= 1u << e;
+          if (left < 32) w &= (1u << left) - 1u;
+          if (!row_in) w = 0u;
         }
-      } else {
-        for (int r = 0; r < nrows; ++r) {
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            const int col = c0 + 32 * c + lane;
-            const bool keep = col < p.KVB && fa_mask_mod(gb, gh, q0 + rbase + r, k0 + col);
-            const unsigned vote = __ballot_sync(0xffffffffu, keep);
-            if (lane == r) roww[c] = vote;
-            colw[c] |= (keep ? 1u : 0u) << r;
-          }
-        }
+        cnt += __popc(w);
+        r_words[c][threadIdx.x] = w;  // (read back by this thread)
+        if (p.bits_t != nullptr) t_words[32 * c + lane][warp] = fa_bit_transpose(w, lane);
       }
-      cnt += __popc(roww[0]) + __popc(roww[1]) + __popc(roww[2]) + __popc(roww[3]);
       if (p.bits != nullptr) {
         // the row's words of this sub-tile; keys beyond KV_LEN are 0, and the last block also writes the padding words
-        const int q = q0 + rbase + lane;
-        if (lane < nrows && q < p.Q_LEN) {
+        if (row_in && q < p.Q_LEN) {
           unsigned* dst = p.bits + ((long long)bh * p.Q_LEN + q) * p.stride;
           const int w0 = (k0 + c0) >> 5;
           const int wend = (kvb == p.nKV - 1 && c0 + 128 >= p.KVB) ? (int)p.stride : min(w0 + 4, (k0 + p.KVB) >> 5);
+          unsigned roww[4];
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
             const int left = p.KV_LEN - (k0 + c0 + 32 * c);
+            roww[c] = r_words[c][threadIdx.x];
             if (left < 32) roww[c] &= left <= 0 ? 0u : (1u << left) - 1u;
           }
           if ((w0 & 3) == 0 && w0 + 4 <= wend) {
@@ -82,8 +85,6 @@ extern "C" __global__ void __launch_bounds__(128) fa_mask_scan_kernel(const __gr
         }
       }
       if (p.bits_t != nullptr) {
-#pragma unroll
-        for (int c = 0; c < 4; ++c) t_words[32 * c + lane][warp] = colw[c];
         __syncthreads();
         const int col = c0 + (int)threadIdx.x, kv = k0 + col;
         if (col < p.KVB && kv < p.KV_LEN) {
