@@ -438,7 +438,7 @@ def create_block_mask(
     flaxattention/core/blockmask.py:277-322), one entry along batch / heads when ``mask_mod`` does
     not read ``b`` / ``h``: on the partial tiles the attention kernels read a row's words instead of
     evaluating ``mask_mod`` 128 times per row.  It is built when it takes at most 64 MiB, and transposed too
-    (for the fp32 backward) when both together do
+    (for the backward) when both together do
     (``_mask_bits=True`` / ``False`` forces it on or off), from the same evaluation as the tables.  A mask
     that reads captured tensors gets one when these are on the device and take at most 256 KiB; the
     attention calls then compare them, on the device, with a copy taken here, and evaluate ``mask_mod``

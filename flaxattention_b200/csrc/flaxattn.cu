@@ -110,7 +110,7 @@ std::string cache_dir() {
 }
 
 const char* const kTemplateFiles[] = {"fa_params.h", "fa_common.cuh", "fa_fwd.cuh", "fa_bwd.cuh",
-                                      "fa_decode.cuh", "fa_blockmask.cuh", "fa_sm100.cuh", "fa_fwd_tc.cuh", "fa_bwd_tc.cuh", "fa_bwd_f32.cuh", "fa_selftest.cuh"};
+                                      "fa_decode.cuh", "fa_blockmask.cuh", "fa_sm100.cuh", "fa_fwd_tc.cuh", "fa_bwd_items.cuh", "fa_bwd_tc.cuh", "fa_bwd_tc128.cuh", "fa_bwd_f32.cuh", "fa_selftest.cuh"};
 std::string g_templates_hash;
 int templates_hash(std::string& out) {
   if (g_templates_hash.empty()) {
@@ -882,21 +882,20 @@ __global__ void fa_bwd_prep_kernel(FaTensor o, FaTensor dout, const float* __res
   }
 }
 
-// dq = scale * dq_acc for the tcgen05 backward.  The fp32 accumulation buffer holds, per
-// (b, h, 128-row q tile), two [128 rows][32 columns] blocks (columns 0-31, then 32-63), and the
-// eight 16-byte chunks of a block row r sit at position k ^ (r & 7).
-template <int DT>
+// dq = scale * dq_acc for the tcgen05 backward.  The fp32 accumulation buffer holds, per (b, h, 128-row q tile), D / 32 blocks
+// of [128 rows][32 columns], and the eight 16-byte chunks of a block row r sit at position k ^ (r & 7).
+template <int DT, int D>
 __global__ void fa_dq_convert_kernel(const float* __restrict__ acc, FaTensor dq, int Hq, int Sq, int sq_pad, float scale,
                                      int n_bh) {
   // grid: x over the rows of one (batch, head), one 8-element output chunk per thread; (y, z) over the heads
   grid_wait();
   const int bh = blockIdx.y + blockIdx.z * gridDim.y;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int k8 = i & 7, q = i >> 3;
+  const int k8 = i % (D / 8), q = i / (D / 8);
   if (bh >= n_bh || q >= Sq) return;
   const int b = bh / Hq, h = bh - b * Hq;
   const int r = q & 127, c = 2 * (k8 & 3);
-  const float* src = acc + ((long long)bh * sq_pad + (q - r)) * 64 + (k8 >> 2) * (128 * 32) + r * 32;
+  const float* src = acc + ((long long)bh * sq_pad + (q - r)) * D + (k8 >> 2) * (128 * 32) + r * 32;
   const float4 lo = *(const float4*)(src + ((c ^ (r & 7)) * 4));
   const float4 hi = *(const float4*)(src + (((c + 1) ^ (r & 7)) * 4));
   char* dst = (char*)dq.ptr + ((long long)b * dq.sb + (long long)h * dq.sh + (long long)q * dq.ss) * 2 + k8 * 16;
@@ -907,40 +906,6 @@ __global__ void fa_dq_convert_kernel(const float* __restrict__ acc, FaTensor dq,
   } else {
     __nv_bfloat162 o[4] = {__floats2bfloat162_rn(lo.x * scale, lo.y * scale), __floats2bfloat162_rn(lo.z * scale, lo.w * scale),
                            __floats2bfloat162_rn(hi.x * scale, hi.y * scale), __floats2bfloat162_rn(hi.z * scale, hi.w * scale)};
-    *(uint4*)dst = *reinterpret_cast<uint4*>(o);
-  }
-}
-
-// The same for head dim 128, where the kernel accumulates dQ transposed: per (b, h, 64-row q
-// tile) the buffer holds two [128 head-dim lanes][32 query columns] blocks (query columns 0-31,
-// then 32-63), 16-byte chunks of a block row d at position k ^ (d & 7).  A warp takes 32
-// consecutive query rows and one group of 8 head-dim values: each of its 8 reads is one 128-byte
-// row of a block, and every thread writes one 16-byte chunk of its output row.
-template <int DT>
-__global__ void fa_dq_convert_t_kernel(const float* __restrict__ acc, FaTensor dq, int Hq, int Sq, int sq_pad, float scale,
-                                       int n_bh) {
-  grid_wait();
-  const int bh = blockIdx.y + blockIdx.z * gridDim.y;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int dg = (i >> 5) & 15, q = ((i >> 9) << 5) | (i & 31);
-  if (bh >= n_bh || q >= Sq) return;
-  const int b = bh / Hq, h = bh - b * Hq;
-  const int c = q & 63, hf = c >> 5, k = (c & 31) >> 2, w = c & 3;
-  const float* src = acc + ((long long)bh * (sq_pad >> 6) + (q >> 6)) * (128 * 64) + hf * (128 * 32) + w;
-  float v[8];
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const int d = dg * 8 + j;
-    v[j] = src[d * 32 + ((k ^ (d & 7)) << 2)] * scale;
-  }
-  char* dst = (char*)dq.ptr + ((long long)b * dq.sb + (long long)h * dq.sh + (long long)q * dq.ss) * 2 + dg * 16;
-  if (DT == FA_F16) {
-    __half2 o[4] = {__floats2half2_rn(v[0], v[1]), __floats2half2_rn(v[2], v[3]), __floats2half2_rn(v[4], v[5]),
-                    __floats2half2_rn(v[6], v[7])};
-    *(uint4*)dst = *reinterpret_cast<uint4*>(o);
-  } else {
-    __nv_bfloat162 o[4] = {__floats2bfloat162_rn(v[0], v[1]), __floats2bfloat162_rn(v[2], v[3]),
-                           __floats2bfloat162_rn(v[4], v[5]), __floats2bfloat162_rn(v[6], v[7])};
     *(uint4*)dst = *reinterpret_cast<uint4*>(o);
   }
 }
@@ -1400,8 +1365,8 @@ struct FaBwdTcParamsHost {
   int chunk_heads;
 };
 
-// pairs one item of fa_bwd_tc.cuh may list (fa_btc::MAXPL)
-int bwd_tc_max_pairs(int D) { return D == 64 ? 1024 : 2048; }
+// (query head, 128-row q tile) pairs one item of the tcgen05 backward may list (fa_btc::MAXPL, fa_b128::MAXPL)
+constexpr int kBwdTcMaxPairs = 1024;
 
 bool tc_bwd_eligible(const fa_attn_params* p) {
   if (p->flags & FA_FLAG_GENERAL_KERNELS) return false;
@@ -1409,11 +1374,10 @@ bool tc_bwd_eligible(const fa_attn_params* p) {
   if (p->D != p->Dv || !(p->D == 64 || p->D == 128)) return false;
   if (p->Sq < 128 || p->Skv < 128) return false;
   // a CTA lists the (query head, q tile) pairs of an item in shared memory: at most 256 q tiles
-  // of 128 rows per head, and the pairs of one item must fit the list (a pair is 128 q rows with
-  // D = 64, 64 with D = 128)
+  // of 128 rows per head, and the pairs of one item must fit the list
   const int n_qtiles = (p->Sq + 127) / 128;
   if (n_qtiles > 256) return false;
-  if ((long long)n_qtiles * (p->D / 64) * (p->Hq / p->Hkv) > bwd_tc_max_pairs(p->D)) return false;
+  if ((long long)n_qtiles * (p->Hq / p->Hkv) > kBwdTcMaxPairs) return false;
   const fa_block_tables& t = p->tables;
   if (t.kv_num_blocks) {
     if (!(t.num_q_blocks == 1 || t.q_block_size % 128 == 0)) return false;
@@ -1503,16 +1467,22 @@ int launch_bwd_f32_tc(fa_module* m, const fa_attn_params* p, FaParams kp, const 
   return launch(kf, rerun_grid((long long)p->B * p->Hkv * n_tiles, kf->smem), dim3(c.warps * 32), &kp, stream);
 }
 
-// kv2: two K / V buffers and one of dS^T instead of one and two (head dim 64)
+// kv2 (head dim 64): two K / V buffers and one of dS^T instead of one and two
 int get_bwd_tc_kernel(fa_module* m, int dtype, int D, int flags, bool kv2, Kernel** k) {
-  // must match the shared-memory map of fa_bwd_tc.cuh (fa_btc::SMEM_BYTES)
-  const int bq = D == 64 ? 128 : 64, kvbuf = (D == 64 && kv2) ? 2 : 1, nstage = 3, nds = kvbuf == 1 ? 2 : 1;
-  const int kv_bytes = (D / 64) * 16384, q_bytes = 16384, ds_bytes = (bq / 64) * 16384;
-  const int smem = 2 * kvbuf * kv_bytes + 2 * nstage * q_bytes + nds * ds_bytes + 128 * 32 * 4 + nstage * 2 * bq * 4 +
-                   (2 + 3 * nstage + 15) * 8 + 16 + 32 + 2 * bwd_tc_max_pairs(D) * 4 + 64 + 1024;
   const int rnd = round_flag(dtype, flags);
+  const int lists = 2 * kBwdTcMaxPairs * 4 + 64 + 1024;
+  if (D == 128) {
+    // must match the shared-memory map of fa_bwd_tc128.cuh (fa_b128::SMEM_BYTES): thirteen blocks of 128 rows x 128 bytes
+    const int smem = 13 * 16384 + 2 * 2 * 128 * 4 + 22 * 8 + 16 + 32 + lists;
+    return get_kernel(m, kernel_key(kIdBwdTc, {{dtype, 2}, {D, 9}, {rnd, 1}, {1, 2}}), "fa_bwd_tc128.cuh",
+                      [&] { return defs({{"FA_DTYPE", dtype}, {"FA_ROUND_SCORES", rnd}}); }, "fa_bwd_tc_kernel", smem, k);
+  }
+  // must match the shared-memory map of fa_bwd_tc.cuh (fa_btc::SMEM_BYTES)
+  const int kvbuf = kv2 ? 2 : 1, nstage = 3, nds = kvbuf == 1 ? 2 : 1;
+  const int smem = 2 * kvbuf * 16384 + 2 * nstage * 16384 + nds * 32768 + 128 * 32 * 4 + nstage * 2 * 128 * 4 +
+                   (2 + 3 * nstage + 15) * 8 + 16 + 32 + lists;
   return get_kernel(m, kernel_key(kIdBwdTc, {{dtype, 2}, {D, 9}, {rnd, 1}, {kvbuf, 2}}), "fa_bwd_tc.cuh",
-                    [&] { return defs({{"FA_DTYPE", dtype}, {"FA_D", D}, {"FA_ROUND_SCORES", rnd}, {"FA_BWD_KV2", kvbuf == 2 ? 1 : 0}}); },
+                    [&] { return defs({{"FA_DTYPE", dtype}, {"FA_ROUND_SCORES", rnd}, {"FA_BWD_KV2", kvbuf == 2 ? 1 : 0}}); },
                     "fa_bwd_tc_kernel", smem, k);
 }
 
@@ -1683,11 +1653,10 @@ int fa_bwd(fa_module* m, const fa_attn_params* p, const fa_tensor* dout, const f
     tp.ndelta = ndelta;
     tp.work_counter = work_counter;
     tp.chunk_heads = bwd_tc_chunk_heads(p);
-    const int bq = p->D == 64 ? 128 : 64;  // q rows of a (kv tile, q tile) pair of the kernel
-    if (int rc = make_map(&tp.tq, p->dtype, p->q, p->D, p->Sq, p->Hq, p->B, bq)) return rc;
+    if (int rc = make_map(&tp.tq, p->dtype, p->q, p->D, p->Sq, p->Hq, p->B)) return rc;
     if (int rc = make_map(&tp.tk, p->dtype, p->k, p->D, p->Skv, p->Hkv, p->B)) return rc;
     if (int rc = make_map(&tp.tv, p->dtype, p->v, p->Dv, p->Skv, p->Hkv, p->B)) return rc;
-    if (int rc = make_map(&tp.tdo, p->dtype, *dout, p->Dv, p->Sq, p->Hq, p->B, bq)) return rc;
+    if (int rc = make_map(&tp.tdo, p->dtype, *dout, p->Dv, p->Sq, p->Hq, p->B)) return rc;
     if (int rc = make_map(&tp.tdk, p->dtype, *dk, p->D, p->Skv, p->Hkv, p->B)) return rc;
     if (int rc = make_map(&tp.tdv, p->dtype, *dv, p->Dv, p->Skv, p->Hkv, p->B)) return rc;
     // persistent: one CTA per SM (fewer when there are fewer items), items handed out through the counter
@@ -1696,8 +1665,8 @@ int fa_bwd(fa_module* m, const fa_attn_params* p, const fa_tensor* dout, const f
     {
       // one 16-byte output chunk per thread: D / 8 chunks per row
       const dim3 grid((unsigned)(((long long)sq_pad * (p->D / 8) + 255) / 256), (unsigned)gy, (unsigned)((n_bh + gy - 1) / gy));
-      const auto convert = p->D == 64 ? (p->dtype == FA_F16 ? fa_dq_convert_kernel<FA_F16> : fa_dq_convert_kernel<FA_BF16>)
-                                      : (p->dtype == FA_F16 ? fa_dq_convert_t_kernel<FA_F16> : fa_dq_convert_t_kernel<FA_BF16>);
+      const auto convert = p->D == 64 ? (p->dtype == FA_F16 ? fa_dq_convert_kernel<FA_F16, 64> : fa_dq_convert_kernel<FA_BF16, 64>)
+                                      : (p->dtype == FA_F16 ? fa_dq_convert_kernel<FA_F16, 128> : fa_dq_convert_kernel<FA_BF16, 128>);
       if (int rc = launch_here("fa_dq_convert_kernel", convert, grid, dim3(256), stream, dq_acc, kp.dq, p->Hq, p->Sq, sq_pad, p->scale, n_bh))
         return rc;
     }

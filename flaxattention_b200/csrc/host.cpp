@@ -275,8 +275,7 @@ struct AttentionBackward : public torch::autograd::Node {
     size_t bytes = 0;
     const at::Tensor ws = workspace(p, fa_bwd_workspace_bytes, q.device(), bytes);
     void* stream = (void*)c10::cuda::getCurrentCUDAStream(q.device().index()).stream();
-    at::Tensor hold;
-    if (p.dtype == FA_F32) hold = check_snapshot(call, p, q.device(), stream);  // (the 16-bit backward reads no matrix)
+    const at::Tensor hold = check_snapshot(call, p, q.device(), stream);
     int rc;
     {
       BuffersLock buffers(*call.mods);

@@ -1,0 +1,174 @@
+// What the tcgen05 backward kernels share: launch parameters, small PTX helpers, the order of the items, the
+// list of the pairs of one, and the masks read from the bit matrix.
+#pragma once
+#include "fa_sm100.cuh"
+
+struct FaBwdTcParams {
+  FaParams p;
+  FaTensorMap tq, tk, tv, tdo;  // 4-d maps (D, S, H, B), 128-byte swizzle, box 64 x 128 rows
+  FaTensorMap tdk, tdv;         // the outputs dK and dV, like tk and tv
+  float* dq_acc;                // per (b, h, 128-row q tile): D / 32 fp32 blocks [128 rows][32 columns], 16-byte chunks of a row permuted
+  const float* nlse2;           // [B, Hq, ceil(Sq/128)*128]: -lse * log2(e); -inf for rows without mass / beyond Sq
+  const float* ndelta;          // same shape: -rowsum(O * dO); 0 beyond Sq
+  int* work_counter;            // zero at launch: items beyond the first of every CTA are handed out through it
+  int chunk_heads;              // (batch, kv head) pairs whose items are numbered together (see item_of)
+};
+
+namespace fa_bwd_items {
+
+__device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+__device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
+}
+__device__ __forceinline__ void bulk_reduce_add_f32(float* gdst, fa_u32 ssrc, fa_u32 bytes) {
+  asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;" ::"l"(gdst), "r"(ssrc), "r"(bytes)
+               : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait_read0() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait0() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+// brings a tile into L2 ahead of the load that will need it
+__device__ __forceinline__ void tma_prefetch_l2_4d(const FaTensorMap* map, int c0, int c1, int c2, int c3) {
+  asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global.tile [%0, {%1, %2, %3, %4}];" ::"l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
+               : "memory");
+}
+
+// byte offset (in 16-byte units) of k-step kk of a K-major operand whose 64-element column groups
+// are `atom_bytes` apart: 32 bytes per step inside a 128-byte row, four steps per group
+__device__ __forceinline__ constexpr fa_u32 kstep_kmajor(int kk, int atom_bytes) {
+  return (fa_u32)(((kk >> 2) * atom_bytes + (kk & 3) * 32) >> 4);
+}
+
+// Item number -> (kv head, batch, kv tile).  The first kv tiles of all heads come first (under a causal mask and
+// with attention sinks they are the heaviest), then chunk by chunk of `ch` heads, in a chunk heads fastest and the
+// kv tile slowest.  The CTAs work through the items in this order, so that at any time the dQ accumulator, Q and dO
+// of about one chunk of heads are in use: the host sizes it to stay in L2.
+struct Item {
+  int hk, b, kt;
+};
+__device__ __forceinline__ Item item_of(int idx, int Hkv, int B, int n_kvt, int ch) {
+  const unsigned heads = Hkv * B, i = idx;
+  unsigned head = i, kt = 0;
+  if ((unsigned)ch >= heads) {  // one chunk
+    kt = i / heads;
+    head = i - kt * heads;
+  } else if (i >= heads) {
+    const unsigned r = i - heads, per = ch * (n_kvt - 1), c = r / per, rr = r - c * per;
+    const unsigned n = min((unsigned)ch, heads - c * ch);
+    kt = rr / n;
+    head = c * ch + rr - kt * n;
+    ++kt;
+  }
+  const unsigned b = head / Hkv;
+  return {(int)(head - b * Hkv), (int)b, (int)kt};
+}
+
+// The (query head, q tile) pairs of one item, written to `pl` by one warp: per head of the group,
+// the 128-row q tiles the BlockMask lists for the item's kv tile (class 1: apply mask_mod, 2: full)
+// in ascending order, each as 128 / BQ pairs.  Without tables every tile is listed.  Returns the
+// number of pairs (the same in every lane).  `cl` is scratch: one bit per q tile and class.
+template <int BQ, int MAXPL, int MAXC>
+__device__ __forceinline__ int build_pair_list(const FaParams& p, int hk, int b, int kt, int G, int n_ctiles,
+                                               unsigned* cl, int* pl, int lane) {
+  constexpr int PPT = 128 / BQ;
+  const bool tables = p.t.kv_num != nullptr && p.t.q_num != nullptr;
+  int w = 0;
+  for (int g = 0; g < G; ++g) {
+    if (!tables) {
+      const int nq = (p.Sq + BQ - 1) / BQ;
+      const int mode = FA_HAS_MASK_MOD ? 1 : 2;
+      // the items of a head start at different q tiles, so that the CTAs on one head do not add to the same
+      // dQ tile at the same time
+      const int rot = kt % nq;
+      for (int e = lane; e < nq && w + e < MAXPL; e += 32) pl[w + e] = (e + rot < nq ? e + rot : e + rot - nq) | (mode << 16) | (g << 20);
+      w += nq;
+      continue;
+    }
+    const int h = hk * G + g;
+    if (lane < 2 * MAXC / 32) cl[lane] = 0u;
+    __syncwarp();
+    {
+      // both counts are read before either index list (two round trips to memory, not four)
+      const int bm = p.t.mB == 1 ? 0 : b, hm = p.t.mH == 1 ? 0 : h;
+      const int kvblk = min(kt * 128 / p.t.KVB, p.t.nKV - 1);
+      const long long row = ((long long)bm * p.t.mH + hm) * p.t.nKV + kvblk;
+      const int tpb = p.t.nQ == 1 ? n_ctiles : p.t.QB / 128;
+      int num[2];
+#pragma unroll
+      for (int which = 0; which < 2; ++which) {
+        const int* nump = which ? p.t.full_q_num : p.t.q_num;
+        num[which] = nump != nullptr ? min(max(nump[row], 0), p.t.nQ) * tpb : 0;
+      }
+#pragma unroll
+      for (int which = 0; which < 2; ++which) {
+        const int* idxp = which ? p.t.full_q_idx : p.t.q_idx;
+        for (int e = lane; e < num[which]; e += 32) {
+          const int bi = e / tpb, ti = e - bi * tpb;
+          const int t = min(max(idxp[row * p.t.nQ + bi], 0), p.t.nQ - 1) * tpb + ti;
+          // (atomicOr on a generic address is 17 KB of code here, and its instruction-cache misses were paid by all warps)
+          if (t < n_ctiles)
+            asm volatile("red.shared.or.b32 [%0], %1;" ::"r"(fa_smem_u32(cl + which * (MAXC / 32) + (t >> 5))), "r"(1u << (t & 31)) : "memory");
+        }
+        __syncwarp();
+      }
+    }
+    for (int t0 = 0; t0 < n_ctiles; t0 += 32) {
+      const int t = t0 + lane;
+      // (only tiles below n_ctiles have a bit; a tile in both lists counts as full)
+      const int c = (cl[MAXC / 32 + (t0 >> 5)] >> lane) & 1u ? 2 : (int)((cl[t0 >> 5] >> lane) & 1u);
+      int n_t = 0;
+      if (c != 0)
+        for (int v = 0; v < PPT; ++v) n_t += (t * PPT + v) * BQ < p.Sq ? 1 : 0;
+      int inc = n_t;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const int o = __shfl_up_sync(0xffffffffu, inc, d);
+        if (lane >= d) inc += o;
+      }
+      for (int v = 0; v < n_t; ++v)
+        if (w + inc - n_t + v < MAXPL) pl[w + inc - n_t + v] = (t * PPT + v) | (c << 16) | (g << 20);
+      w += __shfl_sync(0xffffffffu, inc, 31);
+    }
+    __syncwarp();
+  }
+  return min(w, MAXPL);
+}
+
+// Row `kv` of the transposed mask bit matrix (of its first (batch, head) entry), or null: not built, or out of date.
+__device__ __forceinline__ const unsigned* bits_row(const FaParams& p, int kv) {
+  const bool there = p.t.mask_bits_t != nullptr && (p.t.mask_hold == nullptr || *p.t.mask_hold != 0);
+  return there ? p.t.mask_bits_t + (long long)kv * p.t.mask_t_stride : nullptr;
+}
+// mask_mod of kv row `kv` and q columns q0 .. q0+63 as bits: from that row, else from a rolled loop, which keeps the code
+// small (unrolled over a thread's columns it is 64 copies of the user's mask).
+__device__ __forceinline__ void keep_bits(fa_u32 (&keep)[2], const unsigned* bits, const FaParams& p, int b, int h, int gb, int gh, int q0, int kv) {
+#if FA_HAS_MASK_MOD
+  if (bits != nullptr) {
+    const long long entry = (long long)(p.t.mask_B == 1 ? 0 : b) * p.t.mask_H + (p.t.mask_H == 1 ? 0 : h);
+    const uint2 w = *(const uint2*)(bits + entry * p.t.mask_t_rows * p.t.mask_t_stride + (q0 >> 5));
+    keep[0] = w.x;
+    keep[1] = w.y;
+  } else {
+    fa_u32 w0 = 0u, w1 = 0u;
+#pragma unroll 2
+    for (int e = 0; e < 32; ++e) {
+      w0 |= (fa_mask_mod(gb, gh, q0 + e, kv) ? 1u : 0u) << e;
+      w1 |= (fa_mask_mod(gb, gh, q0 + 32 + e, kv) ? 1u : 0u) << e;
+    }
+    keep[0] = w0;
+    keep[1] = w1;
+  }
+#endif
+}
+// The low 16 keep bits of `w` as masks over pairs of 16-bit values.  P^T and dS^T are masked where they are packed, by two ANDs per
+// pair in a block that only masked tiles enter: the code of all others stays what it is without a mask.  (What the
+// exponential gave for a masked position, infinity too, goes with it.)
+__device__ __forceinline__ void keep_words(fa_u32 (&m)[8], fa_u32 w) {
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    const fa_u32 lo = (fa_u32)((int)(w << (31 - 2 * e)) >> 31), hi = (fa_u32)((int)(w << (30 - 2 * e)) >> 31);
+    m[e] = __byte_perm(lo, hi, 0x5410);
+  }
+}
+
+}  // namespace fa_bwd_items

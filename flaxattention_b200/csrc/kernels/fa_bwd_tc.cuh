@@ -1,5 +1,5 @@
 // Flash-attention backward for sm_100a on the 5th-generation tensor cores (fp16 / bf16,
-// D = Dv = 64 or 128).  One kernel computes dK, dV and dQ in a single pass over the
+// D = Dv = 64; D = 128: fa_bwd_tc128.cuh).  One kernel computes dK, dV and dQ in a single pass over the
 // (kv tile, q tile) pairs the BlockMask lists: five tcgen05.mma products per pair and one
 // exponential per score, where the two-scan reference kernel
 // (flaxattention/kernel/attention.py:423-553) and fa_bwd.cuh need seven products and two
@@ -8,19 +8,16 @@
 // The unit of work (an item) is a 128-row kv tile of one (batch, kv head) together with the q tiles
 // of the query heads that share it.  The kernel is persistent: one CTA per SM, every CTA works
 // through items it takes from a counter in global memory, and TMEM and the barriers are set up
-// once per CTA.  A pair is 128 kv rows x BQ query rows, BQ = 128 with D = 64 and 64 with
-// D = 128 (the 512 TMEM columns hold two D-wide accumulators, dK and dV, next to the pair's
-// score tiles only for the smaller q tile).  Everything is kept transposed so that dK and dV
+// once per CTA.  A pair is 128 kv rows x 128 query rows.  Everything is kept transposed so that dK and dV
 // have kv rows (TMEM lanes) and P^T can be fed to the tensor core straight from TMEM:
-//   1. S^T  = K Q^T                      (TMEM, 128 kv x BQ q, fp32)
+//   1. S^T  = K Q^T                      (TMEM, 128 kv x 128 q, fp32)
 //   2. dP^T = V dO^T                     (TMEM)
-//      p = 2^(x - lse), ds = p (dp - delta) score_mod'      thread (kv row, BQ/2 q columns)
+//      p = 2^(x - lse), ds = p (dp - delta) score_mod'      thread (kv row, 64 q columns)
 //      P^T -> TMEM (16 bit),  dS^T -> shared memory (16 bit, [kv][q], 128-byte swizzle)
 //   3. dV += P^T dO                      (A from TMEM)
 //   4. dK += dS^T Q                      (A = dS^T from smem, K-major)
-//   5. D = 64:   dQ   = dS K             (A = the same dS^T tile read MN-major, B = K; 128 q x 64 d)
-//      D = 128:  dQ^T = K^T dS^T         (A = K read MN-major, B = dS^T read MN-major; 128 d x 64 q)
-// Either way the dQ tile of a pair is 128 TMEM lanes x 64 columns of fp32.  It leaves through a
+//   5. dQ = dS K                         (A = the same dS^T tile read MN-major, B = K; 128 q x 64 d)
+// The dQ tile of a pair leaves through a
 // staging buffer and two bulk reduce-adds into an fp32 accumulation buffer (summation order
 // over kv tiles is not fixed; a small kernel scales, un-permutes and converts it afterwards).
 // dK and dV are written once per item.
@@ -31,37 +28,21 @@
 // S^T/dP^T of pair n+1 are issued as soon as the compute warps hold pair n in registers, so
 // the tensor core runs ahead of the element-wise work.
 //
-// TMEM (512 columns)   D = 64:  S^T 0-127, dP^T 128-255, P^T 256-319, dV 320-383, dK 384-447, dQ 448-511
-//                      D = 128: S^T 0-63, dP^T 64-127, P^T 128-159, dQ^T 192-255, dV 256-383, dK 384-511
+// TMEM (512 columns): S^T 0-127, dP^T 128-255, P^T 256-319, dV 320-383, dK 384-447, dQ 448-511
 // Every mbarrier wait is bounded (see fa_sm100.cuh).
 //
-// Compile-time parameters (macros): FA_DTYPE (0 fp16, 1 bf16), FA_D (64 or 128; Dv = D), FA_BWD_KV2
-// (two K / V buffers and one of dS^T instead of one and two, head dim 64 only).
+// Compile-time parameters (macros): FA_DTYPE (0 fp16, 1 bf16), FA_BWD_KV2 (two K / V buffers and one of dS^T instead of
+// one and two).
 #pragma once
-#include "fa_sm100.cuh"
-
-#ifndef FA_D
-#define FA_D 64
-#endif
-
-struct FaBwdTcParams {
-  FaParams p;
-  FaTensorMap tq, tk, tv, tdo;  // 4-d maps (D, S, H, B), 128-byte swizzle; box 64 x 128 rows (k, v), 64 x BQ rows (q, do)
-  FaTensorMap tdk, tdv;         // the outputs dK and dV, like tk and tv
-  float* dq_acc;                // per (b, h, BQ-row q tile): two [128 lanes][32 columns] fp32 blocks, 16-byte chunks of a row permuted
-  const float* nlse2;           // [B, Hq, ceil(Sq/128)*128]: -lse * log2(e); -inf for rows without mass / beyond Sq
-  const float* ndelta;          // same shape: -rowsum(O * dO); 0 beyond Sq
-  int* work_counter;            // zero at launch: items beyond the first of every CTA are handed out through it
-  int chunk_heads;              // (batch, kv head) pairs whose items are numbered together (see item_of)
-};
+#include "fa_bwd_items.cuh"
 
 namespace fa_btc {
+using namespace fa_bwd_items;
 
 constexpr int DT = FA_DTYPE;
-constexpr int D = FA_D;
-static_assert(D == 64 || D == 128, "head dim 64 or 128");
+constexpr int D = 64;
 constexpr int BT = 128;                    // kv rows of a tile
-constexpr int BQ = D == 64 ? 128 : 64;     // q rows of a pair
+constexpr int BQ = 128;                    // q rows of a pair
 constexpr int CW = BQ / 2;                 // q columns of one compute thread
 constexpr int DATOMS = D / 64;             // 64-element (128-byte) column groups of a K / V / Q / dO row
 constexpr int ATOM_BYTES = 128 * 128;      // 128 rows x 128 bytes
@@ -72,21 +53,20 @@ constexpr int DS_ATOMS = BQ / 64;                    // dS^T: [128 kv][BQ q] as 
 // K / V and dS^T buffers.  The pace of a pair is set by the hand-over of P^T and dS^T: with one dS^T buffer the
 // compute warps may store pair n + 1 only when products 3-5 of pair n are complete.  With two they wait for
 // product 3 of pair n (issued first) and, by the order of issue, products 4-5 of pair n - 1, which is
-// long past; the Q / dO ring gives up its fourth stage for it at D = 64.  Measured against one buffer and four
-// (three at D = 128) stages, backward alone, us: dense B8 H8 S2048 D64 231 -> 225, B4 H16/4 S2048 D64
-// 251 -> 239, dense B4 H8 S4096 D128 769 -> 745, causal B2 H16/4 S3001 D128 403 -> 388.
-// With D = 64 shared memory holds, instead of the second dS^T buffer, a second K / V buffer (FA_BWD_KV2): K and V of
+// long past; the Q / dO ring gives up its fourth stage for it.  Measured against one buffer and four
+// stages, backward alone, us: dense B8 H8 S2048 231 -> 225, B4 H16/4 S2048 251 -> 239.
+// Shared memory holds, instead of the second dS^T buffer, a second K / V buffer (FA_BWD_KV2): K and V of
 // the next item are loaded while the current one is computed and nothing waits at the change of items, which pays
 // when items are short (causal B8 H8 S2048, 8.5 pairs per item on average: 150 against 155 us) and costs when they
 // are long.  The host picks.
 #ifndef FA_BWD_KV2
 #define FA_BWD_KV2 0
 #endif
-constexpr int KVBUF = (D == 64 && FA_BWD_KV2) ? 2 : 1;
+constexpr int KVBUF = FA_BWD_KV2 ? 2 : 1;
 constexpr int NSTAGE = 3;
 constexpr int NDS = KVBUF == 1 ? 2 : 1;                // dS^T buffers
 constexpr int DS_BYTES = DS_ATOMS * ATOM_BYTES;
-constexpr int MAXPL = D == 64 ? 1024 : 2048;  // (head, q tile) pairs of one item (two such lists fit in shared memory)
+constexpr int MAXPL = 1024;              // (head, q tile) pairs of one item (two such lists fit in shared memory)
 constexpr int MAXC = 256;                // 128-row q tiles per head (Sq <= 32768)
 constexpr int NT = 512;
 constexpr int WARP_PRODUCER = 12, WARP_MMA = 13, WARP_MMA_B = 14, WARP_MMA_C = 15;
@@ -120,10 +100,7 @@ constexpr int SMEM_BYTES = OFF_CLS + 2 * MAXC / 8 + 1024;
 static_assert(SMEM_BYTES + 8 * 8 <= 227 * 1024, "shared memory");
 constexpr int TMEM_COLS = 512;
 constexpr int COL_S = 0, COL_DP = BQ, COL_P = 2 * BQ;
-constexpr int COL_DQ = D == 64 ? 448 : 192;
-constexpr int COL_DV = D == 64 ? 320 : 256;
-constexpr int COL_DK = D == 64 ? 384 : 384;
-static_assert(COL_P + BQ / 2 <= (D == 64 ? COL_DV : COL_DQ), "TMEM map");
+constexpr int COL_DV = 320, COL_DK = 384, COL_DQ = 448;
 
 constexpr int BAR_KV = 0;                   // [2] K and V of an item have landed in buffer kb
 // A stage's Q tile (with the row scalars) and dO tile are released separately: dO is last read by
@@ -143,29 +120,6 @@ constexpr int BAR_KVFREE = BAR_SFULL + 13;  // [2] (two K / V buffers) the store
 constexpr int LIST_CONSUMERS = 3 + 8 + 4;   // MMA issuers, compute warps, drain warps (one arrival each)
 
 __device__ __forceinline__ fa_u32 bar_addr(fa_u32 sb, int i) { return sb + OFF_BAR + i * 8; }
-
-__device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
-  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
-}
-__device__ __forceinline__ void bulk_reduce_add_f32(float* gdst, fa_u32 ssrc, fa_u32 bytes) {
-  asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;" ::"l"(gdst), "r"(ssrc), "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void bulk_wait_read0() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-__device__ __forceinline__ void bulk_wait0() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-// brings a tile into L2 ahead of the load that will need it
-__device__ __forceinline__ void tma_prefetch_l2_4d(const FaTensorMap* map, int c0, int c1, int c2, int c3) {
-  asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global.tile [%0, {%1, %2, %3, %4}];" ::"l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
-               : "memory");
-}
-
-// byte offset (in 16-byte units) of k-step kk of a K-major operand whose 64-element column groups
-// are `atom_bytes` apart: 32 bytes per step inside a 128-byte row, four steps per group
-__device__ __forceinline__ constexpr fa_u32 kstep_kmajor(int kk, int atom_bytes) {
-  return (fa_u32)(((kk >> 2) * atom_bytes + (kk & 3) * 32) >> 4);
-}
 
 // Element-wise work of one thread on a W-column chunk: scores s and dp (fp32, raw) for kv row
 // `kv` and q columns q0 .. q0+W-1 -> packed P^T and dS^T (16 bit).  q0 is a multiple of W (the
@@ -271,30 +225,12 @@ __device__ __forceinline__ void chunk(const float (&s)[W], const float (&dp)[W],
 }
 
 
-// Item number -> (kv head, batch, kv tile).  The first kv tiles of all heads come first (under a causal mask and
-// with attention sinks they are the heaviest), then chunk by chunk of `ch` heads, in a chunk heads fastest and the
-// kv tile slowest.  The CTAs work through the items in this order, so that at any time the dQ accumulator, Q and dO
-// of about one chunk of heads are in use: the host sizes it to stay in L2.  (Not with two K / V buffers: there the
-// items are short and the time to their first loads counts, causal B1 H8 S8192 D64 228 -> 242 us.)
-struct Item {
-  int hk, b, kt;
-};
-__device__ __forceinline__ Item item_of(int idx, int Hkv, int B, int n_kvt, int ch) {
+// Item number -> (kv head, batch, kv tile): with one K / V buffer by chunks of heads (fa_bwd_items::item_of), with two heads
+// fastest and the kv tile slowest (there the items are short and the time to their first loads counts, causal
+// B1 H8 S8192 228 -> 242 us).
+__device__ __forceinline__ Item item_at(int idx, int Hkv, int B, int n_kvt, int ch) {
   if (KVBUF == 2) return {idx % Hkv, (idx / Hkv) % B, idx / (Hkv * B)};
-  const unsigned heads = Hkv * B, i = idx;
-  unsigned head = i, kt = 0;
-  if ((unsigned)ch >= heads) {  // one chunk
-    kt = i / heads;
-    head = i - kt * heads;
-  } else if (i >= heads) {
-    const unsigned r = i - heads, per = ch * (n_kvt - 1), c = r / per, rr = r - c * per;
-    const unsigned n = min((unsigned)ch, heads - c * ch);
-    kt = rr / n;
-    head = c * ch + rr - kt * n;
-    ++kt;
-  }
-  const unsigned b = head / Hkv;
-  return {(int)(head - b * Hkv), (int)b, (int)kt};
+  return item_of(idx, Hkv, B, n_kvt, ch);
 }
 
 // What the producer has published of an item.  With two K / V buffers that is the item's number, `idx`, which the
@@ -303,74 +239,6 @@ __device__ __forceinline__ Item item_of(int idx, int Hkv, int B, int n_kvt, int 
 __device__ __forceinline__ Item read_item(int idx, const volatile int* item, int Hkv, int B) {
   if (KVBUF == 2) return {idx % Hkv, (idx / Hkv) % B, idx / (Hkv * B)};
   return {item[0], item[1], item[2]};
-}
-
-// The (query head, q tile) pairs of one item, written to `pl` by one warp: per head of the group,
-// the 128-row q tiles the BlockMask lists for the item's kv tile (class 1: apply mask_mod, 2: full)
-// in ascending order, each as 128 / BQ pairs.  Without tables every tile is listed.  Returns the
-// number of pairs (the same in every lane).  `cl` is scratch: one bit per q tile and class.
-__device__ __forceinline__ int build_pair_list(const FaParams& p, int hk, int b, int kt, int G, int n_ctiles,
-                                               unsigned* cl, int* pl, int lane) {
-  constexpr int PPT = 128 / BQ;
-  const bool tables = p.t.kv_num != nullptr && p.t.q_num != nullptr;
-  int w = 0;
-  for (int g = 0; g < G; ++g) {
-    if (!tables) {
-      const int nq = (p.Sq + BQ - 1) / BQ;
-      const int mode = FA_HAS_MASK_MOD ? 1 : 2;
-      // the items of a head start at different q tiles, so that the CTAs on one head do not add to the same
-      // dQ tile at the same time
-      const int rot = kt % nq;
-      for (int e = lane; e < nq && w + e < MAXPL; e += 32) pl[w + e] = (e + rot < nq ? e + rot : e + rot - nq) | (mode << 16) | (g << 20);
-      w += nq;
-      continue;
-    }
-    const int h = hk * G + g;
-    if (lane < 2 * MAXC / 32) cl[lane] = 0u;
-    __syncwarp();
-    {
-      // both counts are read before either index list (two round trips to memory, not four)
-      const int bm = p.t.mB == 1 ? 0 : b, hm = p.t.mH == 1 ? 0 : h;
-      const int kvblk = min(kt * BT / p.t.KVB, p.t.nKV - 1);
-      const long long row = ((long long)bm * p.t.mH + hm) * p.t.nKV + kvblk;
-      const int tpb = p.t.nQ == 1 ? n_ctiles : p.t.QB / 128;
-      int num[2];
-#pragma unroll
-      for (int which = 0; which < 2; ++which) {
-        const int* nump = which ? p.t.full_q_num : p.t.q_num;
-        num[which] = nump != nullptr ? min(max(nump[row], 0), p.t.nQ) * tpb : 0;
-      }
-#pragma unroll
-      for (int which = 0; which < 2; ++which) {
-        const int* idxp = which ? p.t.full_q_idx : p.t.q_idx;
-        for (int e = lane; e < num[which]; e += 32) {
-          const int bi = e / tpb, ti = e - bi * tpb;
-          const int t = min(max(idxp[row * p.t.nQ + bi], 0), p.t.nQ - 1) * tpb + ti;
-          if (t < n_ctiles) atomicOr(cl + which * (MAXC / 32) + (t >> 5), 1u << (t & 31));
-        }
-        __syncwarp();
-      }
-    }
-    for (int t0 = 0; t0 < n_ctiles; t0 += 32) {
-      const int t = t0 + lane;
-      // (only tiles below n_ctiles have a bit; a tile in both lists counts as full)
-      const int c = (cl[MAXC / 32 + (t0 >> 5)] >> lane) & 1u ? 2 : (int)((cl[t0 >> 5] >> lane) & 1u);
-      int n_t = 0;
-      if (c != 0)
-        for (int v = 0; v < PPT; ++v) n_t += (t * PPT + v) * BQ < p.Sq ? 1 : 0;
-      int inc = n_t;
-#pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        const int o = __shfl_up_sync(0xffffffffu, inc, d);
-        if (lane >= d) inc += o;
-      }
-      for (int v = 0; v < n_t; ++v)
-        if (w + inc - n_t + v < MAXPL) pl[w + inc - n_t + v] = (t * PPT + v) | (c << 16) | (g << 20);
-      w += __shfl_sync(0xffffffffu, inc, 31);
-    }
-    __syncwarp();
-  }
-  return min(w, MAXPL);
 }
 
 }  // namespace fa_btc
@@ -469,10 +337,10 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
       if (itc >= 2) ok = fa_mbar_wait_warp(bar_addr(sb, BAR_LISTFREE + lb), (fa_u32)(((itc >> 1) - 1) & 1), abort_flag);
       if (!ok) break;
       int* pl = pairs + lb * MAXPL;
-      const Item it = item_of(min(idx, n_items - 1), p.Hkv, p.B, n_kvt, P.chunk_heads);
+      const Item it = item_at(min(idx, n_items - 1), p.Hkv, p.B, n_kvt, P.chunk_heads);
       const int hk = it.hk, b = it.b, kt = it.kt;
       int np = -1;
-      if (idx < n_items) np = build_pair_list(p, hk, b, kt, G, n_ctiles, (unsigned*)(sm + OFF_CLS), pl, lane);
+      if (idx < n_items) np = build_pair_list<BQ, MAXPL, MAXC>(p, hk, b, kt, G, n_ctiles, (unsigned*)(sm + OFF_CLS), pl, lane);
       if (lane == 0) {
         item[4 * lb] = KVBUF == 2 ? idx : hk;
         item[4 * lb + 1] = b;
@@ -525,7 +393,7 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
         // K and V of the next item are asked into L2 now; their loads can only start when this
         // item is complete, and then they find the tiles close by
         if (KVBUF == 1 && ok && next < n_items) {
-          const Item i2 = item_of(next, p.Hkv, p.B, n_kvt, P.chunk_heads);
+          const Item i2 = item_at(next, p.Hkv, p.B, n_kvt, P.chunk_heads);
           const int hk2 = i2.hk, b2 = i2.b, n2 = i2.kt * BT;
           for (int a = 0; a < DATOMS; ++a) {
             tma_prefetch_l2_4d(&P.tk, a * 64, n2, hk2, b2);
@@ -670,17 +538,11 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
         if (!ok) break;
         fa_tc_fence_after();
         const fa_u32 loDS_mn = fa_desc_lo(sb + OFF_DS + (gn % NDS) * DS_BYTES, ATOM_BYTES);
-        // 5. K = 128 kv rows, a k-step is 16 rows = 2048 bytes of either operand.
-        //    D = 64:  dQ = dS K       A = dS^T read MN-major (M = 128 q: two 64-column atoms), B = K (N = 64 d)
-        //    D = 128: dQ^T = K^T dS^T A = K read MN-major (M = 128 d: two atoms), B = dS^T (N = 64 q)
+        // 5. dQ = dS K: K = 128 kv rows, a k-step is 16 rows = 2048 bytes of either operand; A = dS^T read MN-major
+        //    (M = 128 q: two 64-column atoms), B = K (N = 64 d)
 #pragma unroll
         for (int kk = 0; kk < BT / 16; ++kk)
-          if (leader) {
-            if (D == 64)
-              fa_mma_ss(tmem_u + COL_DQ, fa_desc_make(loDS_mn + kk * 128, HI), fa_desc_make(loK_mn + kk * 128, HI), IDESC_NN, kk > 0);
-            else
-              fa_mma_ss(tmem_u + COL_DQ, fa_desc_make(loK_mn + kk * 128, HI), fa_desc_make(loDS_mn + kk * 128, HI), IDESC_NN, kk > 0);
-          }
+          if (leader) fa_mma_ss(tmem_u + COL_DQ, fa_desc_make(loDS_mn + kk * 128, HI), fa_desc_make(loK_mn + kk * 128, HI), IDESC_NN, kk > 0);
         if (leader) {
           if (NDS == 1) fa_mma_commit(bar_addr(sb, BAR_PFREE));
           fa_mma_commit(bar_addr(sb, BAR_DQFULL));
@@ -752,15 +614,10 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
     ds[(C) / 2 + e] = d8[e];                                                                               \
   }                                                                                                        \
   if (!(LAST)) fa_tmem_wait_ld();
-          if (CW == 64) {
-            FA_STEP(sA, dA, sB, dB, 0, false)
-            FA_STEP(sB, dB, sA, dA, 16, false)
-            FA_STEP(sA, dA, sB, dB, 32 % CW, false)
-            FA_STEP(sB, dB, sA, dA, 48 % CW, true)
-          } else {
-            FA_STEP(sA, dA, sB, dB, 0, false)
-            FA_STEP(sB, dB, sA, dA, 16, true)
-          }
+          FA_STEP(sA, dA, sB, dB, 0, false)
+          FA_STEP(sB, dB, sA, dA, 16, false)
+          FA_STEP(sA, dA, sB, dB, 32, false)
+          FA_STEP(sB, dB, sA, dA, 48, true)
 #undef FA_STEP
         }
         // pin the packed results here: without this the compiler sinks part of the math below the
@@ -802,7 +659,7 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
   } else if (warp < 12) {
     // ================================ drain warps: dQ of every pair, dK / dV of every item =======
     const int lane_base = (warp & 3) * 32;
-    const int r = lane_base + lane;  // TMEM lane: q row of the pair (D = 64) or head-dim index (D = 128); kv row for dK / dV
+    const int r = lane_base + lane;  // TMEM lane: q row of the pair; kv row for dK / dV
     const fa_u32 t_lane = tmem + ((fa_u32)lane_base << 16);
     const fa_u32 t_dq = t_lane + COL_DQ;
     const int dtid = tid - 256;
