@@ -128,7 +128,7 @@ __device__ __forceinline__ fa_u32 bar_addr(fa_u32 sb, int i) { return sb + OFF_B
 // tile row.  nlse2 / ndelta point at the row scalars of column q0.
 template <int W>
 __device__ __forceinline__ void chunk(const float (&s)[W], const float (&dp)[W], const float* nlse2, const float* ndelta,
-                                      fa_u32 (&pp)[W / 2], fa_u32 (&ds)[W / 2], int mode, int q0, int kv, int gb, int gh,
+                                      fa_u32 (&pp)[W / 2], fa_u32 (&ds)[W / 2], int q0, int kv, int gb, int gh,
                                       float scale, float sc2) {
 #if !FA_ROUND_SCORES && (!FA_HAS_SCORE_MOD || defined(FA_SCORE_AFFINE))
   // no score_mod, or an affine one: two elements per instruction (packed fp32) wherever the
@@ -164,13 +164,7 @@ __device__ __forceinline__ void chunk(const float (&s)[W], const float (&dp)[W],
 #endif
       float x0, x1;
       fa_f2_unpack(x2, x0, x1);
-      float p0 = fa_ex2(x0), p1 = fa_ex2(x1);
-#if FA_HAS_MASK_MOD
-      if (mode == 1) {
-        p0 = fa_mask_mod(gb, gh, qi0, kv) ? p0 : 0.f;
-        p1 = fa_mask_mod(gb, gh, qi1, kv) ? p1 : 0.f;
-      }
-#endif
+      const float p0 = fa_ex2(x0), p1 = fa_ex2(x1);
       fa_u64 d2 = fa_mul2(fa_f2(p0, p1), fa_add2(fa_f2(dp[e + u], dp[e + u + 1]), nd2));
 #if FA_HAS_SCORE_MOD
       d2 = fa_mul2(d2, g2);
@@ -209,10 +203,7 @@ __device__ __forceinline__ void chunk(const float (&s)[W], const float (&dp)[W],
 #else
       x = fmaf(x, sc2, nlu);
 #endif
-      float pr = fa_ex2(x);
-#if FA_HAS_MASK_MOD
-      if (mode == 1) pr = fa_mask_mod(gb, gh, qi, kv) ? pr : 0.f;
-#endif
+      const float pr = fa_ex2(x);
       pv[u] = pr;
       dv[u] = pr * (dp[e + u] + ndu) * g;
     }
@@ -573,10 +564,15 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
       const int gb = b + p.b_off;
       const int kv = n0 + r;
       const bool row_ok = kv < p.Skv;
+      const unsigned* bits = bits_row(p, kv);
       for (int n = 0; n < np && ok; ++n, ++gn) {
         const int s = gn % NSTAGE;
         const int pr = pl[n];
-        const int m0 = (pr & 0xffff) * BQ, mode = (pr >> 16) & 0xf, gh = hk * G + (pr >> 20) + p.h_off;
+        const int m0 = (pr & 0xffff) * BQ, h = hk * G + (pr >> 20), gh = h + p.h_off;
+        const bool masked = FA_HAS_MASK_MOD && ((pr >> 16) & 0xf) == 1;
+        // the mask of this thread's 64 columns, read (where it was evaluated beforehand: while S^T is waited for) or evaluated
+        fa_u32 keep[2] = {0xffffffffu, 0xffffffffu};
+        if (masked && row_ok) keep_bits(keep, bits, p, b, h, gb, gh, m0 + half * CW, kv);
         ok = fa_mbar_wait_warp(bar_addr(sb, BAR_SFULL), (fa_u32)(gn & 1), abort_flag);
         if (ok) ok = fa_mbar_wait_warp(bar_addr(sb, BAR_QFULL + s), (fa_u32)((gn / NSTAGE) & 1), abort_flag);
         if (!ok) break;
@@ -605,7 +601,7 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
     fa_mbar_arrive(bar_addr(sb, BAR_SFREE));                                                               \
   }                                                                                                        \
   if (row_ok) {                                                                                            \
-    chunk<16>(SC, DC, rowp + c0 + (C), rowp + BQ + c0 + (C), p8, d8, mode, m0 + c0 + (C), kv, gb, gh, p.scale, sc2); \
+    chunk<16>(SC, DC, rowp + c0 + (C), rowp + BQ + c0 + (C), p8, d8, m0 + c0 + (C), kv, gb, gh, p.scale, sc2); \
   } else {                                                                                                 \
     _Pragma("unroll") for (int e = 0; e < 8; ++e) p8[e] = d8[e] = 0u;                                      \
   }                                                                                                        \
@@ -624,6 +620,18 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
         // wait that follows, onto the critical path between two groups of products
 #pragma unroll
         for (int e = 0; e < CW / 2; ++e) asm volatile("" : "+r"(pp[e]), "+r"(ds[e]));
+        if (masked) {
+          fa_u32 m8[8];
+#pragma unroll
+          for (int c = 0; c < CW / 16; ++c) {
+            keep_words(m8, keep[c >> 1] >> ((c & 1) * 16));
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              pp[8 * c + e] &= m8[e];
+              ds[8 * c + e] &= m8[e];
+            }
+          }
+        }
         // product 3 of the previous pair must be done with P^T, and products 4-5 of the last pair that used this
         // dS^T buffer with that
         if (gn > 0) {
