@@ -77,8 +77,8 @@ constexpr int WARP_PRODUCER = 12, WARP_MMA = 13, WARP_MMA_B = 14, WARP_MMA_C = 1
 // drain and issuing warps spilled, and the kernel was 4-5 % slower (dense backward 218 against 205 us,
 // attention sink 934 against 895; 192 / 64, 176 / 80, 168 / 88, 152 / 104 and 144 / 112 all lie within
 // 1 % of 160 / 96, 184 / 72 was as slow as 200 / 56).
-constexpr int REGS_COMPUTE = 160, REGS_OTHER = 96;
-static_assert(256 * (REGS_COMPUTE - 128) <= 256 * (128 - REGS_OTHER), "setmaxnreg.inc would wait forever");
+constexpr int REGS_COMPUTE = 152, REGS_DRAIN = 112, REGS_OTHER = 96;
+static_assert(2 * REGS_COMPUTE + REGS_DRAIN + REGS_OTHER <= 4 * 128, "setmaxnreg.inc would wait forever");
 
 // shared memory map (from a 1024-byte aligned base)
 constexpr int OFF_K = 0;
@@ -311,7 +311,8 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
   // a copy the compiler can see is the same in every lane (read through a broadcast)
   const fa_u32 tmem_u = __shfl_sync(0xffffffffu, tmem, 0);
 
-  if (warp >= 8) fa_setmaxnreg_dec<REGS_OTHER>();
+  if (warp >= 12) fa_setmaxnreg_dec<REGS_OTHER>();
+  else if (warp >= 8) fa_setmaxnreg_dec<REGS_DRAIN>();
 
   // Barrier phases: the pair-indexed barriers count the pairs of the CTA across its items (gn);
   // BAR_KV, BAR_FINAL and BAR_DKVFREE count the items that have pairs (kvc) - an item without
@@ -672,6 +673,7 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
     const fa_u32 t_dq = t_lane + COL_DQ;
     const int dtid = tid - 256;
     const int n_qtiles = sq_pad / BQ;
+    unsigned char* const dqrow = sm + OFF_DQ + r * 128;  // this thread's row of the staging buffer
     bool ok = true;
     int gn = 0, kvc = 0;
     for (int itc = 0; ok; ++itc) {
@@ -695,45 +697,33 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
         const int pr = pl[n];
         const int qt = pr & 0xffff, h = hk * G + (pr >> 20);
         ok = fa_mbar_wait_warp(bar_addr(sb, BAR_DQFULL), (fa_u32)(gn & 1), abort_flag);
-        if (!ok) misc[3] = 1;  // (read by all four warps behind the first barrier of the pair)
         fa_tc_fence_after();
-        // The 128 x 64 fp32 tile leaves in two halves of 32 columns through one 16 KB staging buffer:
-        // each half is one contiguous 16 KB block of the accumulation buffer.  16-byte chunk k of
-        // lane r goes to position k ^ (r & 7), which spreads the rows of a warp over the banks.
-        float* gdst = P.dq_acc + (((long long)b * p.Hq + h) * n_qtiles + qt) * (128 * 64);
-        unsigned char* strow = sm + OFF_DQ + r * 128;
-        float a[32];
-        if (ok) {
-          fa_tmem_ld32(t_dq, a);
-          fa_tmem_wait_ld();
-        }
+        if (!ok) break;
+        // The whole row comes into registers, so that the columns are free at once; it leaves by 32 columns through the
+        // warp's own 4 KB of staging, each time one bulk reduce-add of 4 KB (no barrier between the warps).  16-byte chunk k of
+        // lane r goes to position k ^ (r & 7), which spreads the rows over the banks.
+        float* gdst = P.dq_acc + (((long long)b * p.Hq + h) * n_qtiles + qt) * (128 * D) + (warp & 3) * 1024;
+        float a[2][32];
+        fa_tmem_ld32(t_dq, a[0]);
+        fa_tmem_ld32(t_dq + 32, a[1]);
+        fa_tmem_wait_ld();
+        fa_tc_fence_before();
+        fa_mbar_arrive(bar_addr(sb, BAR_DQFREE));
 #pragma unroll
-        for (int hf = 0; hf < 2; ++hf) {
-          // the previous bulk reduce must have finished reading the staging buffer
-          if (dtid == 0) bulk_wait_read0();
-          named_bar_sync(1, 128);
-          if (hf == 0 && misc[3] != 0) {
-            ok = false;
-            break;
-          }
+        for (int c = 0; c < 2; ++c) {
+          if (lane == 0) bulk_wait_read0();  // the previous reduce (or store) has read the staging buffer
+          __syncwarp();
 #pragma unroll
           for (int k = 0; k < 8; ++k)
-            *(float4*)(strow + ((k ^ (r & 7)) * 16)) = make_float4(a[4 * k], a[4 * k + 1], a[4 * k + 2], a[4 * k + 3]);
-          if (hf == 0) {
-            fa_tmem_ld32(t_dq + 32, a);
-            fa_tmem_wait_ld();
-            fa_tc_fence_before();
-            fa_mbar_arrive(bar_addr(sb, BAR_DQFREE));
-          }
+            *(float4*)(dqrow + ((k ^ (r & 7)) * 16)) = make_float4(a[c][4 * k], a[c][4 * k + 1], a[c][4 * k + 2], a[c][4 * k + 3]);
           fence_proxy_async();
-          named_bar_sync(1, 128);
-          if (dtid == 0) {
-            bulk_reduce_add_f32(gdst + hf * (DQ_HALF_BYTES / 4), sb + OFF_DQ, DQ_HALF_BYTES);
+          __syncwarp();
+          if (lane == 0) {
+            bulk_reduce_add_f32(gdst + c * 4096, sb + OFF_DQ + (warp & 3) * 4096, 4096);
             bulk_commit();
           }
         }
       }
-      if (!ok) break;
       // ---- dK (scaled) and dV of the item.  A thread owns one kv row (TMEM lane); 64 columns at a
       // time are converted into the staging buffer in the layout of a K tile (128-byte rows, 16-byte
       // chunk k of row r at k ^ (r & 7)) and leave through one tensor-map store, which writes whole
@@ -742,7 +732,7 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
       // An item without pairs has zeros written.
       if (np > 0) {
         const int kb = kvc % KVBUF;
-        ok = fa_mbar_wait_warp(bar_addr(sb, BAR_FINAL + kb), (fa_u32)((kvc / KVBUF) & 1), abort_flag);
+        if (ok) ok = fa_mbar_wait_warp(bar_addr(sb, BAR_FINAL + kb), (fa_u32)((kvc / KVBUF) & 1), abort_flag);
         if (!ok) misc[3] = 1;
         named_bar_sync(1, 128);
         if (misc[3] != 0) {
@@ -759,8 +749,8 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
           const int st_off = KVBUF == 2 ? (which == 0 ? OFF_K : OFF_V) + kb * KV_BYTES + a * ATOM_BYTES : OFF_DQ;
           unsigned char* strow = sm + st_off + r * 128;
           if (KVBUF == 1) {
-            // the previous bulk operation must have finished reading the staging buffer
-            if (dtid == 0) bulk_wait_read0();
+            // the previous bulk operations must have finished reading the staging buffer
+            if (lane == 0) bulk_wait_read0();
             named_bar_sync(1, 128);
           }
 #pragma unroll
@@ -814,11 +804,17 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
           }
         }
       }
-      if (np > 0) ++kvc;
+      if (np > 0) {
+        if (KVBUF == 1) {  // (the staging buffer is the warps' own again once the last store has read it)
+          if (dtid == 0) bulk_wait_read0();
+          named_bar_sync(1, 128);
+        }
+        ++kvc;
+      }
       __syncwarp();
       if (lane == 0) fa_mbar_arrive(bar_addr(sb, BAR_LISTFREE + lb));
     }
-    if (dtid == 0) bulk_wait0();
+    if (lane == 0) bulk_wait0();
   }
 
   // ---- teardown ------------------------------------------------------------------------------
