@@ -130,9 +130,9 @@ template <int W>
 __device__ __forceinline__ void chunk(const float (&s)[W], const float (&dp)[W], const float* nlse2, const float* ndelta,
                                       fa_u32 (&pp)[W / 2], fa_u32 (&ds)[W / 2], int q0, int kv, int gb, int gh,
                                       float scale, float sc2) {
-#if !FA_ROUND_SCORES && (!FA_HAS_SCORE_MOD || defined(FA_SCORE_AFFINE))
+#if !FA_HAS_SCORE_MOD || defined(FA_SCORE_AFFINE)
   // no score_mod, or an affine one: two elements per instruction (packed fp32) wherever the
-  // hardware has the form; only the exponentials and the mask are per element
+  // hardware has the form; only the exponentials are per element, and the rounding of the raw scores where it is asked for
 #if FA_HAS_SCORE_MOD && defined(FA_SCORE_LINEAR_Q)
   // the multiplier does not read q and the bias is linear in it (relative-position biases such as
   // ALiBi): both are taken once, at the first column of the chunk, and column e adds e times the slope
@@ -150,7 +150,11 @@ __device__ __forceinline__ void chunk(const float (&s)[W], const float (&dp)[W],
       const int qi0 = q0 | (e + u), qi1 = q0 | (e + u + 1);
       const fa_u64 nl2 = u == 0 ? fa_f2(nl.x, nl.y) : fa_f2(nl.z, nl.w);
       const fa_u64 nd2 = u == 0 ? fa_f2(nd.x, nd.y) : fa_f2(nd.z, nd.w);
-      const fa_u64 s2 = fa_f2(s[e + u], s[e + u + 1]);
+      float s0 = s[e + u], s1 = s[e + u + 1];
+#if FA_ROUND_SCORES
+      fa_round2<DT>(s0, s1);
+#endif
+      const fa_u64 s2 = fa_f2(s0, s1);
 #if FA_HAS_SCORE_MOD && defined(FA_SCORE_LINEAR_Q)
       const fa_u64 g2 = lin_g2;
       const fa_u64 b2 = fa_add2(fa_fma2(fa_f2((float)(e + u), (float)(e + u + 1)), lin_d2, lin_b2), nl2);
@@ -187,22 +191,14 @@ __device__ __forceinline__ void chunk(const float (&s)[W], const float (&dp)[W],
       const float nlu = u == 0 ? nl.x : (u == 1 ? nl.y : (u == 2 ? nl.z : nl.w));
       const float ndu = u == 0 ? nd.x : (u == 1 ? nd.y : (u == 2 ? nd.z : nd.w));
       float x = s[e + u];
-      float g = 1.f;
 #if FA_ROUND_SCORES
       {
         float dummy = 0.f;
         fa_round2<DT>(x, dummy);
       }
 #endif
-#if FA_HAS_SCORE_MOD && defined(FA_SCORE_AFFINE)
-      g = fa_score_mul(0.f, gb, gh, qi, kv);
-      x = fmaf(x, g * sc2, fa_score_add2(0.f, gb, gh, qi, kv) + nlu);
-#elif FA_HAS_SCORE_MOD
-      g = fa_score_mod_grad(x * scale, gb, gh, qi, kv);
+      const float g = fa_score_mod_grad(x * scale, gb, gh, qi, kv);
       x = fa_score_mod(x * scale, gb, gh, qi, kv) * FA_LOG2E + nlu;
-#else
-      x = fmaf(x, sc2, nlu);
-#endif
       const float pr = fa_ex2(x);
       pv[u] = pr;
       dv[u] = pr * (dp[e + u] + ndu) * g;

@@ -82,7 +82,7 @@ __device__ __forceinline__ fa_u32 bar_addr(fa_u32 sb, int i) { return sb + OFF_B
 // (the compiler can see that from how the caller builds it).  nlse2 points at the row scalar of column q0.
 __device__ __forceinline__ void p_chunk(const float (&s)[16], const float* nlse2, fa_u32 (&pp)[8], float* pg, int q0, int kv, int gb,
                                         int gh, float scale, float sc2) {
-#if !FA_ROUND_SCORES && (!FA_HAS_SCORE_MOD || defined(FA_SCORE_AFFINE))
+#if !FA_HAS_SCORE_MOD || defined(FA_SCORE_AFFINE)
 #if FA_HAS_SCORE_MOD && defined(FA_SCORE_LINEAR_Q)
   // (a bias linear in q under a multiplier that does not read it: see fa_bwd_tc.cuh)
   const float lin_g = fa_score_mul(0.f, gb, gh, q0, kv);
@@ -94,7 +94,11 @@ __device__ __forceinline__ void p_chunk(const float (&s)[16], const float* nlse2
   for (int e = 0; e < 16; e += 2) {
     const float2 nl = *(const float2*)(nlse2 + e);
     const fa_u64 nl2 = fa_f2(nl.x, nl.y);
-    const fa_u64 s2 = fa_f2(s[e], s[e + 1]);
+    float s0 = s[e], s1 = s[e + 1];
+#if FA_ROUND_SCORES
+    fa_round2<DT>(s0, s1);
+#endif
+    const fa_u64 s2 = fa_f2(s0, s1);
 #if FA_HAS_SCORE_MOD && defined(FA_SCORE_LINEAR_Q)
     const fa_u64 g2 = lin_g2;
     const fa_u64 x2 = fa_fma2(s2, lin_gs2, fa_add2(fa_fma2(fa_f2((float)e, (float)(e + 1)), lin_d2, lin_b2), nl2));
@@ -126,22 +130,14 @@ __device__ __forceinline__ void p_chunk(const float (&s)[16], const float* nlse2
     for (int u = 0; u < 2; ++u) {
       const float nlu = u == 0 ? nl.x : nl.y;
       float x = s[e + u];
-      float g = 1.f;
 #if FA_ROUND_SCORES
       {
         float dummy = 0.f;
         fa_round2<DT>(x, dummy);
       }
 #endif
-#if FA_HAS_SCORE_MOD && defined(FA_SCORE_AFFINE)
-      g = fa_score_mul(0.f, gb, gh, q0 | (e + u), kv);
-      x = fmaf(x, g * sc2, fa_score_add2(0.f, gb, gh, q0 | (e + u), kv) + nlu);
-#elif FA_HAS_SCORE_MOD
-      g = fa_score_mod_grad(x * scale, gb, gh, q0 | (e + u), kv);
+      const float g = fa_score_mod_grad(x * scale, gb, gh, q0 | (e + u), kv);
       x = fa_score_mod(x * scale, gb, gh, q0 | (e + u), kv) * FA_LOG2E + nlu;
-#else
-      x = fmaf(x, sc2, nlu);
-#endif
       const float pr = fa_ex2(x);
       pv[u] = pr;
       pg[e + u] = pr * g;
