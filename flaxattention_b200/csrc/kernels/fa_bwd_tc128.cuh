@@ -14,8 +14,8 @@
 // Why this shape: an instruction with N = 128 reads 8 KB of operands for 64 clocks of math, one with N = 64 6 KB for 32,
 // and shared memory delivers 128 bytes a clock: per 128 x 128 scores the five products read 256 KB (dV and dK take their A
 // operand from TMEM) where pairs of 64 query rows read 384, and a pair has the same number of hand-overs between
-// the roles for twice the work.  Against pairs of 64 query rows (kernel alone, us): dense B4 H8 S4096 668 -> 582, attention sink
-// B4 H16 S8192 881 -> 832, causal B2 H8 S4096 199 -> 176, causal + ALiBi B4 H16 S2048 238 -> 227, causal B2 H16/4 S3001 307 -> 268.
+// the roles for twice the work.  Against pairs of 64 query rows (kernel alone, us): dense B4 H8 S4096 668 -> 579, attention sink
+// B4 H16 S8192 881 -> 815, causal B2 H8 S4096 199 -> 170, causal + ALiBi B4 H16 S2048 238 -> 206.
 #pragma once
 #include "fa_bwd_items.cuh"
 
@@ -79,9 +79,11 @@ __device__ __forceinline__ fa_u32 bar_addr(fa_u32 sb, int i) { return sb + OFF_B
 
 // First half of the element-wise work on 16 columns of a thread's row: scores (raw) of kv row `kv`, q columns q0 .. q0+15
 // -> P^T packed to 16 bits and pg = p * (derivative of the score_mod), what dS^T needs of them.  q0 is a multiple of 16
-// (the compiler can see that from how the caller builds it).  nlse2 points at the row scalar of column q0.
-__device__ __forceinline__ void p_chunk(const float (&s)[16], const float* nlse2, fa_u32 (&pp)[8], float* pg, int q0, int kv, int gb,
-                                        int gh, float scale, float sc2) {
+// (the compiler can see that from how the caller builds it).  nlse2 points at the row scalar of column q0.  Bit e of
+// `keep` is the mask of column e, looked at if `masked`: as a select per element, which is faster here than masking the packed
+// words as at head dim 64 (causal + ALiBi B4 H16 S2048 206 against 224 us, attention sink 815 / 823) and masks dS^T too.
+__device__ __forceinline__ void p_chunk(const float (&s)[16], const float* nlse2, fa_u32 (&pp)[8], float* pg, bool masked, fa_u32 keep,
+                                        int q0, int kv, int gb, int gh, float scale, float sc2) {
 #if !FA_HAS_SCORE_MOD || defined(FA_SCORE_AFFINE)
 #if FA_HAS_SCORE_MOD && defined(FA_SCORE_LINEAR_Q)
   // (a bias linear in q under a multiplier that does not read it: see fa_bwd_tc.cuh)
@@ -112,7 +114,13 @@ __device__ __forceinline__ void p_chunk(const float (&s)[16], const float* nlse2
 #endif
     float x0, x1;
     fa_f2_unpack(x2, x0, x1);
-    const float p0 = fa_ex2(x0), p1 = fa_ex2(x1);
+    float p0 = fa_ex2(x0), p1 = fa_ex2(x1);
+#if FA_HAS_MASK_MOD
+    if (masked) {
+      p0 = (keep >> e) & 1u ? p0 : 0.f;
+      p1 = (keep >> (e + 1)) & 1u ? p1 : 0.f;
+    }
+#endif
     pp[e / 2] = fa_pack2<DT>(p0, p1);
 #if FA_HAS_SCORE_MOD
     fa_f2_unpack(fa_mul2(fa_f2(p0, p1), g2), pg[e], pg[e + 1]);
@@ -138,7 +146,10 @@ __device__ __forceinline__ void p_chunk(const float (&s)[16], const float* nlse2
 #endif
       const float g = fa_score_mod_grad(x * scale, gb, gh, q0 | (e + u), kv);
       x = fa_score_mod(x * scale, gb, gh, q0 | (e + u), kv) * FA_LOG2E + nlu;
-      const float pr = fa_ex2(x);
+      float pr = fa_ex2(x);
+#if FA_HAS_MASK_MOD
+      if (masked) pr = (keep >> (e + u)) & 1u ? pr : 0.f;
+#endif
       pv[u] = pr;
       pg[e + u] = pr * g;
     }
@@ -441,17 +452,13 @@ extern "C" __global__ void __launch_bounds__(fa_b128::NT, 1) fa_bwd_tc_kernel(co
         float pg[CW];
         {
           float sA[16], sB[16];
-          fa_u32 p8[8], m8[8];
+          fa_u32 p8[8];
           fa_tmem_ld16(tS, sA);
           fa_tmem_wait_ld();
 #define FA_STEP(CUR, NEXT, C)                                                                                      \
   if ((C) + 16 < CW) fa_tmem_ld16(tS + (C) + 16, NEXT);                                                            \
   if (row_ok) {                                                                                                    \
-    p_chunk(CUR, rowp + (C), p8, pg + (C), m0 + c0 + (C), kv, gb, gh, p.scale, sc2);                               \
-    if (masked) {                                                                                                  \
-      keep_words(m8, keep[(C) >> 5] >> ((C) & 31));                                                                \
-      _Pragma("unroll") for (int e = 0; e < 8; ++e) p8[e] &= m8[e];                                                \
-    }                                                                                                              \
+    p_chunk(CUR, rowp + (C), p8, pg + (C), masked, keep[(C) >> 5] >> ((C) & 31), m0 + c0 + (C), kv, gb, gh, p.scale, sc2); \
   } else {                                                                                                         \
     _Pragma("unroll") for (int e = 0; e < 8; ++e) p8[e] = 0u;                                                      \
     _Pragma("unroll") for (int e = 0; e < 16; ++e) pg[(C) + e] = 0.f;                                              \
@@ -473,7 +480,7 @@ extern "C" __global__ void __launch_bounds__(fa_b128::NT, 1) fa_bwd_tc_kernel(co
         fa_tc_fence_after();
         {
           float dA[16], dB[16];
-          fa_u32 d8[8], m8[8];
+          fa_u32 d8[8];
           fa_tmem_ld16(tD, dA);
           fa_tmem_wait_ld();
           // dS^T row r, to TMEM in the way of P^T and to shared memory: 16-byte chunk k of a 128-byte atom row goes to
@@ -482,10 +489,6 @@ extern "C" __global__ void __launch_bounds__(fa_b128::NT, 1) fa_bwd_tc_kernel(co
   if ((C) + 16 < CW) fa_tmem_ld16(tD + (C) + 16, NEXT);                                                            \
   if (row_ok) {                                                                                                    \
     ds_chunk(CUR, rowp + BQ + (C), pg + (C), d8);                                                                  \
-    if (masked) {                                                                                                  \
-      keep_words(m8, keep[(C) >> 5] >> ((C) & 31));                                                                \
-      _Pragma("unroll") for (int e = 0; e < 8; ++e) d8[e] &= m8[e];                                                \
-    }                                                                                                              \
   } else {                                                                                                         \
     _Pragma("unroll") for (int e = 0; e < 8; ++e) d8[e] = 0u;                                                      \
   }                                                                                                                \
