@@ -13,7 +13,8 @@
 // lane's own bits over the keys are a word of the row-major matrix (one predicated OR per position), what a mask reads per
 // query (a captured document id) is loaded once per lane and what it reads per key is a broadcast; five exchange steps
 // between the lanes turn the 32 words into those of the transposed matrix (some 25 instructions per 1024 positions).  Both matrices and
-// the block's count come out of one evaluation.  Bound by instruction issue.  8192 x 8192 positions of an attention-sink mask:
+// the block's count come out of one evaluation.  Where interval arithmetic over the mask's expression (fa_mask_range, from
+// the tracer) says that 32 x 32 positions are all kept or all not, none is evaluated.  Bound by instruction issue.  8192 x 8192 positions of an attention-sink mask:
 // 29 us; with lane = key, a ballot per row and a select for its word, 41.
 // Needs key blocks of whole 32-bit words and query blocks of whole words or a single one; other block sizes go to the
 // classify kernel below.
@@ -51,9 +52,17 @@ extern "C" __global__ void __launch_bounds__(128) fa_mask_scan_kernel(const __gr
         const int kv = k0 + c0 + 32 * c, left = p.KVB - (c0 + 32 * c);
         unsigned w = 0u;
         if (left > 0) {  // (the same for all threads)
+          int known = 1;
+#ifdef FA_HAS_MASK_RANGE
+          known = fa_mask_range(gb, gh, q - lane, q - lane + 31, kv, kv + 31);  // (the same for the warp)
+#endif
+          if (known == 1) {
 #pragma unroll
-          for (int e = 0; e < 32; ++e)
-            if (fa_mask_mod(gb, gh, q, kv + e)) w |= 1u << e;
+            for (int e = 0; e < 32; ++e)
+              if (fa_mask_mod(gb, gh, q, kv + e)) w |= 1u << e;
+          } else {
+            w = known ? 0xffffffffu : 0u;
+          }
           if (left < 32) w &= (1u << left) - 1u;
           if (!row_in) w = 0u;
         }

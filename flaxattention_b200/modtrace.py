@@ -1327,6 +1327,108 @@ def to_cuda(mod: TracedMod, name: str) -> str:
     return "\n".join([head] + lines + [f"  return {ret};", "}"]) + "\n"
 
 
+def to_cuda_range(mod: TracedMod, name: str) -> Optional[str]:
+    """Device function text of what a mask is over a rectangle of positions, by interval arithmetic on its graph:
+    ``int name(int b, int h, int q0, int q1, int kv0, int kv1)`` (bounds inclusive) gives 0 where it is false for every
+    position, 2 where it is true for every one, 1 where the intervals do not tell.  None if they never would.
+
+    An integer node is a pair of bounds, a boolean one a pair (certainly true, certainly false); floats, loads from
+    captured tensors and whatever else has no rule here is unknown.  A node whose values could leave int32 for indices below
+    ``_IDX_BOUND`` is unknown too (the arithmetic of the mask wraps there), and so is every rectangle beyond that bound."""
+    lines: List[str] = []
+    env: Dict[int, Optional[tuple]] = {}  # int: (lo text, hi text, static lo, static hi); bool: (true text, false text)
+    n = 0
+
+    def fresh(pair, ctype, static=None):
+        nonlocal n
+        a, b = f"a{n}", f"z{n}"
+        n += 1
+        lines.append(f"  const {ctype} {a} = {pair[0]}, {b} = {pair[1]};")
+        return (a, b) if static is None else (a, b) + static
+
+    def integer(lo, hi, slo, shi):
+        if slo < -(1 << 31) or shi >= 1 << 31:
+            return None
+        return fresh((lo, hi), "int", (slo, shi))
+
+    for e in _topo(mod.root):
+        x = [env.get(id(a)) for a in e.args]
+        known = all(v is not None for v in x)
+        ints = known and all(a.dtype == I32 for a in e.args)
+        c = e.args[1].value if len(e.args) == 2 and e.args[1].op == "const" and e.args[1].dtype == I32 else None
+        r = None
+        op = e.op
+        if op in ("q", "kv"):
+            r = (op + "0", op + "1", 0, _IDX_BOUND - 1)
+        elif op in ("b", "h"):
+            r = (op, op, 0, _IDX_BOUND - 1)
+        elif op == "const":
+            if e.dtype == I32:
+                v = f"({e.value})" if e.value != -(1 << 31) else "(-2147483647 - 1)"
+                r = (v, v, e.value, e.value)
+            elif e.dtype == B1:
+                r = ("true", "false") if e.value else ("false", "true")
+        elif e.dtype == I32 and ints:
+            if op == "add":
+                r = integer(f"{x[0][0]} + {x[1][0]}", f"{x[0][1]} + {x[1][1]}", x[0][2] + x[1][2], x[0][3] + x[1][3])
+            elif op == "sub":
+                r = integer(f"{x[0][0]} - {x[1][1]}", f"{x[0][1]} - {x[1][0]}", x[0][2] - x[1][3], x[0][3] - x[1][2])
+            elif op == "neg":
+                r = integer(f"-{x[0][1]}", f"-{x[0][0]}", -x[0][3], -x[0][2])
+            elif op in ("min", "max"):
+                f = min if op == "min" else max
+                r = integer(f"{op}({x[0][0]}, {x[1][0]})", f"{op}({x[0][1]}, {x[1][1]})", f(x[0][2], x[1][2]), f(x[0][3], x[1][3]))
+            elif op == "abs":
+                m = max(abs(x[0][2]), abs(x[0][3]))
+                r = integer(f"({x[0][0]} > 0 ? {x[0][0]} : ({x[0][1]} < 0 ? -{x[0][1]} : 0))", f"max(-{x[0][0]}, {x[0][1]})", 0, m) if m < 1 << 31 else None
+            elif op == "mul" and (c is not None or (e.args[0].op == "const")):
+                k, y = (c, x[0]) if c is not None else (e.args[0].value, x[1])
+                lo, hi = (y[0], y[1]) if k >= 0 else (y[1], y[0])
+                r = integer(f"{lo} * ({k})", f"{hi} * ({k})", min(y[2] * k, y[3] * k), max(y[2] * k, y[3] * k)) if k != -(1 << 31) else None
+            elif op == "floordiv" and c is not None and c > 0:
+                r = integer(f"fa_floordiv_i32({x[0][0]}, {c})", f"fa_floordiv_i32({x[0][1]}, {c})", x[0][2] // c, x[0][3] // c)
+            elif op == "rem" and c is not None and c > 0:
+                same = f"fa_floordiv_i32({x[0][0]}, {c}) == fa_floordiv_i32({x[0][1]}, {c})"
+                r = integer(f"({same}) ? fa_pymod_i32({x[0][0]}, {c}) : 0", f"({same}) ? fa_pymod_i32({x[0][1]}, {c}) : {c - 1}", 0, c - 1)
+            elif op == "shr" and c is not None and 0 <= c < 32:
+                r = integer(f"{x[0][0]} >> {c}", f"{x[0][1]} >> {c}", x[0][2] >> c, x[0][3] >> c)
+        elif e.dtype == I32 and op == "select" and known and e.args[0].dtype == B1:
+            (t, f), u, v = x
+            r = integer(f"{t} ? {u[0]} : ({f} ? {v[0]} : min({u[0]}, {v[0]}))", f"{t} ? {u[1]} : ({f} ? {v[1]} : max({u[1]}, {v[1]}))",
+                        min(u[2], v[2]), max(u[3], v[3]))
+        elif e.dtype == B1 and op in ("lt", "le", "gt", "ge", "eq", "ne") and ints:
+            u, v = (x[1], x[0]) if op in ("gt", "ge") else (x[0], x[1])
+            if op in ("lt", "gt"):
+                r = fresh((f"{u[1]} < {v[0]}", f"{u[0]} >= {v[1]}"), "bool")
+            elif op in ("le", "ge"):
+                r = fresh((f"{u[1]} <= {v[0]}", f"{u[0]} > {v[1]}"), "bool")
+            else:
+                same = f"{u[0]} == {v[1]} && {u[1]} == {v[0]}"
+                apart = f"{u[1]} < {v[0]} || {v[1]} < {u[0]}"
+                r = fresh((same, apart) if op == "eq" else (apart, same), "bool")
+        elif e.dtype == B1 and op in ("and", "or"):
+            u, v = (y if y is not None else ("false", "false") for y in x)
+            if x[0] is not None or x[1] is not None:
+                j, k = ("&&", "||") if op == "and" else ("||", "&&")
+                r = fresh((f"{u[0]} {j} {v[0]}", f"{u[1]} {k} {v[1]}"), "bool")
+        elif e.dtype == B1 and op == "not" and known:
+            r = (x[0][1], x[0][0])
+        elif e.dtype == B1 and op == "select" and known and all(a.dtype == B1 for a in e.args):
+            (t, f), u, v = x
+            r = fresh((f"({t} && {u[0]}) || ({f} && {v[0]}) || ({u[0]} && {v[0]})", f"({t} && {u[1]}) || ({f} && {v[1]}) || ({u[1]} && {v[1]})"), "bool")
+        elif op == "cast_b1" and ints:
+            r = fresh((f"{x[0][0]} > 0 || {x[0][1]} < 0", f"{x[0][0]} == 0 && {x[0][1]} == 0"), "bool")
+        elif op == "cast_i32" and known and e.args[0].dtype == B1:
+            r = integer(f"{x[0][0]} ? 1 : 0", f"{x[0][1]} ? 0 : 1", 0, 1)
+        env[id(e)] = r
+    root = env[id(mod.root)]
+    if root is None:
+        return None
+    bound = " || ".join(f"(unsigned){v} >= {_IDX_BOUND}u" for v in ("b", "h", "q0", "q1", "kv0", "kv1"))
+    return "\n".join([f"__device__ __forceinline__ int {name}(int b, int h, int q0, int q1, int kv0, int kv1) {{",
+                      f"  if ({bound}) return 1;"] + lines + [f"  return {root[0]} ? 2 : ({root[1]} ? 0 : 1);", "}"]) + "\n"
+
+
 def _buffer_storage(buf, span: int) -> np.ndarray:
     """The first `span` elements of the storage behind a captured tensor (strided view undone)."""
     try:
@@ -1523,6 +1625,9 @@ class ModSet:
         self.mask_reads_h = self.mask is not None and _depends_on(self.mask.root, "h", {})
         if self.mask is not None:
             parts.append(to_cuda(self.mask, "fa_mask_mod"))
+            over_range = to_cuda_range(self.mask, "fa_mask_range")
+            if over_range is not None:
+                parts.append("#define FA_HAS_MASK_RANGE 1\n" + over_range)
         else:
             parts.append("__device__ __forceinline__ bool fa_mask_mod(int, int, int, int) { return true; }\n")
         self.source = "".join(parts)
