@@ -1722,13 +1722,22 @@ static int fill_waves(long long bh, int cmax, int slots) {
 //     merge; at least four tiles per CTA.
 //   * Many heads: one split leaves SMs with one CTA beside SMs with two.  Over long caches (24 tiles per CTA and more) several
 //     waves that end nearly full are faster then.
+//   * More than 16 rows: the products, not the keys' way from memory, set the pace, and the SM with the most CTAs the end. Splits
+//     there are where they take a quarter off that (B5 H32/8 62 rows Skv1935 D128: one split 98 us, three 79).
 //   * Few heads: up to FA_DECODE_MAX_CLUSTER splits are merged inside a cluster, more by the combine kernel; where even a
 //     cluster per head leaves SMs idle, one CTA per SM.
 // Against as many CTAs as fit with the last wave 95 % full (us, before / now): B16 H32/8 Skv8191 D128 124 / 113, B4 H32
 // Skv8192 D64 76.8 / 65.6, B4 H8 Skv8192 D128 54 / 41, B8 H32/8 8 rows Skv5000 D128 76.8 / 55.3, B32 H8 Skv2048 42.0 / 38.9.
-static int general_decode_splits(long long bh, int tiles, int per_sm, int sm_count) {
+static int general_decode_splits(long long bh, int tiles, int per_sm, int sm_count, int row_groups) {
   const int cmax = std::min(std::max(tiles / 4, 1), 64);
   const int c = (int)std::min<long long>(cmax, std::max<long long>(1, std::min(per_sm, 2) * sm_count / bh));
+  if (c == 1 && row_groups > 1) {
+    const auto most = [&](int k) { return (double)((bh * k + sm_count - 1) / sm_count) / k; };
+    int best = 1;
+    for (int k = 2; k <= cmax; ++k)
+      if (most(k) <= 0.75 * most(1) && (best == 1 || most(k) + 0.1 * k < most(best) + 0.1 * best)) best = k;
+    return best;
+  }
   if (c == 1) {
     int best = 1;
     double best_fill = 0.88;
@@ -1762,12 +1771,12 @@ int fa_decode_num_splits(const fa_attn_params* p, int sm_count) {
   }
   // general kernel: as many CTAs per SM as its shared memory allows (at most four by registers)
   int per_sm = 2;
-  DecCfg c;
+  DecCfg c{16, 0, 0};
   if (pick_decode(p->dtype, p->D, p->Dv, pack ? p->Sq * (p->Hq / p->Hkv) : p->Sq, nullptr, c) == FA_OK) {
     per_sm = (228 * 1024) / (c.smem + 1024);
     per_sm = per_sm < 1 ? 1 : (per_sm > 4 ? 4 : per_sm);
   }
-  return general_decode_splits(bh, tiles, per_sm, sm_count);
+  return general_decode_splits(bh, tiles, per_sm, sm_count, c.BM / 16);
 }
 
 size_t fa_decode_workspace_bytes(const fa_attn_params* p, int num_splits) {
