@@ -1717,27 +1717,24 @@ static int fill_waves(long long bh, int cmax, int slots) {
   return best;
 }
 
+// CTAs of the general decode kernel that share an SM: by shared memory, at most four by registers
+static int decode_ctas_per_sm(const DecCfg& c) { return std::min(std::max((228 * 1024) / (c.smem + 1024), 1), 4); }
+
 // Splits of the general decode kernel for `bh` tiles of query rows over `tiles` 128-key tiles.
 //   * Two CTAs per SM, all resident at once, stream as fast as more do, and every further split costs its start and its
 //     merge; at least four tiles per CTA.
 //   * Many heads: one split leaves SMs with one CTA beside SMs with two.  Over long caches (24 tiles per CTA and more) several
 //     waves that end nearly full are faster then.
-//   * More than 16 rows: the products, not the keys' way from memory, set the pace, and the SM with the most CTAs the end. Splits
-//     there are where they take a quarter off that (B5 H32/8 62 rows Skv1935 D128: one split 98 us, three 79).
+//   * More than 16 rows: the products, not the keys' way from memory, set the pace, and what counts is a last wave that is nearly
+//     full (B5 H32/8 62 rows Skv1935 D128: one split 96 us, three 87; B7 H32 64 rows Skv30000 1260 / 960 with nine).
 //   * Few heads: up to FA_DECODE_MAX_CLUSTER splits are merged inside a cluster, more by the combine kernel; where even a
 //     cluster per head leaves SMs idle, one CTA per SM.
 // Against as many CTAs as fit with the last wave 95 % full (us, before / now): B16 H32/8 Skv8191 D128 124 / 113, B4 H32
-// Skv8192 D64 76.8 / 65.6, B4 H8 Skv8192 D128 54 / 41, B8 H32/8 8 rows Skv5000 D128 76.8 / 55.3, B32 H8 Skv2048 42.0 / 38.9.
+// Skv8192 D64 76.8 / 65.6, B4 H8 Skv8192 D128 54 / 41, B32 H8 Skv2048 42.0 / 38.9.
 static int general_decode_splits(long long bh, int tiles, int per_sm, int sm_count, int row_groups) {
   const int cmax = std::min(std::max(tiles / 4, 1), 64);
+  if (row_groups > 1) return fill_waves(bh, cmax, per_sm * sm_count);
   const int c = (int)std::min<long long>(cmax, std::max<long long>(1, std::min(per_sm, 2) * sm_count / bh));
-  if (c == 1 && row_groups > 1) {
-    const auto most = [&](int k) { return (double)((bh * k + sm_count - 1) / sm_count) / k; };
-    int best = 1;
-    for (int k = 2; k <= cmax; ++k)
-      if (most(k) <= 0.75 * most(1) && (best == 1 || most(k) + 0.1 * k < most(best) + 0.1 * best)) best = k;
-    return best;
-  }
   if (c == 1) {
     int best = 1;
     double best_fill = 0.88;
@@ -1773,8 +1770,7 @@ int fa_decode_num_splits(const fa_attn_params* p, int sm_count) {
   int per_sm = 2;
   DecCfg c{16, 0, 0};
   if (pick_decode(p->dtype, p->D, p->Dv, pack ? p->Sq * (p->Hq / p->Hkv) : p->Sq, nullptr, c) == FA_OK) {
-    per_sm = (228 * 1024) / (c.smem + 1024);
-    per_sm = per_sm < 1 ? 1 : (per_sm > 4 ? 4 : per_sm);
+    per_sm = decode_ctas_per_sm(c);
   }
   return general_decode_splits(bh, tiles, per_sm, sm_count, c.BM / 16);
 }
@@ -1806,8 +1802,10 @@ int fa_decode(fa_module* m, const fa_attn_params* p, int num_splits, void* works
   // partial results in memory (us: B8 H8 Skv2048 D64 21.4 -> 16.4, B4 H8 Skv8192 D128 46 -> 41).  Where the grid takes several waves
   // a cluster has to wait for room for all its CTAs (B32 H8 Skv16384 D64, five splits: 188 -> 197), and the partial
   // results go through memory and the combine kernel.
+  // (Clusters fill the SMs of a GPC in whole: at two CTAs per SM, 288 of 296 places in clusters of six take a second round, 54 -> 78 us.)
+  const long long places = tc ? 0 : std::min<long long>(2, decode_ctas_per_sm(c)) * device_sm_count();
   const bool cluster = !tc && num_splits > 1 && num_splits <= FA_DECODE_MAX_CLUSTER &&
-                       (long long)p->B * (pack ? p->Hkv : p->Hq) * num_splits <= 2 * device_sm_count();
+                       (long long)p->B * (pack ? p->Hkv : p->Hq) * num_splits <= (decode_ctas_per_sm(c) > 2 ? places : places * 87 / 100);
   if (need && !cluster) {
     const size_t rows = (size_t)p->B * p->Hq * num_splits * p->Sq;
     kp.part_o = (float*)workspace;
