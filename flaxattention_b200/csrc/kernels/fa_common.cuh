@@ -74,6 +74,15 @@ __device__ __forceinline__ void fa_round2(float& a, float& b) {
     b = __uint_as_float(r & 0xffff0000u);
   }
 }
+// what the rounding to DT leaves of two values (exact in fp32)
+template <int DT>
+__device__ __forceinline__ void fa_rest2(float a, float b, float& ra, float& rb) {
+  ra = a;
+  rb = b;
+  fa_round2<DT>(a, b);
+  ra -= a;
+  rb -= b;
+}
 #ifndef FA_ROUND_SCORES
 #define FA_ROUND_SCORES 0
 #endif
@@ -333,9 +342,9 @@ __device__ __forceinline__ void fa_mma_nt_smemA(float (&acc)[NN / 8][4], fa_u32 
     }
   }
 }
-// out[16 x NN] += P[16 x KK] * B, P taken from an accumulator (rounded to DT), B stored
-// [KK rows][NN cols] row-major ("NN")
-template <int DT, int KK, int NN>
+// out[16 x NN] += P[16 x KK] * B, P taken from an accumulator (rounded to DT; TWO: and what the rounding
+// left of it, rounded again, as a second product), B stored [KK rows][NN cols] row-major ("NN")
+template <int DT, int KK, int NN, bool TWO = false>
 __device__ __forceinline__ void fa_mma_nn(float (&out)[NN / 8][4], const float (&pacc)[KK / 8][4], fa_u32 sB, int pitchB,
                                           int lane) {
 #pragma unroll
@@ -345,6 +354,16 @@ __device__ __forceinline__ void fa_mma_nn(float (&out)[NN / 8][4], const float (
     a[1] = fa_pack2<DT>(pacc[2 * kj][2], pacc[2 * kj][3]);
     a[2] = fa_pack2<DT>(pacc[2 * kj + 1][0], pacc[2 * kj + 1][1]);
     a[3] = fa_pack2<DT>(pacc[2 * kj + 1][2], pacc[2 * kj + 1][3]);
+    fa_u32 rest[4];
+    if (TWO) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float (&x)[4] = pacc[2 * kj + (i >> 1)];
+        float r0, r1;
+        fa_rest2<DT>(x[(i & 1) * 2], x[(i & 1) * 2 + 1], r0, r1);
+        rest[i] = fa_pack2<DT>(r0, r1);
+      }
+    }
 #pragma unroll
     for (int dj = 0; dj < NN / 16; ++dj) {
       fa_u32 r0, r1, r2, r3;
@@ -353,6 +372,10 @@ __device__ __forceinline__ void fa_mma_nn(float (&out)[NN / 8][4], const float (
       fa_ldsm_x4_t(sB + r * pitchB + c * 2, r0, r1, r2, r3);
       fa_mma16816<DT>(out[2 * dj], a, r0, r1);
       fa_mma16816<DT>(out[2 * dj + 1], a, r2, r3);
+      if (TWO) {
+        fa_mma16816<DT>(out[2 * dj], rest, r0, r1);
+        fa_mma16816<DT>(out[2 * dj + 1], rest, r2, r3);
+      }
     }
   }
 }

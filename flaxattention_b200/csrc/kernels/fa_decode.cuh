@@ -72,6 +72,14 @@ constexpr int MRG_PITCH = DV + 4;  // floats per merged row: O[DV], m, l, pad
 constexpr int MRG_BYTES = CG * BM * MRG_PITCH * 4;
 constexpr int PIPE_BYTES = STAGES * (K_BYTES + V_BYTES);
 constexpr int SMEM_BYTES = Q_BYTES + (PIPE_BYTES > MRG_BYTES ? PIPE_BYTES : MRG_BYTES);
+// With one row group the probabilities go into P.V in two parts, rounded and what the rounding left.  One part alone has no error
+// where a probability is exactly 1, at a running maximum, so that the fewer of these (fewer splits) the worse the results:
+// B16 H32/8 Skv8191 D128 bf16, relative error against 64 bits, 2.11e-3 with three splits, 2.20e-3 with two, 1.66e-3 in two parts, nearly all
+// of it the rounding of the output.  Up to 8 rows the second part lies in the 8 rows of the instruction that hold no query
+// and costs nothing; up to 16 it takes a second instruction (B3 H16 Skv4096 D128, 16 rows: 28.3 us, 28.7 without).  The 16 rows of one
+// head at head dim 64 have no time for that (B8 H8 Skv8192 34.3 us, 31.5 without) and stay with one part (error 2.18e-3 bf16; of the tcgen05 kernel there 2.32e-3).
+constexpr bool TWO_PARTS = RG == 1;
+constexpr bool SECOND_MMA = TWO_PARTS && (PACK || D > 64);
 
 static_assert(DT != FA_DT_F32, "the decode kernel takes 16-bit inputs");
 static_assert(BM == 16 || BM == 32 || BM == 64, "BM must be 16, 32 or 64");
@@ -203,7 +211,11 @@ extern "C" __global__ void __launch_bounds__(fa_dec::NT) fa_decode_kernel(const 
       // rows 8..15 of a row group hold no query when there are at most 8 (+ 16 rg) rows: nothing to do for them
       if (rg * 16 + hh * 8 >= R) {
 #pragma unroll
-        for (int j = 0; j < WN / 8; ++j) s[j][hh * 2] = s[j][hh * 2 + 1] = 0.f;
+        for (int j = 0; j < WN / 8; ++j) {
+          // (hh = 1, TWO_PARTS: the second part of the rows 8 above)
+          if (TWO_PARTS) fa_rest2<DT>(s[j][0], s[j][1], s[j][2], s[j][3]);
+          else s[j][hh * 2] = s[j][hh * 2 + 1] = 0.f;
+        }
         continue;
       }
       const int row = rg * 16 + hh * 8 + (lane >> 2);
@@ -258,6 +270,10 @@ extern "C" __global__ void __launch_bounds__(fa_dec::NT) fa_decode_kernel(const 
         for (int j = 0; j < DV / 8; ++j) {
           o[j][hh * 2] *= corr;
           o[j][hh * 2 + 1] *= corr;
+          if (TWO_PARTS && R <= 8) {
+            o[j][2] *= corr;
+            o[j][3] *= corr;
+          }
         }
       }
     }
@@ -270,7 +286,8 @@ extern "C" __global__ void __launch_bounds__(fa_dec::NT) fa_decode_kernel(const 
     have_nxt = have && next_tile(n0_nxt, full_nxt);
     if (have_nxt) load_k(cur, n0_nxt);
     fa_cp_commit();
-    fa_mma_nn<DT, WN, DV>(o, s, sV + cur * V_BYTES + cg * WN * PV, PV, lane);
+    if (SECOND_MMA && R > 8) fa_mma_nn<DT, WN, DV, true>(o, s, sV + cur * V_BYTES + cg * WN * PV, PV, lane);
+    else fa_mma_nn<DT, WN, DV>(o, s, sV + cur * V_BYTES + cg * WN * PV, PV, lane);
     cur ^= 1;
   }
 
@@ -279,6 +296,13 @@ extern "C" __global__ void __launch_bounds__(fa_dec::NT) fa_decode_kernel(const 
   fa_cp_wait<0>();
   __syncthreads();
   float* mrg = (float*)(smem + Q_BYTES);
+  if (TWO_PARTS && R <= 8) {
+#pragma unroll
+    for (int j = 0; j < DV / 8; ++j) {
+      o[j][0] += o[j][2];
+      o[j][1] += o[j][3];
+    }
+  }
 #pragma unroll
   for (int hh = 0; hh < 2; ++hh) {
     float l = l_run[hh];

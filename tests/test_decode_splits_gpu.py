@@ -53,3 +53,27 @@ def test_many_splits_match_the_oracle():
     ref, ref_lse = flax_attention_oracle(q.float(), k.float(), v.float())
     assert (out.double() - ref.double()).abs().max().item() <= 2e-2
     assert lse_err(lse, ref_lse)[0] <= 1e-4
+
+
+@pytest.mark.parametrize("Hq,Hkv,Sq,Skv,D,Dv", [
+    (3, 3, 1, 2000, 64, 64),
+    (8, 2, 2, 1111, 128, 128),   # eight rows of a packed tile: the second part lies over all eight spare rows
+    (2, 2, 9, 1024, 128, 48),    # the first that takes a second instruction
+    (4, 1, 4, 900, 64, 16),      # the last, four heads to a tile
+    (1, 1, 5, 1500, 256, 256),
+])
+@pytest.mark.parametrize("splits", [1, 2, 9])
+@pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16])
+def test_up_to_16_rows_lose_no_more_than_the_output_rounds(Hq, Hkv, Sq, Skv, D, Dv, splits, dt):
+    """Against 64 bits of the same inputs.  Bound: half a unit in the last place of the result, and of the sum a part of
+    max|v|: what two parts leave of a probability (2^-17 bf16, 2^-23 fp16, relative), and exponential and fp32 sums (2^-22 and
+    at most 2^-19 over up to 30 steps of 16 keys in a warp and 16 merges).  Probabilities of one part miss it."""
+    q, k, v = qkv(2, Hq, Hkv, Sq, Skv, D, Dv, dtype=dt)
+    out, _ = _run(q, k, v, None, splits)
+    G = Hq // Hkv
+    kd, vd = (t.double().repeat_interleave(G, 1) for t in (k, v))
+    ref = torch.softmax(q.double() @ kd.transpose(-1, -2) * D ** -0.5, -1) @ vd
+    bf16 = dt == torch.bfloat16
+    half = torch.ldexp(torch.ones_like(ref), torch.frexp(ref).exponent - (9 if bf16 else 12)).clamp(min=0.0 if bf16 else 2.0 ** -25)
+    over = ((out.double() - ref).abs() - half).max().item()
+    assert over <= (2.0 ** -17 + 2.0 ** -18 if bf16 else 2.0 ** -18) * v.double().abs().max().item()
