@@ -155,10 +155,11 @@ __device__ __forceinline__ void elem16(float (&s)[16], float (&dp)[16], const fl
 #else
       x = fmaf(s[e + u], sc2, nlu);
 #endif
-      float pr = fa_ex2(x);
-      pr = ((keep >> (e + u)) & 1u) ? pr : 0.f;
-      s[e + u] = pr;
-      dp[e + u] = pr * (dp[e + u] + ndu) * g;
+      // (both are selected: the derivative of a score_mod may be infinite where the mask is false, and 0 times that is NaN)
+      const bool in = (keep >> (e + u)) & 1u;
+      const float pr = fa_ex2(x);
+      s[e + u] = in ? pr : 0.f;
+      dp[e + u] = in ? pr * (dp[e + u] + ndu) * g : 0.f;
     }
   }
 }

@@ -81,7 +81,10 @@ __device__ __forceinline__ fa_u32 bar_addr(fa_u32 sb, int i) { return sb + OFF_B
 // -> P^T packed to 16 bits and pg = p * (derivative of the score_mod), what dS^T needs of them.  q0 is a multiple of 16
 // (the compiler can see that from how the caller builds it).  nlse2 points at the row scalar of column q0.  Bit e of
 // `keep` is the mask of column e, looked at if `masked`: as a select per element, which is faster here than masking the packed
-// words as at head dim 64 (causal + ALiBi B4 H16 S2048 206 against 224 us, attention sink 815 / 823) and masks dS^T too.
+// words as at head dim 64 (causal + ALiBi B4 H16 S2048 206 against 224 us, attention sink 815 / 823).  Both the probability and pg
+// are selected, unless the tracer knows the derivative of the score_mod to be finite everywhere (FA_SCORE_GRAD_FINITE): it may be
+// infinite where the mask is false, and 0 times that is NaN (the second select: causal + ALiBi B8 H8 S2048, with the conversion of
+// dQ, 245 -> 254 us).
 __device__ __forceinline__ void p_chunk(const float (&s)[16], const float* nlse2, fa_u32 (&pp)[8], float* pg, bool masked, fa_u32 keep,
                                         int q0, int kv, int gb, int gh, float scale, float sc2) {
 #if !FA_HAS_SCORE_MOD || defined(FA_SCORE_AFFINE)
@@ -124,6 +127,12 @@ __device__ __forceinline__ void p_chunk(const float (&s)[16], const float* nlse2
     pp[e / 2] = fa_pack2<DT>(p0, p1);
 #if FA_HAS_SCORE_MOD
     fa_f2_unpack(fa_mul2(fa_f2(p0, p1), g2), pg[e], pg[e + 1]);
+#if FA_HAS_MASK_MOD && !defined(FA_SCORE_GRAD_FINITE)
+    if (masked) {
+      pg[e] = (keep >> e) & 1u ? pg[e] : 0.f;
+      pg[e + 1] = (keep >> (e + 1)) & 1u ? pg[e + 1] : 0.f;
+    }
+#endif
 #else
     pg[e] = p0;
     pg[e + 1] = p1;
@@ -147,11 +156,11 @@ __device__ __forceinline__ void p_chunk(const float (&s)[16], const float* nlse2
       const float g = fa_score_mod_grad(x * scale, gb, gh, q0 | (e + u), kv);
       x = fa_score_mod(x * scale, gb, gh, q0 | (e + u), kv) * FA_LOG2E + nlu;
       float pr = fa_ex2(x);
+      pg[e + u] = pr * g;
 #if FA_HAS_MASK_MOD
-      if (masked) pr = (keep >> (e + u)) & 1u ? pr : 0.f;
+      if (masked && !((keep >> (e + u)) & 1u)) pr = pg[e + u] = 0.f;
 #endif
       pv[u] = pr;
-      pg[e + u] = pr * g;
     }
     pp[e / 2] = fa_pack2<DT>(pv[0], pv[1]);
   }

@@ -1195,6 +1195,65 @@ def _int_range(e: Expr, memo: Dict[int, Optional[Tuple[int, int]]]) -> Optional[
     return r
 
 
+def _float_range(e: Expr, memo: Dict[int, Optional[Tuple[float, float]]], ints: Dict[int, Optional[Tuple[int, int]]]) -> Optional[Tuple[float, float]]:
+    """Conservative value range of an fp32 expression that is neither infinite nor NaN at any position (indices below
+    ``_IDX_BOUND``), or None when that is not known.  A range in ``memo`` for the score leaf counts for it."""
+    got = memo.get(id(e), 0)
+    if got != 0:
+        return got
+    r = None
+    if e.op == "const":
+        r = (float(e.value), float(e.value))
+    elif e.op == "cast_f32":
+        a = e.args[0]
+        r = (0.0, 1.0) if a.dtype == B1 else (_int_range(a, ints) or (-2.0 ** 31, 2.0 ** 31)) if a.dtype == I32 else None
+    elif e.op == "select":
+        a, b = (_float_range(x, memo, ints) for x in e.args[1:])
+        if a and b:
+            r = (min(a[0], b[0]), max(a[1], b[1]))
+    elif e.op in ("add", "sub", "mul", "div", "min", "max", "neg", "abs", "exp", "exp2", "tanh", "sigmoid", "sin", "cos"):
+        x = [_float_range(a, memo, ints) if a.dtype == F32 else None for a in e.args]
+        if all(x):
+            (lo, hi), (lo2, hi2) = x[0], x[-1]
+            if e.op == "add":
+                r = (lo + lo2, hi + hi2)
+            elif e.op == "sub":
+                r = (lo - hi2, hi - lo2)
+            elif e.op == "mul":
+                p = (lo * lo2, lo * hi2, hi * lo2, hi * hi2)
+                r = (min(p), max(p))
+            elif e.op == "div":
+                if lo2 > 1e-30 or hi2 < -1e-30:
+                    p = (lo / lo2, lo / hi2, hi / lo2, hi / hi2)
+                    r = (min(p), max(p))
+            elif e.op in ("min", "max"):
+                f = min if e.op == "min" else max
+                r = (f(lo, lo2), f(hi, hi2))
+            elif e.op == "neg":
+                r = (-hi, -lo)
+            elif e.op == "abs":
+                r = (0.0, max(abs(lo), abs(hi)))
+            elif e.op in ("exp", "exp2"):
+                r = (0.0, 2.0 ** (1.5 * max(hi, 0.0))) if hi < 60 else None
+            elif e.op == "sigmoid":
+                r = (0.0, 1.0) if lo > -80 else None
+            else:
+                r = (-1.0, 1.0)
+    if r is not None and not max(abs(r[0]), abs(r[1])) <= 1e30:
+        r = None
+    memo[id(e)] = r
+    return r
+
+
+def always_finite(roots, score_is_zero: bool) -> bool:
+    """Whether the fp32 expressions are finite at every position: for any score, or for a score of zero."""
+    for root in roots:
+        memo = {id(x): (0.0, 0.0) for x in _topo(root) if x.op == "score"} if score_is_zero else {}
+        if _float_range(root, memo, {}) is None:
+            return False
+    return True
+
+
 _CTYPE = {I32: "int", F32: "float", B1: "bool"}
 
 
@@ -1590,6 +1649,8 @@ class ModSet:
             parts.append(to_cuda(self.score, "fa_score_mod"))
             parts.append(to_cuda(self.grad, "fa_score_mod_grad"))
             self.affine = affine_parts(self.score)
+            if always_finite([self.affine[0].root if self.affine is not None else self.grad.root], False):
+                parts.append("#define FA_SCORE_GRAD_FINITE 1\n")  # (0 times it is 0)
             if self.affine is not None:
                 # score_mod(s) == fa_score_mul(...) * s + fa_score_add(...); both ignore `score`
                 parts.append("#define FA_SCORE_AFFINE 1\n")
