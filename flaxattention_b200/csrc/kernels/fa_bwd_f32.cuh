@@ -434,6 +434,9 @@ extern "C" __global__ void __launch_bounds__(fa_bf32::NT, 1) fa_bwd_f32_kernel(c
           }
         }
 #endif
+        // (a score_mod may not be finite beyond Sq, and there the zero rows of Q and dO do not help)
+        const int left = p.Sq - q0;
+        if (left < CW) keep &= left <= 0 ? 0u : (1u << left) - 1u;
         ok = fa_mbar_wait_warp(bar_addr(sb, BAR_SFULL), (fa_u32)(gn & 1), abort_flag);
         if (ok) ok = fa_mbar_wait_warp(bar_addr(sb, BAR_FULL + s), (fa_u32)(((2 * gn + 1) / 3) & 1), abort_flag);  // (the row scalars)
         if (!ok) break;

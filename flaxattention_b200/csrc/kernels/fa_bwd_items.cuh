@@ -160,6 +160,21 @@ __device__ __forceinline__ void keep_bits(fa_u32 (&keep)[2], const unsigned* bit
   }
 #endif
 }
+// Query columns beyond Sq have zero rows of Q and dO and a row scalar of -infinity, and a probability of zero with that, unless a
+// score_mod is not finite there (score / (Sq - q)): then their keep bits have to go, on tiles of every kind.
+#if FA_HAS_SCORE_MOD && !defined(FA_SCORE_FINITE_AT_0)
+#define FA_BWD_CLEAR_BEYOND 1
+#else
+#define FA_BWD_CLEAR_BEYOND 0
+#endif
+// clears the bits of columns from `left` on (the number of columns below Sq); false: there are none
+__device__ __forceinline__ bool clear_beyond(fa_u32 (&keep)[2], int left) {
+  if (!FA_BWD_CLEAR_BEYOND || left >= 64) return false;
+  const unsigned long long in = left <= 0 ? 0ull : (1ull << left) - 1ull;
+  keep[0] &= (fa_u32)in;
+  keep[1] &= (fa_u32)(in >> 32);
+  return true;
+}
 // The low 16 keep bits of `w` as masks over pairs of 16-bit values, for P^T and dS^T after packing (head dim 64): two ANDs per pair in
 // a block that only masked tiles enter, so that the code of all others stays what it is without a mask.  (What the
 // exponential gave for a masked position, infinity too, goes with it.  A select per element made the kernel 15-20 % slower under a

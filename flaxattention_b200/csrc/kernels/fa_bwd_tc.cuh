@@ -566,10 +566,11 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
         const int s = gn % NSTAGE;
         const int pr = pl[n];
         const int m0 = (pr & 0xffff) * BQ, h = hk * G + (pr >> 20), gh = h + p.h_off;
-        const bool masked = FA_HAS_MASK_MOD && ((pr >> 16) & 0xf) == 1;
+        bool masked = FA_HAS_MASK_MOD && ((pr >> 16) & 0xf) == 1;
         // the mask of this thread's 64 columns, read (where it was evaluated beforehand: while S^T is waited for) or evaluated
         fa_u32 keep[2] = {0xffffffffu, 0xffffffffu};
         if (masked && row_ok) keep_bits(keep, bits, p, b, h, gb, gh, m0 + half * CW, kv);
+        masked |= clear_beyond(keep, p.Sq - (m0 + half * CW));
         ok = fa_mbar_wait_warp(bar_addr(sb, BAR_SFULL), (fa_u32)(gn & 1), abort_flag);
         if (ok) ok = fa_mbar_wait_warp(bar_addr(sb, BAR_QFULL + s), (fa_u32)((gn / NSTAGE) & 1), abort_flag);
         if (!ok) break;

@@ -118,7 +118,7 @@ __device__ __forceinline__ void p_chunk(const float (&s)[16], const float* nlse2
     float x0, x1;
     fa_f2_unpack(x2, x0, x1);
     float p0 = fa_ex2(x0), p1 = fa_ex2(x1);
-#if FA_HAS_MASK_MOD
+#if FA_HAS_MASK_MOD || FA_BWD_CLEAR_BEYOND
     if (masked) {
       p0 = (keep >> e) & 1u ? p0 : 0.f;
       p1 = (keep >> (e + 1)) & 1u ? p1 : 0.f;
@@ -127,7 +127,7 @@ __device__ __forceinline__ void p_chunk(const float (&s)[16], const float* nlse2
     pp[e / 2] = fa_pack2<DT>(p0, p1);
 #if FA_HAS_SCORE_MOD
     fa_f2_unpack(fa_mul2(fa_f2(p0, p1), g2), pg[e], pg[e + 1]);
-#if FA_HAS_MASK_MOD && !defined(FA_SCORE_GRAD_FINITE)
+#if (FA_HAS_MASK_MOD || FA_BWD_CLEAR_BEYOND) && !defined(FA_SCORE_GRAD_FINITE)
     if (masked) {
       pg[e] = (keep >> e) & 1u ? pg[e] : 0.f;
       pg[e + 1] = (keep >> (e + 1)) & 1u ? pg[e + 1] : 0.f;
@@ -157,7 +157,7 @@ __device__ __forceinline__ void p_chunk(const float (&s)[16], const float* nlse2
       x = fa_score_mod(x * scale, gb, gh, q0 | (e + u), kv) * FA_LOG2E + nlu;
       float pr = fa_ex2(x);
       pg[e + u] = pr * g;
-#if FA_HAS_MASK_MOD
+#if FA_HAS_MASK_MOD || FA_BWD_CLEAR_BEYOND
       if (masked && !((keep >> (e + u)) & 1u)) pr = pg[e + u] = 0.f;
 #endif
       pv[u] = pr;
@@ -447,10 +447,11 @@ extern "C" __global__ void __launch_bounds__(fa_b128::NT, 1) fa_bwd_tc_kernel(co
         const int s = gn % NQS;
         const int pr = pl[n];
         const int m0 = (pr & 0xffff) * BQ, h = hk * G + (pr >> 20), gh = h + p.h_off;
-        const bool masked = FA_HAS_MASK_MOD && ((pr >> 16) & 0xf) == 1;
+        bool masked = FA_HAS_MASK_MOD && ((pr >> 16) & 0xf) == 1;
         // the mask of this thread's 64 columns, read (where it was evaluated beforehand: while S^T is waited for) or evaluated
         fa_u32 keep[2] = {0xffffffffu, 0xffffffffu};
         if (masked && row_ok) keep_bits(keep, bits, p, b, h, gb, gh, m0 + c0, kv);
+        masked |= clear_beyond(keep, p.Sq - (m0 + c0));
         const float* rowp = (const float*)(sm + OFF_ROW + s * 2 * BQ * 4) + c0;
         ok = fa_mbar_wait_warp(bar_addr(sb, BAR_QFULL + s), (fa_u32)((gn / NQS) & 1), abort_flag);
         if (ok) ok = fa_mbar_wait_warp(bar_addr(sb, BAR_SFULL), (fa_u32)(gn & 1), abort_flag);

@@ -1651,6 +1651,9 @@ class ModSet:
             self.affine = affine_parts(self.score)
             if always_finite([self.affine[0].root if self.affine is not None else self.grad.root], False):
                 parts.append("#define FA_SCORE_GRAD_FINITE 1\n")  # (0 times it is 0)
+            whole = [t.root for t in self.affine] if self.affine is not None else [self.score.root, self.grad.root]
+            if always_finite(whole, True):
+                parts.append("#define FA_SCORE_FINITE_AT_0 1\n")  # value and derivative, at a score of 0
             if self.affine is not None:
                 # score_mod(s) == fa_score_mul(...) * s + fa_score_add(...); both ignore `score`
                 parts.append("#define FA_SCORE_AFFINE 1\n")

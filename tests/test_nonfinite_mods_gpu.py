@@ -1,5 +1,5 @@
-"""score_mods that are not finite, or whose derivative is not, at positions that do not count: masked ones.  Nothing of them may
-reach the gradients: 0 times infinity in a probability's product would be NaN for a whole row of dQ and dK.
+"""score_mods that are not finite, or whose derivative is not, at positions that do not count: masked ones, and the query
+rows beyond the last that fill up a tile.  Nothing of them may reach the gradients: 0 times infinity in a probability's product would be NaN for a whole row of dQ and dK.
 
 Tolerance: gradients <= 5e-2 relative to a reference in 64 bits of the same inputs for 16-bit types, the bar of the other
 backward tests, and 1e-4 for fp32."""
@@ -7,6 +7,8 @@ import pytest
 import torch
 
 from _util import DTYPES, rel_err
+from flaxattention_b200 import fnp
+from flaxattention_b200.masks import causal_mask
 
 pytestmark = pytest.mark.gpu
 
@@ -55,3 +57,21 @@ def test_masked_positions(name, Sq, Skv, D, dt):
     score, values = MASKED[name]
     x, got = _grads(score, _below, Sq, Skv, D, dt)
     _check(x, got, values, lambda i, j: i > j, dt)
+
+
+BEYOND = {  # not finite from q = Sq on
+    "inverse": lambda Sq: (lambda s, b, h, q, kv: s / (Sq - q), lambda s, i, j: s / (Sq - i)),
+    "root": lambda Sq: (lambda s, b, h, q, kv: s * fnp.sqrt((Sq - 1 - q) * 1.0), lambda s, i, j: s * (Sq - 1.0 - i).sqrt()),
+    "log": lambda Sq: (lambda s, b, h, q, kv: s + fnp.log((Sq - q) * 1.0), lambda s, i, j: s + (Sq - i).double().log()),
+    "square": lambda Sq: (lambda s, b, h, q, kv: s * s / (Sq - q), lambda s, i, j: s * s / (Sq - i)),
+}
+
+
+@pytest.mark.parametrize("D,dt", [(64, "bf16"), (64, "f32"), (128, "bf16"), (32, "f16")])
+@pytest.mark.parametrize("Sq", [129, 192, 255, 1000])
+@pytest.mark.parametrize("masked", [False, True])
+@pytest.mark.parametrize("name", list(BEYOND))
+def test_rows_beyond_the_last(name, masked, Sq, D, dt):
+    score, values = BEYOND[name](Sq)
+    x, got = _grads(score, causal_mask if masked else None, Sq, 200, D, dt)
+    _check(x, got, values, (lambda i, j: i >= j) if masked else None, dt)
