@@ -24,8 +24,9 @@
 #include "fa_common.cuh"
 
 // ---- thread-block clusters: barrier over all threads, reads of another CTA's shared memory ----
+// (not the .aligned forms: the loops in front of the barriers leave the threads of a warp one by one)
 __device__ __forceinline__ void fa_cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
 __device__ __forceinline__ fa_u32 fa_mapa(fa_u32 addr, int rank) {
   fa_u32 r;
