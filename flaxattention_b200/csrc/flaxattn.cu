@@ -1113,12 +1113,12 @@ int get_bwd_rerun_kernel(fa_module* m, int dtype, int D, int Dv, const BwdCfg& c
                                        {"FA_WARPS", c.warps}, {"FA_ROUND_SCORES", 0}, {"FA_RERUN", 1}}); },
                     "fa_bwd_rerun_kernel", std::max(c.smem_dq, c.smem_dkdv), k);
 }
-int get_decode_kernel(fa_module* m, int dtype, int D, int Dv, int flags, const DecCfg& c, bool pack, Kernel** k) {
+int get_decode_kernel(fa_module* m, int dtype, int D, int Dv, int flags, const DecCfg& c, bool pack, bool cluster, Kernel** k) {
   const int rnd = round_flag(dtype, flags);
-  return get_kernel(m, kernel_key(kIdDecode, {{dtype, 2}, {D, 9}, {Dv, 9}, {c.BM, 9}, {c.BN, 9}, {rnd, 1}, {pack ? 1 : 0, 1}}),
+  return get_kernel(m, kernel_key(kIdDecode, {{dtype, 2}, {D, 9}, {Dv, 9}, {c.BM, 9}, {c.BN, 9}, {rnd, 1}, {pack ? 1 : 0, 1}, {cluster ? 1 : 0, 1}}),
                     "fa_decode.cuh",
                     [&] { return defs({{"FA_DTYPE", dtype}, {"FA_D", D}, {"FA_DV", Dv}, {"FA_BM", c.BM}, {"FA_BN", c.BN},
-                                       {"FA_ROUND_SCORES", rnd}, {"FA_PACK_HEADS", pack ? 1 : 0}}); },
+                                       {"FA_ROUND_SCORES", rnd}, {"FA_PACK_HEADS", pack ? 1 : 0}, {"FA_CLUSTER", cluster ? 1 : 0}}); },
                     "fa_decode_kernel", c.smem, k);
 }
 // Grouped-query decode: the G query heads of a kv head share one CTA (their G * Sq rows form one
@@ -1555,7 +1555,9 @@ int fa_module_prepare(fa_module* m, int kind, int dtype, int D, int Dv, int Sq_h
       if (int rc = pick_decode(dtype, D, Dv, Sq_hint, nullptr, c)) return rc;
       if (dtype != FA_F32 && D == 64 && Dv == 64 && Sq_hint > 16)
         if (int rc = get_fwd_tc_kernel(m, dtype, D, 0, &k, true)) return rc;
-      return get_decode_kernel(m, dtype, D, Dv, 0, c, false, &k);
+      if (c.BM == 16)
+        if (int rc = get_decode_kernel(m, dtype, D, Dv, 0, c, false, true, &k)) return rc;
+      return get_decode_kernel(m, dtype, D, Dv, 0, c, false, false, &k);
     }
     case FA_KIND_BLOCKMASK:
       if (int rc = get_blockmask_kernel(m, false, &k)) return rc;
@@ -1804,7 +1806,9 @@ int fa_decode(fa_module* m, const fa_attn_params* p, int num_splits, void* works
   // results go through memory and the combine kernel.
   // (Clusters fill the SMs of a GPC in whole: at two CTAs per SM, 288 of 296 places in clusters of six take a second round, 54 -> 78 us.)
   const long long places = tc ? 0 : std::min<long long>(2, decode_ctas_per_sm(c)) * device_sm_count();
-  const bool cluster = !tc && num_splits > 1 && num_splits <= FA_DECODE_MAX_CLUSTER &&
+  // (More than 16 rows: the merge of that many rows costs more inside the cluster than the combine kernel does, B1 H32/8 Skv1024 D128
+  // 16 rows of each head 31.2 -> 32.9, 64 rows 26.4 -> 28.9.)
+  const bool cluster = !tc && c.BM == 16 && num_splits > 1 && num_splits <= FA_DECODE_MAX_CLUSTER &&
                        (long long)p->B * (pack ? p->Hkv : p->Hq) * num_splits <= (decode_ctas_per_sm(c) > 2 ? places : places * 87 / 100);
   if (need && !cluster) {
     const size_t rows = (size_t)p->B * p->Hq * num_splits * p->Sq;
@@ -1816,7 +1820,7 @@ int fa_decode(fa_module* m, const fa_attn_params* p, int num_splits, void* works
     if (int rc = launch_decode_tc(m, p, kp, num_splits, stream)) return rc;
   } else {
     Kernel* k = nullptr;
-    if (int rc = get_decode_kernel(m, p->dtype, p->D, p->Dv, p->flags, c, pack, &k)) return rc;
+    if (int rc = get_decode_kernel(m, p->dtype, p->D, p->Dv, p->flags, c, pack, cluster, &k)) return rc;
     if (int rc = launch(k, dim3(num_splits, pack ? p->Hkv : p->Hq, p->B), dim3(128), &kp, stream, cluster ? num_splits : 1)) return rc;
   }
   if (num_splits > 1 && !cluster) {

@@ -47,6 +47,9 @@ __device__ __forceinline__ float4 fa_ld_cluster_f4(fa_u32 addr) {
 #ifndef FA_PACK_HEADS
 #define FA_PACK_HEADS 0
 #endif
+#ifndef FA_CLUSTER
+#define FA_CLUSTER 0  // the splits of a tile of rows are launched as a cluster (a variant of its own: with the merge in the kernel of
+#endif                // all calls those without it took up to 7 % more, B16 H16 Skv1024 D64 16 rows 17.4 -> 18.6 us)
 
 namespace fa_dec {
 
@@ -326,7 +329,7 @@ extern "C" __global__ void __launch_bounds__(fa_dec::NT) fa_decode_kernel(const 
   const int rows = min(R, BM);
   // Splits in one cluster: the CTA's merged rows stay in shared memory, O over the first column group's and the
   // maximum and sum over the query tile, and the CTAs of the cluster read each other's.
-  const bool in_cluster = p.num_splits > 1 && p.part_o == nullptr;
+  constexpr bool in_cluster = FA_CLUSTER != 0;
   float2* ml = (float2*)smem;  // [BM]
   for (int i = tid; i < rows * DV; i += NT) {
     const int r = i / DV, c = i - r * DV;
@@ -370,7 +373,7 @@ extern "C" __global__ void __launch_bounds__(fa_dec::NT) fa_decode_kernel(const 
         p.lse[bh * p.Sq + qr] = lstar > 0.f ? (mstar + log2f(lstar)) * FA_LN2 : FA_NEG_INF;
     }
   }
-  if (!in_cluster) return;
+#if FA_CLUSTER
   // ---- merge the splits: four columns of a row per thread, the rows spread over the CTAs -----------
   fa_cluster_sync();
   const int ns = p.num_splits;
@@ -402,4 +405,5 @@ extern "C" __global__ void __launch_bounds__(fa_dec::NT) fa_decode_kernel(const 
       p.lse[((long long)b * p.Hq + h) * p.Sq + qr] = lstar > 0.f ? (mstar + log2f(lstar)) * FA_LN2 : FA_NEG_INF;
   }
   fa_cluster_sync();  // nobody leaves while its rows are being read
+#endif
 }
