@@ -171,7 +171,7 @@ class _Call:
             t.q_block_size, t.kv_block_size = bm.BLOCK_SIZE
             mb = bm.mask_bits if bm.bits_hold() and (not bm._bits_sources or stream is not None) else None
             if mb is not None and self.mask_mod is bm.mask_mod and mb.device == q.device and mb.shape[2] >= self.Sq \
-                    and mb.shape[3] * 32 >= self.Skv and mb.shape[0] in (1, self.B) and mb.shape[1] in (1, self.Hq):
+                    and mb.shape[3] * 32 >= self.Skv and bm.bits_cover(self.B, self.Hq, self.b_offset, self.h_offset):
                 if mb.dtype != torch.int32 or not mb.is_contiguous():
                     raise ValueError("BlockMask.mask_bits must be a contiguous int32 tensor")
                 t.mask_bits, t.mask_bits_stride, t.mask_bits_rows = mb.data_ptr(), mb.shape[3], mb.shape[2]

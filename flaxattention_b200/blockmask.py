@@ -119,7 +119,7 @@ class BlockMask:
 
     def __init__(self, kv_num_blocks, kv_indices, full_kv_num_blocks, full_kv_indices, q_num_blocks, q_indices,
                  full_q_num_blocks, full_q_indices, BLOCK_SIZE, mask_mod, mask_bits=None, mask_bits_t=None,
-                 _bits_sources=(), _bits_snapshot=None):
+                 _bits_sources=(), _bits_snapshot=None, _bits_at=(None, None)):
         if kv_indices.ndim < 2:
             raise RuntimeError("BlockMask must have at least 2 dimensions")
         assert kv_num_blocks is not None, "kv_num_blocks must be provided"
@@ -151,11 +151,19 @@ class BlockMask:
         self._bits_mod = mask_mod
         self._bits_sources = _bits_sources
         self._bits_snapshot = _bits_snapshot
+        # For batch and heads: the index the first entry of the matrices was made for, None where mask_mod does not
+        # read it.  A call with other entries (a broadcast mask over several heads, another offset) evaluates mask_mod.
+        self._bits_at = _bits_at
 
     def bits_hold(self) -> bool:
         """Whether ``mask_bits`` is still what ``mask_mod`` gives, as far as the host can see."""
         return (self.mask_bits is not None and self.mask_mod is self._bits_mod
                 and all(t is None or t._version == v for t, v in self._bits_sources))
+
+    def bits_cover(self, B: int, H: int, b_offset: int, h_offset: int) -> bool:
+        """Whether the entries of ``mask_bits`` are those of a call over these batch entries and heads."""
+        return all(n in (1, size) if at is None else (n == size and at == offset)
+                   for n, size, offset, at in zip(self.mask_bits.shape[:2], (B, H), (b_offset, h_offset), self._bits_at))
 
     def launch_check(self, buffers, stream) -> torch.Tensor:
         """Queues the comparison of the captured tensors (``buffers``, on the device) with the copy taken when
@@ -238,13 +246,13 @@ class BlockMask:
                          *self._moved_bits(mv))
 
     def _moved_bits(self, fn):
-        """(mask_bits, mask_bits_t, sources, snapshot) of a copy whose tensors went through ``fn``."""
+        """(mask_bits, mask_bits_t, sources, snapshot, first entries) of a copy whose tensors went through ``fn``."""
         if not self.bits_hold():
-            return None, None, (), None
+            return None, None, (), None, (None, None)
         bits, snapshot = fn(self.mask_bits), self._bits_snapshot
         if snapshot is not None and snapshot.device != bits.device:
             snapshot = snapshot.to(bits.device)
-        return bits, fn(self.mask_bits_t), self._bits_sources, snapshot
+        return bits, fn(self.mask_bits_t), self._bits_sources, snapshot, self._bits_at
 
     def shard(self, b_slice: slice, h_slice: slice) -> "BlockMask":
         """Tables of one batch x heads shard (broadcast axes are kept whole)."""
@@ -254,10 +262,14 @@ class BlockMask:
             bs = b_slice if t.shape[0] != 1 else slice(None)
             hs = h_slice if t.shape[1] != 1 else slice(None)
             return t[bs, hs].contiguous()
-        return BlockMask(cut(self.kv_num_blocks), cut(self.kv_indices), cut(self.full_kv_num_blocks),
+        part = BlockMask(cut(self.kv_num_blocks), cut(self.kv_indices), cut(self.full_kv_num_blocks),
                          cut(self.full_kv_indices), cut(self.q_num_blocks), cut(self.q_indices),
                          cut(self.full_q_num_blocks), cut(self.full_q_indices), self.BLOCK_SIZE, self.mask_mod,
                          *self._moved_bits(cut))
+        if part.mask_bits is not None:
+            part._bits_at = tuple(at if at is None or n == 1 else at + range(n)[sl].start
+                                  for at, n, sl in zip(self._bits_at, self.mask_bits.shape[:2], (b_slice, h_slice)))
+        return part
 
     def __repr__(self):
         def shape_or_none(x):
@@ -466,16 +478,17 @@ def create_block_mask(
     host = _cabi.host()
     module = module_for(None, mask)
     ms = lower_mods(None, mask)
+    b0, h0 = (int(b_offset) if ms.mask_reads_b else 0), (int(h_offset) if ms.mask_reads_h else 0)
+    bits_at = (b0 if ms.mask_reads_b else None, h0 if ms.mask_reads_h else None)
     cache_key = None
     if _compile and not ms.buffers:
         cache_key = (ms.key, B, H, Q_LEN, KV_LEN, Q_BLOCK_SIZE, KV_BLOCK_SIZE, int(b_offset), int(h_offset), str(dev))
         hit = _TABLE_CACHE.get(cache_key)
         if hit is not None:
             _TABLE_CACHE.move_to_end(cache_key)
-            return BlockMask(*hit[:8], (Q_BLOCK_SIZE, KV_BLOCK_SIZE), mask_mod, hit[8], hit[9])
+            return BlockMask(*hit[:8], (Q_BLOCK_SIZE, KV_BLOCK_SIZE), mask_mod, hit[8], hit[9], _bits_at=bits_at)
     # a mask that does not read the batch (head) index is evaluated once for all of them
     nb, nh = (B if ms.mask_reads_b else 1), (H if ms.mask_reads_h else 1)
-    b0, h0 = (int(b_offset) if ms.mask_reads_b else 0), (int(h_offset) if ms.mask_reads_h else 0)
     want_bits = _wants_bits(ms, dev, nb, nh, Q_LEN, KV_LEN, Q_BLOCK_SIZE, KV_BLOCK_SIZE, _mask_bits)
     buffers = device_buffers(ms, dev)
     sources = ()
@@ -488,4 +501,5 @@ def create_block_mask(
         _TABLE_CACHE[cache_key] = tables
         while len(_TABLE_CACHE) > _TABLE_CACHE_MAX:
             _TABLE_CACHE.popitem(last=False)
-    return BlockMask(*tables[:8], (Q_BLOCK_SIZE, KV_BLOCK_SIZE), mask_mod, tables[8], tables[9], sources, tables[10])
+    return BlockMask(*tables[:8], (Q_BLOCK_SIZE, KV_BLOCK_SIZE), mask_mod, tables[8], tables[9], sources, tables[10],
+                     bits_at)

@@ -68,7 +68,7 @@ PyObject *g_identity = nullptr, *g_noop = nullptr, *g_error = nullptr, *g_check_
 // lock, so that calls with other tensors on the same module from other threads do not come between.
 std::mutex g_buffers_mu;
 
-PyObject *s_mask_mod, *s_block_size, *s_mask_bits, *s_mask_bits_t, *s_bits_mod, *s_bits_sources, *s_bits_snapshot;
+PyObject *s_mask_mod, *s_block_size, *s_mask_bits, *s_mask_bits_t, *s_bits_mod, *s_bits_sources, *s_bits_snapshot, *s_bits_at;
 PyObject* s_tables[8];
 
 // A reference that is dropped at the end of its scope.
@@ -367,6 +367,16 @@ bool read_block_mask(PyObject* bm, PyObject* mask_mod, c10::Device dev, Call& c)
   if (mb.dim() != 4 || mb.size(2) < c.p.Sq || mb.size(3) * 32 < c.p.Skv || !(mb.size(0) == 1 || mb.size(0) == c.p.B) ||
       !(mb.size(1) == 1 || mb.size(1) == c.p.Hq))
     return true;
+  // (a mask that reads the batch or head index: entries of other indices than the call's are none, see BlockMask._bits_at)
+  Ref at(PyObject_GetAttr(bm, s_bits_at));
+  if (at.p == nullptr || !PyTuple_Check(at.p) || PyTuple_GET_SIZE(at.p) != 2) return false;
+  for (int i = 0; i < 2; ++i) {
+    PyObject* first = PyTuple_GET_ITEM(at.p, i);
+    if (first == Py_None) continue;
+    const long index = PyLong_AsLong(first);
+    if (index == -1 && PyErr_Occurred()) return false;
+    if (mb.size(i) != (i == 0 ? c.p.B : c.p.Hq) || index != (i == 0 ? c.p.b_offset : c.p.h_offset)) return true;
+  }
   t.mask_bits = (const uint32_t*)b;
   t.mask_bits_stride = mb.size(3);
   t.mask_bits_rows = (int32_t)mb.size(2);
@@ -659,5 +669,6 @@ PyMODINIT_FUNC PyInit__host(void) {
   s_bits_mod = PyUnicode_InternFromString("_bits_mod");
   s_bits_sources = PyUnicode_InternFromString("_bits_sources");
   s_bits_snapshot = PyUnicode_InternFromString("_bits_snapshot");
+  s_bits_at = PyUnicode_InternFromString("_bits_at");
   return PyModule_Create(&kModule);
 }
