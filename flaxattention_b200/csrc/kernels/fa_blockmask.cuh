@@ -9,13 +9,15 @@
 #pragma once
 #include "fa_params.h"
 
-// One CTA of four warps per block, in 128 x 128 sub-tiles: a warp takes 32 rows, a lane one of them, 32 keys at a time.  The
-// lane's own bits over the keys are a word of the row-major matrix (one predicated OR per position), what a mask reads per
-// query (a captured document id) is loaded once per lane and what it reads per key is a broadcast; five exchange steps
-// between the lanes turn the 32 words into those of the transposed matrix (some 25 instructions per 1024 positions).  Both matrices and
-// the block's count come out of one evaluation.  Where interval arithmetic over the mask's expression (fa_mask_range, from
-// the tracer) says that 32 x 32 positions are all kept or all not, none is evaluated.  Bound by instruction issue.  8192 x 8192 positions of an attention-sink mask:
-// 29 us; with lane = key, a ballot per row and a select for its word, 41.
+// One CTA of four warps per block, in 128 x 128 sub-tiles: a warp takes 32 rows, a lane one key out of each group of 32.  Lane = key
+// makes what a mask reads per key (a captured document id) a coalesced load outside the row loop and what it reads per query a broadcast
+// that serves four groups.  The lane's own bits over the rows are a word of the transposed matrix (one predicated OR per position),
+// and five exchange steps between the lanes turn the 32 words into those of the row-major one.  Both matrices and the block's
+// count come out of one evaluation.  Where interval arithmetic over the mask's expression (fa_mask_range, from
+// the tracer) says that 32 x 32 positions are all kept or all not, none is evaluated.
+// Bound by instruction issue.  8192 x 8192 positions of an attention-sink mask: 14.2 us for the call (a ballot per row and every
+// position evaluated: 45).  Lane = row instead took up to 1.6 times as long with masks that read by key (8192 x 8192, one id per key: 27.9 ->
+// 44.9 us, now 18.1) and with few rows (one row, 32768 keys: 10.7 -> 15.6, now 9.8).
 // Needs key blocks of whole 32-bit words and query blocks of whole words or a single one; other block sizes go to the
 // classify kernel below.
 constexpr int FA_SCAN_WARPS = 4;
@@ -34,7 +36,6 @@ extern "C" __global__ void __launch_bounds__(128) fa_mask_scan_kernel(const __gr
   FA_MOD_BUFS_INIT(p);
   fa_grid_wait();
   __shared__ __align__(16) unsigned t_words[128][FA_SCAN_WARPS];
-  __shared__ unsigned r_words[4][128];
   __shared__ int s_cnt[FA_SCAN_WARPS];
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -44,45 +45,84 @@ extern "C" __global__ void __launch_bounds__(128) fa_mask_scan_kernel(const __gr
   const int q0 = qb * p.QB, k0 = kvb * p.KVB;
   int cnt = 0;
   for (int r0 = 0; r0 < p.QB; r0 += 128) {
-    const int row = r0 + warp * 32 + lane, q = q0 + row;  // this lane's row inside the block, and its query
-    const bool row_in = row < p.QB;
+    const int row = r0 + warp * 32 + lane, q = q0 + row;  // the row of the block whose words this lane writes, and its query
+    const int qw = q - lane, nrows = min(32, p.QB - (row - lane));  // first query of the warp, and how many it has
     for (int c0 = 0; c0 < p.KVB; c0 += 128) {
-#pragma unroll 1
-      for (int c = 0; c < 4; ++c) {
-        const int kv = k0 + c0 + 32 * c, left = p.KVB - (c0 + 32 * c);
-        unsigned w = 0u;
-        if (left > 0) {  // (the same for all threads)
-          int known = 1;
+      const int k4 = k0 + c0;
+      unsigned colw[4] = {0u, 0u, 0u, 0u};  // bit r: query qw + r, key k4 + 32 c + lane
+      unsigned roww[4] = {0u, 0u, 0u, 0u};  // bit k: query q, key k4 + 32 c + k
+      if (nrows == 32) {
+        int open = c0 + 128 <= p.KVB ? 0xf : (1 << ((p.KVB - c0 + 31) / 32)) - 1;  // groups of 32 keys to evaluate (the same for the warp)
 #ifdef FA_HAS_MASK_RANGE
-          known = fa_mask_range(gb, gh, q - lane, q - lane + 31, kv, kv + 31);  // (the same for the warp)
-#endif
-          if (known == 1) {
 #pragma unroll
-            for (int e = 0; e < 32; ++e)
-              if (fa_mask_mod(gb, gh, q, kv + e)) w |= 1u << e;
-          } else {
-            w = known ? 0xffffffffu : 0u;
+        for (int c = 0; c < 4; ++c) {
+          const int known = (open >> c) & 1 ? fa_mask_range(gb, gh, qw, qw + 31, k4 + 32 * c, k4 + 32 * c + 31) : 1;
+          if (known != 1) {
+            open &= ~(1 << c);
+            colw[c] = known ? 0xffffffffu : 0u;
           }
-          if (left < 32) w &= (1u << left) - 1u;
-          if (!row_in) w = 0u;
         }
-        cnt += __popc(w);
-        r_words[c][threadIdx.x] = w;  // (read back by this thread)
-        if (p.bits_t != nullptr) t_words[32 * c + lane][warp] = fa_bit_transpose(w, lane);
+#endif
+        if (open == 0xf) {
+#pragma unroll 1
+          for (int r = 0; r < 32; r += 8) {
+            unsigned m[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+#pragma unroll
+              for (int c = 0; c < 4; ++c)
+                if (fa_mask_mod(gb, gh, qw + r + e, k4 + 32 * c + lane)) m[c] |= 1u << e;
+            }
+#pragma unroll
+            for (int c = 0; c < 4; ++c) colw[c] |= m[c] << r;
+          }
+        } else {
+#pragma unroll 1
+          for (; open != 0; open &= open - 1) {
+            const int c1 = __ffs(open) - 1;
+            unsigned w = 0u;
+#pragma unroll 1
+            for (int r = 0; r < 32; r += 8) {
+              unsigned m = 0u;
+#pragma unroll
+              for (int e = 0; e < 8; ++e)
+                if (fa_mask_mod(gb, gh, qw + r + e, k4 + 32 * c1 + lane)) m |= 1u << e;
+              w |= m << r;
+            }
+#pragma unroll
+            for (int c = 0; c < 4; ++c) colw[c] = c == c1 ? w : colw[c];
+          }
+        }
+      } else {  // few rows: a vote gives a row's word
+#pragma unroll 1
+        for (int r = 0; r < nrows; ++r) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            const bool keep = c0 + 32 * c + lane < p.KVB && fa_mask_mod(gb, gh, qw + r, k4 + 32 * c + lane);
+            const unsigned vote = __ballot_sync(0xffffffffu, keep);
+            if (keep) colw[c] |= 1u << r;
+            if (lane == r) roww[c] = vote;
+          }
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        if (c0 + 32 * c + lane >= p.KVB) colw[c] = 0u;
+        cnt += __popc(colw[c]);
+        if (p.bits_t != nullptr) t_words[32 * c + lane][warp] = colw[c];
       }
       if (p.bits != nullptr) {
         // the row's words of this sub-tile; keys beyond KV_LEN are 0, and the last block also writes the padding words
-        if (row_in && q < p.Q_LEN) {
-          unsigned* dst = p.bits + ((long long)bh * p.Q_LEN + q) * p.stride;
-          const int w0 = (k0 + c0) >> 5;
-          const int wend = (kvb == p.nKV - 1 && c0 + 128 >= p.KVB) ? (int)p.stride : min(w0 + 4, (k0 + p.KVB) >> 5);
-          unsigned roww[4];
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            const int left = p.KV_LEN - (k0 + c0 + 32 * c);
-            roww[c] = r_words[c][threadIdx.x];
-            if (left < 32) roww[c] &= left <= 0 ? 0u : (1u << left) - 1u;
-          }
+        for (int c = 0; c < 4; ++c) {
+          const int left = p.KV_LEN - (k4 + 32 * c);
+          if (nrows == 32) roww[c] = fa_bit_transpose(colw[c], lane);
+          if (left < 32) roww[c] &= left <= 0 ? 0u : (1u << left) - 1u;
+        }
+        if (row < p.QB && q < p.Q_LEN) {
+          unsigned* dst = p.bits + ((long long)bh * p.Q_LEN + q) * p.stride;
+          const int w0 = k4 >> 5;
+          const int wend = (kvb == p.nKV - 1 && c0 + 128 >= p.KVB) ? (int)p.stride : min(w0 + 4, (k0 + p.KVB) >> 5);
           if ((w0 & 3) == 0 && w0 + 4 <= wend) {
             *(uint4*)(dst + w0) = make_uint4(roww[0], roww[1], roww[2], roww[3]);
           } else {

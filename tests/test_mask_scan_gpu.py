@@ -90,3 +90,28 @@ def test_bits_asked_for_beside_blocks_of_part_words(Q, KV, block):
         dense = head_dependent(0, h, q, kv)
         assert np.array_equal(_unpack(bm.mask_bits, KV)[0, h][:Q], dense)
         assert np.array_equal(_unpack(bm.mask_bits_t, Q)[0, h][:KV], dense.T)
+
+
+@pytest.mark.parametrize("Q,KV,block", [(1, 300, 128), (31, 256, 128), (64, 160, (64, 32)), (128, 384, 128), (300, 500, 128), (256, 256, 256)])
+@pytest.mark.parametrize("name", ["key", "query", "in_part", "all_but_one"])
+def test_positions_decided_by_range_and_by_evaluation(name, Q, KV, block):
+    """Masks over captured ids: per key, per query, with groups of 32 keys that interval arithmetic decides between others that it
+    does not, and with one position that differs from all others."""
+    import flaxattention_b200 as fa
+
+    ids = torch.arange(1024, device="cuda", dtype=torch.int32) // 37
+    host = ids.cpu().numpy()
+    mod = {
+        "key": lambda b, h, q, kv: kv < ids[kv] * 40 + 5,
+        "query": lambda b, h, q, kv: kv < ids[q] * 40 + 5,
+        "in_part": lambda b, h, q, kv: (kv < 70) | ((ids[q] == ids[kv]) & (kv < 190)),
+        "all_but_one": lambda b, h, q, kv: (q != 30) | (kv != 100),
+    }[name]
+    q, kv = np.arange(Q)[:, None], np.arange(KV)[None, :]
+    dense = {"key": kv < host[kv] * 40 + 5, "query": kv < host[q] * 40 + 5,
+             "in_part": (kv < 70) | ((host[q] == host[kv]) & (kv < 190)), "all_but_one": (q != 30) | (kv != 100)}[name]
+    dense = np.broadcast_to(dense, (Q, KV))
+    bm = fa.create_block_mask(mod, None, None, Q, KV, BLOCK_SIZE=block)
+    torch.cuda.synchronize()
+    assert np.array_equal(_unpack(bm.mask_bits, KV)[0, 0][:Q], dense)
+    assert np.array_equal(_unpack(bm.mask_bits_t, Q)[0, 0][:KV], dense.T)
