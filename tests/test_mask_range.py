@@ -36,6 +36,19 @@ def _masks():
     }
 
 
+# of 300 rectangles, at least so many are told to be dropped and kept: about half of what the rules give, so that one that has stopped
+# to work is seen (remainders, quotients of negative numbers, minima, selects, shifts, one unknown operand of an or)
+TOLD = {"causal": (60, 60), "offset": (85, 40), "window": (95, 11), "sink": (100, 8), "document": (60, 0), "document_or": (0, 7), "dilated": (65, 1),
+        "tiles": (90, 18), "negative": (23, 105), "by_head": (50, 75), "absolute": (70, 35), "bounds": (85, 45), "where": (65, 55), "float": (0, 1),
+        "wrap": (0, 120), "shift": (2, 125), "all": (0, 300)}
+
+
+def test_values_that_may_wrap_are_not_told():
+    """Products that leave int32 for indices within the bound: no range, in a mask of them alone no function."""
+    assert modtrace.to_cuda_range(modtrace.lower_mods(None, lambda b, h, q, kv: q * 70000 >= kv * 70001).mask, "f") is None
+    assert modtrace.to_cuda_range(modtrace.lower_mods(None, lambda b, h, q, kv: (q + 1) * (kv + 1) > 9).mask, "f") is None
+
+
 def _range_function(mod, tmp_path):
     text = modtrace.to_cuda_range(mod, "fa_mask_range")
     if text is None:
@@ -54,11 +67,9 @@ def test_a_rectangle_that_is_known_is_right(name, tmp_path):
     ms = modtrace.lower_mods(None, _masks()[name])
     mod = ms.mask
     f = None if mod is None else _range_function(mod, tmp_path)
-    if f is None:
-        assert name == "all" or "float" in name
-        return
+    assert f is not None
     rng = np.random.RandomState(1)
-    told = 0
+    told = [0, 0]  # dropped, kept
     for _ in range(300):
         hq, hk = rng.choice([1, 7, 32, 128], 2)
         q0, k0 = (int(x) for x in rng.randint(0, 400, 2))
@@ -67,8 +78,7 @@ def test_a_rectangle_that_is_known_is_right(name, tmp_path):
         q, kv = np.arange(q0, q0 + hq, dtype=np.int32)[:, None], np.arange(k0, k0 + hk, dtype=np.int32)[None]
         want = np.broadcast_to(modtrace.evaluate(mod, None, np.int32(b), np.int32(h), q, kv), (hq, hk))
         if got != 1:
-            told += 1
+            told[got // 2] += 1
             assert want.all() if got == 2 else not want.any(), (name, got, b, h, q0, hq, k0, hk)
-    if name in ("causal", "offset", "window", "sink", "tiles", "absolute", "by_head"):
-        assert told >= 100
+    assert told[0] >= TOLD[name][0] and told[1] >= TOLD[name][1], told
     assert f(0, 0, 0, 1 << 21, 0, 31) == 1 and f(0, 0, -1, 30, 0, 31) == 1  # beyond the indices the bounds are for
