@@ -50,8 +50,7 @@ extern "C" __global__ void __launch_bounds__(128) fa_mask_scan_kernel(const __gr
     for (int c0 = 0; c0 < p.KVB; c0 += 128) {
       const int k4 = k0 + c0;
       unsigned colw[4] = {0u, 0u, 0u, 0u};  // bit r: query qw + r, key k4 + 32 c + lane
-      unsigned roww[4] = {0u, 0u, 0u, 0u};  // bit k: query q, key k4 + 32 c + k
-      if (nrows == 32) {
+      if (nrows >= 16) {  // (rows that the block does not have are evaluated with the others and dropped)
         int open = c0 + 128 <= p.KVB ? 0xf : (1 << ((p.KVB - c0 + 31) / 32)) - 1;  // groups of 32 keys to evaluate (the same for the warp)
 #ifdef FA_HAS_MASK_RANGE
 #pragma unroll
@@ -93,30 +92,28 @@ extern "C" __global__ void __launch_bounds__(128) fa_mask_scan_kernel(const __gr
             for (int c = 0; c < 4; ++c) colw[c] = c == c1 ? w : colw[c];
           }
         }
-      } else {  // few rows: a vote gives a row's word
+      } else {
 #pragma unroll 1
         for (int r = 0; r < nrows; ++r) {
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            const bool keep = c0 + 32 * c + lane < p.KVB && fa_mask_mod(gb, gh, qw + r, k4 + 32 * c + lane);
-            const unsigned vote = __ballot_sync(0xffffffffu, keep);
-            if (keep) colw[c] |= 1u << r;
-            if (lane == r) roww[c] = vote;
-          }
+          for (int c = 0; c < 4; ++c)
+            if (fa_mask_mod(gb, gh, qw + r, k4 + 32 * c + lane)) colw[c] |= 1u << r;
         }
       }
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         if (c0 + 32 * c + lane >= p.KVB) colw[c] = 0u;
+        if (nrows < 32) colw[c] &= (1u << max(nrows, 0)) - 1u;
         cnt += __popc(colw[c]);
         if (p.bits_t != nullptr) t_words[32 * c + lane][warp] = colw[c];
       }
       if (p.bits != nullptr) {
         // the row's words of this sub-tile; keys beyond KV_LEN are 0, and the last block also writes the padding words
+        unsigned roww[4];
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
           const int left = p.KV_LEN - (k4 + 32 * c);
-          if (nrows == 32) roww[c] = fa_bit_transpose(colw[c], lane);
+          roww[c] = fa_bit_transpose(colw[c], lane);
           if (left < 32) roww[c] &= left <= 0 ? 0u : (1u << left) - 1u;
         }
         if (row < p.QB && q < p.Q_LEN) {
