@@ -1486,14 +1486,12 @@ int get_bwd_tc_kernel(fa_module* m, int dtype, int D, int flags, bool kv2, Kerne
                     "fa_bwd_tc_kernel", smem, k);
 }
 
-// With a BlockMask the items are short or uneven and the variant with two K / V buffers wins or ties (us, against two
-// dS^T buffers): causal S512 35.8 / 35.8, S1024 64.5 / 66.6, S2048 150.5 / 154.6 (B8 H8), S4096 136 / 138, S6144 261 /
-// 261 (B2 H8); at 64 q tiles it loses, causal S8192 230 / 228 (B1 H8), attention sink S8192 247 / 239 (B2 H8).  Without
-// one every item has all the q tiles and two dS^T buffers win.
-bool bwd_tc_kv2(const fa_attn_params* p) {
-  if (p->D != 64 || !p->tables.kv_num_blocks) return false;
-  return (long long)((p->Sq + 127) / 128) * (p->Hq / p->Hkv) <= 64;
-}
+// With a BlockMask the items are short or uneven and the variant with two K / V buffers wins or ties.  Measured (us, one K / V buffer and
+// two dS^T buffers / two and one, a backward pass at head dim 64): causal B2 H8 S4096 129 / 126, B1 H8 S8192 225 / 221, B1 H2 S32768
+// 808 / 804, causal + checkerboard B2 H16/4 S3001 243 / 225, causal + ALiBi B8 H8 S2048 160 / 156, packed documents B4 H8 S4096 93.4 / 92.2,
+// attention sink B2 H8 S8192 173 / 172, B1 H4 S32768 563 / 565.  Without one every item has all the q tiles and two dS^T buffers
+// win (dense B8 H8 S2048, see fa_bwd_tc.cuh).
+bool bwd_tc_kv2(const fa_attn_params* p) { return p->D == 64 && p->tables.kv_num_blocks != nullptr; }
 
 // (batch, kv head) pairs whose items the backward works through together (item_of in fa_bwd_tc.cuh): as many as
 // keep their dQ accumulators, Q and dO in L2 (126 MB), if that leaves an item for every SM, or three where items

@@ -139,26 +139,56 @@ __device__ __forceinline__ const unsigned* bits_row(const FaParams& p, int kv) {
   const bool there = p.t.mask_bits_t != nullptr && (p.t.mask_hold == nullptr || *p.t.mask_hold != 0);
   return there ? p.t.mask_bits_t + (long long)kv * p.t.mask_t_stride : nullptr;
 }
-// mask_mod of kv row `kv` and q columns q0 .. q0+63 as bits: from that row, else from a rolled loop, which keeps the code
-// small (unrolled over a thread's columns it is 64 copies of the user's mask).
-__device__ __forceinline__ void keep_bits(fa_u32 (&keep)[2], const unsigned* bits, const FaParams& p, int b, int h, int gb, int gh, int q0, int kv) {
+// Its words of q columns q0 .. q0+63, of entry (b, h)
+__device__ __forceinline__ const unsigned* keep_words(const unsigned* bits, const FaParams& p, int b, int h, int q0) {
+  const unsigned entry = (p.t.mask_B == 1 ? 0 : b) * p.t.mask_H + (p.t.mask_H == 1 ? 0 : h);
+  return bits + (long long)entry * p.t.mask_t_rows * p.t.mask_t_stride + (q0 >> 5);
+}
+__device__ __forceinline__ void read_keep(fa_u32 (&keep)[2], const unsigned* bits, const FaParams& p, int b, int h, int q0) {
+  const uint2 w = *(const uint2*)keep_words(bits, p, b, h, q0);
+  keep[0] = w.x;
+  keep[1] = w.y;
+}
+// The same if `want`, all ones else, for a pair that comes later: as one predicated instruction it leaves no branch behind whose end
+// would wait for the load.
+__device__ __forceinline__ void ask_keep(fa_u32 (&keep)[2], const unsigned* bits, const FaParams& p, int b, int h, int q0, bool want) {
+  keep[0] = keep[1] = 0xffffffffu;
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %3, 0;\n\t@q ld.global.nc.v2.u32 {%0, %1}, [%2];\n\t}"
+               : "+r"(keep[0]), "+r"(keep[1]) : "l"(keep_words(bits, p, b, h, q0)), "r"((int)(want && bits != nullptr)));
+}
+// Without a matrix (attention sink B1 H4 S32768, head dims 64 and 128, us: 695 -> 565, 785 -> 684; evaluated in line, in the
+// first place: 659, 817): mask_mod of 32 columns at a time, from its range over them where that tells, else from a rolled loop over
+// both words, which keeps the code small (unrolled over a thread's columns it is 64 copies of the user's mask).
+__device__ __forceinline__ void eval_keep(fa_u32 (&keep)[2], int gb, int gh, int q0, int kv) {
 #if FA_HAS_MASK_MOD
-  if (bits != nullptr) {
-    const long long entry = (long long)(p.t.mask_B == 1 ? 0 : b) * p.t.mask_H + (p.t.mask_H == 1 ? 0 : h);
-    const uint2 w = *(const uint2*)(bits + entry * p.t.mask_t_rows * p.t.mask_t_stride + (q0 >> 5));
-    keep[0] = w.x;
-    keep[1] = w.y;
-  } else {
-    fa_u32 w0 = 0u, w1 = 0u;
+  int k0 = 1, k1 = 1;  // 0: none of the 32 columns, 2: all of them, 1: not known
+#ifdef FA_HAS_MASK_RANGE
+  k0 = fa_mask_range(gb, gh, q0, q0 + 31, kv, kv);
+  k1 = fa_mask_range(gb, gh, q0 + 32, q0 + 63, kv, kv);
+#endif
+  fa_u32 w0 = 0u, w1 = 0u;
+  if (k0 == 1 || k1 == 1) {
 #pragma unroll 2
     for (int e = 0; e < 32; ++e) {
       w0 |= (fa_mask_mod(gb, gh, q0 + e, kv) ? 1u : 0u) << e;
       w1 |= (fa_mask_mod(gb, gh, q0 + 32 + e, kv) ? 1u : 0u) << e;
     }
-    keep[0] = w0;
-    keep[1] = w1;
   }
+  keep[0] = k0 == 1 ? w0 : (k0 == 2 ? 0xffffffffu : 0u);
+  keep[1] = k1 == 1 ? w1 : (k1 == 2 ? 0xffffffffu : 0u);
 #endif
+}
+// Which of a thread's four steps of 16 columns have anything to compute: those in which a lane of its warp keeps a column (`masked`,
+// the same for the warp), and none for a row beyond Skv.  At head dim 128, where the compute warps set the pace of a masked tile, this
+// and asking for the words a pair ahead (ask_keep) took a pass over the long first items of an attention sink, B2 H16/4 S3001, from 345 to
+// 314 us (pairs of 64 query rows: 310).  At head dim 64 it costs more than it saves (B2 H8 S8192 185 -> 195 us).
+__device__ __forceinline__ fa_u32 live_steps(const fa_u32 (&keep)[2], bool masked, bool row_ok) {
+  fa_u32 live = row_ok ? 0xfu : 0u;
+  if (masked) {
+    const fa_u32 a = __reduce_or_sync(0xffffffffu, row_ok ? keep[0] : 0u), b = __reduce_or_sync(0xffffffffu, row_ok ? keep[1] : 0u);
+    live &= ((a & 0xffffu) ? 1u : 0u) | ((a >> 16) ? 2u : 0u) | ((b & 0xffffu) ? 4u : 0u) | ((b >> 16) ? 8u : 0u);
+  }
+  return live;
 }
 // Query columns beyond Sq have zero rows of Q and dO and a row scalar of -infinity, and a probability of zero with that, unless a
 // score_mod is not finite there (score / (Sq - q)): then their keep bits have to go, on tiles of every kind.
@@ -167,6 +197,7 @@ __device__ __forceinline__ void keep_bits(fa_u32 (&keep)[2], const unsigned* bit
 #else
 #define FA_BWD_CLEAR_BEYOND 0
 #endif
+#define FA_BWD_MASKS (FA_HAS_MASK_MOD || FA_BWD_CLEAR_BEYOND)  // some pairs are masked
 // clears the bits of columns from `left` on (the number of columns below Sq); false: there are none
 __device__ __forceinline__ bool clear_beyond(fa_u32 (&keep)[2], int left) {
   if (!FA_BWD_CLEAR_BEYOND || left >= 64) return false;
@@ -175,15 +206,23 @@ __device__ __forceinline__ bool clear_beyond(fa_u32 (&keep)[2], int left) {
   keep[1] &= (fa_u32)(in >> 32);
   return true;
 }
-// The low 16 keep bits of `w` as masks over pairs of 16-bit values, for P^T and dS^T after packing (head dim 64): two ANDs per pair in
-// a block that only masked tiles enter, so that the code of all others stays what it is without a mask.  (What the
+// Clears in 16 pairs of 16-bit values the columns whose bit of `w` is not set, for P^T and dS^T after packing (head dim 64): one AND
+// per pair in a block that only masked tiles enter, so that the code of all others stays what it is without a mask.  (What the
 // exponential gave for a masked position, infinity too, goes with it.  A select per element made the kernel 15-20 % slower under a
-// plain causal mask: B2 H8 S4096 126 -> 151 us.)
-__device__ __forceinline__ void keep_words(fa_u32 (&m)[8], fa_u32 w) {
+// plain causal mask: B2 H8 S4096 126 -> 151 us.)  prmt copies the sign bit of a byte over eight bits where a selector's fourth bit is
+// set: of w << s these are bits 7 - s, 15 - s, 23 - s and 31 - s, so that seven shifts and one prmt per pair make all masks of a word
+// (five instructions per pair before: attention sink B2 H8 S8192 186 -> 172 us a pass, packed documents B4 H8 S4096 99 -> 92).
+__device__ __forceinline__ void mask_pairs(fa_u32* pp, fa_u32* ds, fa_u32 w) {
+  fa_u32 a[8];
 #pragma unroll
-  for (int e = 0; e < 8; ++e) {
-    const fa_u32 lo = (fa_u32)((int)(w << (31 - 2 * e)) >> 31), hi = (fa_u32)((int)(w << (30 - 2 * e)) >> 31);
-    m[e] = __byte_perm(lo, hi, 0x5410);
+  for (int s = 0; s < 8; ++s) a[s] = w << s;
+#pragma unroll
+  for (int e = 0; e < 16; ++e) {
+    const int s = 7 - ((2 * e) & 7), k = (2 * e) >> 3;
+    fa_u32 m;
+    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(m) : "r"(a[s]), "r"(a[s - 1]), "r"(0xcc88 + 0x1111 * k));
+    pp[e] &= m;
+    ds[e] &= m;
   }
 }
 

@@ -17,9 +17,9 @@
 //   3. dV += P^T dO                      (A from TMEM)
 //   4. dK += dS^T Q                      (A = dS^T from smem, K-major)
 //   5. dQ = dS K                         (A = the same dS^T tile read MN-major, B = K; 128 q x 64 d)
-// The dQ tile of a pair leaves through a
-// staging buffer and two bulk reduce-adds into an fp32 accumulation buffer (summation order
-// over kv tiles is not fixed; a small kernel scales, un-permutes and converts it afterwards).
+// The dQ tile of a pair leaves warp by warp, 32 columns at a time, through 4 KB of staging and a bulk reduce-add each, into
+// an fp32 accumulation buffer (summation order over kv tiles is not fixed; a small kernel scales, un-permutes and
+// converts it afterwards).
 // dK and dV are written once per item.
 //
 // Warp roles (16 warps): 0-3 and 4-7 compute (first / second half of the q columns of the pair),
@@ -57,8 +57,7 @@ constexpr int DS_ATOMS = BQ / 64;                    // dS^T: [128 kv][BQ q] as 
 // stages, backward alone, us: dense B8 H8 S2048 231 -> 225, B4 H16/4 S2048 251 -> 239.
 // Shared memory holds, instead of the second dS^T buffer, a second K / V buffer (FA_BWD_KV2): K and V of
 // the next item are loaded while the current one is computed and nothing waits at the change of items, which pays
-// when items are short (causal B8 H8 S2048, 8.5 pairs per item on average: 150 against 155 us) and costs when they
-// are long.  The host picks.
+// when items are short or uneven.  The host picks (bwd_tc_kv2).
 #ifndef FA_BWD_KV2
 #define FA_BWD_KV2 0
 #endif
@@ -70,13 +69,11 @@ constexpr int MAXPL = 1024;              // (head, q tile) pairs of one item (tw
 constexpr int MAXC = 256;                // 128-row q tiles per head (Sq <= 32768)
 constexpr int NT = 512;
 constexpr int WARP_PRODUCER = 12, WARP_MMA = 13, WARP_MMA_B = 14, WARP_MMA_C = 15;
-// Register split (setmaxnreg): the kernel starts with 128 registers per thread (65536 / 512).  The
-// eight warps that are not compute warps give up 32 each and the eight compute warps take 32 each;
-// an increase that asked for more than the decrease releases would wait forever.  The compute warps
-// need no more than 160 (their 16-column steps keep few values live); with 200 / 56 the producer,
-// drain and issuing warps spilled, and the kernel was 4-5 % slower (dense backward 218 against 205 us,
-// attention sink 934 against 895; 192 / 64, 176 / 80, 168 / 88, 152 / 104 and 144 / 112 all lie within
-// 1 % of 160 / 96, 184 / 72 was as slow as 200 / 56).
+// Register split (setmaxnreg): the kernel starts with 128 registers per thread (65536 / 512).  The drain warps hold a row of dQ
+// (64 values, so that its TMEM columns are free after one round of loads) and give up 16 each, producer and issuers 32, and the eight
+// compute warps take 24 each; an increase that asked for more than the decrease releases would wait forever.  160 / 96 / 96 is as
+// fast (causal B2 H16/4 S3001 224.6 / 226.9 us, attention sink B2 H8 S8192 186 / 187); with 56 for all but the compute warps these
+// spilled, and the kernel was 4-5 % slower.  What is left of spills is 8 to 20 bytes of scalars, with either split.
 constexpr int REGS_COMPUTE = 152, REGS_DRAIN = 112, REGS_OTHER = 96;
 static_assert(2 * REGS_COMPUTE + REGS_DRAIN + REGS_OTHER <= 4 * 128, "setmaxnreg.inc would wait forever");
 
@@ -86,7 +83,7 @@ constexpr int OFF_V = OFF_K + KVBUF * KV_BYTES;
 constexpr int OFF_Q = OFF_V + KVBUF * KV_BYTES;             // NSTAGE tiles
 constexpr int OFF_DO = OFF_Q + NSTAGE * Q_BYTES;            // NSTAGE tiles
 constexpr int OFF_DS = OFF_DO + NSTAGE * Q_BYTES;           // dS^T
-constexpr int OFF_DQ = OFF_DS + NDS * DS_BYTES;      // fp32 staging 128 x 32 (half of the dQ tile at a time)
+constexpr int OFF_DQ = OFF_DS + NDS * DS_BYTES;      // fp32 staging 128 x 32, 4 KB of each drain warp
 constexpr int DQ_HALF_BYTES = 128 * 32 * 4;
 constexpr int OFF_ROW = OFF_DQ + DQ_HALF_BYTES;             // NSTAGE x (nlse2[BQ], ndelta[BQ]) floats
 constexpr int OFF_BAR = OFF_ROW + NSTAGE * 2 * BQ * 4;
@@ -567,9 +564,14 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
         const int pr = pl[n];
         const int m0 = (pr & 0xffff) * BQ, h = hk * G + (pr >> 20), gh = h + p.h_off;
         bool masked = FA_HAS_MASK_MOD && ((pr >> 16) & 0xf) == 1;
-        // the mask of this thread's 64 columns, read (where it was evaluated beforehand: while S^T is waited for) or evaluated
-        fa_u32 keep[2] = {0xffffffffu, 0xffffffffu};
-        if (masked && row_ok) keep_bits(keep, bits, p, b, h, gb, gh, m0 + half * CW, kv);
+        // the mask of this thread's 64 columns, read (where it was evaluated beforehand: while S^T is waited for) or evaluated.  (Asked
+        // for a pair ahead, as at head dim 128, the words cost more registers than they save: packed documents 97 -> 99 us.)
+        fa_u32 keep[2];
+        keep[0] = keep[1] = 0xffffffffu;
+        if (masked && row_ok) {
+          if (bits != nullptr) read_keep(keep, bits, p, b, h, m0 + half * CW);
+          else eval_keep(keep, gb, gh, m0 + half * CW, kv);
+        }
         masked |= clear_beyond(keep, p.Sq - (m0 + half * CW));
         ok = fa_mbar_wait_warp(bar_addr(sb, BAR_SFULL), (fa_u32)(gn & 1), abort_flag);
         if (ok) ok = fa_mbar_wait_warp(bar_addr(sb, BAR_QFULL + s), (fa_u32)((gn / NSTAGE) & 1), abort_flag);
@@ -619,16 +621,8 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
 #pragma unroll
         for (int e = 0; e < CW / 2; ++e) asm volatile("" : "+r"(pp[e]), "+r"(ds[e]));
         if (masked) {
-          fa_u32 m8[8];
-#pragma unroll
-          for (int c = 0; c < CW / 16; ++c) {
-            keep_words(m8, keep[c >> 1] >> ((c & 1) * 16));
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-              pp[8 * c + e] &= m8[e];
-              ds[8 * c + e] &= m8[e];
-            }
-          }
+          mask_pairs(pp, ds, keep[0]);
+          mask_pairs(pp + 16, ds + 16, keep[1]);
         }
         // product 3 of the previous pair must be done with P^T, and products 4-5 of the last pair that used this
         // dS^T buffer with that

@@ -443,15 +443,21 @@ extern "C" __global__ void __launch_bounds__(fa_b128::NT, 1) fa_bwd_tc_kernel(co
       const int kv = n0 + r;
       const bool row_ok = kv < p.Skv;
       const unsigned* bits = bits_row(p, kv);
+      fa_u32 keep[2];  // the mask of this thread's 64 columns, of the next pair from the moment on that this one's is applied
+      auto ask = [&](int n) {
+        const int pr = pl[n];  // (of pair np: a word behind the list's last, not looked at)
+        ask_keep(keep, bits, p, b, hk * G + (pr >> 20), (pr & 0xffff) * BQ + c0, n < np && row_ok && ((pr >> 16) & 0xf) == 1);
+      };
+      if (FA_HAS_MASK_MOD) ask(0);
       for (int n = 0; n < np && ok; ++n, ++gn) {
         const int s = gn % NQS;
         const int pr = pl[n];
-        const int m0 = (pr & 0xffff) * BQ, h = hk * G + (pr >> 20), gh = h + p.h_off;
+        const int m0 = (pr & 0xffff) * BQ, gh = hk * G + (pr >> 20) + p.h_off;
         bool masked = FA_HAS_MASK_MOD && ((pr >> 16) & 0xf) == 1;
-        // the mask of this thread's 64 columns, read (where it was evaluated beforehand: while S^T is waited for) or evaluated
-        fa_u32 keep[2] = {0xffffffffu, 0xffffffffu};
-        if (masked && row_ok) keep_bits(keep, bits, p, b, h, gb, gh, m0 + c0, kv);
+        if (!FA_HAS_MASK_MOD) keep[0] = keep[1] = 0xffffffffu;
+        if (masked && row_ok && bits == nullptr) eval_keep(keep, gb, gh, m0 + c0, kv);
         masked |= clear_beyond(keep, p.Sq - (m0 + c0));
+        const fa_u32 live = live_steps(keep, masked, row_ok);
         const float* rowp = (const float*)(sm + OFF_ROW + s * 2 * BQ * 4) + c0;
         ok = fa_mbar_wait_warp(bar_addr(sb, BAR_QFULL + s), (fa_u32)((gn / NQS) & 1), abort_flag);
         if (ok) ok = fa_mbar_wait_warp(bar_addr(sb, BAR_SFULL), (fa_u32)(gn & 1), abort_flag);
@@ -467,7 +473,7 @@ extern "C" __global__ void __launch_bounds__(fa_b128::NT, 1) fa_bwd_tc_kernel(co
           fa_tmem_wait_ld();
 #define FA_STEP(CUR, NEXT, C)                                                                                      \
   if ((C) + 16 < CW) fa_tmem_ld16(tS + (C) + 16, NEXT);                                                            \
-  if (row_ok) {                                                                                                    \
+  if (FA_BWD_MASKS ? (live >> ((C) / 16)) & 1u : row_ok) {                                                  \
     p_chunk(CUR, rowp + (C), p8, pg + (C), masked, keep[(C) >> 5] >> ((C) & 31), m0 + c0 + (C), kv, gb, gh, p.scale, sc2); \
   } else {                                                                                                         \
     _Pragma("unroll") for (int e = 0; e < 8; ++e) p8[e] = 0u;                                                      \
@@ -484,6 +490,7 @@ extern "C" __global__ void __launch_bounds__(fa_b128::NT, 1) fa_bwd_tc_kernel(co
         fa_tmem_wait_st();
         fa_tc_fence_before();
         fa_mbar_arrive(bar_addr(sb, BAR_PREADY));
+        if (FA_HAS_MASK_MOD) ask(n + 1);
         // dP^T is there: and dS^T of the pair before is not read any more (the order of issue)
         ok = fa_mbar_wait_warp(bar_addr(sb, BAR_DPFULL), (fa_u32)(gn & 1), abort_flag);
         if (!ok) break;
@@ -497,7 +504,7 @@ extern "C" __global__ void __launch_bounds__(fa_b128::NT, 1) fa_bwd_tc_kernel(co
           // position k ^ (r & 7) (the 128-byte swizzle of the operand layout)
 #define FA_STEP(CUR, NEXT, C)                                                                                      \
   if ((C) + 16 < CW) fa_tmem_ld16(tD + (C) + 16, NEXT);                                                            \
-  if (row_ok) {                                                                                                    \
+  if (FA_BWD_MASKS ? (live >> ((C) / 16)) & 1u : row_ok) {                                                  \
     ds_chunk(CUR, rowp + BQ + (C), pg + (C), d8);                                                                  \
   } else {                                                                                                         \
     _Pragma("unroll") for (int e = 0; e < 8; ++e) d8[e] = 0u;                                                      \

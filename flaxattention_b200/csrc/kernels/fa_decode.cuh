@@ -369,8 +369,9 @@ extern "C" __global__ void __launch_bounds__(fa_dec::NT) fa_decode_kernel(const 
         asm("cvt.rn.bf16.f32 %0, %1;" : "=h"(hv) : "f"(val));
         ((fa_u16*)og)[c] = hv;
       }
+      // (log2f, as in the merges, takes 1.5 us of 34 here: B16 H16 Skv1024 D64, 64 rows)
       if (c == 0 && p.lse != nullptr)
-        p.lse[bh * p.Sq + qr] = lstar > 0.f ? (mstar + log2f(lstar)) * FA_LN2 : FA_NEG_INF;
+        p.lse[bh * p.Sq + qr] = lstar > 0.f ? (mstar + fa_lg2(lstar)) * FA_LN2 : FA_NEG_INF;
     }
   }
 #if FA_CLUSTER
