@@ -34,6 +34,7 @@
 #ifndef FA_STATIC_SCRATCH_BYTES
 #define FA_STATIC_SCRATCH_BYTES (16u << 20)
 #endif
+constexpr size_t kStaticScratchBytes = (size_t)FA_STATIC_SCRATCH_BYTES;
 
 namespace {
 
@@ -1288,21 +1289,11 @@ int launch_fwd_f32_tc(fa_module* m, const fa_attn_params* p, FaParams kp, void* 
 
 // Shapes the split-KV variant of the tcgen05 kernel covers (`num_splits` CTAs per (batch, head), one
 // partial result per CTA and row); everything else runs on the general decode kernel.
-bool tc_decode_eligible(const fa_attn_params* p) {
+bool tc_decode_covers(const fa_attn_params* p) {
   if (p->flags & FA_FLAG_GENERAL_KERNELS) return false;
   if (p->dtype == FA_F32) return false;
   if (p->D != 64 || p->Dv != 64) return false;
-  // The kernel gives every query row two threads (64 kv columns of a tile each), whatever Sq is, and streams K / V through TMA
-  // and a five-stage ring; the general kernel's time grows with the row groups of 16, but two or three of its CTAs share an SM, and
-  // its splits are merged in a cluster.  Measured (us, this one / general, 8 heads unless said, L2 flushed):
-  //   rows      B1 Skv4096   B1 32768     B8 2048      B8 16384     B16 8192     B32 2048     B32 16384
-  //   2         17.4 / 13.3  29.7 / 29.7  21.5 / 16.8  74.8 / 65.6  83.0 / 65.6  52.4 / 37.8  196.6 / 185.3
-  //   16        19.5 / 14.6  31.7 / 31.7  21.5 / 18.5  74.8 / 69.6  83.0 / 68.6  54.3 / 40.9  199.6 / 192.6
-  //   32        19.5 / 17.4  31.7 / 35.8  21.5 / 20.5  76.8 / 73.7  89.1 / 71.9  58.4 / 42.0  205.8 / 233.5
-  //   64        19.5 / 21.5  31.7 / 46.1  23.6 / 27.5  80.8 / 107   99.3 / 107   68.6 / 61.4  220.2 / 374.8
-  // So: up to 16 rows the general kernel, up to 32 over at most 4096 keys, beyond that many heads over short caches.
-  if (p->Sq > 64 || p->Skv < 1024 || p->Skv > 32768) return false;
-  if (p->Sq <= 16 || (p->Sq <= 32 && p->Skv <= 4096) || (p->Skv <= 2048 && (long long)p->B * p->Hq >= 128)) return false;
+  if (p->Sq < 2 || p->Sq > 64 || p->Skv < 1024 || p->Skv > 32768) return false;
   if (!(p->scale > 0.f)) return false;
   const fa_block_tables& t = p->tables;
   if (t.kv_num_blocks) {
@@ -1310,6 +1301,22 @@ bool tc_decode_eligible(const fa_attn_params* p) {
     if (!(t.num_kv_blocks == 1 || t.kv_block_size % 128 == 0)) return false;
   }
   return true;
+}
+// And those it takes.  The kernel gives every query row two threads (64 kv columns of a tile each), whatever Sq is, and streams K / V
+// through TMA and a five-stage ring, one CTA to an SM and at least two splits; the general kernel's time grows with the row groups of 16,
+// but two or three of its CTAs share an SM, and up to 16 rows its splits are merged in a cluster.  So the tcgen05 kernel loses up to 16
+// rows, and above them where many heads over short caches make it several waves of short CTAs.  Measured (us, this one / general, D 64
+// fp16, inputs from memory), heads x keys:
+//   rows   64 x 1024    64 x 4096    128 x 2048   128 x 4096   256 x 1536   256 x 2048   256 x 4096   512 x 1024   512 x 1536   512 x 2048
+//   17     12.2 / 12.4  21.5 / 23.4  27.1 / 23.9  37.6 / 38.4  41.3 / 28.1  47.4 / 35.2  80.5 / 76.5  61.2 / 38.8  71.2 / 53.0  81.3 / 79.6
+//   32     12.3 / 13.8  21.5 / 25.4  27.6 / 25.9  38.1 / 40.9  44.1 / 29.9  50.3 / 37.1  85.1 / 87.5  66.1 / 42.3  76.2 / 56.7  86.6 / 92.7
+//   33     12.6 / 17.2  22.1 / 33.6  28.1 / 34.6  39.0 / 57.8  45.5 / 42.7  51.5 / 54.5  87.0 / 114   67.7 / 58.4  78.2 / 81.0  88.5 / 119
+//   64     13.3 / 19.5  22.9 / 36.4  31.8 / 38.7  42.7 / 62.2  51.1 / 46.5  57.6 / 58.3  97.6 / 135   79.8 / 65.5  90.4 / 88.7  101 / 144
+// (2 to 16 rows: 64 x 2048 20.6 / 18.6 with 8 rows, 256 x 8192 115 / 94 with 16, 64 x 8192 31.6 / 31.5.)
+bool tc_decode_eligible(const fa_attn_params* p) {
+  if (!tc_decode_covers(p) || p->Sq <= 16) return false;
+  const long long heads = (long long)p->B * p->Hq, keys = heads * p->Skv;
+  return p->Sq <= 32 ? heads < 128 || p->Skv > 2048 || keys > 768 << 10 : heads < 256 || p->Skv > 1536 || keys > 512 << 10;
 }
 int launch_decode_tc(fa_module* m, const fa_attn_params* p, const FaParams& kp, int num_splits, void* stream) {
   Kernel* k = nullptr;
@@ -1736,15 +1743,18 @@ static int general_decode_splits(long long bh, int tiles, int per_sm, int sm_cou
   if (row_groups > 1) return fill_waves(bh, cmax, per_sm * sm_count);
   const int c = (int)std::min<long long>(cmax, std::max<long long>(1, std::min(per_sm, 2) * sm_count / bh));
   if (c == 1) {
+    // (how full the waves of k splits are; 0 for less than one)
+    const auto fill = [&](int k) {
+      const double waves = (double)(bh * k) / (per_sm * sm_count);
+      return waves > 1.0 ? waves / (double)(long long)(waves + 0.999999) : 0.0;
+    };
     int best = 1;
-    double best_fill = 0.88;
-    for (int k = 2; k <= std::min(FA_DECODE_MAX_CLUSTER, tiles / 24); ++k) {
-      const double waves = (double)(bh * k) / (per_sm * sm_count), fill = waves / (double)(long long)(waves + 0.999999);
-      if (waves > 1.0 && fill > best_fill) {
+    double best_fill = std::max(0.88, fill(1));
+    for (int k = 2; k <= std::min(FA_DECODE_MAX_CLUSTER, tiles / 24); ++k)
+      if (fill(k) > best_fill) {
         best = k;
-        best_fill = fill;
+        best_fill = fill(k);
       }
-    }
     return best;
   }
   if (c <= FA_DECODE_MAX_CLUSTER) return c;
@@ -1759,20 +1769,25 @@ int fa_decode_num_splits(const fa_attn_params* p, int sm_count) {
   const bool pack = decode_packs_heads(p);
   const long long bh = (long long)p->B * (pack ? p->Hkv : p->Hq);
   const int tiles = (p->Skv + 127) / 128;
-  if (!pack && tc_decode_eligible(p)) {
-    // tcgen05 kernel: one CTA per SM and split, at least eight kv tiles per CTA; its partial results
-    // always go through the combine kernel, so there are at least two splits
-    const int cmax = tiles / 8 > 1 ? (tiles / 8 < 64 ? tiles / 8 : 64) : 1;
-    const int c = fill_waves(bh, cmax, sm_count);
-    return c < 2 ? 2 : c;
-  }
+  // tcgen05 kernel: one CTA per SM and split, at least eight kv tiles per CTA; its partial results
+  // always go through the combine kernel, so there are at least two splits
+  const auto tc_splits = [&] { return std::max(2, fill_waves(bh, std::min(std::max(tiles / 8, 1), 64), sm_count)); };
+  if (!pack && tc_decode_eligible(p)) return tc_splits();
   // general kernel: as many CTAs per SM as its shared memory allows (at most four by registers)
   int per_sm = 2;
   DecCfg c{16, 0, 0};
   if (pick_decode(p->dtype, p->D, p->Dv, pack ? p->Sq * (p->Hq / p->Hkv) : p->Sq, nullptr, c) == FA_OK) {
     per_sm = decode_ctas_per_sm(c);
   }
-  return general_decode_splits(bh, tiles, per_sm, sm_count, c.BM / 16);
+  const int n = general_decode_splits(bh, tiles, per_sm, sm_count, c.BM / 16);
+  // Callers of fa_decode_static have room for kStaticScratchBytes of partial results.  Where this count needs more, and the one
+  // that fills waves (of the tcgen05 kernel where it covers the call) does not, that one is taken: many rows over many heads,
+  // whose grids have CTAs enough with either.
+  if (n > 1 && fa_decode_workspace_bytes(p, n) > kStaticScratchBytes) {
+    const int waves = !pack && tc_decode_covers(p) ? tc_splits() : fill_waves(bh, std::min(std::max(tiles / 4, 1), 64), per_sm * sm_count);
+    if (fa_decode_workspace_bytes(p, waves) <= kStaticScratchBytes) return waves;
+  }
+  return n;
 }
 
 size_t fa_decode_workspace_bytes(const fa_attn_params* p, int num_splits) {
@@ -1955,7 +1970,6 @@ namespace {
 
 // Scratch for the split-KV partial results of fa_decode_static.  It is part of the loaded
 // library image: every GPU that loads the library holds these bytes until the process exits.
-constexpr size_t kStaticScratchBytes = (size_t)FA_STATIC_SCRATCH_BYTES;
 static __device__ __align__(256) unsigned char g_static_scratch[kStaticScratchBytes];
 
 std::mutex g_static_mu;

@@ -153,6 +153,19 @@ def test_decode_static_rejects_bad_arguments_first():
     assert L.fa_decode_static(m.handle, None, 4, None) == -1
 
 
+@pytest.mark.parametrize("B,Hq,Hkv,Sq,Skv,D", [
+    (8, 32, 32, 32, 4096, 64), (16, 32, 8, 32, 4096, 64), (8, 64, 64, 33, 2048, 64), (256, 16, 16, 4, 32768, 64), (256, 32, 8, 1, 32768, 64),
+    (32, 64, 64, 2, 32768, 128), (256, 64, 64, 1, 8191, 128), (128, 64, 8, 16, 131072, 128), (256, 32, 8, 1, 32768, 128),
+    (64, 32, 32, 4, 16384, 256), (256, 16, 16, 1, 131072, 256), (128, 16, 1, 9, 131072, 64),
+])
+def test_split_counts_stay_within_the_static_scratch(B, Hq, Hkv, Sq, Skv, D):
+    """Problems that the built-in scratch has room for when their splits fill waves: the library's own count has to fit as well."""
+    L = _cabi.lib()
+    p = _params(B=B, Hq=Hq, Hkv=Hkv, Sq=Sq, Skv=Skv, D=D, Dv=D)
+    n = L.fa_decode_num_splits(C.byref(p), 148)
+    assert 1 <= n <= 64 and L.fa_decode_workspace_bytes(C.byref(p), n) <= L.fa_decode_static_capacity()
+
+
 def test_status_word_raises_on_the_next_check():
     """A kernel that gave up on a barrier wait ORs a bit into the status word; the wrapper raises
     on the next call or on check_status() and clears the word."""

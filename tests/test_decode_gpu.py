@@ -84,14 +84,13 @@ def test_decode_benchmark_shape():
 
 
 @pytest.mark.parametrize("dt", ["f16", "bf16"])
-@pytest.mark.parametrize("Sq,splits", [(2, 4), (5, 0), (16, 8), (17, 4), (24, 0), (32, 8), (33, 4), (48, 8), (64, 12), (64, 3), (40, 0), (64, 24)])
+@pytest.mark.parametrize("Sq,splits", [(17, 4), (19, 12), (24, 0), (31, 5), (32, 8), (32, 0), (33, 4), (48, 8), (64, 12), (64, 3), (40, 0), (64, 24)])
 def test_tcgen05_decode_and_general_decode_agree_with_the_oracle(Sq, splits, dt):
-    """2..64 query rows with a split count that is a multiple of four run on the split-KV variant
-    of the tcgen05 kernel (four partial results per CTA: two warpgroups x two column halves), any
-    other count or the `general` option on the general decode kernel: both within tolerance of the
-    oracle and close to each other, and the status word of the tcgen05 kernel (bounded waits)
-    stays 0."""
+    """17..64 query rows over few heads run on the split-KV variant of the tcgen05 kernel with any split count from two on,
+    with the `general` option on the general decode kernel: each on its own kernel, both within tolerance of the
+    oracle and close to each other, and the status word of the tcgen05 kernel (bounded waits) stays 0."""
     import flaxattention_b200 as fa
+    from flaxattention_b200 import _cabi
 
     B, Hq, Hkv, Skv, D = 2, 4, 4, 3000, 64      # ragged last tile, 24 kv tiles
     s, m = _mods(Hq, Sq, Skv, "offset")
@@ -100,12 +99,17 @@ def test_tcgen05_decode_and_general_decode_agree_with_the_oracle(Sq, splits, dt)
     bm = fa.create_block_mask(m, B, Hq, Sq, Skv)
     status = torch.zeros(1, dtype=torch.int32, device="cuda")
     outs = []
-    for opts in ({"path": "decode", "status": status}, {"path": "decode", "kernels": "general"}):
+    for opts, kernel in (({"path": "decode", "status": status}, "fa_fwd_tc_kernel"), ({"path": "decode", "kernels": "general"}, "fa_decode_kernel")):
         if splits:
             opts["num_splits"] = splits
-        out, lse = fa.flax_attention(q.cuda(), k.cuda(), v.cuda(), score_mod=s, block_mask=bm, return_lse=True,
-                                     kernel_options=opts)
-        torch.cuda.synchronize()
+        _cabi.profile_enable(True)
+        try:
+            out, lse = fa.flax_attention(q.cuda(), k.cuda(), v.cuda(), score_mod=s, block_mask=bm, return_lse=True,
+                                         kernel_options=opts)
+            torch.cuda.synchronize()
+            assert kernel in [name for name, _ in _cabi.profile_read()]
+        finally:
+            _cabi.profile_enable(False)
         assert max_abs(out.cpu(), ref) <= 2e-2
         err, same = lse_err(lse.cpu(), ref_lse)
         assert same and err <= 2e-2 * max(1.0, ref_lse.abs().max().item())
