@@ -914,8 +914,10 @@ __global__ void fa_dq_convert_kernel(const float* __restrict__ acc, FaTensor dq,
 // Combines the per-split partial results of the decode kernels: one warp per output row.  Lane s takes the (max, sum)
 // pair of split s and its weight 2^(m_s - m*), 32 splits at a time; the weights then go round by shuffle.  A lane owns four
 // columns, and where the row has fewer than 128 the warp takes several splits at once; the reads of eight rounds
-// are under way together (one at a time, the latency of each was paid in turn: half a microsecond per split).
-template <int DT>
+// are under way together (one at a time, the latency of each was paid in turn: half a microsecond per split), of two where
+// that takes all splits: many rows of few splits are bound by instructions and by the warps that their registers let on an SM.
+// WIDE: more than 128 columns.
+template <int DT, int U, bool WIDE>
 __global__ void fa_decode_combine_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
                                          FaTensor o, float* __restrict__ lse, int Hq, int Sq, int Dv, int ns,
                                          long long n_rows) {
@@ -936,8 +938,7 @@ __global__ void fa_decode_combine_kernel(const float* __restrict__ part_o, const
   const int per = groups < 32 ? groups : 32;            // lanes of a split
   const int sub = 32 / per, mine = lane / per;          // splits at once; this lane's (beyond sub: idle)
   const int c0 = (lane - mine * per) * 4;               // first column; head dims above 128: and 128 columns on
-  const bool active = mine < sub, second = c0 + 128 < Dv;
-  constexpr int U = 8;
+  const bool active = mine < sub, second = WIDE && c0 + 128 < Dv;
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f), acc2 = acc;
   float lstar = 0.f;
   for (int s0 = 0; s0 < ns; s0 += 32) {
@@ -950,7 +951,7 @@ __global__ void fa_decode_combine_kernel(const float* __restrict__ part_o, const
     const int cnt = ns - s0 < 32 ? ns - s0 : 32;
     for (int t0 = 0; t0 < cnt; t0 += U * sub) {
       float wt[U];
-      float4 x[U], y[U];
+      float4 x[U], y[WIDE ? U : 1];
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         const int t = t0 + u * sub + mine;
@@ -958,12 +959,12 @@ __global__ void fa_decode_combine_kernel(const float* __restrict__ part_o, const
         if (!active || t >= cnt) wt[u] = 0.f;
         const float* src = part_o + prow(s0 + t) * Dv + c0;
         x[u] = wt[u] != 0.f ? *(const float4*)src : make_float4(0.f, 0.f, 0.f, 0.f);
-        y[u] = wt[u] != 0.f && second ? *(const float4*)(src + 128) : make_float4(0.f, 0.f, 0.f, 0.f);
+        if (WIDE) y[u] = wt[u] != 0.f && second ? *(const float4*)(src + 128) : make_float4(0.f, 0.f, 0.f, 0.f);
       }
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         acc.x += wt[u] * x[u].x; acc.y += wt[u] * x[u].y; acc.z += wt[u] * x[u].z; acc.w += wt[u] * x[u].w;
-        acc2.x += wt[u] * y[u].x; acc2.y += wt[u] * y[u].y; acc2.z += wt[u] * y[u].z; acc2.w += wt[u] * y[u].w;
+        if (WIDE) { acc2.x += wt[u] * y[u].x; acc2.y += wt[u] * y[u].y; acc2.z += wt[u] * y[u].z; acc2.w += wt[u] * y[u].w; }
       }
     }
   }
@@ -1839,8 +1840,14 @@ int fa_decode(fa_module* m, const fa_attn_params* p, int num_splits, void* works
   if (num_splits > 1 && !cluster) {
     const long long n_rows = (long long)p->B * p->Hq * p->Sq;
     const unsigned blocks = (unsigned)((n_rows + 3) / 4);
-    if (int rc = launch_here("fa_decode_combine_kernel", p->dtype == FA_F16 ? fa_decode_combine_kernel<FA_F16> : fa_decode_combine_kernel<FA_BF16>,
-                             dim3(blocks), dim3(128), stream, kp.part_o, kp.part_ml, kp.o, kp.lse, p->Hq, p->Sq, p->Dv, num_splits, n_rows))
+    const bool few = num_splits <= 2 * (32 / std::min(p->Dv / 4, 32)), wide = p->Dv > 128;
+    const auto pick = [&](auto dt) {
+      constexpr int DT = decltype(dt)::value;
+      return wide ? (few ? fa_decode_combine_kernel<DT, 2, true> : fa_decode_combine_kernel<DT, 8, true>)
+                  : (few ? fa_decode_combine_kernel<DT, 2, false> : fa_decode_combine_kernel<DT, 8, false>);
+    };
+    const auto combine = p->dtype == FA_F16 ? pick(std::integral_constant<int, FA_F16>{}) : pick(std::integral_constant<int, FA_BF16>{});
+    if (int rc = launch_here("fa_decode_combine_kernel", combine, dim3(blocks), dim3(128), stream, kp.part_o, kp.part_ml, kp.o, kp.lse, p->Hq, p->Sq, p->Dv, num_splits, n_rows))
       return rc;
   }
   return FA_OK;
