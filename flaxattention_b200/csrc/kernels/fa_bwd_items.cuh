@@ -65,17 +65,16 @@ __device__ __forceinline__ Item item_of(int idx, int Hkv, int B, int n_kvt, int 
 
 // The (query head, q tile) pairs of one item, written to `pl` by one warp: per head of the group,
 // the 128-row q tiles the BlockMask lists for the item's kv tile (class 1: apply mask_mod, 2: full)
-// in ascending order, each as 128 / BQ pairs.  Without tables every tile is listed.  Returns the
+// in ascending order, one pair each.  Without tables every tile is listed.  Returns the
 // number of pairs (the same in every lane).  `cl` is scratch: one bit per q tile and class.
-template <int BQ, int MAXPL, int MAXC>
+template <int MAXPL, int MAXC>
 __device__ __forceinline__ int build_pair_list(const FaParams& p, int hk, int b, int kt, int G, int n_ctiles,
                                                unsigned* cl, int* pl, int lane) {
-  constexpr int PPT = 128 / BQ;
   const bool tables = p.t.kv_num != nullptr && p.t.q_num != nullptr;
   int w = 0;
   for (int g = 0; g < G; ++g) {
     if (!tables) {
-      const int nq = (p.Sq + BQ - 1) / BQ;
+      const int nq = (p.Sq + 127) / 128;
       const int mode = FA_HAS_MASK_MOD ? 1 : 2;
       // the items of a head start at different q tiles, so that the CTAs on one head do not add to the same
       // dQ tile at the same time
@@ -116,18 +115,10 @@ __device__ __forceinline__ int build_pair_list(const FaParams& p, int hk, int b,
       const int t = t0 + lane;
       // (only tiles below n_ctiles have a bit; a tile in both lists counts as full)
       const int c = (cl[MAXC / 32 + (t0 >> 5)] >> lane) & 1u ? 2 : (int)((cl[t0 >> 5] >> lane) & 1u);
-      int n_t = 0;
-      if (c != 0)
-        for (int v = 0; v < PPT; ++v) n_t += (t * PPT + v) * BQ < p.Sq ? 1 : 0;
-      int inc = n_t;
-#pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        const int o = __shfl_up_sync(0xffffffffu, inc, d);
-        if (lane >= d) inc += o;
-      }
-      for (int v = 0; v < n_t; ++v)
-        if (w + inc - n_t + v < MAXPL) pl[w + inc - n_t + v] = (t * PPT + v) | (c << 16) | (g << 20);
-      w += __shfl_sync(0xffffffffu, inc, 31);
+      const unsigned listed = __ballot_sync(0xffffffffu, c != 0);
+      const int at = w + __popc(listed & ((1u << lane) - 1u));
+      if (c != 0 && at < MAXPL) pl[at] = t | (c << 16) | (g << 20);
+      w += __popc(listed);
     }
     __syncwarp();
   }

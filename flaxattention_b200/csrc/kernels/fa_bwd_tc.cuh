@@ -44,12 +44,7 @@ constexpr int D = 64;
 constexpr int BT = 128;                    // kv rows of a tile
 constexpr int BQ = 128;                    // q rows of a pair
 constexpr int CW = BQ / 2;                 // q columns of one compute thread
-constexpr int DATOMS = D / 64;             // 64-element (128-byte) column groups of a K / V / Q / dO row
-constexpr int ATOM_BYTES = 128 * 128;      // 128 rows x 128 bytes
-constexpr int KV_BYTES = DATOMS * ATOM_BYTES;        // one K or V tile
-constexpr int Q_ATOM_BYTES = BQ * 128;               // BQ rows x 128 bytes
-constexpr int Q_BYTES = DATOMS * Q_ATOM_BYTES;       // one Q or dO tile (16 KB in both configurations)
-constexpr int DS_ATOMS = BQ / 64;                    // dS^T: [128 kv][BQ q] as atoms of 64 q columns
+constexpr int TILE_BYTES = 128 * 128;      // a K, V, Q or dO tile: 128 rows x 128 bytes (64 values)
 // K / V and dS^T buffers.  The pace of a pair is set by the hand-over of P^T and dS^T: with one dS^T buffer the
 // compute warps may store pair n + 1 only when products 3-5 of pair n are complete.  With two they wait for
 // product 3 of pair n (issued first) and, by the order of issue, products 4-5 of pair n - 1, which is
@@ -64,7 +59,7 @@ constexpr int DS_ATOMS = BQ / 64;                    // dS^T: [128 kv][BQ q] as 
 constexpr int KVBUF = FA_BWD_KV2 ? 2 : 1;
 constexpr int NSTAGE = 3;
 constexpr int NDS = KVBUF == 1 ? 2 : 1;                // dS^T buffers
-constexpr int DS_BYTES = DS_ATOMS * ATOM_BYTES;
+constexpr int DS_BYTES = 2 * TILE_BYTES;               // dS^T: [128 kv][128 q] as two blocks of 64 q columns
 constexpr int MAXPL = 1024;              // (head, q tile) pairs of one item (two such lists fit in shared memory)
 constexpr int MAXC = 256;                // 128-row q tiles per head (Sq <= 32768)
 constexpr int NT = 512;
@@ -79,10 +74,10 @@ static_assert(2 * REGS_COMPUTE + REGS_DRAIN + REGS_OTHER <= 4 * 128, "setmaxnreg
 
 // shared memory map (from a 1024-byte aligned base)
 constexpr int OFF_K = 0;
-constexpr int OFF_V = OFF_K + KVBUF * KV_BYTES;
-constexpr int OFF_Q = OFF_V + KVBUF * KV_BYTES;             // NSTAGE tiles
-constexpr int OFF_DO = OFF_Q + NSTAGE * Q_BYTES;            // NSTAGE tiles
-constexpr int OFF_DS = OFF_DO + NSTAGE * Q_BYTES;           // dS^T
+constexpr int OFF_V = OFF_K + KVBUF * TILE_BYTES;
+constexpr int OFF_Q = OFF_V + KVBUF * TILE_BYTES;             // NSTAGE tiles
+constexpr int OFF_DO = OFF_Q + NSTAGE * TILE_BYTES;            // NSTAGE tiles
+constexpr int OFF_DS = OFF_DO + NSTAGE * TILE_BYTES;           // dS^T
 constexpr int OFF_DQ = OFF_DS + NDS * DS_BYTES;      // fp32 staging 128 x 32, 4 KB of each drain warp
 constexpr int DQ_HALF_BYTES = 128 * 32 * 4;
 constexpr int OFF_ROW = OFF_DQ + DQ_HALF_BYTES;             // NSTAGE x (nlse2[BQ], ndelta[BQ]) floats
@@ -325,7 +320,7 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
       const Item it = item_at(min(idx, n_items - 1), p.Hkv, p.B, n_kvt, P.chunk_heads);
       const int hk = it.hk, b = it.b, kt = it.kt;
       int np = -1;
-      if (idx < n_items) np = build_pair_list<BQ, MAXPL, MAXC>(p, hk, b, kt, G, n_ctiles, (unsigned*)(sm + OFF_CLS), pl, lane);
+      if (idx < n_items) np = build_pair_list<MAXPL, MAXC>(p, hk, b, kt, G, n_ctiles, (unsigned*)(sm + OFF_CLS), pl, lane);
       if (lane == 0) {
         item[4 * lb] = KVBUF == 2 ? idx : hk;
         item[4 * lb + 1] = b;
@@ -349,11 +344,9 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
             if (use > 0) ok = fa_mbar_wait(bar_addr(sb, (KVBUF == 2 ? BAR_KVFREE : BAR_FINAL) + kb), (fa_u32)((use - 1) & 1), abort_flag);
             if (!ok) break;
             const fa_u32 full = bar_addr(sb, BAR_KV + kb);
-            fa_mbar_expect_tx(full, 2 * KV_BYTES);
-            for (int a = 0; a < DATOMS; ++a) {
-              fa_tma_load_4d(sb + OFF_K + kb * KV_BYTES + a * ATOM_BYTES, &P.tk, full, a * 64, n0, hk, b);
-              fa_tma_load_4d(sb + OFF_V + kb * KV_BYTES + a * ATOM_BYTES, &P.tv, full, a * 64, n0, hk, b);
-            }
+            fa_mbar_expect_tx(full, 2 * TILE_BYTES);
+            fa_tma_load_4d(sb + OFF_K + kb * TILE_BYTES, &P.tk, full, 0, n0, hk, b);
+            fa_tma_load_4d(sb + OFF_V + kb * TILE_BYTES, &P.tv, full, 0, n0, hk, b);
           }
           const int s = gn % NSTAGE;
           const fa_u32 ph = (fa_u32)((gn / NSTAGE) & 1);
@@ -365,13 +358,11 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
           // one transaction count covers all the copies
           const long long rbase = ((long long)b * p.Hq + h) * sq_pad + m0;
           const fa_u32 full = bar_addr(sb, BAR_QFULL + s);
-          fa_mbar_expect_tx(full, 2 * Q_BYTES + 2 * BQ * 4);
-          for (int a = 0; a < DATOMS; ++a)
-            fa_tma_load_4d(sb + OFF_DO + s * Q_BYTES + a * Q_ATOM_BYTES, &P.tdo, full, a * 64, m0, h, b);
+          fa_mbar_expect_tx(full, 2 * TILE_BYTES + 2 * BQ * 4);
+          fa_tma_load_4d(sb + OFF_DO + s * TILE_BYTES, &P.tdo, full, 0, m0, h, b);
           if (gn >= NSTAGE) ok = fa_mbar_wait(bar_addr(sb, BAR_QEMPTY + s), ph ^ 1u, abort_flag);
           if (!ok) break;
-          for (int a = 0; a < DATOMS; ++a)
-            fa_tma_load_4d(sb + OFF_Q + s * Q_BYTES + a * Q_ATOM_BYTES, &P.tq, full, a * 64, m0, h, b);
+          fa_tma_load_4d(sb + OFF_Q + s * TILE_BYTES, &P.tq, full, 0, m0, h, b);
           fa_bulk_load(sb + OFF_ROW + s * 2 * BQ * 4, P.nlse2 + rbase, BQ * 4, full);
           fa_bulk_load(sb + OFF_ROW + s * 2 * BQ * 4 + BQ * 4, P.ndelta + rbase, BQ * 4, full);
         }
@@ -380,10 +371,8 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
         if (KVBUF == 1 && ok && next < n_items) {
           const Item i2 = item_at(next, p.Hkv, p.B, n_kvt, P.chunk_heads);
           const int hk2 = i2.hk, b2 = i2.b, n2 = i2.kt * BT;
-          for (int a = 0; a < DATOMS; ++a) {
-            tma_prefetch_l2_4d(&P.tk, a * 64, n2, hk2, b2);
-            tma_prefetch_l2_4d(&P.tv, a * 64, n2, hk2, b2);
-          }
+          tma_prefetch_l2_4d(&P.tk, 0, n2, hk2, b2);
+          tma_prefetch_l2_4d(&P.tv, 0, n2, hk2, b2);
         }
       }
       if (np > 0) ++kvc;
@@ -412,7 +401,7 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
       if (np < 0) break;
       if (np == 0) continue;
       const int kb = kvc % KVBUF;
-      const fa_u32 loK_k = fa_desc_lo(sb + OFF_K + kb * KV_BYTES, 16), loV_k = fa_desc_lo(sb + OFF_V + kb * KV_BYTES, 16);
+      const fa_u32 loK_k = fa_desc_lo(sb + OFF_K + kb * TILE_BYTES, 16), loV_k = fa_desc_lo(sb + OFF_V + kb * TILE_BYTES, 16);
       ok = fa_mbar_wait_all(bar_addr(sb, BAR_KV + kb), (fa_u32)((kvc / KVBUF) & 1), abort_flag);
       for (int n = 0; n < np && ok; ++n, ++gn) {
         const int s = gn % NSTAGE;
@@ -420,17 +409,17 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
         if (ok && gn > 0) ok = fa_mbar_wait_all(bar_addr(sb, BAR_SFREE), (fa_u32)((gn - 1) & 1), abort_flag);
         if (!ok) break;
         fa_tc_fence_after();
-        const fa_u32 loQ = fa_desc_lo(sb + OFF_Q + s * Q_BYTES, 16), loDO = fa_desc_lo(sb + OFF_DO + s * Q_BYTES, 16);
+        const fa_u32 loQ = fa_desc_lo(sb + OFF_Q + s * TILE_BYTES, 16), loDO = fa_desc_lo(sb + OFF_DO + s * TILE_BYTES, 16);
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk)
           if (leader)
-            fa_mma_ss(tmem_u + COL_S, fa_desc_make(loK_k + kstep_kmajor(kk, ATOM_BYTES), HI),
-                      fa_desc_make(loQ + kstep_kmajor(kk, Q_ATOM_BYTES), HI), IDESC_KK, kk > 0);
+            fa_mma_ss(tmem_u + COL_S, fa_desc_make(loK_k + kstep_kmajor(kk, TILE_BYTES), HI),
+                      fa_desc_make(loQ + kstep_kmajor(kk, TILE_BYTES), HI), IDESC_KK, kk > 0);
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk)
           if (leader)
-            fa_mma_ss(tmem_u + COL_DP, fa_desc_make(loV_k + kstep_kmajor(kk, ATOM_BYTES), HI),
-                      fa_desc_make(loDO + kstep_kmajor(kk, Q_ATOM_BYTES), HI), IDESC_KK, kk > 0);
+            fa_mma_ss(tmem_u + COL_DP, fa_desc_make(loV_k + kstep_kmajor(kk, TILE_BYTES), HI),
+                      fa_desc_make(loDO + kstep_kmajor(kk, TILE_BYTES), HI), IDESC_KK, kk > 0);
         if (leader) {
           fa_mma_commit(bar_addr(sb, BAR_SFULL));
           fa_mma_commit(bar_addr(sb, BAR_QEMPTY + s));  // first of the two arrivals that free each tile of the stage
@@ -462,10 +451,10 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
         if (ok && n == 0 && kvc > 0) ok = fa_mbar_wait_all(bar_addr(sb, BAR_DKVFREE), (fa_u32)((kvc - 1) & 1), abort_flag);
         if (!ok) break;
         fa_tc_fence_after();
-        // B operands read MN-major: the D columns are 64-element groups Q_ATOM_BYTES apart, a
+        // B operands read MN-major: the D columns are 64-element groups TILE_BYTES apart, a
         // k-step is 16 q rows = 2048 bytes
-        const fa_u32 loQ_mn = fa_desc_lo(sb + OFF_Q + s * Q_BYTES, Q_ATOM_BYTES);
-        const fa_u32 loDO_mn = fa_desc_lo(sb + OFF_DO + s * Q_BYTES, Q_ATOM_BYTES);
+        const fa_u32 loQ_mn = fa_desc_lo(sb + OFF_Q + s * TILE_BYTES, TILE_BYTES);
+        const fa_u32 loDO_mn = fa_desc_lo(sb + OFF_DO + s * TILE_BYTES, TILE_BYTES);
         const fa_u32 loDS_k = fa_desc_lo(sb + OFF_DS + (gn % NDS) * DS_BYTES, 16);
         const fa_u32 acc = n > 0;  // the first pair of an item starts its dK and dV
         // 3. dV += P^T dO      (K = BQ q values; A from TMEM)
@@ -481,7 +470,7 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
 #pragma unroll
         for (int kk = 0; kk < BQ / 16; ++kk)
           if (leader)
-            fa_mma_ss(tmem_u + COL_DK, fa_desc_make(loDS_k + kstep_kmajor(kk, ATOM_BYTES), HI),
+            fa_mma_ss(tmem_u + COL_DK, fa_desc_make(loDS_k + kstep_kmajor(kk, TILE_BYTES), HI),
                       fa_desc_make(loQ_mn + kk * 128, HI), IDESC_TN, acc | (kk > 0));
         if (leader) {
           fa_mma_commit(bar_addr(sb, BAR_QEMPTY + s));   // second arrival: the Q tile and row scalars are free
@@ -509,7 +498,7 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
       if (np < 0) break;
       if (np == 0) continue;
       const int kb = kvc % KVBUF;
-      const fa_u32 loK_mn = fa_desc_lo(sb + OFF_K + kb * KV_BYTES, ATOM_BYTES);
+      const fa_u32 loK_mn = fa_desc_lo(sb + OFF_K + kb * TILE_BYTES, TILE_BYTES);
       ok = fa_mbar_wait_all(bar_addr(sb, BAR_KV + kb), (fa_u32)((kvc / KVBUF) & 1), abort_flag);
       for (int n = 0; n < np && ok; ++n, ++gn) {
         ok = fa_mbar_wait_all(bar_addr(sb, BAR_PREADY), (fa_u32)(gn & 1), abort_flag);
@@ -522,7 +511,7 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
         if (ok && gn > 0) ok = fa_mbar_wait_all(bar_addr(sb, BAR_DQFREE), (fa_u32)((gn - 1) & 1), abort_flag);
         if (!ok) break;
         fa_tc_fence_after();
-        const fa_u32 loDS_mn = fa_desc_lo(sb + OFF_DS + (gn % NDS) * DS_BYTES, ATOM_BYTES);
+        const fa_u32 loDS_mn = fa_desc_lo(sb + OFF_DS + (gn % NDS) * DS_BYTES, TILE_BYTES);
         // 5. dQ = dS K: K = 128 kv rows, a k-step is 16 rows = 2048 bytes of either operand; A = dS^T read MN-major
         //    (M = 128 q: two 64-column atoms), B = K (N = 64 d)
 #pragma unroll
@@ -640,7 +629,7 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
 #pragma unroll
           for (int c = 0; c < CW / 8; ++c) {
             const int col = half * CW + 8 * c;
-            unsigned char* dsrow = sm + OFF_DS + (gn % NDS) * DS_BYTES + (col >> 6) * ATOM_BYTES + r * 128;
+            unsigned char* dsrow = sm + OFF_DS + (gn % NDS) * DS_BYTES + (col >> 6) * TILE_BYTES + r * 128;
             uint4 w;
             w.x = ds[4 * c]; w.y = ds[4 * c + 1]; w.z = ds[4 * c + 2]; w.w = ds[4 * c + 3];
             *(uint4*)(dsrow + ((((col & 63) >> 3) ^ (r & 7)) * 16)) = w;
@@ -732,12 +721,11 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
         }
         fa_tc_fence_after();
 #pragma unroll 1
-        for (int part = 0; part < 2 * DATOMS; ++part) {
-          const int which = part / DATOMS, a = part - which * DATOMS;  // dK atoms first, then dV
+        for (int which = 0; which < 2; ++which) {  // dK, dV
           const float mul = which == 0 ? p.scale : 1.f;
           // two K / V buffers: the staging buffers are the item's own K and V tiles, which nothing reads
           // any more; one: the parts go through the dQ staging buffer one after the other
-          const int st_off = KVBUF == 2 ? (which == 0 ? OFF_K : OFF_V) + kb * KV_BYTES + a * ATOM_BYTES : OFF_DQ;
+          const int st_off = KVBUF == 2 ? (which == 0 ? OFF_K : OFF_V) + kb * TILE_BYTES : OFF_DQ;
           unsigned char* strow = sm + st_off + r * 128;
           if (KVBUF == 1) {
             // the previous bulk operations must have finished reading the staging buffer
@@ -747,7 +735,7 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
             float o[16];
-            fa_tmem_ld16(t_lane + (which == 0 ? COL_DK : COL_DV) + a * 64 + c * 16, o);
+            fa_tmem_ld16(t_lane + (which == 0 ? COL_DK : COL_DV) + c * 16, o);
             fa_tmem_wait_ld();
 #pragma unroll
             for (int e = 0; e < 16; e += 8) {
@@ -759,24 +747,22 @@ extern "C" __global__ void __launch_bounds__(fa_btc::NT, 1) fa_bwd_tc_kernel(con
               *(uint4*)(strow + (((2 * c + (e >> 3)) ^ (r & 7)) * 16)) = w;
             }
           }
-          if (part == 2 * DATOMS - 1) {
+          if (which == 1) {
             // dK and dV are out of TMEM: the next item's first products may overwrite them
             fa_tc_fence_before();
             fa_mbar_arrive(bar_addr(sb, BAR_DKVFREE));
           }
-          if (KVBUF == 1 || part == 2 * DATOMS - 1) {
+          if (KVBUF == 1 || which == 1) {
             fence_proxy_async();
             named_bar_sync(1, 128);
           }
           if (dtid == 0) {
             if (KVBUF == 1) {
-              fa_tma_store_4d(which == 0 ? &P.tdk : &P.tdv, sb + OFF_DQ, a * 64, n0, hk, b);
+              fa_tma_store_4d(which == 0 ? &P.tdk : &P.tdv, sb + OFF_DQ, 0, n0, hk, b);
               bulk_commit();
-            } else if (part == 2 * DATOMS - 1) {
-              for (int a2 = 0; a2 < DATOMS; ++a2) {
-                fa_tma_store_4d(&P.tdk, sb + OFF_K + kb * KV_BYTES + a2 * ATOM_BYTES, a2 * 64, n0, hk, b);
-                fa_tma_store_4d(&P.tdv, sb + OFF_V + kb * KV_BYTES + a2 * ATOM_BYTES, a2 * 64, n0, hk, b);
-              }
+            } else if (which == 1) {
+              fa_tma_store_4d(&P.tdk, sb + OFF_K + kb * TILE_BYTES, 0, n0, hk, b);
+              fa_tma_store_4d(&P.tdv, sb + OFF_V + kb * TILE_BYTES, 0, n0, hk, b);
               bulk_commit();
               bulk_wait_read0();
               fa_mbar_arrive(bar_addr(sb, BAR_KVFREE + kb));

@@ -255,7 +255,7 @@ extern "C" __global__ void __launch_bounds__(fa_b128::NT, 1) fa_bwd_tc_kernel(co
       const Item it = item_of(min(idx, n_items - 1), p.Hkv, p.B, n_kvt, P.chunk_heads);
       const int hk = it.hk, b = it.b, kt = it.kt;
       int np = -1;
-      if (idx < n_items) np = build_pair_list<BQ, MAXPL, MAXC>(p, hk, b, kt, G, n_qtiles, (unsigned*)(sm + OFF_CLS), pl, lane);
+      if (idx < n_items) np = build_pair_list<MAXPL, MAXC>(p, hk, b, kt, G, n_qtiles, (unsigned*)(sm + OFF_CLS), pl, lane);
       if (lane == 0) {
         item[4 * lb] = hk;
         item[4 * lb + 1] = b;
