@@ -68,7 +68,7 @@ MIN_LEG_SECONDS = 0.5
 # kernels without a capture are absent.
 NCU_TRAFFIC = {
     "cfg2": {"fa_fwd_tc_kernel": 4 * 12.65e6, "fa_bwd_tc_kernel": 4 * 25.58e6},
-    "cfg4": {"fa_fwd_tc_kernel": 2 * (248.4e6 + 49.8e6), "fa_bwd_tc_kernel": 2 * (649.6e6 + 360.2e6)},
+    "cfg4": {"fa_fwd_tc_kernel": 2 * (248.4e6 + 49.8e6), "fa_bwd_tc_kernel": 2 * (598.5e6 + 316.1e6)},
 }
 
 # S x S x D products per computed block pair that count as algorithmic work of each kernel: the

@@ -1501,12 +1501,11 @@ int get_bwd_tc_kernel(fa_module* m, int dtype, int D, int flags, bool kv2, Kerne
 // win (dense B8 H8 S2048, see fa_bwd_tc.cuh).
 bool bwd_tc_kv2(const fa_attn_params* p) { return p->D == 64 && p->tables.kv_num_blocks != nullptr; }
 
-// (batch, kv head) pairs whose items the backward works through together (item_of in fa_bwd_tc.cuh): as many as
-// keep their dQ accumulators, Q and dO in L2 (126 MB), if that leaves an item for every SM, or three where items
-// are uneven (tables: the heavy items of a late chunk end up alone otherwise, causal B2 H16/4 S3001 D128
-// 388 -> 435 us).  Measured with all heads together and with chunks (us): attention sink B4 H16 S8192 D128
-// 1061 -> 1023 with 96 MB; dense B4 H8 S4096 D128 745 -> 738 with 96 MB, 714 with 24 MB.  Where the items are
-// uneven small chunks cost balance: causal + ALiBi B8 H8 S2048 D64 174 -> 189 with 24 MB.
+// (batch, kv head) pairs whose items the backward works through together (item_of in fa_bwd_items.cuh; not with two K / V buffers): as
+// many as keep their dQ accumulators, Q and dO in L2 (126 MB), if that leaves an item for every SM, or three where items are uneven
+// (tables: the heavy items of a late chunk end up alone otherwise).  Kernel alone at head dim 128, us, all heads together / chunks of
+// 96 / 48 / 24 / 12 MB: attention sink B4 H16 S8192 856 / 807 / 814 / 818 / 824, dense B4 H8 S4096 623 / 613 / 596 / 590 / 592, causal B2 H8
+// S4096 179 / 181 / 222 / 223 / 234; causal + ALiBi B4 H16 S2048 205 / 220 / 223 / 248 / 242, where the rule takes 96 MB and all would be better.
 int bwd_tc_chunk_heads(const fa_attn_params* p) {
   const long long heads = (long long)p->B * p->Hkv, n_kvt = (p->Skv + 127) / 128;
   const long long per_head = (long long)(p->Hq / p->Hkv) * ((p->Sq + 127) / 128 * 128) * p->D * (4 + 2 + 2);

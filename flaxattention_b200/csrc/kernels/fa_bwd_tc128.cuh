@@ -14,8 +14,9 @@
 // Why this shape: an instruction with N = 128 reads 8 KB of operands for 64 clocks of math, one with N = 64 6 KB for 32,
 // and shared memory delivers 128 bytes a clock: per 128 x 128 scores the five products read 256 KB (dV and dK take their A
 // operand from TMEM) where pairs of 64 query rows read 384, and a pair has the same number of hand-overs between
-// the roles for twice the work.  Against pairs of 64 query rows (kernel alone, us): dense B4 H8 S4096 668 -> 579, attention sink
-// B4 H16 S8192 881 -> 815, causal B2 H8 S4096 199 -> 170, causal + ALiBi B4 H16 S2048 238 -> 206.
+// the roles for twice the work.  Against pairs of 64 query rows (kernel alone, us, both from one box): dense B4 H8 S4096
+// 666 -> 582, attention sink B4 H16 S8192 865 -> 799, causal B2 H8 S4096 199 -> 173, causal + ALiBi B4 H16 S2048 234 -> 218.  Few rows that
+// end early in a tile lose (B2 H4 S192, a pass: 17.0 -> 18.1): their last pair has 128 rows all the same.
 #pragma once
 #include "fa_bwd_items.cuh"
 

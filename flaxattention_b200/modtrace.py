@@ -1392,7 +1392,7 @@ def to_cuda_range(mod: TracedMod, name: str) -> Optional[str]:
     position, 2 where it is true for every one, 1 where the intervals do not tell.  None if they never would.
 
     An integer node is a pair of bounds, a boolean one a pair (certainly true, certainly false); floats, loads from
-    captured tensors and whatever else has no rule here is unknown.  A node whose values could leave int32 for indices below
+    captured tensors and whatever else has no rule here (a remainder by a power of two is a bitwise and) is unknown.  A node whose values could leave int32 for indices below
     ``_IDX_BOUND`` is unknown too (the arithmetic of the mask wraps there), and so is every rectangle beyond that bound."""
     lines: List[str] = []
     env: Dict[int, Optional[tuple]] = {}  # int: (lo text, hi text, static lo, static hi); bool: (true text, false text)
