@@ -116,6 +116,7 @@ class BlockMask:
     mask_bits: Optional[torch.Tensor] = None
     # the same matrix transposed [1 or B, 1 or H, KV_LEN, words], or None
     mask_bits_t: Optional[torch.Tensor] = None
+    _bits_at = (None, None)  # (of objects that were saved without it)
 
     def __init__(self, kv_num_blocks, kv_indices, full_kv_num_blocks, full_kv_indices, q_num_blocks, q_indices,
                  full_q_num_blocks, full_q_indices, BLOCK_SIZE, mask_mod, mask_bits=None, mask_bits_t=None,
