@@ -1115,12 +1115,13 @@ int get_bwd_rerun_kernel(fa_module* m, int dtype, int D, int Dv, const BwdCfg& c
                                        {"FA_WARPS", c.warps}, {"FA_ROUND_SCORES", 0}, {"FA_RERUN", 1}}); },
                     "fa_bwd_rerun_kernel", std::max(c.smem_dq, c.smem_dkdv), k);
 }
-int get_decode_kernel(fa_module* m, int dtype, int D, int Dv, int flags, const DecCfg& c, bool pack, bool cluster, Kernel** k) {
+int get_decode_kernel(fa_module* m, int dtype, int D, int Dv, int flags, const DecCfg& c, bool pack, bool cluster, bool two, Kernel** k) {
   const int rnd = round_flag(dtype, flags);
-  return get_kernel(m, kernel_key(kIdDecode, {{dtype, 2}, {D, 9}, {Dv, 9}, {c.BM, 9}, {c.BN, 9}, {rnd, 1}, {pack ? 1 : 0, 1}, {cluster ? 1 : 0, 1}}),
+  return get_kernel(m, kernel_key(kIdDecode, {{dtype, 2}, {D, 9}, {Dv, 9}, {c.BM, 9}, {c.BN, 9}, {rnd, 1}, {pack ? 1 : 0, 1}, {cluster ? 1 : 0, 1}, {two ? 1 : 0, 1}}),
                     "fa_decode.cuh",
                     [&] { return defs({{"FA_DTYPE", dtype}, {"FA_D", D}, {"FA_DV", Dv}, {"FA_BM", c.BM}, {"FA_BN", c.BN},
-                                       {"FA_ROUND_SCORES", rnd}, {"FA_PACK_HEADS", pack ? 1 : 0}, {"FA_CLUSTER", cluster ? 1 : 0}}); },
+                                       {"FA_ROUND_SCORES", rnd}, {"FA_PACK_HEADS", pack ? 1 : 0}, {"FA_CLUSTER", cluster ? 1 : 0},
+                                       {"FA_TWO_PARTS", two ? 1 : 0}}); },
                     "fa_decode_kernel", c.smem, k);
 }
 // Grouped-query decode: the G query heads of a kv head share one CTA (their G * Sq rows form one
@@ -1560,9 +1561,10 @@ int fa_module_prepare(fa_module* m, int kind, int dtype, int D, int Dv, int Sq_h
       if (int rc = pick_decode(dtype, D, Dv, Sq_hint, nullptr, c)) return rc;
       if (dtype != FA_F32 && D == 64 && Dv == 64 && Sq_hint > 16)
         if (int rc = get_fwd_tc_kernel(m, dtype, D, 0, &k, true)) return rc;
+      const bool two = c.BM == 16 && Sq_hint > 8 && !(D == 64 && Dv == 64 && Skv_hint >= 1024 && Skv_hint <= 32768);
       if (c.BM == 16)
-        if (int rc = get_decode_kernel(m, dtype, D, Dv, 0, c, false, true, &k)) return rc;
-      return get_decode_kernel(m, dtype, D, Dv, 0, c, false, false, &k);
+        if (int rc = get_decode_kernel(m, dtype, D, Dv, 0, c, false, true, two, &k)) return rc;
+      return get_decode_kernel(m, dtype, D, Dv, 0, c, false, false, two, &k);
     }
     case FA_KIND_BLOCKMASK:
       if (int rc = get_blockmask_kernel(m, false, &k)) return rc;
@@ -1833,7 +1835,9 @@ int fa_decode(fa_module* m, const fa_attn_params* p, int num_splits, void* works
     if (int rc = launch_decode_tc(m, p, kp, num_splits, stream)) return rc;
   } else {
     Kernel* k = nullptr;
-    if (int rc = get_decode_kernel(m, p->dtype, p->D, p->Dv, p->flags, c, pack, cluster, &k)) return rc;
+    // (the second part of P as an instruction of its own: see fa_decode.cuh)
+    const bool two = c.BM == 16 && (pack ? p->Sq * (p->Hq / p->Hkv) : p->Sq) > 8 && (pack || !tc_decode_covers(p));
+    if (int rc = get_decode_kernel(m, p->dtype, p->D, p->Dv, p->flags, c, pack, cluster, two, &k)) return rc;
     if (int rc = launch(k, dim3(num_splits, pack ? p->Hkv : p->Hq, p->B), dim3(128), &kp, stream, cluster ? num_splits : 1)) return rc;
   }
   if (num_splits > 1 && !cluster) {

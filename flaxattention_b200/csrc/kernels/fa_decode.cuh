@@ -47,6 +47,9 @@ __device__ __forceinline__ float4 fa_ld_cluster_f4(fa_u32 addr) {
 #ifndef FA_PACK_HEADS
 #define FA_PACK_HEADS 0
 #endif
+#ifndef FA_TWO_PARTS
+#define FA_TWO_PARTS 0  // 9 to 16 rows: the second part of the probabilities as a second instruction
+#endif
 #ifndef FA_CLUSTER
 #define FA_CLUSTER 0  // the splits of a tile of rows are launched as a cluster (a variant of its own: with the merge in the kernel of
 #endif                // all calls those without it took up to 7 % more, B16 H16 Skv1024 D64 16 rows 17.4 -> 18.6 us)
@@ -80,10 +83,10 @@ constexpr int SMEM_BYTES = Q_BYTES + (PIPE_BYTES > MRG_BYTES ? PIPE_BYTES : MRG_
 // where a probability is exactly 1, at a running maximum, so that the fewer of these (fewer splits) the worse the results:
 // B16 H32/8 Skv8191 D128 bf16, relative error against 64 bits, 2.11e-3 with three splits, 2.20e-3 with two, 1.66e-3 in two parts, nearly all
 // of it the rounding of the output.  Up to 8 rows the second part lies in the 8 rows of the instruction that hold no query
-// and costs nothing; up to 16 it takes a second instruction (B3 H16 Skv4096 D128, 16 rows: 28.3 us, 28.7 without).  The 16 rows of one
-// head at head dim 64 have no time for that (B8 H8 Skv8192 34.3 us, 31.5 without) and stay with one part (error 2.18e-3 bf16; of the tcgen05 kernel there 2.32e-3).
+// and costs nothing; up to 16 it takes a second instruction (FA_TWO_PARTS; B3 H16 Skv4096 D128, 16 rows: 28.3 us, 28.7 without), which
+// the host asks for but where the tcgen05 kernel could run too: there one part is as good as that one (B8 H8 Skv8192 D64, 16 rows, bf16: error
+// 2.18e-3 against 2.32e-3), and the second instruction costs time (34.3 us, 31.5 without).
 constexpr bool TWO_PARTS = RG == 1;
-constexpr bool SECOND_MMA = TWO_PARTS && (PACK || D > 64);
 
 static_assert(DT != FA_DT_F32, "the decode kernel takes 16-bit inputs");
 static_assert(BM == 16 || BM == 32 || BM == 64, "BM must be 16, 32 or 64");
@@ -290,7 +293,7 @@ extern "C" __global__ void __launch_bounds__(fa_dec::NT) fa_decode_kernel(const 
     have_nxt = have && next_tile(n0_nxt, full_nxt);
     if (have_nxt) load_k(cur, n0_nxt);
     fa_cp_commit();
-    if (SECOND_MMA && R > 8) fa_mma_nn<DT, WN, DV, true>(o, s, sV + cur * V_BYTES + cg * WN * PV, PV, lane);
+    if (TWO_PARTS && FA_TWO_PARTS && R > 8) fa_mma_nn<DT, WN, DV, true>(o, s, sV + cur * V_BYTES + cg * WN * PV, PV, lane);
     else fa_mma_nn<DT, WN, DV>(o, s, sV + cur * V_BYTES + cg * WN * PV, PV, lane);
     cur ^= 1;
   }

@@ -60,6 +60,7 @@ def test_many_splits_match_the_oracle():
     (8, 2, 2, 1111, 128, 128),   # eight rows of a packed tile: the second part lies over all eight spare rows
     (2, 2, 9, 1024, 128, 48),    # the first that takes a second instruction
     (4, 1, 4, 900, 64, 16),      # the last, four heads to a tile
+    (2, 2, 16, 1100, 64, 64),
     (1, 1, 5, 1500, 256, 256),
 ])
 @pytest.mark.parametrize("splits", [1, 2, 9])
