@@ -1732,8 +1732,11 @@ static int decode_ctas_per_sm(const DecCfg& c) { return std::min(std::max((228 *
 // Splits of the general decode kernel for `bh` tiles of query rows over `tiles` 128-key tiles.
 //   * Two CTAs per SM, all resident at once, stream as fast as more do, and every further split costs its start and its
 //     merge; at least four tiles per CTA.
-//   * Many heads: one split leaves SMs with one CTA beside SMs with two.  Over long caches (24 tiles per CTA and more) several
-//     waves that end nearly full are faster then.
+//   * One split, all resident at once: it leaves SMs with one CTA beside SMs with two.  Over long caches (24 tiles per CTA and more)
+//     several waves that end nearly full are faster then.
+//   * More tiles of rows than that: the first count whose waves end nearly full, unless one split's do (D 64, one row, us, one split /
+//     so: 512 x 4096 keys 103 / 89, 512 x 8192 208 / 167, 320 x 8192 124 / 108, 640 x 4096 113 / 108, 1024 x 4096 173 / 166; 768, whose
+//     one split is 0.865 full, 127 / 128 with four).
 //   * More than 16 rows: the products, not the keys' way from memory, set the pace, and what counts is a last wave that is nearly
 //     full (B5 H32/8 62 rows Skv1935 D128: one split 96 us, three 87; B7 H32 64 rows Skv30000 1260 / 960 with nine).
 //   * Few heads: up to FA_DECODE_MAX_CLUSTER splits are merged inside a cluster, more by the combine kernel; where even a
@@ -1745,15 +1748,18 @@ static int general_decode_splits(long long bh, int tiles, int per_sm, int sm_cou
   if (row_groups > 1) return fill_waves(bh, cmax, per_sm * sm_count);
   const int c = (int)std::min<long long>(cmax, std::max<long long>(1, std::min(per_sm, 2) * sm_count / bh));
   if (c == 1) {
-    // (how full the waves of k splits are; 0 for less than one)
-    const auto fill = [&](int k) {
-      const double waves = (double)(bh * k) / (per_sm * sm_count);
-      return waves > 1.0 ? waves / (double)(long long)(waves + 0.999999) : 0.0;
-    };
+    const auto waves = [&](int k) { return (double)(bh * k) / (per_sm * sm_count); };
+    const auto fill = [&](int k) { return waves(k) / (double)(long long)(waves(k) + 0.999999); };  // of the last wave and those before it
+    if (bh > 2LL * sm_count) {
+      if (fill(1) >= 0.86) return 1;
+      for (int k = 2; k <= std::min(FA_DECODE_MAX_CLUSTER, tiles / 4); ++k)
+        if (fill(k) >= 0.88) return k;
+      return 1;
+    }
     int best = 1;
-    double best_fill = std::max(0.88, fill(1));
+    double best_fill = 0.88;
     for (int k = 2; k <= std::min(FA_DECODE_MAX_CLUSTER, tiles / 24); ++k)
-      if (fill(k) > best_fill) {
+      if (waves(k) > 1.0 && fill(k) > best_fill) {
         best = k;
         best_fill = fill(k);
       }
