@@ -1200,7 +1200,7 @@ bool tc_fwd_eligible(const fa_attn_params* p) {
 int get_fwd_tc_kernel(fa_module* m, int dtype, int D, int flags, Kernel** k, bool decode = false, int nq = 2) {
   // must match the shared-memory map of fa_fwd_tc.cuh (fa_tc::SMEM_BYTES)
   const int atoms = dtype == FA_F32 ? 3 : D / 64, nstage = decode ? 5 : (dtype == FA_F32 ? 1 : (D == 64 ? nq + 1 : nq));
-  const int smem = nq * atoms * 16384 + 2 * nstage * atoms * 16384 + (1 + 4 * nstage + 8) * 8 + 16 + 256 * 2 + 256 * 2 +
+  const int smem = nq * atoms * 16384 + 2 * nstage * atoms * 16384 + (1 + 4 * nstage + 13) * 8 + 16 + (256 + 4) * 4 +
                    2 * 256 + (256 / 32) * 4 + 1024;
   const int rnd = round_flag(dtype, flags);
   return get_kernel(m, kernel_key(kIdFwdTc, {{dtype, 2}, {D, 9}, {rnd, 1}, {decode ? 1 : 0, 1}, {nq, 2}}), "fa_fwd_tc.cuh",

@@ -27,14 +27,19 @@
 // past both (or one, see NQ: then without warps 4-7, and the roles below move up).  Warp roles (12 warps = 3 warpgroups):
 //   warps 0-3  softmax warpgroup of query tile 0      warps 4-7  of query tile 1
 //   warp 8     TMA producer (one lane)
-//   warps 9-10 MMA issuers; warp 9 also allocates / frees TMEM.  With D = 64 warp 9 issues the S products and
-//              warp 10 the PV products (one lane each); where P lies over S (D = 128, fp32) warp 9 issues
-//              all products of both query tiles in turn; warp 11 is idle
+//   warps 9-10 MMA issuers; warp 9 also allocates / frees TMEM.  With D = 64 each issues the products of one query tile;
+//              where P lies over S for the rest of the step (D = 128, fp32) warp 9 issues all products of both query
+//              tiles in turn; in the decode variant warp 9 issues the S products and warp 10 the PV products.  Warp 11 is idle
 // Registers are moved from the third warpgroup to the two softmax warpgroups (setmaxnreg),
 // which hold a whole 128-column score row per thread.
-// The S columns of a tile are released as soon as its scores are in registers, so with D = 64
-// S of step j+1 is computed while the softmax of step j runs; with D = 128 (P over the S
-// columns) the products of a tile form the chain  PV(j), S(j+1), PV(j+1) ...
+// With D = 64 the S columns of a tile are released as soon as its scores are in registers, and S of step j+1 is
+// computed while the softmax of step j runs (see ROT); with D = 128 (P over the S columns) the products of a tile form
+// the chain  PV(j), S(j+1), PV(j+1) ... and all the latencies between them count: P is handed over in two parts (see
+// SPLIT_P), and the issuing warp has waited for everything else that a product needs before P is there.
+// What bounds it (clock stamps, dense, two tiles): D = 64, a step of both tiles is 2400 clk, of which 2060 are the
+// instructions of the two softmax warps of a scheduler (two warps in a loop of their own, without barriers and
+// products, take that; the SFU alone 1536); D = 128, 2900 clk of chain against 2048 clk of products.  B8 H8 S2048 D64
+// checkerboard 124 -> 116 us, B4 H8 S4096 D64 208 -> 198, D128 267 -> 258, attention sink B4 H16 S8192 D128 411 -> 363.
 // The running maximum is only raised when it grew by more than 2^8 (the stale maximum is
 // exact as long as it is used consistently), so rescaling O in TMEM is rare.
 //
@@ -91,25 +96,28 @@ constexpr int NSTAGE = DECODE ? 5 : (F32 ? 1 : (D == 64 ? NQ + 1 : NQ));
 constexpr int Q_BYTES = NQ * ATOMS * ATOM_BYTES;
 constexpr int KV_STAGE = ATOMS * ATOM_BYTES;
 constexpr int MAXT = 256;                // kv tiles per row of the block grid (Skv <= 32768)
-constexpr int NBARS = 1 + 4 * NSTAGE + 8;
+constexpr int NBARS = 1 + 4 * NSTAGE + 13;
 constexpr int OFF_K = Q_BYTES;
 constexpr int OFF_V = OFF_K + NSTAGE * KV_STAGE;
 constexpr int OFF_BAR = OFF_V + NSTAGE * KV_STAGE;
 constexpr int OFF_MISC = OFF_BAR + NBARS * 8;       // tmem base, abort flag, nsteps, pad
-constexpr int OFF_SCHED = OFF_MISC + 16;            // short tile[MAXT]
-constexpr int OFF_MODE = OFF_SCHED + MAXT * 2;      // uchar mode[MAXT][2]
-constexpr int OFF_CLS = OFF_MODE + MAXT * 2;        // uchar cls[2][MAXT]
+constexpr int OFF_SCHED = OFF_MISC + 16;            // u32 sched[MAXT + 4]: kv tile | mode of query tile 0 << 16 | mode of query tile 1 << 24
+constexpr int OFF_CLS = OFF_SCHED + (MAXT + 4) * 4; // uchar cls[2][MAXT]
 constexpr int OFF_WCNT = OFF_CLS + 2 * MAXT;        // int wcount[MAXT / 32]: listed tiles per warp of the schedule build
 constexpr int SMEM_BYTES = OFF_WCNT + (MAXT / 32) * 4 + 1024;  // + slack for the 1024-byte alignment
 constexpr int TMEM_COLS = 256 * NQ;
 // fp32: scores of tile i in columns 192 i .. + 127.  The softmax writes the parts of P over the scores it
 // has just read, 16 columns (32 keys) at a time: hi and mid of keys 32 c .. + 31 go to columns 32 c .. + 15
 // and 32 c + 16 .. + 31, lo to 128 + 16 c .. + 15.  O of tile i and step in 384 + 64 i.
-constexpr int COL_S = 0, COL_O = F32 ? 384 : 128 * NQ, S_STRIDE = F32 ? 192 : 128;
-// With D = 64 there is TMEM left for P next to S (columns 384..511): S of the next kv step can
-// then be produced while the softmax of the current step is still writing P.  With D = 128 the
-// 512 columns are taken by S and O, and P overwrites the S columns it was computed from.
-constexpr bool SEP_P = D == 64 && !F32;
+// Head dim 64, forward (ROT): each tile has 192 columns for S and P.  In even steps S takes columns 0-127 and P
+// goes over columns 0-63, in odd steps S takes columns 64-191 and P goes over columns 128-191.  S of the next step
+// then never lies over P of this one (it is computed during this step's softmax), and P of a step never lies over
+// P of the last one, so the softmax does not wait for any P.V product.
+constexpr bool ROT = D == 64 && !F32 && !DECODE;
+constexpr int COL_S = 0, COL_O = F32 ? 384 : (ROT ? 192 : 128) * NQ, S_STRIDE = F32 || ROT ? 192 : 128;
+// In the decode variant P has columns of its own (384..511).  With D = 128 the 512 columns are taken by S and O, and
+// P overwrites the S columns it was computed from.
+constexpr bool SEP_P = DECODE;
 constexpr int COL_P = 192 * NQ;
 // One pair of exponentials in FA_TC_POLY_EVERY goes to the FMA pipe (a cubic, see fa_ex2_poly2).
 // Measured (B8 H8 S2048 D64): every fourth pair takes the forward without a score_mod from 0.118 to
@@ -139,10 +147,19 @@ __device__ constexpr int PROD_A[6] = {F32 ? 1 : 0, 0, 2, 0, 1, 0}, PROD_B[6] = {
 __device__ __forceinline__ fa_u32 bar_addr(fa_u32 sbase, int i) { return sbase + OFF_BAR + i * 8; }
 constexpr int BAR_Q = 0;
 constexpr int BAR_KFULL = 1, BAR_KEMPTY = 1 + NSTAGE, BAR_VFULL = 1 + 2 * NSTAGE, BAR_VEMPTY = 1 + 3 * NSTAGE;
-constexpr int BAR_S = 1 + 4 * NSTAGE, BAR_P = BAR_S + 2, BAR_O = BAR_S + 4;
-// With separate P columns the S columns of a tile are released as soon as the softmax warps
-// hold the scores in registers, and S of the next step is produced during the softmax.
-constexpr int BAR_SFREE2 = BAR_S + 6;
+// ROT: two barriers per tile for P and O, BAR_P + i and BAR_O + i for even steps, + 2 for odd ones.  (The warps of a
+// tile only meet at its S: one that is ahead may hand over P of a step before the others have handed over that of
+// the last one, and the softmax does not look at every PV product.)
+constexpr int BAR_S = 1 + 4 * NSTAGE, BAR_P = BAR_S + 2, BAR_O = BAR_S + 6;
+// Where P does not lie over S of the same step for long (ROT, SEP_P), the S columns of a tile are released as soon as
+// the softmax warps hold the scores in registers, and S of the next step is produced during the softmax.
+constexpr int BAR_SFREE2 = BAR_S + 10;
+constexpr int BAR_LAG = BAR_S + 12;  // (ROT) the first scores of the first tile are in registers; used once
+constexpr bool EARLY_S = ROT || SEP_P;
+// Head dim 128: P is handed over in two parts, keys 0-95 (BAR_P) and 96-127 (BAR_P2), so that most of the PV product
+// runs under the last exponentials.  It is the first link of the chain PV(j), S(j+1) that the tile then waits for.
+constexpr bool SPLIT_P = !ROT && !SEP_P && !F32;
+constexpr int BAR_P2 = BAR_S + 10;
 
 // Work on one 32-column chunk of a score row held in registers (columns C0 .. C0+31 of the kv
 // tile that starts at key n0).  C0 is a template parameter and n0 a multiple of 128, so the low
@@ -159,35 +176,17 @@ __device__ __forceinline__ void max_chunk(const float (&v)[32], RowMax& mx) {
     mx.d = fa_max3(mx.d, v[e + 6], v[e + 7]);
   }
 }
-// score_mod (and the rounding of the raw scores to the input type, when asked for) in place;
-// the results are in log2 units.  An affine score_mod (A * score + B) costs one FMA: A and B
-// absorb the scale and log2(e).
+// score_mod (and the rounding of the raw scores to the input type, when asked for) in place.  With a score_mod the
+// results are in log2 units and relative to the row's running maximum (negm is added): where that does not move, the
+// exponentials are taken of them as they are, without a subtraction of their own.  An affine score_mod
+// (A * score + B) costs one packed FMA per pair: A and B absorb the scale, log2(e) and the maximum.
+// (Without a score_mod the scores stay raw, the exponent's FMA applies the scale.)
+struct ModLinear {
+  fa_u64 m2, d2, b2;  // multiplier, slope over kv, bias at the first key of the tile (with the maximum)
+};
 template <int C0>
-__device__ __forceinline__ void mod_chunk(float (&v)[32], int n0, int qi, int gb, int gh, float scale, float sc2) {
-#if FA_HAS_SCORE_MOD && defined(FA_SCORE_AFFINE) && defined(FA_SCORE_LINEAR_KV)
-  // The multiplier does not read kv and the bias is linear in it (relative-position biases such as
-  // ALiBi): both are taken once, at the first column of the chunk, and column e adds e times the
-  // slope - two packed FMAs per pair instead of an integer subtraction, an int-to-float conversion
-  // (which shares the SFU with the exponentials) and a multiplication per element.
-  {
-    const int kv0 = n0 | C0;
-    const float mulsc = fa_score_mul(0.f, gb, gh, qi, kv0) * sc2;
-    const float base = fa_score_add2(0.f, gb, gh, qi, kv0);
-    const float dkv = fa_score_add2_dkv(0.f, gb, gh, qi, kv0);
-    const fa_u64 m2 = fa_f2(mulsc, mulsc), b2 = fa_f2(base, base), d2 = fa_f2(dkv, dkv);
-#pragma unroll
-    for (int e = 0; e < 32; e += 2) {
-      float x0 = v[e], x1 = v[e + 1];
-#if FA_ROUND_SCORES
-      fa_round2<DT>(x0, x1);
-#endif
-      fa_f2_unpack(fa_fma2(fa_f2(x0, x1), m2, fa_fma2(fa_f2((float)e, (float)(e + 1)), d2, b2)), x0, x1);
-      v[e] = x0;
-      v[e + 1] = x1;
-    }
-    return;
-  }
-#endif
+__device__ __forceinline__ void mod_chunk(float (&v)[32], int n0, int qi, int gb, int gh, float scale, float sc2, float negm,
+                                          const ModLinear& lin) {
 #pragma unroll
   for (int e = 0; e < 32; e += 2) {
     float x0 = v[e], x1 = v[e + 1];
@@ -196,15 +195,20 @@ __device__ __forceinline__ void mod_chunk(float (&v)[32], int n0, int qi, int gb
 #if FA_ROUND_SCORES
     fa_round2<DT>(x0, x1);
 #endif
-#if FA_HAS_SCORE_MOD && defined(FA_SCORE_AFFINE)
-    x0 = fmaf(x0, fa_score_mul(0.f, gb, gh, qi, kv0) * sc2, fa_score_add2(0.f, gb, gh, qi, kv0));
-    x1 = fmaf(x1, fa_score_mul(0.f, gb, gh, qi, kv1) * sc2, fa_score_add2(0.f, gb, gh, qi, kv1));
+#if FA_HAS_SCORE_MOD && defined(FA_SCORE_AFFINE) && defined(FA_SCORE_LINEAR_KV)
+    // The multiplier does not read kv and the bias is linear in it (relative-position biases such as ALiBi): both are
+    // taken once per step, at the first key of the tile, and column c adds c times the slope - two packed FMAs per
+    // pair instead of an integer subtraction, an int-to-float conversion (which shares the SFU with the exponentials)
+    // and a multiplication per element.
+    fa_f2_unpack(fa_fma2(fa_f2(x0, x1), lin.m2, fa_fma2(fa_f2((float)(C0 + e), (float)(C0 + e + 1)), lin.d2, lin.b2)), x0, x1);
+#elif FA_HAS_SCORE_MOD && defined(FA_SCORE_MUL_ONLY)
+    fa_f2_unpack(fa_fma2(fa_f2(x0, x1), fa_f2(fa_score_mul(0.f, gb, gh, qi, kv0) * sc2, fa_score_mul(0.f, gb, gh, qi, kv1) * sc2), fa_f2(negm, negm)), x0, x1);
+#elif FA_HAS_SCORE_MOD && defined(FA_SCORE_AFFINE)
+    fa_f2_unpack(fa_fma2(fa_f2(x0, x1), fa_f2(fa_score_mul(0.f, gb, gh, qi, kv0) * sc2, fa_score_mul(0.f, gb, gh, qi, kv1) * sc2),
+                         fa_add2(fa_f2(fa_score_add2(0.f, gb, gh, qi, kv0), fa_score_add2(0.f, gb, gh, qi, kv1)), fa_f2(negm, negm))), x0, x1);
 #elif FA_HAS_SCORE_MOD
-    x0 = fa_score_mod(x0 * scale, gb, gh, qi, kv0) * FA_LOG2E;
-    x1 = fa_score_mod(x1 * scale, gb, gh, qi, kv1) * FA_LOG2E;
-#else
-    x0 *= sc2;
-    x1 *= sc2;
+    x0 = fmaf(fa_score_mod(x0 * scale, gb, gh, qi, kv0), FA_LOG2E, negm);
+    x1 = fmaf(fa_score_mod(x1 * scale, gb, gh, qi, kv1), FA_LOG2E, negm);
 #endif
     v[e] = x0;
     v[e + 1] = x1;
@@ -218,7 +222,7 @@ __device__ __forceinline__ void mod_chunk(float (&v)[32], int n0, int qi, int gb
 // against 3.5k for a plain one: the step no longer fitted the instruction cache.)
 template <int NW>
 __device__ __forceinline__ void mask_bits(fa_u32 (&w)[NW], bool use_mask, int kv0, int qi, int gb, int gh, int Skv,
-                                          const unsigned* rowbits) {
+                                          bool have_words, const uint4& m) {
   // the end of the sequence alone needs no loop: word c covers keys kv0 + 32 c .. + 31
 #pragma unroll
   for (int c = 0; c < NW; ++c) {
@@ -226,15 +230,10 @@ __device__ __forceinline__ void mask_bits(fa_u32 (&w)[NW], bool use_mask, int kv
     w[c] = left >= 32 ? 0xffffffffu : (left <= 0 ? 0u : ((1u << left) - 1u));
   }
 #if FA_HAS_MASK_MOD
-  if (use_mask && rowbits != nullptr) {
+  if (use_mask && have_words) {
     // mask_mod was evaluated once for all positions (FaTables::mask_bits): this row's words of the tile
-    if (NW == 4) {
-      const uint4 m = *(const uint4*)(rowbits + (kv0 >> 5));
-      w[0] &= m.x; w[1] &= m.y; w[NW > 2 ? 2 : 0] &= m.z; w[NW > 2 ? 3 : 0] &= m.w;
-    } else {
-      const uint2 m = *(const uint2*)(rowbits + (kv0 >> 5));
-      w[0] &= m.x; w[1] &= m.y;
-    }
+    w[0] &= m.x; w[1] &= m.y;
+    if (NW == 4) { w[NW > 2 ? 2 : 0] &= m.z; w[NW > 2 ? 3 : 0] &= m.w; }
   } else if (use_mask) {
     // one rolled loop, the NW words side by side (independent evaluations in every iteration)
     fa_u32 m[NW];
@@ -250,18 +249,27 @@ __device__ __forceinline__ void mask_bits(fa_u32 (&w)[NW], bool use_mask, int kv
   }
 #endif
 }
+// the words of a row of the bit matrix for the NW * 32 keys from kv0 on
+template <int NW>
+__device__ __forceinline__ uint4 mask_words(const unsigned* rowbits, int kv0) {
+  if (NW == 4) return *(const uint4*)(rowbits + (kv0 >> 5));
+  const uint2 m = *(const uint2*)(rowbits + (kv0 >> 5));
+  return make_uint4(m.x, m.y, 0u, 0u);
+}
 __device__ __forceinline__ void mask_apply(float (&v)[32], fa_u32 bits) {
 #pragma unroll
   for (int e = 0; e < 32; ++e) v[e] = ((bits >> e) & 1u) ? v[e] : FA_NEG_INF;
 }
 
-// Pass-2 work on one chunk: p = 2^(x * cmul - m), packed to 16 bits, and the row-sum chains.
-__device__ __forceinline__ void pass2_chunk(const float (&v)[32], fa_u32 (&pk)[16], fa_u64 cmul, fa_u64 negm,
-                                            fa_u64& sum_a, fa_u64& sum_b) {
+// Pass-2 work on one chunk: p = 2^(x * cmul - m) (REL: 2^x, the scores are relative to m already), packed to 16 bits,
+// and the row-sum chains.
+template <bool REL, int E0, int E1>
+__device__ __forceinline__ void pass2_part(const float (&v)[32], fa_u32 (&pk)[16], fa_u64 cmul, fa_u64 negm,
+                                           fa_u64& sum_a, fa_u64& sum_b) {
 #pragma unroll
-  for (int e = 0; e < 16; ++e) {
-    float a0, a1;
-    fa_f2_unpack(fa_fma2(fa_f2(v[2 * e], v[2 * e + 1]), cmul, negm), a0, a1);
+  for (int e = E0; e < E1; ++e) {
+    float a0 = v[2 * e], a1 = v[2 * e + 1];
+    if (!REL) fa_f2_unpack(fa_fma2(fa_f2(a0, a1), cmul, negm), a0, a1);
     // one pair in FA_TC_POLY_EVERY takes its exponentials on the FMA pipe: the SFU (16 per clock
     // and SM) is what bounds this loop
     float p0, p1;
@@ -278,6 +286,12 @@ __device__ __forceinline__ void pass2_chunk(const float (&v)[32], fa_u32 (&pk)[1
   }
 }
 
+template <bool REL>
+__device__ __forceinline__ void pass2_chunk(const float (&v)[32], fa_u32 (&pk)[16], fa_u64 cmul, fa_u64 negm,
+                                            fa_u64& sum_a, fa_u64& sum_b) {
+  pass2_part<REL, 0, 16>(v, pk, cmul, negm, sum_a, sum_b);
+}
+
 // State of one softmax warpgroup thread that a kv step reads and updates.
 struct SoftmaxCtx {
   const FaParams& p;
@@ -286,10 +300,10 @@ struct SoftmaxCtx {
   int half;  // decode variant: which 64 kv columns of a tile this thread owns (0 in the forward)
   float sc2;
   volatile int* abort_flag;
-  const short* sched_tile;
   float m_ref, l;
   fa_u32 cnt;
   const unsigned* rowbits;  // this query row of the mask bit matrix, or null
+  fa_u64 m2, d2;            // a score_mod that is linear over kv: multiplier (with the scale) and slope
 };
 
 // One kv step of this warpgroup's tile.  The few tiles that need mask_mod or end beyond the
@@ -299,34 +313,46 @@ struct SoftmaxCtx {
 // copy without and a copy with the block (head dim 128, where the run-time flag made the common,
 // unmasked steps 16 % slower).
 template <int VARIANT>
-__device__ __forceinline__ bool softmax_step(SoftmaxCtx& c, const int j, const int mode, const bool masked_rt) {
+__device__ __forceinline__ bool softmax_step(SoftmaxCtx& c, const int tile, const int mode, const bool masked_rt) {
   const bool masked = VARIANT == 2 ? masked_rt : VARIANT == 1;
   const FaParams& p = c.p;
-  const fa_u32 sb = c.sb, t_s = c.t_s, t_o = c.t_o, t_p = c.t_p;
+  const fa_u32 sb = c.sb, t_o = c.t_o;
   const int i = c.i, qi = c.qi, gb = c.gb, gh = c.gh;
   const float sc2 = c.sc2;
   volatile int* abort_flag = c.abort_flag;
   float& m_ref = c.m_ref;
   float& l = c.l;
   fa_u32& cnt = c.cnt;
-  const short* sched_tile = c.sched_tile;
+  const fa_u32 odd = ROT ? (cnt & 1u) : 0u;
+  const fa_u32 t_s = c.t_s + odd * 64u, t_p = c.t_p + odd * 128u;
   // first key of this thread's columns (decode variant: the thread's 64-column half of the tile)
-  const int n0 = (int)sched_tile[DECODE ? 2 * j + i : j] * BN + (DECODE ? c.half * 64 : 0);
+  const int n0 = tile * BN + (DECODE ? c.half * 64 : 0);
   const fa_u32 t_sh = DECODE ? t_s + c.half * 64 : t_s;
+  constexpr bool REL = FA_HAS_SCORE_MOD;
+  // what the scores are taken relative to (REL): the running maximum, 0 while the row has none
+  const float m_base = m_ref == FA_NEG_INF ? 0.f : m_ref;
+  ModLinear lin = {};
+#if FA_HAS_SCORE_MOD && defined(FA_SCORE_AFFINE) && defined(FA_SCORE_LINEAR_KV)
+  {
+    const float b0 = fa_score_add2(0.f, gb, gh, qi, n0) - m_base;
+    lin = {c.m2, c.d2, fa_f2(b0, b0)};
+  }
+#endif
+  const bool use_mask = FA_HAS_MASK_MOD && mode == 1;
+  const bool have_words = masked && use_mask && c.rowbits != nullptr;
+  uint4 words = make_uint4(0u, 0u, 0u, 0u);
+  if (have_words) words = mask_words<DECODE ? 2 : 4>(c.rowbits, n0);  // (on their way during the wait)
   if (!fa_mbar_wait_warp(bar_addr(sb, BAR_S + i), cnt & 1u, abort_flag)) return false;
   fa_tc_fence_after();
   // ---- pass 1: the whole score row (128 fp32 values) comes into registers, chunk by chunk,
-  // with the score_mod (when there is one), the mask and the row maximum of a chunk computed
-  // while the next chunk is on its way.  Without a score_mod the raw scores are kept and the
-  // scale is folded into the exponent of pass 2.  The S columns are free again as soon as the
+  // with the score_mod (when there is one) and the row maximum of a chunk computed
+  // while the next chunk is on its way.  The S columns are free again as soon as the
   // last load has landed, long before the softmax of the step is done.
   float s0[32], s1[32], s2[32], s3[32];
   RowMax rm = {FA_NEG_INF, FA_NEG_INF, FA_NEG_INF, FA_NEG_INF};
   // (the host routes a non-positive scale, which would turn the maximum around, elsewhere)
-  constexpr bool in_place = FA_HAS_SCORE_MOD || FA_ROUND_SCORES;
-  const bool use_mask = FA_HAS_MASK_MOD && mode == 1;
-#define FA_P1(V, C0)                                                          \
-  if (in_place) mod_chunk<C0>(V, n0, qi, gb, gh, p.scale, sc2);                \
+#define FA_P1(V, C0)                                                                        \
+  if (FA_HAS_SCORE_MOD || FA_ROUND_SCORES) mod_chunk<C0>(V, n0, qi, gb, gh, p.scale, sc2, -m_base, lin); \
   max_chunk(V, rm);
   fa_tmem_ld32(t_sh, s0);
   fa_tmem_wait_ld();
@@ -345,7 +371,7 @@ __device__ __forceinline__ bool softmax_step(SoftmaxCtx& c, const int j, const i
     fa_tmem_ld32(t_s + 96, s3);
     FA_P1(s2, 64)
     fa_tmem_wait_ld();
-    if (SEP_P) {
+    if (EARLY_S) {
       fa_tc_fence_before();
       fa_mbar_arrive(bar_addr(sb, BAR_SFREE2 + i));
     }
@@ -355,7 +381,7 @@ __device__ __forceinline__ bool softmax_step(SoftmaxCtx& c, const int j, const i
   if (masked) {
     // (the row maximum taken on the way is of the unmasked scores: it is taken again)
     fa_u32 keep[DECODE ? 2 : 4];
-    mask_bits(keep, use_mask, n0, qi, gb, gh, p.Skv, c.rowbits);
+    mask_bits(keep, use_mask, n0, qi, gb, gh, p.Skv, have_words, words);
     mask_apply(s0, keep[0]);
     mask_apply(s1, keep[1]);
     rm = {FA_NEG_INF, FA_NEG_INF, FA_NEG_INF, FA_NEG_INF};
@@ -369,24 +395,28 @@ __device__ __forceinline__ bool softmax_step(SoftmaxCtx& c, const int j, const i
     }
   }
   float mx = fmaxf(fmaxf(rm.a, rm.b), fmaxf(rm.c, rm.d));
-  if (!in_place) mx *= sc2;
+  if (!REL) mx *= sc2;
   // running maximum, raised lazily
-  const float m_new = fmaxf(m_ref, mx);
+  const float m_new = fmaxf(m_ref, REL ? m_base + mx : mx);
   bool need = false;
-  float corr = 1.f;
+  float corr = 1.f, delta = 0.f;
   if (m_ref == FA_NEG_INF) {
     m_ref = m_new;  // nothing accumulated yet for this row
+    if (REL && m_new != FA_NEG_INF) delta = m_new;
   } else if (m_new - m_ref > RESCALE_THRESHOLD) {
     need = true;
-    corr = fa_ex2(m_ref - m_new);
+    delta = m_new - m_ref;
+    corr = fa_ex2(-delta);
     m_ref = m_new;
     l *= corr;
   }
   const bool rescale = cnt > 0 && __any_sync(0xffffffffu, need);
   if (cnt > 0 && (SEP_P || rescale)) {
-    // the previous PV product of this tile must be complete: it reads the P columns that
-    // are about to be overwritten (separate P columns), and O is rescaled in place
-    if (!fa_mbar_wait_warp(bar_addr(sb, BAR_O + i), (cnt - 1) & 1u, abort_flag)) return false;
+    // O is rescaled in place, and with separate P columns the previous PV product reads the P columns that are
+    // about to be overwritten: it must be complete
+    const fa_u32 last = cnt - 1;
+    const int bar = ROT ? BAR_O + 2 * (int)(last & 1u) + i : BAR_O + i;
+    if (!fa_mbar_wait_warp(bar_addr(sb, bar), (ROT ? last >> 1 : last) & 1u, abort_flag)) return false;
     fa_tc_fence_after();
   }
   if (rescale) {
@@ -400,26 +430,45 @@ __device__ __forceinline__ bool softmax_step(SoftmaxCtx& c, const int j, const i
       fa_tmem_st16f(t_o + c * 16, o);
     }
   }
-  // ---- pass 2: p = 2^(x * cmul - m) and the row sum; P goes to TMEM as 16-bit pairs (its own
-  // columns with D = 64, over the first 64 score columns otherwise).
+  if (REL && __any_sync(0xffffffffu, delta != 0.f)) {
+    // the maximum has moved (the first step of a row, hardly ever later): the scores follow it
+    const fa_u64 nd = fa_f2(-delta, -delta);
+#pragma unroll
+    for (int e = 0; e < 32; e += 2) {
+      fa_f2_unpack(fa_add2(fa_f2(s0[e], s0[e + 1]), nd), s0[e], s0[e + 1]);
+      fa_f2_unpack(fa_add2(fa_f2(s1[e], s1[e + 1]), nd), s1[e], s1[e + 1]);
+      if (!DECODE) {
+        fa_f2_unpack(fa_add2(fa_f2(s2[e], s2[e + 1]), nd), s2[e], s2[e + 1]);
+        fa_f2_unpack(fa_add2(fa_f2(s3[e], s3[e + 1]), nd), s3[e], s3[e + 1]);
+      }
+    }
+  }
+  // ---- pass 2: p = 2^(x * scale - m) and the row sum; P goes to TMEM as 16-bit pairs.
   // (Packed 16-bit exponentials - ex2.approx.f16x2, one SFU operation per pair - were measured
   // slower: 143 against 131 us, the conversions around them cost more than the SFU time they save.)
   const float m_use = (m_ref == FA_NEG_INF) ? 0.f : m_ref;
   const fa_u64 negm = fa_f2(-m_use, -m_use);
-  const float cm = in_place ? 1.f : sc2;
-  const fa_u64 cmul = fa_f2(cm, cm);
+  const fa_u64 cmul = fa_f2(sc2, sc2);
   fa_u64 sum_a = fa_f2(0.f, 0.f), sum_b = fa_f2(0.f, 0.f);
   {
     fa_u32 pk[16];
     const fa_u32 t_ph = DECODE ? t_p + c.half * 32 : t_p;  // (the other 32 columns of the lane stay zero)
-    pass2_chunk(s0, pk, cmul, negm, sum_a, sum_b);
+    pass2_chunk<REL>(s0, pk, cmul, negm, sum_a, sum_b);
     fa_tmem_st16(t_ph, pk);
-    pass2_chunk(s1, pk, cmul, negm, sum_a, sum_b);
+    pass2_chunk<REL>(s1, pk, cmul, negm, sum_a, sum_b);
     fa_tmem_st16(t_ph + 16, pk);
     if (!DECODE) {
-      pass2_chunk(s2, pk, cmul, negm, sum_a, sum_b);
+      pass2_chunk<REL>(s2, pk, cmul, negm, sum_a, sum_b);
       fa_tmem_st16(t_p + 32, pk);
-      pass2_chunk(s3, pk, cmul, negm, sum_a, sum_b);
+      if (SPLIT_P) {
+        pass2_part<REL, 0, 8>(s3, pk, cmul, negm, sum_a, sum_b);
+        fa_tmem_wait_st();
+        fa_tc_fence_before();
+        fa_mbar_arrive(bar_addr(sb, BAR_P + i));
+        pass2_part<REL, 8, 16>(s3, pk, cmul, negm, sum_a, sum_b);
+      } else {
+        pass2_chunk<REL>(s3, pk, cmul, negm, sum_a, sum_b);
+      }
       fa_tmem_st16(t_p + 48, pk);
     }
   }
@@ -432,7 +481,7 @@ __device__ __forceinline__ bool softmax_step(SoftmaxCtx& c, const int j, const i
   l += sum;
   fa_tmem_wait_st();
   fa_tc_fence_before();
-  fa_mbar_arrive(bar_addr(sb, BAR_P + i));
+  fa_mbar_arrive(bar_addr(sb, (SPLIT_P ? BAR_P2 : BAR_P + 2 * (int)odd) + i));
   ++cnt;
   return true;
 }
@@ -460,17 +509,22 @@ __device__ __forceinline__ void mod32_f32(float (&v)[32], const SoftmaxCtx& c, i
   for (int e = 0; e < 32; ++e) v[e] = fa_score_mod(v[e] * c.p.scale, c.gb, c.gh, c.qi, n0 | (C0 + e)) * FA_LOG2E;
 #endif
 }
-__device__ __forceinline__ bool softmax_step_f32(SoftmaxCtx& c, float (&acc)[D], const int j, const int mode, const bool masked) {
+__device__ __forceinline__ bool softmax_step_f32(SoftmaxCtx& c, float (&acc)[D], const int tile, const int mode, const bool masked) {
   const FaParams& p = c.p;
   const fa_u32 t_s = c.t_s;
-  const int n0 = (int)c.sched_tile[j] * BN;
+  const int n0 = tile * BN;
   if (!fa_mbar_wait_warp(bar_addr(c.sb, BAR_S + c.i), c.cnt & 1u, c.abort_flag)) return false;
   fa_tc_fence_after();
   float a[32], b[32];
   constexpr bool mod = FA_HAS_SCORE_MOD;
   fa_u32 keep[4] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu};
   fa_tmem_ld32(t_s, a);
-  if (masked) mask_bits(keep, FA_HAS_MASK_MOD && mode == 1, n0, c.qi, c.gb, c.gh, p.Skv, c.rowbits);
+  if (masked) {
+    const bool have_words = FA_HAS_MASK_MOD && mode == 1 && c.rowbits != nullptr;
+    uint4 words = make_uint4(0u, 0u, 0u, 0u);
+    if (have_words) words = mask_words<4>(c.rowbits, n0);
+    mask_bits(keep, FA_HAS_MASK_MOD && mode == 1, n0, c.qi, c.gb, c.gh, p.Skv, have_words, words);
+  }
   float mx0 = FA_NEG_INF, mx1 = FA_NEG_INF;
 #define FA_P1(V, N, C)                                                                                  \
   fa_tmem_wait_ld();                                                                                    \
@@ -575,8 +629,7 @@ extern "C" __global__ void __launch_bounds__(fa_tc::NT, fa_tc::NQ == 1 ? 2 : 1) 
   const int gb = b + p.b_off, gh = h + p.h_off;
 
   volatile int* misc = (volatile int*)(sm + OFF_MISC);  // [0] tmem base, [1] abort, [2] nsteps
-  short* sched_tile = (short*)(sm + OFF_SCHED);
-  unsigned char* sched_mode = sm + OFF_MODE;
+  volatile fa_u32* sched = (volatile fa_u32*)(sm + OFF_SCHED);
   unsigned char* cls = sm + OFF_CLS;
 
   // The BlockMask table reads of this CTA go out first: the two counts and, speculatively, this
@@ -611,16 +664,19 @@ extern "C" __global__ void __launch_bounds__(fa_tc::NT, fa_tc::NQ == 1 ? 2 : 1) 
     fa_mbar_init(bar_addr(sb, BAR_Q), 1);
     for (int s = 0; s < NSTAGE; ++s) {
       fa_mbar_init(bar_addr(sb, BAR_KFULL + s), 1);
-      fa_mbar_init(bar_addr(sb, BAR_KEMPTY + s), 1);
+      fa_mbar_init(bar_addr(sb, BAR_KEMPTY + s), ROT ? NQ : 1);
       fa_mbar_init(bar_addr(sb, BAR_VFULL + s), 1);
-      fa_mbar_init(bar_addr(sb, BAR_VEMPTY + s), 1);
+      fa_mbar_init(bar_addr(sb, BAR_VEMPTY + s), ROT ? NQ : 1);
     }
     for (int i = 0; i < 2; ++i) {
       fa_mbar_init(bar_addr(sb, BAR_S + i), 1);
       fa_mbar_init(bar_addr(sb, BAR_P + i), 128);
+      fa_mbar_init(bar_addr(sb, BAR_P + 2 + i), 128);
       fa_mbar_init(bar_addr(sb, BAR_O + i), 1);
+      fa_mbar_init(bar_addr(sb, BAR_O + 2 + i), 1);
       fa_mbar_init(bar_addr(sb, BAR_SFREE2 + i), 128);
     }
+    fa_mbar_init(bar_addr(sb, BAR_LAG), 1);
     fa_mbar_init_fence();
     misc[1] = 0;
     misc[2] = 0;
@@ -695,20 +751,17 @@ extern "C" __global__ void __launch_bounds__(fa_tc::NT, fa_tc::NQ == 1 ? 2 : 1) 
       const int per = (total + (int)gridDim.x - 1) / (int)gridDim.x;
       const int lo = split * per, hi = min(total, lo + per);
       if (listed && pos >= lo && pos < hi) {
-        sched_tile[pos - lo] = (short)tid;
-        sched_mode[pos - lo] = c0;
+        sched[pos - lo] = (fa_u32)tid | ((fa_u32)c0 << 16);
       }
       if (tid == 0) {
         const int k = max(hi - lo, 0);
-        sched_mode[k] = 0;  // an odd share leaves the second warpgroup without a tile in the last step
+        sched[k] = 0;  // an odd share leaves the second warpgroup without a tile in the last step
         misc[2] = (k + 1) / 2;
         misc[3] = k;
       }
 #else
       if (listed) {
-        sched_tile[pos] = (short)tid;
-        sched_mode[2 * pos] = c0;
-        sched_mode[2 * pos + 1] = c1;
+        sched[pos] = (fa_u32)tid | ((fa_u32)c0 << 16) | ((fa_u32)c1 << 24);
       }
       if (tid == 0) {
         misc[2] = total;
@@ -736,7 +789,7 @@ extern "C" __global__ void __launch_bounds__(fa_tc::NT, fa_tc::NQ == 1 ? 2 : 1) 
       for (int j = 0; j < nloads && ok; ++j) {
         const int s = j % NSTAGE;
         const fa_u32 ph = (fa_u32)((j / NSTAGE) & 1);
-        const int n0 = (int)sched_tile[j] * BN;
+        const int n0 = (int)(sched[j] & 0xffffu) * BN;
         if (j >= NSTAGE) ok = fa_mbar_wait(bar_addr(sb, BAR_KEMPTY + s), ph ^ 1u, abort_flag);
         if (!ok) break;
         fa_mbar_expect_tx(bar_addr(sb, BAR_KFULL + s), KV_STAGE);
@@ -765,7 +818,7 @@ extern "C" __global__ void __launch_bounds__(fa_tc::NT, fa_tc::NQ == 1 ? 2 : 1) 
           int s = j % NSTAGE;
           if (!DECODE) ok = fa_mbar_wait(bar_addr(sb, BAR_KFULL + s), (fa_u32)((j / NSTAGE) & 1), abort_flag);
           for (int i = 0; i < NQ && ok; ++i) {
-            if (!sched_mode[2 * j + i]) continue;
+            if (!(sched[2 * j + i] >> 16)) continue;
             if (DECODE) {
               const int t = 2 * j + i;
               s = t % NSTAGE;
@@ -797,7 +850,7 @@ extern "C" __global__ void __launch_bounds__(fa_tc::NT, fa_tc::NQ == 1 ? 2 : 1) 
           int s = j % NSTAGE;
           if (!DECODE) ok = fa_mbar_wait(bar_addr(sb, BAR_VFULL + s), (fa_u32)((j / NSTAGE) & 1), abort_flag);
           for (int i = 0; i < NQ && ok; ++i) {
-            if (!sched_mode[2 * j + i]) continue;
+            if (!(sched[2 * j + i] >> 16)) continue;
             if (DECODE) {
               const int t = 2 * j + i;
               s = t % NSTAGE;
@@ -820,94 +873,189 @@ extern "C" __global__ void __launch_bounds__(fa_tc::NT, fa_tc::NQ == 1 ? 2 : 1) 
         }
       }
     }
-  } else if (!SEP_P && warp == WARP_MMA) {
-    // ============ one MMA issuer for both query tiles (D = 128, fp32) ======================
-    // P overwrites the S columns here, so the products of one tile form a chain  PV_i(j), S_i(j+1),
-    // PV_i(j+1) ...  One warp issues the two chains in turn, PV_0(j) S_0(j+1) PV_1(j) S_1(j+1), so that the
-    // products of a tile run as one block while the other tile is in its softmax.  (With an issuing warp
-    // per tile the tensor core took instructions of both in turn, both tiles got their scores at the
-    // same time, and the products of one never ran under the softmax of the other: clock stamps of a
-    // step showed both waiting for the tensor core and both in the softmax together.)  The whole
-    // warp runs the loop and one elected lane issues: in uniform control flow the operands of tcgen05.mma
+  } else if (ROT && warp >= WARP_MMA && warp < WARP_MMA + NQ) {
+    // ============ head dim 64: an issuing warp per query tile ==============================
+    // S(j+1) lies over the P columns of step j-1, whose product this warp has issued before it.  The whole warp runs the loop and one elected lane issues: in uniform control flow the
+    // operands of tcgen05.mma sit in uniform registers, which makes the instructions cheaper to issue than from a
+    // single-lane branch.  (With one warp for both tiles the issue of one tile's products delayed the other's.)
+    const int i = __shfl_sync(0xffffffffu, warp - WARP_MMA, 0);
+    const bool leader = fa_elect_one();
+    const fa_u32 tmem_u = __shfl_sync(0xffffffffu, tmem, 0);
+    const int nsteps_u = __shfl_sync(0xffffffffu, nsteps, 0);
+    constexpr fa_u32 IDESC_S = fa_idesc(DT, BM, BN, 0, 0);
+    constexpr fa_u32 IDESC_O = fa_idesc(DT, BM, D, 0, 1);
+    constexpr fa_u32 HI = fa_desc_hi_sw128();
+    bool ok = nsteps_u == 0 || fa_mbar_wait_all(bar_addr(sb, BAR_Q), 0, abort_flag);
+    fa_u32 ns = 0, cnt = 0;  // S and PV products issued so far
+    auto word = [&](int j) { return __shfl_sync(0xffffffffu, sched[j], 0); };
+    auto active = [&](fa_u32 w) { return ((w >> (16 + 8 * i)) & 0xffu) != 0u; };
+    auto wait_k = [&](int j) { return fa_mbar_wait_all(bar_addr(sb, BAR_KFULL + j % NSTAGE), (fa_u32)((j / NSTAGE) & 1), abort_flag); };
+    const fa_u32 loQ = fa_desc_lo(sb + i * ATOMS * ATOM_BYTES, 16);
+    // S(j), and K of the step is released (every step's K is waited for before that, with or without a product)
+    auto do_s = [&](int j, fa_u32 wj) {
+      if (active(wj)) {
+        if (ns > 0 && !fa_mbar_wait_all(bar_addr(sb, BAR_SFREE2 + i), (ns - 1) & 1u, abort_flag)) return false;
+        if (NQ == 2 && i == 0 && ns == 1 && leader) fa_mbar_arrive(bar_addr(sb, BAR_LAG));
+        fa_tc_fence_after();
+        const fa_u32 loK = fa_desc_lo(sb + OFF_K + (j % NSTAGE) * KV_STAGE, 16);
+        const fa_u32 t_s = tmem_u + COL_S + i * S_STRIDE + (ns & 1u) * 64u;
+        if (leader) {
+#pragma unroll
+          for (int kk = 0; kk < D / 16; ++kk)
+            fa_mma_ss(t_s, fa_desc_make(loQ + kk * 2, HI), fa_desc_make(loK + kk * 2, HI), IDESC_S, kk > 0);
+          fa_mma_commit(bar_addr(sb, BAR_S + i));
+        }
+        ++ns;
+      }
+      if (leader) fa_mma_commit(bar_addr(sb, BAR_KEMPTY + j % NSTAGE));
+      return true;
+    };
+    fa_u32 w = word(0);
+    if (ok && nsteps_u > 0) {
+      ok = wait_k(0);
+      // The second tile starts when the first has its scores in registers, and the two stay apart like that: in step,
+      // the loads and waits of one do not run under the exponentials of the other (us, in step / apart by the loads /
+      // apart by a whole step: dense B4 H8 S4096 226 / 198 / 208, causal B2 H8 S8192 212 / 198 / 198).
+      if (NQ == 2 && i == 1 && nsteps_u > 1 && ((w >> 16) & 0xffu) != 0u && ((word(1) >> 16) & 0xffu) != 0u && active(w))
+        ok = ok && fa_mbar_wait_all(bar_addr(sb, BAR_LAG), 0, abort_flag);
+      ok = ok && do_s(0, w);
+    }
+    for (int j = 0; j < nsteps_u && ok; ++j) {
+      const bool more = j + 1 < nsteps_u;
+      const fa_u32 w1 = more ? word(j + 1) : 0u;
+      // S(j+1) as soon as the scores of step j are in registers, PV(j) when P is there
+      if (more) ok = wait_k(j + 1) && do_s(j + 1, w1);
+      if (ok) ok = fa_mbar_wait_all(bar_addr(sb, BAR_VFULL + j % NSTAGE), (fa_u32)((j / NSTAGE) & 1), abort_flag);
+      if (!ok) break;
+      if (active(w)) {
+        const fa_u32 loV = fa_desc_lo(sb + OFF_V + (j % NSTAGE) * KV_STAGE, ATOM_BYTES);
+        const fa_u32 t_p = tmem_u + COL_S + i * S_STRIDE + (cnt & 1u) * 128u, t_o = tmem_u + COL_O + i * D;
+        const int odd = 2 * (int)(cnt & 1u) + i;
+        ok = fa_mbar_wait_all(bar_addr(sb, BAR_P + odd), (cnt >> 1) & 1u, abort_flag);
+        if (!ok) break;
+        fa_tc_fence_after();
+        if (leader) {
+#pragma unroll
+          for (int kk = 0; kk < BN / 16; ++kk)
+            fa_mma_ts(t_o, t_p + kk * 8, fa_desc_make(loV + kk * 128, HI), IDESC_O, (cnt > 0) | (kk > 0));
+          fa_mma_commit(bar_addr(sb, BAR_O + odd));
+        }
+        ++cnt;
+      }
+      if (leader) fa_mma_commit(bar_addr(sb, BAR_VEMPTY + j % NSTAGE));
+      w = w1;
+    }
+  } else if (!SEP_P && !ROT && warp == WARP_MMA) {
+    // ============ one MMA issuer for both query tiles ======================================
+    // The whole warp runs the loop and one elected lane issues: in uniform control flow the operands of tcgen05.mma
     // sit in uniform registers, which makes the instructions cheaper to issue than from a single-lane branch.
-    {
-      const bool leader = fa_elect_one();
-      const fa_u32 tmem_u = __shfl_sync(0xffffffffu, tmem, 0);
-      const int nsteps_u = __shfl_sync(0xffffffffu, nsteps, 0);
-      constexpr fa_u32 IDESC_S = fa_idesc(DT, BM, BN, 0, 0);
-      constexpr fa_u32 IDESC_O = fa_idesc(DT, BM, D, 0, 1);
-      bool ok = nsteps_u == 0 || fa_mbar_wait_all(bar_addr(sb, BAR_Q), 0, abort_flag);
-      fa_u32 cnt[2] = {0, 0};  // PV products of each tile issued so far
-      // Descriptors: constant high word; the low word (start address and MN-chunk distance in
-      // 16-byte units) is stepped with one add per k-step.
-      constexpr fa_u32 HI = fa_desc_hi_sw128();
-      // S_i = Q_i K^T for step j
-      auto issue_s = [&](int j, int i) {
-        const int s = j % NSTAGE;
-        const fa_u32 loQ = fa_desc_lo(sb + i * ATOMS * ATOM_BYTES, 16);
-        const fa_u32 loK = fa_desc_lo(sb + OFF_K + s * KV_STAGE, 16);
+    // Everything a product needs besides what the softmax hands over (the K / V tile, the modes of the step) is
+    // waited for before that, so that the products follow the hand-over at once.
+    const bool leader = fa_elect_one();
+    const fa_u32 tmem_u = __shfl_sync(0xffffffffu, tmem, 0);
+    const int nsteps_u = __shfl_sync(0xffffffffu, nsteps, 0);
+    constexpr fa_u32 IDESC_S = fa_idesc(DT, BM, BN, 0, 0);
+    constexpr fa_u32 IDESC_O = fa_idesc(DT, BM, D, 0, 1);
+    bool ok = nsteps_u == 0 || fa_mbar_wait_all(bar_addr(sb, BAR_Q), 0, abort_flag);
+    fa_u32 cnt[2] = {0, 0};  // PV products of each tile issued so far
+    // Descriptors: constant high word; the low word (start address and MN-chunk distance in
+    // 16-byte units) is stepped with one add per k-step.
+    constexpr fa_u32 HI = fa_desc_hi_sw128();
+    auto word = [&](int j) { return __shfl_sync(0xffffffffu, sched[j], 0); };
+    auto active = [&](fa_u32 w, int i) { return ((w >> (16 + 8 * i)) & 0xffu) != 0u; };
+    auto wait_k = [&](int j) { return fa_mbar_wait_all(bar_addr(sb, BAR_KFULL + j % NSTAGE), (fa_u32)((j / NSTAGE) & 1), abort_flag); };
+    auto wait_v = [&](int j) { return fa_mbar_wait_all(bar_addr(sb, BAR_VFULL + j % NSTAGE), (fa_u32)((j / NSTAGE) & 1), abort_flag); };
+    // S_i = Q_i K^T for step j
+    auto issue_s = [&](int j, int i) {
+      const int s = j % NSTAGE;
+      const fa_u32 loQ = fa_desc_lo(sb + i * ATOMS * ATOM_BYTES, 16);
+      const fa_u32 loK = fa_desc_lo(sb + OFF_K + s * KV_STAGE, 16);
+      if (leader) {
 #pragma unroll
         for (int pr = 0; pr < NPROD; ++pr) {
 #pragma unroll
           for (int kk = 0; kk < D / 16; ++kk) {
             const fa_u32 koff = ((kk / 4) * ATOM_BYTES + (kk % 4) * 32) >> 4;
             const fa_u32 pa = (PROD_A[pr] * ATOM_BYTES) >> 4, pb = (PROD_B[pr] * ATOM_BYTES) >> 4;
-            if (leader)
-              fa_mma_ss(tmem_u + COL_S + i * S_STRIDE, fa_desc_make(loQ + pa + koff, HI), fa_desc_make(loK + pb + koff, HI), IDESC_S, pr > 0 || kk > 0);
+            fa_mma_ss(tmem_u + COL_S + i * S_STRIDE, fa_desc_make(loQ + pa + koff, HI), fa_desc_make(loK + pb + koff, HI), IDESC_S, pr > 0 || kk > 0);
           }
         }
-        if (leader) fa_mma_commit(bar_addr(sb, BAR_S + i));
-      };
-      // O_i += P_i V for step j (P_i: 16-bit, from the first column of S_i on; fp32: three parts, and O_i = P_i V)
-      auto issue_pv = [&](int j, int i, bool first) {
-        const int s = j % NSTAGE;
-        const fa_u32 loV = fa_desc_lo(sb + OFF_V + s * KV_STAGE, ATOM_BYTES);
-        const fa_u32 acc = !F32 && !first;
+        fa_mma_commit(bar_addr(sb, BAR_S + i));
+      }
+    };
+    // O_i += P_i V for step j (P_i: 16-bit, from the first column of S_i on; fp32: three parts, and O_i = P_i V)
+    auto issue_pv = [&](int j, int i) {
+      const int s = j % NSTAGE;
+      const fa_u32 loV = fa_desc_lo(sb + OFF_V + s * KV_STAGE, ATOM_BYTES);
+      const fa_u32 acc = !F32 && cnt[i] > 0;
+      const fa_u32 t_p = tmem_u + COL_S + i * S_STRIDE, t_o = tmem_u + COL_O + i * D;
+      constexpr int K1 = SPLIT_P ? 6 : BN / 16;
+      if (leader) {
 #pragma unroll
         for (int pr = 0; pr < NPROD; ++pr) {
 #pragma unroll
-          for (int kk = 0; kk < BN / 16; ++kk)
-            if (leader)
-              fa_mma_ts(tmem_u + COL_O + i * D, tmem_u + COL_S + i * S_STRIDE + (!F32 ? kk * 8 : (PROD_A[pr] == 2 ? 128 + kk * 8 : (kk >> 1) * 32 + PROD_A[pr] * 16 + (kk & 1) * 8)),
-                        fa_desc_make(loV + ((PROD_B[pr] * ATOM_BYTES) >> 4) + kk * 128, HI), IDESC_O, acc | (pr > 0 || kk > 0));
-        }
-        if (leader) fa_mma_commit(bar_addr(sb, BAR_O + i));
-      };
-      if (ok && nsteps_u > 0) {
-        ok = fa_mbar_wait_all(bar_addr(sb, BAR_KFULL + 0), 0, abort_flag);
-        if (ok) {
-          fa_tc_fence_after();
-          for (int i = 0; i < NQ; ++i)
-            if (sched_mode[i]) issue_s(0, i);
-          if (leader) fa_mma_commit(bar_addr(sb, BAR_KEMPTY + 0));
+          for (int kk = 0; kk < K1; ++kk)
+            fa_mma_ts(t_o, t_p + (!F32 ? kk * 8 : (PROD_A[pr] == 2 ? 128 + kk * 8 : (kk >> 1) * 32 + PROD_A[pr] * 16 + (kk & 1) * 8)),
+                      fa_desc_make(loV + ((PROD_B[pr] * ATOM_BYTES) >> 4) + kk * 128, HI), IDESC_O, acc | (pr > 0 || kk > 0));
         }
       }
+      if (SPLIT_P) {
+        if (!fa_mbar_wait_all(bar_addr(sb, BAR_P2 + i), cnt[i] & 1u, abort_flag)) return false;
+        fa_tc_fence_after();
+      }
+      if (leader) {
+#pragma unroll
+        for (int kk = K1; kk < BN / 16; ++kk)
+          fa_mma_ts(t_o, t_p + kk * 8, fa_desc_make(loV + kk * 128, HI), IDESC_O, 1u);
+        fa_mma_commit(bar_addr(sb, BAR_O + i));
+      }
+      ++cnt[i];
+      return true;
+    };
+    fa_u32 w = word(0);
+    if (ok && nsteps_u > 0) {
+      ok = wait_k(0);
+      if (ok) {
+        fa_tc_fence_after();
+        for (int i = 0; i < NQ; ++i)
+          if (active(w, i)) issue_s(0, i);
+        if (leader) fa_mma_commit(bar_addr(sb, BAR_KEMPTY + 0));
+      }
+    }
+    {
+      // P overwrites the S columns here (D = 128, fp32), so the products of one tile form a chain  PV_i(j), S_i(j+1),
+      // PV_i(j+1) ...  One warp issues the two chains in turn, PV_0(j) S_0(j+1) PV_1(j) S_1(j+1), so that the
+      // products of a tile run as one block while the other tile is in its softmax.  (With an issuing warp
+      // per tile the tensor core took instructions of both in turn, both tiles got their scores at the
+      // same time, and the products of one never ran under the softmax of the other: clock stamps of a
+      // step showed both waiting for the tensor core and both in the softmax together.)
       for (int j = 0; j < nsteps_u && ok; ++j) {
-        const int s = j % NSTAGE, s1 = (j + 1) % NSTAGE;
         const bool more = j + 1 < nsteps_u;
-        ok = fa_mbar_wait_all(bar_addr(sb, BAR_VFULL + s), (fa_u32)((j / NSTAGE) & 1), abort_flag);
-#pragma unroll 1
-        for (int i = 0; i < NQ && ok; ++i) {
-          if (sched_mode[2 * j + i]) {
+        const fa_u32 w_next = more ? word(j + 1) : 0u;
+        // (every step waits for its stage to be full before it releases it, with or without a product; with one
+        // stage K of the next step is still on its way and PV goes first)
+        ok = wait_v(j) && (!more || NSTAGE == 1 || wait_k(j + 1));
+#pragma unroll (F32 ? 1 : NQ)
+        for (int i = 0; i < NQ; ++i) {
+          if (!ok) break;
+          if (active(w, i)) {
             ok = fa_mbar_wait_all(bar_addr(sb, BAR_P + i), cnt[i] & 1u, abort_flag);
             if (!ok) break;
             fa_tc_fence_after();
-            issue_pv(j, i, cnt[i] == 0);
-            ++cnt[i];
-          }
-          if (i == NQ - 1 && leader) fa_mma_commit(bar_addr(sb, BAR_VEMPTY + s));
-          if (more) {
-            // (every step waits for its stage to be full before it releases it, with or without a product)
-            ok = fa_mbar_wait_all(bar_addr(sb, BAR_KFULL + s1), (fa_u32)(((j + 1) / NSTAGE) & 1), abort_flag);
+            ok = issue_pv(j, i);
             if (!ok) break;
-            // S of the next step overwrites the columns P was read from: it follows the PV product
-            if (sched_mode[2 * (j + 1) + i]) {
-              fa_tc_fence_after();
-              issue_s(j + 1, i);
-            }
-            if (i == NQ - 1 && leader) fa_mma_commit(bar_addr(sb, BAR_KEMPTY + s1));
           }
+          if (i == NQ - 1 && leader) fa_mma_commit(bar_addr(sb, BAR_VEMPTY + j % NSTAGE));
+          if (NSTAGE == 1 && more && i == 0) {
+            ok = wait_k(j + 1);
+            if (!ok) break;
+            fa_tc_fence_after();
+          }
+          // S of the next step overwrites the columns P was read from: it follows the PV product
+          if (more && active(w_next, i)) issue_s(j + 1, i);
         }
+        if (leader && ok && more) fa_mma_commit(bar_addr(sb, BAR_KEMPTY + (j + 1) % NSTAGE));
+        w = w_next;
       }
     }
   } else if (warp < NSOFT) {
@@ -929,7 +1077,14 @@ extern "C" __global__ void __launch_bounds__(fa_tc::NT, fa_tc::NQ == 1 ? 2 : 1) 
     const unsigned* rowbits = (p.t.mask_bits != nullptr && qi < p.Sq && (p.t.mask_hold == nullptr || *p.t.mask_hold != 0))
         ? p.t.mask_bits + (((long long)(p.t.mask_B == 1 ? 0 : b) * p.t.mask_H + (p.t.mask_H == 1 ? 0 : h)) * p.t.mask_rows + qi) * p.t.mask_stride
         : nullptr;
-    SoftmaxCtx c = {p, sb, t_s, t_o, t_p, i, warp, qi, gb, gh, half, p.scale * FA_LOG2E, abort_flag, sched_tile, FA_NEG_INF, 0.f, 0u, rowbits};
+    SoftmaxCtx c = {p, sb, t_s, t_o, t_p, i, warp, qi, gb, gh, half, p.scale * FA_LOG2E, abort_flag, FA_NEG_INF, 0.f, 0u, rowbits, 0ull, 0ull};
+#if FA_HAS_SCORE_MOD && defined(FA_SCORE_AFFINE) && defined(FA_SCORE_LINEAR_KV)
+    {
+      const float mul = fa_score_mul(0.f, gb, gh, qi, 0) * c.sc2, slope = fa_score_add2_dkv(0.f, gb, gh, qi, 0);
+      c.m2 = fa_f2(mul, mul);
+      c.d2 = fa_f2(slope, slope);
+    }
+#endif
     if (DECODE) {
       // the P columns of the other half of this lane's kv columns are never written again
       fa_u32 z[16];
@@ -944,8 +1099,13 @@ extern "C" __global__ void __launch_bounds__(fa_tc::NT, fa_tc::NQ == 1 ? 2 : 1) 
 #pragma unroll
     for (int e = 0; e < D; ++e) acc[e] = 0.f;
 #endif
+    // (the schedule entry of a step is read during the one before)
+    fa_u32 w_next = sched[DECODE ? i : 0];
     for (int j = 0; j < nsteps && ok; ++j) {
-      const int mode = sched_mode[2 * j + i];
+      const fa_u32 w = w_next;
+      w_next = sched[DECODE ? min(2 * j + 2 + i, MAXT) : j + 1];
+      const int mode = DECODE ? (int)(w >> 16) : (int)((w >> (16 + 8 * i)) & 0xffu);
+      const int tile = (int)(w & 0xffffu);
       if (mode == 0) continue;
       if (!warp_active) {
         // in step with the working warps: S of this step is there, then both arrivals they also make
@@ -962,18 +1122,19 @@ extern "C" __global__ void __launch_bounds__(fa_tc::NT, fa_tc::NQ == 1 ? 2 : 1) 
         ++idle_cnt;
         continue;
       }
-      const bool masked = (FA_HAS_MASK_MOD && mode == 1) || (int)sched_tile[DECODE ? 2 * j + i : j] * BN + BN > p.Skv;
+      const bool masked = (FA_HAS_MASK_MOD && mode == 1) || tile * BN + BN > p.Skv;
 #if FA_DTYPE == FA_DT_F32
-      ok = softmax_step_f32(c, acc, j, mode, masked);
+      ok = softmax_step_f32(c, acc, tile, mode, masked);
       continue;
 #endif
-      if (SEP_P) ok = softmax_step<2>(c, j, mode, masked);
-      else ok = masked ? softmax_step<1>(c, j, mode, true) : softmax_step<0>(c, j, mode, false);
+      if (D == 64) ok = softmax_step<2>(c, tile, mode, masked);
+      else ok = masked ? softmax_step<1>(c, tile, mode, true) : softmax_step<0>(c, tile, mode, false);
     }
     const float m_ref = c.m_ref, l = c.l;
     const fa_u32 cnt = warp_active ? c.cnt : idle_cnt;
     // ---- epilogue: O / l and the logsumexp of this thread's row ---------------------------
-    if (ok && cnt > 0) ok = fa_mbar_wait_warp(bar_addr(sb, BAR_O + i), (cnt - 1) & 1u, abort_flag);
+    if (ok && cnt > 0)
+      ok = fa_mbar_wait_warp(bar_addr(sb, BAR_O + i + (ROT ? 2 * (int)((cnt - 1) & 1u) : 0)), (ROT ? (cnt - 1) >> 1 : cnt - 1) & 1u, abort_flag);
 #if FA_TC_DECODE
     // The four partial results of a query row (two warpgroups x two column halves) are merged
     // inside the CTA: every thread puts its (O, maximum, sum) into shared memory, over the K / V

@@ -53,21 +53,15 @@ __device__ __forceinline__ fa_u64 fa_globaltimer() {
 #ifndef FA_WAIT_LIMIT_NS
 #define FA_WAIT_LIMIT_NS 2000000000ull
 #endif
-#ifndef FA_WAIT_SLEEP_NS
-#define FA_WAIT_SLEEP_NS 40
-#endif
-#ifndef FA_WAIT_ISSUER_SLEEP
-#define FA_WAIT_ISSUER_SLEEP 0
-#endif
 // SLEEP: back off between polls so that waiting warps leave the issue slots of their scheduler
-// to the warps that have work (the MMA issuer polls without sleeping).
+// to the warps that have work.
 template <bool SLEEP>
 __device__ __forceinline__ bool fa_mbar_wait_t(fa_u32 bar, fa_u32 parity, volatile int* abort_flag) {
   if (fa_mbar_try(bar, parity)) return true;
   fa_u64 t0 = 0;
   for (fa_u32 it = 0;; ++it) {
     if (fa_mbar_try(bar, parity)) return true;
-    if (SLEEP) __nanosleep(FA_WAIT_SLEEP_NS);
+    if (SLEEP) __nanosleep(40);
     if ((it & 63u) == 63u) {  // the expensive checks only now and then
       if (*abort_flag != 0) return false;
       const fa_u64 t = fa_globaltimer();
@@ -80,7 +74,7 @@ __device__ __forceinline__ bool fa_mbar_wait_t(fa_u32 bar, fa_u32 parity, volati
   }
 }
 __device__ __forceinline__ bool fa_mbar_wait(fa_u32 bar, fa_u32 parity, volatile int* abort_flag) {
-  return fa_mbar_wait_t<FA_WAIT_ISSUER_SLEEP != 0>(bar, parity, abort_flag);
+  return fa_mbar_wait_t<false>(bar, parity, abort_flag);
 }
 // warp-uniform variant: every lane waits, the warp agrees on the outcome (needed before
 // warp-collective tcgen05 instructions)
@@ -88,13 +82,29 @@ __device__ __forceinline__ bool fa_mbar_wait_warp(fa_u32 bar, fa_u32 parity, vol
   const bool ok = fa_mbar_wait_t<true>(bar, parity, abort_flag);
   return __all_sync(0xffffffffu, ok);
 }
-
-// every lane polls (no back-off) and the warp agrees on the outcome: for a warp whose control
-// flow stays uniform while one elected lane issues the tcgen05.mma instructions (every lane,
-// the elected one included, has then observed the barrier itself)
+// The same for a warp whose control flow stays uniform while one elected lane issues the tcgen05.mma instructions
+// (every lane, the elected one included, has then observed the barrier itself).  The vote is taken on the poll, so that a
+// satisfied wait is one poll (61 clocks), one vote and a branch that the warp takes together; with the poll in a loop
+// that each lane leaves by itself and a vote behind it, it takes 127, and an issuing warp has up to six of them between
+// two products (attention sink B4 H16 S8192 D128: forward 363 -> 360 us, backward 937 -> 935; in the warps that compute,
+// this form made that backward 2 % slower).
 __device__ __forceinline__ bool fa_mbar_wait_all(fa_u32 bar, fa_u32 parity, volatile int* abort_flag) {
-  const bool ok = fa_mbar_wait_t<false>(bar, parity, abort_flag);
-  return __all_sync(0xffffffffu, ok);
+  if (__all_sync(0xffffffffu, fa_mbar_try(bar, parity))) return true;
+  fa_u64 t0 = 0;
+#pragma unroll 1
+  for (fa_u32 it = 0;; ++it) {
+    if (__all_sync(0xffffffffu, fa_mbar_try(bar, parity))) return true;
+    if ((it & 63u) == 63u) {
+      bool stop = *abort_flag != 0;
+      const fa_u64 t = fa_globaltimer();
+      if (t0 == 0) t0 = t;
+      if (!stop && t - t0 > FA_WAIT_LIMIT_NS) {
+        *abort_flag = 1;
+        stop = true;
+      }
+      if (__any_sync(0xffffffffu, stop)) return false;
+    }
+  }
 }
 // true in exactly one lane of a converged warp
 __device__ __forceinline__ bool fa_elect_one() {
