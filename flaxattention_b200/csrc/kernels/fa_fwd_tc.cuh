@@ -190,8 +190,7 @@ __device__ __forceinline__ void mod_chunk(float (&v)[32], int n0, int qi, int gb
 #pragma unroll
   for (int e = 0; e < 32; e += 2) {
     float x0 = v[e], x1 = v[e + 1];
-    const int kv0 = n0 | (C0 + e);
-    const int kv1 = n0 | (C0 + e + 1);
+    [[maybe_unused]] const int kv0 = n0 | (C0 + e), kv1 = n0 | (C0 + e + 1);
 #if FA_ROUND_SCORES
     fa_round2<DT>(x0, x1);
 #endif
@@ -502,9 +501,17 @@ __device__ __forceinline__ void mod32_f32(float (&v)[32], const SoftmaxCtx& c, i
 #if FA_HAS_SCORE_MOD && defined(FA_SCORE_MUL_ONLY)
 #pragma unroll
   for (int e = 0; e < 32; ++e) v[e] *= fa_score_mul(0.f, c.gb, c.gh, c.qi, n0 | (C0 + e)) * c.sc2;
+#elif FA_HAS_SCORE_MOD && defined(FA_SCORE_AFFINE)
+  // (an additive bias is applied before the change to log2 units, as in fa_fwd.cuh: folding the factor into it would round
+  //  a large bias at another place.  The FMA is written out: which product of  score * scale + a * b  is fused is otherwise
+  //  up to the compiler, and the backward has to see the same scores: with ALiBi, S856, gradients were off by 1.0e-5 to 1.3e-5
+  //  instead of 0.8e-5 to 1.1e-5 where the two differed)
+#pragma unroll
+  for (int e = 0; e < 32; ++e) {
+    const int kv = n0 | (C0 + e);
+    v[e] = fmaf(v[e], fa_score_mul(0.f, c.gb, c.gh, c.qi, kv) * c.p.scale, fa_score_add(0.f, c.gb, c.gh, c.qi, kv)) * FA_LOG2E;
+  }
 #elif FA_HAS_SCORE_MOD
-  // (an additive bias is applied before the change to log2 units, as in fa_fwd.cuh: folding the factor into it
-  //  would round a large bias at another place)
 #pragma unroll
   for (int e = 0; e < 32; ++e) v[e] = fa_score_mod(v[e] * c.p.scale, c.gb, c.gh, c.qi, n0 | (C0 + e)) * FA_LOG2E;
 #endif
