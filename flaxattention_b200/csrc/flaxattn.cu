@@ -460,7 +460,7 @@ int pick_bwd(int dtype, int D, int Dv, const FaTables* t, BwdCfg& c) {
 }
 
 struct DecCfg {
-  int BM, BN, smem;
+  int BM, BN, smem, stages;
 };
 int pick_decode(int dtype, int D, int Dv, int Sq, const FaTables* t, DecCfg& c) {
   if (dtype == FA_F32) return fail(FA_EUNSUPPORTED, "the decode kernel takes fp16 / bf16 inputs");
@@ -479,10 +479,19 @@ int pick_decode(int dtype, int D, int Dv, int Sq, const FaTables* t, DecCfg& c) 
     const int mrg = CG * BM * (Dv + 4) * 4;
     const int smem = BM * pitch(D, 2) + (pipe > mrg ? pipe : mrg);
     if (smem > kMaxSmem) continue;
-    c = {BM, BN, smem};
+    c = {BM, BN, smem, 2};
     return FA_OK;
   }
   return fail(FA_EUNSUPPORTED, "no decode tile configuration fits this head dim / BlockMask block size");
+}
+
+// the same with three buffers of K and of V, where two CTAs of up to 16 rows still share an SM then
+bool decode_third_buffer(DecCfg& c, int D, int Dv) {
+  const int smem = c.smem + c.BN * (pitch(D, 2) + pitch(Dv, 2));
+  if (c.BM != 16 || 2 * (smem + 1024) > 228 * 1024) return false;
+  c.smem = smem;
+  c.stages = 3;
+  return true;
 }
 
 std::string defs(std::initializer_list<std::pair<const char*, int>> kv) {
@@ -1117,11 +1126,11 @@ int get_bwd_rerun_kernel(fa_module* m, int dtype, int D, int Dv, const BwdCfg& c
 }
 int get_decode_kernel(fa_module* m, int dtype, int D, int Dv, int flags, const DecCfg& c, bool pack, bool cluster, bool two, Kernel** k) {
   const int rnd = round_flag(dtype, flags);
-  return get_kernel(m, kernel_key(kIdDecode, {{dtype, 2}, {D, 9}, {Dv, 9}, {c.BM, 9}, {c.BN, 9}, {rnd, 1}, {pack ? 1 : 0, 1}, {cluster ? 1 : 0, 1}, {two ? 1 : 0, 1}}),
+  return get_kernel(m, kernel_key(kIdDecode, {{dtype, 2}, {D, 9}, {Dv, 9}, {c.BM, 9}, {c.BN, 9}, {rnd, 1}, {pack ? 1 : 0, 1}, {cluster ? 1 : 0, 1}, {two ? 1 : 0, 1}, {c.stages, 2}}),
                     "fa_decode.cuh",
                     [&] { return defs({{"FA_DTYPE", dtype}, {"FA_D", D}, {"FA_DV", Dv}, {"FA_BM", c.BM}, {"FA_BN", c.BN},
                                        {"FA_ROUND_SCORES", rnd}, {"FA_PACK_HEADS", pack ? 1 : 0}, {"FA_CLUSTER", cluster ? 1 : 0},
-                                       {"FA_TWO_PARTS", two ? 1 : 0}}); },
+                                       {"FA_TWO_PARTS", two ? 1 : 0}, {"FA_STAGES", c.stages}}); },
                     "fa_decode_kernel", c.smem, k);
 }
 // Grouped-query decode: the G query heads of a kv head share one CTA (their G * Sq rows form one
@@ -1562,9 +1571,13 @@ int fa_module_prepare(fa_module* m, int kind, int dtype, int D, int Dv, int Sq_h
       if (dtype != FA_F32 && D == 64 && Dv == 64 && Sq_hint > 16)
         if (int rc = get_fwd_tc_kernel(m, dtype, D, 0, &k, true)) return rc;
       const bool two = c.BM == 16 && Sq_hint > 8 && !(D == 64 && Dv == 64 && Skv_hint >= 1024 && Skv_hint <= 32768);
-      if (c.BM == 16)
-        if (int rc = get_decode_kernel(m, dtype, D, Dv, 0, c, false, true, two, &k)) return rc;
-      return get_decode_kernel(m, dtype, D, Dv, 0, c, false, false, two, &k);
+      for (int pass = 0; pass < 2; ++pass) {  // two buffers, and three where they fit
+        if (c.BM == 16)
+          if (int rc = get_decode_kernel(m, dtype, D, Dv, 0, c, false, true, two, &k)) return rc;
+        if (int rc = get_decode_kernel(m, dtype, D, Dv, 0, c, false, false, two, &k)) return rc;
+        if (!decode_third_buffer(c, D, Dv)) break;
+      }
+      return FA_OK;
     }
     case FA_KIND_BLOCKMASK:
       if (int rc = get_blockmask_kernel(m, false, &k)) return rc;
@@ -1783,7 +1796,7 @@ int fa_decode_num_splits(const fa_attn_params* p, int sm_count) {
   if (!pack && tc_decode_eligible(p)) return tc_splits();
   // general kernel: as many CTAs per SM as its shared memory allows (at most four by registers)
   int per_sm = 2;
-  DecCfg c{16, 0, 0};
+  DecCfg c{16, 0, 0, 2};
   if (pick_decode(p->dtype, p->D, p->Dv, pack ? p->Sq * (p->Hq / p->Hkv) : p->Sq, nullptr, c) == FA_OK) {
     per_sm = decode_ctas_per_sm(c);
   }
@@ -1831,6 +1844,10 @@ int fa_decode(fa_module* m, const fa_attn_params* p, int num_splits, void* works
   // 16 rows of each head 31.2 -> 32.9, 64 rows 26.4 -> 28.9.)
   const bool cluster = !tc && c.BM == 16 && num_splits > 1 && num_splits <= FA_DECODE_MAX_CLUSTER &&
                        (long long)p->B * (pack ? p->Hkv : p->Hq) * num_splits <= (decode_ctas_per_sm(c) > 2 ? places : places * 87 / 100);
+  // Three buffers of K and of V where no SM gets more than two CTAs anyway: two thirds more bytes in flight (us, two / three: B8 H8 Skv2048 D64
+  // 12.0 / 10.7, B16 H32/8 Skv8191 D128 95.2 / 92.5).  With more CTAs the third one that two buffers leave room for is worth more
+  // (B32 H8 Skv16384 D64, 1 row 169 / 173, 16 rows 180 / 185); clusters want the same room to spare as above.
+  if (!tc && (long long)p->B * (pack ? p->Hkv : p->Hq) * num_splits <= (cluster ? places * 87 / 100 : 2LL * device_sm_count())) decode_third_buffer(c, p->D, p->Dv);
   if (need && !cluster) {
     const size_t rows = (size_t)p->B * p->Hq * num_splits * p->Sq;
     kp.part_o = (float*)workspace;

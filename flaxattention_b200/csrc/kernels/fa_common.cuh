@@ -233,23 +233,30 @@ struct FaWalk {
     const long long row = ((long long)bm * t.mH + hm) * t.nKV + kvblk;
     init_rows<T>(t.q_num, t.q_idx, t.full_q_num, t.full_q_idx, row, t.nQ, t.QB, Sq);
   }
-  // slot -> first token of the tile (or -1 when the tile lies beyond S); full = skip mask_mod
+  // the table entry of a block of the walk (0 where there is none)
+  __device__ __forceinline__ int entry(int bi) const {
+    if (idx[0] == nullptr || bi >= num[0] + num[1]) return 0;
+    const int* list = bi >= num[0] ? idx[1] : idx[0];
+    return list != nullptr ? list[bi >= num[0] ? bi - num[0] : bi] : 0;
+  }
+  // block of the walk, tile in it, the block's table entry -> first token of the tile (or -1 when the tile lies beyond S);
+  // full = skip mask_mod.  Without tables every tile is a block.
   template <int T>
-  __device__ __forceinline__ int tile_start(int slot, bool& full) const {
-    if (idx[0] == nullptr) {  // no tables
+  __device__ __forceinline__ int start_of(int bi, int ti, int entry, bool& full) const {
+    if (idx[0] == nullptr) {
       full = false;
-      const long long n0 = (long long)slot * T;
+      const long long n0 = (long long)bi * T;
       return n0 < S ? (int)n0 : -1;
     }
-    int bi = tpb == 1 ? slot : slot / tpb;
-    const int ti = slot - bi * tpb;
-    int which = 0;
-    if (bi >= num[0]) { bi -= num[0]; which = 1; }
-    full = which == 1;
-    int blk = 0;
-    if (idx[which] != nullptr) blk = min(max(idx[which][bi], 0), ncols - 1);
-    const long long n0 = (long long)blk * BS + (long long)ti * T;
+    full = bi >= num[0];
+    const long long n0 = (long long)min(max(entry, 0), ncols - 1) * BS + (long long)ti * T;
     return n0 < S ? (int)n0 : -1;
+  }
+  template <int T>
+  __device__ __forceinline__ int tile_start(int slot, bool& full) const {
+    if (idx[0] == nullptr) return start_of<T>(slot, 0, 0, full);
+    const int bi = tpb == 1 ? slot : slot / tpb;
+    return start_of<T>(bi, slot - bi * tpb, entry(bi), full);
   }
   template <int T>
   __device__ __forceinline__ bool next(int& slot, int& start, bool& full) const {

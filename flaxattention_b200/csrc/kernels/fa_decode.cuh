@@ -21,7 +21,7 @@
 // Compile-time parameters (macros): FA_DTYPE (fp16 / bf16), FA_D, FA_DV, FA_BM (16, 32, 64),
 // FA_BN (kv tile), FA_PACK_HEADS.
 #pragma once
-#include "fa_common.cuh"
+#include "fa_sm100.cuh"
 
 // ---- thread-block clusters: barrier over all threads, reads of another CTA's shared memory ----
 // (not the .aligned forms: the loops in front of the barriers leave the threads of a warp one by one)
@@ -54,6 +54,10 @@ __device__ __forceinline__ float4 fa_ld_cluster_f4(fa_u32 addr) {
 #define FA_CLUSTER 0  // the splits of a tile of rows are launched as a cluster (a variant of its own: with the merge in the kernel of
 #endif                // all calls those without it took up to 7 % more, B16 H16 Skv1024 D64 16 rows 17.4 -> 18.6 us)
 
+#ifndef FA_STAGES
+#define FA_STAGES 2  // buffers of K and of V
+#endif
+
 namespace fa_dec {
 
 constexpr bool PACK = FA_PACK_HEADS != 0;
@@ -63,7 +67,7 @@ constexpr int D = FA_D;
 constexpr int DV = FA_DV;
 constexpr int BM = FA_BM;
 constexpr int BN = FA_BN;
-constexpr int STAGES = 2;
+constexpr int STAGES = FA_STAGES;
 constexpr int NWARPS = 4;
 constexpr int NT = NWARPS * 32;
 constexpr int RG = BM / 16;
@@ -88,13 +92,16 @@ constexpr int SMEM_BYTES = Q_BYTES + (PIPE_BYTES > MRG_BYTES ? PIPE_BYTES : MRG_
 // 2.18e-3 against 2.32e-3), and the second instruction costs time (34.3 us, 31.5 without).
 constexpr bool TWO_PARTS = RG == 1;
 
+// CTAs that share an SM by their shared memory: the registers must not allow fewer (170 at three)
+constexpr int MIN_CTAS = 228 * 1024 / (SMEM_BYTES + 1024) >= 3 ? 3 : (228 * 1024 / (SMEM_BYTES + 1024) >= 2 ? 2 : 1);
+
 static_assert(DT != FA_DT_F32, "the decode kernel takes 16-bit inputs");
 static_assert(BM == 16 || BM == 32 || BM == 64, "BM must be 16, 32 or 64");
 static_assert(WN % 16 == 0, "each warp needs at least 16 kv columns per tile");
 
 }  // namespace fa_dec
 
-extern "C" __global__ void __launch_bounds__(fa_dec::NT) fa_decode_kernel(const __grid_constant__ FaParams p) {
+extern "C" __global__ void __launch_bounds__(fa_dec::NT, fa_dec::MIN_CTAS) fa_decode_kernel(const __grid_constant__ FaParams p) {
   using namespace fa_dec;
   extern __shared__ __align__(128) unsigned char smem[];
   FA_MOD_BUFS_INIT(p);
@@ -132,14 +139,25 @@ extern "C" __global__ void __launch_bounds__(fa_dec::NT) fa_decode_kernel(const 
 
   FaWalk walk;
   walk.init_kv<BN>(p.t, b, h0, 0, p.Skv);
-  // this split's run of tile slots
+  // this split's run of tile slots, gone through block by block (without tables every tile is a block)
   const int per = (walk.total + p.num_splits - 1) / p.num_splits;
-  int slot = min(split * per, walk.total);
-  const int slot_end = min(slot + per, walk.total);
+  const int slot0 = min(split * per, walk.total);
+  int left = min(slot0 + per, walk.total) - slot0;  // slots still to be taken
+  const bool tables = walk.idx[0] != nullptr;
+  int block = !tables || walk.tpb == 1 ? slot0 : slot0 / walk.tpb, tile = tables ? slot0 - block * walk.tpb : 0;  // of the next slot
+  // The table entry of a block is read when the last tile of the one before it is taken, a tile before its loads go out.
+  // (Read when it is needed, it is a trip to L2 in front of every load: causal offset mask, B32 H8 Skv16384 D64, 1 row
+  // 173 -> 168 us, 16 rows 184 -> 178.)
+  int entry = walk.entry(block);
   auto next_tile = [&](int& n0, bool& full) -> bool {
-    while (slot < slot_end) {
-      n0 = walk.tile_start<BN>(slot, full);
-      ++slot;
+    while (left > 0) {
+      n0 = walk.start_of<BN>(block, tile, entry, full);
+      --left;
+      if (!tables || ++tile == walk.tpb) {
+        tile = 0;
+        ++block;
+        entry = walk.entry(block);
+      }
       if (n0 >= 0) return true;
     }
     return false;
@@ -173,38 +191,54 @@ extern "C" __global__ void __launch_bounds__(fa_dec::NT) fa_decode_kernel(const 
   float m_run[2] = {FA_NEG_INF, FA_NEG_INF}, l_run[2] = {0.f, 0.f};
 
   // K and V are released and asked for separately: the K buffer of a tile is free as soon as its scores are
-  // there, so K of the tile after next is under way during this tile's P.V, and V of the next one during its
-  // scores.  One and a half tiles are always in flight from two buffers of each (with both loads issued
-  // together at the top of the loop it was one).
-  int n0_cur = 0, n0_nxt = 0;
-  bool full_cur = false, full_nxt = false;
-  bool have = next_tile(n0_cur, full_cur), have_nxt = false;
-  if (have) load_k(0, n0_cur);
-  fa_cp_commit();
-  if (have) {
-    load_v(0, n0_cur);
-    have_nxt = next_tile(n0_nxt, full_nxt);
+  // there, so K of the tile STAGES further on is under way during this tile's P.V, and V of the one STAGES - 1 further on
+  // during its scores: STAGES - 1/2 tiles are always in flight (with both loads issued together at the top of the loop it
+  // would be STAGES - 1).
+  int n0_at[STAGES];       // this tile and the ones whose K has been asked for
+  bool full_at[STAGES], have[STAGES];
+#pragma unroll
+  for (int t = 0; t < STAGES; ++t) {
+    n0_at[t] = 0;
+    full_at[t] = false;
+    have[t] = (t == 0 || have[t > 0 ? t - 1 : 0]) && next_tile(n0_at[t], full_at[t]);
+    if (have[t]) load_k(t, n0_at[t]);
+    fa_cp_commit();
+    if (t < STAGES - 1) {
+      if (have[t]) load_v(t, n0_at[t]);
+      fa_cp_commit();
+    }
   }
-  fa_cp_commit();
-  if (have_nxt) load_k(1, n0_nxt);
-  fa_cp_commit();
+#if FA_HAS_SCORE_MOD && defined(FA_SCORE_AFFINE) && defined(FA_SCORE_LINEAR_KV)
+  // A bias that is linear over kv (ALiBi) under a multiplier that does not read it: multiplier and slope of this thread's two rows
+  // are taken here, the bias once per tile at the thread's first key, and the other keys add multiples of the slope.
+  fa_u64 lin_m[2], lin_d[2];
+#pragma unroll
+  for (int hh = 0; hh < 2; ++hh) {
+    const int row = rg * 16 + hh * 8 + (lane >> 2);
+    const int g_row = PACK ? row / p.Sq : 0;
+    const int qi = row - g_row * p.Sq, gh = h0 + g_row + p.h_off;
+    const float mul = fa_score_mul(0.f, gb, gh, qi, 0) * (p.scale * FA_LOG2E), slope = fa_score_add2_dkv(0.f, gb, gh, qi, 0);
+    lin_m[hh] = fa_f2(mul, mul);
+    lin_d[hh] = fa_f2(slope, slope);
+  }
+#endif
   fa_u32 qf[D / 16][4];
   bool q_loaded = false;
   int cur = 0;  // buffer of the tile being computed
 
-  while (have) {
-    fa_cp_wait<2>();  // K of this tile (V of it and K of the next one may still be on their way)
+  while (have[0]) {
+    fa_cp_wait<2 * (STAGES - 1)>();  // K of this tile (what was asked for after it may still be on its way)
     if (PRIVATE && q_loaded) __syncwarp();
     else __syncthreads();  // (first iteration: the query tile was loaded by all threads)
-    if (have_nxt) load_v(cur ^ 1, n0_nxt);
+    if (have[STAGES - 1]) load_v(cur == 0 ? STAGES - 1 : cur - 1, n0_at[STAGES - 1]);
     fa_cp_commit();
 
     if (!q_loaded) {
       q_loaded = true;
       fa_load_a_frags<D>(qf, sQ, PQ, rg * 16, lane);
     }
-    const int n0 = n0_cur + cg * WN;
-    const bool full = full_cur;
+    const int n0 = n0_at[0] + cg * WN;
+    const bool full = full_at[0];
     float s[WN / 8][4];
 #pragma unroll
     for (int j = 0; j < WN / 8; ++j) s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
@@ -229,31 +263,48 @@ extern "C" __global__ void __launch_bounds__(fa_dec::NT) fa_decode_kernel(const 
       const int g_row = PACK ? row / p.Sq : 0;
       const int qi = row - g_row * p.Sq;
       const int gh = h0 + g_row + p.h_off;
-      float mx = FA_NEG_INF;
+      const int kv0 = n0 + (lane & 3) * 2;  // first key of this thread
+#if FA_HAS_SCORE_MOD && defined(FA_SCORE_AFFINE) && defined(FA_SCORE_LINEAR_KV)
+      const float bias0 = fa_score_add2(0.f, gb, gh, qi, kv0);
+      const fa_u64 lin_b = fa_f2(bias0, bias0);
+#endif
 #pragma unroll
       for (int j = 0; j < WN / 8; ++j) {
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int kv = n0 + j * 8 + (lane & 3) * 2 + e;
-          float x = s[j][hh * 2 + e];
-#if FA_HAS_SCORE_MOD && defined(FA_SCORE_AFFINE)
-          // affine score_mod: scale and log2(e) folded into one FMA
-          x = fmaf(x, fa_score_mul(0.f, gb, gh, qi, kv) * sc2, fa_score_add2(0.f, gb, gh, qi, kv));
+        const int kv = kv0 + j * 8;
+        float x0 = s[j][hh * 2], x1 = s[j][hh * 2 + 1];
+#if FA_HAS_SCORE_MOD && defined(FA_SCORE_AFFINE) && defined(FA_SCORE_LINEAR_KV)
+        fa_f2_unpack(fa_fma2(fa_f2(x0, x1), lin_m[hh], fa_fma2(fa_f2((float)(j * 8), (float)(j * 8 + 1)), lin_d[hh], lin_b)), x0, x1);
+#elif FA_HAS_SCORE_MOD && defined(FA_SCORE_AFFINE)
+        // affine score_mod: scale and log2(e) folded into one FMA
+        x0 = fmaf(x0, fa_score_mul(0.f, gb, gh, qi, kv) * sc2, fa_score_add2(0.f, gb, gh, qi, kv));
+        x1 = fmaf(x1, fa_score_mul(0.f, gb, gh, qi, kv + 1) * sc2, fa_score_add2(0.f, gb, gh, qi, kv + 1));
 #elif FA_HAS_SCORE_MOD
-          x = fa_score_mod(x * p.scale, gb, gh, qi, kv) * FA_LOG2E;
+        x0 = fa_score_mod(x0 * p.scale, gb, gh, qi, kv) * FA_LOG2E;
+        x1 = fa_score_mod(x1 * p.scale, gb, gh, qi, kv + 1) * FA_LOG2E;
 #else
-          x *= sc2;
+        x0 *= sc2;
+        x1 *= sc2;
 #endif
-          bool keep = true;
+        s[j][hh * 2] = x0;
+        s[j][hh * 2 + 1] = x1;
+      }
+      if (ragged || (FA_HAS_MASK_MOD && !full)) {
+#pragma unroll
+        for (int j = 0; j < WN / 8; ++j) {
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const int kv = kv0 + j * 8 + e;
+            bool keep = kv < p.Skv;
 #if FA_HAS_MASK_MOD
-          if (!full) keep = fa_mask_mod(gb, gh, qi, kv);
+            if (!full) keep = keep && fa_mask_mod(gb, gh, qi, kv);
 #endif
-          if (ragged) keep = keep && (kv < p.Skv);
-          x = keep ? x : FA_NEG_INF;
-          s[j][hh * 2 + e] = x;
-          mx = fmaxf(mx, x);
+            if (!keep) s[j][hh * 2 + e] = FA_NEG_INF;
+          }
         }
       }
+      float mx = FA_NEG_INF;
+#pragma unroll
+      for (int j = 0; j < WN / 8; ++j) mx = fa_max3(mx, s[j][hh * 2], s[j][hh * 2 + 1]);
       mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
       mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
       const float m_new = fmaxf(m_run[hh], mx);
@@ -284,18 +335,21 @@ extern "C" __global__ void __launch_bounds__(fa_dec::NT) fa_decode_kernel(const 
         }
       }
     }
-    fa_cp_wait<2>();  // V of this tile
+    fa_cp_wait<2 * (STAGES - 1)>();  // V of this tile
     if (PRIVATE) __syncwarp();
     else __syncthreads();
-    have = have_nxt;
-    n0_cur = n0_nxt;
-    full_cur = full_nxt;
-    have_nxt = have && next_tile(n0_nxt, full_nxt);
-    if (have_nxt) load_k(cur, n0_nxt);
+#pragma unroll
+    for (int t = 0; t + 1 < STAGES; ++t) {
+      have[t] = have[t + 1];
+      n0_at[t] = n0_at[t + 1];
+      full_at[t] = full_at[t + 1];
+    }
+    have[STAGES - 1] = have[STAGES - 1] && next_tile(n0_at[STAGES - 1], full_at[STAGES - 1]);
+    if (have[STAGES - 1]) load_k(cur, n0_at[STAGES - 1]);
     fa_cp_commit();
     if (TWO_PARTS && FA_TWO_PARTS && R > 8) fa_mma_nn<DT, WN, DV, true>(o, s, sV + cur * V_BYTES + cg * WN * PV, PV, lane);
     else fa_mma_nn<DT, WN, DV>(o, s, sV + cur * V_BYTES + cg * WN * PV, PV, lane);
-    cur ^= 1;
+    cur = cur + 1 == STAGES ? 0 : cur + 1;
   }
 
   fa_grid_release();
