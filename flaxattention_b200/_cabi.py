@@ -17,6 +17,7 @@ HOST_PATH = os.path.join(_HERE, "_host.so")
 FA_F16, FA_BF16, FA_F32 = 0, 1, 2
 FLAG_ROUND_SCORES = 1
 FLAG_GENERAL_KERNELS = 16
+FLAG_KV_TILES_SHIFT = 8  # FA_FLAG_KV_TILES
 KIND_FWD, KIND_BWD, KIND_DECODE, KIND_BLOCKMASK = 0, 1, 2, 3
 
 

@@ -160,6 +160,7 @@ class _Call:
         bm = self.block_mask
         if bm is not None:
             t = p.tables
+            p.flags |= getattr(bm, "_kv_tiles", 0) << _cabi.FLAG_KV_TILES_SHIFT
             if bm.kv_num_blocks.device != q.device:
                 raise ValueError("the BlockMask tables live on a different device than the inputs")
             t.kv_num_blocks, t.kv_indices = _ptr(bm.kv_num_blocks), _ptr(bm.kv_indices)

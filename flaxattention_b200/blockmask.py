@@ -117,6 +117,9 @@ class BlockMask:
     # the same matrix transposed [1 or B, 1 or H, KV_LEN, words], or None
     mask_bits_t: Optional[torch.Tensor] = None
     _bits_at = (None, None)  # (of objects that were saved without it)
+    # about how many 128-key tiles the tables list per 128 query rows, 0 where that is not known: a hint for the choice
+    # of a kernel variant, nothing depends on it
+    _kv_tiles = 0
 
     def __init__(self, kv_num_blocks, kv_indices, full_kv_num_blocks, full_kv_indices, q_num_blocks, q_indices,
                  full_q_num_blocks, full_q_indices, BLOCK_SIZE, mask_mod, mask_bits=None, mask_bits_t=None,
@@ -241,10 +244,12 @@ class BlockMask:
 
     def to(self, device):
         mv = lambda t: None if t is None else t.to(device)  # noqa: E731
-        return BlockMask(mv(self.kv_num_blocks), mv(self.kv_indices), mv(self.full_kv_num_blocks),
-                         mv(self.full_kv_indices), mv(self.q_num_blocks), mv(self.q_indices),
-                         mv(self.full_q_num_blocks), mv(self.full_q_indices), self.BLOCK_SIZE, self.mask_mod,
-                         *self._moved_bits(mv))
+        moved = BlockMask(mv(self.kv_num_blocks), mv(self.kv_indices), mv(self.full_kv_num_blocks),
+                          mv(self.full_kv_indices), mv(self.q_num_blocks), mv(self.q_indices),
+                          mv(self.full_q_num_blocks), mv(self.full_q_indices), self.BLOCK_SIZE, self.mask_mod,
+                          *self._moved_bits(mv))
+        moved._kv_tiles = self._kv_tiles
+        return moved
 
     def _moved_bits(self, fn):
         """(mask_bits, mask_bits_t, sources, snapshot, first entries) of a copy whose tensors went through ``fn``."""
@@ -267,6 +272,7 @@ class BlockMask:
                          cut(self.full_kv_indices), cut(self.q_num_blocks), cut(self.q_indices),
                          cut(self.full_q_num_blocks), cut(self.full_q_indices), self.BLOCK_SIZE, self.mask_mod,
                          *self._moved_bits(cut))
+        part._kv_tiles = self._kv_tiles
         if part.mask_bits is not None:
             part._bits_at = tuple(at if at is None or n == 1 else at + range(n)[sl].start
                                   for at, n, sl in zip(self._bits_at, self.mask_bits.shape[:2], (b_slice, h_slice)))
@@ -487,7 +493,9 @@ def create_block_mask(
         hit = _TABLE_CACHE.get(cache_key)
         if hit is not None:
             _TABLE_CACHE.move_to_end(cache_key)
-            return BlockMask(*hit[:8], (Q_BLOCK_SIZE, KV_BLOCK_SIZE), mask_mod, hit[8], hit[9], _bits_at=bits_at)
+            bm = BlockMask(*hit[:8], (Q_BLOCK_SIZE, KV_BLOCK_SIZE), mask_mod, hit[8], hit[9], _bits_at=bits_at)
+            bm._kv_tiles = ms.kv_tiles(Q_LEN, KV_LEN)
+            return bm
     # a mask that does not read the batch (head) index is evaluated once for all of them
     nb, nh = (B if ms.mask_reads_b else 1), (H if ms.mask_reads_h else 1)
     want_bits = _wants_bits(ms, dev, nb, nh, Q_LEN, KV_LEN, Q_BLOCK_SIZE, KV_BLOCK_SIZE, _mask_bits)
@@ -502,5 +510,7 @@ def create_block_mask(
         _TABLE_CACHE[cache_key] = tables
         while len(_TABLE_CACHE) > _TABLE_CACHE_MAX:
             _TABLE_CACHE.popitem(last=False)
-    return BlockMask(*tables[:8], (Q_BLOCK_SIZE, KV_BLOCK_SIZE), mask_mod, tables[8], tables[9], sources, tables[10],
-                     bits_at)
+    bm = BlockMask(*tables[:8], (Q_BLOCK_SIZE, KV_BLOCK_SIZE), mask_mod, tables[8], tables[9], sources, tables[10],
+                   bits_at)
+    bm._kv_tiles = ms.kv_tiles(Q_LEN, KV_LEN)
+    return bm

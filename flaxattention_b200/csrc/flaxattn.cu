@@ -1350,10 +1350,17 @@ int launch_decode_tc(fa_module* m, const fa_attn_params* p, const FaParams& kp, 
 //   more, D = 64       dense S2048 121 / 115, S2560 107 / 100, S3072 126 / 133, S4096 109 / 118;
 //                      causal S2048 78 / 76, S2560 59 / 57, S3072 77 / 76, S4096 62 / 64
 //   more, D = 128      dense S2048 152 / 152, S3072 160 / 164, S4096 139 / 145; causal 98 / 94, 98 / 98, 80 / 82
-// The dense lengths cross between 2560 and 3072 keys.  A mask that leaves few steps of many keys would rather have one
-// (window of 256: S4096 33.5 / 31.5, S8192 60 / 52, at D = 128 42 / 39, 77 / 66), but the host does not know the steps.
+// The dense lengths cross between 2560 and 3072 keys.  Under a BlockMask that leaves few steps the fixed part weighs more:
+// one where the caller says that it lists up to 16 tiles of keys per query tile (D = 64) or up to 10 (D = 128).  Two against one:
+//   D = 64   B4 H8 S4096 window 256 46 / 41, 1024 72 / 68, attention sink 77 / 73, 12 documents 50 / 43, causal (16.5 tiles) 112 / 112;
+//            B2 H8 S8192 47 / 42, 81 / 74, 90 / 79, 59 / 55, causal (32.5) 193 / 199
+//   D = 128  the same 61 / 54, 91 / 89, 94 / 94, 61 / 49, 135 / 149; 66 / 58, 108 / 102, 114 / 107, 71 / 63, 236 / 269;
+//            B4 H16 S8192 245 / 222, 406 / 417, 437 / 389, 271 / 233; causal B8 H16 S1000 (4.5) 64 / 60, B4 H8 S2560 (10.5) 67 / 67,
+//            B2 H16/4 S3001 (12.5) 87 / 91
 int fwd_tc_query_tiles(const fa_attn_params* p) {
   const long long tiles = (long long)p->B * p->Hq * ((p->Sq + 127) / 128);
+  const int listed = p->tables.kv_num_blocks ? (p->flags >> 8) & 0xffff : 0;
+  if (listed > 0 && listed <= (p->D == 64 ? 16 : 10)) return 1;
   return (p->D == 64 && p->Skv <= 2048) || tiles <= device_sm_count() ? 1 : 2;
 }
 int launch_fwd_tc(fa_module* m, const fa_attn_params* p, const FaParams& kp, void* stream) {

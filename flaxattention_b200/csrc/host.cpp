@@ -68,7 +68,7 @@ PyObject *g_identity = nullptr, *g_noop = nullptr, *g_error = nullptr, *g_check_
 // lock, so that calls with other tensors on the same module from other threads do not come between.
 std::mutex g_buffers_mu;
 
-PyObject *s_mask_mod, *s_block_size, *s_mask_bits, *s_mask_bits_t, *s_bits_mod, *s_bits_sources, *s_bits_snapshot, *s_bits_at;
+PyObject *s_mask_mod, *s_block_size, *s_mask_bits, *s_mask_bits_t, *s_bits_mod, *s_bits_sources, *s_bits_snapshot, *s_bits_at, *s_kv_tiles;
 PyObject* s_tables[8];
 
 // A reference that is dropped at the end of its scope.
@@ -339,6 +339,10 @@ bool read_block_mask(PyObject* bm, PyObject* mask_mod, c10::Device dev, Call& c)
   if (qb <= 0 || kvb <= 0 || qb > INT32_MAX || kvb > INT32_MAX) return false;
   t.q_block_size = (int)qb;
   t.kv_block_size = (int)kvb;
+  Ref listed(PyObject_GetAttr(bm, s_kv_tiles));  // (a hint)
+  if (listed.p == nullptr) PyErr_Clear();
+  const long n_tiles = listed.p != nullptr && PyLong_Check(listed.p) ? PyLong_AsLong(listed.p) : 0;
+  if (n_tiles > 0 && n_tiles <= 65535) c.p.flags |= FA_FLAG_KV_TILES((int)n_tiles);
   // the bit matrices belong to the mask_mod they were built from, and to the contents its captured tensors had then
   Ref bits(PyObject_GetAttr(bm, s_mask_bits));
   if (bits.p == nullptr) return false;
@@ -670,5 +674,6 @@ PyMODINIT_FUNC PyInit__host(void) {
   s_bits_sources = PyUnicode_InternFromString("_bits_sources");
   s_bits_snapshot = PyUnicode_InternFromString("_bits_snapshot");
   s_bits_at = PyUnicode_InternFromString("_bits_at");
+  s_kv_tiles = PyUnicode_InternFromString("_kv_tiles");
   return PyModule_Create(&kModule);
 }

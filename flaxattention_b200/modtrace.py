@@ -1687,6 +1687,8 @@ class ModSet:
         # whether the mask differs between batch entries / heads
         self.mask_reads_b = self.mask is not None and _depends_on(self.mask.root, "b", {})
         self.mask_reads_h = self.mask is not None and _depends_on(self.mask.root, "h", {})
+        self._documents = self.mask is not None and bool(self.buffers) and _same_ids(self.mask.root)
+        self._kv_tiles: Dict[Tuple[int, int], int] = {}
         if self.mask is not None:
             parts.append(to_cuda(self.mask, "fa_mask_mod"))
             over_range = to_cuda_range(self.mask, "fa_mask_range")
@@ -1696,6 +1698,30 @@ class ModSet:
             parts.append("__device__ __forceinline__ bool fa_mask_mod(int, int, int, int) { return true; }\n")
         self.source = "".join(parts)
         self.key = hashlib.sha256(self.source.encode()).hexdigest()
+
+    def kv_tiles(self, Q_LEN: int, KV_LEN: int) -> int:
+        """About how many 128-key tiles the mask leaves of the keys per 128 query rows, 0 where that is not known: from the
+        first, middle and last position of the tiles under up to eight query tiles.  Of masks over captured tensors
+        only document masks are known, to leave few."""
+        if self.mask is None or self.buffers:
+            return 8 if self._documents else 0
+        n = self._kv_tiles.get((Q_LEN, KV_LEN))
+        if n is None:
+            nq, nkv = (Q_LEN + 127) // 128, (KV_LEN + 127) // 128
+            tiles = np.unique(np.linspace(0, nq - 1, min(nq, 8)).round().astype(np.int64))
+            at = np.array([0, 64, 127])
+            q = np.minimum(128 * tiles[:, None] + at, Q_LEN - 1).reshape(-1, 1)
+            kv = np.minimum(128 * np.arange(nkv)[:, None] + at, KV_LEN - 1).reshape(1, -1)
+            try:
+                keep = np.broadcast_to(evaluate(self.mask, None, 0, 0, q, kv), (q.size, kv.size))
+                listed = keep.reshape(len(tiles), 3, nkv, 3).any(axis=(1, 3)).sum(axis=1)
+                n = min(max(int(round(float(listed.mean()))), 1), 65535)
+            except NotImplementedError:
+                n = 0
+            if len(self._kv_tiles) >= 64:
+                self._kv_tiles.clear()
+            self._kv_tiles[(Q_LEN, KV_LEN)] = n
+        return n
 
 
 def _trace_any(fn: Callable, kind: str, bufs: List[object]) -> TracedMod:
@@ -1857,6 +1883,17 @@ class _TensorWatch(TorchDispatchMode):
     def __torch_dispatch__(self, func, types, args=(), kwargs=None):
         self.used = True
         return func(*args, **(kwargs or {}))
+
+
+def _same_ids(e: Expr) -> bool:
+    """Whether a mask keeps only pairs whose query and key read the same value of a captured tensor (document ids)."""
+    if e.op == "and":
+        return any(_same_ids(x) for x in e.args)
+    if e.op != "eq" or any(x.op != "load" for x in e.args):
+        return False
+    x, y = e.args
+    reads = [(_depends_on(z, "q", {}), _depends_on(z, "kv", {})) for z in (x, y)]
+    return x.value == y.value and sorted(reads) == [(False, True), (True, False)]
 
 
 class _Template:
