@@ -122,9 +122,11 @@ constexpr int COL_P = 192 * NQ;
 // One pair of exponentials in FA_TC_POLY_EVERY goes to the FMA pipe (a cubic, see fa_ex2_poly2).
 // Measured (B8 H8 S2048 D64): every fourth pair takes the forward without a score_mod from 0.118 to
 // 0.114 ms, with the checkerboard mod from 0.133 to 0.129 and causal + ALiBi from 0.088 to 0.085;
-// every eighth is about the same, every third and every second are slower again (the issue slots).
+// every eighth is about the same, every third and every second are slower again (the issue slots).  Two query tiles
+// without a score_mod: every fifth, at head dim 128 under a mask only (us, fourth / fifth: D64 B2 H8 S8192 dense 365 / 363, causal
+// 193 / 188; D128 causal B4 H8 S4096 136 / 133, B2 H16/4 S3001 90.9 / 88.8, dense S4096 245 / 248; with ALiBi 154 / 156).
 #ifndef FA_TC_POLY_EVERY
-#define FA_TC_POLY_EVERY 4
+#define FA_TC_POLY_EVERY (FA_TC_NQ == 2 && !FA_HAS_SCORE_MOD && !FA_TC_DECODE && (FA_HAS_MASK_MOD || FA_D == 64) ? 5 : 4)
 #endif
 constexpr int NSOFT = 4 * NQ;           // softmax warps
 constexpr int NT = (NSOFT + 4) * 32;
@@ -971,6 +973,7 @@ extern "C" __global__ void __launch_bounds__(fa_tc::NT, fa_tc::NQ == 1 ? 2 : 1) 
     auto word = [&](int j) { return __shfl_sync(0xffffffffu, sched[j], 0); };
     auto active = [&](fa_u32 w, int i) { return ((w >> (16 + 8 * i)) & 0xffu) != 0u; };
     auto wait_k = [&](int j) { return fa_mbar_wait_all(bar_addr(sb, BAR_KFULL + j % NSTAGE), (fa_u32)((j / NSTAGE) & 1), abort_flag); };
+    auto have_k = [&](int j) { return __all_sync(0xffffffffu, fa_mbar_try(bar_addr(sb, BAR_KFULL + j % NSTAGE), (fa_u32)((j / NSTAGE) & 1))) != 0; };
     auto wait_v = [&](int j) { return fa_mbar_wait_all(bar_addr(sb, BAR_VFULL + j % NSTAGE), (fa_u32)((j / NSTAGE) & 1), abort_flag); };
     // S_i = Q_i K^T for step j
     auto issue_s = [&](int j, int i) {
@@ -1039,9 +1042,10 @@ extern "C" __global__ void __launch_bounds__(fa_tc::NT, fa_tc::NQ == 1 ? 2 : 1) 
       for (int j = 0; j < nsteps_u && ok; ++j) {
         const bool more = j + 1 < nsteps_u;
         const fa_u32 w_next = more ? word(j + 1) : 0u;
-        // (every step waits for its stage to be full before it releases it, with or without a product; with one
-        // stage K of the next step is still on its way and PV goes first)
-        ok = wait_v(j) && (!more || NSTAGE == 1 || wait_k(j + 1));
+        // (every step waits for its stage to be full before it releases it, with or without a product; where K of the
+        // next step is still on its way, PV goes first)
+        ok = wait_v(j);
+        bool k_there = !more || (NSTAGE > 1 && have_k(j + 1));
 #pragma unroll (F32 ? 1 : NQ)
         for (int i = 0; i < NQ; ++i) {
           if (!ok) break;
@@ -1053,9 +1057,10 @@ extern "C" __global__ void __launch_bounds__(fa_tc::NT, fa_tc::NQ == 1 ? 2 : 1) 
             if (!ok) break;
           }
           if (i == NQ - 1 && leader) fa_mma_commit(bar_addr(sb, BAR_VEMPTY + j % NSTAGE));
-          if (NSTAGE == 1 && more && i == 0) {
+          if (!k_there) {
             ok = wait_k(j + 1);
             if (!ok) break;
+            k_there = true;
             fa_tc_fence_after();
           }
           // S of the next step overwrites the columns P was read from: it follows the PV product
