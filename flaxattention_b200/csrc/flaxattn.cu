@@ -461,6 +461,7 @@ int pick_bwd(int dtype, int D, int Dv, const FaTables* t, BwdCfg& c) {
 
 struct DecCfg {
   int BM, BN, smem, stages;
+  bool tma;
 };
 int pick_decode(int dtype, int D, int Dv, int Sq, const FaTables* t, DecCfg& c) {
   if (dtype == FA_F32) return fail(FA_EUNSUPPORTED, "the decode kernel takes fp16 / bf16 inputs");
@@ -479,15 +480,23 @@ int pick_decode(int dtype, int D, int Dv, int Sq, const FaTables* t, DecCfg& c) 
     const int mrg = CG * BM * (Dv + 4) * 4;
     const int smem = BM * pitch(D, 2) + (pipe > mrg ? pipe : mrg);
     if (smem > kMaxSmem) continue;
-    c = {BM, BN, smem, 2};
+    c = {BM, BN, smem, 2, false};
     return FA_OK;
   }
   return fail(FA_EUNSUPPORTED, "no decode tile configuration fits this head dim / BlockMask block size");
 }
 
+// K and V by TMA (fa_decode.cuh): up to 16 rows, head dim 64 or 128
+bool decode_by_tma(DecCfg& c, int dtype, int D, int Dv) {
+  if (dtype == FA_F32 || c.BM != 16 || D != Dv || !(D == 64 || D == 128)) return false;
+  const int pipe = 2 * c.stages * c.BN * D * 2, mrg = 4 * c.BM * (Dv + 4) * 4;
+  c.smem = c.BM * pitch(D, 2) + std::max(pipe, mrg) + (4 * c.stages * 2 + 1) * 8 + 1024;  // fa_dec::SMEM_BYTES
+  c.tma = true;
+  return true;
+}
 // the same with three buffers of K and of V, where two CTAs of up to 16 rows still share an SM then
 bool decode_third_buffer(DecCfg& c, int D, int Dv) {
-  const int smem = c.smem + c.BN * (pitch(D, 2) + pitch(Dv, 2));
+  const int smem = c.smem + (c.tma ? 2 * c.BN * D * 2 + 4 * 2 * 8 : c.BN * (pitch(D, 2) + pitch(Dv, 2)));
   if (c.BM != 16 || 2 * (smem + 1024) > 228 * 1024) return false;
   c.smem = smem;
   c.stages = 3;
@@ -1126,11 +1135,11 @@ int get_bwd_rerun_kernel(fa_module* m, int dtype, int D, int Dv, const BwdCfg& c
 }
 int get_decode_kernel(fa_module* m, int dtype, int D, int Dv, int flags, const DecCfg& c, bool pack, bool cluster, bool two, Kernel** k) {
   const int rnd = round_flag(dtype, flags);
-  return get_kernel(m, kernel_key(kIdDecode, {{dtype, 2}, {D, 9}, {Dv, 9}, {c.BM, 9}, {c.BN, 9}, {rnd, 1}, {pack ? 1 : 0, 1}, {cluster ? 1 : 0, 1}, {two ? 1 : 0, 1}, {c.stages, 2}}),
+  return get_kernel(m, kernel_key(kIdDecode, {{dtype, 2}, {D, 9}, {Dv, 9}, {c.BM, 9}, {c.BN, 9}, {rnd, 1}, {pack ? 1 : 0, 1}, {cluster ? 1 : 0, 1}, {two ? 1 : 0, 1}, {c.stages, 2}, {c.tma ? 1 : 0, 1}}),
                     "fa_decode.cuh",
                     [&] { return defs({{"FA_DTYPE", dtype}, {"FA_D", D}, {"FA_DV", Dv}, {"FA_BM", c.BM}, {"FA_BN", c.BN},
                                        {"FA_ROUND_SCORES", rnd}, {"FA_PACK_HEADS", pack ? 1 : 0}, {"FA_CLUSTER", cluster ? 1 : 0},
-                                       {"FA_TWO_PARTS", two ? 1 : 0}, {"FA_STAGES", c.stages}}); },
+                                       {"FA_TWO_PARTS", two ? 1 : 0}, {"FA_STAGES", c.stages}, {"FA_TMA", c.tma ? 1 : 0}}); },
                     "fa_decode_kernel", c.smem, k);
 }
 // Grouped-query decode: the G query heads of a kv head share one CTA (their G * Sq rows form one
@@ -1150,6 +1159,10 @@ static_assert(sizeof(FaTensorMapHost) == sizeof(CUtensorMap), "tensor map size")
 struct FaTcParamsHost {
   FaParams p;
   FaTensorMapHost tq, tk, tv, to;
+};
+struct FaDecodeParamsHost {
+  FaParams p;
+  FaTensorMapHost tk, tv;
 };
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -1578,11 +1591,13 @@ int fa_module_prepare(fa_module* m, int kind, int dtype, int D, int Dv, int Sq_h
       if (dtype != FA_F32 && D == 64 && Dv == 64 && Sq_hint > 16)
         if (int rc = get_fwd_tc_kernel(m, dtype, D, 0, &k, true)) return rc;
       const bool two = c.BM == 16 && Sq_hint > 8 && !(D == 64 && Dv == 64 && Skv_hint >= 1024 && Skv_hint <= 32768);
-      for (int pass = 0; pass < 2; ++pass) {  // two buffers, and three where they fit
+      // (the first kind, by cp.async, also stands in where tensors have no tensor map; then by TMA, with two buffers and with three)
+      for (int kind = 0; kind < 3; ++kind) {
         if (c.BM == 16)
           if (int rc = get_decode_kernel(m, dtype, D, Dv, 0, c, false, true, two, &k)) return rc;
         if (int rc = get_decode_kernel(m, dtype, D, Dv, 0, c, false, false, two, &k)) return rc;
-        if (!decode_third_buffer(c, D, Dv)) break;
+        if (kind == 0 && decode_by_tma(c, dtype, D, Dv)) continue;
+        if (c.stages == 3 || !decode_third_buffer(c, D, Dv)) break;
       }
       return FA_OK;
     }
@@ -1789,6 +1804,36 @@ static int general_decode_splits(long long bh, int tiles, int per_sm, int sm_cou
   return std::max(FA_DECODE_MAX_CLUSTER, (int)std::min<long long>(c, (sm_count + bh - 1) / bh));
 }
 
+// The same where K and V come by TMA.  us, with two buffers (b2) and three (b3):
+//   * More than 148 tiles of rows are not split: one wave of CTAs with no merge behind it streams at 7 TB/s (16384 keys, D 64, one row: 256
+//     tiles 152 with one split, 160 with five; 320: 190 / 198; 1024 keys, 512: 26 / 28), and so does a grid of several waves with the buffers
+//     that fill them (decode_third).
+//   * Up to 1.15 of them per SM, 4096 keys and more, would leave SMs with one CTA beside SMs with two: two splits (D 64, 160 x 8192 keys 59 -> 55).
+//     With more than 8 rows, whose products weigh more, as long as all splits are resident, from 2048 keys on (160 x 2048 25 -> 23, 192 x 8192
+//     83 -> 72).
+//   * Up to 148: two CTAs per SM, up to FA_DECODE_MAX_CLUSTER of them merged in a cluster.  Beyond that, head dim 128 or more than 8 rows take
+//     as many (D 128, 16 x 16384 keys, 16 rows: 10 splits 43, 18 34; one row 32 / 30), others one CTA per SM.
+static int tma_decode_splits(long long bh, int tiles, int sm_count, int rows, int D) {
+  const int cmax = std::min(std::max(tiles / 4, 1), 64);
+  if (bh > sm_count) {
+    const bool two = rows > 8 ? 2 * bh <= 3LL * sm_count && tiles >= 16 : 100 * bh <= 115LL * sm_count && tiles >= 32;
+    return two ? 2 : 1;
+  }
+  const int c = (int)std::min<long long>(cmax, 2 * sm_count / bh);
+  if (c <= FA_DECODE_MAX_CLUSTER || rows > 8 || D > 64) return std::max(c, 1);
+  return std::max(FA_DECODE_MAX_CLUSTER, (int)std::min<long long>(c, (sm_count + bh - 1) / bh));
+}
+// Three buffers (and two CTAs per SM) instead of two (and three)?  us, two / three: more than 8 rows, 256 CTAs over 8192 keys 89 / 83; few tiles per
+// CTA, 64 heads x 2048 keys in four splits 11.0 / 10.7; few CTAs, D 128, 192 x 16384 keys 241 / 229.  But 256 CTAs with up to 8 rows over longer
+// runs 79 / 83: with more bytes in flight than it takes, memory serves them in a worse order.  Several waves: what fills the last one better
+// (512 x 2048 keys 48 / 44, 640 53 / 58).
+static bool decode_third(long long ctas, int tiles_per_cta, int num_splits, int sm_count, int rows) {
+  if (100 * ctas <= 2 * 87LL * sm_count) return rows > 8 || tiles_per_cta <= 8 || 10 * ctas <= 13LL * sm_count;
+  if (ctas <= 3LL * sm_count || num_splits > 1) return false;
+  const auto fill = [&](long long places) { return (double)ctas / (double)((ctas + places - 1) / places * places); };
+  return fill(2LL * sm_count) > fill(3LL * sm_count) + 0.05;
+}
+
 int fa_decode_packs_heads(const fa_attn_params* p) { return (p && decode_packs_heads(p)) ? 1 : 0; }
 
 int fa_decode_num_splits(const fa_attn_params* p, int sm_count) {
@@ -1803,11 +1848,13 @@ int fa_decode_num_splits(const fa_attn_params* p, int sm_count) {
   if (!pack && tc_decode_eligible(p)) return tc_splits();
   // general kernel: as many CTAs per SM as its shared memory allows (at most four by registers)
   int per_sm = 2;
-  DecCfg c{16, 0, 0, 2};
+  DecCfg c{16, 0, 0, 2, false};
   if (pick_decode(p->dtype, p->D, p->Dv, pack ? p->Sq * (p->Hq / p->Hkv) : p->Sq, nullptr, c) == FA_OK) {
     per_sm = decode_ctas_per_sm(c);
   }
-  const int n = general_decode_splits(bh, tiles, per_sm, sm_count, c.BM / 16);
+  const int rows = pack ? p->Sq * (p->Hq / p->Hkv) : p->Sq;
+  const int n = decode_by_tma(c, p->dtype, p->D, p->Dv) ? tma_decode_splits(bh, tiles, sm_count, rows, p->D)
+                                                        : general_decode_splits(bh, tiles, per_sm, sm_count, c.BM / 16);
   // Callers of fa_decode_static have room for kStaticScratchBytes of partial results.  Where this count needs more, and the one
   // that fills waves (of the tcgen05 kernel where it covers the call) does not, that one is taken: many rows over many heads,
   // whose grids have CTAs enough with either.
@@ -1851,10 +1898,6 @@ int fa_decode(fa_module* m, const fa_attn_params* p, int num_splits, void* works
   // 16 rows of each head 31.2 -> 32.9, 64 rows 26.4 -> 28.9.)
   const bool cluster = !tc && c.BM == 16 && num_splits > 1 && num_splits <= FA_DECODE_MAX_CLUSTER &&
                        (long long)p->B * (pack ? p->Hkv : p->Hq) * num_splits <= (decode_ctas_per_sm(c) > 2 ? places : places * 87 / 100);
-  // Three buffers of K and of V where no SM gets more than two CTAs anyway: two thirds more bytes in flight (us, two / three: B8 H8 Skv2048 D64
-  // 12.0 / 10.7, B16 H32/8 Skv8191 D128 95.2 / 92.5).  With more CTAs the third one that two buffers leave room for is worth more
-  // (B32 H8 Skv16384 D64, 1 row 169 / 173, 16 rows 180 / 185); clusters want the same room to spare as above.
-  if (!tc && (long long)p->B * (pack ? p->Hkv : p->Hq) * num_splits <= (cluster ? places * 87 / 100 : 2LL * device_sm_count())) decode_third_buffer(c, p->D, p->Dv);
   if (need && !cluster) {
     const size_t rows = (size_t)p->B * p->Hq * num_splits * p->Sq;
     kp.part_o = (float*)workspace;
@@ -1867,8 +1910,21 @@ int fa_decode(fa_module* m, const fa_attn_params* p, int num_splits, void* works
     Kernel* k = nullptr;
     // (the second part of P as an instruction of its own: see fa_decode.cuh)
     const bool two = c.BM == 16 && (pack ? p->Sq * (p->Hq / p->Hkv) : p->Sq) > 8 && (pack || !tc_decode_covers(p));
+    FaDecodeParamsHost dp;
+    dp.p = kp;
+    DecCfg t = c;
+    const bool by_tma = decode_by_tma(t, p->dtype, p->D, p->Dv);
+    if (by_tma && make_map(&dp.tk, p->dtype, p->k, p->D, p->Skv, p->Hkv, p->B, c.BN / 4) == FA_OK &&
+        make_map(&dp.tv, p->dtype, p->v, p->Dv, p->Skv, p->Hkv, p->B, c.BN / 4) == FA_OK)
+      c = t;
+    // (cp.async: three buffers where no SM gets more than two CTAs anyway; not for strides that no tensor map takes)
+    const long long ctas = (long long)p->B * (pack ? p->Hkv : p->Hq) * num_splits;
+    const int tiles = (p->Skv + 127) / 128, rows = pack ? p->Sq * (p->Hq / p->Hkv) : p->Sq;
+    if (c.tma ? decode_third(ctas, (tiles + num_splits - 1) / num_splits, num_splits, device_sm_count(), rows)
+              : !by_tma && ctas <= (cluster ? places * 87 / 100 : 2LL * device_sm_count()))
+      decode_third_buffer(c, p->D, p->Dv);
     if (int rc = get_decode_kernel(m, p->dtype, p->D, p->Dv, p->flags, c, pack, cluster, two, &k)) return rc;
-    if (int rc = launch(k, dim3(num_splits, pack ? p->Hkv : p->Hq, p->B), dim3(128), &kp, stream, cluster ? num_splits : 1)) return rc;
+    if (int rc = launch(k, dim3(num_splits, pack ? p->Hkv : p->Hq, p->B), dim3(128), &dp, stream, cluster ? num_splits : 1)) return rc;
   }
   if (num_splits > 1 && !cluster) {
     const long long n_rows = (long long)p->B * p->Hq * p->Sq;
