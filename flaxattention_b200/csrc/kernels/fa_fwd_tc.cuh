@@ -184,11 +184,13 @@ __device__ __forceinline__ void max_chunk(const float (&v)[32], RowMax& mx) {
 // (A * score + B) costs one packed FMA per pair: A and B absorb the scale, log2(e) and the maximum.
 // (Without a score_mod the scores stay raw, the exponent's FMA applies the scale.)
 struct ModLinear {
-  fa_u64 m2, d2, b2;  // multiplier, slope over kv, bias at the first key of the tile (with the maximum)
+  fa_u64 m2, od[4];  // multiplier; 0 and 1, 2 and 3, 4 and 5, 6 and 7 times the slope over kv
+  float d, b;        // slope; bias at the first key of the tile (with the maximum)
 };
 template <int C0>
 __device__ __forceinline__ void mod_chunk(float (&v)[32], int n0, int qi, int gb, int gh, float scale, float sc2, float negm,
                                           const ModLinear& lin) {
+  [[maybe_unused]] float at8 = 0.f;
 #pragma unroll
   for (int e = 0; e < 32; e += 2) {
     float x0 = v[e], x1 = v[e + 1];
@@ -198,10 +200,13 @@ __device__ __forceinline__ void mod_chunk(float (&v)[32], int n0, int qi, int gb
 #endif
 #if FA_HAS_SCORE_MOD && defined(FA_SCORE_AFFINE) && defined(FA_SCORE_LINEAR_KV)
     // The multiplier does not read kv and the bias is linear in it (relative-position biases such as ALiBi): both are
-    // taken once per step, at the first key of the tile, and column c adds c times the slope - two packed FMAs per
-    // pair instead of an integer subtraction, an int-to-float conversion (which shares the SFU with the exponentials)
-    // and a multiplication per element.
-    fa_f2_unpack(fa_fma2(fa_f2(x0, x1), lin.m2, fa_fma2(fa_f2((float)(C0 + e), (float)(C0 + e + 1)), lin.d2, lin.b2)), x0, x1);
+    // taken once per step, at the first key of the tile; every eighth column is reached from there with one FMA and the
+    // columns behind it with an addition, both packed - instead of an integer subtraction, an int-to-float conversion
+    // (which shares the SFU with the exponentials) and a multiplication per element.  (A packed FMA per pair with the column
+    // numbers as constants needs those in registers, two moves per pair: B2 H1 S8192, D64 rounded 103 us against 99, D128 104 against 103,
+    // causal D64 88 against 82.)
+    if (e % 8 == 0) at8 = fmaf((float)(C0 + e), lin.d, lin.b);
+    fa_f2_unpack(fa_fma2(fa_f2(x0, x1), lin.m2, fa_add2(fa_f2(at8, at8), lin.od[(e % 8) / 2])), x0, x1);
 #elif FA_HAS_SCORE_MOD && defined(FA_SCORE_MUL_ONLY)
     fa_f2_unpack(fa_fma2(fa_f2(x0, x1), fa_f2(fa_score_mul(0.f, gb, gh, qi, kv0) * sc2, fa_score_mul(0.f, gb, gh, qi, kv1) * sc2), fa_f2(negm, negm)), x0, x1);
 #elif FA_HAS_SCORE_MOD && defined(FA_SCORE_AFFINE)
@@ -304,7 +309,7 @@ struct SoftmaxCtx {
   float m_ref, l;
   fa_u32 cnt;
   const unsigned* rowbits;  // this query row of the mask bit matrix, or null
-  fa_u64 m2, d2;            // a score_mod that is linear over kv: multiplier (with the scale) and slope
+  ModLinear lin;            // a score_mod that is linear over kv
 };
 
 // One kv step of this warpgroup's tile.  The few tiles that need mask_mod or end beyond the
@@ -334,10 +339,8 @@ __device__ __forceinline__ bool softmax_step(SoftmaxCtx& c, const int tile, cons
   const float m_base = m_ref == FA_NEG_INF ? 0.f : m_ref;
   ModLinear lin = {};
 #if FA_HAS_SCORE_MOD && defined(FA_SCORE_AFFINE) && defined(FA_SCORE_LINEAR_KV)
-  {
-    const float b0 = fa_score_add2(0.f, gb, gh, qi, n0) - m_base;
-    lin = {c.m2, c.d2, fa_f2(b0, b0)};
-  }
+  lin = c.lin;
+  lin.b = fa_score_add2(0.f, gb, gh, qi, n0) - m_base;
 #endif
   const bool use_mask = FA_HAS_MASK_MOD && mode == 1;
   const bool have_words = masked && use_mask && c.rowbits != nullptr;
@@ -1089,12 +1092,13 @@ extern "C" __global__ void __launch_bounds__(fa_tc::NT, fa_tc::NQ == 1 ? 2 : 1) 
     const unsigned* rowbits = (p.t.mask_bits != nullptr && qi < p.Sq && (p.t.mask_hold == nullptr || *p.t.mask_hold != 0))
         ? p.t.mask_bits + (((long long)(p.t.mask_B == 1 ? 0 : b) * p.t.mask_H + (p.t.mask_H == 1 ? 0 : h)) * p.t.mask_rows + qi) * p.t.mask_stride
         : nullptr;
-    SoftmaxCtx c = {p, sb, t_s, t_o, t_p, i, warp, qi, gb, gh, half, p.scale * FA_LOG2E, abort_flag, FA_NEG_INF, 0.f, 0u, rowbits, 0ull, 0ull};
+    SoftmaxCtx c = {p, sb, t_s, t_o, t_p, i, warp, qi, gb, gh, half, p.scale * FA_LOG2E, abort_flag, FA_NEG_INF, 0.f, 0u, rowbits, {}};
 #if FA_HAS_SCORE_MOD && defined(FA_SCORE_AFFINE) && defined(FA_SCORE_LINEAR_KV)
     {
       const float mul = fa_score_mul(0.f, gb, gh, qi, 0) * c.sc2, slope = fa_score_add2_dkv(0.f, gb, gh, qi, 0);
-      c.m2 = fa_f2(mul, mul);
-      c.d2 = fa_f2(slope, slope);
+      c.lin.m2 = fa_f2(mul, mul);
+      c.lin.d = slope;
+      for (int e = 0; e < 4; ++e) c.lin.od[e] = fa_f2(2 * e * slope, (2 * e + 1) * slope);
     }
 #endif
     if (DECODE) {
