@@ -127,11 +127,14 @@ __device__ __forceinline__ void chunk(const float (&s)[W], const float (&dp)[W],
   // hardware has the form; only the exponentials are per element, and the rounding of the raw scores where it is asked for
 #if FA_HAS_SCORE_MOD && defined(FA_SCORE_LINEAR_Q)
   // the multiplier does not read q and the bias is linear in it (relative-position biases such as
-  // ALiBi): both are taken once, at the first column of the chunk, and column e adds e times the slope
+  // ALiBi): both are taken once, at the first column of the chunk; every eighth column is reached from there with one FMA,
+  // the ones behind it by adding multiples of the slope that are kept (column numbers as packed constants would take two
+  // moves per pair).  A derivative of 1 is not multiplied with.
   const float lin_g = fa_score_mul(0.f, gb, gh, q0, kv);
   const fa_u64 lin_g2 = fa_f2(lin_g, lin_g), lin_gs2 = fa_f2(lin_g * sc2, lin_g * sc2);
   const float lin_base = fa_score_add2(0.f, gb, gh, q0, kv), lin_dq = fa_score_add2_dq(0.f, gb, gh, q0, kv);
-  const fa_u64 lin_b2 = fa_f2(lin_base, lin_base), lin_d2 = fa_f2(lin_dq, lin_dq);
+  const fa_u64 lin_od[4] = {fa_f2(0.f, lin_dq), fa_f2(2.f * lin_dq, 3.f * lin_dq), fa_f2(4.f * lin_dq, 5.f * lin_dq), fa_f2(6.f * lin_dq, 7.f * lin_dq)};
+  float at8 = lin_base;
 #endif
 #pragma unroll
   for (int e = 0; e < W; e += 4) {
@@ -148,8 +151,9 @@ __device__ __forceinline__ void chunk(const float (&s)[W], const float (&dp)[W],
 #endif
       const fa_u64 s2 = fa_f2(s0, s1);
 #if FA_HAS_SCORE_MOD && defined(FA_SCORE_LINEAR_Q)
-      const fa_u64 g2 = lin_g2;
-      const fa_u64 b2 = fa_add2(fa_fma2(fa_f2((float)(e + u), (float)(e + u + 1)), lin_d2, lin_b2), nl2);
+      [[maybe_unused]] const fa_u64 g2 = lin_g2;
+      if (e > 0 && (e + u) % 8 == 0) at8 = fmaf((float)(e + u), lin_dq, lin_base);
+      const fa_u64 b2 = fa_add2(fa_add2(fa_f2(at8, at8), nl2), lin_od[((e + u) % 8) / 2]);  // (large ones first: they cancel)
       const fa_u64 x2 = fa_fma2(s2, lin_gs2, b2);
 #elif FA_HAS_SCORE_MOD
       const fa_u64 g2 = fa_f2(fa_score_mul(0.f, gb, gh, qi0, kv), fa_score_mul(0.f, gb, gh, qi1, kv));
@@ -162,7 +166,7 @@ __device__ __forceinline__ void chunk(const float (&s)[W], const float (&dp)[W],
       fa_f2_unpack(x2, x0, x1);
       const float p0 = fa_ex2(x0), p1 = fa_ex2(x1);
       fa_u64 d2 = fa_mul2(fa_f2(p0, p1), fa_add2(fa_f2(dp[e + u], dp[e + u + 1]), nd2));
-#if FA_HAS_SCORE_MOD
+#if FA_HAS_SCORE_MOD && !defined(FA_SCORE_MUL_ONE)
       d2 = fa_mul2(d2, g2);
 #endif
       float d0, d1;

@@ -94,7 +94,8 @@ __device__ __forceinline__ void p_chunk(const float (&s)[16], const float* nlse2
   const float lin_g = fa_score_mul(0.f, gb, gh, q0, kv);
   const fa_u64 lin_g2 = fa_f2(lin_g, lin_g), lin_gs2 = fa_f2(lin_g * sc2, lin_g * sc2);
   const float lin_base = fa_score_add2(0.f, gb, gh, q0, kv), lin_dq = fa_score_add2_dq(0.f, gb, gh, q0, kv);
-  const fa_u64 lin_b2 = fa_f2(lin_base, lin_base), lin_d2 = fa_f2(lin_dq, lin_dq);
+  const fa_u64 lin_od[4] = {fa_f2(0.f, lin_dq), fa_f2(2.f * lin_dq, 3.f * lin_dq), fa_f2(4.f * lin_dq, 5.f * lin_dq), fa_f2(6.f * lin_dq, 7.f * lin_dq)};
+  float at8 = lin_base;
 #endif
 #pragma unroll
   for (int e = 0; e < 16; e += 2) {
@@ -106,8 +107,9 @@ __device__ __forceinline__ void p_chunk(const float (&s)[16], const float* nlse2
 #endif
     const fa_u64 s2 = fa_f2(s0, s1);
 #if FA_HAS_SCORE_MOD && defined(FA_SCORE_LINEAR_Q)
-    const fa_u64 g2 = lin_g2;
-    const fa_u64 x2 = fa_fma2(s2, lin_gs2, fa_add2(fa_fma2(fa_f2((float)e, (float)(e + 1)), lin_d2, lin_b2), nl2));
+    [[maybe_unused]] const fa_u64 g2 = lin_g2;
+    if (e == 8) at8 = fmaf(8.f, lin_dq, lin_base);
+    const fa_u64 x2 = fa_fma2(s2, lin_gs2, fa_add2(fa_add2(fa_f2(at8, at8), nl2), lin_od[(e % 8) / 2]));
 #elif FA_HAS_SCORE_MOD
     const int qi0 = q0 | e, qi1 = q0 | (e + 1);
     const fa_u64 g2 = fa_f2(fa_score_mul(0.f, gb, gh, qi0, kv), fa_score_mul(0.f, gb, gh, qi1, kv));
@@ -126,7 +128,7 @@ __device__ __forceinline__ void p_chunk(const float (&s)[16], const float* nlse2
     }
 #endif
     pp[e / 2] = fa_pack2<DT>(p0, p1);
-#if FA_HAS_SCORE_MOD
+#if FA_HAS_SCORE_MOD && !defined(FA_SCORE_MUL_ONE)
     fa_f2_unpack(fa_mul2(fa_f2(p0, p1), g2), pg[e], pg[e + 1]);
 #if (FA_HAS_MASK_MOD || FA_BWD_CLEAR_BEYOND) && !defined(FA_SCORE_GRAD_FINITE)
     if (masked) {

@@ -1657,6 +1657,8 @@ class ModSet:
             if self.affine is not None:
                 # score_mod(s) == fa_score_mul(...) * s + fa_score_add(...); both ignore `score`
                 parts.append("#define FA_SCORE_AFFINE 1\n")
+                if _is_const(self.affine[0].root, 1):
+                    parts.append("#define FA_SCORE_MUL_ONE 1\n")  # nothing but an additive part
                 if _is_const(self.affine[1].root, 0):
                     parts.append("#define FA_SCORE_MUL_ONLY 1\n")  # no additive part
                 n_ops = sum(1 for t in self.affine for e in _topo(t.root) if e.args)
