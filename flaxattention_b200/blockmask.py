@@ -395,7 +395,16 @@ _TABLE_CACHE: "collections.OrderedDict" = collections.OrderedDict()
 _TABLE_CACHE_MAX = 64
 
 
+_CUDA_DEVICES = {}
+
+
 def _require_cuda(device) -> torch.device:
+    if device is None and torch.cuda.is_initialized():
+        index = torch.cuda.current_device()
+        dev = _CUDA_DEVICES.get(index)
+        if dev is None:
+            dev = _CUDA_DEVICES[index] = torch.device("cuda", index)
+        return dev
     if not torch.cuda.is_available():
         raise RuntimeError("flaxattention_b200 needs a CUDA device (B200, sm_100a); there is no CPU path")
     dev = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)

@@ -601,7 +601,9 @@ void fill_params(fa_module* m, const fa_attn_params* p, FaParams& k) {
 // its full list.  The reference orders a row by a stable descending argsort of the 0/1 block grid
 // (flaxattention/core/blockmask.py:57-64): set columns ascending, then the unset columns ascending.
 // The class grid may have fewer (batch, head) entries than the tables (masks that do not read the batch
-// or the head index are evaluated once).
+// or the head index are evaluated once): a warp works a row out once and writes it to `per` of the entries that share it.  Bound
+// by the writes.  (With a warp per row of every entry the lists were worked out anew for each: 64 entries of 64 x 64 blocks
+// 7.0 -> 5.4 us.)
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
@@ -609,19 +611,25 @@ struct FaTableOut {
   int *num[4], *idx[4];  // partial and full lists of the kv tables, then of the q tables (null: not wanted)
 };
 __global__ void __launch_bounds__(128) fa_tables_kernel(const signed char* __restrict__ cls, int B, int H, int clsB, int clsH, int nQ,
-                                                        int nKV, FaTableOut out) {
+                                                        int nKV, int per, FaTableOut out) {
   grid_wait();
   const long long row = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
-  const long long n_kv_rows = (long long)B * H * nQ, n_rows = n_kv_rows + (long long)B * H * nKV;
+  // distinct rows; entries (copies) of each, this warp's share of them: copy_lo .. copy_hi - 1
+  const long long n_kv_rows = (long long)clsB * clsH * nQ, n_rows = n_kv_rows + (long long)clsB * clsH * nKV;
   if (row >= n_rows) return;
+  const int copies = (clsB == 1 ? B : 1) * (clsH == 1 ? H : 1);
+  const int copy_lo = (int)blockIdx.y * per, copy_hi = min(copy_lo + per, copies);
   const bool transposed = row >= n_kv_rows;
   const int rows_per_bh = transposed ? nKV : nQ, cols = transposed ? nQ : nKV;
-  const long long trow = transposed ? row - n_kv_rows : row;  // row of the table
-  const long long bh = trow / rows_per_bh;
-  const int r = (int)(trow - bh * rows_per_bh);
-  const int b = (int)(bh / H), h = (int)(bh - (long long)b * H);
-  const long long cbh = (long long)(clsB == 1 ? 0 : b) * clsH + (clsH == 1 ? 0 : h);
+  const long long drow = transposed ? row - n_kv_rows : row;
+  const long long cbh = drow / rows_per_bh;
+  const int r = (int)(drow - cbh * rows_per_bh);
+  const int db = (int)(cbh / clsH), dh = (int)(cbh - (long long)db * clsH);
+  // copy k is entry  first + k * apart  of the tables
+  const int first = (clsB == 1 ? 0 : db) * H + (clsH == 1 ? 0 : dh), apart = clsH == 1 ? 1 : H;
+  const long long row0 = ((long long)first + (long long)copy_lo * apart) * rows_per_bh + r, rows_apart = (long long)apart * rows_per_bh;
+  const int n_copies = copy_hi - copy_lo;
   const signed char* g = cls + cbh * (long long)nQ * nKV + (transposed ? (long long)r : (long long)r * nKV);
   const int step = transposed ? nKV : 1;
   int total[2] = {0, 0};
@@ -637,7 +645,6 @@ __global__ void __launch_bounds__(128) fa_tables_kernel(const signed char* __res
     int* num = transposed ? out.num[2 + which] : out.num[which];
     int* idx = transposed ? out.idx[2 + which] : out.idx[which];
     if (num == nullptr) continue;
-    idx += trow * cols;
     int n_set = 0;
     for (int c0 = 0; c0 < cols; c0 += 32) {
       const int c = c0 + lane;
@@ -645,10 +652,16 @@ __global__ void __launch_bounds__(128) fa_tables_kernel(const signed char* __res
       const bool s = in && (int)g[(long long)c * step] == which + 1;
       const unsigned bs = __ballot_sync(0xffffffffu, s);
       const int before = n_set + __popc(bs & lt);  // set columns in front of this one
-      if (in) idx[s ? before : total[which] + c - before] = c;
+      const int at = s ? before : total[which] + c - before;
+      if (in) {
+        int* dst = idx + row0 * cols + at;
+        const long long step_out = rows_apart * cols;
+#pragma unroll 4
+        for (int k = 0; k < n_copies; ++k, dst += step_out) *dst = c;
+      }
       n_set += __popc(bs);
     }
-    if (lane == 0) num[trow] = total[which];
+    for (int k = lane; k < n_copies; k += 32) num[row0 + k * rows_apart] = total[which];
   }
 }
 
@@ -1545,8 +1558,14 @@ int bwd_tc_chunk_heads(const fa_attn_params* p) {
 }
 
 // scan = false: the kernel that takes any block size
+// Groups of 32 keys that a warp of fa_mask_scan_kernel takes: all four of a sub-tile, with four warps, where the mask reads captured
+// tensors (a read per query serves four groups: 8.6 us against 10.5 with eight warps for 12 documents at 4096 x 4096), else two, with
+// eight warps (attention sink 8192 x 8192: 10.1 us against 11.1).
+int mask_scan_groups(const fa_module* m) { return m->mod_source.find("FA_NUM_MOD_BUFS") != std::string::npos ? 4 : 2; }
+
 int get_blockmask_kernel(fa_module* m, bool scan, Kernel** k) {
-  return get_kernel(m, kernel_key(scan ? kIdMaskScan : kIdMaskClassify, {}), "fa_blockmask.cuh", [] { return std::string(); },
+  return get_kernel(m, kernel_key(scan ? kIdMaskScan : kIdMaskClassify, {}), "fa_blockmask.cuh",
+                    [&] { return scan ? "#define FA_SCAN_GROUPS " + std::to_string(mask_scan_groups(m)) + "\n" : std::string(); },
                     scan ? "fa_mask_scan_kernel" : "fa_blockmask_classify_kernel", 0, k);
 }
 
@@ -2048,13 +2067,17 @@ int fa_block_mask_build(fa_module* m, const fa_mask_build* mb, void* stream) {
   mp.Q_LEN = mb->Q_LEN; mp.KV_LEN = mb->KV_LEN;
   mp.b_off = mb->b_offset; mp.h_off = mb->h_offset;
   fill_buffers(m, mp.mod_buf);
-  if (int rc = launch(k, dim3(nKV, nQ, (unsigned)nbh), dim3(words ? 128 : 256), &mp, stream)) return rc;
+  const int threads = words ? 512 / mask_scan_groups(m) : 256;
+  if (int rc = launch(k, dim3(nKV, nQ, (unsigned)nbh), dim3(threads), &mp, stream)) return rc;
   if (!tables) return FA_OK;
   FaTableOut out = {{mb->kv_num_blocks, mb->full_kv_num_blocks, mb->q_num_blocks, mb->full_q_num_blocks},
                     {mb->kv_indices, mb->full_kv_indices, mb->q_indices, mb->full_q_indices}};
-  const long long n_rows = (long long)mb->B * mb->H * ((long long)nQ + (mb->q_num_blocks || mb->full_q_num_blocks ? nKV : 0));
-  return launch_here("fa_tables_kernel", fa_tables_kernel, dim3((unsigned)((n_rows + 3) / 4)), dim3(128), stream, mp.cls, mb->B,
-                     mb->H, mb->distinct_B, mb->distinct_H, nQ, nKV, out);
+  const long long n_rows = nbh * ((long long)nQ + (mb->q_num_blocks || mb->full_q_num_blocks ? nKV : 0));
+  // entries per warp: several, while that leaves sixteen warps per SM
+  const long long copies = (long long)mb->B * mb->H / nbh;
+  const int per = (int)std::min<long long>(copies, std::max<long long>(1, n_rows * copies / (16LL * device_sm_count())));
+  return launch_here("fa_tables_kernel", fa_tables_kernel, dim3((unsigned)((n_rows + 3) / 4), (unsigned)((copies + per - 1) / per)), dim3(128),
+                     stream, mp.cls, mb->B, mb->H, mb->distinct_B, mb->distinct_H, nQ, nKV, per, out);
 }
 
 }  // extern "C"

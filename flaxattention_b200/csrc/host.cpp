@@ -548,8 +548,8 @@ PyObject* build_block_mask(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const auto up = [](int64_t v) { return (v + 3) / 4 * 4; };
     const int64_t idx = up(B * H * nq * nkv), num_q = up(B * H * nq), num_kv = up(B * H * nkv);
     const size_t ws = fa_block_mask_workspace_bytes(mb.distinct_B, mb.distinct_H, mb.Q_LEN, mb.KV_LEN, mb.q_block, mb.kv_block);
-    at::Tensor base = empty({4 * idx + 2 * num_q + 2 * num_kv}, at::kInt, dev);
-    at::Tensor work = empty({(int64_t)std::max<size_t>(ws, 16)}, at::kByte, dev);
+    const int64_t n_tables = 4 * idx + 2 * num_q + 2 * num_kv;
+    at::Tensor base = empty({n_tables + (int64_t)(std::max<size_t>(ws, 16) + 3) / 4}, at::kInt, dev);
     int64_t off = 0;
     int32_t* ptr[8];
     for (int i = 0; i < 8; ++i) {
@@ -561,7 +561,7 @@ PyObject* build_block_mask(PyObject*, PyObject* const* a, Py_ssize_t n) {
     }
     mb.kv_num_blocks = ptr[0]; mb.kv_indices = ptr[1]; mb.full_kv_num_blocks = ptr[2]; mb.full_kv_indices = ptr[3];
     mb.q_num_blocks = ptr[4]; mb.q_indices = ptr[5]; mb.full_q_num_blocks = ptr[6]; mb.full_q_indices = ptr[7];
-    mb.workspace = work.mutable_data_ptr();
+    mb.workspace = (int32_t*)base.mutable_data_ptr() + n_tables;
     mb.workspace_bytes = ws;
     // the matrices come out of the same evaluation where the blocks are whole words, else out of one of their own
     const bool apart = want_bits && ((nq > 1 && mb.q_block % 32) || (nkv > 1 && mb.kv_block % 32));
@@ -570,12 +570,16 @@ PyObject* build_block_mask(PyObject*, PyObject* const* a, Py_ssize_t n) {
     own.q_block = own.kv_block = 128;
     fa_mask_build& with_bits = apart ? own : mb;
     if (want_bits) {
-      out.push_back(empty({mb.distinct_B, mb.distinct_H, mb.Q_LEN, fa_mask_bits_row_words(mb.KV_LEN)}, at::kInt, dev));
+      // (rows of whole 16 bytes: the second matrix begins at such a boundary)
+      const int64_t words = fa_mask_bits_row_words(mb.KV_LEN), words_t = fa_mask_bits_row_words(mb.Q_LEN);
+      const int64_t n = (int64_t)mb.distinct_B * mb.distinct_H * mb.Q_LEN * words, n_t = want_bits > 1 ? (int64_t)mb.distinct_B * mb.distinct_H * mb.KV_LEN * words_t : 0;
+      at::Tensor both = empty({n + n_t}, at::kInt, dev);
+      out.push_back(part(both, 0, {mb.distinct_B, mb.distinct_H, mb.Q_LEN, words}));
       with_bits.bits = (uint32_t*)out[8].mutable_data_ptr();
-    }
-    if (want_bits > 1) {
-      out.push_back(empty({mb.distinct_B, mb.distinct_H, mb.KV_LEN, fa_mask_bits_row_words(mb.Q_LEN)}, at::kInt, dev));
-      with_bits.bits_t = (uint32_t*)out[9].mutable_data_ptr();
+      if (want_bits > 1) {
+        out.push_back(part(both, n, {mb.distinct_B, mb.distinct_H, mb.KV_LEN, words_t}));
+        with_bits.bits_t = (uint32_t*)out[9].mutable_data_ptr();
+      }
     }
     void* stream = (void*)c10::cuda::getCurrentCUDAStream(dev.index()).stream();
     out.resize(10);

@@ -115,3 +115,36 @@ def test_positions_decided_by_range_and_by_evaluation(name, Q, KV, block):
     torch.cuda.synchronize()
     assert np.array_equal(_unpack(bm.mask_bits, KV)[0, 0][:Q], dense)
     assert np.array_equal(_unpack(bm.mask_bits_t, Q)[0, 0][:KV], dense.T)
+
+
+@pytest.mark.parametrize("reads", ["nothing", "batch", "head", "both"])
+def test_entries_that_share_their_rows(reads):
+    """A warp of the table kernel writes one distinct row to several entries, and what is left of them at the end: 13 x 61 entries of
+    5 x 7 blocks, four to a warp (793, 61 and 13 are one more than a multiple).  The mask keeps and drops whole 128 x 128 blocks,
+    with ragged ones at both ends."""
+    import flaxattention_b200 as fa
+
+    B, H, Q, KV = 13, 61, 600, 860
+    n = {"nothing": lambda b, h: 0, "batch": lambda b, h: b, "head": lambda b, h: h, "both": lambda b, h: b + h}[reads]
+    mod = lambda b, h, q, kv: (kv < 128) | ((q + 40 >= kv) & (q < kv + 300 + 7 * n(b, h)))  # noqa: E731
+    bm = fa.create_block_mask(mod, B, H, Q, KV)
+    torch.cuda.synchronize()
+    nQ, nKV = 5, 7
+    q, kv = np.arange(Q)[:, None], np.arange(KV)[None, :]
+    kinds = {}
+    tables = {k: getattr(bm, k).cpu().numpy() for k in TABLE_KEYS}
+    # (the bits of 793 distinct masks are beyond the size that is kept without being asked for)
+    bits = None if reads == "both" else (_unpack(bm.mask_bits, KV), _unpack(bm.mask_bits_t, Q))
+    for b in range(B):
+        for h in range(H):
+            i = int(n(b, h))
+            if i not in kinds:
+                dense = np.broadcast_to(mod(b, h, q, kv), (Q, KV))
+                want = create_block_mask_oracle(lambda _b, _h, q, kv, b=b, h=h: mod(b, h, q, kv), 1, 1, Q, KV)
+                kinds[i] = dense, want
+                if bits is not None:
+                    at = min(b, bits[0].shape[0] - 1), min(h, bits[0].shape[1] - 1)
+                    assert np.array_equal(bits[0][at][:Q], dense) and np.array_equal(bits[1][at][:KV], dense.T)
+            for k in TABLE_KEYS:
+                assert np.array_equal(tables[k][b, h], kinds[i][1][k][0, 0]), (k, b, h)
+    assert tables["kv_indices"].shape[-2:] == (nQ, nKV)
