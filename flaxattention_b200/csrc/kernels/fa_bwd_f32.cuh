@@ -307,19 +307,19 @@ extern "C" __global__ void __launch_bounds__(fa_bf32::NT, 1) fa_bwd_f32_kernel(c
                       IDESC_KK, pr > 0 || kk > 0);
     };
     auto tile_lo = [&](int t) { return fa_desc_lo(sb + OFF_RING + (t % 3) * Q_BYTES, 16); };
-    auto wait_tile = [&](int t) { return fa_mbar_wait_all(bar_addr(sb, BAR_FULL + t % 3), (fa_u32)((t / 3) & 1), abort_flag); };
+    auto wait_tile = [&](int t) { return fa_mbar_wait_each(bar_addr(sb, BAR_FULL + t % 3), (fa_u32)((t / 3) & 1), abort_flag); };
     bool ok = true;
     int gn = 0, kvc = 0;
     for (int itc = 0; ok; ++itc) {
       const int lb = itc & 1;
-      ok = fa_mbar_wait_all(bar_addr(sb, BAR_LISTFULL + lb), (fa_u32)((itc >> 1) & 1), abort_flag);
+      ok = fa_mbar_wait_each(bar_addr(sb, BAR_LISTFULL + lb), (fa_u32)((itc >> 1) & 1), abort_flag);
       if (!ok) break;
       const int np = __shfl_sync(0xffffffffu, item[2 * lb + 1], 0);
       __syncwarp();
       if (leader) fa_mbar_arrive(bar_addr(sb, BAR_LISTFREE + lb));
       if (np < 0) break;
       if (np == 0) continue;
-      ok = fa_mbar_wait_all(bar_addr(sb, BAR_KV), (fa_u32)(kvc & 1), abort_flag);
+      ok = fa_mbar_wait_each(bar_addr(sb, BAR_KV), (fa_u32)(kvc & 1), abort_flag);
       // the scores of an item's first pair (those of the later ones are issued a pair ahead)
       if (ok) ok = wait_tile(2 * gn) && wait_tile(2 * gn + 1);
       if (!ok) break;
@@ -329,8 +329,8 @@ extern "C" __global__ void __launch_bounds__(fa_bf32::NT, 1) fa_bwd_f32_kernel(c
       if (leader) fa_mma_commit(bar_addr(sb, BAR_SFULL));
       for (int n = 0; n < np && ok; ++n, ++gn) {
         const fa_u32 prev = (fa_u32)((gn - 1) & 1);
-        ok = fa_mbar_wait_all(bar_addr(sb, BAR_PREADY), (fa_u32)(gn & 1), abort_flag);
-        if (ok && gn > 0) ok = fa_mbar_wait_all(bar_addr(sb, BAR_DVFREE), prev, abort_flag);
+        ok = fa_mbar_wait_each(bar_addr(sb, BAR_PREADY), (fa_u32)(gn & 1), abort_flag);
+        if (ok && gn > 0) ok = fa_mbar_wait_each(bar_addr(sb, BAR_DVFREE), prev, abort_flag);
         if (!ok) break;
         fa_tc_fence_after();
         const fa_u32 loDO = tile_lo(2 * gn), loQ = tile_lo(2 * gn + 1);
@@ -359,7 +359,7 @@ extern "C" __global__ void __launch_bounds__(fa_bf32::NT, 1) fa_bwd_f32_kernel(c
           if (leader) fa_mma_commit(bar_addr(sb, BAR_SFULL));
         }
         // 4. dK = dS^T Q
-        if (gn > 0) ok = fa_mbar_wait_all(bar_addr(sb, BAR_DKFREE), prev, abort_flag);
+        if (gn > 0) ok = fa_mbar_wait_each(bar_addr(sb, BAR_DKFREE), prev, abort_flag);
         if (!ok) break;
         fa_tc_fence_after();
 #pragma unroll
@@ -374,7 +374,7 @@ extern "C" __global__ void __launch_bounds__(fa_bf32::NT, 1) fa_bwd_f32_kernel(c
           fa_mma_commit(bar_addr(sb, BAR_DKFULL));
         }
         // 5. dQ = dS K: [hi; mid] with the parts of K, lo first, and [mid; lo] with hi of K
-        if (gn > 0) ok = fa_mbar_wait_all(bar_addr(sb, BAR_DQFREE), prev, abort_flag);
+        if (gn > 0) ok = fa_mbar_wait_each(bar_addr(sb, BAR_DQFREE), prev, abort_flag);
         if (!ok) break;
         fa_tc_fence_after();
 #pragma unroll
