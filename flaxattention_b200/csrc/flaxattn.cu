@@ -1383,10 +1383,15 @@ int launch_decode_tc(fa_module* m, const fa_attn_params* p, const FaParams& kp, 
 //   D = 128  the same 61 / 54, 91 / 89, 94 / 94, 61 / 49, 135 / 149; 66 / 58, 108 / 102, 114 / 107, 71 / 63, 236 / 269;
 //            B4 H16 S8192 245 / 222, 406 / 417, 437 / 389, 271 / 233; causal B8 H16 S1000 (4.5) 64 / 60, B4 H8 S2560 (10.5) 67 / 67,
 //            B2 H16/4 S3001 (12.5) 87 / 91
+// At D = 64 also one where the tables list half of the key tiles or fewer, so that query tiles differ (causal), and there are up to four
+// tiles per SM: a long and a short one share an SM, where two neighbours in one CTA are both long.  Two against one: causal B2 H4 S4828
+// 69 / 54, B1 H4 S8192 101 / 83, H8 S6144 84 / 71, B2 H8 S4096 (512 tiles) 59.5 / 60, B1 H8 S8192 110 / 106, with ALiBi 124 / 89 at
+// B1 H4 S8192.  (Not at D = 128, causal: 63 / 62, 118 / 134; nor where all tiles are alike, dense B1 H4 S8192: 97 / 112.)
 int fwd_tc_query_tiles(const fa_attn_params* p) {
   const long long tiles = (long long)p->B * p->Hq * ((p->Sq + 127) / 128);
   const int listed = p->tables.kv_num_blocks ? (p->flags >> 8) & 0xffff : 0;
   if (listed > 0 && listed <= (p->D == 64 ? 16 : 10)) return 1;
+  if (listed > 0 && p->D == 64 && 2 * listed <= (p->Skv + 127) / 128 + 2 && tiles <= 4LL * device_sm_count()) return 1;
   return (p->D == 64 && p->Skv <= 2048) || tiles <= device_sm_count() ? 1 : 2;
 }
 int launch_fwd_tc(fa_module* m, const fa_attn_params* p, const FaParams& kp, void* stream) {
