@@ -122,11 +122,12 @@ constexpr int COL_P = 192 * NQ;
 // One pair of exponentials in FA_TC_POLY_EVERY goes to the FMA pipe (a cubic, see fa_ex2_poly2).
 // Measured (B8 H8 S2048 D64): every fourth pair takes the forward without a score_mod from 0.118 to
 // 0.114 ms, with the checkerboard mod from 0.133 to 0.129 and causal + ALiBi from 0.088 to 0.085;
-// every eighth is about the same, every third and every second are slower again (the issue slots).  Two query tiles
-// without a score_mod: every fifth, at head dim 128 under a mask only (us, fourth / fifth: D64 B2 H8 S8192 dense 365 / 363, causal
-// 193 / 188; D128 causal B4 H8 S4096 136 / 133, B2 H16/4 S3001 90.9 / 88.8, dense S4096 245 / 248; with ALiBi 154 / 156).
+// every eighth is about the same, every third and every second are slower again (the issue slots).
+// The same for one and for two query tiles per CTA: which of the two a call gets depends on its batch size and on a hint,
+// and its results must not.  (Every fifth with two tiles and no score_mod takes D64 B2 H8 S8192 causal from 193 to 188 us, D128 B2 H16/4
+// S3001 from 90.9 to 88.8, but then the rows of a shard differ from those of the whole.)
 #ifndef FA_TC_POLY_EVERY
-#define FA_TC_POLY_EVERY (FA_TC_NQ == 2 && !FA_HAS_SCORE_MOD && !FA_TC_DECODE && (FA_HAS_MASK_MOD || FA_D == 64) ? 5 : 4)
+#define FA_TC_POLY_EVERY 4
 #endif
 constexpr int NSOFT = 4 * NQ;           // softmax warps
 constexpr int NT = (NSOFT + 4) * 32;

@@ -38,3 +38,26 @@ def test_forward_on_both_sides_of_the_line(B, H, Sq, Skv, D, dt, mask):
     ref = torch.where(seen[..., None], torch.exp(s - ref_lse.masked_fill(~seen, 0.0)[..., None]) @ v.float(), 0.0)
     assert max_abs(out, ref) <= 2e-2
     assert torch.equal(seen, torch.isfinite(lse)) and max_abs(lse[seen], ref_lse[seen]) <= 2e-2
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("mask", ["causal", "window"])
+@pytest.mark.parametrize("mod", [None, "alibi"])
+def test_results_do_not_depend_on_the_form(D, mask, mod):
+    """256 tiles take two per CTA where no hint says otherwise, the 128 of one batch entry take one, and the hint decides for
+    either: the same bits every time."""
+    import flaxattention_b200 as fa
+    from flaxattention_b200.masks import causal_mask, generate_sliding_window
+    from flaxattention_b200.mods import generate_alibi_bias
+
+    B, H, S = 2, 4, 4096
+    g = torch.Generator(device="cuda").manual_seed(6)
+    q, k, v = (torch.randn(B, H, S, D, generator=g, device="cuda").bfloat16() for _ in range(3))
+    bm = fa.create_block_mask(causal_mask if mask == "causal" else generate_sliding_window(300), None, None, S, S)
+    score = None if mod is None else generate_alibi_bias(H)
+    results = []
+    for hint, n in ((0, B), (0, 1), (1, B), (65535, B)):
+        bm._kv_tiles = hint
+        results.append(fa.flax_attention_pallas(q[:n], k[:n], v[:n], score_mod=score, block_mask=bm, return_lse=True))
+    for out, lse in results[1:]:
+        assert torch.equal(out, results[0][0][:len(out)]) and torch.equal(lse, results[0][1][:len(lse)])
