@@ -29,3 +29,13 @@ def test_captured_tensors():
     assert n(lambda b, h, q, kv: (q >= kv) | (ids[q] == ids[kv])) == 0
     assert n(lambda b, h, q, kv: kv < ids[b]) == 0
     assert modtrace.lower_mods(None, None).kv_tiles(256, 256) == 0
+
+
+def test_a_failure_is_no_failure_of_the_call(monkeypatch):
+    ms = modtrace.lower_mods(None, generate_sliding_window(77))
+
+    def fail(*_):
+        raise MemoryError("no room")
+
+    monkeypatch.setattr(modtrace.np, "linspace", fail)
+    assert ms.kv_tiles(1024, 1024) == 0
