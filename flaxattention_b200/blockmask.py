@@ -117,8 +117,8 @@ class BlockMask:
     # the same matrix transposed [1 or B, 1 or H, KV_LEN, words], or None
     mask_bits_t: Optional[torch.Tensor] = None
     _bits_at = (None, None)  # (of objects that were saved without it)
-    # about how many 128-key tiles the tables list per 128 query rows, 0 where that is not known: a hint for the choice
-    # of a kernel variant, nothing depends on it
+    # a guess at how many 128-key tiles the tables list per 128 query rows, 0 where there is none: a hint for the choice
+    # of a kernel variant, no result depends on it
     _kv_tiles = 0
 
     def __init__(self, kv_num_blocks, kv_indices, full_kv_num_blocks, full_kv_indices, q_num_blocks, q_indices,

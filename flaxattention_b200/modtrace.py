@@ -1386,29 +1386,101 @@ def to_cuda(mod: TracedMod, name: str) -> str:
     return "\n".join([head] + lines + [f"  return {ret};", "}"]) + "\n"
 
 
-def to_cuda_range(mod: TracedMod, name: str) -> Optional[str]:
-    """Device function text of what a mask is over a rectangle of positions, by interval arithmetic on its graph:
-    ``int name(int b, int h, int q0, int q1, int kv0, int kv1)`` (bounds inclusive) gives 0 where it is false for every
-    position, 2 where it is true for every one, 1 where the intervals do not tell.  None if they never would.
+class _RangeText:
+    """What ``_range_walk`` builds from: C++ text, a line for each pair of bounds."""
+
+    true, false = "true", "false"
+
+    def __init__(self):
+        self.lines: List[str] = []
+
+    def keep(self, pair, ctype):
+        i = len(self.lines)
+        a, b = f"a{i}", f"z{i}"
+        self.lines.append(f"  const {ctype} {a} = {pair[0]}, {b} = {pair[1]};")
+        return a, b
+
+    def index(self, name):
+        return (name + "0", name + "1") if name in ("q", "kv") else (name, name)
+
+    def const(self, v):
+        return f"({v})" if v != -(1 << 31) else "(-2147483647 - 1)"
+
+    def op(self, sign, u, v):
+        return f"{u} {sign} {v}"
+
+    def neg(self, u):
+        return f"-{u}"
+
+    def min(self, u, v):
+        return f"min({u}, {v})"
+
+    def max(self, u, v):
+        return f"max({u}, {v})"
+
+    def floordiv(self, u, c):
+        return f"fa_floordiv_i32({u}, {c})"
+
+    def pymod(self, u, c):
+        return f"fa_pymod_i32({u}, {c})"
+
+    def where(self, c, u, v):
+        return f"{c} ? {u} : {v}"
+
+    def all(self, *x):
+        return " && ".join(x)
+
+    def any(self, *x):
+        return " || ".join(x)
+
+    def par(self, u):
+        return f"({u})"
+
+
+class _RangeNumpy:
+    """The same on arrays of rectangles (bounds in int64: nothing that is kept leaves int32)."""
+
+    true, false = np.bool_(True), np.bool_(False)
+    _OPS = {"+": np.add, "-": np.subtract, "*": np.multiply, ">>": np.right_shift, "<": np.less, "<=": np.less_equal,
+            ">": np.greater, ">=": np.greater_equal, "==": np.equal}
+    neg, min, max, const = staticmethod(np.negative), staticmethod(np.minimum), staticmethod(np.maximum), staticmethod(np.int64)
+    floordiv, pymod, where = staticmethod(np.floor_divide), staticmethod(np.remainder), staticmethod(np.where)
+
+    def __init__(self, q, kv):
+        self._index = {"q": q, "kv": kv}
+
+    def keep(self, pair, ctype):
+        return pair
+
+    def index(self, name):
+        return self._index[name]
+
+    def op(self, sign, u, v):
+        return self._OPS[sign](u, v)
+
+    def all(self, *x):
+        return functools.reduce(np.logical_and, x)
+
+    def any(self, *x):
+        return functools.reduce(np.logical_or, x)
+
+    def par(self, u):
+        return u
+
+
+def _range_walk(mod: TracedMod, K):
+    """What a mask is over a rectangle of positions, by interval arithmetic on its graph: the pair (certainly true, certainly false)
+    in the terms of K, None if it would never be told.
 
     An integer node is a pair of bounds, a boolean one a pair (certainly true, certainly false); floats, loads from
     captured tensors and whatever else has no rule here (a remainder by a power of two is a bitwise and) is unknown.  A node whose values could leave int32 for indices below
-    ``_IDX_BOUND`` is unknown too (the arithmetic of the mask wraps there), and so is every rectangle beyond that bound."""
-    lines: List[str] = []
-    env: Dict[int, Optional[tuple]] = {}  # int: (lo text, hi text, static lo, static hi); bool: (true text, false text)
-    n = 0
-
-    def fresh(pair, ctype, static=None):
-        nonlocal n
-        a, b = f"a{n}", f"z{n}"
-        n += 1
-        lines.append(f"  const {ctype} {a} = {pair[0]}, {b} = {pair[1]};")
-        return (a, b) if static is None else (a, b) + static
+    ``_IDX_BOUND`` is unknown too (the arithmetic of the mask wraps there)."""
+    env: Dict[int, Optional[tuple]] = {}  # int: (lo, hi, static lo, static hi); bool: (true, false)
 
     def integer(lo, hi, slo, shi):
         if slo < -(1 << 31) or shi >= 1 << 31:
             return None
-        return fresh((lo, hi), "int", (slo, shi))
+        return K.keep((lo, hi), "int") + (slo, shi)
 
     for e in _topo(mod.root):
         x = [env.get(id(a)) for a in e.args]
@@ -1417,75 +1489,82 @@ def to_cuda_range(mod: TracedMod, name: str) -> Optional[str]:
         c = e.args[1].value if len(e.args) == 2 and e.args[1].op == "const" and e.args[1].dtype == I32 else None
         r = None
         op = e.op
-        if op in ("q", "kv"):
-            r = (op + "0", op + "1", 0, _IDX_BOUND - 1)
-        elif op in ("b", "h"):
-            r = (op, op, 0, _IDX_BOUND - 1)
+        if op in ("q", "kv", "b", "h"):
+            r = tuple(K.index(op)) + (0, _IDX_BOUND - 1)
         elif op == "const":
             if e.dtype == I32:
-                v = f"({e.value})" if e.value != -(1 << 31) else "(-2147483647 - 1)"
-                r = (v, v, e.value, e.value)
+                r = (K.const(e.value), K.const(e.value), e.value, e.value)
             elif e.dtype == B1:
-                r = ("true", "false") if e.value else ("false", "true")
+                r = (K.true, K.false) if e.value else (K.false, K.true)
         elif e.dtype == I32 and ints:
             if op == "add":
-                r = integer(f"{x[0][0]} + {x[1][0]}", f"{x[0][1]} + {x[1][1]}", x[0][2] + x[1][2], x[0][3] + x[1][3])
+                r = integer(K.op("+", x[0][0], x[1][0]), K.op("+", x[0][1], x[1][1]), x[0][2] + x[1][2], x[0][3] + x[1][3])
             elif op == "sub":
-                r = integer(f"{x[0][0]} - {x[1][1]}", f"{x[0][1]} - {x[1][0]}", x[0][2] - x[1][3], x[0][3] - x[1][2])
+                r = integer(K.op("-", x[0][0], x[1][1]), K.op("-", x[0][1], x[1][0]), x[0][2] - x[1][3], x[0][3] - x[1][2])
             elif op == "neg":
-                r = integer(f"-{x[0][1]}", f"-{x[0][0]}", -x[0][3], -x[0][2])
+                r = integer(K.neg(x[0][1]), K.neg(x[0][0]), -x[0][3], -x[0][2])
             elif op in ("min", "max"):
-                f = min if op == "min" else max
-                r = integer(f"{op}({x[0][0]}, {x[1][0]})", f"{op}({x[0][1]}, {x[1][1]})", f(x[0][2], x[1][2]), f(x[0][3], x[1][3]))
+                f, g = (min, K.min) if op == "min" else (max, K.max)
+                r = integer(g(x[0][0], x[1][0]), g(x[0][1], x[1][1]), f(x[0][2], x[1][2]), f(x[0][3], x[1][3]))
             elif op == "abs":
                 m = max(abs(x[0][2]), abs(x[0][3]))
-                r = integer(f"({x[0][0]} > 0 ? {x[0][0]} : ({x[0][1]} < 0 ? -{x[0][1]} : 0))", f"max(-{x[0][0]}, {x[0][1]})", 0, m) if m < 1 << 31 else None
+                lo, hi = x[0][:2]
+                least = K.par(K.where(K.op(">", lo, 0), lo, K.par(K.where(K.op("<", hi, 0), K.neg(hi), 0))))
+                r = integer(least, K.max(K.neg(lo), hi), 0, m) if m < 1 << 31 else None
             elif op == "mul" and (c is not None or (e.args[0].op == "const")):
                 k, y = (c, x[0]) if c is not None else (e.args[0].value, x[1])
                 lo, hi = (y[0], y[1]) if k >= 0 else (y[1], y[0])
-                r = integer(f"{lo} * ({k})", f"{hi} * ({k})", min(y[2] * k, y[3] * k), max(y[2] * k, y[3] * k)) if k != -(1 << 31) else None
+                r = integer(K.op("*", lo, K.const(k)), K.op("*", hi, K.const(k)), min(y[2] * k, y[3] * k), max(y[2] * k, y[3] * k)) if k != -(1 << 31) else None
             elif op == "floordiv" and c is not None and c > 0:
-                r = integer(f"fa_floordiv_i32({x[0][0]}, {c})", f"fa_floordiv_i32({x[0][1]}, {c})", x[0][2] // c, x[0][3] // c)
+                r = integer(K.floordiv(x[0][0], c), K.floordiv(x[0][1], c), x[0][2] // c, x[0][3] // c)
             elif op == "rem" and c is not None and c > 0:
-                same = f"fa_floordiv_i32({x[0][0]}, {c}) == fa_floordiv_i32({x[0][1]}, {c})"
-                r = integer(f"({same}) ? fa_pymod_i32({x[0][0]}, {c}) : 0", f"({same}) ? fa_pymod_i32({x[0][1]}, {c}) : {c - 1}", 0, c - 1)
+                same = K.par(K.op("==", K.floordiv(x[0][0], c), K.floordiv(x[0][1], c)))
+                r = integer(K.where(same, K.pymod(x[0][0], c), 0), K.where(same, K.pymod(x[0][1], c), c - 1), 0, c - 1)
             elif op == "shr" and c is not None and 0 <= c < 32:
-                r = integer(f"{x[0][0]} >> {c}", f"{x[0][1]} >> {c}", x[0][2] >> c, x[0][3] >> c)
+                r = integer(K.op(">>", x[0][0], c), K.op(">>", x[0][1], c), x[0][2] >> c, x[0][3] >> c)
         elif e.dtype == I32 and op == "select" and known and e.args[0].dtype == B1:
             (t, f), u, v = x
-            r = integer(f"{t} ? {u[0]} : ({f} ? {v[0]} : min({u[0]}, {v[0]}))", f"{t} ? {u[1]} : ({f} ? {v[1]} : max({u[1]}, {v[1]}))",
+            r = integer(K.where(t, u[0], K.par(K.where(f, v[0], K.min(u[0], v[0])))), K.where(t, u[1], K.par(K.where(f, v[1], K.max(u[1], v[1])))),
                         min(u[2], v[2]), max(u[3], v[3]))
         elif e.dtype == B1 and op in ("lt", "le", "gt", "ge", "eq", "ne") and ints:
             u, v = (x[1], x[0]) if op in ("gt", "ge") else (x[0], x[1])
             if op in ("lt", "gt"):
-                r = fresh((f"{u[1]} < {v[0]}", f"{u[0]} >= {v[1]}"), "bool")
+                r = K.keep((K.op("<", u[1], v[0]), K.op(">=", u[0], v[1])), "bool")
             elif op in ("le", "ge"):
-                r = fresh((f"{u[1]} <= {v[0]}", f"{u[0]} > {v[1]}"), "bool")
+                r = K.keep((K.op("<=", u[1], v[0]), K.op(">", u[0], v[1])), "bool")
             else:
-                same = f"{u[0]} == {v[1]} && {u[1]} == {v[0]}"
-                apart = f"{u[1]} < {v[0]} || {v[1]} < {u[0]}"
-                r = fresh((same, apart) if op == "eq" else (apart, same), "bool")
+                same = K.all(K.op("==", u[0], v[1]), K.op("==", u[1], v[0]))
+                apart = K.any(K.op("<", u[1], v[0]), K.op("<", v[1], u[0]))
+                r = K.keep((same, apart) if op == "eq" else (apart, same), "bool")
         elif e.dtype == B1 and op in ("and", "or"):
-            u, v = (y if y is not None else ("false", "false") for y in x)
+            u, v = (y if y is not None else (K.false, K.false) for y in x)
             if x[0] is not None or x[1] is not None:
-                j, k = ("&&", "||") if op == "and" else ("||", "&&")
-                r = fresh((f"{u[0]} {j} {v[0]}", f"{u[1]} {k} {v[1]}"), "bool")
+                j, k = (K.all, K.any) if op == "and" else (K.any, K.all)
+                r = K.keep((j(u[0], v[0]), k(u[1], v[1])), "bool")
         elif e.dtype == B1 and op == "not" and known:
             r = (x[0][1], x[0][0])
         elif e.dtype == B1 and op == "select" and known and all(a.dtype == B1 for a in e.args):
             (t, f), u, v = x
-            r = fresh((f"({t} && {u[0]}) || ({f} && {v[0]}) || ({u[0]} && {v[0]})", f"({t} && {u[1]}) || ({f} && {v[1]}) || ({u[1]} && {v[1]})"), "bool")
+            r = K.keep(tuple(K.any(K.par(K.all(t, u[i])), K.par(K.all(f, v[i])), K.par(K.all(u[i], v[i]))) for i in (0, 1)), "bool")
         elif op == "cast_b1" and ints:
-            r = fresh((f"{x[0][0]} > 0 || {x[0][1]} < 0", f"{x[0][0]} == 0 && {x[0][1]} == 0"), "bool")
+            r = K.keep((K.any(K.op(">", x[0][0], 0), K.op("<", x[0][1], 0)), K.all(K.op("==", x[0][0], 0), K.op("==", x[0][1], 0))), "bool")
         elif op == "cast_i32" and known and e.args[0].dtype == B1:
-            r = integer(f"{x[0][0]} ? 1 : 0", f"{x[0][1]} ? 0 : 1", 0, 1)
+            r = integer(K.where(x[0][0], 1, 0), K.where(x[0][1], 0, 1), 0, 1)
         env[id(e)] = r
-    root = env[id(mod.root)]
+    return env[id(mod.root)]
+
+
+def to_cuda_range(mod: TracedMod, name: str) -> Optional[str]:
+    """Device function text of ``_range_walk``: ``int name(int b, int h, int q0, int q1, int kv0, int kv1)`` (bounds inclusive)
+    gives 0 where the mask is false for every position, 2 where it is true for every one, 1 where the intervals do not tell
+    and for rectangles beyond ``_IDX_BOUND``.  None if they never would."""
+    K = _RangeText()
+    root = _range_walk(mod, K)
     if root is None:
         return None
     bound = " || ".join(f"(unsigned){v} >= {_IDX_BOUND}u" for v in ("b", "h", "q0", "q1", "kv0", "kv1"))
     return "\n".join([f"__device__ __forceinline__ int {name}(int b, int h, int q0, int q1, int kv0, int kv1) {{",
-                      f"  if ({bound}) return 1;"] + lines + [f"  return {root[0]} ? 2 : ({root[1]} ? 0 : 1);", "}"]) + "\n"
+                      f"  if ({bound}) return 1;"] + K.lines + [f"  return {root[0]} ? 2 : ({root[1]} ? 0 : 1);", "}"]) + "\n"
 
 
 def _buffer_storage(buf, span: int) -> np.ndarray:
@@ -1702,28 +1781,34 @@ class ModSet:
         self.key = hashlib.sha256(self.source.encode()).hexdigest()
 
     def kv_tiles(self, Q_LEN: int, KV_LEN: int) -> int:
-        """About how many 128-key tiles the mask leaves of the keys per 128 query rows, 0 where that is not known: from the
-        first, middle and last position of the tiles under up to eight query tiles.  Of masks over captured tensors
-        only document masks are known, to leave few."""
-        if self.mask is None or self.buffers:
-            return 8 if self._documents else 0
+        """A guess at how many 128-key tiles the mask leaves of the keys per 128 query rows, 0 where there is none: what
+        interval arithmetic does not rule out (``_range_walk``), the average over up to eight query tiles.  Masks over captured
+        tensors have none, but for document masks: at most eight, as many documents leave."""
+        if self.mask is None or self.mask_reads_b or self.mask_reads_h or (self.buffers and not self._documents):
+            return 0
         n = self._kv_tiles.get((Q_LEN, KV_LEN))
         if n is None:
             try:
-                nq, nkv = (Q_LEN + 127) // 128, (KV_LEN + 127) // 128
-                tiles = np.unique(np.linspace(0, nq - 1, min(nq, 8)).round().astype(np.int64))
-                at = np.array([0, 64, 127])
-                q = np.minimum(128 * tiles[:, None] + at, Q_LEN - 1).reshape(-1, 1)
-                kv = np.minimum(128 * np.arange(nkv)[:, None] + at, KV_LEN - 1).reshape(1, -1)
-                keep = np.broadcast_to(evaluate(self.mask, None, 0, 0, q, kv), (q.size, kv.size))
-                listed = keep.reshape(len(tiles), 3, nkv, 3).any(axis=(1, 3)).sum(axis=1)
-                n = min(max(int(round(float(listed.mean()))), 1), 65535)
-            except Exception:  # (whatever it is, no result needs the hint)
+                n = self._count_kv_tiles(Q_LEN, KV_LEN)
+            except Exception:  # (whatever it is, no result needs the guess)
                 n = 0
+            if self._documents:
+                n = min(n, 8)
             if len(self._kv_tiles) >= 64:
                 self._kv_tiles.clear()
             self._kv_tiles[(Q_LEN, KV_LEN)] = n
         return n
+
+    def _count_kv_tiles(self, Q_LEN: int, KV_LEN: int) -> int:
+        if not 0 < min(Q_LEN, KV_LEN) <= max(Q_LEN, KV_LEN) <= _IDX_BOUND:
+            return 0
+        nq, nkv = (Q_LEN + 127) // 128, (KV_LEN + 127) // 128
+        q = 128 * np.linspace(0, nq - 1, min(nq, 8)).round().astype(np.int64)[:, None]
+        kv = 128 * np.arange(nkv, dtype=np.int64)[None]
+        told = _range_walk(self.mask, _RangeNumpy((q, np.minimum(q + 127, Q_LEN - 1)), (kv, np.minimum(kv + 127, KV_LEN - 1))))
+        dropped = _RangeNumpy.false if told is None else told[1]
+        listed = ~np.broadcast_to(dropped, (len(q), nkv))
+        return min(max(int(round(float(listed.sum(axis=1).mean()))), 1), 65535)
 
 
 def _trace_any(fn: Callable, kind: str, bufs: List[object]) -> TracedMod:

@@ -46,8 +46,8 @@ extern "C" {
 #define FA_FLAG_ROUND_SCORES 1
 /* Use the general (mma.sync) kernels even where a tcgen05 kernel covers the shape. */
 #define FA_FLAG_GENERAL_KERNELS 16
-/* A hint that may be ORed in: the average number of 128-key tiles that the BlockMask lists for 128 query rows
- * (1 to 65535; 0, no such bits: not known).  It picks between kernel variants with the same results. */
+/* A hint that may be ORed in: a guess at the average number of 128-key tiles that the BlockMask lists for 128 query rows
+ * (1 to 65535; 0, no such bits: none).  It picks between kernel variants with the same results. */
 #define FA_FLAG_KV_TILES(n) ((n) << 8)
 
 enum fa_dtype { FA_F16 = 0, FA_BF16 = 1, FA_F32 = 2 };

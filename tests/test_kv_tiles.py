@@ -39,3 +39,23 @@ def test_a_failure_is_no_failure_of_the_call(monkeypatch):
 
     monkeypatch.setattr(modtrace.np, "linspace", fail)
     assert ms.kv_tiles(1024, 1024) == 0
+
+
+def test_masks_of_scattered_positions():
+    """Every tile has some: a stride, one position per row, a band between the samples that a look at a few positions would take."""
+    n = lambda mask: modtrace.lower_mods(None, mask).kv_tiles(8192, 8192)  # noqa: E731
+    assert n(lambda b, h, q, kv: (kv % 128 == 5) | (q == kv)) == 64
+    assert n(lambda b, h, q, kv: (kv // 16) % 8 == 3) == 64
+    assert n(lambda b, h, q, kv: (q - kv >= 20) & (q - kv < 26)) == 2
+
+
+@pytest.mark.parametrize("mask", [lambda b, h, q, kv: (q >= kv) & (b > 0), lambda b, h, q, kv: q + 1000 * h >= kv], ids=["batch", "head"])
+def test_masks_that_differ_between_entries_are_not_known(mask):
+    assert modtrace.lower_mods(None, mask).kv_tiles(8192, 8192) == 0
+
+
+def test_documents_are_a_guess_bounded_by_the_rest_of_the_mask():
+    ids = torch.arange(8192) // 700
+    causal = modtrace.lower_mods(None, lambda b, h, q, kv: (ids[q] == ids[kv]) & (q >= kv))
+    assert causal.kv_tiles(8192, 8192) == 8 and causal.kv_tiles(640, 640) == 3
+    assert modtrace.lower_mods(None, lambda b, h, q, kv: ids[q] == ids[kv]).kv_tiles(8192, 8192) == 8
