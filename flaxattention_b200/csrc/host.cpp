@@ -544,12 +544,17 @@ PyObject* build_block_mask(PyObject*, PyObject* const* a, Py_ssize_t n) {
     pybind11::gil_scoped_release no_gil;
     c10::cuda::OptionalCUDAGuard guard(dev);
     const int64_t B = mb.B, H = mb.H, nq = mb.Q_LEN / mb.q_block, nkv = mb.KV_LEN / mb.kv_block;
-    // one allocation for the tables (16-byte aligned parts) and the class grid behind them
+    // one allocation for the tables (16-byte aligned parts), and the class grid behind them while it is small: an allocation less, but
+    // it lives as long as they do; a large one is given back at once
+    constexpr size_t kScratchInTables = 64 << 10;
     const auto up = [](int64_t v) { return (v + 3) / 4 * 4; };
     const int64_t idx = up(B * H * nq * nkv), num_q = up(B * H * nq), num_kv = up(B * H * nkv);
     const size_t ws = fa_block_mask_workspace_bytes(mb.distinct_B, mb.distinct_H, mb.Q_LEN, mb.KV_LEN, mb.q_block, mb.kv_block);
     const int64_t n_tables = 4 * idx + 2 * num_q + 2 * num_kv;
-    at::Tensor base = empty({n_tables + (int64_t)(std::max<size_t>(ws, 16) + 3) / 4}, at::kInt, dev);
+    const int64_t n_scratch = (int64_t)(std::max<size_t>(ws, 16) + 3) / 4;
+    const bool own_scratch = ws > kScratchInTables;
+    at::Tensor base = empty({n_tables + (own_scratch ? 0 : n_scratch)}, at::kInt, dev);
+    at::Tensor scratch = own_scratch ? empty({n_scratch}, at::kInt, dev) : at::Tensor();
     int64_t off = 0;
     int32_t* ptr[8];
     for (int i = 0; i < 8; ++i) {
@@ -561,7 +566,7 @@ PyObject* build_block_mask(PyObject*, PyObject* const* a, Py_ssize_t n) {
     }
     mb.kv_num_blocks = ptr[0]; mb.kv_indices = ptr[1]; mb.full_kv_num_blocks = ptr[2]; mb.full_kv_indices = ptr[3];
     mb.q_num_blocks = ptr[4]; mb.q_indices = ptr[5]; mb.full_q_num_blocks = ptr[6]; mb.full_q_indices = ptr[7];
-    mb.workspace = (int32_t*)base.mutable_data_ptr() + n_tables;
+    mb.workspace = own_scratch ? (int32_t*)scratch.mutable_data_ptr() : (int32_t*)base.mutable_data_ptr() + n_tables;
     mb.workspace_bytes = ws;
     // the matrices come out of the same evaluation where the blocks are whole words, else out of one of their own
     const bool apart = want_bits && ((nq > 1 && mb.q_block % 32) || (nkv > 1 && mb.kv_block % 32));

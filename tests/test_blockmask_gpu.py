@@ -142,6 +142,24 @@ def test_mask_bits_equal_the_mask_of_the_oracle():
     assert tuple(bm.mask_bits.shape[:2]) == (1, 1) and np.array_equal(_unpack_bits(bm.mask_bits, 256)[0, 0], want)
 
 
+@pytest.mark.parametrize("B", [64, 65])  # (the class grid: 64 KiB, which stays with the tables, and one entry more)
+def test_a_large_class_grid_is_given_back(B):
+    import flaxattention_b200 as fa
+
+    H, S = 4, 2048
+    mod = lambda b, h, q, kv: (q >= kv) & (q - kv < 40 * (b + 1) + 300 * h)  # noqa: E731
+    bm = fa.create_block_mask(mod, B, H, S, S, device="cuda")
+    tables = [getattr(bm, k) for k in TABLE_KEYS]
+    words = sum(t.numel() for t in tables)
+    held = bm.kv_indices.untyped_storage().nbytes()
+    grid = B * H * (S // 128) ** 2
+    assert all(t.untyped_storage().data_ptr() == bm.kv_indices.untyped_storage().data_ptr() for t in tables)
+    assert held == 4 * words + (grid if grid <= 64 << 10 else 0)
+    want = create_block_mask_oracle(lambda b, h, q, kv: mod(b + B - 1, h, q, kv), 1, H, S, S)
+    for k in TABLE_KEYS:
+        assert np.array_equal(getattr(bm, k)[B - 1:].cpu().numpy(), want[k])
+
+
 @pytest.mark.parametrize("D,dtype", [(64, torch.float16), (128, torch.bfloat16)])
 def test_attention_is_the_same_with_and_without_mask_bits(D, dtype):
     """The kernels read the bit matrix on partial tiles instead of evaluating mask_mod: forward and
