@@ -311,8 +311,11 @@ extern "C" __global__ void __launch_bounds__(fa_dec::NT, fa_dec::MIN_CTAS) fa_de
   }
 #if FA_HAS_SCORE_MOD && defined(FA_SCORE_AFFINE) && defined(FA_SCORE_LINEAR_KV)
   // A bias that is linear over kv (ALiBi) under a multiplier that does not read it: multiplier and slope of this thread's two rows
-  // are taken here, the bias once per tile at the thread's first key, and the other keys add multiples of the slope.
-  fa_u64 lin_m[2], lin_d[2];
+  // are taken here, the bias once per tile at the thread's first key, and the other keys add multiples of the slope.  To the scores:
+  // added to the bias, they would round a large one once more per key (60000 + kv / 2048: error of the probabilities 2.9e-3,
+  // where three roundings are 2.7e-3).
+  constexpr int LIN_KEPT = WN / 8 <= 4 ? WN / 8 : 0;  // (pairs of multiples in registers)
+  fa_u64 lin_m[2], lin_d[2], lin_od[2][LIN_KEPT > 0 ? LIN_KEPT : 1];
 #pragma unroll
   for (int hh = 0; hh < 2; ++hh) {
     const int row = rg * 16 + hh * 8 + (lane >> 2);
@@ -321,6 +324,8 @@ extern "C" __global__ void __launch_bounds__(fa_dec::NT, fa_dec::MIN_CTAS) fa_de
     const float mul = fa_score_mul(0.f, gb, gh, qi, 0) * (p.scale * FA_LOG2E), slope = fa_score_add2_dkv(0.f, gb, gh, qi, 0);
     lin_m[hh] = fa_f2(mul, mul);
     lin_d[hh] = fa_f2(slope, slope);
+#pragma unroll
+    for (int j = 0; j < LIN_KEPT; ++j) lin_od[hh][j] = fa_f2((float)(j * 8) * slope, (float)(j * 8 + 1) * slope);
   }
 #endif
   fa_u32 qf[D / 16][4];
@@ -387,7 +392,8 @@ extern "C" __global__ void __launch_bounds__(fa_dec::NT, fa_dec::MIN_CTAS) fa_de
         const int kv = kv0 + j * 8;
         float x0 = s[j][hh * 2], x1 = s[j][hh * 2 + 1];
 #if FA_HAS_SCORE_MOD && defined(FA_SCORE_AFFINE) && defined(FA_SCORE_LINEAR_KV)
-        fa_f2_unpack(fa_fma2(fa_f2(x0, x1), lin_m[hh], fa_fma2(fa_f2((float)(j * 8), (float)(j * 8 + 1)), lin_d[hh], lin_b)), x0, x1);
+        const fa_u64 od = LIN_KEPT > 0 ? lin_od[hh][LIN_KEPT > 0 ? j : 0] : fa_mul2(fa_f2((float)(j * 8), (float)(j * 8 + 1)), lin_d[hh]);
+        fa_f2_unpack(fa_add2(fa_fma2(fa_f2(x0, x1), lin_m[hh], od), lin_b), x0, x1);
 #elif FA_HAS_SCORE_MOD && defined(FA_SCORE_AFFINE)
         // affine score_mod: scale and log2(e) folded into one FMA
         x0 = fmaf(x0, fa_score_mul(0.f, gb, gh, qi, kv) * sc2, fa_score_add2(0.f, gb, gh, qi, kv));
