@@ -494,8 +494,11 @@ bool decode_by_tma(DecCfg& c, int dtype, int D, int Dv) {
   c.tma = true;
   return true;
 }
-// the same with three buffers of K and of V, where two CTAs of up to 16 rows still share an SM then
+// the same with three buffers of K and of V, where two CTAs of up to 16 rows still share an SM then; by cp.async only for tiles of
+// more than 16 KB of K and V (us, two / three: D 16, B16 H4 Skv8191, one row 15.0 / 16.4, D 32 18.1 / 21.1; D 48 32.3 / 26.5, D 96 55.5 / 47.0, D 128
+// with values of 64, 16 rows 48.7 / 40.4)
 bool decode_third_buffer(DecCfg& c, int D, int Dv) {
+  if (!c.tma && D + Dv <= 64) return false;
   const int smem = c.smem + (c.tma ? 2 * c.BN * D * 2 + 4 * 2 * 8 : c.BN * (pitch(D, 2) + pitch(Dv, 2)));
   if (c.BM != 16 || 2 * (smem + 1024) > 228 * 1024) return false;
   c.smem = smem;
