@@ -112,8 +112,11 @@ constexpr int SMEM_BYTES = Q_BYTES + PIPE_SPAN + BAR_BYTES + (TMA ? 1024 : 0);  
 // 2.18e-3 against 2.32e-3), and the second instruction costs time (34.3 us, 31.5 without).
 constexpr bool TWO_PARTS = RG == 1;
 
-// CTAs that share an SM by their shared memory: the registers must not allow fewer (170 at three)
-constexpr int MIN_CTAS = 228 * 1024 / (SMEM_BYTES + 1024) >= 3 ? 3 : (228 * 1024 / (SMEM_BYTES + 1024) >= 2 ? 2 : 1);
+// CTAs that share an SM by their shared memory: the registers must not allow fewer, up to three (170 registers), four (128) for two row
+// groups of short rows (24 rows, B32 H8 Skv4096 D 16: 31.9 us with four, 45.3 with three, D 32 likewise; D 80 wants three for short
+// caches).  Not with four row groups, whose warps need them (48 rows, B32 H8 Skv4096 D 32: 69 without, 78.6 with).
+constexpr int SMEM_CTAS = 228 * 1024 / (SMEM_BYTES + 1024), MOST_CTAS = RG == 4 ? 1 : (RG == 2 && D + DV <= 64 ? 4 : 3);
+constexpr int MIN_CTAS = SMEM_CTAS < MOST_CTAS ? (SMEM_CTAS > 0 ? SMEM_CTAS : 1) : MOST_CTAS;
 
 static_assert(!TMA || (RG == 1 && D == DV && D % 64 == 0 && WN % 8 == 0), "TMA: warps on their own, whole column groups");
 static_assert(DT != FA_DT_F32, "the decode kernel takes 16-bit inputs");
