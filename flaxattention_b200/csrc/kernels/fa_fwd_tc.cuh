@@ -117,7 +117,6 @@ constexpr bool ROT = D == 64 && !F32 && !DECODE;
 constexpr int COL_S = 0, COL_O = F32 ? 384 : (ROT ? 192 : 128) * NQ, S_STRIDE = F32 || ROT ? 192 : 128;
 // In the decode variant P has columns of its own (384..511).  With D = 128 the 512 columns are taken by S and O, and
 // P overwrites the S columns it was computed from.
-constexpr bool SEP_P = DECODE;
 constexpr int COL_P = 192 * NQ;
 // One pair of exponentials in FA_TC_POLY_EVERY goes to the FMA pipe (a cubic, see fa_ex2_poly2).
 // Measured (B8 H8 S2048 D64): every fourth pair takes the forward without a score_mod from 0.118 to
@@ -154,14 +153,14 @@ constexpr int BAR_KFULL = 1, BAR_KEMPTY = 1 + NSTAGE, BAR_VFULL = 1 + 2 * NSTAGE
 // tile only meet at its S: one that is ahead may hand over P of a step before the others have handed over that of
 // the last one, and the softmax does not look at every PV product.)
 constexpr int BAR_S = 1 + 4 * NSTAGE, BAR_P = BAR_S + 2, BAR_O = BAR_S + 6;
-// Where P does not lie over S of the same step for long (ROT, SEP_P), the S columns of a tile are released as soon as
+// Where P does not lie over S of the same step for long (ROT, DECODE), the S columns of a tile are released as soon as
 // the softmax warps hold the scores in registers, and S of the next step is produced during the softmax.
 constexpr int BAR_SFREE2 = BAR_S + 10;
 constexpr int BAR_LAG = BAR_S + 12;  // (ROT) the first scores of the first tile are in registers; used once
-constexpr bool EARLY_S = ROT || SEP_P;
+constexpr bool EARLY_S = ROT || DECODE;
 // Head dim 128: P is handed over in two parts, keys 0-95 (BAR_P) and 96-127 (BAR_P2), so that most of the PV product
 // runs under the last exponentials.  It is the first link of the chain PV(j), S(j+1) that the tile then waits for.
-constexpr bool SPLIT_P = !ROT && !SEP_P && !F32;
+constexpr bool SPLIT_P = !ROT && !DECODE && !F32;
 constexpr int BAR_P2 = BAR_S + 10;
 
 // Work on one 32-column chunk of a score row held in registers (columns C0 .. C0+31 of the kv
@@ -416,7 +415,7 @@ __device__ __forceinline__ bool softmax_step(SoftmaxCtx& c, const int tile, cons
     l *= corr;
   }
   const bool rescale = cnt > 0 && __any_sync(0xffffffffu, need);
-  if (cnt > 0 && (SEP_P || rescale)) {
+  if (cnt > 0 && (DECODE || rescale)) {
     // O is rescaled in place, and with separate P columns the previous PV product reads the P columns that are
     // about to be overwritten: it must be complete
     const fa_u32 last = cnt - 1;
@@ -815,8 +814,8 @@ extern "C" __global__ void __launch_bounds__(fa_tc::NT, fa_tc::NQ == 1 ? 2 : 1) 
           fa_tma_load_4d(sb + OFF_V + s * KV_STAGE + a * ATOM_BYTES, &P.tv, bar_addr(sb, BAR_VFULL + s), a * 64, n0, hk, b);
       }
     }
-  } else if (SEP_P && (warp == WARP_MMA || warp == WARP_MMA_B)) {
-    // ============ two MMA issuers (D = 64): warp A issues the S products, warp B the PV products ====
+  } else if (DECODE && (warp == WARP_MMA || warp == WARP_MMA_B)) {
+    // ============ decode variant: warp A issues the S products, warp B the PV products ======
     // With P in its own TMEM columns the two streams only meet through the softmax warps, so each
     // issuer waits on its own barriers and the waits of one overlap the issue of the other.
     if (lane == 0 && nsteps > 0) {
@@ -826,18 +825,12 @@ extern "C" __global__ void __launch_bounds__(fa_tc::NT, fa_tc::NQ == 1 ? 2 : 1) 
         bool ok = fa_mbar_wait(bar_addr(sb, BAR_Q), 0, abort_flag);
         fa_u32 nsi[2] = {0, 0};
         for (int j = 0; j < nsteps && ok; ++j) {
-          // the kv tile of (step, query tile): the same for both tiles in the forward, alternate
-          // tiles of the CTA's share in the decode variant
-          int s = j % NSTAGE;
-          if (!DECODE) ok = fa_mbar_wait(bar_addr(sb, BAR_KFULL + s), (fa_u32)((j / NSTAGE) & 1), abort_flag);
+          // (the warpgroups take the CTA's share of the kv tiles in turn)
           for (int i = 0; i < NQ && ok; ++i) {
-            if (!(sched[2 * j + i] >> 16)) continue;
-            if (DECODE) {
-              const int t = 2 * j + i;
-              s = t % NSTAGE;
-              ok = fa_mbar_wait(bar_addr(sb, BAR_KFULL + s), (fa_u32)((t / NSTAGE) & 1), abort_flag);
-              if (!ok) break;
-            }
+            const int t = 2 * j + i, s = t % NSTAGE;
+            if (!(sched[t] >> 16)) continue;
+            ok = fa_mbar_wait(bar_addr(sb, BAR_KFULL + s), (fa_u32)((t / NSTAGE) & 1), abort_flag);
+            if (!ok) break;
             if (nsi[i] > 0) {
               ok = fa_mbar_wait(bar_addr(sb, BAR_SFREE2 + i), (nsi[i] - 1) & 1u, abort_flag);
               if (!ok) break;
@@ -850,26 +843,20 @@ extern "C" __global__ void __launch_bounds__(fa_tc::NT, fa_tc::NQ == 1 ? 2 : 1) 
               fa_mma_ss(tmem + COL_S + i * BN, fa_desc_make(loQ + koff, HI), fa_desc_make(loK + koff, HI), IDESC_S, kk > 0);
             }
             fa_mma_commit(bar_addr(sb, BAR_S + i));
-            if (DECODE) fa_mma_commit(bar_addr(sb, BAR_KEMPTY + s));
+            fa_mma_commit(bar_addr(sb, BAR_KEMPTY + s));
             ++nsi[i];
           }
-          if (!DECODE) fa_mma_commit(bar_addr(sb, BAR_KEMPTY + s));
         }
       } else {
         constexpr fa_u32 IDESC_O = fa_idesc(DT, BM, D, 0, 1);
         bool ok = true;
         fa_u32 cnt[2] = {0, 0};
         for (int j = 0; j < nsteps && ok; ++j) {
-          int s = j % NSTAGE;
-          if (!DECODE) ok = fa_mbar_wait(bar_addr(sb, BAR_VFULL + s), (fa_u32)((j / NSTAGE) & 1), abort_flag);
           for (int i = 0; i < NQ && ok; ++i) {
-            if (!(sched[2 * j + i] >> 16)) continue;
-            if (DECODE) {
-              const int t = 2 * j + i;
-              s = t % NSTAGE;
-              ok = fa_mbar_wait(bar_addr(sb, BAR_VFULL + s), (fa_u32)((t / NSTAGE) & 1), abort_flag);
-              if (!ok) break;
-            }
+            const int t = 2 * j + i, s = t % NSTAGE;
+            if (!(sched[t] >> 16)) continue;
+            ok = fa_mbar_wait(bar_addr(sb, BAR_VFULL + s), (fa_u32)((t / NSTAGE) & 1), abort_flag);
+            if (!ok) break;
             ok = fa_mbar_wait(bar_addr(sb, BAR_P + i), cnt[i] & 1u, abort_flag);
             if (!ok) break;
             fa_tc_fence_after();
@@ -879,10 +866,9 @@ extern "C" __global__ void __launch_bounds__(fa_tc::NT, fa_tc::NQ == 1 ? 2 : 1) 
             for (int kk = 0; kk < BN / 16; ++kk)
               fa_mma_ts(tmem + COL_O + i * D, tmem + COL_P + i * 64 + kk * 8, fa_desc_make(loV + kk * 128, HI), IDESC_O, acc | (kk > 0));
             fa_mma_commit(bar_addr(sb, BAR_O + i));
-            if (DECODE) fa_mma_commit(bar_addr(sb, BAR_VEMPTY + s));
+            fa_mma_commit(bar_addr(sb, BAR_VEMPTY + s));
             ++cnt[i];
           }
-          if (!DECODE) fa_mma_commit(bar_addr(sb, BAR_VEMPTY + s));
         }
       }
     }
@@ -958,7 +944,7 @@ extern "C" __global__ void __launch_bounds__(fa_tc::NT, fa_tc::NQ == 1 ? 2 : 1) 
       if (leader) fa_mma_commit(bar_addr(sb, BAR_VEMPTY + j % NSTAGE));
       w = w1;
     }
-  } else if (!SEP_P && !ROT && warp == WARP_MMA) {
+  } else if (!DECODE && !ROT && warp == WARP_MMA) {
     // ============ one MMA issuer for both query tiles ======================================
     // The whole warp runs the loop and one elected lane issues: in uniform control flow the operands of tcgen05.mma
     // sit in uniform registers, which makes the instructions cheaper to issue than from a single-lane branch.
@@ -1087,7 +1073,7 @@ extern "C" __global__ void __launch_bounds__(fa_tc::NT, fa_tc::NQ == 1 ? 2 : 1) 
     fa_u32 idle_cnt = 0;
     const fa_u32 t_s = tmem + ((fa_u32)lane_base << 16) + COL_S + i * S_STRIDE;
     const fa_u32 t_o = tmem + ((fa_u32)lane_base << 16) + COL_O + i * D;
-    const fa_u32 t_p = SEP_P ? tmem + ((fa_u32)lane_base << 16) + COL_P + i * 64 : t_s;
+    const fa_u32 t_p = DECODE ? tmem + ((fa_u32)lane_base << 16) + COL_P + i * 64 : t_s;
     bool ok = true;
     // (rows beyond Sq have no row in the bit matrix: their scores are never stored, the mask is evaluated)
     const unsigned* rowbits = (p.t.mask_bits != nullptr && qi < p.Sq && (p.t.mask_hold == nullptr || *p.t.mask_hold != 0))
@@ -1134,7 +1120,7 @@ extern "C" __global__ void __launch_bounds__(fa_tc::NT, fa_tc::NQ == 1 ? 2 : 1) 
         if (!ok) break;
         fa_tc_fence_after();
         fa_tc_fence_before();
-        if (SEP_P) fa_mbar_arrive(bar_addr(sb, BAR_SFREE2 + i));
+        if (DECODE) fa_mbar_arrive(bar_addr(sb, BAR_SFREE2 + i));
         fa_mbar_arrive(bar_addr(sb, BAR_P + i));
         ++idle_cnt;
         continue;
