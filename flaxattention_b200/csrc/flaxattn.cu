@@ -176,6 +176,7 @@ constexpr int kMaxModBuffers = FA_MAX_MOD_BUFS;
 
 struct fa_module {
   std::string mod_source;
+  bool has_score_mod = false, linear_score_mod = false;  // (as its defines say, for the choice between variants; linear: over the keys)
   std::unordered_map<uint64_t, Kernel*> kernels;  // key: kernel_key of the variant
   const void* bufs[kMaxModBuffers] = {nullptr};  // device addresses of the captured buffers of the mods
   int nbufs = 0;
@@ -1097,6 +1098,8 @@ int fa_module_create(const char* mod_source, fa_module** out) {
   if (!out) return fail(FA_EINVAL, "out is null");
   fa_module* m = new fa_module();
   m->mod_source = (mod_source && *mod_source) ? mod_source : kDefaultMods;
+  m->has_score_mod = m->mod_source.find("#define FA_HAS_SCORE_MOD 1") != std::string::npos;
+  m->linear_score_mod = m->mod_source.find("#define FA_SCORE_LINEAR_KV 1") != std::string::npos;
   *out = m;
   return FA_OK;
 }
@@ -1380,26 +1383,39 @@ int launch_decode_tc(fa_module* m, const fa_attn_params* p, const FaParams& kp, 
 //                      causal S2048 78 / 76, S2560 59 / 57, S3072 77 / 76, S4096 62 / 64
 //   more, D = 128      dense S2048 152 / 152, S3072 160 / 164, S4096 139 / 145; causal 98 / 94, 98 / 98, 80 / 82
 // The dense lengths cross between 2560 and 3072 keys.  Under a BlockMask that leaves few steps the fixed part weighs more:
-// one where the caller says that it lists up to 16 tiles of keys per query tile (D = 64) or up to 10 (D = 128).  Two against one:
-//   D = 64   B4 H8 S4096 window 256 46 / 41, 1024 72 / 68, attention sink 77 / 73, 12 documents 50 / 43, causal (16.5 tiles) 112 / 112;
-//            B2 H8 S8192 47 / 42, 81 / 74, 90 / 79, 59 / 55, causal (32.5) 193 / 199
-//   D = 128  the same 61 / 54, 91 / 89, 94 / 94, 61 / 49, 135 / 149; 66 / 58, 108 / 102, 114 / 107, 71 / 63, 236 / 269;
+// one where the caller says that it lists up to 12 tiles of keys per query tile (D = 64; up to 16 where these are three eighths of the key tiles or
+// fewer, or with rounded scores, whose steps cost more: window 1700, 14 tiles, B2 H8 S8192 107 / 105, rounded 124 / 117) or up to 10 (D = 128).
+// Two against one:
+//   D = 64   B4 H8 S4096 window 256 46 / 41, 1024 74 / 70, 2000 (12.7 tiles) 97.6 / 96.6, attention sink 78 / 75, 12 documents 49 / 44, causal (16.5)
+//            112 / 117; B2 H8 S8192 window 256 47 / 42, 1024 85 / 75, 2000 (15.3) 111 / 113, sink 91 / 81, documents 60 / 55, causal (32.5) 193 / 207
+//   D = 128  B4 H8 S4096 the same 61 / 54, 91 / 89, -, 94 / 94, 61 / 49, 135 / 149; B2 H8 S8192 66 / 58, 108 / 102, -, 114 / 107, 71 / 63, 236 / 269;
 //            B4 H16 S8192 245 / 222, 406 / 417, 437 / 389, 271 / 233; causal B8 H16 S1000 (4.5) 64 / 60, B4 H8 S2560 (10.5) 67 / 67,
 //            B2 H16/4 S3001 (12.5) 87 / 91
-// At D = 64 also one where the tables list half of the key tiles or fewer, so that query tiles differ (causal), and there are up to four
-// tiles per SM: a long and a short one share an SM, where two neighbours in one CTA are both long.  Two against one: causal B2 H4 S4828
-// 69 / 54, B1 H4 S8192 101 / 83, H8 S6144 84 / 71, B2 H8 S4096 (512 tiles) 59.5 / 60, B1 H8 S8192 110 / 106, with ALiBi 124 / 89 at
-// B1 H4 S8192.  (Not at D = 128, causal: 63 / 62, 118 / 134; nor where all tiles are alike, dense B1 H4 S8192: 97 / 112.)
-int fwd_tc_query_tiles(const fa_attn_params* p) {
-  const long long tiles = (long long)p->B * p->Hq * ((p->Sq + 127) / 128);
-  const int listed = p->tables.kv_num_blocks ? (p->flags >> 8) & 0xffff : 0;
-  if (listed > 0 && listed <= (p->D == 64 ? 16 : 10)) return 1;
-  if (listed > 0 && p->D == 64 && 2 * listed <= (p->Skv + 127) / 128 + 2 && tiles <= 4LL * device_sm_count()) return 1;
+// At D = 64 also one where the tables list half of the key tiles or fewer, so that query tiles differ (causal), and there are up to three
+// tiles per SM, four if they list three eighths or fewer or the scores are rounded without a score_mod: a long and a short one share an SM, where
+// two neighbours in one CTA are both long.  Two against one: causal B2 H4 S4828 69 / 54, B1 H4 S8192 101 / 83, H12 S4096 (384 tiles) 59 / 53;
+// B2 H8 S4096 (512) 59 / 63, B1 H8 S8192 103 / 111, but rounded 129 / 128 and with a window of 3000 92 / 84.  (Not at D = 128, causal: 63 / 62,
+// 118 / 134; nor where all tiles are alike, dense B1 H4 S8192: 97 / 112.)
+// At D = 64 under any tables with a score_mod: the two tiles of a CTA then fall into step, two CTAs do not.  Two against one, ALiBi:
+// causal B4 H8 S4096 130 / 127, B8 H8 250 / 237, B1 H8 S16384 454 / 421, window 3000 B2 H8 S8192 164 / 156, all keys B2 H8 S8192 490 / 422,
+// S2304 43 / 42; checkerboard: 123 / 120, 233 / 222, 412 / 391, -, 455 / 394, 40.4 / 39.4.  With rounded scores the same (244 / 240 causal, 512 / 452
+// all keys, B2 H8 S8192), except where the mod is linear over the keys (ALiBi: causal 247 / 257, B8 H8 S4096 263 / 270, all keys 462 / 483).
+int fwd_tc_query_tiles(const fa_module* m, const fa_attn_params* p) {
+  const long long tiles = (long long)p->B * p->Hq * ((p->Sq + 127) / 128), kv_tiles = (p->Skv + 127) / 128;
+  if (p->tables.kv_num_blocks) {
+    const int listed = (p->flags >> 8) & 0xffff;
+    const bool rounded = round_flag(p->dtype, p->flags);
+    const bool few = 8 * listed <= 3 * kv_tiles;
+    if (listed > 0 && listed <= (p->D == 64 ? (rounded || few ? 16 : 12) : 10)) return 1;
+    if (p->D == 64 && m->has_score_mod && !(rounded && m->linear_score_mod)) return 1;
+    const int per_sm = 2 * listed > kv_tiles + 2 ? 0 : few || (rounded && !m->has_score_mod) ? 4 : 3;
+    if (p->D == 64 && listed > 0 && tiles <= (long long)per_sm * device_sm_count()) return 1;
+  }
   return (p->D == 64 && p->Skv <= 2048) || tiles <= device_sm_count() ? 1 : 2;
 }
 int launch_fwd_tc(fa_module* m, const fa_attn_params* p, const FaParams& kp, void* stream) {
   Kernel* k = nullptr;
-  const int nq = fwd_tc_query_tiles(p);
+  const int nq = fwd_tc_query_tiles(m, p);
   if (int rc = get_fwd_tc_kernel(m, p->dtype, p->D, p->flags, &k, false, nq)) return rc;
   FaTcParamsHost tp;
   tp.p = kp;

@@ -156,7 +156,7 @@ constexpr int BAR_S = 1 + 4 * NSTAGE, BAR_P = BAR_S + 2, BAR_O = BAR_S + 6;
 // Where P does not lie over S of the same step for long (ROT, DECODE), the S columns of a tile are released as soon as
 // the softmax warps hold the scores in registers, and S of the next step is produced during the softmax.
 constexpr int BAR_SFREE2 = BAR_S + 10;
-constexpr int BAR_LAG = BAR_S + 12;  // (ROT) the first scores of the first tile are in registers; used once
+constexpr int BAR_LAG = BAR_S + 12;  // (ROT) the first PV product of the second tile is complete; used once
 constexpr bool EARLY_S = ROT || DECODE;
 // Head dim 128: P is handed over in two parts, keys 0-95 (BAR_P) and 96-127 (BAR_P2), so that most of the PV product
 // runs under the last exponentials.  It is the first link of the chain PV(j), S(j+1) that the tile then waits for.
@@ -345,7 +345,10 @@ __device__ __forceinline__ bool softmax_step(SoftmaxCtx& c, const int tile, cons
   const bool use_mask = FA_HAS_MASK_MOD && mode == 1;
   const bool have_words = masked && use_mask && c.rowbits != nullptr;
   uint4 words = make_uint4(0u, 0u, 0u, 0u);
-  if (have_words) words = mask_words<DECODE ? 2 : 4>(c.rowbits, n0);  // (on their way during the wait)
+  // The mask words are on their way during the wait for the scores; not where few of many steps are partial (two tiles at head dim 64), where
+  // they cost registers in every step
+  constexpr bool LATE_WORDS = ROT && NQ == 2;
+  if (!LATE_WORDS && have_words) words = mask_words<DECODE ? 2 : 4>(c.rowbits, n0);
   if (!fa_mbar_wait_warp(bar_addr(sb, BAR_S + i), cnt & 1u, abort_flag)) return false;
   fa_tc_fence_after();
   // ---- pass 1: the whole score row (128 fp32 values) comes into registers, chunk by chunk,
@@ -385,6 +388,7 @@ __device__ __forceinline__ bool softmax_step(SoftmaxCtx& c, const int tile, cons
   if (masked) {
     // (the row maximum taken on the way is of the unmasked scores: it is taken again)
     fa_u32 keep[DECODE ? 2 : 4];
+    if (LATE_WORDS && have_words) words = mask_words<DECODE ? 2 : 4>(c.rowbits, n0);
     mask_bits(keep, use_mask, n0, qi, gb, gh, p.Skv, have_words, words);
     mask_apply(s0, keep[0]);
     mask_apply(s1, keep[1]);
@@ -894,7 +898,6 @@ extern "C" __global__ void __launch_bounds__(fa_tc::NT, fa_tc::NQ == 1 ? 2 : 1) 
     auto do_s = [&](int j, fa_u32 wj) {
       if (active(wj)) {
         if (ns > 0 && !fa_mbar_wait_all(bar_addr(sb, BAR_SFREE2 + i), (ns - 1) & 1u, abort_flag)) return false;
-        if (NQ == 2 && i == 0 && ns == 1 && leader) fa_mbar_arrive(bar_addr(sb, BAR_LAG));
         fa_tc_fence_after();
         const fa_u32 loK = fa_desc_lo(sb + OFF_K + (j % NSTAGE) * KV_STAGE, 16);
         const fa_u32 t_s = tmem_u + COL_S + i * S_STRIDE + (ns & 1u) * 64u;
@@ -912,10 +915,13 @@ extern "C" __global__ void __launch_bounds__(fa_tc::NT, fa_tc::NQ == 1 ? 2 : 1) 
     fa_u32 w = word(0);
     if (ok && nsteps_u > 0) {
       ok = wait_k(0);
-      // The second tile starts when the first has its scores in registers, and the two stay apart like that: in step,
-      // the loads and waits of one do not run under the exponentials of the other (us, in step / apart by the loads /
-      // apart by a whole step: dense B4 H8 S4096 226 / 198 / 208, causal B2 H8 S8192 212 / 198 / 198).
-      if (NQ == 2 && i == 1 && nsteps_u > 1 && ((w >> 16) & 0xffu) != 0u && ((word(1) >> 16) & 0xffu) != 0u && active(w))
+      // The first tile starts when the first PV product of the second is complete, and the two stay apart like that: in step, the loads
+      // and waits of one do not run under the exponentials of the other.  us, in step / apart by the loads / by this: dense B2 H8 S8192 420 / 375 /
+      // 380, B1 H4 S8192 113.5 / 112.6 / 109.5, S2304 (16 heads) 37.7 / 37.4 / 35.0, causal B1 H8 S8192 109 / 111 / 103, B2 H8 S8192 206 / 195 / 191,
+      // S4096 61.9 / 60.2 / 58.8, B8 H8 S4096 226 / 212 / 214, ALiBi B2 H8 S8192 493 / 445 / 442.  The second tile goes first since under a
+      // causal mask it has a step more, and without one it is faster too (first tile first, by the loads: causal B2 H8 S8192 199, B1 H8
+      // 110, dense B1 H8 S8192 205 against 200).  Turns at every step, each tile's scores behind the other's loads, were slower (dense B2 H8 S8192 415).
+      if (NQ == 2 && i == 0 && nsteps_u > 1 && ((w >> 24) & 0xffu) != 0u && ((word(1) >> 24) & 0xffu) != 0u && active(w))
         ok = ok && fa_mbar_wait_all(bar_addr(sb, BAR_LAG), 0, abort_flag);
       ok = ok && do_s(0, w);
     }
@@ -938,6 +944,7 @@ extern "C" __global__ void __launch_bounds__(fa_tc::NT, fa_tc::NQ == 1 ? 2 : 1) 
           for (int kk = 0; kk < BN / 16; ++kk)
             fa_mma_ts(t_o, t_p + kk * 8, fa_desc_make(loV + kk * 128, HI), IDESC_O, (cnt > 0) | (kk > 0));
           fa_mma_commit(bar_addr(sb, BAR_O + odd));
+          if (NQ == 2 && i == 1 && cnt == 0) fa_mma_commit(bar_addr(sb, BAR_LAG));
         }
         ++cnt;
       }
