@@ -138,6 +138,7 @@ constexpr int REGS_LAUNCH = NQ == 2 ? 168 : 128, REGS_SOFTMAX = NQ == 2 ? 200 : 
 static_assert(NQ * (REGS_SOFTMAX - REGS_LAUNCH) <= REGS_LAUNCH - REGS_OTHER, "setmaxnreg.inc would wait forever");
 constexpr int WARP_PRODUCER = NSOFT, WARP_MMA = NSOFT + 1, WARP_MMA_B = NSOFT + 2;
 constexpr float RESCALE_THRESHOLD = 8.0f;  // log2 units
+constexpr float REL_FLOOR = -64.0f;         // log2 units
 
 static_assert(D == 64 || D == 128, "head dim 64 or 128");
 static_assert(!DECODE || D == 64, "the decode variant is written for head dim 64");
@@ -179,8 +180,8 @@ __device__ __forceinline__ void max_chunk(const float (&v)[32], RowMax& mx) {
   }
 }
 // score_mod (and the rounding of the raw scores to the input type, when asked for) in place.  With a score_mod the
-// results are in log2 units and relative to the row's running maximum (negm is added): where that does not move, the
-// exponentials are taken of them as they are, without a subtraction of their own.  An affine score_mod
+// results are in log2 units and relative to the row's running maximum (negm is added; not where that is far below 0, see
+// m_base): where that does not move, the exponentials are taken of them as they are, without a subtraction of their own.  An affine score_mod
 // (A * score + B) costs one packed FMA per pair: A and B absorb the scale, log2(e) and the maximum.
 // (Without a score_mod the scores stay raw, the exponent's FMA applies the scale.)
 struct ModLinear {
@@ -335,8 +336,10 @@ __device__ __forceinline__ bool softmax_step(SoftmaxCtx& c, const int tile, cons
   const int n0 = tile * BN + (DECODE ? c.half * 64 : 0);
   const fa_u32 t_sh = DECODE ? t_s + c.half * 64 : t_s;
   constexpr bool REL = FA_HAS_SCORE_MOD;
-  // what the scores are taken relative to (REL): the running maximum, 0 while the row has none
-  const float m_base = m_ref == FA_NEG_INF ? 0.f : m_ref;
+  // What the scores are taken relative to (REL): the running maximum; 0 while the row has none, and where it is far below 0: a score_mod that
+  // puts -1e30 in the place of scores makes it the maximum of a row whose first tile has no others, and added to that the
+  // scores of later tiles are lost (at -1e4 all but their first bits).  From -64 on what they lose is below 2^-18.
+  const float m_base = m_ref >= REL_FLOOR ? m_ref : 0.f;
   ModLinear lin = {};
 #if FA_HAS_SCORE_MOD && defined(FA_SCORE_AFFINE) && defined(FA_SCORE_LINEAR_KV)
   lin = c.lin;
@@ -407,17 +410,16 @@ __device__ __forceinline__ bool softmax_step(SoftmaxCtx& c, const int tile, cons
   // running maximum, raised lazily
   const float m_new = fmaxf(m_ref, REL ? m_base + mx : mx);
   bool need = false;
-  float corr = 1.f, delta = 0.f;
+  float corr = 1.f;
   if (m_ref == FA_NEG_INF) {
     m_ref = m_new;  // nothing accumulated yet for this row
-    if (REL && m_new != FA_NEG_INF) delta = m_new;
   } else if (m_new - m_ref > RESCALE_THRESHOLD) {
     need = true;
-    delta = m_new - m_ref;
-    corr = fa_ex2(-delta);
+    corr = fa_ex2(m_ref - m_new);
     m_ref = m_new;
     l *= corr;
   }
+  const float delta = REL && m_ref != FA_NEG_INF ? m_ref - m_base : 0.f;
   const bool rescale = cnt > 0 && __any_sync(0xffffffffu, need);
   if (cnt > 0 && (DECODE || rescale)) {
     // O is rescaled in place, and with separate P columns the previous PV product reads the P columns that are
@@ -439,7 +441,7 @@ __device__ __forceinline__ bool softmax_step(SoftmaxCtx& c, const int tile, cons
     }
   }
   if (REL && __any_sync(0xffffffffu, delta != 0.f)) {
-    // the maximum has moved (the first step of a row, hardly ever later): the scores follow it
+    // the maximum has moved (the first step of a row, hardly ever later) or is far below 0: the scores follow it
     const fa_u64 nd = fa_f2(-delta, -delta);
 #pragma unroll
     for (int e = 0; e < 32; e += 2) {
