@@ -339,11 +339,17 @@ __device__ __forceinline__ bool softmax_step(SoftmaxCtx& c, const int tile, cons
   // What the scores are taken relative to (REL): the running maximum; 0 while the row has none, and where it is far below 0: a score_mod that
   // puts -1e30 in the place of scores makes it the maximum of a row whose first tile has no others, and added to that the
   // scores of later tiles are lost (at -1e4 all but their first bits).  From -64 on what they lose is below 2^-18.
-  const float m_base = m_ref >= REL_FLOOR ? m_ref : 0.f;
+  // A bias that is linear over the keys says by itself where the scores of the tile are: the bias of its first key takes the place of a
+  // maximum that is more than 16 below, and of none.  (A large bias is then rounded once a tile: taken from 0 it would be rounded
+  // at the eighth keys, at every key and in the sum again.)
   ModLinear lin = {};
 #if FA_HAS_SCORE_MOD && defined(FA_SCORE_AFFINE) && defined(FA_SCORE_LINEAR_KV)
   lin = c.lin;
-  lin.b = fa_score_add2(0.f, gb, gh, qi, n0) - m_base;
+  const float bias0 = fa_score_add2(0.f, gb, gh, qi, n0);
+  const float m_base = bias0 - m_ref <= 16.f ? m_ref : (fabsf(bias0) < -FA_NEG_INF ? bias0 : 0.f);
+  lin.b = bias0 - m_base;
+#else
+  const float m_base = m_ref >= REL_FLOOR ? m_ref : 0.f;
 #endif
   const bool use_mask = FA_HAS_MASK_MOD && mode == 1;
   const bool have_words = masked && use_mask && c.rowbits != nullptr;
