@@ -1048,7 +1048,7 @@ extern "C" __global__ void __launch_bounds__(fa_tc::NT, fa_tc::NQ == 1 ? 2 : 1) 
         const bool more = j + 1 < nsteps_u;
         const fa_u32 w_next = more ? word(j + 1) : 0u;
         // (every step waits for its stage to be full before it releases it, with or without a product; where K of the
-        // next step is still on its way, PV goes first)
+        // next step is still on its way, PV of the first tile goes first)
         ok = wait_v(j);
         bool k_there = !more || (NSTAGE > 1 && have_k(j + 1));
 #pragma unroll (F32 ? 1 : NQ)

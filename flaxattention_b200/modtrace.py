@@ -1783,7 +1783,8 @@ class ModSet:
     def kv_tiles(self, Q_LEN: int, KV_LEN: int) -> int:
         """A guess at how many 128-key tiles the mask leaves of the keys per 128 query rows, 0 where there is none: what
         interval arithmetic does not rule out (``_range_walk``), the average over up to eight query tiles.  Masks over captured
-        tensors have none, but for document masks: at most eight, as many documents leave."""
+        tensors have none, but for document masks: at most eight, as many documents leave.  (Forward, us, two query tiles per
+        CTA against the one that eight asks for, head dim 128, B2 H8 S8192: 12 documents 75 / 67, 4 121 / 114, 3 148 / 133, 2 158 / 172.)"""
         if self.mask is None or self.mask_reads_b or self.mask_reads_h or (self.buffers and not self._documents):
             return 0
         n = self._kv_tiles.get((Q_LEN, KV_LEN))
