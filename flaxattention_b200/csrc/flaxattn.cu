@@ -256,7 +256,8 @@ int ready_kernel(Kernel* k) {
     FA_CUDA_CHECK(cudaLibraryLoadData(&k->lib, k->cubin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0));
     FA_CUDA_CHECK(cudaLibraryGetKernel(&k->fn, k->lib, k->entry.c_str()));
   }
-  if (k->smem > 48 * 1024)
+  // (the 48 KB that need no leave include static shared memory: the table of captured buffers, which a kernel has only with such mods)
+  if (k->smem > 32 * 1024)
     FA_CUDA_CHECK(cudaFuncSetAttribute((const void*)k->fn, cudaFuncAttributeMaxDynamicSharedMemorySize, k->smem));
   k->ready.fetch_or(bit, std::memory_order_release);
   return FA_OK;
